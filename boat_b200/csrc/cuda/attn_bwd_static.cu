@@ -61,7 +61,14 @@ int boat_cuda_attn_bwd_static(int mma, int64_t units, int64_t S, int64_t hs, int
                              "initialises the library, because initialising allocates");
     if (int rc = ensure_init()) return rc;     // already initialised: only makes the bound device current
     if (units < 0 || S < 0 || hs < 0) return set_error(41, "boat_cuda_attn_bwd_static: negative size");
-    const size_t need = boat_cuda_attn_bwd_scratch_bytes(mma, units, S, hs);
+    size_t need = boat_cuda_attn_bwd_scratch_bytes(mma, units, S, hs);
+    bool tensor_cores = true;
+    if (need > kStaticScratchBytes && S % 128 != 0) {
+        // A sequence that is no whole number of tiles: the CUDA-core kernels need no dQ buffer, so far
+        // larger problems of this kind fit the block with them.
+        tensor_cores = false;
+        need = boat_cuda_attn_bwd_scratch_bytes(BOAT_MMA_FP32, units, S, hs);
+    }
     if (need > kStaticScratchBytes)
         return set_error(42, "boat_cuda_attn_bwd_static: this problem needs %zu bytes of scratch, the built-in "
                              "block holds %zu; use boat_cuda_attn_bwd with your own scratch",
@@ -70,8 +77,8 @@ int boat_cuda_attn_bwd_static(int mma, int64_t units, int64_t S, int64_t hs, int
     if (int rc = scratch_address(&scratch)) return rc;
     // Everything the kernels expect to start from zero (the dQ sum) is cleared by the call
     // below on the library stream before it is used; the delta part is fully rewritten.
-    return boat_cuda_attn_bwd(mma, units, S, hs, causal, scale, Q, K, V, O, dO, lse, io_type, dQ, dK, dV, scratch,
-                              kStaticScratchBytes);
+    return attn_bwd_core(mma, tensor_cores, units, S, hs, causal, scale, Q, K, V, O, dO, lse, io_type, dQ, dK, dV, scratch,
+                         kStaticScratchBytes);
 }
 
 }  // extern "C"

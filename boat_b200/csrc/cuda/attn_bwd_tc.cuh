@@ -77,8 +77,9 @@ struct BwdCfg {
 };
 
 struct BwdParams {
-    const float* lse2;     // [units*S]  -lse * log2(e): the exponent offset in the log2 domain
-    const float* delta2;   // [units*S]  -delta / sqrt(hs)
+    const float* lse2;     // [units, whole tiles]  -lse * log2(e): the exponent offset in the log2 domain;
+                           // -inf beyond the end of the sequence, where P is then exactly zero
+    const float* delta2;   // [units, whole tiles]  -delta / sqrt(hs)
     float* dq_accum;       // [units*S, hs] FP32, zeroed before the launch
     void* dK;
     void* dV;
@@ -136,7 +137,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     volatile uint32_t* drain_ok = tmem_slot + 3;       // same idea for the dQ warps
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = p.S / kTile;
+    const int n_tiles = (p.S + kTile - 1) / kTile;
     // CTA order: units in groups of p.group; inside a group the key-tile pair is the slow index.
     // The CTAs that run at the same time then belong to a few (batch, head) units, so the FP32 dQ
     // rows they reduce into (S*HS*4 bytes per unit) and the unit's Q and dO stay in L2 - with
@@ -162,7 +163,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const int ibA = p.causal ? jtA : 0, ibB = p.causal ? jtB : 0;
     const int nA = n_tiles - ibA;                       // query tiles of the first walk
     const int n_q = nA + (has_b ? n_tiles - ibB : 0);   // of both
-    const int row_base = unit * p.S;
+    const int64_t stat_base = (int64_t)unit * n_tiles * kTile;    // the statistics are padded to whole tiles
     // query tile and key tile of step gt of the combined walk
     auto qtile = [&](int gt) { return gt < nA ? ibA + gt : ibB + gt - nA; };
 
@@ -198,14 +199,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // tensor-memory allocation and the CTA's first barrier.
         mbar_arrive_expect_tx(kv_full, 2 * C::TILE_BYTES);
         for (int b = 0; b < C::NBOX; ++b) {
-            tma_load_2d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 64, row_base + jtA * kTile);
-            tma_load_2d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 64, row_base + jtA * kTile);
+            tma_load_3d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 64, jtA * kTile, unit);
+            tma_load_3d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 64, jtA * kTile, unit);
         }
         for (int t = 0; t < n_q && t < C::Q_STAGES; ++t) {
             mbar_arrive_expect_tx(&do_full[t], C::TILE_BYTES);
             for (int b = 0; b < C::NBOX; ++b)
-                tma_load_2d(do_smem + t * C::TILE_BYTES + b * kBoxBytes, &map_do, &do_full[t], b * 64,
-                            row_base + qtile(t) * kTile);
+                tma_load_3d(do_smem + t * C::TILE_BYTES + b * kBoxBytes, &map_do, &do_full[t], b * 64, qtile(t) * kTile, unit);
         }
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -220,8 +220,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             auto load_kv = [&](int jt) {
                 mbar_arrive_expect_tx(kv_full, 2 * C::TILE_BYTES);
                 for (int b = 0; b < C::NBOX; ++b) {
-                    tma_load_2d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 64, row_base + jt * kTile);
-                    tma_load_2d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 64, row_base + jt * kTile);
+                    tma_load_3d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 64, jt * kTile, unit);
+                    tma_load_3d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 64, jt * kTile, unit);
                 }
             };
             for (int t = 0; t < n_q; ++t) {
@@ -233,14 +233,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 if (!mbar_wait(&q_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) break;
                 mbar_arrive_expect_tx(&q_full[s], C::TILE_BYTES);
                 for (int b = 0; b < C::NBOX; ++b)
-                    tma_load_2d(q_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[s], b * 64,
-                                row_base + qtile(t) * kTile);
+                    tma_load_3d(q_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[s], b * 64, qtile(t) * kTile, unit);
                 // the tile's 128 exponent offsets and 128 deltas, into the buffer of its parity once
                 // the tile before last has left it
                 if (!mbar_wait(&stat_empty[t & 1], ((t >> 1) & 1) ^ 1, p.status, kTimeoutProducer)) break;
                 mbar_arrive_expect_tx(&stat_full[t & 1], 1024);
-                bulk_load_1d(stat_s + (t & 1) * 256, p.lse2 + row_base + qtile(t) * kTile, 512, &stat_full[t & 1]);
-                bulk_load_1d(stat_s + (t & 1) * 256 + 128, p.delta2 + row_base + qtile(t) * kTile, 512, &stat_full[t & 1]);
+                bulk_load_1d(stat_s + (t & 1) * 256, p.lse2 + stat_base + qtile(t) * kTile, 512, &stat_full[t & 1]);
+                bulk_load_1d(stat_s + (t & 1) * 256 + 128, p.delta2 + stat_base + qtile(t) * kTile, 512, &stat_full[t & 1]);
             }
         }
     } else if (warp == 1) {
@@ -371,7 +370,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         auto store_dkdv = [&](int jt, uint32_t phase) -> bool {
             if (!mbar_wait_warp(all_done, phase, p.status, kTimeoutEpilogue)) return false;
             tc_fence_after_sync();
-            const int64_t grow = (int64_t)row_base + (int64_t)jt * kTile + r;
+            const int64_t grow = (int64_t)unit * p.S + (int64_t)jt * kTile + r;
+            const bool live = jt * kTile + r < p.S;
             __nv_bfloat16* out = (__nv_bfloat16*)(half ? p.dK : p.dV) + grow * HS;
             const uint32_t col = half ? C::COL_DK : C::COL_DV;
 #pragma unroll 1
@@ -379,6 +379,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 uint32_t v[32];
                 tmem_ld32(tmem_base + col + lane_addr + c * 32, v);
                 tmem_wait_ld();
+                if (!live) continue;
 #pragma unroll
                 for (int x = 0; x < 32; x += 8) {
                     uint4 o;
@@ -391,6 +392,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
             return true;
         };
+        auto key_live = [&](int t) { return (t < nA ? jtA : jtB) * kTile + r < p.S; };
         for (int t = 0; t < n_q; ++t) {
             const int i = qtile(t);
             // -lse*log2e and -delta/sqrt(hs) of this query tile, put into the buffer of this tile's
@@ -446,6 +448,12 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 };
                 if (diag) phase_a(std::true_type{});
                 else      phase_a(std::false_type{});
+                // A key row beyond the end of the sequence has zero scores, whose exp2(-lse) may overflow;
+                // its dS^T meets a zero row of K, so it has to be a number.
+                if (!key_live(t)) {
+#pragma unroll
+                    for (int x = 0; x < 32; ++x) ph[x] = 0u;
+                }
                 // P^T over this thread's own S^T columns: 64 BF16 = 32 columns starting at col0
                 tmem_st32(tmem_base + C::COL_S + lane_addr + col0, ph);
             }
@@ -524,7 +532,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             named_barrier_sync(2, 128);
             if (drain_ok[0] == 0u) break;
             tc_fence_after_sync();
-            const int y = row_base + qtile(t) * kTile;
+            const int y = qtile(t) * kTile;
             uint8_t* stage = do_smem + s * C::TILE_BYTES;
             auto stage_box = [&](const uint32_t (&v)[32], int slot) {
                 uint8_t* row = stage + slot * kBoxBytes + r * 128;
@@ -543,7 +551,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             named_barrier_sync(2, 128);
             if (tid128 == 0) {
                 for (int b = 0; b < C::NBOX; ++b) {
-                    tma_reduce_add_2d(&map_dq, stage + b * kBoxBytes, b * 32, y);
+                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, b * 32, y, unit);
                     tma_commit_group();
                 }
             }
@@ -564,7 +572,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 fence_proxy_async_smem();
                 named_barrier_sync(2, 128);
                 if (tid128 == 0) {
-                    tma_reduce_add_2d(&map_dq, stage + b * kBoxBytes, (C::NBOX + b) * 32, y);
+                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, (C::NBOX + b) * 32, y, unit);
                     tma_commit_group();
                 }
             }
@@ -572,8 +580,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
                 for (int b = 0; b < C::NBOX; ++b) {
                     wait_read(C::NBOX - 1 - b);             // the last group that used slot b has been read
-                    tma_load_2d(stage + b * kBoxBytes, &map_do, &do_full[s], b * 64,
-                                row_base + qtile(t + C::Q_STAGES) * kTile);
+                    tma_load_3d(stage + b * kBoxBytes, &map_do, &do_full[s], b * 64, qtile(t + C::Q_STAGES) * kTile, unit);
                 }
             }
         }

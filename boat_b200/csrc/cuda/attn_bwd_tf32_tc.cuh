@@ -93,11 +93,10 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     uint32_t* tmem_slot = (uint32_t*)(bars + 6);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = p.S / kTile;
+    const int n_tiles = (p.S + kTile - 1) / kTile;
     const int unit = blockIdx.x % p.units;
     const int qt = n_tiles - 1 - blockIdx.x / p.units;       // long (late) rows first when causal
     const int n_kv = p.causal ? qt + 1 : n_tiles;
-    const int row_base = unit * p.S;
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -125,17 +124,17 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             bool ok = true;
             mbar_arrive_expect_tx(q_full, 2 * kBwd32Tile);
             for (int b = 0; b < 2; ++b) {
-                tma_load_2d(q_smem + b * kBoxBytes, &map_q, q_full, b * 32, row_base + qt * kTile);
-                tma_load_2d(do_smem + b * kBoxBytes, &map_do, q_full, b * 32, row_base + qt * kTile);
+                tma_load_3d(q_smem + b * kBoxBytes, &map_q, q_full, b * 32, qt * kTile, unit);
+                tma_load_3d(do_smem + b * kBoxBytes, &map_do, q_full, b * 32, qt * kTile, unit);
             }
             for (int j = 0; j < n_kv && ok; ++j) {
                 if (!mbar_wait(kv_empty, (j & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
                 mbar_arrive_expect_tx(kv_full, 3 * kBwd32Tile);
-                const int y = row_base + j * kTile;
+                const int y = j * kTile;
                 for (int b = 0; b < 2; ++b) {
-                    tma_load_2d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 32, y);
-                    tma_load_2d(kmn_smem + b * kBoxBytes, &map_k_mn, kv_full, b * 32, y);
-                    tma_load_2d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 32, y);
+                    tma_load_3d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 32, y, unit);
+                    tma_load_3d(kmn_smem + b * kBoxBytes, &map_k_mn, kv_full, b * 32, y, unit);
+                    tma_load_3d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 32, y, unit);
                 }
             }
             if (!ok)
@@ -179,15 +178,18 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const int lane_group = warp & 3;
         const int r_in_tile = lane_group * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(lane_group * 32) << 16;
-        const int64_t grow = (int64_t)row_base + (int64_t)qt * kTile + r_in_tile;
+        const int64_t grow = (int64_t)unit * p.S + (int64_t)qt * kTile + r_in_tile;
+        const bool live = qt * kTile + r_in_tile < p.S;         // a row of the sequence (the last tile may be short)
         const float sl2 = p.scale * 1.4426950408889634f;
-        const float neg_lse2 = -p.lse[grow] * 1.4426950408889634f;
-        const float neg_delta_s = -p.delta[grow] * p.scale;
+        const float neg_lse2 = live ? -p.lse[grow] * 1.4426950408889634f : 0.f;
+        const float neg_delta_s = live ? -p.delta[grow] * p.scale : 0.f;
         bool ok = true;
         for (int j = 0; j < n_kv; ++j) {
             if (!mbar_wait(s_full, j & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
             tc_fence_after_sync();
-            const bool diag = p.causal && j == qt;
+            // keys beyond the diagonal, or without a mask beyond the end of the sequence
+            const bool masked = p.causal ? j == qt : j == n_tiles - 1;
+            const int last = p.causal ? r_in_tile : p.S - 1 - j * kTile;
 #pragma unroll 1
             for (int c = 0; c < kTile / 32; ++c) {
                 uint32_t s[32], d[32];
@@ -197,7 +199,7 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
                 for (int i = 0; i < 32; ++i) {
                     float pr = fast_exp2(fmaf(__uint_as_float(s[i]), sl2, neg_lse2));
-                    if (diag && c * 32 + i > r_in_tile) pr = 0.f;
+                    if (masked && c * 32 + i > last) pr = 0.f;
                     // P * (dP - delta) / sqrt(hs)
                     s[i] = to_tf32(pr * fmaf(__uint_as_float(d[i]), p.scale, neg_delta_s));
                 }
@@ -215,6 +217,7 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 uint32_t r[32];
                 tmem_ld32(tmem_dq + lane_addr + c * 32, r);
                 tmem_wait_ld();
+                if (!live) continue;
 #pragma unroll
                 for (int i = 0; i < 32; i += 4)
                     *reinterpret_cast<float4*>(out + c * 32 + i) =
@@ -261,12 +264,11 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     volatile uint32_t* wait_ok = tmem_slot + 1;      // [2] outcome of the bounded wait, by tile parity
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tiles = p.S / kTile;
+    const int n_tiles = (p.S + kTile - 1) / kTile;
     const int unit = blockIdx.x % p.units;
     const int jt = blockIdx.x / p.units;                     // early key tiles have the long walks when causal
     const int i0 = p.causal ? jt : 0;
     const int n_q = n_tiles - i0;
-    const int row_base = unit * p.S;
 
     if (threadIdx.x == 0) {
         mbar_init(kv_full, 1);
@@ -296,18 +298,18 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             bool ok = true;
             mbar_arrive_expect_tx(kv_full, 2 * kBwd32Tile);
             for (int b = 0; b < 2; ++b) {
-                tma_load_2d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 32, row_base + jt * kTile);
-                tma_load_2d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 32, row_base + jt * kTile);
+                tma_load_3d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 32, jt * kTile, unit);
+                tma_load_3d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 32, jt * kTile, unit);
             }
             for (int t = 0; t < n_q && ok; ++t) {
                 if (!mbar_wait(q_empty, (t & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
                 mbar_arrive_expect_tx(q_full, 4 * kBwd32Tile);
-                const int y = row_base + (i0 + t) * kTile;
+                const int y = (i0 + t) * kTile;
                 for (int b = 0; b < 2; ++b) {
-                    tma_load_2d(q_smem + b * kBoxBytes, &map_q, q_full, b * 32, y);
-                    tma_load_2d(qmn_smem + b * kBoxBytes, &map_q_mn, q_full, b * 32, y);
-                    tma_load_2d(do_smem + b * kBoxBytes, &map_do, q_full, b * 32, y);
-                    tma_load_2d(domn_smem + b * kBoxBytes, &map_do_mn, q_full, b * 32, y);
+                    tma_load_3d(q_smem + b * kBoxBytes, &map_q, q_full, b * 32, y, unit);
+                    tma_load_3d(qmn_smem + b * kBoxBytes, &map_q_mn, q_full, b * 32, y, unit);
+                    tma_load_3d(do_smem + b * kBoxBytes, &map_do, q_full, b * 32, y, unit);
+                    tma_load_3d(domn_smem + b * kBoxBytes, &map_do_mn, q_full, b * 32, y, unit);
                 }
             }
             if (!ok)
@@ -365,9 +367,11 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             // buffer, and it cannot reach tile t+2 before every thread has passed the barrier of t+1.
             float* lse_s = stat_s + (t & 1) * 256;
             float* delta_s = lse_s + 128;
-            const int64_t qrow = (int64_t)row_base + (int64_t)i * kTile + tid;
-            lse_s[tid] = p.lse[qrow] * -1.4426950408889634f;
-            delta_s[tid] = p.delta[qrow] * -p.scale;
+            // Queries beyond the end of the sequence get an offset of -inf: their P is exactly zero.
+            const int64_t qrow = (int64_t)unit * p.S + (int64_t)i * kTile + tid;
+            const bool query = i * kTile + tid < p.S;
+            lse_s[tid] = query ? p.lse[qrow] * -1.4426950408889634f : -INFINITY;
+            delta_s[tid] = query ? p.delta[qrow] * -p.scale : 0.f;
             // One thread does the bounded wait and publishes the outcome, so that all 128 take the
             // same branch and nobody is left alone at the named barrier of the next tile.  The flag
             // of this parity is rewritten two tiles later, after the barrier of the tile in between.
@@ -405,7 +409,8 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         // every thread waits for itself here: no barrier follows
         if (ok && mbar_wait(acc_done, 0, p.status, kTimeoutEpilogue)) {
             tc_fence_after_sync();
-            const int64_t grow = (int64_t)row_base + (int64_t)jt * kTile + r;
+            const int64_t grow = (int64_t)unit * p.S + (int64_t)jt * kTile + r;
+            const bool live = jt * kTile + r < p.S;
 #pragma unroll 1
             for (int which = 0; which < 2; ++which) {
                 float* out = (which ? p.dK : p.dV) + grow * HS;
@@ -415,6 +420,7 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     uint32_t v[32];
                     tmem_ld32(col + lane_addr + c * 32, v);
                     tmem_wait_ld();
+                    if (!live) continue;
 #pragma unroll
                     for (int x = 0; x < 32; x += 4)
                         *reinterpret_cast<float4*>(out + c * 32 + x) =

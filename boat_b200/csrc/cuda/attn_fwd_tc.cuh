@@ -62,7 +62,7 @@ struct FwdCfg {
 struct FwdParams {
     void* O;
     float* lse;
-    int S;             // sequence length (multiple of 128)
+    int S;             // sequence length
     int units;
     int causal;
     float scale;       // 1/sqrt(hs)
@@ -135,7 +135,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     uint32_t* tmem_slot = (uint32_t*)(o_done + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q_tiles = p.S / kTile;
+    const int q_tiles = (p.S + kTile - 1) / kTile;
     const int n_pairs = (q_tiles + 1) / 2;
     // CTA order: units in groups of p.group, so that the K and V tiles which the CTAs running at one
     // time stream through shared memory (every CTA of a unit reads all of the unit's K and V) stay
@@ -164,7 +164,9 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const int n_a = p.causal ? qt_a + 1 : q_tiles;
     const int n_b = has_b ? (p.causal ? qt_b + 1 : q_tiles) : 0;
     const int n_kv = n_a > n_b ? n_a : n_b;
-    const int row_base = unit * p.S;                       // first row of this unit in [units*S, hs]
+    // A last tile that is only partly filled: its missing rows read as zeros (the tensor maps end with
+    // the unit), missing query rows are not stored, missing keys are masked.
+    const int tail = p.S - (q_tiles - 1) * kTile;          // rows of the last tile
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -189,16 +191,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         mbar_arrive_expect_tx(q_full, (has_b ? 2 : 1) * C::TILE_BYTES);
         for (int g = 0; g < (has_b ? 2 : 1); ++g)
             for (int b = 0; b < C::NBOX; ++b)
-                tma_load_2d(q_smem + g * C::TILE_BYTES + b * kBoxBytes, &map_q, q_full, b * C::BOXC,
-                            row_base + (qt_a + g) * kTile);
+                tma_load_3d(q_smem + g * C::TILE_BYTES + b * kBoxBytes, &map_q, q_full, b * C::BOXC, (qt_a + g) * kTile, unit);
         for (int j = 0; j < n_kv && j < ST; ++j) {
-            const int y = row_base + j * kTile;
+            const int y = j * kTile;
             mbar_arrive_expect_tx(&k_full[j], C::TILE_BYTES);
             for (int b = 0; b < C::NBOX; ++b)
-                tma_load_2d(k_smem + j * C::TILE_BYTES + b * kBoxBytes, &map_k, &k_full[j], b * C::BOXC, y);
+                tma_load_3d(k_smem + j * C::TILE_BYTES + b * kBoxBytes, &map_k, &k_full[j], b * C::BOXC, y, unit);
             mbar_arrive_expect_tx(&v_full[j], C::TILE_BYTES);
             for (int b = 0; b < C::NBOX; ++b)
-                tma_load_2d(v_smem + j * C::TILE_BYTES + b * kBoxBytes, &map_v, &v_full[j], b * C::BOXC, y);
+                tma_load_3d(v_smem + j * C::TILE_BYTES + b * kBoxBytes, &map_v, &v_full[j], b * C::BOXC, y, unit);
         }
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
@@ -214,15 +215,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             for (int j = ST; j < n_kv && ok; ++j) {               // the first ST tiles are on their way
                 const int s = j % ST;
                 const uint32_t par = ((j / ST) & 1) ^ 1;
-                const int y = row_base + j * kTile;
+                const int y = j * kTile;
                 if (!mbar_wait(&k_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
                 mbar_arrive_expect_tx(&k_full[s], C::TILE_BYTES);
                 for (int b = 0; b < C::NBOX; ++b)
-                    tma_load_2d(k_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_k, &k_full[s], b * C::BOXC, y);
+                    tma_load_3d(k_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_k, &k_full[s], b * C::BOXC, y, unit);
                 if (!mbar_wait(&v_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
                 mbar_arrive_expect_tx(&v_full[s], C::TILE_BYTES);
                 for (int b = 0; b < C::NBOX; ++b)
-                    tma_load_2d(v_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_v, &v_full[s], b * C::BOXC, y);
+                    tma_load_3d(v_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_v, &v_full[s], b * C::BOXC, y, unit);
             }
             if (!ok)
                 for (int i = 0; i < 1000; ++i) __nanosleep(1000);
@@ -308,7 +309,10 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         for (int j = 0; j < n_g; ++j) {
             if (!mbar_wait(&s_full[g], j & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
             tc_fence_after_sync();
-            const bool diag = p.causal && j == qt;
+            // Keys this row does not see in this tile: beyond the diagonal, or - without a mask - beyond the
+            // end of the sequence (under the mask no stored row reaches that far).
+            const bool masked = p.causal ? j == qt : (j == q_tiles - 1 && tail < kTile);
+            const int last = p.causal ? r_in_tile : tail - 1;
             // The whole row of scores (128 columns) comes into registers with one wait; the maximum and
             // the exponentials both work from there.
             uint32_t sc[kTile];
@@ -316,16 +320,16 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             for (int c = 0; c < kTile / 32; ++c)
                 tmem_ld32(tmem_s + lane_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(sc + c * 32));
             tmem_wait_ld();
-            // row maximum of the visible scores (the mask only exists on the diagonal tile)
+            // row maximum of the visible scores (the mask exists in one tile only)
             float tmax;
             {
                 float t8[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) t8[i] = -FLT_MAX;
-                if (diag) {
+                if (masked) {
 #pragma unroll
                     for (int i = 0; i < kTile; ++i)
-                        t8[i & 7] = fmaxf(t8[i & 7], i <= r_in_tile ? __uint_as_float(sc[i]) : -FLT_MAX);
+                        t8[i & 7] = fmaxf(t8[i & 7], i <= last ? __uint_as_float(sc[i]) : -FLT_MAX);
                 } else {
 #pragma unroll
                     for (int i = 0; i < kTile; i += 2)
@@ -363,7 +367,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             const float neg_m = -m_ref * sl2;
             float lsum;
             {
-                lsum = diag ? exp_row<TF32, true>(sc, sl2, neg_m, r_in_tile) : exp_row<TF32, false>(sc, sl2, neg_m, r_in_tile);
+                lsum = masked ? exp_row<TF32, true>(sc, sl2, neg_m, last) : exp_row<TF32, false>(sc, sl2, neg_m, r_in_tile);
                 constexpr int P_CHUNKS = TF32 ? kTile / 32 : kTile / 64;
 #pragma unroll
                 for (int c = 0; c < P_CHUNKS; ++c)
@@ -378,13 +382,15 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (n_g > 0 && ok && mbar_wait(o_done, 0, p.status, kTimeoutEpilogue)) {
             tc_fence_after_sync();
             const float inv = 1.f / l;
-            const int64_t grow = (int64_t)row_base + (int64_t)qt * kTile + r_in_tile;
+            const int64_t grow = (int64_t)unit * p.S + (int64_t)qt * kTile + r_in_tile;
+            const bool live = qt * kTile + r_in_tile < p.S;
             T* out = (T*)p.O + grow * HS;
 #pragma unroll 1
             for (int c = 0; c < HS / 32; ++c) {
                 uint32_t r[32];
                 tmem_ld32(tmem_o + lane_addr + c * 32, r);
                 tmem_wait_ld();
+                if (!live) continue;
                 if (TF32) {
 #pragma unroll
                     // TF32-valued output: it feeds the TF32 output projection
@@ -408,7 +414,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     }
                 }
             }
-            p.lse[grow] = m_ref * p.scale + logf(l);
+            if (live) p.lse[grow] = m_ref * p.scale + logf(l);
         }
     }
     tc_fence_before_sync();

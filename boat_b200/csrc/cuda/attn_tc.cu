@@ -16,12 +16,11 @@ int launch_fwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
                void* O, float* lse) {
     using C = FwdCfg<T, HS>;
     CUtensorMap mq, mk, mv;
-    const uint64_t rows = (uint64_t)units * (uint64_t)S;
-    if (int rc = make_tensor_map_2d(&mq, Q, C::ES, rows, HS, HS, kTile, C::BOXC)) return rc;
-    if (int rc = make_tensor_map_2d(&mk, K, C::ES, rows, HS, HS, kTile, C::BOXC)) return rc;
+    if (int rc = make_tensor_map_units(&mq, Q, C::ES, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mk, K, C::ES, units, S, HS, kTile)) return rc;
     // V is read by the tensor core along its contiguous head dimension: FP32 needs the
     // 32-byte-unit swizzle for that
-    if (int rc = make_tensor_map_2d(&mv, V, C::ES, rows, HS, HS, kTile, C::BOXC, C::TF32)) return rc;
+    if (int rc = make_tensor_map_units(&mv, V, C::ES, units, S, HS, kTile, C::TF32)) return rc;
     FwdParams p;
     p.O = O;
     p.lse = lse;
@@ -46,7 +45,7 @@ int launch_fwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
         BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured = true;
     }
-    const int64_t grid = units * ((S / kTile + 1) / 2);      // one CTA per pair of query tiles
+    const int64_t grid = units * ((ceil_div(S, kTile) + 1) / 2);      // one CTA per pair of query tiles
     ProfileScope prof("attn_fwd_tc");
     kern<<<(unsigned)grid, kFwdThreads, C::SMEM, stream()>>>(mq, mk, mv, p);
     BOATCU_LAUNCH_OK("attn_fwd_tc");
@@ -56,8 +55,7 @@ int launch_fwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
 }  // namespace
 
 bool attn_tc_supported(int mma, int64_t units, int64_t S, int64_t hs, int io_type) {
-    if (S < kTile || S % kTile != 0) return false;
-    if (units * (S / kTile) > 0x7fffffffLL || units * S > 0x7fffffffLL) return false;
+    if (S < 1 || units * ceil_div(S, kTile) * kTile > 0x7fffffffLL) return false;
     if (mma == BOAT_MMA_BF16) return io_type == BOAT_CUDA_BF16 && (hs == 64 || hs == 128);
     if (mma == BOAT_MMA_TF32) return io_type == BOAT_CUDA_F32 && hs == 64;
     return false;
@@ -82,16 +80,17 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
                float* stats2) {
     using C = BwdCfg<HS>;
     CUtensorMap mq, mk, mv, mdo, mdq;
-    const uint64_t rows = (uint64_t)units * (uint64_t)S;
-    if (int rc = make_tensor_map_2d(&mq, Q, 2, rows, HS, HS, kTile, 64)) return rc;
-    if (int rc = make_tensor_map_2d(&mk, K, 2, rows, HS, HS, kTile, 64)) return rc;
-    if (int rc = make_tensor_map_2d(&mv, V, 2, rows, HS, HS, kTile, 64)) return rc;
-    if (int rc = make_tensor_map_2d(&mdo, dO, 2, rows, HS, HS, kTile, 64)) return rc;
-    if (int rc = make_tensor_map_2d(&mdq, dq_accum, 4, rows, HS, HS, kTile, 32)) return rc;   // FP32 reduce-add target
+    const int64_t n_tiles = ceil_div(S, kTile);
+    const int64_t stat_rows = units * n_tiles * kTile;        // the statistics are padded to whole tiles
+    if (int rc = make_tensor_map_units(&mq, Q, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mk, K, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mv, V, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mdo, dO, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mdq, dq_accum, 4, units, S, HS, kTile)) return rc;   // FP32 reduce-add target
     const size_t n = (size_t)units * (size_t)S * HS;
     BwdParams p;
     p.lse2 = stats2;
-    p.delta2 = stats2 + rows;
+    p.delta2 = stats2 + stat_rows;
     p.dq_accum = dq_accum;
     p.dK = dK;
     p.dV = dV;
@@ -106,7 +105,6 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     // equalise the CTAs when causal: 5-10 % at 8- and 16-tile walks.  With equal CTAs the last
     // wave is a loss that many short CTAs would fill, and at 64-tile walks the per-CTA cost is
     // small anyway (measured: no gain at 64 tiles, 10 % slower when only 3.5 waves of pairs exist).
-    const int64_t n_tiles = S / kTile;
     p.pair = (n_tiles <= 32 && units * ((n_tiles + 1) / 2) >= 8 * (int64_t)sm_count()) ? 1 : 0;
     {
         // BOAT_BWD_PAIR=0/1 in the environment overrides the rule; it is read at every launch so
@@ -126,12 +124,12 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
         // the per-row statistics in the form the kernel's inner loops consume them:
         // -lse * log2(e) and -scale * rowsum(dO o O)
         ProfileScope prof("attn_delta");
-        if (int rc = rowdot_stats(dO, O, BOAT_CUDA_BF16, (int64_t)rows, HS, lse, scale, stats2 + rows, stats2)) return rc;
+        if (int rc = rowdot_stats(dO, O, BOAT_CUDA_BF16, units, S, n_tiles * kTile, HS, lse, scale, stats2 + stat_rows, stats2)) return rc;
     }
     {
         ProfileScope prof("attn_bwd_tc");
         BOATCU_CHECK(cudaMemsetAsync(dq_accum, 0, n * sizeof(float), stream()));
-        const int64_t grid = units * (p.pair ? (S / kTile + 1) / 2 : S / kTile);
+        const int64_t grid = units * (p.pair ? (n_tiles + 1) / 2 : n_tiles);
         kern<<<(unsigned)grid, kBwdThreads, C::SMEM, stream()>>>(mq, mk, mv, mdo, mdq, p);
         BOATCU_LAUNCH_OK("attn_bwd_tc");
         // the summed FP32 contributions become the BF16 output
@@ -147,16 +145,15 @@ int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const voi
     using C = Bwd32Cfg;
     constexpr int HS = kBwd32HS;
     CUtensorMap mq, mq_mn, mk, mk_mn, mv, mdo, mdo_mn;
-    const uint64_t rows = (uint64_t)units * (uint64_t)S;
     // the same matrices with both shared-memory layouts: 16-byte swizzle units for operands read
     // along hs, 32-byte units for operands read along their rows
-    if (int rc = make_tensor_map_2d(&mq, Q, 4, rows, HS, HS, kTile, 32)) return rc;
-    if (int rc = make_tensor_map_2d(&mq_mn, Q, 4, rows, HS, HS, kTile, 32, true)) return rc;
-    if (int rc = make_tensor_map_2d(&mk, K, 4, rows, HS, HS, kTile, 32)) return rc;
-    if (int rc = make_tensor_map_2d(&mk_mn, K, 4, rows, HS, HS, kTile, 32, true)) return rc;
-    if (int rc = make_tensor_map_2d(&mv, V, 4, rows, HS, HS, kTile, 32)) return rc;
-    if (int rc = make_tensor_map_2d(&mdo, dO, 4, rows, HS, HS, kTile, 32)) return rc;
-    if (int rc = make_tensor_map_2d(&mdo_mn, dO, 4, rows, HS, HS, kTile, 32, true)) return rc;
+    if (int rc = make_tensor_map_units(&mq, Q, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mq_mn, Q, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_units(&mk, K, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mk_mn, K, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_units(&mv, V, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mdo, dO, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mdo_mn, dO, 4, units, S, HS, kTile, true)) return rc;
     Bwd32Params p;
     p.lse = lse;
     p.delta = delta;
@@ -174,7 +171,7 @@ int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const voi
         BOATCU_CHECK(cudaFuncSetAttribute(attn_bwd_dkv_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_DKV));
         configured = true;
     }
-    const unsigned grid = (unsigned)(units * (S / kTile));
+    const unsigned grid = (unsigned)(units * ceil_div(S, kTile));
     ProfileScope prof("attn_bwd_tc");
     attn_bwd_dkv_tf32_kernel<<<grid, kBwd32Threads, C::SMEM_DKV, stream()>>>(mq, mq_mn, mk, mv, mdo, mdo_mn, p);
     BOATCU_LAUNCH_OK("attn_bwd_dkv_tf32");
@@ -186,10 +183,12 @@ int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const voi
 }  // namespace
 
 // Scratch of the BF16 tensor-core backward: the FP32 accumulation buffer of dQ, then the two
-// pre-scaled statistics per row.  (units*S is a multiple of 128, so both parts are 512-byte multiples.)
+// pre-scaled statistics per row, padded to whole 128-row tiles of every unit.  (The first part is a
+// multiple of 256 bytes, the parts of the second of 512.)
 size_t attn_bwd_tc_scratch_bytes(int mma, int64_t units, int64_t S, int64_t hs) {
     if (mma != BOAT_MMA_BF16) return 0;
-    return (size_t)units * (size_t)S * (size_t)hs * sizeof(float) + 2 * (size_t)units * (size_t)S * sizeof(float);
+    const size_t stat_rows = (size_t)units * (size_t)ceil_div(S, kTile) * kTile;
+    return (size_t)units * (size_t)S * (size_t)hs * sizeof(float) + 2 * stat_rows * sizeof(float);
 }
 
 int attn_bwd_tc(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,

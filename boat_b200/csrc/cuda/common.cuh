@@ -68,9 +68,10 @@ static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // out[r] = sum_d A[r,d]*B[r,d] over [rows, cols] row-major buffers of storage type `type`.
 int rowdot(const void* A, const void* B, int type, int64_t rows, int64_t cols, float* out);
 // The same pass emitting what the BF16 tensor-core backward reads per row:
-// delta2_out[r] = -scale * sum_d dO[r,d]*O[r,d] and lse2_out[r] = -lse[r] * log2(e).
-int rowdot_stats(const void* dO, const void* O, int type, int64_t rows, int64_t cols, const float* lse, float scale,
-                 float* delta2_out, float* lse2_out);
+// delta2_out[r] = -scale * sum_d dO[r,d]*O[r,d] and lse2_out[r] = -lse[r] * log2(e), each unit of S
+// rows padded to padded_S entries (0 and -inf).  units * padded_S must fit 31 bits.
+int rowdot_stats(const void* dO, const void* O, int type, int64_t units, int64_t S, int64_t padded_S, int64_t cols,
+                 const float* lse, float scale, float* delta2_out, float* lse2_out);
 
 // CUDA-core (exact FP32 accumulate) implementations, any shape.
 int gemm_simt(int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
@@ -80,6 +81,12 @@ int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale,
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, const void* dO, const float* lse, const float* delta, int io_type,
                   void* dQ, void* dK, void* dV);
+
+// boat_cuda_attn_bwd with a say in the kernels: without `tensor_cores` the CUDA-core ones, whose scratch is
+// what boat_cuda_attn_bwd_scratch_bytes gives for FP32 (delta only).
+int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,
+                  const void* K, const void* V, const void* O, const void* dO, const float* lse, int io_type, void* dQ,
+                  void* dK, void* dV, void* scratch, size_t scratch_bytes);
 
 // tcgen05 implementations; return -1 (without setting an error) when the shape is outside
 // what the tensor-core kernels cover, so that the dispatcher can say so.

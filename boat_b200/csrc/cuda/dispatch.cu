@@ -1,7 +1,7 @@
 // dispatch.cu - the extern "C" contraction and attention-core entry points: argument checks
 // and the choice between the tcgen05 kernels and the CUDA-core kernels.  The choice is by
 // shape only: a TF32 or BF16 request whose shape the tensor-core kernels do not cover
-// (sequence not a multiple of 128, head size other than 64 / 128, tiny or unaligned GEMMs)
+// (head size other than 64 / 128, tiny or unaligned GEMMs)
 // runs on the CUDA cores with the same storage types and FP32 FMA arithmetic - at least as
 // accurate as what was asked for, never less.
 #include "common.cuh"
@@ -100,18 +100,28 @@ size_t boat_cuda_attn_bwd_scratch_bytes(int mma, int64_t units, int64_t S, int64
 int boat_cuda_attn_bwd(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,
                        const void* K, const void* V, const void* O, const void* dO, const float* lse,
                        int io_type, void* dQ, void* dK, void* dV, void* scratch, size_t scratch_bytes) {
+    return attn_bwd_core(mma, true, units, S, hs, causal, scale, Q, K, V, O, dO, lse, io_type, dQ, dK, dV, scratch, scratch_bytes);
+}
+
+}  // extern "C"
+
+namespace boatcu {
+
+int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,
+                  const void* K, const void* V, const void* O, const void* dO, const float* lse, int io_type, void* dQ,
+                  void* dK, void* dV, void* scratch, size_t scratch_bytes) {
     if (int rc = check_types("boat_cuda_attn_bwd", mma, io_type)) return rc;
     if (io_type == BOAT_CUDA_F32_TF32) io_type = BOAT_CUDA_F32;
     if (units < 0 || S < 0 || hs < 0) return set_error(11, "boat_cuda_attn_bwd: negative size");
     if (units == 0 || S == 0 || hs == 0) return 0;
     if (!Q || !K || !V || !O || !dO || !lse || !dQ || !dK || !dV) return set_error(11, "boat_cuda_attn_bwd: NULL operand");
-    size_t need = boat_cuda_attn_bwd_scratch_bytes(mma, units, S, hs);
+    const size_t need = boat_cuda_attn_bwd_scratch_bytes(tensor_cores ? mma : (int)BOAT_MMA_FP32, units, S, hs);
     if (!scratch || scratch_bytes < need)
         return set_error(12, "boat_cuda_attn_bwd: scratch of %zu bytes given, %zu needed", scratch_bytes, need);
     if (((uintptr_t)scratch & 255) != 0) return set_error(12, "boat_cuda_attn_bwd: scratch must be 256-byte aligned");
     float* delta = (float*)scratch;
     size_t delta_bytes = ((size_t)units * (size_t)S * sizeof(float) + 255) & ~(size_t)255;
-    const bool tensor_cores = mma != BOAT_MMA_FP32 && attn_tc_supported(mma, units, S, hs, io_type);
+    tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && attn_tc_supported(mma, units, S, hs, io_type);
     if (!(tensor_cores && mma == BOAT_MMA_BF16)) {      // the BF16 kernel's launcher makes its own, pre-scaled
         ProfileScope prof("attn_delta");
         if (int rc = rowdot(dO, O, io_type, units * S, hs, delta)) return rc;
@@ -132,4 +142,4 @@ int boat_cuda_attn_bwd(int mma, int64_t units, int64_t S, int64_t hs, int causal
     return 0;
 }
 
-}  // extern "C"
+}  // namespace boatcu

@@ -285,18 +285,27 @@ __global__ void colsum_kernel(const ColsumTable t, int64_t rows, int64_t cols) {
 // ---- delta[r] = sum_d dO[r,d] * O[r,d]: one warp per row, shuffle reduction --------------------
 // With `lse2_out` the kernel emits the two per-row statistics in the form the BF16 backward's inner
 // loops consume them (one FMA each): out[r] = -delta[r] * scale and lse2_out[r] = -lse[r] * log2(e).
+// These are laid out for whole tiles: S rows of a unit take padded_S entries, the surplus ones hold
+// -inf and 0, with which the backward's missing query rows contribute exactly nothing.
 struct RowStats {
     const float* lse;
     float* lse2_out;
     float scale;
+    int S, padded_S;       // equal when there is nothing to pad
 };
-__device__ __forceinline__ void emit_row(float* __restrict__ out, const RowStats& st, int64_t row, float s) {
+__device__ __forceinline__ void emit_row(float* __restrict__ out, const RowStats& st, int64_t row, int64_t src, float s) {
     if (st.lse2_out) {
-        out[row] = s * -st.scale;
-        st.lse2_out[row] = st.lse[row] * -1.4426950408889634f;
+        out[row] = src < 0 ? 0.f : s * -st.scale;
+        st.lse2_out[row] = src < 0 ? -INFINITY : st.lse[src] * -1.4426950408889634f;
     } else {
         out[row] = s;
     }
+}
+// Input row behind output row `row`, -1 for a padding row.
+__device__ __forceinline__ int64_t source_row(const RowStats& st, int64_t row) {
+    if (st.S == st.padded_S) return row;
+    const int unit = (int)row / st.padded_S, r = (int)row - unit * st.padded_S;
+    return r < st.S ? (int64_t)unit * st.S + r : -1;
 }
 
 template <typename T>
@@ -306,13 +315,14 @@ __global__ void rowdot_kernel(const T* __restrict__ A, const T* __restrict__ B, 
     int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (; row < rows; row += step) {
-        const T* a = A + row * cols;
-        const T* b = B + row * cols;
+        const int64_t src = source_row(st, row);
+        const T* a = A + src * cols;
+        const T* b = B + src * cols;
         float s = 0.f;
-        for (int d = lane; d < cols; d += 32) s += to_f32(a[d]) * to_f32(b[d]);
+        for (int d = lane; d < cols && src >= 0; d += 32) s += to_f32(a[d]) * to_f32(b[d]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) emit_row(out, st, row, s);
+        if (lane == 0) emit_row(out, st, row, src, s);
     }
 }
 
@@ -329,9 +339,10 @@ __global__ void rowdot_vec_kernel(const T* __restrict__ A, const T* __restrict__
     for (int64_t base = warp * rows_per_warp; base < rows; base += nwarps * rows_per_warp) {
         int64_t row = base + sub;
         float s = 0.f;
-        if (row < rows) {
-            const uint4 va = *reinterpret_cast<const uint4*>(A + row * cols + l * VEC);
-            const uint4 vb = *reinterpret_cast<const uint4*>(B + row * cols + l * VEC);
+        const int64_t src = row < rows ? source_row(st, row) : -1;
+        if (src >= 0) {
+            const uint4 va = *reinterpret_cast<const uint4*>(A + src * cols + l * VEC);
+            const uint4 vb = *reinterpret_cast<const uint4*>(B + src * cols + l * VEC);
             if (sizeof(T) == 4) {
                 const float* fa = reinterpret_cast<const float*>(&va);
                 const float* fb = reinterpret_cast<const float*>(&vb);
@@ -348,7 +359,7 @@ __global__ void rowdot_vec_kernel(const T* __restrict__ A, const T* __restrict__
             }
         }
         for (int o = lanes_per_row >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (l == 0 && row < rows) emit_row(out, st, row, s);
+        if (l == 0 && row < rows) emit_row(out, st, row, src, s);
     }
 }
 
@@ -379,12 +390,12 @@ static int rowdot_launch(const void* A, const void* B, int type, int64_t rows, i
 }
 
 int rowdot(const void* A, const void* B, int type, int64_t rows, int64_t cols, float* out) {
-    return rowdot_launch(A, B, type, rows, cols, out, RowStats{nullptr, nullptr, 0.f});
+    return rowdot_launch(A, B, type, rows, cols, out, RowStats{nullptr, nullptr, 0.f, 0, 0});
 }
 
-int rowdot_stats(const void* dO, const void* O, int type, int64_t rows, int64_t cols, const float* lse, float scale,
-                 float* delta2_out, float* lse2_out) {
-    return rowdot_launch(dO, O, type, rows, cols, delta2_out, RowStats{lse, lse2_out, scale});
+int rowdot_stats(const void* dO, const void* O, int type, int64_t units, int64_t S, int64_t padded_S, int64_t cols,
+                 const float* lse, float scale, float* delta2_out, float* lse2_out) {
+    return rowdot_launch(dO, O, type, units * padded_S, cols, delta2_out, RowStats{lse, lse2_out, scale, (int)S, (int)padded_S});
 }
 
 // ---- out[b, j, i] = in[b, i, j], 32x32 shared-memory tiles --------------------------------------

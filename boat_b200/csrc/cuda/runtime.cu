@@ -115,8 +115,8 @@ typedef CUresult (*encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static encode_tiled_fn g_encode = nullptr;
 
-int make_tensor_map_2d(CUtensorMap* map, const void* base, int esize, uint64_t rows, uint64_t cols, uint64_t ld,
-                       uint32_t box_rows, uint32_t box_cols, bool atom32) {
+static int encode_map(CUtensorMap* map, const void* base, int esize, int rank, const cuuint64_t* dims,
+                      const cuuint64_t* strides, const cuuint32_t* box, bool atom32) {
     if (!g_encode) {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
@@ -124,21 +124,34 @@ int make_tensor_map_2d(CUtensorMap* map, const void* base, int esize, uint64_t r
         if (!fn || q != cudaDriverEntryPointSuccess) return set_error(31, "cuTensorMapEncodeTiled is not available");
         g_encode = (encode_tiled_fn)fn;
     }
-    if (((uintptr_t)base & 15) != 0 || ((ld * (uint64_t)esize) & 15) != 0)
+    if (((uintptr_t)base & 15) != 0 || (strides[0] & 15) != 0)
         return set_error(31, "tensor map: base or row pitch not 16-byte aligned");
-    if (box_cols * (uint32_t)esize != 128 || box_rows > 256 || box_rows == 0)
+    if (box[0] * (uint32_t)esize != 128 || box[1] > 256 || box[1] == 0)
         return set_error(31, "tensor map: box must be 128 bytes wide and at most 256 rows");
-    cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {ld * (uint64_t)esize};
-    cuuint32_t box[2] = {box_cols, box_rows};
-    cuuint32_t estr[2] = {1, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
     CUtensorMapDataType dt = esize == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-    CUresult r = g_encode(map, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    CUresult r = g_encode(map, dt, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error(31, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return 0;
+}
+
+int make_tensor_map_2d(CUtensorMap* map, const void* base, int esize, uint64_t rows, uint64_t cols, uint64_t ld,
+                       uint32_t box_rows, uint32_t box_cols, bool atom32) {
+    cuuint64_t dims[2] = {cols, rows};
+    cuuint64_t strides[1] = {ld * (uint64_t)esize};
+    cuuint32_t box[2] = {box_cols, box_rows};
+    return encode_map(map, base, esize, 2, dims, strides, box, atom32);
+}
+
+int make_tensor_map_units(CUtensorMap* map, const void* base, int esize, uint64_t units, uint64_t S, uint64_t hs,
+                          uint32_t box_rows, bool atom32) {
+    cuuint64_t dims[3] = {hs, S, units};
+    cuuint64_t strides[2] = {hs * (uint64_t)esize, S * hs * (uint64_t)esize};
+    cuuint32_t box[3] = {128u / (uint32_t)esize, box_rows, 1};
+    return encode_map(map, base, esize, 3, dims, strides, box, atom32);
 }
 
 // ---- per-kernel timing ---------------------------------------------------------------------

@@ -24,6 +24,12 @@ unsigned int take_kernel_status();
 // tensor core reads along M or N) instead of the usual 16-byte unit.
 int make_tensor_map_2d(CUtensorMap* map, const void* base, int esize, uint64_t rows, uint64_t cols, uint64_t ld,
                        uint32_t box_rows, uint32_t box_cols, bool atom32 = false);
+// The attention kernels' view of a [units*S, hs] matrix: [units, S, hs] with a box of one unit, box_rows
+// rows and 128 bytes.  A box that crosses the end of its unit reads zeros there, and a reduction or
+// store of such a box leaves the next unit alone - a sequence length need not be a multiple of the
+// tile.
+int make_tensor_map_units(CUtensorMap* map, const void* base, int esize, uint64_t units, uint64_t S, uint64_t hs,
+                          uint32_t box_rows, bool atom32 = false);
 
 namespace tc {
 
@@ -106,6 +112,13 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* m
         ::"r"(smem_u32(smem_dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
         : "memory");
 }
+// The same from a map of make_tensor_map_units: x = element of the row, y = row of the unit, z = unit.
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
 // Untiled bulk copy global -> shared (no multicast): `bytes` (a multiple of 16) from a 16-byte
 // aligned global address to a 16-byte aligned shared address, completion counted on `bar`.
 __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
@@ -114,10 +127,10 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gmem_sr
                  : "memory");
 }
 // Tile reduction shared -> global: adds the box at `smem_src` (laid out as a TMA load of the
-// same map would leave it) into the tensor at (x, y).  Completion is tracked by bulk groups.
-__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const void* smem_src, int x, int y) {
-    asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
-                 ::"l"((uint64_t)map), "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+// same map would leave it) into the tensor at (x, y, z).  Completion is tracked by bulk groups.
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, const void* smem_src, int x, int y, int z) {
+    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                 ::"l"((uint64_t)map), "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
 __device__ __forceinline__ void tma_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }

@@ -24,7 +24,7 @@ extern "C" {
 BOAT_API int boat_attention_to_device(boat_attention_t* attention, boat_device_t device);
 
 /* Choose the arithmetic: BOAT_MMA_FP32 (exact CUDA-core path, any shape), BOAT_MMA_TF32
- * or BOAT_MMA_BF16 (tcgen05 tensor-core paths; need seq_len % 128 == 0 and head size 64 or
+ * or BOAT_MMA_BF16 (tcgen05 tensor-core paths; any sequence length, head size 64 or - BF16 only -
  * 128, other shapes run on the CUDA cores with the same storage), or -1 for automatic:
  * BF16 tensors -> BF16, FP32 tensors -> exact FP32 whatever the shape, so that a reference
  * program's numbers never depend on the sequence length; TF32 is always an explicit choice.

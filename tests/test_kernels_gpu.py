@@ -190,6 +190,18 @@ def test_attention_core_matches_float64(gpu_lib, mma, hs, S, causal):
     assert np.abs(got["lse"] - ref["lse"]).max() <= (1e-4 if mma == capi.MMA_FP32 else 2e-2)
 
 
+@pytest.mark.parametrize("mma,hs", [(capi.MMA_BF16, 64), (capi.MMA_BF16, 128), (capi.MMA_TF32, 64)],
+                         ids=["bf16_hs64", "bf16_hs128", "tf32_hs64"])
+@pytest.mark.parametrize("S", [2, 64, 127, 129, 200, 257, 500])
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+def test_attention_core_on_partly_filled_tiles(gpu_lib, mma, hs, S, causal):
+    got, ref = run_core(gpu_lib, mma, 3, S, hs, causal)
+    for key in ("o", "dq", "dk", "dv"):
+        assert np.isfinite(got[key]).all(), key
+        assert rel(got[key], ref[key]) <= TOL[mma], (key, rel(got[key], ref[key]))
+    assert np.abs(got["lse"] - ref["lse"]).max() <= 2e-2
+
+
 def test_attention_core_large_scores_do_not_overflow(gpu_lib):
     """Rows whose running max keeps growing exercise the rescale of the accumulator."""
     lib = gpu_lib
