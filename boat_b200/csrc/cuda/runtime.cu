@@ -7,6 +7,7 @@
 #include <stdlib.h>
 #include <string.h>
 #include <atomic>
+#include <list>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -22,7 +23,10 @@ static int g_device = -1;                       // the one device this process's
 static int g_sm_count = 0;
 static cudaStream_t g_stream = 0;
 static std::atomic<uint64_t> g_launches{0};
-static std::unordered_map<void*, size_t>* g_live = nullptr;
+struct LiveBlock {
+    size_t bytes, block;                        // asked for, handed out
+};
+static std::unordered_map<void*, LiveBlock>* g_live = nullptr;
 static size_t g_live_bytes = 0;
 static unsigned int* g_status_host = nullptr;   // kernel status word, host view
 static unsigned int* g_status_dev = nullptr;    // the same word as kernels see it
@@ -72,13 +76,12 @@ static int init_locked(int device) {
         return set_error(3, "device %d is sm_%d%d; this library contains sm_100a code only",
                          dev, prop.major, prop.minor);
     }
-    // Keep freed blocks in the pool instead of returning them to the driver: a training
-    // step allocates and frees the same sizes every iteration.
+    // What leaves the block cache below stays in the driver's pool rather than being unmapped.
     cudaMemPool_t pool;
     BOATCU_CHECK(cudaDeviceGetDefaultMemPool(&pool, dev));
     uint64_t keep = UINT64_MAX;
     BOATCU_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    if (!g_live) g_live = new std::unordered_map<void*, size_t>();
+    if (!g_live) g_live = new std::unordered_map<void*, LiveBlock>();
     BOATCU_CHECK(cudaHostAlloc((void**)&g_status_host, sizeof(unsigned int), cudaHostAllocMapped));
     *g_status_host = 0;
     BOATCU_CHECK(cudaHostGetDevicePointer((void**)&g_status_dev, g_status_host, 0));
@@ -197,6 +200,47 @@ int ensure_init() {
 
 using namespace boatcu;
 
+// ---- device memory ---------------------------------------------------------------------------
+// A step allocates and frees the same two dozen buffers every time.  Freed blocks are kept by size
+// and handed out again to the next request they fit (within an eighth), instead of a round trip
+// through the driver's pool for each: that round trip costs 1-4 us of host time, which small
+// steps are bound by, and now and then milliseconds when the pool has to remap memory (a step
+// of B16 S2048 d1024 took 1.9 ms of kernels and 1.9-2.7 ms in all).  Everything the library launches
+// is ordered on one stream, so a block freed there may be written by whatever is launched next.
+// Bounded by BOAT_DEVICE_CACHE_MB (default 8192): the longest unused blocks go back to the driver
+// when more than that lies idle; all of them when the stream changes or an allocation fails.
+struct CachedBlock;
+typedef std::multimap<size_t, CachedBlock> BlockCache;
+struct CachedBlock {
+    void* ptr;
+    std::list<BlockCache::iterator>::iterator age;
+};
+static BlockCache* g_cache = new BlockCache();                                        // idle blocks by size
+static std::list<BlockCache::iterator>* g_cache_age = new std::list<BlockCache::iterator>();    // oldest first
+static size_t g_cache_bytes = 0;
+
+static size_t cache_cap() {
+    static const size_t cap = [] {
+        const char* e = getenv("BOAT_DEVICE_CACHE_MB");
+        const long long mb = e && *e ? atoll(e) : 8192;
+        return (size_t)(mb < 0 ? 0 : mb) << 20;
+    }();
+    return cap;
+}
+
+// Gives the oldest idle blocks back until at most `limit` bytes are left (g_mu held).
+static int trim_cache(size_t limit) {
+    while (g_cache_bytes > limit) {
+        const auto it = g_cache_age->front();
+        void* p = it->second.ptr;
+        g_cache_bytes -= it->first;
+        g_cache_age->pop_front();
+        g_cache->erase(it);
+        BOATCU_CHECK(cudaFreeAsync(p, g_stream));
+    }
+    return 0;
+}
+
 extern "C" {
 
 int boat_cuda_init(int device) {
@@ -221,6 +265,11 @@ const char* boat_cuda_last_error(void) { return g_err; }
 void* boat_cuda_stream(void) { return (void*)g_stream; }
 
 int boat_cuda_set_stream(void* s) {
+    if ((cudaStream_t)s != g_stream && g_ready) {
+        // cached blocks are ordered behind the old stream only: hand them back to the driver on it
+        std::lock_guard<std::mutex> lk(g_mu);
+        trim_cache(0);
+    }
     g_stream = (cudaStream_t)s;
     return 0;
 }
@@ -297,9 +346,27 @@ int boat_cuda_malloc(void** ptr, size_t bytes) {
     *ptr = nullptr;
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
-    BOATCU_CHECK(cudaMallocAsync(ptr, bytes, g_stream));
     std::lock_guard<std::mutex> lk(g_mu);
-    (*g_live)[*ptr] = bytes;
+    const size_t want = (bytes + 511) & ~(size_t)511;
+    size_t block = want;
+    auto it = g_cache->lower_bound(want);
+    if (it != g_cache->end() && it->first <= want + want / 8) {
+        block = it->first;
+        *ptr = it->second.ptr;
+        g_cache_age->erase(it->second.age);
+        g_cache->erase(it);
+        g_cache_bytes -= block;
+    } else {
+        cudaError_t err = cudaMallocAsync(ptr, block, g_stream);
+        if (err == cudaErrorMemoryAllocation && g_cache_bytes > 0) {
+            // what the cache holds may be what is missing; the driver's pool takes it back in stream order
+            cudaGetLastError();
+            trim_cache(0);
+            err = cudaMallocAsync(ptr, block, g_stream);
+        }
+        BOATCU_CHECK(err);
+    }
+    (*g_live)[*ptr] = LiveBlock{bytes, block};
     g_live_bytes += bytes;
     return 0;
 }
@@ -311,11 +378,14 @@ int boat_cuda_free(void* ptr) {
         std::lock_guard<std::mutex> lk(g_mu);
         auto it = g_live->find(ptr);
         if (it == g_live->end()) return set_error(5, "boat_cuda_free: %p was not allocated here", ptr);
-        g_live_bytes -= it->second;
+        g_live_bytes -= it->second.bytes;
+        const size_t block = it->second.block;
         g_live->erase(it);
+        const auto entry = g_cache->insert({block, CachedBlock{ptr, {}}});
+        entry->second.age = g_cache_age->insert(g_cache_age->end(), entry);
+        g_cache_bytes += block;
+        return trim_cache(cache_cap());
     }
-    BOATCU_CHECK(cudaFreeAsync(ptr, g_stream));
-    return 0;
 }
 
 size_t boat_cuda_bytes_in_use(void) { return g_live_bytes; }
