@@ -1,271 +1,403 @@
-// attn_simt.cu - CUDA-core attention core, forward and backward, FP32 arithmetic, any
-// sequence length and head size up to 128.  One thread owns one query row (forward, dQ) or
-// one key row (dK, dV); the other side streams through shared memory in tiles that every
-// thread reads as a broadcast, so no cross-thread reduction is needed.  The S x S matrices
-// are never written to memory: probabilities are rebuilt from the saved log-sum-exp.
+// attn_simt.cu - CUDA-core attention core, forward and backward, FP32 arithmetic, any sequence
+// length and head size up to 128.
 //
 // Restates scaled_dot_product_attention_impl (reference src/layers/attention.c:997-1073)
 // and attention_backward (attention.c:1421-1526) for the exact-FP32 mode and for shapes
-// outside the tensor-core kernels.
+// outside the tensor-core kernels.  The S x S matrices are never written to memory:
+// probabilities are rebuilt from the saved log-sum-exp.
+//
+// A CTA of 256 threads (16 x 16) owns 64 rows and walks the other side in tiles of 64 rows.  A score
+// tile is 4 x 4 per thread, contracted along the head dimension with 16-byte shared loads of four
+// elements; rows are HS+4 floats apart, so 8 lanes on 8 rows touch all banks once.  The tile's rows
+// stay with the 16 lanes that made them - soft-max statistics are shuffles, and the products with the
+// probabilities (P.V, dS.K, P^T.dO, dS^T.Q) read rows which the same half warp wrote: a walk has one CTA
+// barrier per tile.  The next tile is fetched (cp.async) while the current one is worked on.
+//
+// Backward: one launch holds CTAs that own query rows (dQ) and CTAs that own key rows (dK, dV).  Both
+// rebuild the scores they need - seven products per tile pair instead of five - and nothing is summed
+// between CTAs, so results do not vary from run to run.  The two kinds are the same walk:
+//   own = Q, dO, walk = K, V:   S = own0.walk0^T   dP = own1.walk1^T   dQ += dS.walk0
+//   own = K, V,  walk = Q, dO:  the same, transposed             dK += dS^T.walk0   dV += P^T.walk1
 #include "common.cuh"
 #include <float.h>
 
 namespace boatcu {
 
-static const int ROWS = 64;   // rows owned by a CTA = threads per CTA
+namespace {
 
-template <int TILE, typename T>
-__device__ __forceinline__ void load_tile(float* dst, const T* src, int64_t row0, int64_t S, int hs, int tid) {
-    // dst[r*hs + d] = src[(row0+r)*hs + d] for r < TILE, zero past the end of the sequence
-    for (int idx = tid; idx < TILE * hs; idx += ROWS) {
-        int r = idx / hs;
-        dst[idx] = (row0 + r < S) ? to_f32(src[row0 * hs + idx]) : 0.f;
+constexpr int kRows = 64;             // rows owned and rows per walked tile
+constexpr int kThreads = 256;
+constexpr int kLdP = kRows + 4;       // shared row pitch of a probability tile
+
+template <int HS>
+struct Tiles {
+    static constexpr int LD = HS + 4;
+    static constexpr int FLOATS = kRows * LD;
+    static constexpr int CPT = HS / 16;                  // output columns per thread
+    static constexpr int BUFS = HS <= 64 ? 2 : 1;        // walked tiles in flight
+    static constexpr int FWD_SMEM = (FLOATS * (1 + 2 * BUFS) + kRows * kLdP) * 4;
+    static constexpr int BWD_SMEM = (FLOATS * (2 + 2 * BUFS) + 2 * kRows * kLdP + 2 * 2 * kRows) * 4;
+    static_assert(BWD_SMEM <= 227 * 1024, "shared memory budget");
+};
+
+// Rows r0..r0+63 of a [S, hs] matrix to shared rows LD apart; zeros beyond S and from hs to HS.
+template <int HS>
+__device__ __forceinline__ void load_rows(float* dst, const float* src, int r0, int S, int hs, bool vec) {
+    if (vec) {
+#pragma unroll
+        for (int e = threadIdx.x; e < kRows * HS / 4; e += kThreads) {
+            const int r = e / (HS / 4), c = (e % (HS / 4)) * 4;
+            const bool in = r0 + r < S && c < hs;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * (HS + 4) + c)),
+                         "l"(in ? src + (int64_t)(r0 + r) * hs + c : src), "r"(in ? 16 : 0) : "memory");
+        }
+    } else {
+        for (int e = threadIdx.x; e < kRows * HS; e += kThreads) {
+            const int r = e / HS, c = e % HS;
+            const bool in = r0 + r < S && c < hs;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * (HS + 4) + c)),
+                         "l"(in ? src + (int64_t)(r0 + r) * hs + c : src), "r"(in ? 4 : 0) : "memory");
+        }
     }
+}
+template <int HS>
+__device__ __forceinline__ void load_rows(float* dst, const __nv_bfloat16* src, int r0, int S, int hs, bool vec) {
+    if (vec) {
+#pragma unroll 4
+        for (int e = threadIdx.x; e < kRows * HS / 4; e += kThreads) {
+            const int r = e / (HS / 4), c = (e % (HS / 4)) * 4;
+            uint2 v = make_uint2(0u, 0u);
+            if (r0 + r < S && c < hs) v = *reinterpret_cast<const uint2*>(src + (int64_t)(r0 + r) * hs + c);
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v.x));
+            const float2 hi = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&v.y));
+            *reinterpret_cast<float4*>(dst + r * (HS + 4) + c) = make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+    } else {
+        for (int e = threadIdx.x; e < kRows * HS; e += kThreads) {
+            const int r = e / HS, c = e % HS;
+            dst[r * (HS + 4) + c] = r0 + r < S && c < hs ? to_f32(src[(int64_t)(r0 + r) * hs + c]) : 0.f;
+        }
+    }
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// s[i][j] = sum_d A[ty*4+i][d] * B[tx+16j][d], ascending d
+template <int HS>
+__device__ __forceinline__ void scores(const float* A, const float* B, int ty, int tx, float (&s)[4][4]) {
+    constexpr int LD = HS + 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+#pragma unroll 4
+    for (int d = 0; d < HS; d += 4) {
+        float4 a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + (ty * 4 + i) * LD + d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(B + (tx + 16 * j) * LD + d);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
+                s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
+                s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
+                s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
+            }
+    }
+}
+
+// First output column of group u (min(CPT,4) columns each) of a thread
+template <int HS> __device__ __forceinline__ int out_col(int tx, int u) {
+    constexpr int CPT = HS / 16, V = CPT < 4 ? CPT : 4;
+    return u * 16 * V + tx * V;
+}
+
+// acc[i][:] += sum_k P[ty*4+i][k] * X[k][cols of this thread], ascending k
+template <int HS>
+__device__ __forceinline__ void accumulate(const float* P, const float* X, int ty, int tx, float (&acc)[4][HS / 16]) {
+    constexpr int LD = HS + 4, CPT = HS / 16, V = CPT < 4 ? CPT : 4;
+#pragma unroll 4
+    for (int k = 0; k < kRows; k += 4) {
+        float p[4][4], x[4][CPT];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 t = *reinterpret_cast<const float4*>(P + (ty * 4 + i) * kLdP + k);
+            p[i][0] = t.x; p[i][1] = t.y; p[i][2] = t.z; p[i][3] = t.w;
+        }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int u = 0; u < CPT / V; ++u) {
+                const float* q = X + (k + kk) * LD + out_col<HS>(tx, u);
+                if constexpr (V == 4) {
+                    const float4 t = *reinterpret_cast<const float4*>(q);
+                    x[kk][4 * u] = t.x; x[kk][4 * u + 1] = t.y; x[kk][4 * u + 2] = t.z; x[kk][4 * u + 3] = t.w;
+                } else {
+#pragma unroll
+                    for (int v = 0; v < V; ++v) x[kk][v] = q[v];
+                }
+            }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int c = 0; c < CPT; ++c) acc[i][c] = fmaf(p[i][kk], x[kk][c], acc[i][c]);
+    }
+}
+
+template <int HS, typename T>
+__device__ __forceinline__ void store_rows(T* dst, int r0, int S, int hs, int ty, int tx, const float (&acc)[4][HS / 16]) {
+    constexpr int CPT = HS / 16, V = CPT < 4 ? CPT : 4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = r0 + ty * 4 + i;
+        if (r >= S) continue;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+            const int d = out_col<HS>(tx, c / V) + c % V;
+            if (d < hs) dst[(int64_t)r * hs + d] = from_f32<T>(acc[i][c]);
+        }
+    }
+}
+
+// reductions over the 16 lanes that share a row
+__device__ __forceinline__ float row_max(float v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float row_sum(float v) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // ---- forward -----------------------------------------------------------------------------------
-template <int HS_MAX, int TILE, typename T>
-__global__ void __launch_bounds__(ROWS)
-attn_fwd_simt_kernel(int64_t S, int hs, int causal, float scale, const T* __restrict__ Q,
-                     const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O,
-                     float* __restrict__ lse) {
-    extern __shared__ float smem[];
-    float* q_s = smem;                       // [hs][ROWS]   column = thread
-    float* k_s = q_s + (size_t)hs * ROWS;    // [TILE][hs]
-    float* v_s = k_s + (size_t)TILE * hs;    // [TILE][hs]
-    const int tid = threadIdx.x;
-    const int64_t unit = blockIdx.y;
-    const int64_t i0 = (int64_t)blockIdx.x * ROWS;
-    const int64_t i = i0 + tid;
-    const T* Qu = Q + unit * S * hs;
-    const T* Ku = K + unit * S * hs;
-    const T* Vu = V + unit * S * hs;
-    const bool live = i < S;
-
-    for (int idx = tid; idx < ROWS * hs; idx += ROWS) {
-        int r = idx / hs, d = idx % hs;
-        q_s[d * ROWS + r] = (i0 + r < S) ? to_f32(Qu[i0 * hs + idx]) : 0.f;
+template <int HS, typename T>
+__global__ void __launch_bounds__(kThreads)
+attn_fwd_simt_kernel(int units, int S, int hs, int causal, float scale, int vec, const T* __restrict__ Q,
+                     const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O, float* __restrict__ lse) {
+    using C = Tiles<HS>;
+    extern __shared__ __align__(16) float smem[];
+    float* q_s = smem;
+    float* kv_s = q_s + C::FLOATS;                        // [BUFS][K, V]
+    float* p_s = kv_s + 2 * C::BUFS * C::FLOATS;
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const int n_tiles = (S + kRows - 1) / kRows;
+    const int unit = blockIdx.x % units, qt = n_tiles - 1 - blockIdx.x / units;      // long rows first when causal
+    const int64_t base = (int64_t)unit * S * hs;
+    const int q0 = qt * kRows, n_kv = causal ? qt + 1 : n_tiles;
+    auto fetch = [&](int j) {
+        float* b = kv_s + (j % C::BUFS) * 2 * C::FLOATS;
+        load_rows<HS>(b, K + base, j * kRows, S, hs, vec);
+        load_rows<HS>(b + C::FLOATS, V + base, j * kRows, S, hs, vec);
+        commit();
+    };
+    load_rows<HS>(q_s, Q + base, q0, S, hs, vec);
+    fetch(0);
+    float o[4][C::CPT], m[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -FLT_MAX;
+        l[i] = 0.f;
+#pragma unroll
+        for (int c = 0; c < C::CPT; ++c) o[i][c] = 0.f;
     }
-    float o[HS_MAX];
-#pragma unroll
-    for (int d = 0; d < HS_MAX; ++d) o[d] = 0.f;
-    float m = -FLT_MAX, l = 0.f;
-
-    const int64_t j_end = causal ? min(S, i0 + ROWS) : S;
-    for (int64_t j0 = 0; j0 < j_end; j0 += TILE) {
-        __syncthreads();
-        load_tile<TILE>(k_s, Ku, j0, S, hs, tid);
-        load_tile<TILE>(v_s, Vu, j0, S, hs, tid);
-        __syncthreads();
-        float s[TILE];
-        float tmax = -FLT_MAX;
-#pragma unroll
-        for (int t = 0; t < TILE; ++t) {
-            float acc = 0.f;
-            for (int d = 0; d < hs; ++d) acc = fmaf(q_s[d * ROWS + tid], k_s[t * hs + d], acc);
-            acc *= scale;
-            int64_t j = j0 + t;
-            bool ok = j < S && (!causal || j <= i);
-            s[t] = ok ? acc : -FLT_MAX;
-            tmax = fmaxf(tmax, s[t]);
+    for (int j = 0; j < n_kv; ++j) {
+        if (C::BUFS == 1 && j > 0) {
+            __syncthreads();
+            fetch(j);
         }
-        if (tmax == -FLT_MAX) continue;          // nothing visible for this row in this tile
-        float m_new = fmaxf(m, tmax);
-        float corr = (m == -FLT_MAX) ? 0.f : expf(m - m_new);
-        l *= corr;
+        wait_all();
+        __syncthreads();
+        if (C::BUFS == 2 && j + 1 < n_kv) fetch(j + 1);
+        const float* k_s = kv_s + (j % C::BUFS) * 2 * C::FLOATS;
+        float s[4][4];
+        scores<HS>(q_s, k_s, ty, tx, s);
 #pragma unroll
-        for (int d = 0; d < HS_MAX; ++d) o[d] *= corr;
+        for (int i = 0; i < 4; ++i) {
+            const int limit = min(S - 1, causal ? q0 + ty * 4 + i : S - 1) - j * kRows;      // last visible key of the tile
+            float t = -FLT_MAX;
 #pragma unroll
-        for (int t = 0; t < TILE; ++t) {
-            float p = (s[t] == -FLT_MAX) ? 0.f : expf(s[t] - m_new);
-            l += p;
+            for (int c = 0; c < 4; ++c) {
+                s[i][c] = tx + 16 * c <= limit ? s[i][c] * scale : -FLT_MAX;
+                t = fmaxf(t, s[i][c]);
+            }
+            const float m_new = fmaxf(m[i], row_max(t));
+            const float corr = expf(m[i] - m_new);          // 0 for the first tile: every row sees its key 0
+            float sum = 0.f;
 #pragma unroll
-            for (int d = 0; d < HS_MAX; ++d)
-                if (d < hs) o[d] = fmaf(p, v_s[t * hs + d], o[d]);
+            for (int c = 0; c < 4; ++c) {
+                const float e = s[i][c] == -FLT_MAX ? 0.f : expf(s[i][c] - m_new);
+                sum += e;
+                p_s[(ty * 4 + i) * kLdP + tx + 16 * c] = e;
+            }
+            l[i] = l[i] * corr + row_sum(sum);
+            m[i] = m_new;
+#pragma unroll
+            for (int c = 0; c < C::CPT; ++c) o[i][c] *= corr;
         }
-        m = m_new;
+        __syncwarp();
+        accumulate<HS>(p_s, k_s + C::FLOATS, ty, tx, o);
+        __syncwarp();
     }
-    if (live) {
-        float inv = 1.f / l;
-        T* Ou = O + unit * S * hs + i * hs;
 #pragma unroll
-        for (int d = 0; d < HS_MAX; ++d)
-            if (d < hs) Ou[d] = from_f32<T>(o[d] * inv);
-        lse[unit * S + i] = m + logf(l);
+    for (int i = 0; i < 4; ++i) {
+        const float inv = 1.f / l[i];
+#pragma unroll
+        for (int c = 0; c < C::CPT; ++c) o[i][c] *= inv;
+        const int r = q0 + ty * 4 + i;
+        if (tx == 0 && r < S) lse[(int64_t)unit * S + r] = m[i] + logf(l[i]);
+    }
+    store_rows<HS, T>(O + base, q0, S, hs, ty, tx, o);
+}
+
+// ---- backward ------------------------------------------------------------------------------------
+template <typename T>
+struct BwdArgs {
+    const T *Q, *K, *V, *dO;
+    const float *lse, *delta;
+    T *dQ, *dK, *dV;
+    int units, S, hs, causal, vec;
+    float scale;
+};
+
+// KEYS: the CTA owns key rows (dK, dV), otherwise query rows (dQ).
+template <int HS, typename T, bool KEYS>
+__device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile, float* smem) {
+    using C = Tiles<HS>;
+    float* own0 = smem;
+    float* own1 = own0 + C::FLOATS;
+    float* walk = own1 + C::FLOATS;                       // [BUFS][walk0, walk1]
+    float* ds_s = walk + 2 * C::BUFS * C::FLOATS;
+    float* p_s = ds_s + kRows * kLdP;
+    float* stat = p_s + kRows * kLdP;                     // [2][lse[64], delta[64]] of the query rows
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    const int S = a.S, hs = a.hs, n_tiles = (S + kRows - 1) / kRows;
+    const int64_t base = (int64_t)unit * S * hs, sbase = (int64_t)unit * S;
+    const int r0 = tile * kRows;
+    const int first = KEYS && a.causal ? tile : 0, end = !KEYS && a.causal ? tile + 1 : n_tiles;
+    const T* w0 = (KEYS ? a.Q : a.K) + base;
+    const T* w1 = (KEYS ? a.dO : a.V) + base;
+    auto load_stats = [&](int q0, int buf) {
+        if (threadIdx.x < 2 * kRows) {
+            const int r = threadIdx.x & (kRows - 1);
+            const float* src = threadIdx.x < kRows ? a.lse : a.delta;
+            stat[buf * 2 * kRows + threadIdx.x] = q0 + r < S ? src[sbase + q0 + r] : 0.f;
+        }
+    };
+    auto fetch = [&](int j) {
+        float* b = walk + (j % C::BUFS) * 2 * C::FLOATS;
+        load_rows<HS>(b, w0, j * kRows, S, hs, a.vec);
+        load_rows<HS>(b + C::FLOATS, w1, j * kRows, S, hs, a.vec);
+        commit();
+        if (KEYS) load_stats(j * kRows, j & 1);
+    };
+    load_rows<HS>(own0, (KEYS ? a.K : a.Q) + base, r0, S, hs, a.vec);
+    load_rows<HS>(own1, (KEYS ? a.V : a.dO) + base, r0, S, hs, a.vec);
+    if (!KEYS) load_stats(r0, 0);
+    fetch(first);
+    float acc0[4][C::CPT], acc1[4][C::CPT];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < C::CPT; ++c) acc0[i][c] = acc1[i][c] = 0.f;
+    for (int j = first; j < end; ++j) {
+        if (C::BUFS == 1 && j > first) {
+            __syncthreads();
+            fetch(j);
+        }
+        wait_all();
+        __syncthreads();
+        if (C::BUFS == 2 && j + 1 < end) fetch(j + 1);
+        const float* x0 = walk + (j % C::BUFS) * 2 * C::FLOATS;
+        const float* x1 = x0 + C::FLOATS;
+        float s[4][4], dp[4][4];
+        scores<HS>(own0, x0, ty, tx, s);
+        scores<HS>(own1, x1, ty, tx, dp);
+        const float* st = stat + (KEYS ? j & 1 : 0) * 2 * kRows;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int mine = r0 + ty * 4 + i, other = j * kRows + tx + 16 * c;
+                const int q = KEYS ? other : mine, k = KEYS ? mine : other;
+                const int q_in = KEYS ? tx + 16 * c : ty * 4 + i;
+                const bool seen = q < S && k < S && (!a.causal || k <= q);
+                const float pr = seen ? expf(s[i][c] * a.scale - st[q_in]) : 0.f;
+                ds_s[(ty * 4 + i) * kLdP + tx + 16 * c] = pr * (dp[i][c] - st[kRows + q_in]) * a.scale;
+                if (KEYS) p_s[(ty * 4 + i) * kLdP + tx + 16 * c] = pr;
+            }
+        __syncwarp();
+        accumulate<HS>(ds_s, x0, ty, tx, acc0);
+        if (KEYS) accumulate<HS>(p_s, x1, ty, tx, acc1);
+        __syncwarp();
+    }
+    if (KEYS) {
+        store_rows<HS, T>(a.dK + base, r0, S, hs, ty, tx, acc0);
+        store_rows<HS, T>(a.dV + base, r0, S, hs, ty, tx, acc1);
+    } else {
+        store_rows<HS, T>(a.dQ + base, r0, S, hs, ty, tx, acc0);
     }
 }
 
-// ---- backward, dQ: thread = query row ------------------------------------------------------------
-template <int HS_MAX, int TILE, typename T>
-__global__ void __launch_bounds__(ROWS)
-attn_bwd_dq_simt_kernel(int64_t S, int hs, int causal, float scale, const T* __restrict__ Q,
-                        const T* __restrict__ K, const T* __restrict__ V, const T* __restrict__ dO,
-                        const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dQ) {
-    extern __shared__ float smem[];
-    float* q_s = smem;                        // [hs][ROWS]
-    float* do_s = q_s + (size_t)hs * ROWS;    // [hs][ROWS]
-    float* k_s = do_s + (size_t)hs * ROWS;    // [TILE][hs]
-    float* v_s = k_s + (size_t)TILE * hs;     // [TILE][hs]
-    const int tid = threadIdx.x;
-    const int64_t unit = blockIdx.y;
-    const int64_t i0 = (int64_t)blockIdx.x * ROWS;
-    const int64_t i = i0 + tid;
-    const int64_t base = unit * S * hs;
-    const bool live = i < S;
-    for (int idx = tid; idx < ROWS * hs; idx += ROWS) {
-        int r = idx / hs, d = idx % hs;
-        bool in = i0 + r < S;
-        q_s[d * ROWS + r] = in ? to_f32(Q[base + i0 * hs + idx]) : 0.f;
-        do_s[d * ROWS + r] = in ? to_f32(dO[base + i0 * hs + idx]) : 0.f;
-    }
-    const float lse_i = live ? lse[unit * S + i] : 0.f;
-    const float delta_i = live ? delta[unit * S + i] : 0.f;
-    float acc[HS_MAX];
-#pragma unroll
-    for (int d = 0; d < HS_MAX; ++d) acc[d] = 0.f;
-
-    const int64_t j_end = causal ? min(S, i0 + ROWS) : S;
-    for (int64_t j0 = 0; j0 < j_end; j0 += TILE) {
-        __syncthreads();
-        load_tile<TILE>(k_s, K + base, j0, S, hs, tid);
-        load_tile<TILE>(v_s, V + base, j0, S, hs, tid);
-        __syncthreads();
-#pragma unroll 1
-        for (int t = 0; t < TILE; ++t) {
-            int64_t j = j0 + t;
-            if (!(live && j < S && (!causal || j <= i))) continue;
-            float s = 0.f, dp = 0.f;
-            for (int d = 0; d < hs; ++d) {
-                s = fmaf(q_s[d * ROWS + tid], k_s[t * hs + d], s);
-                dp = fmaf(do_s[d * ROWS + tid], v_s[t * hs + d], dp);
-            }
-            float p = expf(s * scale - lse_i);
-            float ds = p * (dp - delta_i) * scale;
-#pragma unroll
-            for (int d = 0; d < HS_MAX; ++d)
-                if (d < hs) acc[d] = fmaf(ds, k_s[t * hs + d], acc[d]);
-        }
-    }
-    if (live) {
-        T* out = dQ + base + i * hs;
-#pragma unroll
-        for (int d = 0; d < HS_MAX; ++d)
-            if (d < hs) out[d] = from_f32<T>(acc[d]);
-    }
+template <int HS, typename T>
+__global__ void __launch_bounds__(kThreads)
+attn_bwd_simt_kernel(const BwdArgs<T> a) {
+    extern __shared__ __align__(16) float smem[];
+    // the longest walks first when causal: early key tiles, late query tiles
+    const int n_tiles = (a.S + kRows - 1) / kRows;
+    const int b = blockIdx.x >> 1, unit = b % a.units, t = b / a.units;
+    if (blockIdx.x & 1) bwd_walk<HS, T, false>(a, unit, n_tiles - 1 - t, smem);
+    else                bwd_walk<HS, T, true>(a, unit, t, smem);
 }
 
-// ---- backward, dK (WANT_K) or dV: thread = key row -------------------------------------------------
-template <int HS_MAX, int TILE, typename T, bool WANT_K>
-__global__ void __launch_bounds__(ROWS)
-attn_bwd_kv_simt_kernel(int64_t S, int hs, int causal, float scale, const T* __restrict__ Q,
-                        const T* __restrict__ K, const T* __restrict__ V, const T* __restrict__ dO,
-                        const float* __restrict__ lse, const float* __restrict__ delta, T* __restrict__ dOut) {
-    extern __shared__ float smem[];
-    float* k_s = smem;                        // [hs][ROWS]
-    float* v_s = k_s + (size_t)hs * ROWS;     // [hs][ROWS]
-    float* q_s = v_s + (size_t)hs * ROWS;     // [TILE][hs]
-    float* do_s = q_s + (size_t)TILE * hs;    // [TILE][hs]
-    float* lse_s = do_s + (size_t)TILE * hs;  // [TILE]
-    float* delta_s = lse_s + TILE;            // [TILE]
-    const int tid = threadIdx.x;
-    const int64_t unit = blockIdx.y;
-    const int64_t j0 = (int64_t)blockIdx.x * ROWS;
-    const int64_t j = j0 + tid;
-    const int64_t base = unit * S * hs;
-    const bool live = j < S;
-    for (int idx = tid; idx < ROWS * hs; idx += ROWS) {
-        int r = idx / hs, d = idx % hs;
-        bool in = j0 + r < S;
-        k_s[d * ROWS + r] = in ? to_f32(K[base + j0 * hs + idx]) : 0.f;
-        v_s[d * ROWS + r] = in ? to_f32(V[base + j0 * hs + idx]) : 0.f;
-    }
-    float acc[HS_MAX];
-#pragma unroll
-    for (int d = 0; d < HS_MAX; ++d) acc[d] = 0.f;
-
-    const int64_t i_begin = causal ? (j0 / TILE) * TILE : 0;
-    for (int64_t i0 = i_begin; i0 < S; i0 += TILE) {
-        __syncthreads();
-        load_tile<TILE>(q_s, Q + base, i0, S, hs, tid);
-        load_tile<TILE>(do_s, dO + base, i0, S, hs, tid);
-        if (tid < TILE) {
-            bool in = i0 + tid < S;
-            lse_s[tid] = in ? lse[unit * S + i0 + tid] : 0.f;
-            delta_s[tid] = in ? delta[unit * S + i0 + tid] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll 1
-        for (int t = 0; t < TILE; ++t) {
-            int64_t i = i0 + t;
-            if (!(live && i < S && (!causal || j <= i))) continue;
-            float s = 0.f, dp = 0.f;
-            for (int d = 0; d < hs; ++d) {
-                s = fmaf(q_s[t * hs + d], k_s[d * ROWS + tid], s);
-                if (WANT_K) dp = fmaf(do_s[t * hs + d], v_s[d * ROWS + tid], dp);
-            }
-            float p = expf(s * scale - lse_s[t]);
-            if (WANT_K) {
-                float ds = p * (dp - delta_s[t]) * scale;
-#pragma unroll
-                for (int d = 0; d < HS_MAX; ++d)
-                    if (d < hs) acc[d] = fmaf(ds, q_s[t * hs + d], acc[d]);
-            } else {
-#pragma unroll
-                for (int d = 0; d < HS_MAX; ++d)
-                    if (d < hs) acc[d] = fmaf(p, do_s[t * hs + d], acc[d]);
-            }
-        }
-    }
-    if (live) {
-        T* out = dOut + base + j * hs;
-#pragma unroll
-        for (int d = 0; d < HS_MAX; ++d)
-            if (d < hs) out[d] = from_f32<T>(acc[d]);
-    }
+bool rows_aligned(const void* const* ptrs, int n, int64_t hs, int es) {
+    bool ok = hs % 4 == 0;
+    for (int i = 0; i < n; ++i) ok = ok && ((uintptr_t)ptrs[i] & (4 * es - 1)) == 0;
+    return ok;
 }
 
-static const int TILE = 16;
-
-template <int HS_MAX, typename T>
-static int launch_fwd(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
-                      const void* V, void* O, float* lse) {
-    size_t smem = ((size_t)hs * ROWS + 2 * (size_t)TILE * hs) * sizeof(float);
-    auto kern = attn_fwd_simt_kernel<HS_MAX, TILE, T>;
-    BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)ceil_div(S, ROWS), (unsigned)units);
-    kern<<<grid, ROWS, smem, stream()>>>(S, hs, causal, scale, (const T*)Q, (const T*)K, (const T*)V, (T*)O, lse);
+template <int HS, typename T>
+int launch_fwd(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
+               const void* V, void* O, float* lse) {
+    auto kern = attn_fwd_simt_kernel<HS, T>;
+    static bool configured = false;     // per process = per device: the library binds to one device
+    if (!configured) {
+        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tiles<HS>::FWD_SMEM));
+        configured = true;
+    }
+    const void* in[3] = {Q, K, V};
+    const unsigned grid = (unsigned)(units * ceil_div(S, kRows));
+    kern<<<grid, kThreads, Tiles<HS>::FWD_SMEM, stream()>>>((int)units, (int)S, hs, causal, scale, rows_aligned(in, 3, hs, sizeof(T)),
+                                                             (const T*)Q, (const T*)K, (const T*)V, (T*)O, lse);
     BOATCU_LAUNCH_OK("attn_fwd_simt");
     return 0;
 }
 
-template <int HS_MAX, typename T>
-static int launch_bwd(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
-                      const void* V, const void* dO, const float* lse, const float* delta, void* dQ, void* dK,
-                      void* dV) {
-    dim3 grid((unsigned)ceil_div(S, ROWS), (unsigned)units);
-    {
-        size_t smem = (2 * (size_t)hs * ROWS + 2 * (size_t)TILE * hs) * sizeof(float);
-        auto kern = attn_bwd_dq_simt_kernel<HS_MAX, TILE, T>;
-        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROWS, smem, stream()>>>(S, hs, causal, scale, (const T*)Q, (const T*)K, (const T*)V,
-                                            (const T*)dO, lse, delta, (T*)dQ);
-        BOATCU_LAUNCH_OK("attn_bwd_dq_simt");
+template <int HS, typename T>
+int launch_bwd(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
+               const void* V, const void* dO, const float* lse, const float* delta, void* dQ, void* dK, void* dV) {
+    auto kern = attn_bwd_simt_kernel<HS, T>;
+    static bool configured = false;
+    if (!configured) {
+        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tiles<HS>::BWD_SMEM));
+        configured = true;
     }
-    size_t smem = (2 * (size_t)hs * ROWS + 2 * (size_t)TILE * hs + 2 * TILE) * sizeof(float);
-    {
-        auto kern = attn_bwd_kv_simt_kernel<HS_MAX, TILE, T, true>;
-        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROWS, smem, stream()>>>(S, hs, causal, scale, (const T*)Q, (const T*)K, (const T*)V,
-                                            (const T*)dO, lse, delta, (T*)dK);
-        BOATCU_LAUNCH_OK("attn_bwd_dk_simt");
-    }
-    {
-        auto kern = attn_bwd_kv_simt_kernel<HS_MAX, TILE, T, false>;
-        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROWS, smem, stream()>>>(S, hs, causal, scale, (const T*)Q, (const T*)K, (const T*)V,
-                                            (const T*)dO, lse, delta, (T*)dV);
-        BOATCU_LAUNCH_OK("attn_bwd_dv_simt");
-    }
+    const void* in[4] = {Q, K, V, dO};
+    BwdArgs<T> a;
+    a.Q = (const T*)Q; a.K = (const T*)K; a.V = (const T*)V; a.dO = (const T*)dO;
+    a.lse = lse; a.delta = delta;
+    a.dQ = (T*)dQ; a.dK = (T*)dK; a.dV = (T*)dV;
+    a.units = (int)units; a.S = (int)S; a.hs = hs; a.causal = causal;
+    a.vec = rows_aligned(in, 4, hs, sizeof(T));
+    a.scale = scale;
+    kern<<<(unsigned)(2 * units * ceil_div(S, kRows)), kThreads, Tiles<HS>::BWD_SMEM, stream()>>>(a);
+    BOATCU_LAUNCH_OK("attn_bwd_simt");
     return 0;
 }
 
@@ -273,21 +405,25 @@ static int launch_bwd(int64_t units, int64_t S, int hs, int causal, float scale,
     do {                                                                                      \
         if (io_type == BOAT_CUDA_BF16) {                                                      \
             if (hs <= 16) return FN<16, __nv_bfloat16>(__VA_ARGS__);                          \
+            if (hs <= 32) return FN<32, __nv_bfloat16>(__VA_ARGS__);                          \
             if (hs <= 64) return FN<64, __nv_bfloat16>(__VA_ARGS__);                          \
             return FN<128, __nv_bfloat16>(__VA_ARGS__);                                       \
         } else {                                                                              \
             if (hs <= 16) return FN<16, float>(__VA_ARGS__);                                  \
+            if (hs <= 32) return FN<32, float>(__VA_ARGS__);                                  \
             if (hs <= 64) return FN<64, float>(__VA_ARGS__);                                  \
             return FN<128, float>(__VA_ARGS__);                                               \
         }                                                                                     \
     } while (0)
 
-static int check_shape(int64_t units, int64_t S, int64_t hs) {
+int check_shape(int64_t units, int64_t S, int64_t hs) {
     if (hs > 128) return set_error(8, "attention: head size %lld > 128 is not supported", (long long)hs);
-    if (units > 65535) return set_error(8, "attention: %lld (batch x heads) units exceed 65535", (long long)units);
-    (void)S;
+    if (S > (1ll << 30) || units * ceil_div(S, kRows) > (1ll << 30))
+        return set_error(8, "attention: %lld (batch x heads) units of %lld rows are too many for one launch", (long long)units, (long long)S);
     return 0;
 }
+
+}  // namespace
 
 int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, int io_type, void* O, float* lse) {

@@ -74,8 +74,11 @@ int rowdot_stats(const void* dO, const void* O, int type, int64_t units, int64_t
                  const float* lse, float scale, float* delta2_out, float* lse2_out);
 
 // CUDA-core (exact FP32 accumulate) implementations, any shape.
-int gemm_simt(int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
-              const void* B, int64_t ldb, int in_type, void* C, int64_t ldc, int out_type, const float* bias);
+// gemm_simt_grouped: up to four problems of one shape in one launch; bias may be NULL or hold NULLs; with
+// `colsum` (may be NULL or hold NULLs) problem g also writes the sums of B's columns over K.
+int gemm_simt_grouped(int trans_a, int trans_b, int groups, int64_t M, int64_t N, int64_t K, const void* const* A,
+                      int64_t lda, const void* const* B, int64_t ldb, int in_type, void* const* C, int64_t ldc,
+                      int out_type, const float* const* bias, float* const* colsum);
 int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, int io_type, void* O, float* lse);
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,

@@ -44,7 +44,7 @@ int boat_cuda_gemm(int mma, int ta, int tb, int64_t M, int64_t N, int64_t K, con
         // accurate than the requested tensor-core format, never less).
     }
     ProfileScope prof("gemm_simt");
-    return gemm_simt(ta, tb, M, N, K, A, lda, B, ldb, in_type, C, ldc, out_type, bias);
+    return gemm_simt_grouped(ta, tb, 1, M, N, K, &A, lda, &B, ldb, in_type, &C, ldc, out_type, &bias, nullptr);
 }
 
 int boat_cuda_gemm_set_yielding(int on) {
@@ -63,11 +63,40 @@ int boat_cuda_gemm_grouped(int mma, int ta, int tb, int groups, int64_t M, int64
     for (int g = 0; g < groups && one_launch; ++g)
         one_launch = A[g] && B[g] && C[g] && gemm_tc_supported(mma, ta, tb, M, N, K, A[g], lda, B[g], ldb, store, C[g], ldc, out_type);
     if (one_launch) return gemm_tc_grouped(mma, ta, tb, groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias);
-    // shapes the tensor-core kernel does not cover (or bad arguments, reported by the single call)
+    // the CUDA cores take a group as one launch too
+    bool valid = out_type >= BOAT_CUDA_F32 && out_type <= BOAT_CUDA_F32_TF32 && M > 0 && N > 0 && K >= 0;
+    bool none_tc = true;
+    for (int g = 0; g < groups && valid; ++g) {
+        valid = A[g] && B[g] && C[g];
+        none_tc = none_tc && (mma == BOAT_MMA_FP32 || !gemm_tc_supported(mma, ta, tb, M, N, K, A[g], lda, B[g], ldb, store, C[g], ldc, out_type));
+    }
+    if (valid && none_tc) {
+        ProfileScope prof("gemm_simt");
+        return gemm_simt_grouped(ta, tb, groups, M, N, K, A, lda, B, ldb, store, C, ldc, out_type, bias, nullptr);
+    }
+    // a mixed group (one operand unaligned), or bad arguments, reported by the single call
     for (int g = 0; g < groups; ++g)
         if (int rc = boat_cuda_gemm(mma, ta, tb, M, N, K, A[g], lda, B[g], ldb, in_type, C[g], ldc, out_type, bias ? bias[g] : nullptr))
             return rc;
     return 0;
+}
+
+int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T, const void* const* X, const void* const* dY,
+                           int in_type, float* const* dW, float* const* db) {
+    if (groups < 1 || groups > 4) return set_error(11, "boat_cuda_weight_grads: %d groups (1 to 4)", groups);
+    if (!X || !dY || !dW) return set_error(11, "boat_cuda_weight_grads: NULL operand table");
+    if (int rc = check_types("boat_cuda_weight_grads", mma, in_type)) return rc;
+    bool ok = I > 0 && O > 0 && T > 0;
+    for (int g = 0; g < groups; ++g) ok = ok && X[g] && dY[g] && dW[g];
+    if (ok && mma == BOAT_MMA_FP32) {
+        // the CUDA-core kernel has the rows of dY in its hands anyway: one launch, one pass
+        ProfileScope prof("gemm_simt");
+        return gemm_simt_grouped(1, 0, groups, I, O, T, X, I, dY, O, in_type == BOAT_CUDA_BF16 ? in_type : (int)BOAT_CUDA_F32,
+                                 (void* const*)dW, O, BOAT_CUDA_F32, nullptr, db);
+    }
+    if (int rc = boat_cuda_gemm_grouped(mma, 1, 0, groups, I, O, T, X, I, dY, O, in_type, (void* const*)dW, O, BOAT_CUDA_F32, nullptr))
+        return rc;
+    return db && db[0] ? boat_cuda_colsum_multi(dY, in_type, T, O, db, groups) : 0;
 }
 
 int boat_cuda_attn_fwd(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,

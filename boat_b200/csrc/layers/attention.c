@@ -541,11 +541,11 @@ static bool backward_pipelined(boat_attention_t* a, const boat_tensor_t* grad_ou
         }
     }
     /* sums over all rows: dWo = ctx^T . dOut, dbo = colsum(dOut), dW = X^T . dP, db = colsum(dP) */
-    if (boat_report("dWo", boat_cuda_gemm(mma, 1, 0, H, H, T, a->d_ctx, H, d_go, H, type, d_dw[WO], H, BOAT_CUDA_F32, NULL)) != 0) goto done;
-    if (bias && boat_report("dbo", boat_cuda_colsum(d_go, type, T, H, d_db[WO])) != 0) goto done;
-    for (int i = 0; i < 3; ++i) {
-        if (boat_report("dW", boat_cuda_gemm(mma, 1, 0, H, H, T, a->d_in[i], H, d_dproj[i], H, type, d_dw[i], H, BOAT_CUDA_F32, NULL)) != 0) goto done;
-        if (bias && boat_report("db", boat_cuda_colsum(d_dproj[i], type, T, H, d_db[i])) != 0) goto done;
+    {
+        const void* x[4] = {a->d_in[0], a->d_in[1], a->d_in[2], a->d_ctx};
+        const void* dy[4] = {d_dproj[0], d_dproj[1], d_dproj[2], d_go};
+        if (boat_report("weight gradients", boat_cuda_weight_grads(mma, 4, H, H, T, x, dy, type, d_dw, bias ? d_db : NULL)) != 0)
+            goto done;
     }
     if (a->device != BOAT_DEVICE_CUDA &&
         boat_report("gradient download", boat_cuda_download_async(a->grad_bucket->data, d_dw[0], a->grad_bucket->nbytes)) != 0)
@@ -862,8 +862,11 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
     d_dctx = dev_alloc(act_bytes);
     if (!d_dctx) goto done;
     if (boat_report("dOut.Wo^T", boat_cuda_gemm(mma, 0, 1, T, H, H, d_go, H, p.w[WO], H, type, d_dctx, H, feed_type(mma, type), NULL)) != 0) goto done;
-    if (boat_report("dWo", boat_cuda_gemm(mma, 1, 0, H, H, T, a->d_ctx, H, d_go, H, type, d_dw[WO], H, BOAT_CUDA_F32, NULL)) != 0) goto done;
-    if (bias && boat_report("dbo", boat_cuda_colsum(d_go, type, T, H, d_db[WO])) != 0) goto done;
+    {
+        const void* x[1] = {a->d_ctx};
+        const void* dy[1] = {d_go};
+        if (boat_report("dWo", boat_cuda_weight_grads(mma, 1, H, H, T, x, dy, type, &d_dw[WO], bias ? &d_db[WO] : NULL)) != 0) goto done;
+    }
     /* Data parallel with overlap: dWo and dbo are final here, long before the step ends - their
      * sum over the ranks runs under the attention-core backward. */
     const bool overlap = a->grad_overlap != 0 && a->device == BOAT_DEVICE_CUDA && boat_cuda_comm_world() > 1;
@@ -891,11 +894,9 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
 
     /* input projections: dW = X^T . dP and db = colsum(dP) first - with overlap their sum over
      * the ranks then runs under the three dX = dP . W^T GEMMs that follow */
-    if (boat_report("dW", boat_cuda_gemm_grouped(mma, 1, 0, 3, H, H, T, (const void* const*)a->d_in, H,
-                                                 (const void* const*)d_dproj, H, type, (void* const*)d_dw, H,
-                                                 BOAT_CUDA_F32, NULL)) != 0)
+    if (boat_report("dW", boat_cuda_weight_grads(mma, 3, H, H, T, (const void* const*)a->d_in, (const void* const*)d_dproj,
+                                                 type, d_dw, bias ? d_db : NULL)) != 0)
         goto done;
-    if (bias && boat_report("db", boat_cuda_colsum_multi((const void* const*)d_dproj, type, T, H, d_db, 3)) != 0) goto done;
     if (overlap && a->grad_overlap == 1) {
         float* piece[2] = {d_dw[WQ], d_db[WQ]};            /* dWq|dWk|dWv and dbq|dbk|dbv are contiguous */
         const int64_t count[2] = {3 * H * H, bias ? 3 * H : 0};

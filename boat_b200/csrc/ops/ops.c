@@ -96,7 +96,7 @@ static boat_tensor_t* binary(const boat_tensor_t* a, const boat_tensor_t* b, boo
     if (da.p && db.p && dout.p) {
         int64_t n = (int64_t)a->nelements, cols = (int64_t)b->nelements;
         if (cols == n)
-            rc = is_add ? (boat_cuda_memcpy_d2d(dout.p, da.p, a->nbytes) || boat_cuda_axpy(dout.p, db.p, 1.0f, n))
+            rc = is_add ? boat_cuda_lincomb(dout.p, da.p, 1.0f, db.p, 1.0f, BOAT_CUDA_F32, n)
                         : boat_cuda_mul(dout.p, da.p, db.p, n);
         else if (is_add)
             rc = boat_cuda_add_bias(dout.p, da.p, db.p, n / cols, cols);

@@ -108,6 +108,13 @@ int boat_cuda_gemm_grouped(int mma, int trans_a, int trans_b, int groups, int64_
                            const void* const* A, int64_t lda, const void* const* B, int64_t ldb, int in_type,
                            void* const* C, int64_t ldc, int out_type, const float* const* bias);
 
+/* Parameter gradients of `groups` (1 to 4) projections y = x.W + b of one shape: dW = X^T . dY and, where
+ * db is not NULL, db = column sums of dY (linear_projection_backward, attention.c:1186-1293).  X [T,I]
+ * and dY [T,O] of type `in_type`, dW [I,O] and db [O] FP32, all packed; overwritten.  db must be given for
+ * all groups or none. */
+int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T, const void* const* X,
+                           const void* const* dY, int in_type, float* const* dW, float* const* db);
+
 /* ---- attention core: replaces scaled_dot_product_attention_impl
  *      (src/layers/attention.c:882-1079) ------------------------------------------------
  * Q,K,V,O are [units, S, hs] contiguous: unit u = (b*nh + h) is the block at element
