@@ -201,6 +201,7 @@ PROTOTYPES = {
     "boat_cuda_malloc": (_I, [_PP, _SZ]),
     "boat_cuda_free": (_I, [_P]),
     "boat_cuda_memcpy_h2d": (_I, [_P, _P, _SZ]),
+    "boat_cuda_memcpy_h2d_async": (_I, [_P, _P, _SZ]),
     "boat_cuda_memcpy_d2h": (_I, [_P, _P, _SZ]),
     "boat_cuda_memcpy_d2d": (_I, [_P, _P, _SZ]),
     "boat_cuda_copies_after_compute": (_I, []),
@@ -230,6 +231,7 @@ PROTOTYPES = {
     "boat_cuda_colsum_multi": (_I, [_P, _I, _I64, _I64, _P, _I]),
     "boat_cuda_convert_multi": (_I, [_P, _I, _P, _P, _I]),
     "boat_cuda_axpy": (_I, [_P, _P, _F, _I64]),
+    "boat_cuda_axpy_multi": (_I, [_P, _P, _F, _P, _I]),
     "boat_cuda_scale": (_I, [_P, _P, _F, _I64]),
     "boat_cuda_add_bias": (_I, [_P, _P, _P, _I64, _I64]),
     "boat_cuda_mul": (_I, [_P, _P, _P, _I64]),

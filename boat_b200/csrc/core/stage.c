@@ -1,6 +1,7 @@
 /* stage.c - see stage.h. */
 #include "stage.h"
 #include <stdlib.h>
+#include <string.h>
 #include <strings.h>
 
 int boat_storage_of(boat_dtype_t dt) { return dt == BOAT_DTYPE_BFLOAT16 ? BOAT_CUDA_BF16 : BOAT_CUDA_F32; }
@@ -81,4 +82,57 @@ int boat_default_mma(boat_dtype_t dt) {
     const char* e = getenv("BOAT_MMA");
     if (e && !strcasecmp(e, "tf32")) return BOAT_MMA_TF32;
     return BOAT_MMA_FP32;
+}
+
+bool boat_bundle_send(boat_bundle_t* b, const boat_tensor_t* const* tensors, int n) {
+    memset(b, 0, sizeof *b);
+    size_t total = 0;
+    for (int i = 0; i < n; ++i) {
+        const boat_tensor_t* t = tensors[i];
+        if (!t || t->device == BOAT_DEVICE_CUDA || t->nbytes >= BOAT_BUNDLE_LIMIT || b->count == BOAT_BUNDLE_MAX) continue;
+        bool seen = false;
+        for (int j = 0; j < b->count; ++j) seen = seen || b->tensor[j] == t;
+        if (seen) continue;
+        b->tensor[b->count] = t;
+        b->offset[b->count++] = total;
+        total += boat_align256(t->nbytes);
+    }
+    if (b->count == 0) return true;
+    b->host = boat_cuda_host_alloc(total);
+    b->dev = b->host ? boat_dev_alloc(total) : NULL;
+    if (!b->dev) {                                       /* no image: the tensors are sent one by one */
+        if (b->host) boat_cuda_host_free(b->host);
+        memset(b, 0, sizeof *b);
+        return true;
+    }
+    for (int i = 0; i < b->count; ++i) memcpy((char*)b->host + b->offset[i], b->tensor[i]->data, b->tensor[i]->nbytes);
+    b->sent = true;
+    return boat_report("upload", boat_cuda_memcpy_h2d_async(b->dev, b->host, total)) == 0;
+}
+
+void* boat_bundle_find(const boat_bundle_t* b, const boat_tensor_t* t) {
+    for (int i = 0; i < b->count; ++i)
+        if (b->tensor[i] == t) return (char*)b->dev + b->offset[i];
+    return NULL;
+}
+
+void boat_bundle_settle(boat_bundle_t* b, bool synced) {
+    if (b->sent && !synced) boat_report("upload", boat_cuda_sync());
+    b->sent = false;
+    if (b->host) boat_cuda_host_free(b->host);
+    b->host = NULL;
+}
+
+int boat_scatter_down(const void* dev, size_t total, void* const* host, const size_t* offset, const size_t* bytes, int n) {
+    char* image = total < BOAT_BUNDLE_LIMIT ? (char*)boat_cuda_host_alloc(total) : NULL;
+    int rc = 0;
+    if (image) {
+        rc = boat_cuda_memcpy_d2h(image, dev, total);
+        for (int i = 0; i < n && rc == 0; ++i) memcpy(host[i], image + offset[i], bytes[i]);
+        boat_cuda_host_free(image);
+        return rc;
+    }
+    for (int i = 0; i < n && rc == 0; ++i) rc = boat_cuda_download_async(host[i], (const char*)dev + offset[i], bytes[i]);
+    const int done = boat_cuda_sync();
+    return rc ? rc : done;
 }

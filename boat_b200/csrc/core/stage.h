@@ -18,6 +18,32 @@ boat_tensor_t* boat_emit_out(const int64_t* shape, size_t ndim, const boat_tenso
  * of the same storage type becomes a tensor around *src itself (no copy) and *src is set to NULL,
  * so that the caller's boat_dev_free(*src) is a no-op; every other case copies as boat_emit_out. */
 boat_tensor_t* boat_emit_out_take(const int64_t* shape, size_t ndim, const boat_tensor_t* like, void** src, int type);
+
+/* Host tensors on their way to the GPU for one call.  Every copy has a fixed cost of some 10 us when the
+ * host waits for it, which is all that small tensors cost; so those under BOAT_BUNDLE_LIMIT bytes are
+ * packed into one page-locked image and go up as one copy, larger ones are sent one by one, and
+ * nothing is waited for until the call ends. */
+#define BOAT_BUNDLE_LIMIT ((size_t)256 * 1024)
+enum { BOAT_BUNDLE_MAX = 16 };
+typedef struct {
+    void *host, *dev;                                    /* the image and its copy in HBM */
+    const boat_tensor_t* tensor[BOAT_BUNDLE_MAX];
+    size_t offset[BOAT_BUNDLE_MAX];
+    int count;
+    bool sent;                                           /* uploads of this call may still be reading host memory */
+} boat_bundle_t;
+/* Sends the small host tensors among the n given ones (NULL entries are skipped).  false on failure. */
+bool   boat_bundle_send(boat_bundle_t* b, const boat_tensor_t* const* tensors, int n);
+/* Where tensor `t` lies in HBM, or NULL when it was not packed. */
+void*  boat_bundle_find(const boat_bundle_t* b, const boat_tensor_t* t);
+/* Ends the call: waits for the uploads unless `synced` (the host has waited for a later copy), and
+ * gives the image back.  The HBM copy is the caller's to free (boat_dev_free(b->dev)). */
+void   boat_bundle_settle(boat_bundle_t* b, bool synced);
+/* Copies n pieces of one device block (at `offset`, `bytes` long) to host memory and waits: small totals as
+ * one copy through a page-locked image. */
+int    boat_scatter_down(const void* dev, size_t total, void* const* host, const size_t* offset, const size_t* bytes, int n);
+static inline size_t boat_align256(size_t n) { return (n + 255) & ~(size_t)255; }
+
 /* Arithmetic for FP32/BF16 inputs outside the attention layer: BF16 storage -> BF16 tensor
  * cores; FP32 storage -> env BOAT_MMA (tf32 | fp32), default exact FP32. */
 int    boat_default_mma(boat_dtype_t dt);

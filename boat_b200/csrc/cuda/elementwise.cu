@@ -67,6 +67,26 @@ static int launch_axpy(float* y, const float* x, float alpha, int64_t n) {
     return 0;
 }
 
+// ---- y[t] = alpha*x[t] + y[t] for several tensors, blockIdx.y = tensor: the SGD step of a layer -------
+constexpr int kMaxAxpy = 8;
+struct AxpyTable {
+    float* y[kMaxAxpy];
+    const float* x[kMaxAxpy];
+    int64_t n[kMaxAxpy];
+};
+__global__ void axpy_multi_kernel(const AxpyTable t, float alpha, int vec) {
+    float* __restrict__ y = t.y[blockIdx.y];
+    const float* __restrict__ x = t.x[blockIdx.y];
+    const int64_t n = t.n[blockIdx.y], n4 = vec ? n / 4 : 0;
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < n4; i += step) {
+        const float4 a = reinterpret_cast<const float4*>(x)[i], b = reinterpret_cast<const float4*>(y)[i];
+        reinterpret_cast<float4*>(y)[i] = make_float4(mul_add(alpha, a.x, b.x), mul_add(alpha, a.y, b.y),
+                                                      mul_add(alpha, a.z, b.z), mul_add(alpha, a.w, b.w));
+    }
+    for (int64_t i = n4 * 4 + i0; i < n; i += step) y[i] = mul_add(alpha, x[i], y[i]);
+}
+
 // ---- y = a * b -------------------------------------------------------------------------------
 __global__ void mul_kernel(float* __restrict__ y, const float* __restrict__ a, const float* __restrict__ b,
                            int64_t n, int vec) {
@@ -424,6 +444,28 @@ extern "C" {
 
 int boat_cuda_axpy(float* y, const float* x, float alpha, int64_t n) { return launch_axpy<true>(y, x, alpha, n); }
 int boat_cuda_scale(float* y, const float* x, float alpha, int64_t n) { return launch_axpy<false>(y, x, alpha, n); }
+
+int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, const int64_t* n, int count) {
+    if (count <= 0) return 0;
+    if (count > kMaxAxpy || !y || !x || !n) return set_error(11, "boat_cuda_axpy_multi: bad table (%d tensors, 1 to %d)", count, kMaxAxpy);
+    if (int rc = ensure_init()) return rc;
+    AxpyTable t;
+    int vec = 1;
+    int64_t longest = 0;
+    for (int i = 0; i < kMaxAxpy; ++i) {
+        const int s = i < count ? i : 0;
+        if (n[s] > 0 && (!y[s] || !x[s])) return set_error(11, "boat_cuda_axpy_multi: bad entry %d", s);
+        t.y[i] = y[s];
+        t.x[i] = x[s];
+        t.n[i] = n[s];
+        vec = vec && aligned16(y[s]) && aligned16(x[s]);
+        if (n[s] > longest) longest = n[s];
+    }
+    if (longest <= 0) return 0;
+    axpy_multi_kernel<<<dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, stream()>>>(t, alpha, vec);
+    BOATCU_LAUNCH_OK("axpy_multi");
+    return 0;
+}
 
 int boat_cuda_mul(float* y, const float* a, const float* b, int64_t n) {
     if (n <= 0) return 0;

@@ -399,6 +399,13 @@ int boat_cuda_memcpy_h2d(void* dst, const void* src, size_t bytes) {
     return 0;
 }
 
+int boat_cuda_memcpy_h2d_async(void* dst, const void* src, size_t bytes) {
+    if (bytes == 0) return 0;
+    if (int rc = ensure_init()) return rc;
+    BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g_stream));
+    return 0;
+}
+
 int boat_cuda_memcpy_d2h(void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;

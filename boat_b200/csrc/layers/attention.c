@@ -18,7 +18,7 @@
  *     multi-GPU path reduces them with a single collective; each backward overwrites it
  *     (the reference replaces the tensors, :653-654, :702-703 - same "no accumulation").
  */
-#include "../core/boat_internal.h"
+#include "../core/stage.h"
 #include <boat/layers.h>
 #include <boat_b200.h>
 #include <math.h>
@@ -55,6 +55,7 @@ struct boat_attention_t {
     void*          d_proj[3];           /* Qp, Kp, Vp [B*S, H]                     */
     void*          d_ctx;               /* attention output before Wo              */
     float*         d_lse;               /* [B*nh*S]                                */
+    void*          d_bundle;            /* small host tensors of the forward, some of d_in among them */
 
     /* The four FP32 weights of a CUDA layer in the form the tensor cores read (BF16, or TF32-valued
      * FP32), made by one launch in forward and used again by the backward of the same step.
@@ -68,34 +69,27 @@ struct boat_attention_t {
 
 /* ---- small helpers ---------------------------------------------------------------------- */
 
-static int storage_of(boat_dtype_t dt) { return dt == BOAT_DTYPE_BFLOAT16 ? BOAT_CUDA_BF16 : BOAT_CUDA_F32; }
-static size_t storage_size(int type) { return type == BOAT_CUDA_BF16 ? 2 : 4; }
-static bool dtype_ok(boat_dtype_t dt) { return dt == BOAT_DTYPE_FLOAT32 || dt == BOAT_DTYPE_BFLOAT16; }
-
-static void* dev_alloc(size_t bytes) {
-    void* p = NULL;
-    if (boat_report("device allocation", boat_cuda_malloc(&p, bytes)) != 0) return NULL;
-    return p;
-}
-
-static void dev_free(void* p) {
-    if (p) boat_report("device free", boat_cuda_free(p));
-}
+#define storage_of boat_storage_of
+#define storage_size boat_storage_size
+#define dtype_ok boat_dtype_supported
+#define dev_alloc boat_dev_alloc
+#define dev_free boat_dev_free
 
 /* Device buffer holding tensor `t` in storage type `type`.  *owned says whether the caller
- * must release it (false: it is the tensor's own HBM). */
-static void* stage_in(const boat_tensor_t* t, int type, bool* owned) {
-    int have = storage_of(t->dtype);
-    size_t n = t->nelements;
+ * must release it (false: it is the tensor's own HBM, or part of the bundle). */
+static void* stage_in(boat_bundle_t* b, const boat_tensor_t* t, int type, bool* owned) {
+    const int have = storage_of(t->dtype);
+    const size_t n = t->nelements;
+    void* raw = t->device == BOAT_DEVICE_CUDA ? t->data : boat_bundle_find(b, t);
     *owned = false;
-    if (t->device == BOAT_DEVICE_CUDA && have == type) return t->data;
+    if (raw && have == type) return raw;
     *owned = true;
-    void* raw = t->data;
     void* tmp = NULL;
-    if (t->device != BOAT_DEVICE_CUDA) {
+    if (!raw) {
         tmp = dev_alloc(n * storage_size(have));
         if (!tmp) return NULL;
-        if (boat_report("upload", boat_cuda_memcpy_h2d(tmp, t->data, n * storage_size(have))) != 0) {
+        b->sent = true;
+        if (boat_report("upload", boat_cuda_memcpy_h2d_async(tmp, t->data, n * storage_size(have))) != 0) {
             dev_free(tmp);
             return NULL;
         }
@@ -114,8 +108,8 @@ static void* stage_in(const boat_tensor_t* t, int type, bool* owned) {
 /* Operand for arithmetic `mma`: like stage_in, and for TF32 the values are additionally
  * rounded to the nearest TF32 number (in a private copy - the caller's tensor is never
  * modified), so that the tensor core's truncation of FP32 operands is exact. */
-static void* stage_operand(const boat_tensor_t* t, int mma, int type, bool* owned) {
-    void* p = stage_in(t, type, owned);
+static void* stage_operand(boat_bundle_t* b, const boat_tensor_t* t, int mma, int type, bool* owned) {
+    void* p = stage_in(b, t, type, owned);
     if (!p || mma != BOAT_MMA_TF32) return p;
     void* dst = p;
     if (!*owned) {
@@ -135,33 +129,6 @@ static void* stage_operand(const boat_tensor_t* t, int mma, int type, bool* owne
  * the epilogue rounds to TF32 (the attention kernels do the same for their outputs), so no
  * separate rounding pass runs between kernels. */
 static int feed_type(int mma, int type) { return mma == BOAT_MMA_TF32 ? BOAT_CUDA_F32_TF32 : type; }
-
-/* New tensor with the dtype/device of `like`, filled from device buffer `src` (storage
- * `type`): a cast on the device for a CUDA result, a download (after a cast when the types
- * differ) for a host result.  `src` stays the caller's. */
-static boat_tensor_t* emit_out(const int64_t* shape, size_t ndim, const boat_tensor_t* like, void* src,
-                               int type) {
-    boat_tensor_t* out = boat_tensor_create_uninit(shape, ndim, like->dtype, like->device);
-    if (!out) return NULL;
-    int want = storage_of(like->dtype);
-    size_t n = out->nelements;
-    int rc = 0;
-    if (like->device == BOAT_DEVICE_CUDA) {
-        rc = boat_cuda_cast(out->data, want, src, type, (int64_t)n);
-    } else if (want == type) {
-        rc = boat_cuda_memcpy_d2h(out->data, src, n * storage_size(type));
-    } else {
-        void* tmp = dev_alloc(n * storage_size(want));
-        rc = tmp ? boat_cuda_cast(tmp, want, src, type, (int64_t)n) : 1;
-        if (rc == 0) rc = boat_cuda_memcpy_d2h(out->data, tmp, n * storage_size(want));
-        dev_free(tmp);
-    }
-    if (boat_report("result transfer", rc) != 0) {
-        boat_tensor_free(out);
-        return NULL;
-    }
-    return out;
-}
 
 static int env_precision(void) {
     const char* e = getenv("BOAT_MMA");
@@ -200,6 +167,8 @@ static void drop_forward_state(boat_attention_t* a) {
     a->d_ctx = NULL;
     dev_free(a->d_lse);
     a->d_lse = NULL;
+    dev_free(a->d_bundle);
+    a->d_bundle = NULL;
     a->cached = false;
 }
 
@@ -252,7 +221,7 @@ static bool shadow_weights(boat_attention_t* a, int form, bool backward, staged_
     return true;
 }
 
-static bool stage_params(boat_attention_t* a, int mma, int type, bool backward, staged_params_t* p) {
+static bool stage_params(boat_attention_t* a, boat_bundle_t* b, int mma, int type, bool backward, staged_params_t* p) {
     memset(p, 0, sizeof *p);
     bool shadow = a->device == BOAT_DEVICE_CUDA && (type == BOAT_CUDA_BF16 || mma == BOAT_MMA_TF32);
     for (int i = 0; i < 4 && shadow; ++i) {
@@ -262,10 +231,10 @@ static bool stage_params(boat_attention_t* a, int mma, int type, bool backward, 
     }
     if (shadow && !shadow_weights(a, mma == BOAT_MMA_TF32 ? BOAT_CUDA_F32_TF32 : BOAT_CUDA_BF16, backward, p)) return false;
     for (int i = 0; i < 4; ++i) {
-        if (!shadow) p->w[i] = stage_operand(a->param[WQ + i], mma, type, &p->w_owned[i]);
+        if (!shadow) p->w[i] = stage_operand(b, a->param[WQ + i], mma, type, &p->w_owned[i]);
         if (!p->w[i]) goto fail;
-        if (a->param[BQ + i]) {
-            p->b[i] = (float*)stage_in(a->param[BQ + i], BOAT_CUDA_F32, &p->b_owned[i]);
+        if (a->param[BQ + i] && !backward) {             /* the backward reads no bias */
+            p->b[i] = (float*)stage_in(b, a->param[BQ + i], BOAT_CUDA_F32, &p->b_owned[i]);
             if (!p->b[i]) goto fail;
         }
     }
@@ -338,6 +307,10 @@ static bool stage_param_range(boat_attention_t* a, int type, staged_params_t* p,
  * per row is the same as in the one-piece path.  A host layer's parameters go up on the upload
  * stream as well, behind the first chunk and in the order the kernels need them. */
 enum { MAX_CHUNKS = 8 };
+
+/* Chunks pay when the transfers are long against the launches they multiply: from about this many bytes
+ * per activation tensor (40 us of PCIe) on.  Below, a call sends what it needs up front. */
+#define PIPELINE_MIN_BYTES ((size_t)2 << 20)
 
 static bool on_host(const boat_tensor_t* t) { return t->device != BOAT_DEVICE_CUDA; }
 
@@ -650,12 +623,23 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
     a->gran = gran;
 
     staged_params_t p;
+    memset(&p, 0, sizeof p);
     void* d_out = NULL;
     boat_tensor_t* result = NULL;
-    const bool pipelined = units / gran >= 2 && pipeline_enabled() && on_host(query) && on_host(key) && on_host(value);
+    bool synced = false;
+    const bool pipelined = units / gran >= 2 && act_bytes >= PIPELINE_MIN_BYTES && pipeline_enabled() && on_host(query) &&
+                           on_host(key) && on_host(value);
+    boat_bundle_t bundle;
+    memset(&bundle, 0, sizeof bundle);
+    if (!pipelined) {
+        const boat_tensor_t* t[3 + NPARAM] = {query, key, value};
+        for (int i = 0; i < NPARAM; ++i) t[3 + i] = a->param[i];
+        if (!boat_bundle_send(&bundle, t, 3 + NPARAM)) goto done;
+        a->d_bundle = bundle.dev;
+    }
     /* a host layer's parameters of a chunked call are brought up inside it, behind the first chunk */
     if (!(pipelined && a->device != BOAT_DEVICE_CUDA && prepare_late_params(a, mma, type, true, &p)) &&
-        !stage_params(a, mma, type, false, &p))
+        !stage_params(a, &bundle, mma, type, false, &p))
         goto done;
     if (pipelined) {
         result = forward_pipelined(a, in, mma, type, &p);
@@ -671,7 +655,7 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
             a->d_in[i] = a->d_in[same];
             a->d_in_owned[i] = false;
         } else {
-            a->d_in[i] = stage_operand(in[i], mma, type, &a->d_in_owned[i]);
+            a->d_in[i] = stage_operand(&bundle, in[i], mma, type, &a->d_in_owned[i]);
             if (!a->d_in[i]) goto done;
         }
     }
@@ -712,11 +696,19 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
             if (boat_report("output projection", boat_cuda_gemm(mma, 0, 0, T, H, H, a->d_ctx, H, p.w[WO], H, type,
                                                                 d_out, H, out_type, p.b[WO])) != 0)
                 goto done;
-            result = emit_out(query->shape, query->ndim, query, d_out, out_type);
+            result = boat_tensor_create_uninit(query->shape, query->ndim, query->dtype, query->device);
+            if (!result) goto done;
+            const size_t at = 0;
+            synced = boat_report("result transfer", boat_scatter_down(d_out, result->nbytes, &result->data, &at, &result->nbytes, 1)) == 0;
+            if (!synced) {
+                boat_tensor_free(result);
+                result = NULL;
+            }
         }
     }
     if (result) a->cached = true;
 done:
+    boat_bundle_settle(&bundle, synced);
     dev_free(d_out);
     release_params(&p);
     if (!result) {
@@ -820,10 +812,18 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
     bool ok = false, go_owned = false;
     staged_params_t p;
     memset(&p, 0, sizeof p);
-    void *d_go = NULL, *d_dctx = NULL, *d_dproj[3] = {NULL, NULL, NULL}, *scratch = NULL, *d_dx = NULL;
+    boat_bundle_t bundle;
+    memset(&bundle, 0, sizeof bundle);
+    void *d_go = NULL, *d_dctx = NULL, *d_dproj[3] = {NULL, NULL, NULL}, *scratch = NULL;
     float* d_bucket = NULL;
     boat_tensor_t* gin[3] = {NULL, NULL, NULL};
     size_t scratch_bytes;
+    /* results on their way to the host: one device block, input gradients then the bucket */
+    void* d_down = NULL;
+    void* down_host[4];
+    size_t down_at[4], down_bytes[4], down_total = 0;
+    int down = 0;
+    bool synced = false;
 
     if (!ensure_grads(a)) goto done;
     /* gradient sums of this layer's previous step still on the communication stream read the bucket
@@ -833,18 +833,42 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
         boat_report("gradient all-reduce", boat_cuda_allreduce_join()) != 0)
         goto done;
     a->sums_begun = false;
-    const bool pipelined = units / a->gran >= 2 && pipeline_enabled() && on_host(grad_output) && on_host(a->cache_in[0]) &&
+    const bool pipelined = units / a->gran >= 2 && act_bytes >= PIPELINE_MIN_BYTES && pipeline_enabled() && on_host(grad_output) && on_host(a->cache_in[0]) &&
                            on_host(a->cache_in[1]) && on_host(a->cache_in[2]);
+    if (!pipelined) {
+        const boat_tensor_t* t[5] = {grad_output, a->param[WQ], a->param[WK], a->param[WV], a->param[WO]};
+        if (!boat_bundle_send(&bundle, t, 5)) goto done;
+    }
     if (!(pipelined && a->device != BOAT_DEVICE_CUDA && prepare_late_params(a, mma, type, false, &p))) {
         /* (a host layer's parameters of a chunked call are brought up inside it, behind the first chunk) */
-        const bool staged = stage_params(a, mma, type, true, &p);
+        const bool staged = stage_params(a, &bundle, mma, type, true, &p);
         a->shadow_fresh = false;                /* one backward per forward may trust the forward's copies */
         if (!staged) goto done;
     }
-    /* gradients are produced in HBM; a host layer receives them with one copy at the end */
-    d_bucket = a->device == BOAT_DEVICE_CUDA ? (float*)a->grad_bucket->data
-                                             : (float*)dev_alloc(a->grad_bucket->nbytes);
-    if (!d_bucket) goto done;
+    /* gradients are produced in HBM; host results are copied down together at the end */
+    for (int i = 0; i < 3 && !pipelined; ++i) {
+        const boat_tensor_t* x = a->cache_in[i];
+        gin[i] = boat_tensor_create_uninit(x->shape, x->ndim, x->dtype, x->device);
+        if (!gin[i]) goto done;
+        if (x->device == BOAT_DEVICE_CUDA) continue;
+        down_host[down] = gin[i]->data;
+        down_at[down] = down_total;
+        down_bytes[down++] = gin[i]->nbytes;
+        down_total += boat_align256(gin[i]->nbytes);
+    }
+    if (a->device == BOAT_DEVICE_CUDA) {
+        d_bucket = (float*)a->grad_bucket->data;
+    } else {
+        down_host[down] = a->grad_bucket->data;
+        down_at[down] = down_total;
+        down_bytes[down++] = a->grad_bucket->nbytes;
+        down_total += boat_align256(a->grad_bucket->nbytes);
+    }
+    if (down_total) {
+        d_down = dev_alloc(down_total);
+        if (!d_down) goto done;
+        if (!d_bucket) d_bucket = (float*)((char*)d_down + down_at[down - 1]);
+    }
     float* d_dw[4];
     float* d_db[4];
     for (int i = 0; i < 4; ++i) {
@@ -855,7 +879,7 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
         ok = backward_pipelined(a, grad_output, mma, type, &p, d_dw, d_db, gin);
         goto done;
     }
-    d_go = stage_operand(grad_output, mma, type, &go_owned);
+    d_go = stage_operand(&bundle, grad_output, mma, type, &go_owned);
     if (!d_go) goto done;
 
     /* output projection: d(ctx) = dOut . Wo^T,  dWo = ctx^T . dOut,  dbo = colsum(dOut) */
@@ -907,59 +931,39 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
     const bool yield = overlap && a->grad_overlap == 1;      /* a sum was just started beside these GEMMs */
     if (yield) boat_cuda_gemm_set_yielding(1);
     {
-        /* dX = dP . W^T for the three inputs: one launch when they share device and dtype */
-        const boat_tensor_t* x0 = a->cache_in[0];
-        bool together = x0->device == BOAT_DEVICE_CUDA;
-        for (int i = 1; i < 3; ++i)
-            together = together && a->cache_in[i]->device == BOAT_DEVICE_CUDA && a->cache_in[i]->dtype == x0->dtype;
+        /* dX = dP . W^T for the three inputs, each straight into its tensor's HBM or the block that goes
+         * down: one launch when they share the dtype */
+        const int out_type = storage_of(gin[0]->dtype);
+        bool together = true;
+        void* target[3];
+        for (int i = 0, k = 0; i < 3; ++i) {
+            target[i] = gin[i]->device == BOAT_DEVICE_CUDA ? gin[i]->data : (char*)d_down + down_at[k++];
+            together = together && storage_of(gin[i]->dtype) == out_type;
+        }
         if (together) {
-            void* target[3];
-            for (int i = 0; i < 3; ++i) {
-                const boat_tensor_t* x = a->cache_in[i];
-                /* a CUDA gradient is the GEMM's own output buffer: no copy */
-                gin[i] = boat_tensor_create_uninit(x->shape, x->ndim, x->dtype, BOAT_DEVICE_CUDA);
-                if (!gin[i]) goto done;
-                target[i] = gin[i]->data;
-            }
             if (boat_report("dX", boat_cuda_gemm_grouped(mma, 0, 1, 3, T, H, H, (const void* const*)d_dproj, H,
-                                                         (const void* const*)p.w, H, type, target, H,
-                                                         storage_of(x0->dtype), NULL)) != 0)
+                                                         (const void* const*)p.w, H, type, target, H, out_type, NULL)) != 0)
                 goto done;
         } else {
-            for (int i = 0; i < 3; ++i) {
-                const boat_tensor_t* x = a->cache_in[i];
-                int out_type = storage_of(x->dtype);
-                void* dx_target;
-                if (x->device == BOAT_DEVICE_CUDA) {
-                    gin[i] = boat_tensor_create_uninit(x->shape, x->ndim, x->dtype, BOAT_DEVICE_CUDA);
-                    if (!gin[i]) goto done;
-                    dx_target = gin[i]->data;
-                } else {
-                    d_dx = dev_alloc((size_t)T * H * storage_size(out_type));
-                    if (!d_dx) goto done;
-                    dx_target = d_dx;
-                }
-                if (boat_report("dX", boat_cuda_gemm(mma, 0, 1, T, H, H, d_dproj[i], H, p.w[i], H, type, dx_target, H, out_type, NULL)) != 0) goto done;
-                if (x->device != BOAT_DEVICE_CUDA) {
-                    gin[i] = emit_out(x->shape, x->ndim, x, d_dx, out_type);
-                    dev_free(d_dx);
-                    d_dx = NULL;
-                    if (!gin[i]) goto done;
-                }
-            }
+            for (int i = 0; i < 3; ++i)
+                if (boat_report("dX", boat_cuda_gemm(mma, 0, 1, T, H, H, d_dproj[i], H, p.w[i], H, type, target[i], H,
+                                                     storage_of(gin[i]->dtype), NULL)) != 0)
+                    goto done;
         }
     }
-    if (a->device != BOAT_DEVICE_CUDA &&
-        boat_report("gradient download", boat_cuda_memcpy_d2h(a->grad_bucket->data, d_bucket, a->grad_bucket->nbytes)) != 0)
-        goto done;
+    if (down_total) {
+        if (boat_report("gradient download", boat_scatter_down(d_down, down_total, down_host, down_at, down_bytes, down)) != 0) goto done;
+        synced = true;
+    }
     ok = true;
 done:
     boat_cuda_gemm_set_yielding(0);
-    dev_free(d_dx);
+    boat_bundle_settle(&bundle, synced);
+    dev_free(bundle.dev);
+    dev_free(d_down);
     dev_free(scratch);
     for (int i = 0; i < 3; ++i) dev_free(d_dproj[i]);
     dev_free(d_dctx);
-    if (a->device != BOAT_DEVICE_CUDA) dev_free(d_bucket);
     if (go_owned) dev_free(d_go);
     release_params(&p);
     if (!ok) {
@@ -980,22 +984,58 @@ done:
 void boat_attention_update(boat_attention_t* a, float learning_rate) {
     if (!a || !a->grad_bucket) return;
     a->shadow_fresh = false;
+    float *y[NPARAM], *x[NPARAM];
+    int64_t n[NPARAM];
+    int count = 0;
     for (int i = 0; i < NPARAM; ++i) {
-        boat_tensor_t *w = a->param[i], *g = a->grad[i];
-        if (!w || !g) continue;
-        int64_t n = (int64_t)w->nelements;
-        if (a->device == BOAT_DEVICE_CUDA) {
-            boat_report("SGD step", boat_cuda_axpy((float*)w->data, (const float*)g->data, -learning_rate, n));
-            continue;
-        }
-        bool wo, go;
-        float* dw = (float*)stage_in(w, BOAT_CUDA_F32, &wo);
-        float* dg = (float*)stage_in(g, BOAT_CUDA_F32, &go);
-        if (dw && dg && boat_report("SGD step", boat_cuda_axpy(dw, dg, -learning_rate, n)) == 0)
-            boat_report("parameter download", boat_cuda_memcpy_d2h(w->data, dw, w->nbytes));
-        if (wo) dev_free(dw);
-        if (go) dev_free(dg);
+        if (!a->param[i] || !a->grad[i]) continue;
+        y[count] = (float*)a->param[i]->data;
+        x[count] = (float*)a->grad[i]->data;
+        n[count++] = (int64_t)a->param[i]->nelements;
     }
+    if (a->device == BOAT_DEVICE_CUDA) {
+        boat_report("SGD step", boat_cuda_axpy_multi(y, (const float* const*)x, -learning_rate, n, count));
+        return;
+    }
+    /* a host layer: parameters and gradients up, the step, parameters down */
+    const boat_tensor_t* all[NPARAM + 1];
+    for (int i = 0; i < NPARAM; ++i) all[i] = a->param[i];
+    all[NPARAM] = a->grad_bucket;
+    boat_bundle_t bundle;
+    bool bucket_owned = false, synced = false;
+    void *d_new = NULL, *d_grad = NULL, *host[NPARAM];
+    size_t at[NPARAM], bytes[NPARAM], total = 0;
+    if (!boat_bundle_send(&bundle, all, NPARAM + 1)) goto done;
+    d_grad = stage_in(&bundle, a->grad_bucket, BOAT_CUDA_F32, &bucket_owned);
+    if (!d_grad) goto done;
+    /* small parameters are stepped where the bundle put them, otherwise all get a block of their own */
+    bool packed = true;
+    for (int i = 0; i < NPARAM; ++i) packed = packed && (!a->param[i] || boat_bundle_find(&bundle, a->param[i]));
+    char* base = (char*)bundle.dev;
+    for (int i = 0, k = 0; i < NPARAM; ++i) {
+        if (!a->param[i] || !a->grad[i]) continue;
+        host[k] = a->param[i]->data;
+        bytes[k] = a->param[i]->nbytes;
+        at[k] = packed ? (size_t)((char*)boat_bundle_find(&bundle, a->param[i]) - base) : total;
+        total = at[k] + boat_align256(bytes[k]);
+        x[k++] = (float*)((char*)d_grad + ((char*)a->grad[i]->data - (char*)a->grad_bucket->data));
+    }
+    if (!packed) {
+        d_new = dev_alloc(total);
+        if (!d_new) goto done;
+        base = (char*)d_new;
+        bundle.sent = true;
+        for (int k = 0; k < count; ++k)
+            if (boat_report("parameter upload", boat_cuda_memcpy_h2d_async(base + at[k], host[k], bytes[k])) != 0) goto done;
+    }
+    for (int k = 0; k < count; ++k) y[k] = (float*)(base + at[k]);
+    if (boat_report("SGD step", boat_cuda_axpy_multi(y, (const float* const*)x, -learning_rate, n, count)) == 0)
+        synced = boat_report("parameter download", boat_scatter_down(base, total, host, at, bytes, count)) == 0;
+done:
+    boat_bundle_settle(&bundle, synced);
+    dev_free(bundle.dev);
+    if (bucket_owned) dev_free(d_grad);
+    dev_free(d_new);
 }
 
 BOAT_NOINLINE void boat_attention_set_dropout(boat_attention_t* a, float dropout_prob) {
@@ -1047,8 +1087,11 @@ boat_tensor_t* boat_scaled_dot_product_attention(const boat_tensor_t* query, con
     boat_tensor_t* out = NULL;
     void* d_o = NULL;
     float* d_lse = NULL;
+    boat_bundle_t bundle;
+    bool synced = false;
+    if (!boat_bundle_send(&bundle, in, 3)) goto done;
     for (int i = 0; i < 3; ++i) {
-        d[i] = stage_in(in[i], BOAT_CUDA_F32, &owned[i]);
+        d[i] = stage_in(&bundle, in[i], BOAT_CUDA_F32, &owned[i]);
         if (!d[i]) goto done;
     }
     d_o = dev_alloc(query->nbytes);
@@ -1057,8 +1100,11 @@ boat_tensor_t* boat_scaled_dot_product_attention(const boat_tensor_t* query, con
     if (boat_report("attention core", boat_cuda_attn_fwd(BOAT_MMA_FP32, units, S, hs, causal_mask, scale_factor,
                                                          d[0], d[1], d[2], BOAT_CUDA_F32, d_o, d_lse)) != 0)
         goto done;
-    out = emit_out(value->shape, 4, value, d_o, BOAT_CUDA_F32);
+    synced = value->device != BOAT_DEVICE_CUDA;
+    out = boat_emit_out_take(value->shape, 4, value, &d_o, BOAT_CUDA_F32);
 done:
+    boat_bundle_settle(&bundle, synced && out);
+    dev_free(bundle.dev);
     for (int i = 0; i < 3; ++i)
         if (owned[i]) dev_free(d[i]);
     dev_free(d_o);

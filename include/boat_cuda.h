@@ -43,6 +43,8 @@ int         boat_cuda_sync(void);                /* wait for the library stream 
 int         boat_cuda_malloc(void** ptr, size_t bytes);   /* stream-ordered pool allocation */
 int         boat_cuda_free(void* ptr);
 int         boat_cuda_memcpy_h2d(void* dst, const void* src_host, size_t bytes);  /* returns after arrival */
+int         boat_cuda_memcpy_h2d_async(void* dst, const void* src_host, size_t bytes);   /* in stream order; the source
+                                                 must stay as it is until the library stream has passed the copy */
 int         boat_cuda_memcpy_d2h(void* dst_host, const void* src, size_t bytes);  /* returns after arrival */
 int         boat_cuda_memcpy_d2d(void* dst, const void* src, size_t bytes);       /* asynchronous on the stream */
 /* Copies on their own streams, one per direction, so that PCIe traffic overlaps kernels.
@@ -182,6 +184,8 @@ int boat_cuda_colsum(const void* X, int x_type, int64_t rows, int64_t cols, floa
  * the Q, K and V projections. */
 int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count);
 int boat_cuda_axpy(float* y, const float* x, float alpha, int64_t n);
+/* the same for `count` (1 to 8) pairs in one launch: y[i] += alpha * x[i], n[i] elements each */
+int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, const int64_t* n, int count);
 int boat_cuda_scale(float* y, const float* x, float alpha, int64_t n);
 int boat_cuda_add_bias(float* y, const float* x, const float* bias, int64_t rows, int64_t cols);
 int boat_cuda_mul(float* y, const float* a, const float* b, int64_t n);
