@@ -193,6 +193,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tma_prefetch_desc(&map_v);
         tma_prefetch_desc(&map_do);
         tma_prefetch_desc(&map_dq);
+        griddep_sync();
         // This thread is also the producer: the loads that wait for nothing - K and V of the first
         // walk, dO of the first Q_STAGES query tiles (later ones are loaded by the dQ warps, which
         // stage dQ through the dO buffers and know when one is free again) - start here, under the
@@ -209,6 +210,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
+    griddep_sync();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();

@@ -113,6 +113,7 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         tma_prefetch_desc(&map_do);
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
+    griddep_sync();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -286,6 +287,7 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         tma_prefetch_desc(&map_do_mn);
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
+    griddep_sync();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();

@@ -185,6 +185,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tma_prefetch_desc(&map_q);
         tma_prefetch_desc(&map_k);
         tma_prefetch_desc(&map_v);
+        griddep_sync();
         // This thread is also the producer: the loads that wait for nothing - both query tiles and the
         // first ring-full of key and value tiles - start here, under the tensor-memory allocation
         // and the CTA's first barrier.
@@ -203,6 +204,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
+    griddep_sync();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();

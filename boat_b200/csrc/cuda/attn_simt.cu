@@ -197,6 +197,7 @@ attn_fwd_simt_kernel(int units, int S, int hs, int causal, float scale, int vec,
         load_rows<HS>(b + C::FLOATS, V + base, j * kRows, S, hs, vec);
         commit();
     };
+    griddep_sync();
     load_rows<HS>(q_s, Q + base, q0, S, hs, vec);
     fetch(0);
     float o[4][C::CPT], m[4], l[4];
@@ -297,6 +298,7 @@ __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile
         commit();
         if (KEYS) load_stats(j * kRows, j & 1);
     };
+    griddep_sync();
     load_rows<HS>(own0, (KEYS ? a.K : a.Q) + base, r0, S, hs, a.vec);
     load_rows<HS>(own1, (KEYS ? a.V : a.dO) + base, r0, S, hs, a.vec);
     if (!KEYS) load_stats(r0, 0);
@@ -373,7 +375,7 @@ int launch_fwd(int64_t units, int64_t S, int hs, int causal, float scale, const 
     }
     const void* in[3] = {Q, K, V};
     const unsigned grid = (unsigned)(units * ceil_div(S, kRows));
-    kern<<<grid, kThreads, Tiles<HS>::FWD_SMEM, stream()>>>((int)units, (int)S, hs, causal, scale, rows_aligned(in, 3, hs, sizeof(T)),
+    BOATCU_RUN(kern, grid, kThreads, Tiles<HS>::FWD_SMEM, (int)units, (int)S, hs, causal, scale, rows_aligned(in, 3, hs, sizeof(T)),
                                                              (const T*)Q, (const T*)K, (const T*)V, (T*)O, lse);
     BOATCU_LAUNCH_OK("attn_fwd_simt");
     return 0;
@@ -396,7 +398,7 @@ int launch_bwd(int64_t units, int64_t S, int hs, int causal, float scale, const 
     a.units = (int)units; a.S = (int)S; a.hs = hs; a.causal = causal;
     a.vec = rows_aligned(in, 4, hs, sizeof(T));
     a.scale = scale;
-    kern<<<(unsigned)(2 * units * ceil_div(S, kRows)), kThreads, Tiles<HS>::BWD_SMEM, stream()>>>(a);
+    BOATCU_RUN(kern, (unsigned)(2 * units * ceil_div(S, kRows)), kThreads, Tiles<HS>::BWD_SMEM, a);
     BOATCU_LAUNCH_OK("attn_bwd_simt");
     return 0;
 }

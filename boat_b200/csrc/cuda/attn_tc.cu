@@ -47,7 +47,7 @@ int launch_fwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     }
     const int64_t grid = units * ((ceil_div(S, kTile) + 1) / 2);      // one CTA per pair of query tiles
     ProfileScope prof("attn_fwd_tc");
-    kern<<<(unsigned)grid, kFwdThreads, C::SMEM, stream()>>>(mq, mk, mv, p);
+    BOATCU_RUN(kern, (unsigned)grid, kFwdThreads, C::SMEM, mq, mk, mv, p);
     BOATCU_LAUNCH_OK("attn_fwd_tc");
     return 0;
 }
@@ -130,7 +130,7 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
         ProfileScope prof("attn_bwd_tc");
         BOATCU_CHECK(cudaMemsetAsync(dq_accum, 0, n * sizeof(float), stream()));
         const int64_t grid = units * (p.pair ? (n_tiles + 1) / 2 : n_tiles);
-        kern<<<(unsigned)grid, kBwdThreads, C::SMEM, stream()>>>(mq, mk, mv, mdo, mdq, p);
+        BOATCU_RUN(kern, (unsigned)grid, kBwdThreads, C::SMEM, mq, mk, mv, mdo, mdq, p);
         BOATCU_LAUNCH_OK("attn_bwd_tc");
         // the summed FP32 contributions become the BF16 output
         if (int rc = boat_cuda_cast(dQ, BOAT_CUDA_BF16, dq_accum, BOAT_CUDA_F32, (int64_t)n)) return rc;
@@ -173,9 +173,9 @@ int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const voi
     }
     const unsigned grid = (unsigned)(units * ceil_div(S, kTile));
     ProfileScope prof("attn_bwd_tc");
-    attn_bwd_dkv_tf32_kernel<<<grid, kBwd32Threads, C::SMEM_DKV, stream()>>>(mq, mq_mn, mk, mv, mdo, mdo_mn, p);
+    BOATCU_RUN(attn_bwd_dkv_tf32_kernel, grid, kBwd32Threads, C::SMEM_DKV, mq, mq_mn, mk, mv, mdo, mdo_mn, p);
     BOATCU_LAUNCH_OK("attn_bwd_dkv_tf32");
-    attn_bwd_dq_tf32_kernel<<<grid, kBwd32Threads, C::SMEM_DQ, stream()>>>(mq, mk, mk_mn, mv, mdo, p);
+    BOATCU_RUN(attn_bwd_dq_tf32_kernel, grid, kBwd32Threads, C::SMEM_DQ, mq, mk, mk_mn, mv, mdo, p);
     BOATCU_LAUNCH_OK("attn_bwd_dq_tf32");
     return 0;
 }

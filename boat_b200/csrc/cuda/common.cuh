@@ -45,6 +45,38 @@ struct ProfileScope {
         boatcu::count_launch();                                                     \
     } while (0)
 
+// Kernels of the library follow one another on one stream, and a launch that only begins when its
+// predecessor has drained costs 2-4 us of idle GPU - as much as a small kernel.  So every kernel is
+// launched as the programmatic dependent of the one before: its CTAs may be placed as soon as all CTAs
+// of the predecessor are running, do what depends on nobody (barriers, tensor memory, descriptors), and
+// wait in griddep_sync() until the predecessor is complete and its writes are visible.  EVERY kernel
+// calls it before its first access to global memory, in every thread: completion of a kernel then
+// implies completion of all kernels before it.
+__device__ __forceinline__ void griddep_sync() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream();
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+#define BOATCU_RUN(kern, grid, block, smem, ...) \
+    BOATCU_CHECK(boatcu::launch_dependent(kern, dim3(grid), dim3(block), smem, 1, __VA_ARGS__))
+
 __device__ __forceinline__ float to_f32(float v) { return v; }
 __device__ __forceinline__ float to_f32(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <typename T> __device__ __forceinline__ T from_f32(float v);

@@ -30,6 +30,7 @@ __device__ __forceinline__ float mul_add(float alpha, float x, float y) { return
 // ---- y = alpha*x (+ y), 4 floats per access -------------------------------------------
 template <bool ACCUM>
 __global__ void axpy_vec4(float* __restrict__ y, const float* __restrict__ x, float alpha, int64_t n4) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     float4* y4 = reinterpret_cast<float4*>(y);
@@ -49,6 +50,7 @@ __global__ void axpy_vec4(float* __restrict__ y, const float* __restrict__ x, fl
 
 template <bool ACCUM>
 __global__ void axpy_scalar(float* __restrict__ y, const float* __restrict__ x, float alpha, int64_t n) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (; i < n; i += step) y[i] = ACCUM ? mul_add(alpha, x[i], y[i]) : alpha * x[i];
@@ -59,9 +61,9 @@ static int launch_axpy(float* y, const float* x, float alpha, int64_t n) {
     if (n <= 0) return 0;
     if (int rc = ensure_init()) return rc;
     if (aligned16(y) && aligned16(x) && (n % 4) == 0) {
-        axpy_vec4<ACCUM><<<grid_for(n / 4, kThreads), kThreads, 0, stream()>>>(y, x, alpha, n / 4);
+        BOATCU_RUN(axpy_vec4<ACCUM>, grid_for(n / 4, kThreads), kThreads, 0, y, x, alpha, n / 4);
     } else {
-        axpy_scalar<ACCUM><<<grid_for(n, kThreads), kThreads, 0, stream()>>>(y, x, alpha, n);
+        BOATCU_RUN(axpy_scalar<ACCUM>, grid_for(n, kThreads), kThreads, 0, y, x, alpha, n);
     }
     BOATCU_LAUNCH_OK("axpy");
     return 0;
@@ -75,6 +77,7 @@ struct AxpyTable {
     int64_t n[kMaxAxpy];
 };
 __global__ void axpy_multi_kernel(const AxpyTable t, float alpha, int vec) {
+    griddep_sync();
     float* __restrict__ y = t.y[blockIdx.y];
     const float* __restrict__ x = t.x[blockIdx.y];
     const int64_t n = t.n[blockIdx.y], n4 = vec ? n / 4 : 0;
@@ -90,6 +93,7 @@ __global__ void axpy_multi_kernel(const AxpyTable t, float alpha, int vec) {
 // ---- y = a * b -------------------------------------------------------------------------------
 __global__ void mul_kernel(float* __restrict__ y, const float* __restrict__ a, const float* __restrict__ b,
                            int64_t n, int vec) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {
@@ -107,6 +111,7 @@ __global__ void mul_kernel(float* __restrict__ y, const float* __restrict__ a, c
 // ---- y[i,j] = x[i,j] + bias[j] ---------------------------------------------------------------
 __global__ void add_bias_kernel(float* __restrict__ y, const float* __restrict__ x,
                                 const float* __restrict__ bias, int64_t rows, int64_t cols, int vec) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {
@@ -126,6 +131,7 @@ __global__ void add_bias_kernel(float* __restrict__ y, const float* __restrict__
 template <typename T>
 __global__ void lincomb_kernel(T* __restrict__ y, const T* __restrict__ a, float alpha, const T* __restrict__ b,
                                float beta, int64_t n, int vec) {
+    griddep_sync();
     constexpr int V = 16 / sizeof(T);
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -147,6 +153,7 @@ __global__ void lincomb_kernel(T* __restrict__ y, const T* __restrict__ a, float
 
 // ---- casts -----------------------------------------------------------------------------------
 __global__ void cast_f32_to_bf16(__nv_bfloat16* __restrict__ dst, const float* __restrict__ src, int64_t n, int vec) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {   // 8 elements: two 128-bit loads, one 128-bit store
@@ -167,6 +174,7 @@ __global__ void cast_f32_to_bf16(__nv_bfloat16* __restrict__ dst, const float* _
 }
 
 __global__ void cast_bf16_to_f32(float* __restrict__ dst, const __nv_bfloat16* __restrict__ src, int64_t n, int vec) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {
@@ -196,6 +204,7 @@ __device__ __forceinline__ float round_tf32(float x) {
 }
 
 __global__ void round_tf32_kernel(float* __restrict__ y, const float* __restrict__ x, int64_t n, int vec) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {
@@ -220,6 +229,7 @@ struct ConvertTable {
 // blockIdx.y = tensor; vec: every tensor is 16-byte aligned with a multiple of 8 elements
 template <bool TO_BF16>
 __global__ void convert_multi_kernel(const ConvertTable t, int vec) {
+    griddep_sync();
     const float* __restrict__ src = t.src[blockIdx.y];
     const int64_t n = t.n[blockIdx.y];
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -262,6 +272,7 @@ struct ColsumTable {
 
 template <typename T, int VEC>
 __global__ void colsum_kernel(const ColsumTable t, int64_t rows, int64_t cols) {
+    griddep_sync();
     const T* __restrict__ X = (const T*)t.x[blockIdx.z];
     float* __restrict__ out = t.out[blockIdx.z];
     __shared__ float part[8][32 * VEC + 1];
@@ -331,6 +342,7 @@ __device__ __forceinline__ int64_t source_row(const RowStats& st, int64_t row) {
 template <typename T>
 __global__ void rowdot_kernel(const T* __restrict__ A, const T* __restrict__ B, int64_t rows, int cols,
                               float* __restrict__ out, const RowStats st) {
+    griddep_sync();
     const int lane = threadIdx.x & 31;
     int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -350,6 +362,7 @@ __global__ void rowdot_kernel(const T* __restrict__ A, const T* __restrict__ B, 
 template <typename T, int VEC>
 __global__ void rowdot_vec_kernel(const T* __restrict__ A, const T* __restrict__ B, int64_t rows, int cols,
                                   float* __restrict__ out, const RowStats st) {
+    griddep_sync();
     const int lanes_per_row = cols / VEC;            // power of two <= 32 checked by the launcher
     const int rows_per_warp = 32 / lanes_per_row;
     const int lane = threadIdx.x & 31;
@@ -393,17 +406,17 @@ static int rowdot_launch(const void* A, const void* B, int type, int64_t rows, i
         int rows_per_block = (kThreads / 32) * (int)(32 / lpr);
         int grid = grid_for(rows, rows_per_block);
         if (type == BOAT_CUDA_BF16)
-            rowdot_vec_kernel<__nv_bfloat16, 8><<<grid, kThreads, 0, stream()>>>(
+            BOATCU_RUN((rowdot_vec_kernel<__nv_bfloat16, 8>), grid, kThreads, 0, 
                 (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, rows, (int)cols, out, st);
         else
-            rowdot_vec_kernel<float, 4><<<grid, kThreads, 0, stream()>>>((const float*)A, (const float*)B, rows, (int)cols, out, st);
+            BOATCU_RUN((rowdot_vec_kernel<float, 4>), grid, kThreads, 0, (const float*)A, (const float*)B, rows, (int)cols, out, st);
     } else {
         int grid = grid_for(rows, kThreads / 32);
         if (type == BOAT_CUDA_BF16)
-            rowdot_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream()>>>(
+            BOATCU_RUN(rowdot_kernel<__nv_bfloat16>, grid, kThreads, 0, 
                 (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, rows, (int)cols, out, st);
         else
-            rowdot_kernel<float><<<grid, kThreads, 0, stream()>>>((const float*)A, (const float*)B, rows, (int)cols, out, st);
+            BOATCU_RUN(rowdot_kernel<float>, grid, kThreads, 0, (const float*)A, (const float*)B, rows, (int)cols, out, st);
     }
     BOATCU_LAUNCH_OK("rowdot");
     return 0;
@@ -420,6 +433,7 @@ int rowdot_stats(const void* dO, const void* O, int type, int64_t units, int64_t
 
 // ---- out[b, j, i] = in[b, i, j], 32x32 shared-memory tiles --------------------------------------
 __global__ void transpose_kernel(float* __restrict__ out, const float* __restrict__ in, int64_t rows, int64_t cols) {
+    griddep_sync();
     __shared__ float tile[32][33];
     const float* src = in + (int64_t)blockIdx.z * rows * cols;
     float* dst = out + (int64_t)blockIdx.z * rows * cols;
@@ -462,7 +476,7 @@ int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, co
         if (n[s] > longest) longest = n[s];
     }
     if (longest <= 0) return 0;
-    axpy_multi_kernel<<<dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, stream()>>>(t, alpha, vec);
+    BOATCU_RUN(axpy_multi_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, alpha, vec);
     BOATCU_LAUNCH_OK("axpy_multi");
     return 0;
 }
@@ -471,7 +485,7 @@ int boat_cuda_mul(float* y, const float* a, const float* b, int64_t n) {
     if (n <= 0) return 0;
     if (int rc = ensure_init()) return rc;
     int vec = aligned16(y) && aligned16(a) && aligned16(b) && (n % 4) == 0;
-    mul_kernel<<<grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, stream()>>>(y, a, b, n, vec);
+    BOATCU_RUN(mul_kernel, grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, y, a, b, n, vec);
     BOATCU_LAUNCH_OK("mul");
     return 0;
 }
@@ -481,7 +495,7 @@ int boat_cuda_add_bias(float* y, const float* x, const float* bias, int64_t rows
     if (int rc = ensure_init()) return rc;
     int vec = aligned16(y) && aligned16(x) && aligned16(bias) && (cols % 4) == 0;
     int64_t n = rows * cols;
-    add_bias_kernel<<<grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, stream()>>>(y, x, bias, rows, cols, vec);
+    BOATCU_RUN(add_bias_kernel, grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, y, x, bias, rows, cols, vec);
     BOATCU_LAUNCH_OK("add_bias");
     return 0;
 }
@@ -494,9 +508,9 @@ int boat_cuda_cast(void* dst, int dst_type, const void* src, int src_type, int64
     int grid = grid_for(vec ? n / 8 : n, kThreads);
     ProfileScope prof("cast");
     if (dst_type == BOAT_CUDA_BF16)
-        cast_f32_to_bf16<<<grid, kThreads, 0, stream()>>>((__nv_bfloat16*)dst, (const float*)src, n, vec);
+        BOATCU_RUN(cast_f32_to_bf16, grid, kThreads, 0, (__nv_bfloat16*)dst, (const float*)src, n, vec);
     else
-        cast_bf16_to_f32<<<grid, kThreads, 0, stream()>>>((float*)dst, (const __nv_bfloat16*)src, n, vec);
+        BOATCU_RUN(cast_bf16_to_f32, grid, kThreads, 0, (float*)dst, (const __nv_bfloat16*)src, n, vec);
     BOATCU_LAUNCH_OK("cast");
     return 0;
 }
@@ -509,10 +523,10 @@ int boat_cuda_lincomb(void* y, const void* a, float alpha, const void* b, float 
     int grid = grid_for(vec ? n / V : n, kThreads);
     ProfileScope prof("lincomb");
     if (type == BOAT_CUDA_BF16)
-        lincomb_kernel<__nv_bfloat16><<<grid, kThreads, 0, stream()>>>((__nv_bfloat16*)y, (const __nv_bfloat16*)a, alpha,
+        BOATCU_RUN(lincomb_kernel<__nv_bfloat16>, grid, kThreads, 0, (__nv_bfloat16*)y, (const __nv_bfloat16*)a, alpha,
                                                                        (const __nv_bfloat16*)b, beta, n, vec);
     else
-        lincomb_kernel<float><<<grid, kThreads, 0, stream()>>>((float*)y, (const float*)a, alpha, (const float*)b, beta, n, vec);
+        BOATCU_RUN(lincomb_kernel<float>, grid, kThreads, 0, (float*)y, (const float*)a, alpha, (const float*)b, beta, n, vec);
     BOATCU_LAUNCH_OK("lincomb");
     return 0;
 }
@@ -522,7 +536,7 @@ int boat_cuda_round_tf32(float* y, const float* x, int64_t n) {
     if (int rc = ensure_init()) return rc;
     int vec = aligned16(y) && aligned16(x) && (n % 4) == 0;
     ProfileScope prof("round_tf32");
-    round_tf32_kernel<<<grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, stream()>>>(y, x, n, vec);
+    BOATCU_RUN(round_tf32_kernel, grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, y, x, n, vec);
     BOATCU_LAUNCH_OK("round_tf32");
     return 0;
 }
@@ -554,11 +568,11 @@ int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64
     grid.y = (unsigned)(want < 1 ? 1 : (want > max_y ? max_y : want));
     if (grid.y > 65535) grid.y = 65535;
     if (x_type == BOAT_CUDA_BF16) {
-        if (can_vec) colsum_kernel<__nv_bfloat16, 8><<<grid, kThreads, 0, stream()>>>(t, rows, cols);
-        else         colsum_kernel<__nv_bfloat16, 1><<<grid, kThreads, 0, stream()>>>(t, rows, cols);
+        if (can_vec) BOATCU_RUN((colsum_kernel<__nv_bfloat16, 8>), grid, kThreads, 0, t, rows, cols);
+        else         BOATCU_RUN((colsum_kernel<__nv_bfloat16, 1>), grid, kThreads, 0, t, rows, cols);
     } else {
-        if (can_vec) colsum_kernel<float, 4><<<grid, kThreads, 0, stream()>>>(t, rows, cols);
-        else         colsum_kernel<float, 1><<<grid, kThreads, 0, stream()>>>(t, rows, cols);
+        if (can_vec) BOATCU_RUN((colsum_kernel<float, 4>), grid, kThreads, 0, t, rows, cols);
+        else         BOATCU_RUN((colsum_kernel<float, 1>), grid, kThreads, 0, t, rows, cols);
     }
     BOATCU_LAUNCH_OK("colsum");
     return 0;
@@ -595,8 +609,8 @@ int boat_cuda_convert_multi(void* const* dst, int dst_type, const float* const* 
     if (per_tensor > cap) per_tensor = cap;
     dim3 grid((unsigned)per_tensor, (unsigned)count, 1);
     ProfileScope prof("cast");
-    if (dst_type == BOAT_CUDA_BF16) convert_multi_kernel<true><<<grid, kThreads, 0, stream()>>>(t, vec);
-    else                            convert_multi_kernel<false><<<grid, kThreads, 0, stream()>>>(t, vec);
+    if (dst_type == BOAT_CUDA_BF16) BOATCU_RUN(convert_multi_kernel<true>, grid, kThreads, 0, t, vec);
+    else                            BOATCU_RUN(convert_multi_kernel<false>, grid, kThreads, 0, t, vec);
     BOATCU_LAUNCH_OK("convert_multi");
     return 0;
 }
@@ -606,7 +620,7 @@ int boat_cuda_transpose(float* out, const float* in, int64_t batch, int64_t rows
     if (int rc = ensure_init()) return rc;
     if (batch > 65535) return set_error(6, "boat_cuda_transpose: batch %lld exceeds 65535", (long long)batch);
     dim3 grid((unsigned)ceil_div(cols, 32), (unsigned)ceil_div(rows, 32), (unsigned)batch);
-    transpose_kernel<<<grid, dim3(32, 8, 1), 0, stream()>>>(out, in, rows, cols);
+    BOATCU_RUN(transpose_kernel, grid, dim3(32, 8, 1), 0, out, in, rows, cols);
     BOATCU_LAUNCH_OK("transpose");
     return 0;
 }

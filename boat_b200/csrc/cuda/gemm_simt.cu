@@ -130,6 +130,7 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     auto col = [&](int j) { return B_K ? tx + 16 * j : (j / VN) * 16 * VN + tx * VN + j % VN; };
     auto row = [&](int i) { return (i / VM) * 16 * VM + ty * VM + i % VM; };
 
+    griddep_sync();
     fetch(s0);
     fetch(s0 + 1);
     for (int s = s0; s < s1; ++s) {
@@ -284,18 +285,7 @@ int launch_tile(SimtParams& p, int groups, int split) {
     if (tiles * split > 0x7fffffffLL) return set_error(7, "gemm_simt: %lld x %lld outputs are too many for one launch", (long long)p.M, (long long)p.N);
     p.n_tiles = (int)ceil_div(p.N, S::BN);
     p.split = split;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(tiles * split), 1, (unsigned)groups);
-    cfg.blockDim = dim3(256, 1, 1);
-    cfg.dynamicSmemBytes = S::SMEM;
-    cfg.stream = stream();
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)split;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    BOATCU_CHECK(cudaLaunchKernelEx(&cfg, kern, (const SimtParams)p));
+    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), S::SMEM, (unsigned)split, p));
     BOATCU_LAUNCH_OK("gemm_simt");
     return 0;
 }

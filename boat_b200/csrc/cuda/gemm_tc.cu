@@ -103,6 +103,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         }
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
+    griddep_sync();
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
@@ -309,7 +310,7 @@ int launch(int groups, int64_t M, int64_t N, int64_t K, const void* const* A, in
     // stream has priority) get placed while the GEMM runs, not after it.
     const int grid = (g_yielding || work < sm_count()) ? work : sm_count();
     ProfileScope prof(A_MN ? "gemm_tc_tn" : (B_MN ? "gemm_tc_nn" : "gemm_tc_nt"));
-    kern<<<grid, kThreads, C::SMEM, stream()>>>(maps, p);
+    BOATCU_RUN(kern, grid, kThreads, C::SMEM, maps, p);
     BOATCU_LAUNCH_OK("gemm_tc");
     return 0;
 }

@@ -76,6 +76,7 @@ template <typename T>
 __global__ void __launch_bounds__(kNormThreads)
 layernorm_fwd_kernel(const T* __restrict__ x, int cols, const float* __restrict__ gamma, const float* __restrict__ beta,
                      float eps, T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out) {
+    griddep_sync();
     extern __shared__ float row[];          // [cols] + 32
     float* red = row + cols;
     const int64_t r = blockIdx.x;
@@ -110,6 +111,7 @@ template <typename T>
 __global__ void __launch_bounds__(kNormThreads)
 layernorm_bwd_dx_kernel(const T* __restrict__ dy, const T* __restrict__ x, int cols, const float* __restrict__ gamma,
                         const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx) {
+    griddep_sync();
     extern __shared__ float smem[];         // g[cols], xhat[cols], 32
     float* g = smem;
     float* xh = smem + cols;
@@ -194,6 +196,7 @@ __global__ void __launch_bounds__(kNormThreads)
 layernorm_fwd_warp_kernel(const T* __restrict__ x, int64_t rows, const float* __restrict__ gamma,
                           const float* __restrict__ beta, float eps, T* __restrict__ y, float* __restrict__ mean_out,
                           float* __restrict__ rstd_out) {
+    griddep_sync();
     constexpr int V = Vec16<T>::N, COLS = NV * 32 * V;
     const int lane = threadIdx.x & 31;
     const int64_t r0 = ((int64_t)blockIdx.x * (kNormThreads / 32) + (threadIdx.x >> 5)) * kNormRowsPerWarp;
@@ -256,6 +259,7 @@ layernorm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, int
                           const float* __restrict__ gamma, const float* __restrict__ mean,
                           const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dgamma,
                           float* __restrict__ dbeta) {
+    griddep_sync();
     constexpr int V = Vec16<T>::N, COLS = NV * 32 * V;
     extern __shared__ float part[];                 // [2][COLS] when parameter gradients are wanted
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -329,6 +333,7 @@ template <typename T>
 __global__ void layernorm_bwd_params_kernel(const T* __restrict__ dy, const T* __restrict__ x, int64_t rows, int cols,
                                             const float* __restrict__ mean, const float* __restrict__ rstd,
                                             float* __restrict__ dgamma, float* __restrict__ dbeta) {
+    griddep_sync();
     __shared__ float pg[8][33], pb[8][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int col = blockIdx.x * 32 + tx;
@@ -388,6 +393,7 @@ __device__ __forceinline__ float gelu_grad_f(float x) {
 
 template <typename T, bool BWD>
 __global__ void gelu_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ dy, int64_t n) {
+    griddep_sync();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (; i < n; i += step) {
@@ -403,6 +409,7 @@ constexpr int kGeluUnroll = 4;
 template <typename T, bool BWD>
 __global__ void __launch_bounds__(256)
 gelu_vec_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ dy, int64_t nvec) {
+    griddep_sync();
     constexpr int V = 16 / sizeof(T);
     const int64_t chunk = (int64_t)gridDim.x * 256 * kGeluUnroll;
     for (int64_t base = (int64_t)blockIdx.x * 256 * kGeluUnroll + threadIdx.x; base < nvec; base += chunk) {
@@ -444,9 +451,9 @@ static int launch_gelu(void* out, const void* x, const void* dy, int64_t n) {
     if (blocks > 0x7fffffffLL) blocks = 0x7fffffffLL;
     ProfileScope prof(BWD ? "gelu_bwd" : "gelu_fwd");
     if (vec)
-        gelu_vec_kernel<T, BWD><<<(unsigned)blocks, 256, 0, stream()>>>((T*)out, (const T*)x, (const T*)dy, items);
+        BOATCU_RUN((gelu_vec_kernel<T, BWD>), (unsigned)blocks, 256, 0, (T*)out, (const T*)x, (const T*)dy, items);
     else
-        gelu_kernel<T, BWD><<<(unsigned)blocks, 256, 0, stream()>>>((T*)out, (const T*)x, (const T*)dy, n);
+        BOATCU_RUN((gelu_kernel<T, BWD>), (unsigned)blocks, 256, 0, (T*)out, (const T*)x, (const T*)dy, n);
     BOATCU_LAUNCH_OK("gelu");
     return 0;
 }
@@ -457,7 +464,7 @@ template <typename T, int NV>
 static int fwd_warp_launch(const void* x, int64_t rows, const float* gamma, const float* beta, float eps, void* y,
                            float* mean_out, float* rstd_out) {
     const int64_t blocks = ceil_div(rows, (kNormThreads / 32) * kNormRowsPerWarp);
-    layernorm_fwd_warp_kernel<T, NV><<<(unsigned)blocks, kNormThreads, 0, stream()>>>((const T*)x, rows, gamma, beta, eps,
+    BOATCU_RUN((layernorm_fwd_warp_kernel<T, NV>), (unsigned)blocks, kNormThreads, 0, (const T*)x, rows, gamma, beta, eps,
                                                                                        (T*)y, mean_out, rstd_out);
     BOATCU_LAUNCH_OK("layernorm_fwd_warp");
     return -1;
@@ -470,7 +477,7 @@ static int bwd_warp_launch(const void* dy, const void* x, int64_t rows, const fl
     int64_t blocks = ceil_div(rows, kNormThreads / 32);
     if (blocks > sm_count() * 4) blocks = sm_count() * 4;         // persistent: the column sums live in registers across rows
     const size_t smem = (dgamma || dbeta) ? 2 * COLS * sizeof(float) : 0;
-    layernorm_bwd_warp_kernel<T, NV><<<(unsigned)blocks, kNormThreads, smem, stream()>>>(
+    BOATCU_RUN((layernorm_bwd_warp_kernel<T, NV>), (unsigned)blocks, kNormThreads, smem, 
         (const T*)dy, (const T*)x, rows, gamma, mean, rstd, (T*)dx, dgamma, dbeta);
     BOATCU_LAUNCH_OK("layernorm_bwd_warp");
     return -1;
@@ -528,12 +535,12 @@ int boat_cuda_layernorm_fwd(const void* x, int type, int64_t rows, int64_t cols,
     if (type == BOAT_CUDA_BF16) {
         auto k = layernorm_fwd_kernel<__nv_bfloat16>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<(unsigned)rows, kNormThreads, smem, stream()>>>((const __nv_bfloat16*)x, (int)cols, gamma, beta, eps,
+        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const __nv_bfloat16*)x, (int)cols, gamma, beta, eps,
                                                             (__nv_bfloat16*)y, mean_out, rstd_out);
     } else {
         auto k = layernorm_fwd_kernel<float>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<(unsigned)rows, kNormThreads, smem, stream()>>>((const float*)x, (int)cols, gamma, beta, eps, (float*)y,
+        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const float*)x, (int)cols, gamma, beta, eps, (float*)y,
                                                             mean_out, rstd_out);
     }
     BOATCU_LAUNCH_OK("layernorm_fwd");
@@ -557,19 +564,19 @@ int boat_cuda_layernorm_bwd(const void* dy, const void* x, int type, int64_t row
         typedef __nv_bfloat16 bf;
         auto k = layernorm_bwd_dx_kernel<bf>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<(unsigned)rows, kNormThreads, smem, stream()>>>((const bf*)dy, (const bf*)x, (int)cols, gamma, mean, rstd, (bf*)dx);
+        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const bf*)dy, (const bf*)x, (int)cols, gamma, mean, rstd, (bf*)dx);
         BOATCU_LAUNCH_OK("layernorm_bwd_dx");
         if (dgamma || dbeta) {
-            layernorm_bwd_params_kernel<bf><<<pgrid, 256, 0, stream()>>>((const bf*)dy, (const bf*)x, rows, (int)cols, mean, rstd, dgamma, dbeta);
+            BOATCU_RUN(layernorm_bwd_params_kernel<bf>, pgrid, 256, 0, (const bf*)dy, (const bf*)x, rows, (int)cols, mean, rstd, dgamma, dbeta);
             BOATCU_LAUNCH_OK("layernorm_bwd_params");
         }
     } else {
         auto k = layernorm_bwd_dx_kernel<float>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k<<<(unsigned)rows, kNormThreads, smem, stream()>>>((const float*)dy, (const float*)x, (int)cols, gamma, mean, rstd, (float*)dx);
+        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const float*)dy, (const float*)x, (int)cols, gamma, mean, rstd, (float*)dx);
         BOATCU_LAUNCH_OK("layernorm_bwd_dx");
         if (dgamma || dbeta) {
-            layernorm_bwd_params_kernel<float><<<pgrid, 256, 0, stream()>>>((const float*)dy, (const float*)x, rows, (int)cols, mean, rstd, dgamma, dbeta);
+            BOATCU_RUN(layernorm_bwd_params_kernel<float>, pgrid, 256, 0, (const float*)dy, (const float*)x, rows, (int)cols, mean, rstd, dgamma, dbeta);
             BOATCU_LAUNCH_OK("layernorm_bwd_params");
         }
     }

@@ -50,6 +50,7 @@ __device__ __forceinline__ void adam_one(float& p, float g, float& m, float& v, 
 
 __global__ void __launch_bounds__(kAdamThreads) adam_multi_kernel(const __grid_constant__ AdamTable tab,
                                                                   const AdamConst c, int total_chunks) {
+    griddep_sync();
     for (int chunk = blockIdx.x; chunk < total_chunks; chunk += gridDim.x) {
         // which tensor owns this chunk (the table is short: linear scan, uniform per CTA)
         int t = 0;
@@ -130,7 +131,7 @@ extern "C" int boat_cuda_adam_step(int count, float* const* params, const float*
             ++done;
         }
         if (tab.count == 0) continue;
-        adam_multi_kernel<<<(int)chunks, kAdamThreads, 0, stream()>>>(tab, c, (int)chunks);
+        BOATCU_RUN(adam_multi_kernel, (int)chunks, kAdamThreads, 0, tab, c, (int)chunks);
         BOATCU_LAUNCH_OK("adam_multi_kernel");
     }
     return 0;
