@@ -13,13 +13,27 @@
 //   dX = dY . W^T   A = dY [M,K] K-major      B = W  [N,K] K-major
 //   dW = X^T . dY   A = X  [K,M] M-major      B = dY [K,N] N-major
 //
-// Kernel shape: persistent, one 192-thread CTA per SM.  Warp 0 feeds a 4-stage shared-memory
-// ring with TMA (128-byte swizzle, no multicast); one thread of warp 1 issues tcgen05.mma
-// 128 x BN x (32 bytes of K) and commits stages back to the producer; warps 2-5 drain the
-// accumulator from tensor memory (tcgen05.ld), add the bias, convert and store.  The
-// accumulator is double-buffered in tensor memory (2 x BN columns) so that the epilogue of one
-// tile overlaps the main loop of the next.  Weight gradients have few output tiles and a
-// very long K: they are split along K over several CTAs that add into a zeroed output.
+// Kernel shape: persistent, 192-thread CTAs, alone or as pairs on one tile (CTAS).  Warp 0 feeds a
+// shared-memory ring with TMA (128-byte swizzle, no multicast); one thread of warp 1 issues
+// tcgen05.mma and commits stages back to the producer; warps 2-5 drain the accumulator from tensor
+// memory.  The accumulator is double-buffered in tensor memory (2 x BN columns) so that the epilogue
+// of one tile overlaps the main loop of the next.
+//
+// CTA pairs (cta_group::2, 256 x BN tiles): each CTA holds its 128 rows of A and half of B; the tensor
+// cores of both SMs read both halves of B.  A CTA then brings in and reads 32 KB per 64 of K instead of 48 -
+// a single CTA's 128 x 256 tile keeps the SM's shared-memory port 75 % busy with operands alone.  All
+// loads of a pair count on a barrier of the first CTA, whose thread issues the MMAs; its commits
+// arrive at both CTAs.
+//
+// Epilogue: a warp owns 32 rows of the tile.  It reads 64 BF16 (32 FP32) columns from tensor memory,
+// converts them, writes them as 128-byte rows to a swizzled staging box of its own and stores the box
+// with TMA.  (Storing from registers, where a lane holds a row, gave every 16-byte store a 32-byte
+// sector of its own: 786 TFLOP/s at 32768 x 4096 x 1024.)  The same boxes serve as
+// reductions (cp.reduce .add) for split K and for accumulation into the output.
+//
+// FP32 results (weight gradients) have few tiles and a long K.  Whole waves of tiles are done by one CTA
+// (pair) each; the tiles left over, which would keep most SMs idle for one more wave, are split along K
+// into pieces that add into a zeroed output.
 //
 // Up to kMaxGroups problems of one shape and layout (the Q, K and V projections of a layer, their
 // weight gradients, their input gradients) run as one launch: the persistent CTAs walk the tiles of
@@ -33,59 +47,92 @@ using namespace tc;
 
 namespace {
 
-constexpr int BM = 128;
-constexpr int STAGES = 4;
+constexpr int BM = 128;                          // rows of C per CTA
 constexpr int kThreads = 192;
+constexpr int kMaxGroups = 4;
+constexpr int kBoxRows = 32;                     // rows of a staging box: one epilogue warp's rows
+constexpr int kStageBox = kBoxRows * 128;        // 32 rows x 128 bytes
+constexpr int kOutBoxes = 2;                     // boxes in flight per epilogue warp
 
-template <typename T, int BN>
+template <typename T, int CTAS, int BN>
 struct Cfg {
     static constexpr int ES = sizeof(T);
     static constexpr int BK = 128 / ES;             // one 128-byte swizzle row of K (or of M/N)
     static constexpr int UK = 32 / ES;              // K extent of one tcgen05.mma
+    static constexpr int BNC = BN / CTAS;           // rows of B held by one CTA
     static constexpr int A_BYTES = BM * 128;
-    static constexpr int B_BYTES = BN * 128;
+    static constexpr int B_BYTES = BNC * 128;
+    static constexpr int STAGE = A_BYTES + B_BYTES;
     static constexpr int CHUNK_BYTES = BK * 128;    // one [BK rows x 128 B] box of an MN-major operand
-    static constexpr int SMEM = STAGES * (A_BYTES + B_BYTES) + 1024 /*alignment*/ + 256 /*barriers*/;
+    static constexpr int OUT_BYTES = 4 * kOutBoxes * kStageBox;
+    static constexpr int FIT = (232448 - 1024 - 512 - OUT_BYTES) / STAGE;
+    static constexpr int STAGES = FIT < 8 ? FIT : 8;
+    static constexpr int SMEM = STAGES * STAGE + OUT_BYTES + 1024 /*alignment*/ + 512 /*barriers*/;
     static constexpr uint32_t TMEM_COLS = 2 * BN;   // two accumulators
 };
 
-constexpr int kMaxGroups = 4;
-
 struct GroupMaps {
-    CUtensorMap a[kMaxGroups], b[kMaxGroups];
+    CUtensorMap a[kMaxGroups], b[kMaxGroups], c[kMaxGroups];
 };
 
 struct Params {
-    void* C[kMaxGroups];
     const float* bias[kMaxGroups];
     int groups;
-    int64_t ldc;
     int M, N, K;
     int out_type;
-    int split_k;
+    int full;            // tiles done in one piece; the rest is split along K
+    int split;
+    int add_all;         // every tile adds to the output, not only the pieces of split tiles
     unsigned int* status;
 };
 
-template <typename T, bool A_MN, bool B_MN, int BN>
+struct WorkItem {
+    int g, m0, n0, kb0, kb1;
+    bool first, add;     // first piece of its tile (adds the bias); result is added to the output
+};
+
+template <typename T, bool A_MN, bool B_MN, int CTAS, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ Params p) {
-    using C = Cfg<T, BN>;
+    using C = Cfg<T, CTAS, BN>;
     constexpr bool TF32 = sizeof(T) == 4;
+    constexpr int STAGES = C::STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint8_t* a_smem = smem;
     uint8_t* b_smem = smem + STAGES * C::A_BYTES;
-    uint64_t* bars = (uint64_t*)(smem + STAGES * (C::A_BYTES + C::B_BYTES));
-    uint64_t* full = bars;                 // [STAGES] TMA -> MMA
-    uint64_t* empty = bars + STAGES;       // [STAGES] MMA -> TMA
+    uint8_t* out_smem = b_smem + STAGES * C::B_BYTES;
+    uint64_t* bars = (uint64_t*)(out_smem + C::OUT_BYTES);
+    uint64_t* full = bars;                        // [STAGES] TMA -> MMA (of the first CTA of a pair)
+    uint64_t* empty = bars + STAGES;              // [STAGES] MMA -> TMA
     uint64_t* acc_full = bars + 2 * STAGES;       // [2] MMA -> epilogue
-    uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA
+    uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA (of the first CTA of a pair)
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m_tiles = (p.M + BM - 1) / BM, n_tiles = (p.N + BN - 1) / BN;
+    const uint32_t rank = CTAS == 2 ? cluster_rank() : 0;
+    const int worker = blockIdx.x / CTAS, workers = gridDim.x / CTAS;
+    const int m_tiles = (p.M + BM * CTAS - 1) / (BM * CTAS), n_tiles = (p.N + BN - 1) / BN;
     const int k_blocks = (p.K + C::BK - 1) / C::BK;
-    const int work_items = m_tiles * n_tiles * p.groups * p.split_k;      // w = ((tile * groups) + g) * split_k + split
+    const int tiles = m_tiles * n_tiles * p.groups;
+    const int work_items = p.full + (tiles - p.full) * p.split;
+    auto item = [&](int w) {
+        WorkItem it;
+        // pieces of one K range are neighbours: the CTAs at work together share the rows they stream
+        const int rest = tiles - p.full;
+        const int tile = w < p.full ? w : p.full + (w - p.full) % rest;
+        const int part = w < p.full ? 0 : (w - p.full) / rest;
+        const int pieces = w < p.full ? 1 : p.split;
+        const int mn = tile / p.groups;
+        it.g = tile % p.groups;
+        it.m0 = (mn / n_tiles) * BM * CTAS + (int)rank * BM;
+        it.n0 = (mn % n_tiles) * BN;
+        it.kb0 = (int)((int64_t)part * k_blocks / pieces);
+        it.kb1 = (int)((int64_t)(part + 1) * k_blocks / pieces);
+        it.first = part == 0;
+        it.add = pieces > 1 || p.add_all;
+        return it;
+    };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -94,18 +141,23 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 128);
+            mbar_init(&acc_empty[b], 4 * CTAS);
         }
         fence_barrier_init();
         for (int g = 0; g < p.groups; ++g) {
             tma_prefetch_desc(&maps.a[g]);
             tma_prefetch_desc(&maps.b[g]);
+            tma_prefetch_desc(&maps.c[g]);
         }
     }
-    if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
+    if (warp == 1) {
+        if (CTAS == 2) tmem_alloc_pair(tmem_slot, C::TMEM_COLS);
+        else           tmem_alloc(tmem_slot, C::TMEM_COLS);
+    }
     griddep_sync();
     tc_fence_before_sync();
     __syncthreads();
+    if (CTAS == 2) cluster_sync_all();            // the peer's barriers exist before anything arrives there
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -114,32 +166,32 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (int w = blockIdx.x; w < work_items && ok; w += gridDim.x) {
-                const int split = w % p.split_k, gt = w / p.split_k;
-                const int g = gt % p.groups, tile = gt / p.groups;
-                const CUtensorMap* map_a = &maps.a[g];
-                const CUtensorMap* map_b = &maps.b[g];
-                const int m0 = (tile / n_tiles) * BM, n0 = (tile % n_tiles) * BN;
-                const int kb0 = (int)((int64_t)split * k_blocks / p.split_k);
-                const int kb1 = (int)((int64_t)(split + 1) * k_blocks / p.split_k);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
+            for (int w = worker; w < work_items && ok; w += workers) {
+                const WorkItem t = item(w);
+                const CUtensorMap* map_a = &maps.a[t.g];
+                const CUtensorMap* map_b = &maps.b[t.g];
+                const int nb = t.n0 + (int)rank * C::BNC;             // this CTA's rows of B
+                for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
-                    mbar_arrive_expect_tx(&full[s], C::A_BYTES + C::B_BYTES);
+                    if (rank == 0) mbar_arrive_expect_tx(&full[s], CTAS * C::STAGE);
                     const int k0 = kb * C::BK;
                     uint8_t* a_dst = a_smem + s * C::A_BYTES;
                     uint8_t* b_dst = b_smem + s * C::B_BYTES;
+                    const uint32_t bar = CTAS == 2 ? peer_addr(&full[s], 0) : 0;
+                    auto load = [&](uint8_t* dst, const CUtensorMap* map, int x, int y) {
+                        if (CTAS == 2) tma_load_2d_pair(dst, map, bar, x, y);
+                        else           tma_load_2d(dst, map, &full[s], x, y);
+                    };
                     if (A_MN) {
-                        for (int c = 0; c < BM / C::BK; ++c)
-                            tma_load_2d(a_dst + c * C::CHUNK_BYTES, map_a, &full[s], m0 + c * C::BK, k0);
+                        for (int c = 0; c < BM / C::BK; ++c) load(a_dst + c * C::CHUNK_BYTES, map_a, t.m0 + c * C::BK, k0);
                     } else {
-                        tma_load_2d(a_dst, map_a, &full[s], k0, m0);
+                        load(a_dst, map_a, k0, t.m0);
                     }
                     if (B_MN) {
-                        for (int c = 0; c < BN / C::BK; ++c)
-                            tma_load_2d(b_dst + c * C::CHUNK_BYTES, map_b, &full[s], n0 + c * C::BK, k0);
+                        for (int c = 0; c < C::BNC / C::BK; ++c) load(b_dst + c * C::CHUNK_BYTES, map_b, nb + c * C::BK, k0);
                     } else {
-                        tma_load_2d(b_dst, map_b, &full[s], k0, n0);
+                        load(b_dst, map_b, k0, nb);
                     }
                 }
             }
@@ -150,19 +202,17 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = make_idesc(TF32 ? kTF32 : kBF16, A_MN, B_MN, BM, BN);
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = make_idesc(TF32 ? kTF32 : kBF16, A_MN, B_MN, BM * CTAS, BN);
             uint32_t it = 0, acc_it = 0;
             bool ok = true;
-            for (int w = blockIdx.x; w < work_items && ok; w += gridDim.x, ++acc_it) {
-                const int split = w % p.split_k;
-                const int kb0 = (int)((int64_t)split * k_blocks / p.split_k);
-                const int kb1 = (int)((int64_t)(split + 1) * k_blocks / p.split_k);
+            for (int w = worker; w < work_items && ok; w += workers, ++acc_it) {
+                const WorkItem t = item(w);
                 const int buf = acc_it & 1;
                 if (!mbar_wait(&acc_empty[buf], ((acc_it >> 1) & 1) ^ 1, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
                     tc_fence_after_sync();
@@ -174,180 +224,264 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                                                      : smem_desc_sw128(a_addr + kk * 32, 16, 1024);
                         const uint64_t b_desc = B_MN ? smem_desc_mn(b_addr + kk * C::UK * 128, C::CHUNK_BYTES, TF32)
                                                      : smem_desc_sw128(b_addr + kk * 32, 16, 1024);
-                        mma_ss<TF32>(d_tmem, a_desc, b_desc, idesc, kb > kb0 || kk > 0);
+                        if (CTAS == 2) mma_ss_pair<TF32>(d_tmem, a_desc, b_desc, idesc, kb > t.kb0 || kk > 0);
+                        else           mma_ss<TF32>(d_tmem, a_desc, b_desc, idesc, kb > t.kb0 || kk > 0);
                     }
-                    mma_commit(&empty[s]);            // stage reusable once these MMAs have read it
+                    // stage reusable once these MMAs have read it
+                    if (CTAS == 2) mma_commit_pair(&empty[s]);
+                    else           mma_commit(&empty[s]);
                 }
-                if (ok) mma_commit(&acc_full[buf]);   // accumulator complete
+                if (ok) {                             // accumulator complete
+                    if (CTAS == 2) mma_commit_pair(&acc_full[buf]);
+                    else           mma_commit(&acc_full[buf]);
+                }
             }
         }
     } else {
         // ---------------- epilogue: warps 2..5 ----------------
         const int lane_group = warp & 3;              // TMEM lanes this warp may touch
-        uint32_t acc_it = 0;
-        bool ok = true;
-        for (int w = blockIdx.x; w < work_items && ok; w += gridDim.x, ++acc_it) {
-            const int split = w % p.split_k, gt = w / p.split_k;
-            const int g = gt % p.groups, tile = gt / p.groups;
-            const int m0 = (tile / n_tiles) * BM, n0 = (tile % n_tiles) * BN;
-            void* const out = p.C[g];
-            const float* const bias = p.bias[g];
+        uint8_t* boxes = out_smem + lane_group * kOutBoxes * kStageBox;
+        const int swz = lane & 7;
+        const bool bf16_out = p.out_type == BOAT_CUDA_BF16;
+        const int step = bf16_out ? 64 : 32;          // columns per box
+        uint32_t acc_it = 0, box_it = 0;
+        for (int w = worker; w < work_items; w += workers, ++acc_it) {
+            const WorkItem t = item(w);
+            const CUtensorMap* map_c = &maps.c[t.g];
+            const float* const bias = t.first ? p.bias[t.g] : nullptr;
+            const bool bias16 = ((uintptr_t)bias & 15) == 0;
             const int buf = acc_it & 1;
-            if (!mbar_wait(&acc_full[buf], (acc_it >> 1) & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
+            if (!mbar_wait_warp(&acc_full[buf], (acc_it >> 1) & 1, p.status, kTimeoutEpilogue)) break;
             tc_fence_after_sync();
-            const int row = m0 + lane_group * 32 + lane;
+            const int row0 = t.m0 + lane_group * 32;
             const uint32_t t_addr = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * BN;
-            const bool add_bias = bias != nullptr && split == 0;
+            const int cols = min(BN, p.N - t.n0);
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
-                uint32_t r[32];
-                tmem_ld32(t_addr + c * 32, r);
-                tmem_wait_ld();
-                const int col0 = n0 + c * 32;
-                if (row < p.M && col0 < p.N) {
+            for (int c = 0; c < cols; c += step, ++box_it) {
+                uint8_t* box = boxes + (box_it % kOutBoxes) * kStageBox;
+                // the store that used this box last has read it
+                if (lane == 0) tma_wait_group_read1();
+                __syncwarp();
+                uint8_t* row = box + lane * 128;
+                const int col0 = t.n0 + c;
+                // one 32-column half of the box (all of an FP32 box) at a time
+#pragma unroll 1
+                for (int h = 0; h < step; h += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(t_addr + c + h, r);
+                    tmem_wait_ld();
                     float v[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-                    if (add_bias) {
+                    if (bias) {
+                        const float* b = bias + col0 + h;
+                        if (bias16 && col0 + h + 32 <= p.N) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (col0 + j < p.N) v[j] += __ldg(bias + col0 + j);
+                            for (int j = 0; j < 32; j += 4) {
+                                const float4 q = __ldg(reinterpret_cast<const float4*>(b + j));
+                                v[j] += q.x; v[j + 1] += q.y; v[j + 2] += q.z; v[j + 3] += q.w;
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                if (col0 + h + j < p.N) v[j] += __ldg(b + j);
+                        }
                     }
-                    if (p.split_k > 1) {
-                        float* dst = (float*)out + (int64_t)row * p.ldc + col0;
+                    if (bf16_out) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (col0 + j < p.N) atomicAdd(dst + j, v[j]);
-                    } else if (p.out_type != BOAT_CUDA_BF16) {
+                        for (int u = 0; u < 4; ++u) {
+                            uint32_t o[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                __nv_bfloat162 q = __floats2bfloat162_rn(v[8 * u + 2 * e], v[8 * u + 2 * e + 1]);
+                                o[e] = *reinterpret_cast<uint32_t*>(&q);
+                            }
+                            *reinterpret_cast<uint4*>(row + (((h / 8 + u) ^ swz) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                        }
+                    } else {
                         if (p.out_type == BOAT_CUDA_F32_TF32) {        // feeds another TF32 contraction
 #pragma unroll
                             for (int j = 0; j < 32; ++j) v[j] = round_to_tf32(v[j]);
                         }
-                        float* dst = (float*)out + (int64_t)row * p.ldc + col0;
 #pragma unroll
-                        for (int j = 0; j < 32; j += 4)
-                            if (col0 + j < p.N)       // N is a multiple of 4 on this path
-                                *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                    } else {
-                        __nv_bfloat16* dst = (__nv_bfloat16*)out + (int64_t)row * p.ldc + col0;
-#pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            if (col0 + j < p.N) {     // N is a multiple of 8 on this path
-                                __nv_bfloat162 h0 = __floats2bfloat162_rn(v[j], v[j + 1]);
-                                __nv_bfloat162 h1 = __floats2bfloat162_rn(v[j + 2], v[j + 3]);
-                                __nv_bfloat162 h2 = __floats2bfloat162_rn(v[j + 4], v[j + 5]);
-                                __nv_bfloat162 h3 = __floats2bfloat162_rn(v[j + 6], v[j + 7]);
-                                uint4 o;
-                                o.x = *reinterpret_cast<uint32_t*>(&h0);
-                                o.y = *reinterpret_cast<uint32_t*>(&h1);
-                                o.z = *reinterpret_cast<uint32_t*>(&h2);
-                                o.w = *reinterpret_cast<uint32_t*>(&h3);
-                                *reinterpret_cast<uint4*>(dst + j) = o;
-                            }
-                        }
+                        for (int u = 0; u < 8; ++u)
+                            *reinterpret_cast<float4*>(row + ((u ^ swz) << 4)) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
                     }
                 }
+                if (c + step >= cols) {
+                    // the tile is out of tensor memory
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (CTAS == 2) mbar_arrive_peer(peer_addr(&acc_empty[buf], 0));
+                        else           mbar_arrive(&acc_empty[buf]);
+                    }
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                    if (row0 < p.M) {
+                        if (t.add) tma_reduce_add_2d(map_c, box, col0, row0);
+                        else       tma_store_2d(map_c, box, col0, row0);
+                    }
+                    tma_commit_group();
+                }
             }
-            tc_fence_before_sync();
-            mbar_arrive(&acc_empty[buf]);
         }
+        if (lane == 0) tma_wait_group0();
     }
     tc_fence_before_sync();
     __syncthreads();
+    if (CTAS == 2) cluster_sync_all();            // the peer may still read this CTA's operands or arrive here
     if (warp == 1) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, C::TMEM_COLS);
+        if (CTAS == 2) tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
+        else           tmem_dealloc(tmem_base, C::TMEM_COLS);
     }
 }
 
 bool g_yielding = false;
 
-template <typename T, bool A_MN, bool B_MN, int BN>
-int launch(int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda, const void* const* B,
-           int64_t ldb, void* const* Cp, int64_t ldc, int out_type, const float* const* bias, int split_k) {
-    using C = Cfg<T, BN>;
+struct Problem {
+    int groups;
+    int64_t M, N, K;
+    const void* const* A;
+    int64_t lda;
+    const void* const* B;
+    int64_t ldb;
+    void* const* C;
+    int64_t ldc;
+    int out_type;
+    const float* const* bias;
+    bool add;
+};
+
+// A tile shape and what it costs, measured on B200 at 12 to 512 K-blocks (64 BF16): microseconds per K-block,
+// and once per launch (filling the ring, the epilogue that nothing overlaps).  Pairs on 256 x 256 are
+// fastest per FLOP (1340 TFLOP/s at 32768 x 2048 x 2048; a single CTA's 128 x 256 1220, 128 x 128 900,
+// 128 x 64 510) and slowest to start.
+struct Shape { int ctas, bn; double block_us, once_us; };
+constexpr Shape kShapes[4] = {{2, 256, 0.31, 2.7}, {1, 256, 0.34, 1.1}, {1, 128, 0.23, 0.6}, {1, 64, 0.20, 0.0}};
+
+struct Plan {
+    int64_t tiles, full, split;
+    double us;
+};
+
+// Which tiles are cut along K, into how many pieces, and how long the launch should take.
+Plan make_plan(const Problem& q, const Shape& sh, int bk) {
+    const int64_t workers = sm_count() / sh.ctas, k_blocks = ceil_div(q.K, bk);
+    Plan r;
+    r.tiles = ceil_div(q.M, BM * sh.ctas) * ceil_div(q.N, sh.bn) * q.groups;
+    r.full = r.tiles;
+    r.split = 1;
+    r.us = (double)ceil_div(r.tiles, workers) * (double)k_blocks * sh.block_us + sh.once_us;
+    if (q.out_type != BOAT_CUDA_F32) return r;
+    // FP32 results: the last, partly filled wave of tiles is cut so that its pieces come out even over
+    // all workers; at least 8 K-blocks per piece, and no more than two pieces below K = 2048 (two
+    // addends give the same bits in either order).  An SM gets its part of a piece out at about 36 KB per
+    // microsecond, behind the next piece's main loop but for the last one; the output is cleared first.
+    const int64_t rest = r.tiles % workers, whole = r.tiles / workers;
+    const double out_us = BM * sh.bn * 4.0 / 36e3;
+    const double clear_us = q.add ? 0.0 : 2.0 + (double)q.M * (double)q.N * q.groups * 4.0 / 4e6;
+    int64_t most = k_blocks / 8;
+    if (q.K < 2048 && most > 2) most = 2;
+    if (most > 32) most = 32;
+    for (int64_t s = 2; s <= most && rest > 0; ++s) {
+        double piece = (double)k_blocks / (double)s * sh.block_us;
+        if (piece < out_us) piece = out_us;
+        const double t = (double)whole * (double)k_blocks * sh.block_us + (double)ceil_div(rest * s, workers) * piece + out_us +
+                         clear_us + sh.once_us;
+        if (t < r.us) {
+            r.us = t;
+            r.split = s;
+            r.full = r.tiles - rest;
+        }
+    }
+    return r;
+}
+
+template <typename T, bool A_MN, bool B_MN, int CTAS, int BN>
+int launch(const Problem& q, const Plan& plan) {
+    using C = Cfg<T, CTAS, BN>;
     GroupMaps maps;
     Params p;
-    for (int g = 0; g < kMaxGroups; ++g) {
-        const int s = g < groups ? g : 0;       // unused slots repeat group 0: valid descriptors, never walked
+    const bool bf16_out = q.out_type == BOAT_CUDA_BF16;
+    for (int g = 0; g < q.groups; ++g) {
         // A: K-major -> matrix [M rows, K cols], box [BM, BK].  M-major -> stored [K rows, M cols], box [BK, BK].
-        if (int rc = A_MN ? make_tensor_map_2d(&maps.a[g], A[s], C::ES, (uint64_t)K, (uint64_t)M, (uint64_t)lda, C::BK, C::BK, C::ES == 4)
-                          : make_tensor_map_2d(&maps.a[g], A[s], C::ES, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, C::BK))
+        if (int rc = A_MN ? make_tensor_map_2d(&maps.a[g], q.A[g], C::ES, (uint64_t)q.K, (uint64_t)q.M, (uint64_t)q.lda, C::BK, C::BK, C::ES == 4)
+                          : make_tensor_map_2d(&maps.a[g], q.A[g], C::ES, (uint64_t)q.M, (uint64_t)q.K, (uint64_t)q.lda, BM, C::BK))
             return rc;
-        if (int rc = B_MN ? make_tensor_map_2d(&maps.b[g], B[s], C::ES, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, C::BK, C::BK, C::ES == 4)
-                          : make_tensor_map_2d(&maps.b[g], B[s], C::ES, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, BN, C::BK))
+        if (int rc = B_MN ? make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.ldb, C::BK, C::BK, C::ES == 4)
+                          : make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.N, (uint64_t)q.K, (uint64_t)q.ldb, C::BNC, C::BK))
             return rc;
-        p.C[g] = Cp[s];
-        p.bias[g] = bias ? bias[s] : nullptr;
+        if (int rc = make_tensor_map_2d(&maps.c[g], q.C[g], bf16_out ? 2 : 4, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, bf16_out ? 64 : 32))
+            return rc;
+        p.bias[g] = q.bias ? q.bias[g] : nullptr;
     }
-    const int tiles = (int)(ceil_div(M, BM) * ceil_div(N, BN)) * groups;
-    if (split_k > 1) {
-        for (int g = 0; g < groups; ++g) {
-            if (ldc == N) {
-                BOATCU_CHECK(cudaMemsetAsync(Cp[g], 0, (size_t)M * N * sizeof(float), stream()));
+    const int64_t full = plan.full, split = plan.split, tiles = plan.tiles, workers = sm_count() / CTAS;
+    if (split > 1 && !q.add) {
+        for (int g = 0; g < q.groups; ++g) {
+            if (q.ldc == q.N) {
+                BOATCU_CHECK(cudaMemsetAsync(q.C[g], 0, (size_t)q.M * q.N * sizeof(float), stream()));
             } else {
-                BOATCU_CHECK(cudaMemset2DAsync(Cp[g], (size_t)ldc * sizeof(float), 0, (size_t)N * sizeof(float), (size_t)M, stream()));
+                BOATCU_CHECK(cudaMemset2DAsync(q.C[g], (size_t)q.ldc * sizeof(float), 0, (size_t)q.N * sizeof(float), (size_t)q.M, stream()));
             }
         }
     }
-    p.groups = groups;
-    p.ldc = ldc;
-    p.M = (int)M;
-    p.N = (int)N;
-    p.K = (int)K;
-    p.out_type = out_type;
-    p.split_k = split_k;
+    p.groups = q.groups;
+    p.M = (int)q.M;
+    p.N = (int)q.N;
+    p.K = (int)q.K;
+    p.out_type = q.out_type;
+    p.full = (int)full;
+    p.split = (int)split;
+    p.add_all = q.add ? 1 : 0;
     p.status = kernel_status_ptr();
-    auto kern = gemm_tc_kernel<T, A_MN, B_MN, BN>;
+    auto kern = gemm_tc_kernel<T, A_MN, B_MN, CTAS, BN>;
     static bool configured = false;     // per process = per device: the library binds to one device
     if (!configured) {
         BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
         configured = true;
     }
-    const int work = tiles * split_k;
+    const int64_t work = full + (tiles - full) * split;
     // Persistent by default: one CTA per SM walks the tiles.  A yielding launch has one CTA per tile
     // instead, so that SMs come free all along and the CTAs of a collective started beside it (whose
     // stream has priority) get placed while the GEMM runs, not after it.
-    const int grid = (g_yielding || work < sm_count()) ? work : sm_count();
+    const int64_t grid = (g_yielding || work < workers ? work : workers) * CTAS;
     ProfileScope prof(A_MN ? "gemm_tc_tn" : (B_MN ? "gemm_tc_nn" : "gemm_tc_nt"));
-    BOATCU_RUN(kern, grid, kThreads, C::SMEM, maps, p);
+    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)grid), dim3(kThreads), C::SMEM, CTAS, maps, p));
     BOATCU_LAUNCH_OK("gemm_tc");
     return 0;
 }
 
-template <typename T, int BN>
-int dispatch_layout_bn(int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
-                       const void* const* B, int64_t ldb, void* const* C, int64_t ldc, int out_type,
-                       const float* const* bias, int split_k) {
-    // trans_a: A stored [K,M] (M-major).  trans_b == 0: B stored [K,N] (N-major).
-    if (!ta && !tb) return launch<T, false, true, BN>(groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, split_k);
-    if (!ta && tb) return launch<T, false, false, BN>(groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, split_k);
-    if (ta && !tb) return launch<T, true, true, BN>(groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, split_k);
-    return launch<T, true, false, BN>(groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, split_k);
+// The tile shape with the shortest estimate.
+template <typename T, bool A_MN, bool B_MN>
+int pick_tile(const Problem& q) {
+    int best = 0;
+    Plan plan;
+    for (int i = 0; i < 4; ++i) {
+        const Plan t = make_plan(q, kShapes[i], 128 / (int)sizeof(T));
+        if (i == 0 || t.us < plan.us) {
+            plan = t;
+            best = i;
+        }
+    }
+    switch (best) {
+        case 0: return launch<T, A_MN, B_MN, 2, 256>(q, plan);
+        case 1: return launch<T, A_MN, B_MN, 1, 256>(q, plan);
+        case 2: return launch<T, A_MN, B_MN, 1, 128>(q, plan);
+        default: return launch<T, A_MN, B_MN, 1, 64>(q, plan);
+    }
 }
 
 template <typename T>
-int dispatch_layout(int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
-                    const void* const* B, int64_t ldb, void* const* C, int64_t ldc, int out_type,
-                    const float* const* bias) {
-    const int64_t sms = sm_count();
-    const int64_t tiles = ceil_div(M, BM) * ceil_div(N, 256) * groups;
-    const int64_t k_blocks = ceil_div(K, (int64_t)(128 / sizeof(T)));
-    // Few output tiles and a long K (weight gradients): spread K over the idle SMs, at least 8
-    // K-blocks per piece; the pieces add into a zeroed FP32 output.
-    int64_t split_k = 1;
-    if (out_type == BOAT_CUDA_F32 && tiles * 2 <= sms) {
-        split_k = sms / tiles;
-        if (split_k > k_blocks / 8) split_k = k_blocks / 8;
-        if (split_k < 1) split_k = 1;
-    }
-    // 128 x 256 tiles by default.  A problem with fewer such tiles than SMs (and no long K to split
-    // instead) gets 128 x 128 tiles when those still fit in one wave: twice the CTAs at work, half
-    // the main loop per CTA.  (More narrow tiles than SMs would only add a second, partly empty wave.)
-    const int64_t narrow_tiles = ceil_div(M, BM) * ceil_div(N, 128) * groups;
-    if (tiles < sms && narrow_tiles <= sms && split_k == 1 && N > 128)
-        return dispatch_layout_bn<T, 128>(ta, tb, groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, 1);
-    return dispatch_layout_bn<T, 256>(ta, tb, groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, (int)split_k);
+int dispatch_layout(int ta, int tb, const Problem& q) {
+    // trans_a: A stored [K,M] (M-major).  trans_b == 0: B stored [K,N] (N-major).
+    if (!ta && !tb) return pick_tile<T, false, true>(q);
+    if (!ta && tb) return pick_tile<T, false, false>(q);
+    if (ta && !tb) return pick_tile<T, true, true>(q);
+    return pick_tile<T, true, false>(q);
 }
 
 }  // namespace
@@ -373,9 +507,8 @@ int gemm_tc_grouped(int mma, int ta, int tb, int groups, int64_t M, int64_t N, i
                     const float* const* bias) {
     if (groups < 1 || groups > kMaxGroups) return set_error(11, "gemm_tc_grouped: %d groups (1..%d)", groups, kMaxGroups);
     if (int rc = ensure_init()) return rc;
-    if (mma == BOAT_MMA_BF16)
-        return dispatch_layout<__nv_bfloat16>(ta, tb, groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias);
-    return dispatch_layout<float>(ta, tb, groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias);
+    const Problem q{groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, false};
+    return mma == BOAT_MMA_BF16 ? dispatch_layout<__nv_bfloat16>(ta, tb, q) : dispatch_layout<float>(ta, tb, q);
 }
 
 void gemm_tc_set_yielding(bool on) { g_yielding = on; }
