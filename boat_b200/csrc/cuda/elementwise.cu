@@ -4,6 +4,7 @@
 // pointers and sizes allow it and falls back to scalar accesses otherwise; reductions use
 // warp shuffles.  Reference counterparts are named per function in boat_cuda.h.
 #include "common.cuh"
+#include <cooperative_groups.h>
 
 namespace boatcu {
 
@@ -260,57 +261,116 @@ __global__ void convert_multi_kernel(const ConvertTable t, int vec) {
     }
 }
 
-// ---- column sums: out[j] += sum_i X[i,j] -----------------------------------------------------
-// Block = 32 column lanes x 8 row lanes; a column lane owns VEC adjacent columns.  Row lanes
-// are combined through shared memory, blocks through atomicAdd into a zeroed output.
+// ---- column sums: out[j] = sum_i X[i,j] ------------------------------------------------------
+// A CTA's threads are LANES column lanes (16 bytes of a row each) x row lanes, eight rows' loads in flight
+// per thread; row lanes fold in shared memory.  Two ways to fold the CTAs of a column group:
+//   - a cluster of 8 CTAs, through distributed shared memory in a fixed order: one launch, no cleared
+//     output, the same bits every time.  3 x 8000 x 1024 BF16 in 9 us back to back (18 us the other way).
+//     But clusters pack unevenly onto SMs, which costs bandwidth once a matrix is large (32768 x 2048:
+//     43 us);
+//   - from 32 MB per matrix on, independent CTAs on a full grid that add into a cleared output with
+//     atomics (28 us).
 // blockIdx.z selects one of several matrices of the same shape.
 constexpr int kMaxColsum = 4;
+constexpr int kColsumCluster = 8;
 struct ColsumTable {
     const void* x[kMaxColsum];
     float* out[kMaxColsum];
 };
 
-template <typename T, int VEC>
-__global__ void colsum_kernel(const ColsumTable t, int64_t rows, int64_t cols) {
+template <typename T, int VEC, int LANES, int THREADS, bool CLUSTER>
+__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols) {
+    constexpr int ROWS = THREADS / LANES, COLS = LANES * VEC, UNROLL = 8;
+    __shared__ float part[ROWS * COLS];
+    __shared__ float folded[CLUSTER ? COLS : 1];
     griddep_sync();
     const T* __restrict__ X = (const T*)t.x[blockIdx.z];
-    float* __restrict__ out = t.out[blockIdx.z];
-    __shared__ float part[8][32 * VEC + 1];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t col0 = ((int64_t)blockIdx.x * 32 + tx) * VEC;
+    const int tx = threadIdx.x % LANES, ty = threadIdx.x / LANES;
+    const int64_t group0 = (int64_t)blockIdx.y * COLS, col0 = group0 + tx * VEC;
     float acc[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
     if (col0 < cols) {
-        for (int64_t r = (int64_t)blockIdx.y * 8 + ty; r < rows; r += (int64_t)gridDim.y * 8) {
-            const T* p = X + r * cols + col0;
-            if (VEC == 1) {
-                acc[0] += to_f32(p[0]);
-            } else if (sizeof(T) == 4) {      // VEC == 4
-                float4 v = *reinterpret_cast<const float4*>(p);
-                acc[0] += v.x; acc[1] += v.y; acc[2] += v.z; acc[3] += v.w;
-            } else {                          // bf16, VEC == 8
-                uint4 v = *reinterpret_cast<const uint4*>(p);
-                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+        const int64_t step = (int64_t)gridDim.x * ROWS;
+        int64_t r = (int64_t)blockIdx.x * ROWS + ty;
+        if constexpr (VEC == 1) {
+            for (; r < rows; r += step) acc[0] += to_f32(X[r * cols + col0]);
+        } else {
+            auto add = [&](const uint4& v) {
+                if constexpr (sizeof(T) == 4) {
+                    acc[0] += __uint_as_float(v.x); acc[1] += __uint_as_float(v.y); acc[2] += __uint_as_float(v.z); acc[3] += __uint_as_float(v.w);
+                } else {
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float2 f = __bfloat1622float2(h[k]);
-                    acc[2 * k] += f.x; acc[2 * k + 1] += f.y;
+                    for (int k = 0; k < 4; ++k) {
+                        const float2 f = __bfloat1622float2(h[k]);
+                        acc[2 * k] += f.x;
+                        acc[2 * k + 1] += f.y;
+                    }
                 }
+            };
+            for (; r + (UNROLL - 1) * step < rows; r += UNROLL * step) {
+                uint4 v[UNROLL];
+#pragma unroll
+                for (int u = 0; u < UNROLL; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(X + (r + u * step) * cols + col0));
+#pragma unroll
+                for (int u = 0; u < UNROLL; ++u) add(v[u]);
             }
+            for (; r < rows; r += step) add(__ldg(reinterpret_cast<const uint4*>(X + r * cols + col0)));
         }
     }
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) part[ty][tx * VEC + v] = acc[v];
+    for (int v = 0; v < VEC; ++v) part[ty * COLS + tx * VEC + v] = acc[v];
     __syncthreads();
-    // 256 threads fold the 8 row lanes of 32*VEC columns
-    for (int c = threadIdx.x; c < 32 * VEC; c += blockDim.x) {
+    for (int c = threadIdx.x; c < COLS; c += THREADS) {
         float s = 0.f;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) s += part[k][c];
-        int64_t col = (int64_t)blockIdx.x * 32 * VEC + c;
-        if (col < cols) atomicAdd(out + col, s);
+#pragma unroll 8
+        for (int k = 0; k < ROWS; ++k) s += part[k * COLS + c];
+        if (CLUSTER) folded[c] = s;
+        else if (group0 + c < cols) atomicAdd(t.out[blockIdx.z] + group0 + c, s);
     }
+    if constexpr (CLUSTER) {
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        cluster.sync();
+        if (blockIdx.x == 0) {
+            for (int c = threadIdx.x; c < COLS; c += THREADS) {
+                float s = 0.f;
+#pragma unroll
+                for (int r = 0; r < kColsumCluster; ++r) s += cluster.map_shared_rank(folded, r)[c];
+                if (group0 + c < cols) t.out[blockIdx.z][group0 + c] = s;
+            }
+        }
+        cluster.sync();
+    }
+}
+
+template <typename T, int VEC, int LANES>
+static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t cols, int count) {
+    BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)ceil_div(cols, LANES * VEC), (unsigned)count),
+                                  dim3(512), 0, kColsumCluster, t, rows, cols));
+    BOATCU_LAUNCH_OK("colsum");
+    return 0;
+}
+
+template <typename T, int VEC>
+static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int count) {
+    if (rows * cols * (int64_t)sizeof(T) >= (32ll << 20)) {
+        for (int i = 0; i < count; ++i) BOATCU_CHECK(cudaMemsetAsync(t.out[i], 0, (size_t)cols * sizeof(float), stream()));
+        const int64_t groups = ceil_div(cols, 32 * VEC);
+        int64_t y = (int64_t)sm_count() * 8 / (groups * count);         // eight CTAs per SM
+        if (y < 1) y = 1;
+        if (y > ceil_div(rows, 8)) y = ceil_div(rows, 8);
+        BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, 32, 256, false>, dim3((unsigned)y, (unsigned)groups, (unsigned)count), dim3(256), 0, 1,
+                                      t, rows, cols));
+        BOATCU_LAUNCH_OK("colsum");
+        return 0;
+    }
+    // the runs of a row are 512 bytes where that makes enough CTAs for the GPU, else 256 or 128
+    auto ctas = [&](int lanes) { return ceil_div(cols, lanes * VEC) * kColsumCluster * count; };
+    const int64_t enough = (int64_t)sm_count() * 4 / 5;
+    if (ctas(32) >= enough) return launch_colsum_cluster<T, VEC, 32>(t, rows, cols, count);
+    if (ctas(16) >= enough) return launch_colsum_cluster<T, VEC, 16>(t, rows, cols, count);
+    return launch_colsum_cluster<T, VEC, 8>(t, rows, cols, count);
 }
 
 // ---- delta[r] = sum_d dO[r,d] * O[r,d]: one warp per row, shuffle reduction --------------------
@@ -557,25 +617,10 @@ int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64
         t.out[i] = out[s];
         can_vec = can_vec && aligned16(X[s]);
     }
-    // one clear per output: neighbouring outputs may still be separate allocations, which a single
-    // clear must not span
-    for (int i = 0; i < count; ++i) BOATCU_CHECK(cudaMemsetAsync(out[i], 0, (size_t)cols * sizeof(float), stream()));
-    if (rows <= 0) return 0;
-    const int cols_per_block = 32 * (can_vec ? vec : 1);
-    dim3 grid((unsigned)ceil_div(cols, cols_per_block), 1, (unsigned)count);
-    int64_t want = (int64_t)sm_count() * 8 / ((int64_t)grid.x * count);
-    int64_t max_y = ceil_div(rows, 8);
-    grid.y = (unsigned)(want < 1 ? 1 : (want > max_y ? max_y : want));
-    if (grid.y > 65535) grid.y = 65535;
-    if (x_type == BOAT_CUDA_BF16) {
-        if (can_vec) BOATCU_RUN((colsum_kernel<__nv_bfloat16, 8>), grid, kThreads, 0, t, rows, cols);
-        else         BOATCU_RUN((colsum_kernel<__nv_bfloat16, 1>), grid, kThreads, 0, t, rows, cols);
-    } else {
-        if (can_vec) BOATCU_RUN((colsum_kernel<float, 4>), grid, kThreads, 0, t, rows, cols);
-        else         BOATCU_RUN((colsum_kernel<float, 1>), grid, kThreads, 0, t, rows, cols);
-    }
-    BOATCU_LAUNCH_OK("colsum");
-    return 0;
+    if (rows < 0) rows = 0;
+    if (x_type == BOAT_CUDA_BF16)
+        return can_vec ? launch_colsum<__nv_bfloat16, 8>(t, rows, cols, count) : launch_colsum<__nv_bfloat16, 1>(t, rows, cols, count);
+    return can_vec ? launch_colsum<float, 4>(t, rows, cols, count) : launch_colsum<float, 1>(t, rows, cols, count);
 }
 
 int boat_cuda_colsum(const void* X, int x_type, int64_t rows, int64_t cols, float* out) {
