@@ -136,7 +136,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     uint32_t* tmem_slot = (uint32_t*)(bars + 25);
     volatile uint32_t* drain_ok = tmem_slot + 3;       // same idea for the dQ warps
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
     // CTA order: units in groups of p.group; inside a group the key-tile pair is the slow index.
     // The CTAs that run at the same time then belong to a few (batch, head) units, so the FP32 dQ
@@ -246,11 +246,19 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // The whole warp in step, one elected lane issues: operands stay in uniform registers (see the
+        // forward kernel; a single lane's issue took about 100 cycles per MMA, 40 MMAs per tile pair).
+        {
             constexpr uint32_t idesc_st = make_idesc(kBF16, false, false, kTile, kTile);   // K.Q^T, V.dO^T
             constexpr uint32_t idesc_acc = make_idesc(kBF16, false, true, kTile, HS);      // dV, dK
             constexpr uint32_t idesc_dq = make_idesc(kBF16, true, true, kTile, HS);        // dQ
-            const uint32_t k_addr = smem_u32(k_smem), v_addr = smem_u32(v_smem), ds_addr = smem_u32(ds_smem);
+            const bool leader = elect_one();
+            const uint64_t k_desc = smem_desc_sw128(smem_u32(k_smem), 16, 1024), v_desc = smem_desc_sw128(smem_u32(v_smem), 16, 1024);
+            const uint64_t q_desc = smem_desc_sw128(smem_u32(q_smem), 16, 1024), do_desc = smem_desc_sw128(smem_u32(do_smem), 16, 1024);
+            const uint64_t ds_desc = smem_desc_sw128(smem_u32(ds_smem), 16, 1024);
+            // the same tiles read along their rows
+            const uint64_t k_mn = smem_desc_mn(smem_u32(k_smem), kBoxBytes, false), q_mn = smem_desc_mn(smem_u32(q_smem), kBoxBytes, false);
+            const uint64_t do_mn = smem_desc_mn(smem_u32(do_smem), kBoxBytes, false), ds_mn = smem_desc_mn(smem_u32(ds_smem), kBoxBytes, false);
             // Issue order on the (in-order) tensor pipe, per tile t:
             //   dV(t) S(t+1) | dQ(t) dK(t) | dP(t+1)
             // dV follows phase A; S^T of the next tile overwrites R0 right behind it (dV, ahead on
@@ -260,94 +268,97 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             // cases long before phase B of the next tile asks for it.
             auto issue_s = [&](int t) -> bool {
                 const int s = t % C::Q_STAGES;
-                if (!mbar_wait(&q_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) return false;
+                if (!mbar_wait_warp(&q_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) return false;
                 tc_fence_after_sync();
-                const uint32_t q_addr = smem_u32(q_smem + s * C::TILE_BYTES);
+                const uint64_t qd = q_desc + (s * C::TILE_BYTES >> 4);
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < C::ROWB / 32; ++kk) {
-                    const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-                    mma_ss<false>(tmem_base + C::COL_S, smem_desc_sw128(k_addr + off, 16, 1024),
-                                  smem_desc_sw128(q_addr + off, 16, 1024), idesc_st, kk > 0);
+                    for (int kk = 0; kk < C::ROWB / 32; ++kk) {
+                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                        mma_ss<false>(tmem_base + C::COL_S, k_desc + off, qd + off, idesc_st, kk > 0);
+                    }
+                    mma_commit(s_full);
                 }
-                mma_commit(s_full);
                 return true;
             };
             auto issue_dp = [&](int t) -> bool {        // dP^T = V . dO^T
                 const int s = t % C::Q_STAGES;
-                if (!mbar_wait(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) return false;
+                if (!mbar_wait_warp(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) return false;
                 tc_fence_after_sync();
-                const uint32_t do_addr = smem_u32(do_smem + s * C::TILE_BYTES);
+                const uint64_t dod = do_desc + (s * C::TILE_BYTES >> 4);
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < C::ROWB / 32; ++kk) {
-                    const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-                    mma_ss<false>(tmem_base + C::COL_DP, smem_desc_sw128(v_addr + off, 16, 1024),
-                                  smem_desc_sw128(do_addr + off, 16, 1024), idesc_st, kk > 0);
+                    for (int kk = 0; kk < C::ROWB / 32; ++kk) {
+                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                        mma_ss<false>(tmem_base + C::COL_DP, v_desc + off, dod + off, idesc_st, kk > 0);
+                    }
+                    mma_commit(dp_full);
                 }
-                mma_commit(dp_full);
                 return true;
             };
-            bool ok = mbar_wait(kv_full, 0, p.status, kTimeoutMma);
+            bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutMma);
             ok = ok && issue_s(0);
             ok = ok && issue_dp(0);
             for (int t = 0; t < n_q && ok; ++t) {
                 const int s = t % C::Q_STAGES;
                 const bool first = t == 0 || t == nA;           // first tile of a walk: dK, dV start over
                 const bool early_next = t + 1 < n_q && t + 1 != nA;   // the next tile belongs to the same walk
-                const uint32_t q_addr = smem_u32(q_smem + s * C::TILE_BYTES);
-                const uint32_t do_addr = smem_u32(do_smem + s * C::TILE_BYTES);
+                const uint64_t q_d = q_mn + (s * C::TILE_BYTES >> 4), do_d = do_mn + (s * C::TILE_BYTES >> 4);
                 if (t == nA) {
                     // second walk: wait for its K and V, then the MMAs a walk begins with.  R0 (and with
                     // head size 64 the dP^T columns) are free: phase B of the previous tile is over.
-                    if (!mbar_wait(kv_full, 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (!mbar_wait_warp(kv_full, 1, p.status, kTimeoutMma)) { ok = false; break; }
                     if (!issue_s(t)) { ok = false; break; }
                     // the first walk's last dQ must be out of the columns dP^T borrows
-                    if (!C::DP_OWN && !mbar_wait(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (!C::DP_OWN && !mbar_wait_warp(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
                     if (!issue_dp(t)) { ok = false; break; }
                 }
-                if (!mbar_wait(p_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                if (!mbar_wait(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                if (t == nA && !mbar_wait(acc_free, 0, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(p_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (t == nA && !mbar_wait_warp(acc_free, 0, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < kTile / 16; ++kk)      // dV += P^T . dO      (K = 128 query rows)
-                    mma_ts<false>(tmem_base + C::COL_DV, tmem_base + C::COL_S + (kk / 4) * 64 + (kk % 4) * 8,
-                                  smem_desc_mn(do_addr + kk * 2048, kBoxBytes, false), idesc_acc, !first || kk > 0);
+                    for (int kk = 0; kk < kTile / 16; ++kk)      // dV += P^T . dO      (K = 128 query rows)
+                        mma_ts<false>(tmem_base + C::COL_DV, tmem_base + C::COL_S + (kk / 4) * 64 + (kk % 4) * 8,
+                                      do_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
+                }
                 // R0 is free as soon as dV, ahead on the pipe, has read P^T
                 if (early_next && !issue_s(t + 1)) { ok = false; break; }
-                if (!mbar_wait(ds_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(ds_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
                 if (t > 0) {
                     // the previous dQ must have left its TMEM columns
-                    if (!mbar_wait(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (!mbar_wait_warp(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
                 }
                 tc_fence_after_sync();
                 // dQ first: its completion starts the read-out, whose first step (tensor memory ->
                 // registers) gates the next tile's dP^T when that borrows the dQ columns; dK runs
                 // on the pipe meanwhile.  This tile's dO stage was last read by dV and dP^T, which
                 // are ahead of dQ on the pipe, so it is free for the read-out's staging at dq_full.
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < kTile / 16; ++kk)      // dQ_i = dS . K        (K = 128 key rows)
-                    mma_ss<false>(tmem_base + C::COL_DQ, smem_desc_mn(ds_addr + kk * 2048, kBoxBytes, false),
-                                  smem_desc_mn(k_addr + kk * 2048, kBoxBytes, false), idesc_dq, kk > 0);
-                mma_commit(dq_full);
+                    for (int kk = 0; kk < kTile / 16; ++kk)      // dQ_i = dS . K        (K = 128 key rows)
+                        mma_ss<false>(tmem_base + C::COL_DQ, ds_mn + (kk * 2048 >> 4), k_mn + (kk * 2048 >> 4), idesc_dq, kk > 0);
+                    mma_commit(dq_full);
 #pragma unroll
-                for (int kk = 0; kk < kTile / 16; ++kk) {    // dK += dS^T . Q
-                    const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-                    mma_ss<false>(tmem_base + C::COL_DK, smem_desc_sw128(ds_addr + off, 16, 1024),
-                                  smem_desc_mn(q_addr + kk * 2048, kBoxBytes, false), idesc_acc, !first || kk > 0);
-                }
-                mma_commit(&q_empty[s]);  // also: the dS^T tile is no longer read
-                if (t == nA - 1 && has_b) {
-                    mma_commit(kv_empty);                   // K and V of the first walk are no longer read
-                    mma_commit(all_done);                   // and its dK, dV are complete
+                    for (int kk = 0; kk < kTile / 16; ++kk) {    // dK += dS^T . Q
+                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                        mma_ss<false>(tmem_base + C::COL_DK, ds_desc + off, q_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
+                    }
+                    mma_commit(&q_empty[s]);  // also: the dS^T tile is no longer read
+                    if (t == nA - 1 && has_b) {
+                        mma_commit(kv_empty);                   // K and V of the first walk are no longer read
+                        mma_commit(all_done);                   // and its dK, dV are complete
+                    }
                 }
                 // dS^T of tile t is in shared memory, so the softmax warps are done with dP^T(t)
                 if (early_next) {
                     // borrowed columns: this tile's dQ, just issued, has to complete and leave them first
-                    if (!C::DP_OWN && !mbar_wait(dq_empty, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (!C::DP_OWN && !mbar_wait_warp(dq_empty, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
                     if (!issue_dp(t + 1)) { ok = false; break; }
                 }
             }
-            if (ok) mma_commit(all_done);
+            if (ok && leader) mma_commit(all_done);
         }
     } else if (warp < 10) {
         // ---------------- softmax / dS: warps 2..9 ----------------

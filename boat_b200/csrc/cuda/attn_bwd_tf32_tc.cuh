@@ -92,7 +92,7 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     uint64_t* dq_done = bars + 5;       // last dQ MMA complete
     uint32_t* tmem_slot = (uint32_t*)(bars + 6);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
     const int unit = blockIdx.x % p.units;
     const int qt = n_tiles - 1 - blockIdx.x / p.units;       // long (late) rows first when causal
@@ -142,37 +142,40 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 for (int i = 0; i < 1000; ++i) __nanosleep(1000);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {   // the whole warp in step, one elected lane issues (see the forward kernel)
             constexpr uint32_t idesc_s = make_idesc(kTF32, false, false, kTile, kTile);   // S = Q.K^T, dP = dO.V^T
             constexpr uint32_t idesc_o = make_idesc(kTF32, false, true, kTile, HS);       // dQ += dS.K
-            const uint32_t q_addr = smem_u32(q_smem), do_addr = smem_u32(do_smem), k_addr = smem_u32(k_smem);
-            const uint32_t kmn_addr = smem_u32(kmn_smem), v_addr = smem_u32(v_smem);
-            bool ok = mbar_wait(q_full, 0, p.status, kTimeoutMma);
+            const uint64_t q_d = smem_desc_sw128(smem_u32(q_smem), 16, 1024), do_d = smem_desc_sw128(smem_u32(do_smem), 16, 1024);
+            const uint64_t k_d = smem_desc_sw128(smem_u32(k_smem), 16, 1024), v_d = smem_desc_sw128(smem_u32(v_smem), 16, 1024);
+            const uint64_t k_mn = smem_desc_mn(smem_u32(kmn_smem), kBoxBytes, true);
+            const bool leader = elect_one();
+            bool ok = mbar_wait_warp(q_full, 0, p.status, kTimeoutMma);
             for (int j = 0; j < n_kv && ok; ++j) {
-                if (!mbar_wait(kv_full, j & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(kv_full, j & 1, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < HS * 4 / 32; ++kk) {
-                    const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-                    mma_ss<true>(tmem_s, smem_desc_sw128(q_addr + off, 16, 1024), smem_desc_sw128(k_addr + off, 16, 1024),
-                                 idesc_s, kk > 0);
-                }
+                    for (int kk = 0; kk < HS * 4 / 32; ++kk) {
+                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                        mma_ss<true>(tmem_s, q_d + off, k_d + off, idesc_s, kk > 0);
+                    }
 #pragma unroll
-                for (int kk = 0; kk < HS * 4 / 32; ++kk) {
-                    const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-                    mma_ss<true>(tmem_dp, smem_desc_sw128(do_addr + off, 16, 1024), smem_desc_sw128(v_addr + off, 16, 1024),
-                                 idesc_s, kk > 0);
+                    for (int kk = 0; kk < HS * 4 / 32; ++kk) {
+                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                        mma_ss<true>(tmem_dp, do_d + off, v_d + off, idesc_s, kk > 0);
+                    }
+                    mma_commit(s_full);
                 }
-                mma_commit(s_full);
-                if (!mbar_wait(ds_full, j & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(ds_full, j & 1, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < kTile / 8; ++kk)
-                    mma_ts<true>(tmem_dq, tmem_s + kk * 8, smem_desc_mn(kmn_addr + kk * 8 * 128, kBoxBytes, true), idesc_o,
-                                 j > 0 || kk > 0);
-                mma_commit(kv_empty);
+                    for (int kk = 0; kk < kTile / 8; ++kk)
+                        mma_ts<true>(tmem_dq, tmem_s + kk * 8, k_mn + (kk * 8 * 128 >> 4), idesc_o, j > 0 || kk > 0);
+                    mma_commit(kv_empty);
+                }
             }
-            if (ok) mma_commit(dq_done);
+            if (ok && leader) mma_commit(dq_done);
         }
     } else {
         // softmax warps: thread = query row
@@ -264,7 +267,7 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     uint32_t* tmem_slot = (uint32_t*)(bars + 6);
     volatile uint32_t* wait_ok = tmem_slot + 1;      // [2] outcome of the bounded wait, by tile parity
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
     const int unit = blockIdx.x % p.units;
     const int jt = blockIdx.x / p.units;                     // early key tiles have the long walks when causal
@@ -318,41 +321,43 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 for (int i = 0; i < 1000; ++i) __nanosleep(1000);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
             constexpr uint32_t idesc_s = make_idesc(kTF32, false, false, kTile, kTile);   // S^T = K.Q^T, dP^T = V.dO^T
             constexpr uint32_t idesc_o = make_idesc(kTF32, false, true, kTile, HS);       // dV += P^T.dO, dK += dS^T.Q
-            const uint32_t k_addr = smem_u32(k_smem), v_addr = smem_u32(v_smem), q_addr = smem_u32(q_smem);
-            const uint32_t qmn_addr = smem_u32(qmn_smem), do_addr = smem_u32(do_smem), domn_addr = smem_u32(domn_smem);
-            bool ok = mbar_wait(kv_full, 0, p.status, kTimeoutMma);
+            const uint64_t k_d = smem_desc_sw128(smem_u32(k_smem), 16, 1024), v_d = smem_desc_sw128(smem_u32(v_smem), 16, 1024);
+            const uint64_t q_d = smem_desc_sw128(smem_u32(q_smem), 16, 1024), do_d = smem_desc_sw128(smem_u32(do_smem), 16, 1024);
+            const uint64_t q_mn = smem_desc_mn(smem_u32(qmn_smem), kBoxBytes, true), do_mn = smem_desc_mn(smem_u32(domn_smem), kBoxBytes, true);
+            const bool leader = elect_one();
+            bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutMma);
             for (int t = 0; t < n_q && ok; ++t) {
-                if (!mbar_wait(q_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(q_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < HS * 4 / 32; ++kk) {
-                    const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-                    mma_ss<true>(tmem_st, smem_desc_sw128(k_addr + off, 16, 1024), smem_desc_sw128(q_addr + off, 16, 1024),
-                                 idesc_s, kk > 0);
-                }
+                    for (int kk = 0; kk < HS * 4 / 32; ++kk) {
+                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                        mma_ss<true>(tmem_st, k_d + off, q_d + off, idesc_s, kk > 0);
+                    }
 #pragma unroll
-                for (int kk = 0; kk < HS * 4 / 32; ++kk) {
-                    const uint32_t off = (kk / 4) * kBoxBytes + (kk % 4) * 32;
-                    mma_ss<true>(tmem_dpt, smem_desc_sw128(v_addr + off, 16, 1024), smem_desc_sw128(do_addr + off, 16, 1024),
-                                 idesc_s, kk > 0);
+                    for (int kk = 0; kk < HS * 4 / 32; ++kk) {
+                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                        mma_ss<true>(tmem_dpt, v_d + off, do_d + off, idesc_s, kk > 0);
+                    }
+                    mma_commit(s_full);
                 }
-                mma_commit(s_full);
-                if (!mbar_wait(p_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(p_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
+                if (leader) {
 #pragma unroll
-                for (int kk = 0; kk < kTile / 8; ++kk)
-                    mma_ts<true>(tmem_dv, tmem_st + kk * 8, smem_desc_mn(domn_addr + kk * 8 * 128, kBoxBytes, true), idesc_o,
-                                 t > 0 || kk > 0);
+                    for (int kk = 0; kk < kTile / 8; ++kk)
+                        mma_ts<true>(tmem_dv, tmem_st + kk * 8, do_mn + (kk * 8 * 128 >> 4), idesc_o, t > 0 || kk > 0);
 #pragma unroll
-                for (int kk = 0; kk < kTile / 8; ++kk)
-                    mma_ts<true>(tmem_dk, tmem_dpt + kk * 8, smem_desc_mn(qmn_addr + kk * 8 * 128, kBoxBytes, true), idesc_o,
-                                 t > 0 || kk > 0);
-                mma_commit(q_empty);
+                    for (int kk = 0; kk < kTile / 8; ++kk)
+                        mma_ts<true>(tmem_dk, tmem_dpt + kk * 8, q_mn + (kk * 8 * 128 >> 4), idesc_o, t > 0 || kk > 0);
+                    mma_commit(q_empty);
+                }
             }
-            if (ok) mma_commit(acc_done);
+            if (ok && leader) mma_commit(acc_done);
         }
     } else {
         // softmax warps: thread = key row; the statistics belong to the query columns

@@ -109,7 +109,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
     uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA (of the first CTA of a pair)
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = CTAS == 2 ? cluster_rank() : 0;
     const int worker = blockIdx.x / CTAS, workers = gridDim.x / CTAS;
     const int m_tiles = (p.M + BM * CTAS - 1) / (BM * CTAS), n_tiles = (p.N + BN - 1) / BN;
@@ -202,36 +202,39 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0 && rank == 0) {
+        // the whole warp in step, one elected lane issues, so that the operands stay in uniform registers
+        if (rank == 0) {
             constexpr uint32_t idesc = make_idesc(TF32 ? kTF32 : kBF16, A_MN, B_MN, BM * CTAS, BN);
+            const uint64_t a_desc0 = A_MN ? smem_desc_mn(smem_u32(a_smem), C::CHUNK_BYTES, TF32) : smem_desc_sw128(smem_u32(a_smem), 16, 1024);
+            const uint64_t b_desc0 = B_MN ? smem_desc_mn(smem_u32(b_smem), C::CHUNK_BYTES, TF32) : smem_desc_sw128(smem_u32(b_smem), 16, 1024);
+            const bool leader = elect_one();
             uint32_t it = 0, acc_it = 0;
             bool ok = true;
             for (int w = worker; w < work_items && ok; w += workers, ++acc_it) {
                 const WorkItem t = item(w);
                 const int buf = acc_it & 1;
-                if (!mbar_wait(&acc_empty[buf], ((acc_it >> 1) & 1) ^ 1, p.status, kTimeoutMma)) { ok = false; break; }
+                if (!mbar_wait_warp(&acc_empty[buf], ((acc_it >> 1) & 1) ^ 1, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + buf * BN;
                 for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (!mbar_wait_warp(&full[s], (it / STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
                     tc_fence_after_sync();
-                    const uint32_t a_addr = smem_u32(a_smem + s * C::A_BYTES);
-                    const uint32_t b_addr = smem_u32(b_smem + s * C::B_BYTES);
+                    const uint64_t a_desc = a_desc0 + (s * C::A_BYTES >> 4), b_desc = b_desc0 + (s * C::B_BYTES >> 4);
+                    if (leader) {
 #pragma unroll
-                    for (int kk = 0; kk < C::BK / C::UK; ++kk) {
-                        const uint64_t a_desc = A_MN ? smem_desc_mn(a_addr + kk * C::UK * 128, C::CHUNK_BYTES, TF32)
-                                                     : smem_desc_sw128(a_addr + kk * 32, 16, 1024);
-                        const uint64_t b_desc = B_MN ? smem_desc_mn(b_addr + kk * C::UK * 128, C::CHUNK_BYTES, TF32)
-                                                     : smem_desc_sw128(b_addr + kk * 32, 16, 1024);
-                        if (CTAS == 2) mma_ss_pair<TF32>(d_tmem, a_desc, b_desc, idesc, kb > t.kb0 || kk > 0);
-                        else           mma_ss<TF32>(d_tmem, a_desc, b_desc, idesc, kb > t.kb0 || kk > 0);
+                        for (int kk = 0; kk < C::BK / C::UK; ++kk) {
+                            const uint64_t ad = a_desc + ((A_MN ? kk * C::UK * 128 : kk * 32) >> 4);
+                            const uint64_t bd = b_desc + ((B_MN ? kk * C::UK * 128 : kk * 32) >> 4);
+                            if (CTAS == 2) mma_ss_pair<TF32>(d_tmem, ad, bd, idesc, kb > t.kb0 || kk > 0);
+                            else           mma_ss<TF32>(d_tmem, ad, bd, idesc, kb > t.kb0 || kk > 0);
+                        }
+                        // stage reusable once these MMAs have read it
+                        if (CTAS == 2) mma_commit_pair(&empty[s]);
+                        else           mma_commit(&empty[s]);
                     }
-                    // stage reusable once these MMAs have read it
-                    if (CTAS == 2) mma_commit_pair(&empty[s]);
-                    else           mma_commit(&empty[s]);
                 }
-                if (ok) {                             // accumulator complete
+                if (ok && leader) {                   // accumulator complete
                     if (CTAS == 2) mma_commit_pair(&acc_full[buf]);
                     else           mma_commit(&acc_full[buf]);
                 }
@@ -358,7 +361,7 @@ struct Problem {
 
 // A tile shape and what it costs, measured on B200 at 12 to 512 K-blocks (64 BF16): microseconds per K-block,
 // and once per launch (filling the ring, the epilogue that nothing overlaps).  Pairs on 256 x 256 are
-// fastest per FLOP (1340 TFLOP/s at 32768 x 2048 x 2048; a single CTA's 128 x 256 1220, 128 x 128 900,
+// fastest per FLOP (1440 TFLOP/s at 32768 x 2048 x 2048; a single CTA's 128 x 256 1220, 128 x 128 900,
 // 128 x 64 510) and slowest to start.
 struct Shape { int ctas, bn; double block_us, once_us; };
 constexpr Shape kShapes[4] = {{2, 256, 0.31, 2.7}, {1, 256, 0.34, 1.1}, {1, 128, 0.23, 0.6}, {1, 64, 0.20, 0.0}};

@@ -49,6 +49,9 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 
+// Warp of the CTA, known to the compiler as the same for all lanes (so are branches on it).
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // ---- mbarrier -----------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -176,6 +179,41 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Registers per thread of the calling warpgroup (all four warps call it): give some back, take some over.
+template <int N> __device__ __forceinline__ void regs_release() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_claim() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// ---- work distribution (cluster launch control) ----------------------------------------------------
+// A running CTA takes over the index of one that has not been placed yet: the kernel is launched with one
+// CTA per work item, those on the SMs stay and work the grid off in index order.  The answer (16
+// bytes) arrives in shared memory, counted on `bar`.  No further request after a refused one.
+__device__ __forceinline__ void request_next_cta(void* smem_answer, uint64_t* bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(smem_answer)), "r"(smem_u32(bar))
+                 : "memory");
+}
+// blockIdx.x of the CTA taken over, or -1 when none was left.
+__device__ __forceinline__ int taken_cta(const void* smem_answer) {
+    int x;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+        "ld.shared.b128 h, [%1];\n\t"
+        "mov.b32 %0, -1;\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, h;\n\t}"
+        : "=r"(x)
+        : "r"(smem_u32(smem_answer))
+        : "memory");
+    return x;
+}
+
+// 32 bytes of one lane to global memory: a whole sector per store.
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
 // ---- CTA pairs (cta_group::2): two CTAs of a cluster on neighbouring SMs work on one tile -----------
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;
