@@ -6,8 +6,11 @@
 //
 // A walk: one 128-row key/value tile of one (batch,head) unit against the query tiles that see
 // it (all of them, or those at or below the diagonal when causal).  K and V stay in shared
-// memory, dK and dV accumulate in tensor memory for the whole walk.  A CTA does two walks of
-// its unit back to back (when causal, tile j and tile n-1-j: n+1 query tiles for every CTA).
+// memory, dK and dV accumulate in tensor memory for the whole walk.  One CTA per SM does one walk after
+// the other without a break in the pipeline: loads (with head size 64 also K and V), scores and dP^T of
+// the next walk are under way while the last tile of this one is worked on, and dK, dV are stored behind
+// the exponentials of the next walk's first tile.  (A CTA per walk or two paid some 10000 cycles for
+// start, first loads and end, a quarter of the time at 16-tile walks.)
 // Per query tile, with everything transposed so that key rows sit on the TMEM lanes:
 //
 //   S^T  = K . Q^T                                              SS MMA into region R0
@@ -48,6 +51,7 @@ namespace boatcu {
 namespace attn_tc {
 
 constexpr int kBwdThreads = 448;
+constexpr int kBwdAnswers = 4;        // answers to requests for work in flight
 
 template <int HS>
 struct BwdCfg {
@@ -58,10 +62,11 @@ struct BwdCfg {
     // Q / dO stages: three when they fit (head size 64), so that the dO tile loaded behind a
     // dQ read-out is not needed before the tile after next
     static constexpr int Q_STAGES = HS == 64 ? 3 : 2;
+    static constexpr int KV_BUFS = HS == 64 ? 2 : 1;          // K and V of this walk, and of the next where they fit
     // K,V + Q,dO stages + dS^T + two (lse, delta) buffers + barriers.  With head size 128 this
-    // is 231,680 of the 232,448 bytes a CTA may have, so the base must come 1024-byte aligned
+    // is 231,808 of the 232,448 bytes a CTA may have, so the base must come 1024-byte aligned
     // from the launch (checked at kernel entry) - there is no room for manual alignment slack.
-    static constexpr int SMEM = 2 * TILE_BYTES + Q_STAGES * 2 * TILE_BYTES + DS_BYTES + 2048 + 256;
+    static constexpr int SMEM = KV_BUFS * 2 * TILE_BYTES + Q_STAGES * 2 * TILE_BYTES + DS_BYTES + 2048 + 384;
     // tensor memory columns
     // R0 (columns 0..127) holds S^T, then P^T.  With head size 64 dP^T has 128 columns of its
     // own.  With head size 128 nothing is left (R0 + dQ + dV + dK = 512), and dP^T borrows the dQ
@@ -84,8 +89,7 @@ struct BwdParams {
     void* dK;
     void* dV;
     int S, units, causal;
-    int group;             // units scheduled together, see the kernel
-    int pair;              // 1: a CTA walks two key tiles of its unit, 0: one
+    int group;             // units scheduled together, see bwd_walk
     float scale;
     unsigned int* status;
 };
@@ -97,6 +101,31 @@ __device__ __forceinline__ void named_barrier_sync(int id, int threads) {
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
+}
+
+struct BwdWalk {
+    int unit, jt;          // key tile
+    int i0, n;             // first query tile, number of them
+};
+
+// Walk `index` (n 0: none).  Walk order: units in groups of p.group; inside a group the key tile is the
+// slow index, longest walks first when causal.  The CTAs that run at the same time then belong to a few
+// (batch, head) units, so the FP32 dQ rows they reduce into (S*HS*4 bytes per unit) and the unit's Q and dO
+// stay in L2 - with key tiles as the slow index over all units, the dQ buffer of a large problem (268 MB
+// at 64 units x 8192 x 128) no longer fits and every reduction misses to HBM.
+__device__ __forceinline__ BwdWalk bwd_walk(const BwdParams& p, int index) {
+    BwdWalk w;
+    w.unit = w.jt = w.i0 = w.n = 0;
+    if (index < 0) return w;
+    const int n_tiles = (p.S + kTile - 1) / kTile;
+    const int per_group = p.group * n_tiles;
+    const int grp = index / per_group, rem = index - grp * per_group;
+    const int in_group = min(p.group, p.units - grp * p.group);
+    w.jt = rem / in_group;
+    w.unit = grp * p.group + rem % in_group;
+    w.i0 = p.causal ? w.jt : 0;
+    w.n = n_tiles - w.i0;
+    return w;
 }
 
 template <int HS>
@@ -111,14 +140,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         if (threadIdx.x == 0) atomicCAS(p.status, 0u, (unsigned int)kTimeoutOther + 100u);
         return;
     }
-    uint8_t* k_smem = smem;
-    uint8_t* v_smem = k_smem + C::TILE_BYTES;
-    uint8_t* q_smem = v_smem + C::TILE_BYTES;                          // [Q_STAGES]
+    uint8_t* kv_smem = smem;                                           // [KV_BUFS] K, V
+    uint8_t* q_smem = kv_smem + C::KV_BUFS * 2 * C::TILE_BYTES;        // [Q_STAGES]
     uint8_t* do_smem = q_smem + C::Q_STAGES * C::TILE_BYTES;           // [Q_STAGES]
     uint8_t* ds_smem = do_smem + C::Q_STAGES * C::TILE_BYTES;
     float* stat_s = (float*)(ds_smem + C::DS_BYTES);                   // [2][-lse*log2e[128], -delta/sqrt(hs)[128]]
     uint64_t* bars = (uint64_t*)(stat_s + 512);
-    uint64_t* kv_full = bars;                   // 1
+    uint64_t* kv_full = bars;                   // [KV_BUFS]
     uint64_t* q_full = bars + 16;               // [Q_STAGES] Q tile landed
     uint64_t* s_full = bars + 5;                // S^T complete
     uint64_t* ds_full = bars + 6;               // dS^T in smem (256 arrivals)
@@ -129,46 +157,24 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     uint64_t* do_full = bars + 19;              // [Q_STAGES] dO tile landed
     uint64_t* q_empty = bars + 22;              // [Q_STAGES] S^T and dK of the tile are complete: its Q stage is free
     uint64_t* p_full = bars + 3;                // P^T in TMEM (256 arrivals)
-    uint64_t* kv_empty = bars + 1;              // the first walk's MMAs are complete: K and V may be replaced
-    uint64_t* acc_free = bars + 2;              // dK, dV of the first walk are stored (256 arrivals)
+    uint64_t* kv_empty = bars + 26;             // [KV_BUFS] the walk's MMAs are complete: K and V may be replaced
+    uint64_t* acc_free = bars + 2;              // dK, dV of the walk are out of tensor memory (256 arrivals)
     uint64_t* stat_full = bars + 11;            // [2] the tile's statistics landed
     uint64_t* stat_empty = bars + 13;           // [2] phase B of the tile is over (256 arrivals)
-    uint32_t* tmem_slot = (uint32_t*)(bars + 25);
-    volatile uint32_t* drain_ok = tmem_slot + 3;       // same idea for the dQ warps
+    uint64_t* work_full = bars + 28;            // [kBwdAnswers] the answer to a request for work is there
+    uint64_t* work_empty = bars + 32;           // [kBwdAnswers] producer, MMA issuer, softmax and dQ warps have read it
+    uint8_t* answers = (uint8_t*)(bars + 36);   // [kBwdAnswers] 16 bytes
+    uint32_t* tmem_slot = (uint32_t*)(bars + 44);
+    volatile uint32_t* drain_ok = tmem_slot + 3;       // outcome of the dQ warps' wait
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
-    // CTA order: units in groups of p.group; inside a group the key-tile pair is the slow index.
-    // The CTAs that run at the same time then belong to a few (batch, head) units, so the FP32 dQ
-    // rows they reduce into (S*HS*4 bytes per unit) and the unit's Q and dO stay in L2 - with
-    // key tiles as the slow index over all units, the dQ buffer of a large problem (268 MB at 64
-    // units x 8192 x 128) no longer fits and every reduction misses to HBM.
-    // A CTA walks two key tiles of its unit, one after the other: with a causal mask tile pj and
-    // tile n_tiles-1-pj, whose walks together are n_tiles+1 query tiles for every pj, so all CTAs
-    // carry the same load; without a mask two neighbouring tiles.  Start-up, the last tile's
-    // read-out and the exit of a CTA are paid once per pair, and the second walk starts while the
-    // first one's dQ is still draining.
-    // (p.pair == 0: one walk per CTA - better when the walks are long or the CTAs few, see the
-    // launcher.)
-    const int n_pairs = p.pair ? (n_tiles + 1) / 2 : n_tiles;
-    const int per_group = p.group * n_pairs;
-    const int grp = blockIdx.x / per_group;
-    const int rem = blockIdx.x - grp * per_group;
-    const int in_group = min(p.group, p.units - grp * p.group);
-    const int pj = rem / in_group;
-    const int unit = grp * p.group + rem % in_group;
-    const int jtA = !p.pair || p.causal ? pj : 2 * pj;
-    const int jtB = p.causal ? n_tiles - 1 - pj : 2 * pj + 1;
-    const bool has_b = p.pair && jtB != jtA && jtB < n_tiles;
-    const int ibA = p.causal ? jtA : 0, ibB = p.causal ? jtB : 0;
-    const int nA = n_tiles - ibA;                       // query tiles of the first walk
-    const int n_q = nA + (has_b ? n_tiles - ibB : 0);   // of both
-    const int64_t stat_base = (int64_t)unit * n_tiles * kTile;    // the statistics are padded to whole tiles
-    // query tile and key tile of step gt of the combined walk
-    auto qtile = [&](int gt) { return gt < nA ? ibA + gt : ibB + gt - nA; };
 
     if (threadIdx.x == 0) {
-        mbar_init(kv_full, 1);
+        for (int b = 0; b < C::KV_BUFS; ++b) {
+            mbar_init(&kv_full[b], 1);
+            mbar_init(&kv_empty[b], 1);
+        }
         for (int s = 0; s < C::Q_STAGES; ++s) {
             mbar_init(&q_full[s], 1);
             mbar_init(&do_full[s], 1);
@@ -181,8 +187,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         mbar_init(dq_full, 1);
         mbar_init(dq_empty, 1);
         mbar_init(all_done, 1);
-        mbar_init(kv_empty, 1);
         mbar_init(acc_free, 256);
+        for (int b = 0; b < kBwdAnswers; ++b) {
+            mbar_init(&work_full[b], 1);
+            mbar_init(&work_empty[b], 14);
+        }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&stat_full[b], 1);
             mbar_init(&stat_empty[b], 256);
@@ -193,21 +202,6 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         tma_prefetch_desc(&map_v);
         tma_prefetch_desc(&map_do);
         tma_prefetch_desc(&map_dq);
-        griddep_sync();
-        // This thread is also the producer: the loads that wait for nothing - K and V of the first
-        // walk, dO of the first Q_STAGES query tiles (later ones are loaded by the dQ warps, which
-        // stage dQ through the dO buffers and know when one is free again) - start here, under the
-        // tensor-memory allocation and the CTA's first barrier.
-        mbar_arrive_expect_tx(kv_full, 2 * C::TILE_BYTES);
-        for (int b = 0; b < C::NBOX; ++b) {
-            tma_load_3d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 64, jtA * kTile, unit);
-            tma_load_3d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 64, jtA * kTile, unit);
-        }
-        for (int t = 0; t < n_q && t < C::Q_STAGES; ++t) {
-            mbar_arrive_expect_tx(&do_full[t], C::TILE_BYTES);
-            for (int b = 0; b < C::NBOX; ++b)
-                tma_load_3d(do_smem + t * C::TILE_BYTES + b * kBoxBytes, &map_do, &do_full[t], b * 64, qtile(t) * kTile, unit);
-        }
     }
     if (warp == 1) tmem_alloc(tmem_slot, C::TMEM_COLS);
     griddep_sync();
@@ -216,32 +210,57 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
+    // Walk r + 1 of this CTA: the answer to the request made during walk r (whole warps).
+    auto next_walk = [&](int r, unsigned int code, bool& ok) -> BwdWalk {
+        const int a = r % kBwdAnswers;
+        if (!mbar_wait_warp(&work_full[a], (r / kBwdAnswers) & 1, p.status, code)) {
+            ok = false;
+            return bwd_walk(p, -1);
+        }
+        const int index = taken_cta(answers + a * 16);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&work_empty[a]);
+        return bwd_walk(p, index);
+    };
+
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
+        // ---------------- TMA producer, and the one who asks for work ----------------
         if (lane == 0) {
-            auto load_kv = [&](int jt) {
-                mbar_arrive_expect_tx(kv_full, 2 * C::TILE_BYTES);
+            bool ok = true;
+            uint32_t t = 0;                                  // tiles so far, of all walks
+            BwdWalk w = bwd_walk(p, blockIdx.x);
+            for (int r = 0; ok && w.n > 0; ++r) {
+                const int a = r % kBwdAnswers;
+                if (!mbar_wait(&work_empty[a], ((r / kBwdAnswers) & 1) ^ 1, p.status, kTimeoutProducer)) break;
+                mbar_arrive_expect_tx(&work_full[a], 16);
+                request_next_cta(answers + a * 16, &work_full[a]);
+                const int kb = r % C::KV_BUFS;
+                uint8_t* k_dst = kv_smem + kb * 2 * C::TILE_BYTES;
+                if (!mbar_wait(&kv_empty[kb], ((r / C::KV_BUFS) & 1) ^ 1, p.status, kTimeoutProducer)) break;
+                mbar_arrive_expect_tx(&kv_full[kb], 2 * C::TILE_BYTES);
                 for (int b = 0; b < C::NBOX; ++b) {
-                    tma_load_3d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 64, jt * kTile, unit);
-                    tma_load_3d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 64, jt * kTile, unit);
+                    tma_load_3d(k_dst + b * kBoxBytes, &map_k, &kv_full[kb], b * 64, w.jt * kTile, w.unit);
+                    tma_load_3d(k_dst + C::TILE_BYTES + b * kBoxBytes, &map_v, &kv_full[kb], b * 64, w.jt * kTile, w.unit);
                 }
-            };
-            for (int t = 0; t < n_q; ++t) {
-                if (t == nA) {                  // second walk: its K and V, once the first walk's MMAs are done
-                    if (!mbar_wait(kv_empty, 0, p.status, kTimeoutProducer)) break;
-                    load_kv(jtB);
+                const int64_t stat_base = (int64_t)w.unit * n_tiles * kTile;    // the statistics are padded to whole tiles
+                for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
+                    const int s = t % C::Q_STAGES;
+                    if (!mbar_wait(&q_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+                    mbar_arrive_expect_tx(&q_full[s], C::TILE_BYTES);
+                    for (int b = 0; b < C::NBOX; ++b)
+                        tma_load_3d(q_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[s], b * 64, i * kTile, w.unit);
+                    // the tile's 128 exponent offsets and 128 deltas, into the buffer of its parity once
+                    // the tile before last has left it
+                    if (!mbar_wait(&stat_empty[t & 1], ((t >> 1) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+                    mbar_arrive_expect_tx(&stat_full[t & 1], 1024);
+                    bulk_load_1d(stat_s + (t & 1) * 256, p.lse2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
+                    bulk_load_1d(stat_s + (t & 1) * 256 + 128, p.delta2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
                 }
-                const int s = t % C::Q_STAGES;
-                if (!mbar_wait(&q_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) break;
-                mbar_arrive_expect_tx(&q_full[s], C::TILE_BYTES);
-                for (int b = 0; b < C::NBOX; ++b)
-                    tma_load_3d(q_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[s], b * 64, qtile(t) * kTile, unit);
-                // the tile's 128 exponent offsets and 128 deltas, into the buffer of its parity once
-                // the tile before last has left it
-                if (!mbar_wait(&stat_empty[t & 1], ((t >> 1) & 1) ^ 1, p.status, kTimeoutProducer)) break;
-                mbar_arrive_expect_tx(&stat_full[t & 1], 1024);
-                bulk_load_1d(stat_s + (t & 1) * 256, p.lse2 + stat_base + qtile(t) * kTile, 512, &stat_full[t & 1]);
-                bulk_load_1d(stat_s + (t & 1) * 256 + 128, p.delta2 + stat_base + qtile(t) * kTile, 512, &stat_full[t & 1]);
+                if (!ok || !mbar_wait(&work_full[a], (r / kBwdAnswers) & 1, p.status, kTimeoutProducer)) break;
+                w = bwd_walk(p, taken_cta(answers + a * 16));
+                fence_proxy_async_smem();
+                mbar_arrive(&work_empty[a]);
             }
         }
     } else if (warp == 1) {
@@ -253,11 +272,11 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             constexpr uint32_t idesc_acc = make_idesc(kBF16, false, true, kTile, HS);      // dV, dK
             constexpr uint32_t idesc_dq = make_idesc(kBF16, true, true, kTile, HS);        // dQ
             const bool leader = elect_one();
-            const uint64_t k_desc = smem_desc_sw128(smem_u32(k_smem), 16, 1024), v_desc = smem_desc_sw128(smem_u32(v_smem), 16, 1024);
+            const uint64_t k_desc = smem_desc_sw128(smem_u32(kv_smem), 16, 1024), v_desc = k_desc + (C::TILE_BYTES >> 4);
             const uint64_t q_desc = smem_desc_sw128(smem_u32(q_smem), 16, 1024), do_desc = smem_desc_sw128(smem_u32(do_smem), 16, 1024);
             const uint64_t ds_desc = smem_desc_sw128(smem_u32(ds_smem), 16, 1024);
             // the same tiles read along their rows
-            const uint64_t k_mn = smem_desc_mn(smem_u32(k_smem), kBoxBytes, false), q_mn = smem_desc_mn(smem_u32(q_smem), kBoxBytes, false);
+            const uint64_t k_mn = smem_desc_mn(smem_u32(kv_smem), kBoxBytes, false), q_mn = smem_desc_mn(smem_u32(q_smem), kBoxBytes, false);
             const uint64_t do_mn = smem_desc_mn(smem_u32(do_smem), kBoxBytes, false), ds_mn = smem_desc_mn(smem_u32(ds_smem), kBoxBytes, false);
             // Issue order on the (in-order) tensor pipe, per tile t:
             //   dV(t) S(t+1) | dQ(t) dK(t) | dP(t+1)
@@ -266,107 +285,118 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             // next tile follows them: into its own columns (head size 64), or into the dQ columns
             // once the dQ warps have taken this tile's dQ out of them (head size 128) - in both
             // cases long before phase B of the next tile asks for it.
-            auto issue_s = [&](int t) -> bool {
+            // the last argument is the K/V buffer of the tile's walk
+            auto issue_s = [&](uint32_t t, int kb) -> bool {
                 const int s = t % C::Q_STAGES;
                 if (!mbar_wait_warp(&q_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) return false;
                 tc_fence_after_sync();
-                const uint64_t qd = q_desc + (s * C::TILE_BYTES >> 4);
+                const uint64_t qd = q_desc + (s * C::TILE_BYTES >> 4), kd = k_desc + (kb * 2 * C::TILE_BYTES >> 4);
                 if (leader) {
 #pragma unroll
                     for (int kk = 0; kk < C::ROWB / 32; ++kk) {
                         const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
-                        mma_ss<false>(tmem_base + C::COL_S, k_desc + off, qd + off, idesc_st, kk > 0);
+                        mma_ss<false>(tmem_base + C::COL_S, kd + off, qd + off, idesc_st, kk > 0);
                     }
                     mma_commit(s_full);
                 }
                 return true;
             };
-            auto issue_dp = [&](int t) -> bool {        // dP^T = V . dO^T
+            auto issue_dp = [&](uint32_t t, int kb) -> bool {        // dP^T = V . dO^T
                 const int s = t % C::Q_STAGES;
                 if (!mbar_wait_warp(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) return false;
                 tc_fence_after_sync();
-                const uint64_t dod = do_desc + (s * C::TILE_BYTES >> 4);
+                const uint64_t dod = do_desc + (s * C::TILE_BYTES >> 4), vd = v_desc + (kb * 2 * C::TILE_BYTES >> 4);
                 if (leader) {
 #pragma unroll
                     for (int kk = 0; kk < C::ROWB / 32; ++kk) {
                         const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
-                        mma_ss<false>(tmem_base + C::COL_DP, v_desc + off, dod + off, idesc_st, kk > 0);
+                        mma_ss<false>(tmem_base + C::COL_DP, vd + off, dod + off, idesc_st, kk > 0);
                     }
                     mma_commit(dp_full);
                 }
                 return true;
             };
-            bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutMma);
-            ok = ok && issue_s(0);
-            ok = ok && issue_dp(0);
-            for (int t = 0; t < n_q && ok; ++t) {
-                const int s = t % C::Q_STAGES;
-                const bool first = t == 0 || t == nA;           // first tile of a walk: dK, dV start over
-                const bool early_next = t + 1 < n_q && t + 1 != nA;   // the next tile belongs to the same walk
-                const uint64_t q_d = q_mn + (s * C::TILE_BYTES >> 4), do_d = do_mn + (s * C::TILE_BYTES >> 4);
-                if (t == nA) {
-                    // second walk: wait for its K and V, then the MMAs a walk begins with.  R0 (and with
-                    // head size 64 the dP^T columns) are free: phase B of the previous tile is over.
-                    if (!mbar_wait_warp(kv_full, 1, p.status, kTimeoutMma)) { ok = false; break; }
-                    if (!issue_s(t)) { ok = false; break; }
-                    // the first walk's last dQ must be out of the columns dP^T borrows
-                    if (!C::DP_OWN && !mbar_wait_warp(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                    if (!issue_dp(t)) { ok = false; break; }
-                }
-                if (!mbar_wait_warp(p_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                if (!mbar_wait_warp(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                if (t == nA && !mbar_wait_warp(acc_free, 0, p.status, kTimeoutMma)) { ok = false; break; }
-                tc_fence_after_sync();
-                if (leader) {
-#pragma unroll
-                    for (int kk = 0; kk < kTile / 16; ++kk)      // dV += P^T . dO      (K = 128 query rows)
-                        mma_ts<false>(tmem_base + C::COL_DV, tmem_base + C::COL_S + (kk / 4) * 64 + (kk % 4) * 8,
-                                      do_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
-                }
-                // R0 is free as soon as dV, ahead on the pipe, has read P^T
-                if (early_next && !issue_s(t + 1)) { ok = false; break; }
-                if (!mbar_wait_warp(ds_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                if (t > 0) {
-                    // the previous dQ must have left its TMEM columns
-                    if (!mbar_wait_warp(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                }
-                tc_fence_after_sync();
-                // dQ first: its completion starts the read-out, whose first step (tensor memory ->
-                // registers) gates the next tile's dP^T when that borrows the dQ columns; dK runs
-                // on the pipe meanwhile.  This tile's dO stage was last read by dV and dP^T, which
-                // are ahead of dQ on the pipe, so it is free for the read-out's staging at dq_full.
-                if (leader) {
-#pragma unroll
-                    for (int kk = 0; kk < kTile / 16; ++kk)      // dQ_i = dS . K        (K = 128 key rows)
-                        mma_ss<false>(tmem_base + C::COL_DQ, ds_mn + (kk * 2048 >> 4), k_mn + (kk * 2048 >> 4), idesc_dq, kk > 0);
-                    mma_commit(dq_full);
-#pragma unroll
-                    for (int kk = 0; kk < kTile / 16; ++kk) {    // dK += dS^T . Q
-                        const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
-                        mma_ss<false>(tmem_base + C::COL_DK, ds_desc + off, q_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
-                    }
-                    mma_commit(&q_empty[s]);  // also: the dS^T tile is no longer read
-                    if (t == nA - 1 && has_b) {
-                        mma_commit(kv_empty);                   // K and V of the first walk are no longer read
-                        mma_commit(all_done);                   // and its dK, dV are complete
-                    }
-                }
-                // dS^T of tile t is in shared memory, so the softmax warps are done with dP^T(t)
-                if (early_next) {
-                    // borrowed columns: this tile's dQ, just issued, has to complete and leave them first
-                    if (!C::DP_OWN && !mbar_wait_warp(dq_empty, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
-                    if (!issue_dp(t + 1)) { ok = false; break; }
-                }
+            bool ok = true;
+            uint32_t t = 0;                                  // tiles so far, of all walks
+            BwdWalk w = bwd_walk(p, blockIdx.x);
+            if (w.n > 0) {
+                ok = mbar_wait_warp(&kv_full[0], 0, p.status, kTimeoutMma);
+                ok = ok && issue_s(0, 0);
+                ok = ok && issue_dp(0, 0);
             }
-            if (ok && leader) mma_commit(all_done);
+            for (int r = 0; ok && w.n > 0; ++r) {
+                const int kb = r % C::KV_BUFS;
+                const BwdWalk next = next_walk(r, kTimeoutMma, ok);
+                const uint64_t k_d = k_mn + (kb * 2 * C::TILE_BYTES >> 4);
+                for (int i = 0; i < w.n && ok; ++i, ++t) {
+                    const int s = t % C::Q_STAGES;
+                    const bool first = i == 0;                       // first tile of a walk: dK, dV start over
+                    const bool last = i == w.n - 1;
+                    const bool more = !last || next.n > 0;           // there is a tile t+1
+                    // ... whose scores may be issued now: it uses the same K and V, or K and V have a second buffer
+                    const bool early = more && (!last || C::KV_BUFS == 2);
+                    const int kb_next = last ? (r + 1) % C::KV_BUFS : kb;
+                    const uint64_t q_d = q_mn + (s * C::TILE_BYTES >> 4), do_d = do_mn + (s * C::TILE_BYTES >> 4);
+                    auto next_s = [&]() -> bool {                    // S of tile t+1, the K and V of its walk first
+                        if (last && !mbar_wait_warp(&kv_full[kb_next], ((r + 1) / C::KV_BUFS) & 1, p.status, kTimeoutMma)) return false;
+                        return issue_s(t + 1, kb_next);
+                    };
+                    if (!mbar_wait_warp(p_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (!mbar_wait_warp(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    // the previous walk's dK, dV must have left tensor memory
+                    if (first && r > 0 && !mbar_wait_warp(acc_free, (r - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    tc_fence_after_sync();
+                    if (leader) {
+#pragma unroll
+                        for (int kk = 0; kk < kTile / 16; ++kk)      // dV += P^T . dO      (K = 128 query rows)
+                            mma_ts<false>(tmem_base + C::COL_DV, tmem_base + C::COL_S + (kk / 4) * 64 + (kk % 4) * 8,
+                                          do_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
+                    }
+                    // R0 is free as soon as dV, ahead on the pipe, has read P^T
+                    if (early && !next_s()) { ok = false; break; }
+                    if (!mbar_wait_warp(ds_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (t > 0) {
+                        // the previous dQ must have left its TMEM columns
+                        if (!mbar_wait_warp(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    }
+                    tc_fence_after_sync();
+                    // dQ first: its completion starts the read-out, whose first step (tensor memory ->
+                    // registers) gates the next tile's dP^T when that borrows the dQ columns; dK runs
+                    // on the pipe meanwhile.  This tile's dO stage was last read by dV and dP^T, which
+                    // are ahead of dQ on the pipe, so it is free for the read-out's staging at dq_full.
+                    if (leader) {
+#pragma unroll
+                        for (int kk = 0; kk < kTile / 16; ++kk)      // dQ_i = dS . K        (K = 128 key rows)
+                            mma_ss<false>(tmem_base + C::COL_DQ, ds_mn + (kk * 2048 >> 4), k_d + (kk * 2048 >> 4), idesc_dq, kk > 0);
+                        mma_commit(dq_full);
+#pragma unroll
+                        for (int kk = 0; kk < kTile / 16; ++kk) {    // dK += dS^T . Q
+                            const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
+                            mma_ss<false>(tmem_base + C::COL_DK, ds_desc + off, q_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
+                        }
+                        mma_commit(&q_empty[s]);  // also: the dS^T tile is no longer read
+                        if (last) {
+                            mma_commit(&kv_empty[kb]);              // K and V of the walk are no longer read
+                            mma_commit(all_done);                   // and its dK, dV are complete
+                        }
+                    }
+                    if (more && !early && !next_s()) { ok = false; break; }
+                    // dS^T of tile t is in shared memory, so the softmax warps are done with dP^T(t)
+                    if (more) {
+                        // borrowed columns: this tile's dQ, just issued, has to complete and leave them first
+                        if (!C::DP_OWN && !mbar_wait_warp(dq_empty, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                        if (!issue_dp(t + 1, kb_next)) { ok = false; break; }
+                    }
+                }
+                w = next;
+            }
         }
     } else if (warp < 10) {
         // ---------------- softmax / dS: warps 2..9 ----------------
         // thread = (key row r, half h of the 128 query columns); the two warps that share a
         // TMEM lane group each own 64 columns.
-        const int w = warp - 2;
         const int lane_group = warp & 3;
-        const int half = w >> 2;
+        const int half = (warp - 2) >> 2;
         const int r = lane_group * 32 + lane;                       // key row inside the tile
         const uint32_t lane_addr = (uint32_t)(lane_group * 32) << 16;
         const uint32_t col0 = 64u * half;                           // first query column of this thread
@@ -380,7 +410,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // gives up, the thread leaves the loop; the others see the status word at their next wait
         // and follow.
         // dK, dV of a finished walk: the first four warps store dV, the other four dK.
-        auto store_dkdv = [&](int jt, uint32_t phase) -> bool {
+        auto store_dkdv = [&](int unit, int jt, uint32_t phase) -> bool {
             if (!mbar_wait_warp(all_done, phase, p.status, kTimeoutEpilogue)) return false;
             tc_fence_after_sync();
             const int64_t grow = (int64_t)unit * p.S + (int64_t)jt * kTile + r;
@@ -405,9 +435,12 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             }
             return true;
         };
-        auto key_live = [&](int t) { return (t < nA ? jtA : jtB) * kTile + r < p.S; };
-        for (int t = 0; t < n_q; ++t) {
-            const int i = qtile(t);
+        uint32_t t = 0;                                             // tiles so far, of all walks
+        int jt_before = -1, unit_before = 0;                        // walk whose dK, dV are still to be stored
+        BwdWalk w = bwd_walk(p, blockIdx.x);
+        for (int r_walk = 0; ok && w.n > 0; ++r_walk) {
+        const bool key_live = w.jt * kTile + r < p.S;
+        for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
             // -lse*log2e and -delta/sqrt(hs) of this query tile, put into the buffer of this tile's
             // parity by the producer
             const float* lse_s = stat_s + (t & 1) * 256;
@@ -415,7 +448,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (!mbar_wait_warp(&stat_full[t & 1], (t >> 1) & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
             if (!mbar_wait_warp(s_full, t & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
             tc_fence_after_sync();
-            const bool diag = p.causal && i == (t < nA ? jtA : jtB);
+            const bool diag = p.causal && i == w.jt;
             // ---- phase A: P^T = exp2(S^T*c - lse) for this thread's 64 columns ----
             uint32_t ph[32];                                        // 64 probabilities as BF16 pairs
             {
@@ -463,7 +496,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 else      phase_a(std::false_type{});
                 // A key row beyond the end of the sequence has zero scores, whose exp2(-lse) may overflow;
                 // its dS^T meets a zero row of K, so it has to be a number.
-                if (!key_live(t)) {
+                if (!key_live) {
 #pragma unroll
                     for (int x = 0; x < 32; ++x) ph[x] = 0u;
                 }
@@ -473,6 +506,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             tmem_wait_st();
             tc_fence_before_sync();
             mbar_arrive(p_full);
+            if (i == w.i0 && jt_before >= 0) {
+                // dK, dV of the previous walk leave tensor memory before this one's first dV and dK start
+                // them over; behind its phase A they have been complete for a while
+                if (!store_dkdv(unit_before, jt_before, (r_walk - 1) & 1)) { ok = false; break; }
+                tc_fence_before_sync();
+                mbar_arrive(acc_free);
+            }
             // ---- phase B: dS^T = P^T * (dP^T - delta) / sqrt(hs) ----
             if (!mbar_wait_warp(dp_full, t & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
             tc_fence_after_sync();
@@ -510,16 +550,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             fence_proxy_async_smem();
             mbar_arrive(ds_full);
             mbar_arrive(&stat_empty[t & 1]);                 // this tile's statistics are no longer read
-            if (t == nA - 1 && has_b) {
-                // end of the first walk: its dK, dV leave tensor memory before the second walk's first
-                // dV and dK MMAs start them over
-                if (!store_dkdv(jtA, 0u)) { ok = false; break; }
-                tc_fence_before_sync();
-                mbar_arrive(acc_free);
-            }
         }
-        // final: dK, dV of the walk that ended last
-        if (ok) store_dkdv(has_b ? jtB : jtA, has_b ? 1u : 0u);
+        jt_before = w.jt;
+        unit_before = w.unit;
+        if (!ok) break;
+        w = next_walk(r_walk, kTimeoutSoftmax, ok);
+        if (ok && w.n == 0) store_dkdv(unit_before, jt_before, r_walk & 1);
+        }
     } else {
         // ---------------- dQ reduction: warps 10..13, thread = query row ----------------
         // The FP32 dQ tile is HS/32 boxes of 128 rows x 128 bytes (16 KB each), twice what the tile's
@@ -539,13 +576,41 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (n == 0) tma_wait_group_read0();
             else tma_wait_group_read1();
         };
-        for (int t = 0; t < n_q; ++t) {
+        // dO tiles: the first Q_STAGES are loaded here, every later one into the stage of the tile
+        // Q_STAGES before it
+        int ahead_r = 0, ahead_i = 0;                        // walk and tile of the next dO load
+        BwdWalk ahead = bwd_walk(p, blockIdx.x);
+        auto load_do = [&](uint32_t t_load, auto before_box) {
+            if (ahead.n == 0) return;
+            const int s = t_load % C::Q_STAGES;
+            mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
+            for (int b = 0; b < C::NBOX; ++b) {
+                before_box(b);
+                tma_load_3d(do_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_do, &do_full[s], b * 64, (ahead.i0 + ahead_i) * kTile, ahead.unit);
+            }
+            if (++ahead_i == ahead.n) {
+                // ahead of the warp's own reading of this answer, so it is still there
+                const int a = ahead_r % kBwdAnswers;
+                const bool there = mbar_wait(&work_full[a], (ahead_r / kBwdAnswers) & 1, p.status, kTimeoutOther);
+                ahead = bwd_walk(p, there ? taken_cta(answers + a * 16) : -1);
+                ahead_i = 0;
+                ++ahead_r;
+            }
+        };
+        if (tid128 == 0)
+            for (uint32_t t0 = 0; t0 < C::Q_STAGES; ++t0) load_do(t0, [](int) {});
+        __syncwarp();
+        bool ok = true;
+        uint32_t t = 0;                                      // tiles so far, of all walks
+        BwdWalk w = bwd_walk(p, blockIdx.x);
+        for (int r_walk = 0; ok && w.n > 0; ++r_walk) {
+        for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
             const int s = t % C::Q_STAGES;
             if (tid128 == 0) drain_ok[0] = mbar_wait(dq_full, t & 1, p.status, kTimeoutOther) ? 1u : 0u;
             named_barrier_sync(2, 128);
-            if (drain_ok[0] == 0u) break;
+            if (drain_ok[0] == 0u) { ok = false; break; }
             tc_fence_after_sync();
-            const int y = qtile(t) * kTile;
+            const int y = i * kTile;
             uint8_t* stage = do_smem + s * C::TILE_BYTES;
             auto stage_box = [&](const uint32_t (&v)[32], int slot) {
                 uint8_t* row = stage + slot * kBoxBytes + r * 128;
@@ -564,7 +629,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             named_barrier_sync(2, 128);
             if (tid128 == 0) {
                 for (int b = 0; b < C::NBOX; ++b) {
-                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, b * 32, y, unit);
+                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, b * 32, y, w.unit);
                     tma_commit_group();
                 }
             }
@@ -585,17 +650,16 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 fence_proxy_async_smem();
                 named_barrier_sync(2, 128);
                 if (tid128 == 0) {
-                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, (C::NBOX + b) * 32, y, unit);
+                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, (C::NBOX + b) * 32, y, w.unit);
                     tma_commit_group();
                 }
             }
-            if (tid128 == 0 && t + C::Q_STAGES < n_q) {
-                mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
-                for (int b = 0; b < C::NBOX; ++b) {
-                    wait_read(C::NBOX - 1 - b);             // the last group that used slot b has been read
-                    tma_load_3d(stage + b * kBoxBytes, &map_do, &do_full[s], b * 64, qtile(t + C::Q_STAGES) * kTile, unit);
-                }
-            }
+            // the last group that used slot b has been read
+            if (tid128 == 0) load_do(t + C::Q_STAGES, [&](int b) { wait_read(C::NBOX - 1 - b); });
+            __syncwarp();
+        }
+        if (!ok) break;
+        w = next_walk(r_walk, kTimeoutOther, ok);
         }
         // The CTA may end once the reductions have read their shared-memory source; that they have
         // landed in global memory by the time the next kernel runs is the grid's completion.

@@ -101,17 +101,6 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     const int64_t unit_bytes = S * HS * 16;
     int64_t group = (64ll << 20) / unit_bytes;
     p.group = (int)(group < 1 ? 1 : (group > units ? units : group));
-    // Two walks per CTA halve what a CTA pays once (start-up, the last tile's read-out, exit) and
-    // equalise the CTAs when causal: 5-10 % at 8- and 16-tile walks.  With equal CTAs the last
-    // wave is a loss that many short CTAs would fill, and at 64-tile walks the per-CTA cost is
-    // small anyway (measured: no gain at 64 tiles, 10 % slower when only 3.5 waves of pairs exist).
-    p.pair = (n_tiles <= 32 && units * ((n_tiles + 1) / 2) >= 8 * (int64_t)sm_count()) ? 1 : 0;
-    {
-        // BOAT_BWD_PAIR=0/1 in the environment overrides the rule; it is read at every launch so
-        // that one test process can run both schedules on the same problem
-        const char* e = getenv("BOAT_BWD_PAIR");
-        if (e && (e[0] == '0' || e[0] == '1')) p.pair = e[0] - '0';
-    }
     p.scale = scale;
     p.status = kernel_status_ptr();
     auto kern = attn_bwd_tc_kernel<HS>;
@@ -129,7 +118,7 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     {
         ProfileScope prof("attn_bwd_tc");
         BOATCU_CHECK(cudaMemsetAsync(dq_accum, 0, n * sizeof(float), stream()));
-        const int64_t grid = units * (p.pair ? (n_tiles + 1) / 2 : n_tiles);
+        const int64_t grid = units * n_tiles;           // one CTA per walk; those on the SMs take the others over
         BOATCU_RUN(kern, (unsigned)grid, kBwdThreads, C::SMEM, mq, mk, mv, mdo, mdq, p);
         BOATCU_LAUNCH_OK("attn_bwd_tc");
         // the summed FP32 contributions become the BF16 output
