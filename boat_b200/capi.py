@@ -226,11 +226,14 @@ PROTOTYPES = {
     "boat_cuda_attn_bwd_static": (_I, [_I, _I64, _I64, _I64, _I, _F, _P, _P, _P, _P, _P, _P, _I, _P, _P, _P]),
     "boat_cuda_gemm_set_yielding": (_I, [_I]),
     "boat_cuda_gemm_grouped": (_I, [_I, _I, _I, _I, _I64, _I64, _I64, _P, _I64, _P, _I64, _I, _P, _I64, _I, _P]),
-    "boat_cuda_weight_grads": (_I, [_I, _I, _I64, _I64, _I64, _P, _P, _I, _P, _P]),
+    "boat_cuda_gemm_fused": (_I, [_I, _I, _I, _I, _I64, _I64, _I64, _P, _I64, _P, _I64, _I, _P, _I64, _P, _P]),
+    "boat_cuda_gemm_sum": (_I, [_I, _I, _I, _I, _I64, _I64, _I64, _P, _I64, _P, _I64, _I, _P, _I64, _I]),
+    "boat_cuda_weight_grads": (_I, [_I, _I, _I64, _I64, _I64, _P, _P, _I, _P, _P, _I]),
     "boat_cuda_colsum": (_I, [_P, _I, _I64, _I64, _P]),
     "boat_cuda_colsum_multi": (_I, [_P, _I, _I64, _I64, _P, _I]),
     "boat_cuda_convert_multi": (_I, [_P, _I, _P, _P, _I]),
     "boat_cuda_axpy": (_I, [_P, _P, _F, _I64]),
+    "boat_cuda_sgd_clear": (_I, [_P, _P, _F, _P, _I]),
     "boat_cuda_axpy_multi": (_I, [_P, _P, _F, _P, _I]),
     "boat_cuda_scale": (_I, [_P, _P, _F, _I64]),
     "boat_cuda_add_bias": (_I, [_P, _P, _P, _I64, _I64]),
@@ -241,6 +244,7 @@ PROTOTYPES = {
     "boat_cuda_transpose": (_I, [_P, _P, _I64, _I64, _I64]),
     "boat_cuda_layernorm_fwd": (_I, [_P, _I, _I64, _I64, _P, _P, _F, _P, _P, _P]),
     "boat_cuda_layernorm_bwd": (_I, [_P, _P, _I, _I64, _I64, _P, _P, _P, _P, _P, _P]),
+    "boat_cuda_layernorm_bwd_add": (_I, [_P, _P, _I, _I64, _I64, _P, _P, _P, _P, _P, _P, _P]),
     "boat_cuda_gelu_fwd": (_I, [_P, _P, _I, _I64]),
     "boat_cuda_gelu_bwd": (_I, [_P, _P, _P, _I, _I64]),
     "boat_cuda_adam_step": (_I, [_I, _P, _P, _P, _P, _P, _F, _F, _F, _F, _F, _F]),

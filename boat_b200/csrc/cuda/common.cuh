@@ -107,10 +107,13 @@ int rowdot_stats(const void* dO, const void* O, int type, int64_t units, int64_t
 
 // CUDA-core (exact FP32 accumulate) implementations, any shape.
 // gemm_simt_grouped: up to four problems of one shape in one launch; bias may be NULL or hold NULLs; with
-// `colsum` (may be NULL or hold NULLs) problem g also writes the sums of B's columns over K.
+// `colsum` (may be NULL or hold NULLs) problem g also writes the sums of B's columns over K.  `add`: both are
+// added to what is there (FP32 output).
 int gemm_simt_grouped(int trans_a, int trans_b, int groups, int64_t M, int64_t N, int64_t K, const void* const* A,
                       int64_t lda, const void* const* B, int64_t ldb, int in_type, void* const* C, int64_t ldc,
-                      int out_type, const float* const* bias, float* const* colsum);
+                      int out_type, const float* const* bias, float* const* colsum, bool add = false);
+// boat_cuda_colsum_multi, with `add` adding to the outputs.
+int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count, bool add);
 int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, int io_type, void* O, float* lse);
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
@@ -130,6 +133,16 @@ bool gemm_tc_supported(int mma, int trans_a, int trans_b, int64_t M, int64_t N, 
                        int out_type);
 int gemm_tc(int mma, int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
             const void* B, int64_t ldb, int in_type, void* C, int64_t ldc, int out_type, const float* bias);
+// C += op(A).op(B), FP32 output.
+int gemm_tc_accumulate(int mma, int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
+                       const void* B, int64_t ldb, float* C, int64_t ldc);
+// C = sum over the groups of op(A[g]).op(B[g]), one accumulator.
+int gemm_tc_sum(int mma, int trans_a, int trans_b, int groups, int64_t M, int64_t N, int64_t K, const void* const* A,
+                int64_t lda, const void* const* B, int64_t ldb, void* C, int64_t ldc, int out_type);
+// BF16 products with element-wise work in the epilogue (BOAT_EPI_*); aux is laid out like C.
+bool gemm_tc_fused_supported(int epilogue, int trans_a, int trans_b);
+int gemm_tc_fused(int epilogue, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb,
+                  void* C, int64_t ldc, const float* bias, void* aux);
 void gemm_tc_set_yielding(bool on);
 // `groups` (1..4) problems of one shape, layout and type in one launch; bias may be NULL or hold NULLs.
 int gemm_tc_grouped(int mma, int trans_a, int trans_b, int groups, int64_t M, int64_t N, int64_t K,

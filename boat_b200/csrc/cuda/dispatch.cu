@@ -81,22 +81,59 @@ int boat_cuda_gemm_grouped(int mma, int ta, int tb, int groups, int64_t M, int64
     return 0;
 }
 
+int boat_cuda_gemm_fused(int mma, int epilogue, int ta, int tb, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
+                         const void* B, int64_t ldb, int type, void* C, int64_t ldc, const float* bias, void* aux) {
+    if (epilogue < BOAT_EPI_GELU || epilogue > BOAT_EPI_ADD) return set_error(10, "boat_cuda_gemm_fused: unknown epilogue %d", epilogue);
+    if (int rc = check_types("boat_cuda_gemm_fused", mma, type)) return rc;
+    if (M < 0 || N < 0 || K < 0) return set_error(11, "boat_cuda_gemm_fused: negative size");
+    if (M == 0 || N == 0) return 0;
+    if (!A || !B || !C || !aux) return set_error(11, "boat_cuda_gemm_fused: NULL operand");
+    if (type == BOAT_CUDA_F32_TF32) type = BOAT_CUDA_F32;
+    if (mma == BOAT_MMA_BF16 && gemm_tc_fused_supported(epilogue, ta, tb) && ((uintptr_t)aux & 15) == 0 &&
+        gemm_tc_supported(mma, ta, tb, M, N, K, A, lda, B, ldb, type, C, ldc, type))
+        return gemm_tc_fused(epilogue, M, N, K, A, lda, B, ldb, C, ldc, bias, aux);
+    if (ldc != N) return set_error(11, "boat_cuda_gemm_fused: separate passes need a packed result");
+    void* product = epilogue == BOAT_EPI_GELU ? aux : C;
+    if (int rc = boat_cuda_gemm(mma, ta, tb, M, N, K, A, lda, B, ldb, type, product, ldc, type, bias)) return rc;
+    if (epilogue == BOAT_EPI_GELU) return boat_cuda_gelu_fwd(C, aux, type, M * N);
+    if (epilogue == BOAT_EPI_GELU_GRAD) return boat_cuda_gelu_bwd(C, C, aux, type, M * N);
+    return boat_cuda_lincomb(C, C, 1.0f, aux, 1.0f, type, M * N);
+}
+
+int boat_cuda_gemm_sum(int mma, int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
+                       const void* const* B, int64_t ldb, int in_type, void* C, int64_t ldc, int out_type) {
+    if (groups < 1 || groups > 4) return set_error(11, "boat_cuda_gemm_sum: %d groups (1 to 4)", groups);
+    if (!A || !B || !C) return set_error(11, "boat_cuda_gemm_sum: NULL operand");
+    if (int rc = check_types("boat_cuda_gemm_sum", mma, in_type)) return rc;
+    if (mma == BOAT_MMA_FP32 || M <= 0 || N <= 0 || K <= 0 || out_type < BOAT_CUDA_F32 || out_type > BOAT_CUDA_F32_TF32) return 13;
+    const int store = in_type == BOAT_CUDA_F32_TF32 ? BOAT_CUDA_F32 : in_type;
+    for (int g = 0; g < groups; ++g)
+        if (!A[g] || !B[g] || !gemm_tc_supported(mma, ta, tb, M, N, K, A[g], lda, B[g], ldb, store, C, ldc, out_type)) return 13;
+    return gemm_tc_sum(mma, ta, tb, groups, M, N, K, A, lda, B, ldb, C, ldc, out_type);
+}
+
 int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T, const void* const* X, const void* const* dY,
-                           int in_type, float* const* dW, float* const* db) {
-    if (groups < 1 || groups > 4) return set_error(11, "boat_cuda_weight_grads: %d groups (1 to 4)", groups);
+                           int in_type, float* const* dW, float* const* db, int accumulate) {
+    if (groups < 1 || groups > 4 || (accumulate && groups != 1))
+        return set_error(11, "boat_cuda_weight_grads: %d groups (1 to 4, 1 to accumulate)", groups);
     if (!X || !dY || !dW) return set_error(11, "boat_cuda_weight_grads: NULL operand table");
     if (int rc = check_types("boat_cuda_weight_grads", mma, in_type)) return rc;
+    const int store = in_type == BOAT_CUDA_F32_TF32 ? BOAT_CUDA_F32 : in_type;
     bool ok = I > 0 && O > 0 && T > 0;
     for (int g = 0; g < groups; ++g) ok = ok && X[g] && dY[g] && dW[g];
-    if (ok && mma == BOAT_MMA_FP32) {
+    if (!ok && accumulate) return I > 0 && O > 0 && T <= 0 ? 0 : set_error(11, "boat_cuda_weight_grads: NULL operand");
+    const bool tensor_cores = ok && mma != BOAT_MMA_FP32 && gemm_tc_supported(mma, 1, 0, I, O, T, X[0], I, dY[0], O, store, dW[0], O, BOAT_CUDA_F32);
+    if (ok && (mma == BOAT_MMA_FP32 || (accumulate && !tensor_cores))) {
         // the CUDA-core kernel has the rows of dY in its hands anyway: one launch, one pass
         ProfileScope prof("gemm_simt");
-        return gemm_simt_grouped(1, 0, groups, I, O, T, X, I, dY, O, in_type == BOAT_CUDA_BF16 ? in_type : (int)BOAT_CUDA_F32,
-                                 (void* const*)dW, O, BOAT_CUDA_F32, nullptr, db);
+        return gemm_simt_grouped(1, 0, groups, I, O, T, X, I, dY, O, store, (void* const*)dW, O, BOAT_CUDA_F32, nullptr, db, accumulate != 0);
     }
-    if (int rc = boat_cuda_gemm_grouped(mma, 1, 0, groups, I, O, T, X, I, dY, O, in_type, (void* const*)dW, O, BOAT_CUDA_F32, nullptr))
+    if (accumulate) {
+        if (int rc = gemm_tc_accumulate(mma, 1, 0, I, O, T, X[0], I, dY[0], O, dW[0], O)) return rc;
+    } else if (int rc = boat_cuda_gemm_grouped(mma, 1, 0, groups, I, O, T, X, I, dY, O, in_type, (void* const*)dW, O, BOAT_CUDA_F32, nullptr)) {
         return rc;
-    return db && db[0] ? boat_cuda_colsum_multi(dY, in_type, T, O, db, groups) : 0;
+    }
+    return db && db[0] ? colsum_multi(dY, in_type, T, O, db, groups, accumulate != 0) : 0;
 }
 
 int boat_cuda_attn_fwd(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,

@@ -91,6 +91,24 @@ __global__ void axpy_multi_kernel(const AxpyTable t, float alpha, int vec) {
     for (int64_t i = n4 * 4 + i0; i < n; i += step) y[i] = mul_add(alpha, x[i], y[i]);
 }
 
+// ---- the SGD step of a layer that accumulates its gradients: y -= fl(lr*g), then g = 0 ----------------
+__global__ void sgd_clear_kernel(const AxpyTable t, float lr, int vec) {
+    griddep_sync();
+    float* __restrict__ y = t.y[blockIdx.y];
+    float* __restrict__ g = const_cast<float*>(t.x[blockIdx.y]);
+    const int64_t n = t.n[blockIdx.y], n4 = vec ? n / 4 : 0;
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < n4; i += step) {
+        const float4 a = reinterpret_cast<const float4*>(g)[i], b = reinterpret_cast<const float4*>(y)[i];
+        reinterpret_cast<float4*>(y)[i] = make_float4(mul_add(-lr, a.x, b.x), mul_add(-lr, a.y, b.y), mul_add(-lr, a.z, b.z), mul_add(-lr, a.w, b.w));
+        reinterpret_cast<float4*>(g)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int64_t i = n4 * 4 + i0; i < n; i += step) {
+        y[i] = mul_add(-lr, g[i], y[i]);
+        g[i] = 0.f;
+    }
+}
+
 // ---- y = a * b -------------------------------------------------------------------------------
 __global__ void mul_kernel(float* __restrict__ y, const float* __restrict__ a, const float* __restrict__ b,
                            int64_t n, int vec) {
@@ -279,7 +297,7 @@ struct ColsumTable {
 };
 
 template <typename T, int VEC, int LANES, int THREADS, bool CLUSTER>
-__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols) {
+__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols, int add_to) {
     constexpr int ROWS = THREADS / LANES, COLS = LANES * VEC, UNROLL = 8;
     __shared__ float part[ROWS * COLS];
     __shared__ float folded[CLUSTER ? COLS : 1];
@@ -337,7 +355,8 @@ __global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__
                 float s = 0.f;
 #pragma unroll
                 for (int r = 0; r < kColsumCluster; ++r) s += cluster.map_shared_rank(folded, r)[c];
-                if (group0 + c < cols) t.out[blockIdx.z][group0 + c] = s;
+                float* o = t.out[blockIdx.z] + group0 + c;
+                if (group0 + c < cols) *o = add_to ? *o + s : s;
             }
         }
         cluster.sync();
@@ -345,32 +364,32 @@ __global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__
 }
 
 template <typename T, int VEC, int LANES>
-static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t cols, int count) {
+static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t cols, int count, bool add) {
     BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)ceil_div(cols, LANES * VEC), (unsigned)count),
-                                  dim3(512), 0, kColsumCluster, t, rows, cols));
+                                  dim3(512), 0, kColsumCluster, t, rows, cols, add ? 1 : 0));
     BOATCU_LAUNCH_OK("colsum");
     return 0;
 }
 
 template <typename T, int VEC>
-static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int count) {
+static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int count, bool add) {
     if (rows * cols * (int64_t)sizeof(T) >= (32ll << 20)) {
-        for (int i = 0; i < count; ++i) BOATCU_CHECK(cudaMemsetAsync(t.out[i], 0, (size_t)cols * sizeof(float), stream()));
+        for (int i = 0; i < count && !add; ++i) BOATCU_CHECK(cudaMemsetAsync(t.out[i], 0, (size_t)cols * sizeof(float), stream()));
         const int64_t groups = ceil_div(cols, 32 * VEC);
         int64_t y = (int64_t)sm_count() * 8 / (groups * count);         // eight CTAs per SM
         if (y < 1) y = 1;
         if (y > ceil_div(rows, 8)) y = ceil_div(rows, 8);
         BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, 32, 256, false>, dim3((unsigned)y, (unsigned)groups, (unsigned)count), dim3(256), 0, 1,
-                                      t, rows, cols));
+                                      t, rows, cols, 0));
         BOATCU_LAUNCH_OK("colsum");
         return 0;
     }
     // the runs of a row are 512 bytes where that makes enough CTAs for the GPU, else 256 or 128
     auto ctas = [&](int lanes) { return ceil_div(cols, lanes * VEC) * kColsumCluster * count; };
     const int64_t enough = (int64_t)sm_count() * 4 / 5;
-    if (ctas(32) >= enough) return launch_colsum_cluster<T, VEC, 32>(t, rows, cols, count);
-    if (ctas(16) >= enough) return launch_colsum_cluster<T, VEC, 16>(t, rows, cols, count);
-    return launch_colsum_cluster<T, VEC, 8>(t, rows, cols, count);
+    if (ctas(32) >= enough) return launch_colsum_cluster<T, VEC, 32>(t, rows, cols, count, add);
+    if (ctas(16) >= enough) return launch_colsum_cluster<T, VEC, 16>(t, rows, cols, count, add);
+    return launch_colsum_cluster<T, VEC, 8>(t, rows, cols, count, add);
 }
 
 // ---- delta[r] = sum_d dO[r,d] * O[r,d]: one warp per row, shuffle reduction --------------------
@@ -519,25 +538,48 @@ extern "C" {
 int boat_cuda_axpy(float* y, const float* x, float alpha, int64_t n) { return launch_axpy<true>(y, x, alpha, n); }
 int boat_cuda_scale(float* y, const float* x, float alpha, int64_t n) { return launch_axpy<false>(y, x, alpha, n); }
 
-int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, const int64_t* n, int count) {
-    if (count <= 0) return 0;
-    if (count > kMaxAxpy || !y || !x || !n) return set_error(11, "boat_cuda_axpy_multi: bad table (%d tensors, 1 to %d)", count, kMaxAxpy);
-    if (int rc = ensure_init()) return rc;
-    AxpyTable t;
+static int fill_axpy_table(const char* who, float* const* y, const float* const* x, const int64_t* n, int count, AxpyTable& t,
+                           int& vec_out, int64_t& longest_out) {
+    if (count > kMaxAxpy || !y || !x || !n) return set_error(11, "%s: bad table (%d tensors, 1 to %d)", who, count, kMaxAxpy);
     int vec = 1;
     int64_t longest = 0;
     for (int i = 0; i < kMaxAxpy; ++i) {
         const int s = i < count ? i : 0;
-        if (n[s] > 0 && (!y[s] || !x[s])) return set_error(11, "boat_cuda_axpy_multi: bad entry %d", s);
+        if (n[s] > 0 && (!y[s] || !x[s])) return set_error(11, "%s: bad entry %d", who, s);
         t.y[i] = y[s];
         t.x[i] = x[s];
         t.n[i] = n[s];
         vec = vec && aligned16(y[s]) && aligned16(x[s]);
         if (n[s] > longest) longest = n[s];
     }
+    vec_out = vec;
+    longest_out = longest;
+    return 0;
+}
+
+int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, const int64_t* n, int count) {
+    if (count <= 0) return 0;
+    AxpyTable t;
+    int vec;
+    int64_t longest;
+    if (int rc = fill_axpy_table("boat_cuda_axpy_multi", y, x, n, count, t, vec, longest)) return rc;
     if (longest <= 0) return 0;
+    if (int rc = ensure_init()) return rc;
     BOATCU_RUN(axpy_multi_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, alpha, vec);
     BOATCU_LAUNCH_OK("axpy_multi");
+    return 0;
+}
+
+int boat_cuda_sgd_clear(float* const* y, float* const* g, float lr, const int64_t* n, int count) {
+    if (count <= 0) return 0;
+    AxpyTable t;
+    int vec;
+    int64_t longest;
+    if (int rc = fill_axpy_table("boat_cuda_sgd_clear", y, g, n, count, t, vec, longest)) return rc;
+    if (longest <= 0) return 0;
+    if (int rc = ensure_init()) return rc;
+    BOATCU_RUN(sgd_clear_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, lr, vec);
+    BOATCU_LAUNCH_OK("sgd_clear");
     return 0;
 }
 
@@ -601,7 +643,10 @@ int boat_cuda_round_tf32(float* y, const float* x, int64_t n) {
     return 0;
 }
 
-int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count) {
+}  // extern "C"
+
+namespace boatcu {
+int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count, bool add) {
     if (cols <= 0 || count <= 0) return 0;
     if (count > kMaxColsum) return set_error(11, "boat_cuda_colsum_multi: %d matrices (1 to %d)", count, kMaxColsum);
     if (!X || !out) return set_error(11, "boat_cuda_colsum_multi: NULL table");
@@ -619,8 +664,16 @@ int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64
     }
     if (rows < 0) rows = 0;
     if (x_type == BOAT_CUDA_BF16)
-        return can_vec ? launch_colsum<__nv_bfloat16, 8>(t, rows, cols, count) : launch_colsum<__nv_bfloat16, 1>(t, rows, cols, count);
-    return can_vec ? launch_colsum<float, 4>(t, rows, cols, count) : launch_colsum<float, 1>(t, rows, cols, count);
+        return can_vec ? launch_colsum<__nv_bfloat16, 8>(t, rows, cols, count, add) : launch_colsum<__nv_bfloat16, 1>(t, rows, cols, count, add);
+    return can_vec ? launch_colsum<float, 4>(t, rows, cols, count, add) : launch_colsum<float, 1>(t, rows, cols, count, add);
+}
+
+}  // namespace boatcu
+
+extern "C" {
+
+int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count) {
+    return colsum_multi(X, x_type, rows, cols, out, count, false);
 }
 
 int boat_cuda_colsum(const void* X, int x_type, int64_t rows, int64_t cols, float* out) {

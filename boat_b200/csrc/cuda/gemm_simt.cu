@@ -35,6 +35,7 @@ struct SimtParams {
     int64_t M, N, K, lda, ldb, ldc;
     int n_tiles, split;
     int vec_a, vec_b, vec_c;         // 16-byte accesses possible
+    int add;                         // add to C and colsum instead of overwriting them (FP32 output)
 };
 
 __device__ __forceinline__ void cp_async16(float* dst, const float* src, int bytes) {
@@ -201,6 +202,12 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
 
     TO* C = (TO*)p.C[g];
     const float* bias = p.bias[g];
+    auto put = [&](TO* dst, float v) {
+        if constexpr (std::is_same<TO, float>::value) {
+            if (p.add) v += *dst;
+        }
+        *dst = from_f32<TO>(v);
+    };
     if (split == 1) {
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
@@ -219,7 +226,12 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
                         }
                         if constexpr (!std::is_same<TO, float>::value)
                             v = make_float4(round_to_tf32(v.x), round_to_tf32(v.y), round_to_tf32(v.z), round_to_tf32(v.w));
-                        *reinterpret_cast<float4*>(C + gm * p.ldc + gn) = v;
+                        float4* dst = reinterpret_cast<float4*>(C + gm * p.ldc + gn);
+                        if (p.add) {
+                            const float4 t = *dst;
+                            v = make_float4(t.x + v.x, t.y + v.y, t.z + v.z, t.w + v.w);
+                        }
+                        *dst = v;
                     }
                     continue;
                 }
@@ -227,13 +239,13 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
                 const int64_t gn = n0 + col(j);
-                if (gn < p.N) C[gm * p.ldc + gn] = from_f32<TO>(acc[i][j] + (bias ? bias[gn] : 0.f));
+                if (gn < p.N) put(C + gm * p.ldc + gn, acc[i][j] + (bias ? bias[gn] : 0.f));
             }
         }
         if (sums && ty == 0) {
 #pragma unroll
             for (int j = 0; j < TN; ++j)
-                if (n0 + col(j) < p.N) p.colsum[g][n0 + col(j)] = bsum[j];
+                if (n0 + col(j) < p.N) p.colsum[g][n0 + col(j)] = bsum[j] + (p.add ? p.colsum[g][n0 + col(j)] : 0.f);
         }
         return;
     }
@@ -263,10 +275,10 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
         const int64_t gn = n0 + e % S::BN;
         if (gn >= p.N) continue;
         if (e >= S::BM * S::BN) {
-            p.colsum[g][gn] = v;
+            p.colsum[g][gn] = v + (p.add ? p.colsum[g][gn] : 0.f);
         } else {
             const int64_t gm = m0 + e / S::BN;
-            if (gm < p.M) C[gm * p.ldc + gn] = from_f32<TO>(v + (bias ? bias[gn] : 0.f));
+            if (gm < p.M) put(C + gm * p.ldc + gn, v + (bias ? bias[gn] : 0.f));
         }
     }
     cluster.sync();                                       // nobody leaves while its partial tile is being read
@@ -322,11 +334,12 @@ int pick_layout(SimtParams& p, int groups, int ta, int tb) {
 
 int gemm_simt_grouped(int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
                       const void* const* B, int64_t ldb, int in_type, void* const* C, int64_t ldc, int out_type,
-                      const float* const* bias, float* const* colsum) {
+                      const float* const* bias, float* const* colsum, bool add) {
     if (M <= 0 || N <= 0) return 0;
     if (int rc = ensure_init()) return rc;
     SimtParams p;
     p.M = M; p.N = N; p.K = K; p.lda = lda; p.ldb = ldb; p.ldc = ldc;
+    p.add = add ? 1 : 0;
     p.vec_a = lda % 4 == 0;
     p.vec_b = ldb % 4 == 0;
     p.vec_c = ldc % 4 == 0 && N % 4 == 0;

@@ -31,6 +31,13 @@
 // sector of its own: 786 TFLOP/s at 32768 x 4096 x 1024.)  The same boxes serve as
 // reductions (cp.reduce .add) for split K and for accumulation into the output.
 //
+// The epilogue can carry on with element-wise work on its tile (Epilogue): GELU beside the
+// pre-activation it came from, the product with GELU's derivative, a residual - whose second operand comes
+// in through the same kind of boxes.  Each saves a pass over [T, 4d] or [T, d] matrices.
+//
+// A chained launch sums the products of its groups in one accumulator: the three input gradients of
+// self-attention are one gradient.
+//
 // FP32 results (weight gradients) have few tiles and a long K.  Whole waves of tiles are done by one CTA
 // (pair) each; the tiles left over, which would keep most SMs idle for one more wave, are split along K
 // into pieces that add into a zeroed output.
@@ -40,6 +47,7 @@
 // all groups, group index fastest, so CTAs at work at the same time read the operand the groups
 // share (X for self-attention) from L2.
 #include "tc_common.cuh"
+#include "gelu.cuh"
 
 namespace boatcu {
 
@@ -52,10 +60,11 @@ constexpr int kThreads = 192;
 constexpr int kMaxGroups = 4;
 constexpr int kBoxRows = 32;                     // rows of a staging box: one epilogue warp's rows
 constexpr int kStageBox = kBoxRows * 128;        // 32 rows x 128 bytes
-constexpr int kOutBoxes = 2;                     // boxes in flight per epilogue warp
 
-template <typename T, int CTAS, int BN>
+template <typename T, int CTAS, int BN, int EPI>
 struct Cfg {
+    // boxes per epilogue warp: two results in flight, and two of the second result or operand
+    static constexpr int BOXES = EPI == BOAT_EPI_NONE ? 2 : 4;
     static constexpr int ES = sizeof(T);
     static constexpr int BK = 128 / ES;             // one 128-byte swizzle row of K (or of M/N)
     static constexpr int UK = 32 / ES;              // K extent of one tcgen05.mma
@@ -64,7 +73,7 @@ struct Cfg {
     static constexpr int B_BYTES = BNC * 128;
     static constexpr int STAGE = A_BYTES + B_BYTES;
     static constexpr int CHUNK_BYTES = BK * 128;    // one [BK rows x 128 B] box of an MN-major operand
-    static constexpr int OUT_BYTES = 4 * kOutBoxes * kStageBox;
+    static constexpr int OUT_BYTES = 4 * BOXES * kStageBox;
     static constexpr int FIT = (232448 - 1024 - 512 - OUT_BYTES) / STAGE;
     static constexpr int STAGES = FIT < 8 ? FIT : 8;
     static constexpr int SMEM = STAGES * STAGE + OUT_BYTES + 1024 /*alignment*/ + 512 /*barriers*/;
@@ -73,11 +82,13 @@ struct Cfg {
 
 struct GroupMaps {
     CUtensorMap a[kMaxGroups], b[kMaxGroups], c[kMaxGroups];
+    CUtensorMap aux;         // second result (BOAT_EPI_GELU) or element-wise operand of the epilogue
 };
 
 struct Params {
     const float* bias[kMaxGroups];
     int groups;
+    int chain;           // the groups' products are summed into one result
     int M, N, K;
     int out_type;
     int full;            // tiles done in one piece; the rest is split along K
@@ -91,10 +102,11 @@ struct WorkItem {
     bool first, add;     // first piece of its tile (adds the bias); result is added to the output
 };
 
-template <typename T, bool A_MN, bool B_MN, int CTAS, int BN>
+template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ Params p) {
-    using C = Cfg<T, CTAS, BN>;
+    using C = Cfg<T, CTAS, BN, EPI>;
+    constexpr bool AUX_IN = EPI == BOAT_EPI_GELU_GRAD || EPI == BOAT_EPI_ADD;
     constexpr bool TF32 = sizeof(T) == 4;
     constexpr int STAGES = C::STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -107,14 +119,17 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
     uint64_t* empty = bars + STAGES;              // [STAGES] MMA -> TMA
     uint64_t* acc_full = bars + 2 * STAGES;       // [2] MMA -> epilogue
     uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA (of the first CTA of a pair)
-    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 4);
+    uint64_t* aux_full = bars + 2 * STAGES + 4;   // [4][2] an epilogue warp's operand boxes landed
+    uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 12);
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = CTAS == 2 ? cluster_rank() : 0;
     const int worker = blockIdx.x / CTAS, workers = gridDim.x / CTAS;
     const int m_tiles = (p.M + BM * CTAS - 1) / (BM * CTAS), n_tiles = (p.N + BN - 1) / BN;
-    const int k_blocks = (p.K + C::BK - 1) / C::BK;
-    const int tiles = m_tiles * n_tiles * p.groups;
+    const int k_one = (p.K + C::BK - 1) / C::BK;                   // K-blocks of one product
+    const int k_blocks = p.chain ? k_one * p.groups : k_one;
+    const int results = p.chain ? 1 : p.groups;
+    const int tiles = m_tiles * n_tiles * results;
     const int work_items = p.full + (tiles - p.full) * p.split;
     auto item = [&](int w) {
         WorkItem it;
@@ -123,8 +138,8 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         const int tile = w < p.full ? w : p.full + (w - p.full) % rest;
         const int part = w < p.full ? 0 : (w - p.full) / rest;
         const int pieces = w < p.full ? 1 : p.split;
-        const int mn = tile / p.groups;
-        it.g = tile % p.groups;
+        const int mn = tile / results;
+        it.g = tile % results;
         it.m0 = (mn / n_tiles) * BM * CTAS + (int)rank * BM;
         it.n0 = (mn % n_tiles) * BN;
         it.kb0 = (int)((int64_t)part * k_blocks / pieces);
@@ -143,12 +158,14 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 4 * CTAS);
         }
+        for (int b = 0; b < 8; ++b) mbar_init(&aux_full[b], 1);
         fence_barrier_init();
         for (int g = 0; g < p.groups; ++g) {
             tma_prefetch_desc(&maps.a[g]);
             tma_prefetch_desc(&maps.b[g]);
-            tma_prefetch_desc(&maps.c[g]);
+            if (g < results) tma_prefetch_desc(&maps.c[g]);
         }
+        if (EPI != BOAT_EPI_NONE) tma_prefetch_desc(&maps.aux);
     }
     if (warp == 1) {
         if (CTAS == 2) tmem_alloc_pair(tmem_slot, C::TMEM_COLS);
@@ -168,14 +185,15 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
             bool ok = true;
             for (int w = worker; w < work_items && ok; w += workers) {
                 const WorkItem t = item(w);
-                const CUtensorMap* map_a = &maps.a[t.g];
-                const CUtensorMap* map_b = &maps.b[t.g];
                 const int nb = t.n0 + (int)rank * C::BNC;             // this CTA's rows of B
                 for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
                     if (rank == 0) mbar_arrive_expect_tx(&full[s], CTAS * C::STAGE);
-                    const int k0 = kb * C::BK;
+                    const int g = p.chain ? kb / k_one : t.g;
+                    const CUtensorMap* map_a = &maps.a[g];
+                    const CUtensorMap* map_b = &maps.b[g];
+                    const int k0 = (p.chain ? kb - g * k_one : kb) * C::BK;
                     uint8_t* a_dst = a_smem + s * C::A_BYTES;
                     uint8_t* b_dst = b_smem + s * C::B_BYTES;
                     const uint32_t bar = CTAS == 2 ? peer_addr(&full[s], 0) : 0;
@@ -243,30 +261,51 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
     } else {
         // ---------------- epilogue: warps 2..5 ----------------
         const int lane_group = warp & 3;              // TMEM lanes this warp may touch
-        uint8_t* boxes = out_smem + lane_group * kOutBoxes * kStageBox;
+        uint8_t* boxes = out_smem + lane_group * C::BOXES * kStageBox;        // results, then the second kind
+        uint32_t aux_it = 0;                          // operand boxes asked for so far
+        auto load_aux = [&](int x, int y) {           // by lane 0
+            const uint32_t b = aux_it & 1;
+            mbar_arrive_expect_tx(&aux_full[lane_group * 2 + b], kStageBox);
+            tma_load_2d(boxes + (2 + b) * kStageBox, &maps.aux, &aux_full[lane_group * 2 + b], x, y);
+        };
         const int swz = lane & 7;
         const bool bf16_out = p.out_type == BOAT_CUDA_BF16;
         const int step = bf16_out ? 64 : 32;          // columns per box
         uint32_t acc_it = 0, box_it = 0;
-        for (int w = worker; w < work_items; w += workers, ++acc_it) {
+        bool ok = true;
+        for (int w = worker; w < work_items && ok; w += workers, ++acc_it) {
             const WorkItem t = item(w);
             const CUtensorMap* map_c = &maps.c[t.g];
             const float* const bias = t.first ? p.bias[t.g] : nullptr;
             const bool bias16 = ((uintptr_t)bias & 15) == 0;
             const int buf = acc_it & 1;
-            if (!mbar_wait_warp(&acc_full[buf], (acc_it >> 1) & 1, p.status, kTimeoutEpilogue)) break;
-            tc_fence_after_sync();
             const int row0 = t.m0 + lane_group * 32;
+            if (AUX_IN) {
+                if (lane == 0) load_aux(t.n0, row0);
+                ++aux_it;
+            }
+            if (!mbar_wait_warp(&acc_full[buf], (acc_it >> 1) & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
+            tc_fence_after_sync();
             const uint32_t t_addr = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * BN;
             const int cols = min(BN, p.N - t.n0);
 #pragma unroll 1
             for (int c = 0; c < cols; c += step, ++box_it) {
-                uint8_t* box = boxes + (box_it % kOutBoxes) * kStageBox;
-                // the store that used this box last has read it
+                uint8_t* box = boxes + (box_it & 1) * kStageBox;
+                // the stores that used this box (and its pair) last have read it
                 if (lane == 0) tma_wait_group_read1();
                 __syncwarp();
                 uint8_t* row = box + lane * 128;
                 const int col0 = t.n0 + c;
+                uint8_t* row2 = row + 2 * kStageBox;  // second result
+                if (AUX_IN) {
+                    const uint32_t b = (aux_it - 1) & 1, par = ((aux_it - 1) >> 1) & 1;
+                    row2 = boxes + (2 + b) * kStageBox + lane * 128;
+                    if (c + step < cols) {            // the next operand box, under the work on this one
+                        if (lane == 0) load_aux(col0 + step, row0);
+                        ++aux_it;
+                    }
+                    if (!mbar_wait_warp(&aux_full[lane_group * 2 + b], par, p.status, kTimeoutEpilogue)) { ok = false; break; }
+                }
                 // one 32-column half of the box (all of an FP32 box) at a time
 #pragma unroll 1
                 for (int h = 0; h < step; h += 32) {
@@ -288,6 +327,39 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
 #pragma unroll
                             for (int j = 0; j < 32; ++j)
                                 if (col0 + h + j < p.N) v[j] += __ldg(b + j);
+                        }
+                    }
+                    if (AUX_IN) {                     // BF16 only
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const uint4 q = *reinterpret_cast<const uint4*>(row2 + (((h / 8 + u) ^ swz) << 4));
+                            const uint32_t x[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[e]));
+                                if (EPI == BOAT_EPI_ADD) {
+                                    v[8 * u + 2 * e] += f.x;
+                                    v[8 * u + 2 * e + 1] += f.y;
+                                } else {
+                                    v[8 * u + 2 * e] *= gelu_grad_f(f.x);
+                                    v[8 * u + 2 * e + 1] *= gelu_grad_f(f.y);
+                                }
+                            }
+                        }
+                    }
+                    if (EPI == BOAT_EPI_GELU) {       // the rounded pre-activation, kept, then GELU of it
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            uint32_t o[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                __nv_bfloat162 q = __floats2bfloat162_rn(v[8 * u + 2 * e], v[8 * u + 2 * e + 1]);
+                                o[e] = *reinterpret_cast<uint32_t*>(&q);
+                                const float2 f = __bfloat1622float2(q);
+                                v[8 * u + 2 * e] = gelu_f(f.x);
+                                v[8 * u + 2 * e + 1] = gelu_f(f.y);
+                            }
+                            *reinterpret_cast<uint4*>(row2 + (((h / 8 + u) ^ swz) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
                         }
                     }
                     if (bf16_out) {
@@ -326,12 +398,15 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                     if (row0 < p.M) {
                         if (t.add) tma_reduce_add_2d(map_c, box, col0, row0);
                         else       tma_store_2d(map_c, box, col0, row0);
+                        if (EPI == BOAT_EPI_GELU) tma_store_2d(&maps.aux, box + 2 * kStageBox, col0, row0);
                     }
                     tma_commit_group();
                 }
             }
         }
         if (lane == 0) tma_wait_group0();
+        if (AUX_IN && !ok)                            // an operand box may be in flight
+            for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     }
     tc_fence_before_sync();
     __syncthreads();
@@ -356,7 +431,9 @@ struct Problem {
     int64_t ldc;
     int out_type;
     const float* const* bias;
-    bool add;
+    bool add;            // add to C instead of overwriting it (FP32)
+    bool chain;          // one result: the sum of the groups' products
+    void* aux;           // second result or operand of the epilogue, laid out like C
 };
 
 // A tile shape and what it costs, measured on B200 at 12 to 512 K-blocks (64 BF16): microseconds per K-block,
@@ -373,9 +450,9 @@ struct Plan {
 
 // Which tiles are cut along K, into how many pieces, and how long the launch should take.
 Plan make_plan(const Problem& q, const Shape& sh, int bk) {
-    const int64_t workers = sm_count() / sh.ctas, k_blocks = ceil_div(q.K, bk);
+    const int64_t workers = sm_count() / sh.ctas, k_blocks = ceil_div(q.K, bk) * (q.chain ? q.groups : 1);
     Plan r;
-    r.tiles = ceil_div(q.M, BM * sh.ctas) * ceil_div(q.N, sh.bn) * q.groups;
+    r.tiles = ceil_div(q.M, BM * sh.ctas) * ceil_div(q.N, sh.bn) * (q.chain ? 1 : q.groups);
     r.full = r.tiles;
     r.split = 1;
     r.us = (double)ceil_div(r.tiles, workers) * (double)k_blocks * sh.block_us + sh.once_us;
@@ -404,9 +481,9 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk) {
     return r;
 }
 
-template <typename T, bool A_MN, bool B_MN, int CTAS, int BN>
+template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI>
 int launch(const Problem& q, const Plan& plan) {
-    using C = Cfg<T, CTAS, BN>;
+    using C = Cfg<T, CTAS, BN, EPI>;
     GroupMaps maps;
     Params p;
     const bool bf16_out = q.out_type == BOAT_CUDA_BF16;
@@ -418,10 +495,13 @@ int launch(const Problem& q, const Plan& plan) {
         if (int rc = B_MN ? make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.ldb, C::BK, C::BK, C::ES == 4)
                           : make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.N, (uint64_t)q.K, (uint64_t)q.ldb, C::BNC, C::BK))
             return rc;
+        if (q.chain && g > 0) continue;
         if (int rc = make_tensor_map_2d(&maps.c[g], q.C[g], bf16_out ? 2 : 4, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, bf16_out ? 64 : 32))
             return rc;
         p.bias[g] = q.bias ? q.bias[g] : nullptr;
     }
+    if (EPI != BOAT_EPI_NONE)
+        if (int rc = make_tensor_map_2d(&maps.aux, q.aux, 2, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, 64)) return rc;
     const int64_t full = plan.full, split = plan.split, tiles = plan.tiles, workers = sm_count() / CTAS;
     if (split > 1 && !q.add) {
         for (int g = 0; g < q.groups; ++g) {
@@ -433,6 +513,7 @@ int launch(const Problem& q, const Plan& plan) {
         }
     }
     p.groups = q.groups;
+    p.chain = q.chain ? 1 : 0;
     p.M = (int)q.M;
     p.N = (int)q.N;
     p.K = (int)q.K;
@@ -441,7 +522,7 @@ int launch(const Problem& q, const Plan& plan) {
     p.split = (int)split;
     p.add_all = q.add ? 1 : 0;
     p.status = kernel_status_ptr();
-    auto kern = gemm_tc_kernel<T, A_MN, B_MN, CTAS, BN>;
+    auto kern = gemm_tc_kernel<T, A_MN, B_MN, CTAS, BN, EPI>;
     static bool configured = false;     // per process = per device: the library binds to one device
     if (!configured) {
         BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
@@ -459,7 +540,7 @@ int launch(const Problem& q, const Plan& plan) {
 }
 
 // The tile shape with the shortest estimate.
-template <typename T, bool A_MN, bool B_MN>
+template <typename T, bool A_MN, bool B_MN, int EPI = BOAT_EPI_NONE>
 int pick_tile(const Problem& q) {
     int best = 0;
     Plan plan;
@@ -471,10 +552,10 @@ int pick_tile(const Problem& q) {
         }
     }
     switch (best) {
-        case 0: return launch<T, A_MN, B_MN, 2, 256>(q, plan);
-        case 1: return launch<T, A_MN, B_MN, 1, 256>(q, plan);
-        case 2: return launch<T, A_MN, B_MN, 1, 128>(q, plan);
-        default: return launch<T, A_MN, B_MN, 1, 64>(q, plan);
+        case 0: return launch<T, A_MN, B_MN, 2, 256, EPI>(q, plan);
+        case 1: return launch<T, A_MN, B_MN, 1, 256, EPI>(q, plan);
+        case 2: return launch<T, A_MN, B_MN, 1, 128, EPI>(q, plan);
+        default: return launch<T, A_MN, B_MN, 1, 64, EPI>(q, plan);
     }
 }
 
@@ -510,8 +591,37 @@ int gemm_tc_grouped(int mma, int ta, int tb, int groups, int64_t M, int64_t N, i
                     const float* const* bias) {
     if (groups < 1 || groups > kMaxGroups) return set_error(11, "gemm_tc_grouped: %d groups (1..%d)", groups, kMaxGroups);
     if (int rc = ensure_init()) return rc;
-    const Problem q{groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, false};
+    const Problem q{groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, false, false, nullptr};
     return mma == BOAT_MMA_BF16 ? dispatch_layout<__nv_bfloat16>(ta, tb, q) : dispatch_layout<float>(ta, tb, q);
+}
+
+int gemm_tc_accumulate(int mma, int ta, int tb, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B,
+                       int64_t ldb, float* C, int64_t ldc) {
+    if (int rc = ensure_init()) return rc;
+    void* c = C;
+    const Problem q{1, M, N, K, &A, lda, &B, ldb, &c, ldc, BOAT_CUDA_F32, nullptr, true, false, nullptr};
+    return mma == BOAT_MMA_BF16 ? dispatch_layout<__nv_bfloat16>(ta, tb, q) : dispatch_layout<float>(ta, tb, q);
+}
+
+int gemm_tc_sum(int mma, int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
+                const void* const* B, int64_t ldb, void* C, int64_t ldc, int out_type) {
+    if (int rc = ensure_init()) return rc;
+    const Problem q{groups, M, N, K, A, lda, B, ldb, &C, ldc, out_type, nullptr, false, true, nullptr};
+    return mma == BOAT_MMA_BF16 ? dispatch_layout<__nv_bfloat16>(ta, tb, q) : dispatch_layout<float>(ta, tb, q);
+}
+
+bool gemm_tc_fused_supported(int epilogue, int ta, int tb) {
+    return !ta && (epilogue == BOAT_EPI_GELU_GRAD ? tb != 0 : tb == 0);
+}
+
+int gemm_tc_fused(int epilogue, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb,
+                  void* C, int64_t ldc, const float* bias, void* aux) {
+    if (int rc = ensure_init()) return rc;
+    const Problem q{1, M, N, K, &A, lda, &B, ldb, &C, ldc, BOAT_CUDA_BF16, &bias, false, false, aux};
+    typedef __nv_bfloat16 bf;
+    if (epilogue == BOAT_EPI_GELU) return pick_tile<bf, false, true, BOAT_EPI_GELU>(q);
+    if (epilogue == BOAT_EPI_ADD) return pick_tile<bf, false, true, BOAT_EPI_ADD>(q);
+    return pick_tile<bf, false, false, BOAT_EPI_GELU_GRAD>(q);
 }
 
 void gemm_tc_set_yielding(bool on) { g_yielding = on; }

@@ -8,6 +8,8 @@
 // exact erf form of GELU.  One CTA per row keeps the row in shared memory, so a row is read
 // from HBM once per kernel; 128-bit accesses where the row length allows.
 #include "common.cuh"
+#include "gelu.cuh"
+#include <initializer_list>
 
 namespace boatcu {
 
@@ -137,11 +139,8 @@ layernorm_bwd_dx_kernel(const T* __restrict__ dy, const T* __restrict__ x, int c
     store_row(dx + r * cols, g, cols);
 }
 
-// ---- one warp per row ------------------------------------------------------------------------------
-// For rows of up to 2048 elements whose length is a multiple of 32 vectors of 16 bytes: a lane
-// holds NV vectors of the row in registers, the row statistics are shuffle reductions, and a
-// row costs no shared memory and no CTA barrier.  Lane l owns vectors l, l+32, l+64, ... so that
-// every access of the warp is one contiguous run of 512 bytes.
+// ---- rows of whole 16-byte vectors -------------------------------------------------------------------
+// Both kernels are bound by HBM, which wants some 45 KB in flight per SM.
 template <typename T> struct Vec16 { static constexpr int N = 16 / sizeof(T); };
 
 template <typename T>
@@ -189,59 +188,91 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-constexpr int kNormRowsPerWarp = 4;          // consecutive rows per warp: gamma and beta are loaded once for them
+// Sums of N values over the CTA, one barrier; `red` is one of two buffers used in turn ([32][N] floats).
+template <int N>
+__device__ __forceinline__ void block_sums(float (&v)[N], float* red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    const int warps = blockDim.x >> 5;
+    if (warps == 1) return;
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) red[(threadIdx.x >> 5) * N + k] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = 0.f;
+    for (int w = 0; w < warps; ++w)
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] += red[w * N + k];
+}
 
+constexpr int kNormMaxRowThreads = 512;      // threads per row; longer rows take the kernels above
+
+// A warp per row: lane l holds vectors l, l+32, ... of it, the statistics are shuffles, gamma and beta come from
+// shared memory (in registers they cost as much as the row itself), and the next row is on its way while
+// this one is worked on.
 template <typename T, int NV>
 __global__ void __launch_bounds__(kNormThreads)
-layernorm_fwd_warp_kernel(const T* __restrict__ x, int64_t rows, const float* __restrict__ gamma,
+layernorm_fwd_rows_kernel(const T* __restrict__ x, int64_t rows, int cols, const float* __restrict__ gamma,
                           const float* __restrict__ beta, float eps, T* __restrict__ y, float* __restrict__ mean_out,
                           float* __restrict__ rstd_out) {
+    constexpr int V = Vec16<T>::N;
+    extern __shared__ __align__(16) float params[];          // gamma, beta
     griddep_sync();
-    constexpr int V = Vec16<T>::N, COLS = NV * 32 * V;
-    const int lane = threadIdx.x & 31;
-    const int64_t r0 = ((int64_t)blockIdx.x * (kNormThreads / 32) + (threadIdx.x >> 5)) * kNormRowsPerWarp;
-    if (r0 >= rows) return;
-    float gm[NV][V], bt[NV][V];
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int c0 = (i * 32 + lane) * V;
-        if (gamma) load_param<V>(gamma, c0, gm[i]);
-        if (beta) load_param<V>(beta, c0, bt[i]);
+    for (int i = threadIdx.x; i < cols; i += kNormThreads) {
+        params[i] = gamma ? gamma[i] : 1.f;
+        params[cols + i] = beta ? beta[i] : 0.f;
     }
-#pragma unroll 1
-    for (int rr = 0; rr < kNormRowsPerWarp; ++rr) {
-        const int64_t r = r0 + rr;
-        if (r >= rows) break;
-        const uint4* src = reinterpret_cast<const uint4*>(x + r * COLS);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, nvec = cols / V;
+    const float inv = 1.0f / (float)cols;
+    const int64_t step = (int64_t)gridDim.x * (kNormThreads / 32);
+    int64_t r = (int64_t)blockIdx.x * (kNormThreads / 32) + (threadIdx.x >> 5);
+    uint4 raw[NV];
+    auto fetch = [&](int64_t row) {
+        const uint4* src = reinterpret_cast<const uint4*>(x + row * cols);
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            raw[i] = row < rows && i * 32 + lane < nvec ? src[i * 32 + lane] : make_uint4(0u, 0u, 0u, 0u);
+    };
+    fetch(r);
+    for (; r < rows; r += step) {
         float f[NV][V];
-#pragma unroll
-        for (int i = 0; i < NV; ++i) unpack16<T>(src[i * 32 + lane], f[i]);
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < NV; ++i)
-#pragma unroll
-            for (int k = 0; k < V; ++k) s += f[i][k];
-        const float mean = warp_sum(s) / (float)COLS;
-        float q = 0.f;
-#pragma unroll
-        for (int i = 0; i < NV; ++i)
-#pragma unroll
-            for (int k = 0; k < V; ++k) {
-                const float d = f[i][k] - mean;
-                q += d * d;
-            }
-        const float rstd = 1.0f / sqrtf(warp_sum(q) / (float)COLS + eps);
-        uint4* dst = reinterpret_cast<uint4*>(y + r * COLS);
+        float sum[1] = {0.f};
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
+            unpack16<T>(raw[i], f[i]);
+#pragma unroll
+            for (int k = 0; k < V; ++k) sum[0] += f[i][k];
+        }
+        fetch(r + step);
+        const float mean = warp_sum(sum[0]) * inv;
+        float q = 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const bool in = i * 32 + lane < nvec;
 #pragma unroll
             for (int k = 0; k < V; ++k) {
-                float n = (f[i][k] - mean) * rstd;
-                if (gamma) n = n * gm[i][k];
-                if (beta) n = n + bt[i][k];
-                f[i][k] = n;
+                f[i][k] = in ? f[i][k] - mean : 0.f;
+                q += f[i][k] * f[i][k];
             }
-            dst[i * 32 + lane] = pack16<T>(f[i]);
+        }
+        const float rstd = 1.0f / sqrtf(warp_sum(q) * inv + eps);
+        uint4* dst = reinterpret_cast<uint4*>(y + r * cols);
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            if (i * 32 + lane < nvec) {
+                const int c0 = (i * 32 + lane) * V;
+                float gm[V], bt[V];
+                load_param<V>(params, c0, gm);
+                load_param<V>(params + cols, c0, bt);
+#pragma unroll
+                for (int k = 0; k < V; ++k) f[i][k] = fmaf(f[i][k] * rstd, gm[k], bt[k]);
+                dst[i * 32 + lane] = pack16<T>(f[i]);
+            }
         }
         if (lane == 0) {
             if (mean_out) mean_out[r] = mean;
@@ -250,81 +281,82 @@ layernorm_fwd_warp_kernel(const T* __restrict__ x, int64_t rows, const float* __
     }
 }
 
-// dx as in layernorm_bwd_dx_kernel; in the same pass every warp sums dy*xhat and dy over the
-// rows it walks (a grid-stride loop), per column, in registers; warps of a CTA combine in
-// shared memory and CTAs by atomicAdd into the zeroed dgamma / dbeta - dy and x are read once.
-template <typename T, int NV>
-__global__ void __launch_bounds__(kNormThreads)
-layernorm_bwd_warp_kernel(const T* __restrict__ dy, const T* __restrict__ x, int64_t rows,
-                          const float* __restrict__ gamma, const float* __restrict__ mean,
-                          const float* __restrict__ rstd, T* __restrict__ dx, float* __restrict__ dgamma,
-                          float* __restrict__ dbeta) {
+// dx as in layernorm_bwd_dx_kernel, plus `add` (a residual branch's gradient) if given.  A thread owns one
+// 16-byte vector column of every row its CTA walks (8 BF16 or 4 FP32), so gamma and the sums for dgamma and
+// dbeta are a few registers; a CTA takes R rows at a time, whose loads are all in flight together, and folds
+// their sums with one barrier.  The column sums over a CTA's rows go to its row of `partial` ([2][CTAs, cols]),
+// which a column-sum launch folds (a thousand CTAs adding to the same addresses took 100 us).
+template <typename T, int R>
+__global__ void __launch_bounds__(kNormMaxRowThreads)
+layernorm_bwd_rows_kernel(const T* __restrict__ dy, const T* __restrict__ x, int64_t rows, int cols,
+                          const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
+                          const T* __restrict__ add, T* __restrict__ dx, float* __restrict__ partial) {
+    constexpr int V = Vec16<T>::N;
+    __shared__ float red[2][16 * 2 * R];
     griddep_sync();
-    constexpr int V = Vec16<T>::N, COLS = NV * 32 * V;
-    extern __shared__ float part[];                 // [2][COLS] when parameter gradients are wanted
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool params = dgamma != nullptr || dbeta != nullptr;
-    if (params) {
-        for (int i = threadIdx.x; i < 2 * COLS; i += blockDim.x) part[i] = 0.f;
-        __syncthreads();
+    const int c0 = threadIdx.x * V;
+    const bool mine = c0 < cols;
+    const float inv = 1.0f / (float)cols;
+    float gm[V], ag[V], ab[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        gm[k] = 1.f;
+        ag[k] = ab[k] = 0.f;
     }
-    float ag[NV][V], ab[NV][V];
+    if (mine && gamma) load_param<V>(gamma, c0, gm);
+    int turn = 0;
+    for (int64_t r0 = (int64_t)blockIdx.x * R; r0 < rows; r0 += (int64_t)gridDim.x * R, turn ^= 1) {
+        uint4 graw[R], xraw[R], araw[R];
+        float m[R], rs[R];
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
-#pragma unroll
-        for (int k = 0; k < V; ++k) ag[i][k] = ab[i][k] = 0.f;
-    const int64_t stride = (int64_t)gridDim.x * (kNormThreads / 32);
-    for (int64_t r = (int64_t)blockIdx.x * (kNormThreads / 32) + warp; r < rows; r += stride) {
-        const uint4* gsrc = reinterpret_cast<const uint4*>(dy + r * COLS);
-        const uint4* xsrc = reinterpret_cast<const uint4*>(x + r * COLS);
-        float g[NV][V], xh[NV][V];
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            unpack16<T>(gsrc[i * 32 + lane], g[i]);
-            unpack16<T>(xsrc[i * 32 + lane], xh[i]);
+        for (int r = 0; r < R; ++r) {
+            const bool in = mine && r0 + r < rows;
+            const int64_t at = (r0 + r) * cols + c0;
+            graw[r] = in ? *reinterpret_cast<const uint4*>(dy + at) : make_uint4(0u, 0u, 0u, 0u);
+            xraw[r] = in ? *reinterpret_cast<const uint4*>(x + at) : make_uint4(0u, 0u, 0u, 0u);
+            if (add) araw[r] = in ? *reinterpret_cast<const uint4*>(add + at) : make_uint4(0u, 0u, 0u, 0u);
+            m[r] = r0 + r < rows ? mean[r0 + r] : 0.f;
+            rs[r] = r0 + r < rows ? rstd[r0 + r] : 0.f;
         }
-        const float m = mean[r], rs = rstd[r];
-        float s1 = 0.f, s2 = 0.f;
+        float g[R][V], xh[R][V], s[2 * R];
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            float gm[V];
-            if (gamma) load_param<V>(gamma, (i * 32 + lane) * V, gm);
+        for (int r = 0; r < R; ++r) {
+            unpack16<T>(graw[r], g[r]);
+            unpack16<T>(xraw[r], xh[r]);
+            s[2 * r] = s[2 * r + 1] = 0.f;
 #pragma unroll
             for (int k = 0; k < V; ++k) {
-                const float xi = (xh[i][k] - m) * rs;
-                const float d = g[i][k];
-                ag[i][k] += d * xi;
-                ab[i][k] += d;
-                const float gi = gamma ? d * gm[k] : d;
-                g[i][k] = gi;
-                xh[i][k] = xi;
-                s1 += gi;
-                s2 += gi * xi;
+                xh[r][k] = (xh[r][k] - m[r]) * rs[r];
+                ag[k] = fmaf(g[r][k], xh[r][k], ag[k]);
+                ab[k] += g[r][k];
+                g[r][k] *= gm[k];
+                s[2 * r] += g[r][k];
+                s[2 * r + 1] = fmaf(g[r][k], xh[r][k], s[2 * r + 1]);
             }
         }
-        const float mg = warp_sum(s1) / (float)COLS, mgx = warp_sum(s2) / (float)COLS;
-        uint4* dst = reinterpret_cast<uint4*>(dx + r * COLS);
+        block_sums<2 * R>(s, red[turn]);
 #pragma unroll
-        for (int i = 0; i < NV; ++i) {
+        for (int r = 0; r < R; ++r) {
+            if (!mine || r0 + r >= rows) break;
+            const float mg = s[2 * r] * inv, mgx = s[2 * r + 1] * inv;
 #pragma unroll
-            for (int k = 0; k < V; ++k) g[i][k] = rs * (g[i][k] - mg - xh[i][k] * mgx);
-            dst[i * 32 + lane] = pack16<T>(g[i]);
+            for (int k = 0; k < V; ++k) g[r][k] = rs[r] * (g[r][k] - mg - xh[r][k] * mgx);
+            if (add) {
+                float t[V];
+                unpack16<T>(araw[r], t);
+#pragma unroll
+                for (int k = 0; k < V; ++k) g[r][k] += t[k];
+            }
+            *reinterpret_cast<uint4*>(dx + (r0 + r) * cols + c0) = pack16<T>(g[r]);
         }
     }
-    if (!params) return;
+    if (!mine || !partial) return;
+    float* pg = partial + (int64_t)blockIdx.x * cols + c0;
+    float* pb = pg + (int64_t)gridDim.x * cols;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-        const int c0 = (i * 32 + lane) * V;
-#pragma unroll
-        for (int k = 0; k < V; ++k) {
-            atomicAdd(part + c0 + k, ag[i][k]);
-            atomicAdd(part + COLS + c0 + k, ab[i][k]);
-        }
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < COLS; c += blockDim.x) {
-        if (dgamma) atomicAdd(dgamma + c, part[c]);
-        if (dbeta) atomicAdd(dbeta + c, part[COLS + c]);
+    for (int k = 0; k < V; k += 4) {
+        *reinterpret_cast<float4*>(pg + k) = make_float4(ag[k], ag[k + 1], ag[k + 2], ag[k + 3]);
+        *reinterpret_cast<float4*>(pb + k) = make_float4(ab[k], ab[k + 1], ab[k + 2], ab[k + 3]);
     }
 }
 
@@ -361,36 +393,7 @@ __global__ void layernorm_bwd_params_kernel(const T* __restrict__ dy, const T* _
     }
 }
 
-// ---- GELU, exact erf form ------------------------------------------------------------------------
-// Phi(x) = (1 + erf(x/sqrt 2))/2 and e = exp(-x^2/2) from one exponential: erf by Abramowitz &
-// Stegun 7.1.26, erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1/(1 + p z), |error| <= 1.5e-7,
-// whose exponential at z = |x|/sqrt 2 is the exp(-x^2/2) that the derivative needs anyway.
-// erff + expf cost ~40 instructions per element and made these kernels instruction-bound
-// (55 % of HBM bandwidth); this form needs one ex2, one rcp and a dozen FMAs.
-__device__ __forceinline__ void gelu_parts(float x, float& phi, float& e) {
-    const float z = fabsf(x) * 0.70710678118654752f;
-    // one MUFU instruction each (relative error ~2^-22, far inside the 1.5e-7 of the formula)
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-0.72134752044448170f * x * x));   // exp(-x^2/2)
-    float t;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.3275911f, z, 1.0f)));
-    float poly = fmaf(1.061405429f, t, -1.453152027f);
-    poly = fmaf(poly, t, 1.421413741f);
-    poly = fmaf(poly, t, -0.284496736f);
-    poly = fmaf(poly, t, 0.254829592f);
-    const float half_erfc = 0.5f * poly * t * e;                   // (1 - erf(z)) / 2
-    phi = x >= 0.f ? 1.0f - half_erfc : half_erfc;
-}
-__device__ __forceinline__ float gelu_f(float x) {
-    float phi, e;
-    gelu_parts(x, phi, e);
-    return x * phi;
-}
-__device__ __forceinline__ float gelu_grad_f(float x) {
-    float phi, e;
-    gelu_parts(x, phi, e);
-    return fmaf(x * 0.3989422804014327f, e, phi);
-}
-
+// ---- GELU (gelu.cuh) ------------------------------------------------------------------------------
 template <typename T, bool BWD>
 __global__ void gelu_kernel(T* __restrict__ out, const T* __restrict__ x, const T* __restrict__ dy, int64_t n) {
     griddep_sync();
@@ -458,63 +461,63 @@ static int launch_gelu(void* out, const void* x, const void* dy, int64_t n) {
     return 0;
 }
 
-// Warp-per-row dispatch.  Returns 0 when the shape is not covered (the caller falls back to
-// the CTA-per-row kernels), -1 after a successful launch, an error status otherwise.
-template <typename T, int NV>
-static int fwd_warp_launch(const void* x, int64_t rows, const float* gamma, const float* beta, float eps, void* y,
-                           float* mean_out, float* rstd_out) {
-    const int64_t blocks = ceil_div(rows, (kNormThreads / 32) * kNormRowsPerWarp);
-    BOATCU_RUN((layernorm_fwd_warp_kernel<T, NV>), (unsigned)blocks, kNormThreads, 0, (const T*)x, rows, gamma, beta, eps,
-                                                                                       (T*)y, mean_out, rstd_out);
-    BOATCU_LAUNCH_OK("layernorm_fwd_warp");
-    return -1;
-}
-
-template <typename T, int NV>
-static int bwd_warp_launch(const void* dy, const void* x, int64_t rows, const float* gamma, const float* mean,
-                           const float* rstd, void* dx, float* dgamma, float* dbeta) {
-    constexpr int COLS = NV * 32 * (16 / (int)sizeof(T));
-    int64_t blocks = ceil_div(rows, kNormThreads / 32);
-    if (blocks > sm_count() * 4) blocks = sm_count() * 4;         // persistent: the column sums live in registers across rows
-    const size_t smem = (dgamma || dbeta) ? 2 * COLS * sizeof(float) : 0;
-    BOATCU_RUN((layernorm_bwd_warp_kernel<T, NV>), (unsigned)blocks, kNormThreads, smem, 
-        (const T*)dy, (const T*)x, rows, gamma, mean, rstd, (T*)dx, dgamma, dbeta);
-    BOATCU_LAUNCH_OK("layernorm_bwd_warp");
-    return -1;
-}
-
-static int warp_nv(int type, int64_t cols, const void* a, const void* b, const void* c) {
+// Whether the kernels for rows of 16-byte vectors take this row length and these pointers.
+static bool rows_kernel_fits(int type, int64_t cols, std::initializer_list<const void*> ptrs) {
     const int v = type == BOAT_CUDA_BF16 ? 8 : 4;
-    if (cols % (32 * v) != 0) return 0;
-    const int64_t nv = cols / (32 * v);
-    if (nv != 1 && nv != 2 && nv != 4 && nv != 8) return 0;
-    if ((((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) != 0) return 0;
-    return (int)nv;
+    if (cols % v != 0 || cols / v > kNormMaxRowThreads) return false;
+    for (const void* q : ptrs)
+        if (((uintptr_t)q & 15) != 0) return false;
+    return true;
 }
 
-static int layernorm_fwd_warp(const void* x, int type, int64_t rows, int64_t cols, const float* gamma, const float* beta,
+template <typename T, int NV>
+static int layernorm_fwd_launch(const void* x, int64_t rows, int64_t cols, const float* gamma, const float* beta, float eps, void* y,
+                                float* mean_out, float* rstd_out) {
+    const size_t smem = 2 * (size_t)cols * sizeof(float);
+    int64_t blocks = ceil_div(rows, kNormThreads / 32);
+    if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
+    BOATCU_RUN((layernorm_fwd_rows_kernel<T, NV>), (unsigned)blocks, kNormThreads, smem, (const T*)x, rows, (int)cols, gamma, beta, eps, (T*)y,
+               mean_out, rstd_out);
+    BOATCU_LAUNCH_OK("layernorm_fwd_rows");
+    return 0;
+}
+
+template <typename T>
+static int layernorm_fwd_rows(const void* x, int64_t rows, int64_t cols, const float* gamma, const float* beta,
                               float eps, void* y, float* mean_out, float* rstd_out) {
-    typedef __nv_bfloat16 bf;
-    const int nv = warp_nv(type, cols, x, y, nullptr);
-#define BOAT_LN_FWD(T, NV) case NV: return fwd_warp_launch<T, NV>(x, rows, gamma, beta, eps, y, mean_out, rstd_out)
-    if (type == BOAT_CUDA_BF16) {
-        switch (nv) { BOAT_LN_FWD(bf, 1); BOAT_LN_FWD(bf, 2); BOAT_LN_FWD(bf, 4); BOAT_LN_FWD(bf, 8); default: return 0; }
-    }
-    switch (nv) { BOAT_LN_FWD(float, 1); BOAT_LN_FWD(float, 2); BOAT_LN_FWD(float, 4); BOAT_LN_FWD(float, 8); default: return 0; }
-#undef BOAT_LN_FWD
+    const int64_t nv = ceil_div(cols, 32 * Vec16<T>::N);
+    if (nv <= 1) return layernorm_fwd_launch<T, 1>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
+    if (nv <= 2) return layernorm_fwd_launch<T, 2>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
+    if (nv <= 3) return layernorm_fwd_launch<T, 3>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
+    if (nv <= 4) return layernorm_fwd_launch<T, 4>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
+    return layernorm_fwd_launch<T, 8>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
 }
 
-static int layernorm_bwd_warp(const void* dy, const void* x, int type, int64_t rows, int64_t cols, const float* gamma,
-                              const float* mean, const float* rstd, void* dx, float* dgamma, float* dbeta) {
-    typedef __nv_bfloat16 bf;
-    const int nv = warp_nv(type, cols, dy, x, dx);
-    if (nv > 4) return 0;                           // 8 vectors x 4 live arrays would spill
-#define BOAT_LN_BWD(T, NV) case NV: return bwd_warp_launch<T, NV>(dy, x, rows, gamma, mean, rstd, dx, dgamma, dbeta)
-    if (type == BOAT_CUDA_BF16) {
-        switch (nv) { BOAT_LN_BWD(bf, 1); BOAT_LN_BWD(bf, 2); BOAT_LN_BWD(bf, 4); default: return 0; }
-    }
-    switch (nv) { BOAT_LN_BWD(float, 1); BOAT_LN_BWD(float, 2); BOAT_LN_BWD(float, 4); default: return 0; }
-#undef BOAT_LN_BWD
+template <typename T>
+static int layernorm_bwd_rows(const void* dy, const void* x, int64_t rows, int64_t cols, const float* gamma,
+                              const float* mean, const float* rstd, const void* add, void* dx, float* dgamma, float* dbeta) {
+    const int threads = (int)ceil_div(cols / Vec16<T>::N, 32) * 32;
+    const bool four = rows >= 4 * 2 * (int64_t)sm_count();            // every SM gets two CTAs with four rows at least
+    int64_t blocks = ceil_div(rows, four ? 4 : 1);
+    const int64_t most = (int64_t)sm_count() * (1024 / threads > 8 ? 8 : 1024 / threads);
+    if (blocks > most) blocks = most;
+    void* partial = nullptr;
+    if (dgamma || dbeta)
+        if (int rc = boat_cuda_malloc(&partial, 2 * (size_t)blocks * (size_t)cols * sizeof(float))) return rc;
+    if (four)
+        BOATCU_RUN((layernorm_bwd_rows_kernel<T, 4>), (unsigned)blocks, threads, 0, (const T*)dy, (const T*)x, rows, (int)cols, gamma, mean, rstd,
+                   (const T*)add, (T*)dx, (float*)partial);
+    else
+        BOATCU_RUN((layernorm_bwd_rows_kernel<T, 1>), (unsigned)blocks, threads, 0, (const T*)dy, (const T*)x, rows, (int)cols, gamma, mean, rstd,
+                   (const T*)add, (T*)dx, (float*)partial);
+    BOATCU_LAUNCH_OK("layernorm_bwd_rows");
+    if (!partial) return 0;
+    const void* from[2] = {partial, (const float*)partial + blocks * cols};
+    float* to[2] = {dgamma, dbeta};
+    const int first = dgamma ? 0 : 1, count = (dgamma ? 1 : 0) + (dbeta ? 1 : 0);
+    const int rc = colsum_multi(from + first, BOAT_CUDA_F32, blocks, cols, to + first, count, false);
+    const int freed = boat_cuda_free(partial);
+    return rc ? rc : freed;
 }
 
 }  // namespace boatcu
@@ -531,7 +534,9 @@ int boat_cuda_layernorm_fwd(const void* x, int type, int64_t rows, int64_t cols,
     if (rows > 0x7fffffffLL) return set_error(50, "layernorm: too many rows");
     size_t smem = ((size_t)cols + 32) * sizeof(float);
     ProfileScope prof("layernorm_fwd");
-    if (int done = layernorm_fwd_warp(x, type, rows, cols, gamma, beta, eps, y, mean_out, rstd_out)) return done < 0 ? 0 : done;
+    if (cols <= 8 * 32 * (type == BOAT_CUDA_BF16 ? 8 : 4) && rows_kernel_fits(type, cols, {x, y}))
+        return type == BOAT_CUDA_BF16 ? layernorm_fwd_rows<__nv_bfloat16>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out)
+                                      : layernorm_fwd_rows<float>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
     if (type == BOAT_CUDA_BF16) {
         auto k = layernorm_fwd_kernel<__nv_bfloat16>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -549,14 +554,21 @@ int boat_cuda_layernorm_fwd(const void* x, int type, int64_t rows, int64_t cols,
 
 int boat_cuda_layernorm_bwd(const void* dy, const void* x, int type, int64_t rows, int64_t cols, const float* gamma,
                             const float* mean, const float* rstd, void* dx, float* dgamma, float* dbeta) {
+    return boat_cuda_layernorm_bwd_add(dy, x, type, rows, cols, gamma, mean, rstd, NULL, dx, dgamma, dbeta);
+}
+
+int boat_cuda_layernorm_bwd_add(const void* dy, const void* x, int type, int64_t rows, int64_t cols, const float* gamma,
+                                const float* mean, const float* rstd, const void* add, void* dx, float* dgamma, float* dbeta) {
     if (rows <= 0 || cols <= 0) return 0;
     if (int rc = ensure_init()) return rc;
     if (cols > 12000) return set_error(50, "layernorm: row length %lld exceeds 12000", (long long)cols);
     size_t smem = (2 * (size_t)cols + 32) * sizeof(float);
     ProfileScope prof("layernorm_bwd");
+    if (rows_kernel_fits(type, cols, {dy, x, dx, gamma, add}))
+        return type == BOAT_CUDA_BF16 ? layernorm_bwd_rows<__nv_bfloat16>(dy, x, rows, cols, gamma, mean, rstd, add, dx, dgamma, dbeta)
+                                      : layernorm_bwd_rows<float>(dy, x, rows, cols, gamma, mean, rstd, add, dx, dgamma, dbeta);
     if (dgamma) BOATCU_CHECK(cudaMemsetAsync(dgamma, 0, (size_t)cols * sizeof(float), stream()));
     if (dbeta) BOATCU_CHECK(cudaMemsetAsync(dbeta, 0, (size_t)cols * sizeof(float), stream()));
-    if (int done = layernorm_bwd_warp(dy, x, type, rows, cols, gamma, mean, rstd, dx, dgamma, dbeta)) return done < 0 ? 0 : done;
     dim3 pgrid((unsigned)ceil_div(cols, 32), 1);
     int64_t want = (int64_t)sm_count() * 8 / pgrid.x, max_y = ceil_div(rows, 8);
     pgrid.y = (unsigned)(want < 1 ? 1 : (want > max_y ? max_y : want));
@@ -580,7 +592,7 @@ int boat_cuda_layernorm_bwd(const void* dy, const void* x, int type, int64_t row
             BOATCU_LAUNCH_OK("layernorm_bwd_params");
         }
     }
-    return 0;
+    return add ? boat_cuda_lincomb(dx, dx, 1.0f, add, 1.0f, type, rows * cols) : 0;
 }
 
 int boat_cuda_gelu_fwd(void* y, const void* x, int type, int64_t n) {

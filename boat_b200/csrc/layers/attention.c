@@ -517,7 +517,7 @@ static bool backward_pipelined(boat_attention_t* a, const boat_tensor_t* grad_ou
     {
         const void* x[4] = {a->d_in[0], a->d_in[1], a->d_in[2], a->d_ctx};
         const void* dy[4] = {d_dproj[0], d_dproj[1], d_dproj[2], d_go};
-        if (boat_report("weight gradients", boat_cuda_weight_grads(mma, 4, H, H, T, x, dy, type, d_dw, bias ? d_db : NULL)) != 0)
+        if (boat_report("weight gradients", boat_cuda_weight_grads(mma, 4, H, H, T, x, dy, type, d_dw, bias ? d_db : NULL, 0)) != 0)
             goto done;
     }
     if (a->device != BOAT_DEVICE_CUDA &&
@@ -889,7 +889,7 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
     {
         const void* x[1] = {a->d_ctx};
         const void* dy[1] = {d_go};
-        if (boat_report("dWo", boat_cuda_weight_grads(mma, 1, H, H, T, x, dy, type, &d_dw[WO], bias ? &d_db[WO] : NULL)) != 0) goto done;
+        if (boat_report("dWo", boat_cuda_weight_grads(mma, 1, H, H, T, x, dy, type, &d_dw[WO], bias ? &d_db[WO] : NULL, 0)) != 0) goto done;
     }
     /* Data parallel with overlap: dWo and dbo are final here, long before the step ends - their
      * sum over the ranks runs under the attention-core backward. */
@@ -919,7 +919,7 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
     /* input projections: dW = X^T . dP and db = colsum(dP) first - with overlap their sum over
      * the ranks then runs under the three dX = dP . W^T GEMMs that follow */
     if (boat_report("dW", boat_cuda_weight_grads(mma, 3, H, H, T, (const void* const*)a->d_in, (const void* const*)d_dproj,
-                                                 type, d_dw, bias ? d_db : NULL)) != 0)
+                                                 type, d_dw, bias ? d_db : NULL, 0)) != 0)
         goto done;
     if (overlap && a->grad_overlap == 1) {
         float* piece[2] = {d_dw[WQ], d_db[WQ]};            /* dWq|dWk|dWv and dbq|dbk|dbv are contiguous */

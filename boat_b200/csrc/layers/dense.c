@@ -104,7 +104,7 @@ BOAT_NOINLINE boat_tensor_t* boat_dense_layer_backward(boat_dense_layer_t* l, co
     if (dx && dg && dw && d_dx && d_dw && (!l->bias || d_db) &&
         boat_report("dense dX", boat_cuda_gemm(mma, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, type, NULL)) == 0 &&
         boat_report("dense dW", boat_cuda_weight_grads(mma, 1, I, O, N, (const void* const*)&dx, (const void* const*)&dg,
-                                                       type, &d_dw, l->bias ? &d_db : NULL)) == 0) {
+                                                       type, &d_dw, l->bias ? &d_db : NULL, 0)) == 0) {
         /* accumulate into the layer's gradients, wherever they live */
         boat_tensor_t* grads[2] = {l->grad_weight, l->grad_bias};
         float* fresh[2] = {d_dw, d_db};

@@ -32,6 +32,12 @@ enum { BOAT_CUDA_F32 = 0, BOAT_CUDA_BF16 = 1, BOAT_CUDA_F32_TF32 = 2 };
  *   BF16: tcgen05 kind::f16 on BF16 storage, FP32 accumulate in tensor memory. */
 enum { BOAT_MMA_FP32 = 0, BOAT_MMA_TF32 = 1, BOAT_MMA_BF16 = 2 };
 
+/* What boat_cuda_gemm_fused does to a product before it is stored (z = product + bias):
+ *   GELU:      aux = z, C = GELU(z)                     dense layer and activation
+ *   GELU_GRAD: C = z * dGELU/dx(aux)                    ... and their backward
+ *   ADD:       C = z + aux                              residual connection */
+enum { BOAT_EPI_NONE = 0, BOAT_EPI_GELU = 1, BOAT_EPI_GELU_GRAD = 2, BOAT_EPI_ADD = 3 };
+
 /* ---- runtime: replaces the host-only device stubs of src/core/memory.c:174-186,
  *      :230-247 (allocate / copy / set "on device" were malloc/memcpy/memset) ---------- */
 int         boat_cuda_init(int device);          /* idempotent; device < 0: env BOAT_CUDA_DEVICE or LOCAL_RANK or 0 */
@@ -110,12 +116,24 @@ int boat_cuda_gemm_grouped(int mma, int trans_a, int trans_b, int groups, int64_
                            const void* const* A, int64_t lda, const void* const* B, int64_t ldb, int in_type,
                            void* const* C, int64_t ldc, int out_type, const float* const* bias);
 
+/* C = op(A) . op(B) (+ bias) followed by element-wise work (BOAT_EPI_* above) in the same pass.  A, B, C and
+ * aux have storage type `type`; aux is laid out like C.  The tensor-core kernel does it for BF16 with
+ * C = A.B (GELU, ADD) or A.B^T (GELU_GRAD); other types, layouts and shapes run as separate passes. */
+int boat_cuda_gemm_fused(int mma, int epilogue, int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A,
+                         int64_t lda, const void* B, int64_t ldb, int type, void* C, int64_t ldc, const float* bias, void* aux);
+
+/* C = sum over g of op(A[g]) . op(B[g]) for `groups` (1 to 4) products of one shape, FP32 accumulation
+ * throughout: the gradient of an input that was query, key and value.  Returns 13, without an error text
+ * and without having done anything, where the tensor-core kernel does not cover the shape. */
+int boat_cuda_gemm_sum(int mma, int trans_a, int trans_b, int groups, int64_t M, int64_t N, int64_t K, const void* const* A,
+                       int64_t lda, const void* const* B, int64_t ldb, int in_type, void* C, int64_t ldc, int out_type);
+
 /* Parameter gradients of `groups` (1 to 4) projections y = x.W + b of one shape: dW = X^T . dY and, where
  * db is not NULL, db = column sums of dY (linear_projection_backward, attention.c:1186-1293).  X [T,I]
- * and dY [T,O] of type `in_type`, dW [I,O] and db [O] FP32, all packed; overwritten.  db must be given for
- * all groups or none. */
+ * and dY [T,O] of type `in_type`, dW [I,O] and db [O] FP32, all packed; overwritten, or with `accumulate`
+ * (one group only) added to.  db must be given for all groups or none. */
 int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T, const void* const* X,
-                           const void* const* dY, int in_type, float* const* dW, float* const* db);
+                           const void* const* dY, int in_type, float* const* dW, float* const* db, int accumulate);
 
 /* ---- attention core: replaces scaled_dot_product_attention_impl
  *      (src/layers/attention.c:882-1079) ------------------------------------------------
@@ -186,6 +204,8 @@ int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64
 int boat_cuda_axpy(float* y, const float* x, float alpha, int64_t n);
 /* the same for `count` (1 to 8) pairs in one launch: y[i] += alpha * x[i], n[i] elements each */
 int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, const int64_t* n, int count);
+/* the SGD step of a layer that accumulates: y[i] -= lr * g[i] (rounded product), then g[i] = 0 */
+int boat_cuda_sgd_clear(float* const* y, float* const* g, float lr, const int64_t* n, int count);
 int boat_cuda_scale(float* y, const float* x, float alpha, int64_t n);
 int boat_cuda_add_bias(float* y, const float* x, const float* bias, int64_t rows, int64_t cols);
 int boat_cuda_mul(float* y, const float* a, const float* b, int64_t n);
@@ -211,6 +231,9 @@ int boat_cuda_layernorm_fwd(const void* x, int type, int64_t rows, int64_t cols,
 int boat_cuda_layernorm_bwd(const void* dy, const void* x, int type, int64_t rows, int64_t cols,
                             const float* gamma, const float* mean, const float* rstd,
                             void* dx, float* dgamma, float* dbeta);
+/* ... with a residual branch's gradient `add` (laid out like dx, may be NULL) added to dx in the same pass */
+int boat_cuda_layernorm_bwd_add(const void* dy, const void* x, int type, int64_t rows, int64_t cols, const float* gamma,
+                                const float* mean, const float* rstd, const void* add, void* dx, float* dgamma, float* dbeta);
 int boat_cuda_gelu_fwd(void* y, const void* x, int type, int64_t n);
 int boat_cuda_gelu_bwd(void* dx, const void* dy, const void* x, int type, int64_t n);
 

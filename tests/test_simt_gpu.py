@@ -33,7 +33,7 @@ def test_weight_grads(gpu_lib, mma, shape, groups):
     dw, db = [DeviceBuffer(I * O * 4) for _ in range(groups)], [DeviceBuffer(O * 4) for _ in range(groups)]
     tab = lambda bufs: (C.c_void_p * groups)(*[b.p.value for b in bufs])  # noqa: E731
     check(gpu_lib.boat_cuda_weight_grads(mma, groups, I, O, T, tab(dx), tab(ddy), capi.CUDA_BF16 if bf else capi.CUDA_F32,
-                                         tab(dw), tab(db)), "weight_grads")
+                                         tab(dw), tab(db), 0), "weight_grads")
     check(gpu_lib.boat_cuda_sync(), "sync")
     for g in range(groups):
         assert rel(dw[g].numpy((I, O)), x[g].astype(np.float64).T @ dy[g].astype(np.float64)) <= 1e-5
