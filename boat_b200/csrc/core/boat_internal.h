@@ -27,6 +27,9 @@ boat_tensor_t* boat_tensor_create_uninit(const int64_t* shape, size_t ndim, boat
                                          boat_device_t device);
 /* A CUDA tensor around a buffer from boat_cuda_malloc; the tensor owns the buffer from then on. */
 boat_tensor_t* boat_tensor_adopt_device(const int64_t* shape, size_t ndim, boat_dtype_t dtype, void* device_data);
+/* Gives `t`, of which the caller holds the only reference, another shape of the same element count; the
+ * reference passes to the result (NULL: freed). */
+boat_tensor_t* boat_tensor_with_shape(boat_tensor_t* t, const int64_t* shape, size_t ndim);
 /* A view of `bytes` bytes starting `offset_bytes` into `parent` with its own shape. */
 boat_tensor_t* boat_tensor_window(boat_tensor_t* parent, size_t offset_bytes, const int64_t* shape,
                                   size_t ndim);

@@ -96,6 +96,22 @@ boat_tensor_t* boat_tensor_adopt_device(const int64_t* shape, size_t ndim, boat_
     return t;
 }
 
+boat_tensor_t* boat_tensor_with_shape(boat_tensor_t* t, const int64_t* shape, size_t ndim) {
+    size_t n = 1;
+    for (size_t i = 0; i < ndim; ++i) n *= (size_t)shape[i];
+    int64_t* s = n == t->nelements && t->ref_count == 1 && !t->is_view && ndim > 0
+                     ? (int64_t*)boat_malloc(sizeof(int64_t) * ndim, BOAT_DEVICE_CPU) : NULL;
+    if (!s) {
+        boat_tensor_free(t);
+        return NULL;
+    }
+    memcpy(s, shape, sizeof(int64_t) * ndim);
+    boat_free(t->shape);
+    t->shape = s;
+    t->ndim = ndim;
+    return t;
+}
+
 boat_tensor_t* boat_tensor_create(const int64_t* shape, size_t ndim, boat_dtype_t dtype, boat_device_t device) {
     return create_impl(shape, ndim, dtype, device, true);
 }

@@ -76,6 +76,7 @@ struct FwdParams {
     int units;
     int causal;
     float scale;       // 1/sqrt(hs)
+    int wide;          // O is 32-byte aligned: a whole sector per store
     int group;         // units whose CTAs are scheduled together (their K and V share L2)
     unsigned int* status;
 };
@@ -526,7 +527,13 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                                 o[e] = *reinterpret_cast<uint32_t*>(&h2);
                             }
                         }
-                        st_global_v8(out + c * 32 + x, o);
+                        if (p.wide) {
+                            st_global_v8(out + c * 32 + x, o);
+                        } else {
+                            uint4* dst = reinterpret_cast<uint4*>(out + c * 32 + x);
+                            dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                            dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                        }
                     }
                 }
                 // O has been read before the first P of the next item is announced, and that is what its first

@@ -28,6 +28,7 @@ int launch_fwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     p.units = (int)units;
     p.causal = causal;
     p.scale = scale;
+    p.wide = ((uintptr_t)O & 31) == 0;
     p.status = kernel_status_ptr();
     // units whose K and V (2 * S * hs elements each) together take about a third of L2
     const int64_t group = (40ll << 20) / (2 * S * HS * (int64_t)C::ES);
@@ -110,14 +111,11 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
         configured = true;
     }
     {
-        // the per-row statistics in the form the kernel's inner loops consume them:
-        // -lse * log2(e) and -scale * rowsum(dO o O)
         ProfileScope prof("attn_delta");
-        if (int rc = rowdot_stats(dO, O, BOAT_CUDA_BF16, units, S, n_tiles * kTile, HS, lse, scale, stats2 + stat_rows, stats2)) return rc;
+        if (int rc = attn_bwd_prepare(dO, O, lse, units, S, n_tiles * kTile, HS, scale, stats2 + stat_rows, stats2, dq_accum)) return rc;
     }
     {
         ProfileScope prof("attn_bwd_tc");
-        BOATCU_CHECK(cudaMemsetAsync(dq_accum, 0, n * sizeof(float), stream()));
         const int64_t grid = units * n_tiles;           // one CTA per walk; those on the SMs take the others over
         BOATCU_RUN(kern, (unsigned)grid, kBwdThreads, C::SMEM, mq, mk, mv, mdo, mdq, p);
         BOATCU_LAUNCH_OK("attn_bwd_tc");

@@ -99,11 +99,11 @@ static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // out[r] = sum_d A[r,d]*B[r,d] over [rows, cols] row-major buffers of storage type `type`.
 int rowdot(const void* A, const void* B, int type, int64_t rows, int64_t cols, float* out);
-// The same pass emitting what the BF16 tensor-core backward reads per row:
-// delta2_out[r] = -scale * sum_d dO[r,d]*O[r,d] and lse2_out[r] = -lse[r] * log2(e), each unit of S
-// rows padded to padded_S entries (0 and -inf).  units * padded_S must fit 31 bits.
-int rowdot_stats(const void* dO, const void* O, int type, int64_t units, int64_t S, int64_t padded_S, int64_t cols,
-                 const float* lse, float scale, float* delta2_out, float* lse2_out);
+// What the BF16 tensor-core backward starts from (hs 64 or 128): per row delta2 = -scale * sum_d dO*O and
+// lse2 = -lse * log2(e), each unit of S rows padded to padded_S entries (0 and -inf), and zeros in dq
+// [units*S, hs].  units * padded_S must fit 31 bits.
+int attn_bwd_prepare(const void* dO, const void* O, const float* lse, int64_t units, int64_t S, int64_t padded_S, int64_t hs, float scale,
+                     float* delta2, float* lse2, float* dq);
 
 // CUDA-core (exact FP32 accumulate) implementations, any shape.
 // gemm_simt_grouped: up to four problems of one shape in one launch; bias may be NULL or hold NULLs; with

@@ -187,7 +187,7 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
     if (((uintptr_t)scratch & 255) != 0) return set_error(12, "boat_cuda_attn_bwd: scratch must be 256-byte aligned");
     float* delta = (float*)scratch;
     size_t delta_bytes = ((size_t)units * (size_t)S * sizeof(float) + 255) & ~(size_t)255;
-    tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && attn_tc_supported(mma, units, S, hs, io_type);
+    tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && ((uintptr_t)O & 15) == 0 && attn_tc_supported(mma, units, S, hs, io_type);
     if (!(tensor_cores && mma == BOAT_MMA_BF16)) {      // the BF16 kernel's launcher makes its own, pre-scaled
         ProfileScope prof("attn_delta");
         if (int rc = rowdot(dO, O, io_type, units * S, hs, delta)) return rc;

@@ -392,55 +392,100 @@ static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int c
     return launch_colsum_cluster<T, VEC, 8>(t, rows, cols, count, add);
 }
 
-// ---- delta[r] = sum_d dO[r,d] * O[r,d]: one warp per row, shuffle reduction --------------------
-// With `lse2_out` the kernel emits the two per-row statistics in the form the BF16 backward's inner
-// loops consume them (one FMA each): out[r] = -delta[r] * scale and lse2_out[r] = -lse[r] * log2(e).
-// These are laid out for whole tiles: S rows of a unit take padded_S entries, the surplus ones hold
-// -inf and 0, with which the backward's missing query rows contribute exactly nothing.
-struct RowStats {
-    const float* lse;
-    float* lse2_out;
-    float scale;
-    int S, padded_S;       // equal when there is nothing to pad
-};
-__device__ __forceinline__ void emit_row(float* __restrict__ out, const RowStats& st, int64_t row, int64_t src, float s) {
-    if (st.lse2_out) {
-        out[row] = src < 0 ? 0.f : s * -st.scale;
-        st.lse2_out[row] = src < 0 ? -INFINITY : st.lse[src] * -1.4426950408889634f;
-    } else {
-        out[row] = s;
+// ---- what the BF16 tensor-core backward starts from, in one pass over dO and O --------------------------
+// Per row -delta*scale (delta = sum_d dO*O) and -lse*log2(e), the form its inner loops consume (one FMA each),
+// laid out for whole tiles: S rows of a unit take padded_S entries, the surplus ones hold 0 and -inf, with
+// which missing query rows contribute exactly nothing; and zeros in the FP32 buffer that dQ is summed in.
+// HS/8 lanes per row, 16 bytes each; a thread has the loads of four rows in flight.  HBM-bound: 64 x 8192 x
+// 128 (268 MB read, 268 MB cleared) took 80 us + a 40 us memset as two passes with one row in flight.
+template <int HS>
+__global__ void __launch_bounds__(256) bwd_prepare_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
+                                                          const float* __restrict__ lse, int rows, int S, int padded_S, float scale,
+                                                          float* __restrict__ delta2, float* __restrict__ lse2, float* __restrict__ dq) {
+    constexpr int LANES = HS / 8, ROWS = 256 / LANES, U = 4;
+    griddep_sync();
+    const int l = threadIdx.x % LANES;
+    const int row0 = blockIdx.x * ROWS * U + threadIdx.x / LANES;
+    int64_t src[U];
+    uint4 a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int row = row0 + u * ROWS;
+        src[u] = -1;
+        if (row < rows) {
+            if (S == padded_S) {
+                src[u] = row;
+            } else {
+                const int unit = row / padded_S, r = row - unit * padded_S;
+                if (r < S) src[u] = (int64_t)unit * S + r;
+            }
+        }
+        a[u] = b[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (src[u] >= 0) {
+            a[u] = __ldg(reinterpret_cast<const uint4*>(dO + src[u] * HS + l * 8));
+            b[u] = __ldg(reinterpret_cast<const uint4*>(O + src[u] * HS + l * 8));
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (src[u] >= 0) {
+            float4* z = reinterpret_cast<float4*>(dq + src[u] * HS + l * 8);
+            z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const __nv_bfloat162* ha = reinterpret_cast<const __nv_bfloat162*>(&a[u]);
+        const __nv_bfloat162* hb = reinterpret_cast<const __nv_bfloat162*>(&b[u]);
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 x = __bfloat1622float2(ha[k]), y = __bfloat1622float2(hb[k]);
+            s += x.x * y.x + x.y * y.y;
+        }
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        const int row = row0 + u * ROWS;
+        if (l == 0 && row < rows) {
+            delta2[row] = src[u] < 0 ? 0.f : s * -scale;
+            lse2[row] = src[u] < 0 ? -INFINITY : lse[src[u]] * -1.4426950408889634f;
+        }
     }
 }
-// Input row behind output row `row`, -1 for a padding row.
-__device__ __forceinline__ int64_t source_row(const RowStats& st, int64_t row) {
-    if (st.S == st.padded_S) return row;
-    const int unit = (int)row / st.padded_S, r = (int)row - unit * st.padded_S;
-    return r < st.S ? (int64_t)unit * st.S + r : -1;
+
+int attn_bwd_prepare(const void* dO, const void* O, const float* lse, int64_t units, int64_t S, int64_t padded_S, int64_t hs, float scale,
+                     float* delta2, float* lse2, float* dq) {
+    const int64_t rows = units * padded_S;
+    const int64_t blocks = ceil_div(rows, 256 / (hs / 8) * 4);
+    typedef const __nv_bfloat16* bf;
+    if (hs == 64)
+        BOATCU_RUN(bwd_prepare_kernel<64>, (unsigned)blocks, 256, 0, (bf)dO, (bf)O, lse, (int)rows, (int)S, (int)padded_S, scale, delta2, lse2, dq);
+    else
+        BOATCU_RUN(bwd_prepare_kernel<128>, (unsigned)blocks, 256, 0, (bf)dO, (bf)O, lse, (int)rows, (int)S, (int)padded_S, scale, delta2, lse2, dq);
+    BOATCU_LAUNCH_OK("bwd_prepare");
+    return 0;
 }
 
+// ---- delta[r] = sum_d dO[r,d] * O[r,d]: one warp per row, shuffle reduction --------------------
 template <typename T>
 __global__ void rowdot_kernel(const T* __restrict__ A, const T* __restrict__ B, int64_t rows, int cols,
-                              float* __restrict__ out, const RowStats st) {
+                              float* __restrict__ out) {
     griddep_sync();
     const int lane = threadIdx.x & 31;
     int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (; row < rows; row += step) {
-        const int64_t src = source_row(st, row);
-        const T* a = A + src * cols;
-        const T* b = B + src * cols;
+        const T* a = A + row * cols;
+        const T* b = B + row * cols;
         float s = 0.f;
-        for (int d = lane; d < cols && src >= 0; d += 32) s += to_f32(a[d]) * to_f32(b[d]);
+        for (int d = lane; d < cols; d += 32) s += to_f32(a[d]) * to_f32(b[d]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) emit_row(out, st, row, src, s);
+        if (lane == 0) out[row] = s;
     }
 }
 
 // 128-bit variant: 8 bf16 (or 4 floats) per lane per access; cols must divide accordingly.
 template <typename T, int VEC>
 __global__ void rowdot_vec_kernel(const T* __restrict__ A, const T* __restrict__ B, int64_t rows, int cols,
-                                  float* __restrict__ out, const RowStats st) {
+                                  float* __restrict__ out) {
     griddep_sync();
     const int lanes_per_row = cols / VEC;            // power of two <= 32 checked by the launcher
     const int rows_per_warp = 32 / lanes_per_row;
@@ -451,10 +496,9 @@ __global__ void rowdot_vec_kernel(const T* __restrict__ A, const T* __restrict__
     for (int64_t base = warp * rows_per_warp; base < rows; base += nwarps * rows_per_warp) {
         int64_t row = base + sub;
         float s = 0.f;
-        const int64_t src = row < rows ? source_row(st, row) : -1;
-        if (src >= 0) {
-            const uint4 va = *reinterpret_cast<const uint4*>(A + src * cols + l * VEC);
-            const uint4 vb = *reinterpret_cast<const uint4*>(B + src * cols + l * VEC);
+        if (row < rows) {
+            const uint4 va = *reinterpret_cast<const uint4*>(A + row * cols + l * VEC);
+            const uint4 vb = *reinterpret_cast<const uint4*>(B + row * cols + l * VEC);
             if (sizeof(T) == 4) {
                 const float* fa = reinterpret_cast<const float*>(&va);
                 const float* fb = reinterpret_cast<const float*>(&vb);
@@ -471,11 +515,11 @@ __global__ void rowdot_vec_kernel(const T* __restrict__ A, const T* __restrict__
             }
         }
         for (int o = lanes_per_row >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (l == 0 && row < rows) emit_row(out, st, row, src, s);
+        if (l == 0 && row < rows) out[row] = s;
     }
 }
 
-static int rowdot_launch(const void* A, const void* B, int type, int64_t rows, int64_t cols, float* out, const RowStats st) {
+int rowdot(const void* A, const void* B, int type, int64_t rows, int64_t cols, float* out) {
     if (rows <= 0) return 0;
     if (int rc = ensure_init()) return rc;
     const int vec = type == BOAT_CUDA_BF16 ? 8 : 4;
@@ -486,28 +530,19 @@ static int rowdot_launch(const void* A, const void* B, int type, int64_t rows, i
         int grid = grid_for(rows, rows_per_block);
         if (type == BOAT_CUDA_BF16)
             BOATCU_RUN((rowdot_vec_kernel<__nv_bfloat16, 8>), grid, kThreads, 0, 
-                (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, rows, (int)cols, out, st);
+                (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, rows, (int)cols, out);
         else
-            BOATCU_RUN((rowdot_vec_kernel<float, 4>), grid, kThreads, 0, (const float*)A, (const float*)B, rows, (int)cols, out, st);
+            BOATCU_RUN((rowdot_vec_kernel<float, 4>), grid, kThreads, 0, (const float*)A, (const float*)B, rows, (int)cols, out);
     } else {
         int grid = grid_for(rows, kThreads / 32);
         if (type == BOAT_CUDA_BF16)
             BOATCU_RUN(rowdot_kernel<__nv_bfloat16>, grid, kThreads, 0, 
-                (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, rows, (int)cols, out, st);
+                (const __nv_bfloat16*)A, (const __nv_bfloat16*)B, rows, (int)cols, out);
         else
-            BOATCU_RUN(rowdot_kernel<float>, grid, kThreads, 0, (const float*)A, (const float*)B, rows, (int)cols, out, st);
+            BOATCU_RUN(rowdot_kernel<float>, grid, kThreads, 0, (const float*)A, (const float*)B, rows, (int)cols, out);
     }
     BOATCU_LAUNCH_OK("rowdot");
     return 0;
-}
-
-int rowdot(const void* A, const void* B, int type, int64_t rows, int64_t cols, float* out) {
-    return rowdot_launch(A, B, type, rows, cols, out, RowStats{nullptr, nullptr, 0.f, 0, 0});
-}
-
-int rowdot_stats(const void* dO, const void* O, int type, int64_t units, int64_t S, int64_t padded_S, int64_t cols,
-                 const float* lse, float scale, float* delta2_out, float* lse2_out) {
-    return rowdot_launch(dO, O, type, units * padded_S, cols, delta2_out, RowStats{lse, lse2_out, scale, (int)S, (int)padded_S});
 }
 
 // ---- out[b, j, i] = in[b, i, j], 32x32 shared-memory tiles --------------------------------------

@@ -19,6 +19,7 @@
  *     (the reference replaces the tensors, :653-654, :702-703 - same "no accumulation").
  */
 #include "../core/stage.h"
+#include "fused.h"
 #include <boat/layers.h>
 #include <boat_b200.h>
 #include <math.h>
@@ -600,9 +601,11 @@ void boat_attention_free(boat_attention_t* a) {
 
 /* The step itself, for T token rows holding `units` (batch, head) units of sequence length S; `gran`
  * units form one indivisible piece when host tensors are moved in chunks.  Inputs are [.., H]
- * tensors of T*H elements each; the result has the query's shape. */
+ * tensors of T*H elements each; the result has the query's shape.  A CUDA `residual` of the query's dtype
+ * is added to the result. */
 static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
-                                   const boat_tensor_t* value, int64_t T, int64_t S, int64_t units, int64_t gran) {
+                                   const boat_tensor_t* value, int64_t T, int64_t S, int64_t units, int64_t gran,
+                                   const boat_tensor_t* residual) {
     const boat_tensor_t* in[3] = {query, key, value};
     const int64_t H = (int64_t)a->config.hidden_size, hs = (int64_t)a->config.head_size;
     if (boat_report("CUDA start-up", boat_cuda_init(-1)) != 0) return NULL;
@@ -684,8 +687,14 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
             /* a CUDA result is the GEMM's own output buffer: no copy */
             result = boat_tensor_create_uninit(query->shape, query->ndim, query->dtype, BOAT_DEVICE_CUDA);
             if (!result) goto done;
-            if (boat_report("output projection", boat_cuda_gemm(mma, 0, 0, T, H, H, a->d_ctx, H, p.w[WO], H, type,
-                                                                result->data, H, out_type, p.b[WO])) != 0) {
+            int rc;
+            if (residual && out_type == type)
+                rc = boat_cuda_gemm_fused(mma, BOAT_EPI_ADD, 0, 0, T, H, H, a->d_ctx, H, p.w[WO], H, type, result->data, H, p.b[WO], residual->data);
+            else
+                rc = boat_cuda_gemm(mma, 0, 0, T, H, H, a->d_ctx, H, p.w[WO], H, type, result->data, H, out_type, p.b[WO]);
+            if (rc == 0 && residual && out_type != type)
+                rc = boat_cuda_lincomb(result->data, result->data, 1.0f, residual->data, 1.0f, out_type, T * H);
+            if (boat_report("output projection", rc) != 0) {
                 boat_tensor_free(result);
                 result = NULL;
                 goto done;
@@ -722,9 +731,8 @@ done:
     return result;
 }
 
-boat_tensor_t* boat_attention_forward(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
-                                      const boat_tensor_t* value, const boat_tensor_t* attention_mask) {
-    (void)attention_mask;                       /* ignored, as in the reference (attention.c:1022-1025) */
+static boat_tensor_t* forward_batch(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
+                                    const boat_tensor_t* value, const boat_tensor_t* residual) {
     if (!a || !query || !key || !value) return NULL;
     const boat_tensor_t* in[3] = {query, key, value};
     const int64_t H = (int64_t)a->config.hidden_size, nh = (int64_t)a->config.num_heads;
@@ -736,7 +744,17 @@ boat_tensor_t* boat_attention_forward(boat_attention_t* a, const boat_tensor_t* 
             in[i]->shape[2] != H)
             return NULL;
     }
-    return forward_rows(a, query, key, value, B * S, S, B * nh, nh);
+    return forward_rows(a, query, key, value, B * S, S, B * nh, nh, residual);
+}
+
+boat_tensor_t* boat_attention_forward(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
+                                      const boat_tensor_t* value, const boat_tensor_t* attention_mask) {
+    (void)attention_mask;                       /* ignored, as in the reference (attention.c:1022-1025) */
+    return forward_batch(a, query, key, value, NULL);
+}
+
+boat_tensor_t* boat_attention_forward_add(boat_attention_t* a, const boat_tensor_t* x, const boat_tensor_t* residual) {
+    return forward_batch(a, x, x, x, residual);
 }
 
 /* A contiguous range of (batch, head) units of a larger [B,S,H] problem, given only the token rows
@@ -761,7 +779,7 @@ boat_tensor_t* boat_attention_forward_units(boat_attention_t* a, const boat_tens
     const int64_t R = query->shape[0];
     for (int i = 0; i < 3; ++i)
         if (!dtype_ok(in[i]->dtype) || in[i]->ndim != 2 || in[i]->shape[0] != R || in[i]->shape[1] != H) return NULL;
-    return forward_rows(a, query, key, value, R, seq_len, R / unit_rows, 1);
+    return forward_rows(a, query, key, value, R, seq_len, R / unit_rows, 1, NULL);
 }
 
 /* ---- backward ------------------------------------------------------------------------------ */
@@ -790,8 +808,9 @@ static bool ensure_grads(boat_attention_t* a) {
     return true;
 }
 
-bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_output, boat_tensor_t** grad_query,
-                             boat_tensor_t** grad_key, boat_tensor_t** grad_value) {
+/* `sum`: one tensor was query, key and value; *grad_query gets its gradient, the others nothing. */
+static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output, boat_tensor_t** grad_query,
+                          boat_tensor_t** grad_key, boat_tensor_t** grad_value, bool sum) {
     if (!a || !grad_output) {
         printf("[ERROR] boat_attention_backward: invalid arguments\n");
         return false;
@@ -848,6 +867,7 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
     /* gradients are produced in HBM; host results are copied down together at the end */
     for (int i = 0; i < 3 && !pipelined; ++i) {
         const boat_tensor_t* x = a->cache_in[i];
+        if (sum && i > 0) break;
         gin[i] = boat_tensor_create_uninit(x->shape, x->ndim, x->dtype, x->device);
         if (!gin[i]) goto done;
         if (x->device == BOAT_DEVICE_CUDA) continue;
@@ -930,7 +950,23 @@ bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_outp
     }
     const bool yield = overlap && a->grad_overlap == 1;      /* a sum was just started beside these GEMMs */
     if (yield) boat_cuda_gemm_set_yielding(1);
-    {
+    if (sum) {
+        /* the three input gradients are one: summed in the accumulator, or - where the tensor cores do not
+         * take the shape - product by product */
+        const int out_type = storage_of(gin[0]->dtype);
+        void* target = gin[0]->device == BOAT_DEVICE_CUDA ? gin[0]->data : d_down;
+        int rc = boat_cuda_gemm_sum(mma, 0, 1, 3, T, H, H, (const void* const*)d_dproj, H, (const void* const*)p.w, H, type, target, H, out_type);
+        if (rc == 13) {
+            void* term = dev_alloc((size_t)T * H * storage_size(out_type));
+            rc = term ? boat_cuda_gemm(mma, 0, 1, T, H, H, d_dproj[0], H, p.w[0], H, type, target, H, out_type, NULL) : 1;
+            for (int i = 1; i < 3 && rc == 0; ++i) {
+                rc = boat_cuda_gemm(mma, 0, 1, T, H, H, d_dproj[i], H, p.w[i], H, type, term, H, out_type, NULL);
+                if (rc == 0) rc = boat_cuda_lincomb(target, target, 1.0f, term, 1.0f, out_type, T * H);
+            }
+            dev_free(term);
+        }
+        if (boat_report("dX", rc) != 0) goto done;
+    } else {
         /* dX = dP . W^T for the three inputs, each straight into its tensor's HBM or the block that goes
          * down: one launch when they share the dtype */
         const int out_type = storage_of(gin[0]->dtype);
@@ -974,9 +1010,19 @@ done:
     boat_tensor_t** outp[3] = {grad_query, grad_key, grad_value};
     for (int i = 0; i < 3; ++i) {
         if (outp[i]) *outp[i] = gin[i];
-        else boat_tensor_free(gin[i]);
+        else if (gin[i]) boat_tensor_free(gin[i]);
     }
     return true;
+}
+
+bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_output, boat_tensor_t** grad_query,
+                             boat_tensor_t** grad_key, boat_tensor_t** grad_value) {
+    return backward_impl(a, grad_output, grad_query, grad_key, grad_value, false);
+}
+
+boat_tensor_t* boat_attention_backward_self(boat_attention_t* a, const boat_tensor_t* grad_output) {
+    boat_tensor_t* g = NULL;
+    return backward_impl(a, grad_output, &g, NULL, NULL, true) ? g : NULL;
 }
 
 /* ---- update / setters ------------------------------------------------------------------------ */

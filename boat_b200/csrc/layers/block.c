@@ -8,8 +8,11 @@
  * them; this is the chaining a caller would write with the layer API, kept inside the library so
  * that a step is two calls and the sixty-odd kernel launches of a step are issued back to back.
  * The layers are borrowed: create, fill, place (to_device) and free them with their own API.
- * Works on host or CUDA tensors like the layers it calls. */
-#include "../core/boat_internal.h"
+ * Works on host or CUDA tensors like the layers it calls.  On CUDA tensors the element-wise steps between the
+ * layers are folded into them (fused.h): GELU and its derivative and the residual adds run in the epilogues
+ * of the dense and output projections and in the LayerNorm backward, the three input gradients of the
+ * attention layer are summed in one product - fourteen passes over [T, d] and [T, 4d] tensors less per step. */
+#include "fused.h"
 #include <boat_b200.h>
 #include <boat/ops.h>
 
@@ -77,6 +80,22 @@ boat_tensor_t* boat_encoder_block_forward(boat_encoder_block_t* b, const boat_te
     if (b->u) b->u = drop(b->u, NULL);
     for (int i = 0; i < 3; ++i) b->shape[i] = x->shape[i];
     h1 = boat_layernorm_forward(b->ln1, x);
+    if (x->device == BOAT_DEVICE_CUDA) {
+        r1 = h1 ? boat_attention_forward_add(b->attn, h1, x) : NULL;
+        h2 = r1 ? boat_layernorm_forward(b->ln2, r1) : NULL;
+        h2f = h2 ? boat_tensor_reshape(h2, flat, 2) : NULL;
+        act = h2f ? boat_dense_forward_gelu(b->fc1, h2f, &u) : NULL;
+        m = act ? boat_dense_forward_add(b->fc2, act, r1) : NULL;
+        /* the block's result under the input's shape */
+        out = m ? boat_tensor_with_shape(m, x->shape, 3) : NULL;
+        m = NULL;
+        if (out) {
+            b->u = u;
+            u = NULL;
+        }
+        drop(h1, NULL); drop(r1, NULL); drop(h2f, NULL); drop(h2, NULL); drop(u, NULL); drop(act, NULL);
+        return out;
+    }
     att = h1 ? boat_attention_forward(b->attn, h1, h1, h1, NULL) : NULL;
     r1 = att ? boat_lincomb(x, 1.0f, att, 1.0f) : NULL;
     h2 = r1 ? boat_layernorm_forward(b->ln2, r1) : NULL;
@@ -116,34 +135,43 @@ boat_tensor_t* boat_encoder_block_backward(boat_encoder_block_t* b, const boat_t
     b->sums_begun = false;
     /* MLP branch: out = r1 + dense2(GELU(dense1(LN2(r1)))) */
     g2 = boat_tensor_reshape(grad_output, flat, 2);
-    da = g2 ? boat_dense_layer_backward(b->fc2, g2) : NULL;
-    if (da && begun) {
+    const bool cuda = grad_output->device == BOAT_DEVICE_CUDA && b->u->device == BOAT_DEVICE_CUDA && grad_output->dtype == b->u->dtype;
+    if (cuda) du = g2 ? boat_dense_backward_gelu(b->fc2, g2, b->u) : NULL;
+    else      da = g2 ? boat_dense_layer_backward(b->fc2, g2) : NULL;
+    if ((da || du) && begun) {
         boat_tensor_t* const t[2] = {boat_dense_layer_get_grad_weight(b->fc2), boat_dense_layer_get_grad_bias(b->fc2)};
         begun = begin_sums(t, 2);
         b->sums_in_flight = begun;
     }
-    du = da ? boat_gelu_backward(da, b->u) : NULL;
+    if (!cuda) du = da ? boat_gelu_backward(da, b->u) : NULL;
     dh2 = du ? boat_dense_layer_backward(b->fc1, du) : NULL;
     if (dh2 && begun) {
         boat_tensor_t* const t[2] = {boat_dense_layer_get_grad_weight(b->fc1), boat_dense_layer_get_grad_bias(b->fc1)};
         begun = begin_sums(t, 2);
     }
     dh2_3 = dh2 ? boat_tensor_reshape(dh2, b->shape, 3) : NULL;
-    dln2 = dh2_3 ? boat_layernorm_backward(b->ln2, dh2_3) : NULL;
-    dr1 = dln2 ? boat_lincomb(grad_output, 1.0f, dln2, 1.0f) : NULL;
+    if (cuda) {
+        dr1 = dh2_3 ? boat_layernorm_backward_add(b->ln2, dh2_3, grad_output) : NULL;
+    } else {
+        dln2 = dh2_3 ? boat_layernorm_backward(b->ln2, dh2_3) : NULL;
+        dr1 = dln2 ? boat_lincomb(grad_output, 1.0f, dln2, 1.0f) : NULL;
+    }
     /* attention branch: r1 = x + attention(LN1(x)), query = key = value */
-    if (dr1 && boat_attention_backward(b->attn, dr1, &gq, &gk, &gv)) {
+    if (cuda) {
+        dh1 = dr1 ? boat_attention_backward_self(b->attn, dr1) : NULL;
+        dx = dh1 ? boat_layernorm_backward_add(b->ln1, dh1, dr1) : NULL;
+    } else if (dr1 && boat_attention_backward(b->attn, dr1, &gq, &gk, &gv)) {
         s1 = boat_lincomb(gq, 1.0f, gk, 1.0f);
         dh1 = s1 ? boat_lincomb(s1, 1.0f, gv, 1.0f) : NULL;
         dln1 = dh1 ? boat_layernorm_backward(b->ln1, dh1) : NULL;
         dx = dln1 ? boat_lincomb(dr1, 1.0f, dln1, 1.0f) : NULL;
-        if (dx && begun) {
-            /* the four small LayerNorm gradients as one group */
-            boat_tensor_t* const t[4] = {boat_layernorm_get_grad_weight(b->ln1), boat_layernorm_get_grad_bias(b->ln1),
-                                         boat_layernorm_get_grad_weight(b->ln2), boat_layernorm_get_grad_bias(b->ln2)};
-            begun = begin_sums(t, 4);
-            b->sums_begun = begun;
-        }
+    }
+    if (dx && begun) {
+        /* the four small LayerNorm gradients as one group */
+        boat_tensor_t* const t[4] = {boat_layernorm_get_grad_weight(b->ln1), boat_layernorm_get_grad_bias(b->ln1),
+                                     boat_layernorm_get_grad_weight(b->ln2), boat_layernorm_get_grad_bias(b->ln2)};
+        begun = begin_sums(t, 4);
+        b->sums_begun = begun;
     }
     drop(g2, NULL); drop(da, NULL); drop(du, NULL); drop(dh2_3, NULL); drop(dh2, NULL); drop(dln2, NULL);
     drop(dr1, NULL); drop(gq, NULL); drop(gk, NULL); drop(gv, NULL); drop(s1, NULL); drop(dh1, NULL); drop(dln1, NULL);

@@ -7,6 +7,7 @@
  * p -= lr*g followed by clearing the gradients (:299-327).  The contractions are the same
  * tcgen05 / CUDA-core GEMMs the attention projections use. */
 #include "../core/stage.h"
+#include "fused.h"
 #include <boat/layers.h>
 #include <boat/ops.h>
 #include <boat_b200.h>
@@ -19,6 +20,11 @@ struct boat_dense_layer_t {
     bool use_bias;
     boat_tensor_t *weight, *bias, *grad_weight, *grad_bias;
     boat_tensor_t* cache_input;
+    /* BF16 copy of a CUDA weight, made by a forward and used again by the backward that follows it; trusted
+     * only in between, and not after a call that hands out or changes the weight (as the attention
+     * layer's, see there). */
+    void* shadow;
+    bool shadow_fresh;
 };
 
 boat_dense_layer_t* boat_dense_layer_create(size_t input_features, size_t output_features, bool use_bias) {
@@ -50,10 +56,33 @@ void boat_dense_layer_free(boat_dense_layer_t* l) {
     boat_tensor_t* all[5] = {l->weight, l->bias, l->grad_weight, l->grad_bias, l->cache_input};
     for (int i = 0; i < 5; ++i)
         if (all[i]) boat_tensor_free(all[i]);
+    boat_dev_free(l->shadow);
     boat_free(l);
 }
 
-boat_tensor_t* boat_dense_layer_forward(boat_dense_layer_t* l, const boat_tensor_t* input) {
+/* The weight as an operand of storage `type` (*owned as boat_stage_in). */
+static void* stage_weight(boat_dense_layer_t* l, int type, bool backward, bool* owned) {
+    const boat_tensor_t* w = l->weight;
+    *owned = false;
+    if (type != BOAT_CUDA_BF16 || w->device != BOAT_DEVICE_CUDA || w->dtype != BOAT_DTYPE_FLOAT32)
+        return boat_stage_in(w, type, owned);
+    if (!l->shadow) {
+        l->shadow = boat_dev_alloc(l->in_features * l->out_features * 2);
+        l->shadow_fresh = false;
+        if (!l->shadow) return NULL;
+    }
+    const bool fresh = backward && l->shadow_fresh;
+    l->shadow_fresh = false;
+    if (!fresh && boat_report("weight conversion", boat_cuda_cast(l->shadow, BOAT_CUDA_BF16, w->data, BOAT_CUDA_F32, (int64_t)w->nelements)) != 0)
+        return NULL;
+    l->shadow_fresh = !backward;
+    return l->shadow;
+}
+
+/* Forward with element-wise work behind the product (BOAT_EPI_*; fused.h): `aux` is the residual to add (ADD),
+ * or receives the pre-activation (GELU). */
+static boat_tensor_t* dense_forward(boat_dense_layer_t* l, const boat_tensor_t* input, int epilogue, const boat_tensor_t* residual,
+                                    boat_tensor_t** pre_activation) {
     if (!l || !input) return NULL;
     boat_tensor_ref((boat_tensor_t*)input);
     if (l->cache_input) boat_tensor_unref(l->cache_input);
@@ -62,16 +91,29 @@ boat_tensor_t* boat_dense_layer_forward(boat_dense_layer_t* l, const boat_tensor
     if (boat_report("CUDA start-up", boat_cuda_init(-1)) != 0) return NULL;
     const int mma = boat_default_mma(input->dtype), type = boat_storage_of(input->dtype);
     const int64_t N = input->shape[0], I = (int64_t)l->in_features, O = (int64_t)l->out_features;
+    const int64_t oshape[2] = {N, O};
     bool xo = false, wo = false, bo = false;
     void* dx = boat_stage_in(input, type, &xo);
-    void* dw = boat_stage_in(l->weight, type, &wo);
+    void* dw = stage_weight(l, type, false, &wo);
     float* db = l->bias ? (float*)boat_stage_in(l->bias, BOAT_CUDA_F32, &bo) : NULL;
     void* dy = boat_dev_alloc((size_t)N * O * boat_storage_size(type));
+    void* aux = epilogue == BOAT_EPI_GELU ? boat_dev_alloc((size_t)N * O * boat_storage_size(type))
+                                          : (residual ? residual->data : NULL);
     boat_tensor_t* out = NULL;
-    const int64_t oshape[2] = {N, O};
-    if (dx && dw && dy && (!l->bias || db) &&
-        boat_report("dense forward", boat_cuda_gemm(mma, 0, 0, N, O, I, dx, I, dw, O, type, dy, O, type, db)) == 0)
-        out = boat_emit_out_take(oshape, 2, input, &dy, type);
+    if (dx && dw && dy && (!l->bias || db) && (epilogue == BOAT_EPI_NONE || aux)) {
+        const int rc = epilogue == BOAT_EPI_NONE
+                           ? boat_cuda_gemm(mma, 0, 0, N, O, I, dx, I, dw, O, type, dy, O, type, db)
+                           : boat_cuda_gemm_fused(mma, epilogue, 0, 0, N, O, I, dx, I, dw, O, type, dy, O, db, aux);
+        if (boat_report("dense forward", rc) == 0) out = boat_emit_out_take(oshape, 2, input, &dy, type);
+        if (out && epilogue == BOAT_EPI_GELU) {
+            *pre_activation = boat_emit_out_take(oshape, 2, input, &aux, type);
+            if (!*pre_activation) {
+                boat_tensor_free(out);
+                out = NULL;
+            }
+        }
+    }
+    if (epilogue == BOAT_EPI_GELU) boat_dev_free(aux);
     boat_dev_free(dy);
     if (xo) boat_dev_free(dx);
     if (wo) boat_dev_free(dw);
@@ -79,7 +121,21 @@ boat_tensor_t* boat_dense_layer_forward(boat_dense_layer_t* l, const boat_tensor
     return out;
 }
 
-BOAT_NOINLINE boat_tensor_t* boat_dense_layer_backward(boat_dense_layer_t* l, const boat_tensor_t* grad_output) {
+boat_tensor_t* boat_dense_layer_forward(boat_dense_layer_t* l, const boat_tensor_t* input) {
+    return dense_forward(l, input, BOAT_EPI_NONE, NULL, NULL);
+}
+
+boat_tensor_t* boat_dense_forward_gelu(boat_dense_layer_t* l, const boat_tensor_t* input, boat_tensor_t** pre_activation) {
+    *pre_activation = NULL;
+    return dense_forward(l, input, BOAT_EPI_GELU, NULL, pre_activation);
+}
+
+boat_tensor_t* boat_dense_forward_add(boat_dense_layer_t* l, const boat_tensor_t* input, const boat_tensor_t* residual) {
+    return dense_forward(l, input, BOAT_EPI_ADD, residual, NULL);
+}
+
+/* Backward; with `pre_activation` the layer's input was GELU of it, and its gradient is returned. */
+static boat_tensor_t* dense_backward(boat_dense_layer_t* l, const boat_tensor_t* grad_output, const boat_tensor_t* pre_activation) {
     if (!l || !grad_output || !l->cache_input) return NULL;
     const boat_tensor_t* x = l->cache_input;
     if (x->ndim != 2 || grad_output->ndim != 2) {
@@ -96,36 +152,35 @@ BOAT_NOINLINE boat_tensor_t* boat_dense_layer_backward(boat_dense_layer_t* l, co
     bool xo = false, go = false, wo = false;
     void* dx = boat_stage_in(x, type, &xo);
     void* dg = boat_stage_in(grad_output, type, &go);
-    void* dw = boat_stage_in(l->weight, type, &wo);
+    void* dw = stage_weight(l, type, true, &wo);
     void* d_dx = boat_dev_alloc((size_t)N * I * boat_storage_size(type));
-    float* d_dw = (float*)boat_dev_alloc((size_t)I * O * sizeof(float));
-    float* d_db = l->bias ? (float*)boat_dev_alloc((size_t)O * sizeof(float)) : NULL;
-    boat_tensor_t* out = NULL;
-    if (dx && dg && dw && d_dx && d_dw && (!l->bias || d_db) &&
-        boat_report("dense dX", boat_cuda_gemm(mma, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, type, NULL)) == 0 &&
-        boat_report("dense dW", boat_cuda_weight_grads(mma, 1, I, O, N, (const void* const*)&dx, (const void* const*)&dg,
-                                                       type, &d_dw, l->bias ? &d_db : NULL, 0)) == 0) {
-        /* accumulate into the layer's gradients, wherever they live */
-        boat_tensor_t* grads[2] = {l->grad_weight, l->grad_bias};
-        float* fresh[2] = {d_dw, d_db};
-        int rc = 0;
-        for (int i = 0; i < 2 && rc == 0; ++i) {
-            boat_tensor_t* g = grads[i];
-            if (!g || !fresh[i]) continue;
-            if (g->device == BOAT_DEVICE_CUDA) {
-                rc = boat_cuda_axpy((float*)g->data, fresh[i], 1.0f, (int64_t)g->nelements);
-            } else {
-                float* acc = (float*)boat_dev_alloc(g->nbytes);
-                rc = acc ? boat_cuda_memcpy_h2d(acc, g->data, g->nbytes) : 1;
-                if (rc == 0) rc = boat_cuda_axpy(acc, fresh[i], 1.0f, (int64_t)g->nelements);
-                if (rc == 0) rc = boat_cuda_memcpy_d2h(g->data, acc, g->nbytes);
-                boat_dev_free(acc);
-            }
-        }
-        if (boat_report("dense gradient accumulation", rc) == 0) out = boat_emit_out_take(x->shape, 2, x, &d_dx, type);
+    /* CUDA gradients are added to where they lie; others take a trip through HBM */
+    boat_tensor_t* grads[2] = {l->grad_weight, l->grad_bias};
+    float* target[2] = {NULL, NULL};
+    bool staged[2] = {false, false};
+    int rc = 0;
+    for (int i = 0; i < 2 && rc == 0; ++i) {
+        boat_tensor_t* g = i == 1 && !l->bias ? NULL : grads[i];
+        if (!g) continue;
+        staged[i] = g->device != BOAT_DEVICE_CUDA;
+        target[i] = staged[i] ? (float*)boat_dev_alloc(g->nbytes) : (float*)g->data;
+        if (!target[i]) rc = 1;
+        else if (staged[i]) rc = boat_cuda_memcpy_h2d(target[i], g->data, g->nbytes);
     }
-    boat_dev_free(d_db);
-    boat_dev_free(d_dw);
+    /* a bias set on a layer created without one has no gradient tensor to add to: its gradient is dropped */
+    boat_tensor_t* out = NULL;
+    if (rc == 0 && dx && dg && dw && d_dx && target[0]) {
+        rc = pre_activation ? boat_cuda_gemm_fused(mma, BOAT_EPI_GELU_GRAD, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, NULL, pre_activation->data)
+                            : boat_cuda_gemm(mma, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, type, NULL);
+        if (rc == 0)
+            rc = boat_cuda_weight_grads(mma, 1, I, O, N, (const void* const*)&dx, (const void* const*)&dg, type, &target[0],
+                                        target[1] ? &target[1] : NULL, 1);
+        for (int i = 0; i < 2 && rc == 0; ++i)
+            if (staged[i] && target[i]) rc = boat_cuda_memcpy_d2h(grads[i]->data, target[i], grads[i]->nbytes);
+        if (boat_report("dense backward", rc) == 0) out = boat_emit_out_take(x->shape, 2, x, &d_dx, type);
+    }
+    for (int i = 0; i < 2; ++i)
+        if (staged[i]) boat_dev_free(target[i]);
     boat_dev_free(d_dx);
     if (xo) boat_dev_free(dx);
     if (go) boat_dev_free(dg);
@@ -133,9 +188,35 @@ BOAT_NOINLINE boat_tensor_t* boat_dense_layer_backward(boat_dense_layer_t* l, co
     return out;
 }
 
+BOAT_NOINLINE boat_tensor_t* boat_dense_layer_backward(boat_dense_layer_t* l, const boat_tensor_t* grad_output) {
+    return dense_backward(l, grad_output, NULL);
+}
+
+boat_tensor_t* boat_dense_backward_gelu(boat_dense_layer_t* l, const boat_tensor_t* grad_output, const boat_tensor_t* pre_activation) {
+    return dense_backward(l, grad_output, pre_activation);
+}
+
 BOAT_NOINLINE void boat_dense_layer_update(boat_dense_layer_t* l, float learning_rate) {
     if (!l) return;
+    l->shadow_fresh = false;
     boat_tensor_t* pairs[2][2] = {{l->weight, l->grad_weight}, {l->bias, l->grad_bias}};
+    float *w_cuda[2], *g_cuda[2];
+    int64_t n_cuda[2];
+    int count = 0;
+    bool all_cuda = true;
+    for (int i = 0; i < 2; ++i) {
+        boat_tensor_t *w = pairs[i][0], *g = pairs[i][1];
+        if (!w || !g) continue;
+        all_cuda = all_cuda && w->device == BOAT_DEVICE_CUDA && g->device == BOAT_DEVICE_CUDA &&
+                   w->dtype == BOAT_DTYPE_FLOAT32 && g->dtype == BOAT_DTYPE_FLOAT32 && w->nelements == g->nelements;
+        w_cuda[count] = (float*)w->data;
+        g_cuda[count] = (float*)g->data;
+        n_cuda[count++] = (int64_t)w->nelements;
+    }
+    if (all_cuda) {                                             /* the step and the clearing in one pass */
+        boat_report("dense update", boat_cuda_sgd_clear(w_cuda, g_cuda, learning_rate, n_cuda, count));
+        return;
+    }
     for (int i = 0; i < 2; ++i) {
         boat_tensor_t *w = pairs[i][0], *g = pairs[i][1];
         if (!w || !g) continue;
@@ -158,7 +239,7 @@ static void replace(boat_tensor_t** slot, boat_tensor_t* t) {
 void boat_dense_layer_set_weight(boat_dense_layer_t* l, boat_tensor_t* weight) {
     if (l && weight && weight->ndim == 2 && weight->shape[0] == (int64_t)l->in_features &&
         weight->shape[1] == (int64_t)l->out_features)
-        replace(&l->weight, weight);
+        replace(&l->weight, weight), l->shadow_fresh = false;
 }
 
 void boat_dense_layer_set_bias(boat_dense_layer_t* l, boat_tensor_t* bias) {
@@ -168,13 +249,20 @@ void boat_dense_layer_set_bias(boat_dense_layer_t* l, boat_tensor_t* bias) {
     }
 }
 
-boat_tensor_t* boat_dense_layer_get_weight(const boat_dense_layer_t* l) { return l ? l->weight : NULL; }
+boat_tensor_t* boat_dense_layer_get_weight(const boat_dense_layer_t* l) {
+    if (!l) return NULL;
+    ((boat_dense_layer_t*)l)->shadow_fresh = false;             /* the caller may write through it */
+    return l->weight;
+}
 boat_tensor_t* boat_dense_layer_get_bias(const boat_dense_layer_t* l) { return l ? l->bias : NULL; }
 boat_tensor_t* boat_dense_layer_get_grad_weight(const boat_dense_layer_t* l) { return l ? l->grad_weight : NULL; }
 boat_tensor_t* boat_dense_layer_get_grad_bias(const boat_dense_layer_t* l) { return l ? l->grad_bias : NULL; }
 
 int boat_dense_layer_to_device(boat_dense_layer_t* l, boat_device_t device) {
     if (!l) return 1;
+    boat_dev_free(l->shadow);
+    l->shadow = NULL;
+    l->shadow_fresh = false;
     boat_tensor_t** slots[4] = {&l->weight, &l->bias, &l->grad_weight, &l->grad_bias};
     for (int i = 0; i < 4; ++i) {
         boat_tensor_t* t = *slots[i];

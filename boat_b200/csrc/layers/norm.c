@@ -7,6 +7,7 @@
  * (norm.c:397-412); here backward returns the input gradient and keeps d(weight), d(bias) in
  * the layer, and update is the SGD step the other layers use.  RMSNorm is not on the path. */
 #include "../core/stage.h"
+#include "fused.h"
 #include <boat/layers/norm.h>
 #include <boat/layers.h>
 #include <boat/ops.h>
@@ -108,6 +109,10 @@ static boat_tensor_t* grad_like(boat_tensor_t** slot, const boat_tensor_t* param
 }
 
 boat_tensor_t* boat_layernorm_backward(boat_layernorm_t* n, const boat_tensor_t* grad_output) {
+    return boat_layernorm_backward_add(n, grad_output, NULL);
+}
+
+boat_tensor_t* boat_layernorm_backward_add(boat_layernorm_t* n, const boat_tensor_t* grad_output, const boat_tensor_t* residual) {
     if (!n || !grad_output || !n->cache_input || !n->d_mean) return NULL;
     const boat_tensor_t* x = n->cache_input;
     if (grad_output->nelements != x->nelements || !boat_dtype_supported(grad_output->dtype)) return NULL;
@@ -133,8 +138,8 @@ boat_tensor_t* boat_layernorm_backward(boat_layernorm_t* n, const boat_tensor_t*
         d_dbeta = beta_tmp ? (float*)boat_dev_alloc((size_t)H * 4) : (float*)n->grad_bias->data;
     }
     if (dx_in && dy && dx && (!n->weight || (dg && d_dgamma)) && (!n->bias || d_dbeta) &&
-        boat_report("LayerNorm backward", boat_cuda_layernorm_bwd(dy, dx_in, type, rows, H, dg, n->d_mean, n->d_rstd,
-                                                                  dx, d_dgamma, d_dbeta)) == 0) {
+        boat_report("LayerNorm backward", boat_cuda_layernorm_bwd_add(dy, dx_in, type, rows, H, dg, n->d_mean, n->d_rstd,
+                                                                      residual ? residual->data : NULL, dx, d_dgamma, d_dbeta)) == 0) {
         int rc = 0;
         if (gamma_tmp && d_dgamma) rc = boat_cuda_memcpy_d2h(n->grad_weight->data, d_dgamma, (size_t)H * 4);
         if (rc == 0 && beta_tmp && d_dbeta) rc = boat_cuda_memcpy_d2h(n->grad_bias->data, d_dbeta, (size_t)H * 4);
