@@ -74,6 +74,18 @@ inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, s
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
+static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// Dynamic shared memory of a launch of `ctas` CTAs that need `smem` bytes each: so much that no SM takes
+// more than its even share.  CTAs that are placed behind a running predecessor go where it leaves room, two
+// to an SM while others stay empty: 512 x 512 x 4096 on 128 CTAs of gemm_simt took 146 us, spread 90.
+constexpr int kSpreadSmem = 114 * 1024;                   // the most this asks for: no two of them fit an SM's 228 KB
+inline int spread_smem(int smem, int64_t ctas) {
+    const int64_t share = ceil_div(ctas, sm_count());
+    const int least = share <= 3 ? (int)(228 / (share + 1)) * 1024 : 0;
+    return smem > least ? smem : least;
+}
+
 #define BOATCU_RUN(kern, grid, block, smem, ...) \
     BOATCU_CHECK(boatcu::launch_dependent(kern, dim3(grid), dim3(block), smem, 1, __VA_ARGS__))
 
@@ -95,7 +107,6 @@ __device__ __forceinline__ float round_to_tf32(float v) {
 struct f32_tf32 { float v; };
 template <> __device__ __forceinline__ f32_tf32 from_f32<f32_tf32>(float v) { return f32_tf32{round_to_tf32(v)}; }
 
-static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // out[r] = sum_d A[r,d]*B[r,d] over [rows, cols] row-major buffers of storage type `type`.
 int rowdot(const void* A, const void* B, int type, int64_t rows, int64_t cols, float* out);

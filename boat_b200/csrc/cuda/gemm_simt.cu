@@ -2,17 +2,20 @@
 // tensor-core kernels do not take.  Stands in for boat_matmul's triple loop (reference
 // src/ops/linear.c:116-130).
 //
-// 256 threads as 16 x 16, TM x TN outputs each.  Operand tiles go to shared memory exactly as they
-// lie in global memory (cp.async, three stages of 32 along K), whichever way that is: four steps
-// of K are multiplied at a time, an operand that is contiguous along K is read as one 16-byte load
-// per row and four steps, one that is contiguous along M or N as one 16-byte load per step and four
-// rows.  No transposed copy, no bank conflict either way (K-contiguous rows are 36 floats apart, so
-// 8 lanes on 8 rows cover all banks).  Every output is one chain of fused multiply-adds in ascending
-// K, as before.
+// 256 threads.  A warp computes 64 x 32 outputs, 8 x 8 per lane (lanes as 8 x 4): 64 multiply-adds
+// for four 16-byte shared loads, all of them free of bank conflicts, so that the FMA pipe is the bound
+// and not the shared memory.  The eight warps of a CTA lie as WM x WN tiles times WK slices of K: one
+// 64 x 32 output tile with eight slices keeps every warp at that ratio where a problem has too few
+// outputs to give each warp its own.  Operand tiles go to shared memory exactly as they lie in global
+// memory (cp.async, stages of 32 along K), whichever way that is: no transposed copy.
 //
-// Small outputs with a long K (weight gradients) are split along K over the CTAs of a cluster, which
-// add their partial tiles through distributed shared memory in a fixed order: the result does not
-// vary from run to run.  The columns sums of B that a bias gradient wants come from the same pass.
+// The slices' partial tiles are added through shared memory and, where a long K is also split over
+// the CTAs of a cluster, through distributed shared memory, each in a fixed order: the result does not
+// vary from run to run.  The column sums of B that a bias gradient wants come from the same pass.
+//
+// Before, with 4 x 4 outputs per thread: 1000 x 256 x 256 19.6 us, 4096 x 512 x 512 76 us (28 TFLOP/s),
+// 512 x 512 x 4096 (dW) 147 us; now 8.6,
+// 74 and 90 us.
 #include "common.cuh"
 #include <cooperative_groups.h>
 #include <type_traits>
@@ -22,9 +25,9 @@ namespace boatcu {
 namespace {
 
 constexpr int kBK = 32;              // K per stage
-constexpr int kStages = 3;
 constexpr int kMaxGroups = 4;
 constexpr int kMaxSplit = 8;         // portable cluster size
+constexpr int kWarpM = 64, kWarpN = 32, kWarpTile = kWarpM * kWarpN;
 
 struct SimtParams {
     const void* A[kMaxGroups];
@@ -38,65 +41,116 @@ struct SimtParams {
     int add;                         // add to C and colsum instead of overwriting them (FP32 output)
 };
 
-__device__ __forceinline__ void cp_async16(float* dst, const float* src, int bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, int bytes) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-// A tile of `ROWS` rows of `COLS` contiguous elements, from row r0 and column c0 of a [rows, cols]
-// matrix, to shared rows LD floats apart; zeros beyond the matrix.
-template <int ROWS, int COLS, int LD>
-__device__ __forceinline__ void load_tile(float* dst, const float* src, int64_t ld, int64_t r0, int64_t c0, int64_t rows,
-                                          int64_t cols, int vec) {
-    if (vec) {
+// 16 bytes of shared memory of CTA `rank` of the cluster, at this CTA's shared address `at`
+__device__ __forceinline__ float4 ld_cluster4(uint32_t at, int rank) {
+    uint32_t there;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(there) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// The tiles of one operand along K, in shared rows LD floats apart; zeros beyond the matrix.  K_ROWS: the
+// operand is stored [K, X] and a tile is kBK rows of XT columns, else it is [X, K] and a tile is XT rows
+// of kBK columns.  What does not change along K is worked out once: with 16-byte copies a thread keeps
+// one column of every tile, so that a copy inside the matrix costs little more than itself.
+template <typename T, int XT, bool K_ROWS, int LD>
+struct TileLoader {
+    static constexpr int ROWS = K_ROWS ? kBK : XT, COLS = K_ROWS ? XT : kBK;
+    static constexpr int PER_ROW = COLS / 4, ROW_STEP = 256 / PER_ROW;
+    static_assert(ROWS % ROW_STEP == 0 && 256 % PER_ROW == 0, "whole passes");
+    const T* p;                      // this thread's first element of tile 0
+    uint32_t at;                     // where it goes, in bytes from the start of the shared tile
+    int fixed;                       // K_ROWS: bytes of the thread's column; else rows from its first one to the matrix's end
+    bool whole;                      // the tile is inside the matrix across K
+
+    __device__ __forceinline__ TileLoader(const T* base, int64_t ld, int64_t x0, int64_t X) {
+        const int r = threadIdx.x / PER_ROW, c = (threadIdx.x % PER_ROW) * 4;
+        p = base + (K_ROWS ? r * ld + x0 + c : (x0 + r) * ld + c);
+        const int64_t left = X - x0 - (K_ROWS ? c : r);
+        at = (r * LD + c) * 4;
+        whole = X - x0 >= XT;
+        fixed = K_ROWS ? (int)(left >= 4 ? 16 : (left > 0 ? left * 4 : 0)) : (int)(left > XT ? XT : left);
+    }
+    // dst: the tile in shared memory, dst_at: the same as an address of the shared window
+    __device__ __forceinline__ void fetch(float* dst, uint32_t dst_at, int step, const T* base, int64_t ld, int64_t x0, int64_t X, int64_t K, int vec) const {
+        const int64_t k0 = (int64_t)step * kBK;
+        if constexpr (sizeof(T) == 4) {
+            if (vec) {
+                const int r = threadIdx.x / PER_ROW, c = (threadIdx.x % PER_ROW) * 4;
+                const T* q = p + (K_ROWS ? k0 * ld : k0);
+                const uint32_t d = dst_at + at;
+                if (whole && k0 + kBK <= K) {
 #pragma unroll
-        for (int e = threadIdx.x; e < ROWS * COLS / 4; e += 256) {
-            const int r = e / (COLS / 4), c = (e % (COLS / 4)) * 4;
-            const int64_t gr = r0 + r, gc = c0 + c, left = gr < rows ? cols - gc : 0;
-            const int bytes = left >= 4 ? 16 : (left > 0 ? (int)left * 4 : 0);
-            cp_async16(dst + r * LD + c, bytes ? src + gr * ld + gc : src, bytes);
+                    for (int i = 0; i < ROWS / ROW_STEP; ++i, q += ROW_STEP * ld) cp_async16(d + i * ROW_STEP * LD * 4, q);
+                    return;
+                }
+                const int64_t rest = K - k0 - (K_ROWS ? r : c);
+                const int left = (int)(rest < kBK ? rest : kBK);
+                const int tail = left >= 4 ? 16 : (left > 0 ? left * 4 : 0);
+#pragma unroll 1
+                for (int i = 0; i < ROWS / ROW_STEP; ++i, q += ROW_STEP * ld) {
+                    const int bytes = i * ROW_STEP < (K_ROWS ? left : fixed) ? (K_ROWS ? fixed : tail) : 0;
+                    cp_async16(d + i * ROW_STEP * LD * 4, bytes ? q : base, bytes);
+                }
+                return;
+            }
         }
-    } else {
-#pragma unroll 4
+        const int64_t r0 = K_ROWS ? k0 : x0, c0 = K_ROWS ? x0 : k0, rows = K_ROWS ? K : X, cols = K_ROWS ? X : K;
+#pragma unroll 1
         for (int e = threadIdx.x; e < ROWS * COLS; e += 256) {
-            const int r = e / COLS, c = e % COLS;
-            const int64_t gr = r0 + r, gc = c0 + c;
+            const int er = e / COLS, ec = e % COLS;
+            const int64_t gr = r0 + er, gc = c0 + ec;
             const bool in = gr < rows && gc < cols;
-            cp_async4(dst + r * LD + c, in ? src + gr * ld + gc : src, in ? 4 : 0);
+            if constexpr (sizeof(T) == 4) cp_async4(dst + er * LD + ec, in ? base + gr * ld + gc : base, in ? 4 : 0);
+            else dst[er * LD + ec] = in ? to_f32(base[gr * ld + gc]) : 0.f;
         }
     }
-}
-template <int ROWS, int COLS, int LD>
-__device__ __forceinline__ void load_tile(float* dst, const __nv_bfloat16* src, int64_t ld, int64_t r0, int64_t c0,
-                                          int64_t rows, int64_t cols, int vec) {
-    (void)vec;
-#pragma unroll 4
-    for (int e = threadIdx.x; e < ROWS * COLS; e += 256) {
-        const int r = e / COLS, c = e % COLS;
-        const int64_t gr = r0 + r, gc = c0 + c;
-        dst[r * LD + c] = gr < rows && gc < cols ? to_f32(src[gr * ld + gc]) : 0.f;
-    }
-}
+};
 
 // A_M: A is stored [K, M] (contiguous along M), else [M, K].  B_K: B is stored [N, K], else [K, N].
-template <bool A_M, bool B_K, int TM, int TN>
+// WM x WN warp tiles, 8 / (WM * WN) slices of K.
+template <bool A_M, bool B_K, int WM, int WN>
 struct SimtTile {
-    static constexpr int BM = 16 * TM, BN = 16 * TN;
+    static constexpr int BM = kWarpM * WM, BN = kWarpN * WN, TILES = WM * WN, WK = 8 / TILES;
     static constexpr int LDA = A_M ? BM + 4 : kBK + 4, LDB = B_K ? kBK + 4 : BN + 4;
     static constexpr int A_FLOATS = A_M ? kBK * LDA : BM * LDA, B_FLOATS = B_K ? BN * LDB : kBK * LDB;
     static constexpr int STAGE = A_FLOATS + B_FLOATS;
-    static constexpr int SMEM = kStages * STAGE * 4;
-    static_assert(BM * BN + BN <= kStages * STAGE, "the partial tile must fit the stages");
+    static constexpr int STAGES = WK > 1 ? 4 : 3;
+    static constexpr int PARTS = 8 * kWarpTile, SUMS = 8 * kWarpN;      // the partial tiles take the stages' place
+    static constexpr int SMEM = (STAGES * STAGE > PARTS + SUMS ? STAGES * STAGE : PARTS + SUMS) * 4;
+    static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
 };
 
-template <typename TI, typename TO, bool A_M, bool B_K, int TM, int TN>
-__global__ void __launch_bounds__(256)
+// `N` neighbouring floats of shared memory
+template <int N> __device__ __forceinline__ void load_shared(float (&v)[N], const float* p) {
+    if constexpr (N == 4) {
+        const float4 t = *reinterpret_cast<const float4*>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+        const float2 t = *reinterpret_cast<const float2*>(p);
+        v[0] = t.x; v[1] = t.y;
+    }
+}
+
+template <typename TI, typename TO, bool A_M, bool B_K, int WM, int WN>
+__global__ void __launch_bounds__(256, 2)
 gemm_simt_kernel(const __grid_constant__ SimtParams p) {
-    using S = SimtTile<A_M, B_K, TM, TN>;
+    using S = SimtTile<A_M, B_K, WM, WN>;
     extern __shared__ __align__(16) float smem[];
-    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lm = lane >> 2, ln = lane & 3;
+    const int wk = warp / S::TILES, wm = warp % S::TILES / WN, wn = warp % WN;
     const int g = blockIdx.z, split = p.split;
     const int ks = blockIdx.x % split, tile = blockIdx.x / split;
     const int64_t m0 = (int64_t)(tile / p.n_tiles) * S::BM, n0 = (int64_t)(tile % p.n_tiles) * S::BN;
@@ -104,200 +158,209 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     const TI* B = (const TI*)p.B[g];
     const int steps = (int)((p.K + kBK - 1) / kBK);
     const int s0 = (int)((int64_t)steps * ks / split), s1 = (int)((int64_t)steps * (ks + 1) / split);
-    const bool sums = p.colsum[g] != nullptr && m0 == 0;
+    constexpr bool kSums = A_M && !B_K;                   // a weight gradient
+    const bool sums = kSums && p.colsum[g] != nullptr && m0 == 0;
 
-    auto fetch = [&](int s) {
-        if (s < s1) {
-            float* a = smem + (s % kStages) * S::STAGE;
-            const int64_t k0 = (int64_t)s * kBK;
-            if (A_M) load_tile<kBK, S::BM, S::LDA>(a, A, p.lda, k0, m0, p.K, p.M, p.vec_a);
-            else     load_tile<S::BM, kBK, S::LDA>(a, A, p.lda, m0, k0, p.M, p.K, p.vec_a);
-            if (B_K) load_tile<S::BN, kBK, S::LDB>(a + S::A_FLOATS, B, p.ldb, n0, k0, p.N, p.K, p.vec_b);
-            else     load_tile<kBK, S::BN, S::LDB>(a + S::A_FLOATS, B, p.ldb, k0, n0, p.K, p.N, p.vec_b);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
+    const TileLoader<TI, S::BM, A_M, S::LDA> load_a(A, p.lda, m0, p.M);
+    const TileLoader<TI, S::BN, !B_K, S::LDB> load_b(B, p.ldb, n0, p.N);
 
-    float acc[TM][TN], bsum[TN];
+    const uint32_t smem_at = (uint32_t)__cvta_generic_to_shared(smem);
+    float acc[8][8], bsum = 0.f;                          // bsum: column `lane` of the warp tile
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-        bsum[j] = 0.f;
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-        for (int i = 0; i < TM; ++i) acc[i][j] = 0.f;
-    }
-    // Rows of this thread: ty*TM + i.  Columns: with B contiguous along N groups of min(TN,4) neighbours,
-    // with B contiguous along K tx + 16*j (neighbouring lanes on neighbouring shared rows).
-    constexpr int VN = TN < 4 ? TN : 4, VM = TM < 4 ? TM : 4;
-    auto col = [&](int j) { return B_K ? tx + 16 * j : (j / VN) * 16 * VN + tx * VN + j % VN; };
-    auto row = [&](int i) { return (i / VM) * 16 * VM + ty * VM + i % VM; };
+        for (int i = 0; i < 8; ++i) acc[i][j] = 0.f;
+    // Rows and columns of a lane inside the warp tile: groups of four neighbours where the operand is
+    // contiguous that way, strided by the lanes where it is contiguous along K, so that the lanes of a load
+    // touch all banks once.
+    auto row = [&](int i) { return A_M ? (i / 4) * 32 + lm * 4 + i % 4 : lm + 8 * i; };
+    auto col = [&](int j) { return B_K ? ln + 4 * j : (j / 4) * 16 + ln * 4 + j % 4; };
 
     griddep_sync();
-    fetch(s0);
-    fetch(s0 + 1);
-    for (int s = s0; s < s1; ++s) {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();                                  // stage s has landed, stage s-1 is no longer read
-        fetch(s + 2);
-        const float* a_s = smem + (s % kStages) * S::STAGE;
-        const float* b_s = a_s + S::A_FLOATS;
-#pragma unroll
-        for (int k = 0; k < kBK; k += 4) {
-            float a[TM][4], b[4][TN];
+    // the first rounds only fetch, so that the code of a fetch is there once
+    for (int s = s0 - (S::STAGES - 1); s < s1; ++s) {
+        if (s >= s0) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(S::STAGES - 2) : "memory");
+            __syncthreads();                              // stage s has landed, stage s-1 is no longer read
+        }
+        const int ahead = s + S::STAGES - 1;
+        if (ahead < s1) {
+            const int to = ahead % S::STAGES * S::STAGE;
+            load_a.fetch(smem + to, smem_at + to * 4, ahead, A, p.lda, m0, p.M, p.K, p.vec_a);
+            load_b.fetch(smem + to + S::A_FLOATS, smem_at + (to + S::A_FLOATS) * 4, ahead, B, p.ldb, n0, p.N, p.K, p.vec_b);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (s < s0) continue;
+        constexpr int KW = kBK / S::WK;                   // this warp's share of the stage
+        const float* a_s = smem + s % S::STAGES * S::STAGE + (A_M ? (wk * KW) * S::LDA + wm * kWarpM : wm * kWarpM * S::LDA + wk * KW);
+        const float* b_s = smem + s % S::STAGES * S::STAGE + S::A_FLOATS + (B_K ? wn * kWarpN * S::LDB + wk * KW : (wk * KW) * S::LDB + wn * kWarpN);
+#pragma unroll(KW < 8 ? KW / 2 : 4)
+        for (int k = 0; k < KW; k += 2) {
+            float a[8][2], b[8][2];
             if (A_M) {
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
+                for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
-                    for (int i = 0; i < TM; i += VM) {
-                        const float* q = a_s + (k + kk) * S::LDA + row(i);
-                        if constexpr (VM == 4) {
-                            const float4 v = *reinterpret_cast<const float4*>(q);
-                            a[i][kk] = v.x; a[i + 1][kk] = v.y; a[i + 2][kk] = v.z; a[i + 3][kk] = v.w;
-                        } else {
+                    for (int i = 0; i < 8; i += 4) {
+                        float t[4];
+                        load_shared<4>(t, a_s + (k + kk) * S::LDA + row(i));
 #pragma unroll
-                            for (int u = 0; u < VM; ++u) a[i + u][kk] = q[u];
-                        }
+                        for (int u = 0; u < 4; ++u) a[i + u][kk] = t[u];
                     }
             } else {
 #pragma unroll
-                for (int i = 0; i < TM; ++i) {
-                    const float4 v = *reinterpret_cast<const float4*>(a_s + row(i) * S::LDA + k);
-                    a[i][0] = v.x; a[i][1] = v.y; a[i][2] = v.z; a[i][3] = v.w;
-                }
+                for (int i = 0; i < 8; ++i) load_shared<2>(a[i], a_s + row(i) * S::LDA + k);
             }
             if (B_K) {
 #pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    const float4 v = *reinterpret_cast<const float4*>(b_s + col(j) * S::LDB + k);
-                    b[0][j] = v.x; b[1][j] = v.y; b[2][j] = v.z; b[3][j] = v.w;
-                }
+                for (int j = 0; j < 8; ++j) load_shared<2>(b[j], b_s + col(j) * S::LDB + k);
             } else {
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
+                for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
-                    for (int j = 0; j < TN; j += VN) {
-                        const float* q = b_s + (k + kk) * S::LDB + col(j);
-                        if constexpr (VN == 4) {
-                            const float4 v = *reinterpret_cast<const float4*>(q);
-                            b[kk][j] = v.x; b[kk][j + 1] = v.y; b[kk][j + 2] = v.z; b[kk][j + 3] = v.w;
-                        } else {
+                    for (int j = 0; j < 8; j += 4) {
+                        float t[4];
+                        load_shared<4>(t, b_s + (k + kk) * S::LDB + col(j));
 #pragma unroll
-                            for (int u = 0; u < VN; ++u) b[kk][j + u] = q[u];
-                        }
+                        for (int u = 0; u < 4; ++u) b[j + u][kk] = t[u];
                     }
             }
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
+            for (int kk = 0; kk < 2; ++kk)
 #pragma unroll
-                for (int i = 0; i < TM; ++i)
+                for (int i = 0; i < 8; ++i)
 #pragma unroll
-                    for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i][kk], b[kk][j], acc[i][j]);
-            if (sums) {
+                    for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i][kk], b[j][kk], acc[i][j]);
+        }
+        if (sums && wm == 0) {
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) bsum[j] += b[kk][j];
-            }
+            for (int k = 0; k < KW; ++k) bsum += b_s[k * S::LDB + lane];
         }
     }
 
+    // Partial tiles to shared memory: one block of 64 rows of 32 floats per warp.  The 16-byte units of a
+    // row are permuted by the row's lane, so that neither the lanes of a store nor those of a load meet.
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    auto unit = [&](int r, int c4) {
+        const int l = A_M ? (r >> 2) & 7 : r & 7;
+        return r * kWarpN + ((c4 ^ ((l & 1) << 2 | (l & 2) | l >> 2)) << 2);
+    };
+    float* part = smem + warp * kWarpTile;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = row(i);
+        if constexpr (B_K) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) part[unit(r, j) + ln] = acc[i][j];
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; j += 4)
+                *reinterpret_cast<float4*>(part + unit(r, col(j) >> 2)) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+        }
+    }
+    float* sum_s = smem + S::PARTS;
+    if (sums && wm == 0) sum_s[(wk * WN + wn) * kWarpN + lane] = bsum;
+    __syncthreads();
+
     TO* C = (TO*)p.C[g];
     const float* bias = p.bias[g];
-    auto put = [&](TO* dst, float v) {
-        if constexpr (std::is_same<TO, float>::value) {
-            if (p.add) v += *dst;
-        }
-        *dst = from_f32<TO>(v);
-    };
-    if (split == 1) {
-#pragma unroll
-        for (int i = 0; i < TM; ++i) {
-            const int64_t gm = m0 + row(i);
-            if (gm >= p.M) continue;
-            if constexpr (!B_K && VN == 4 && sizeof(TO) == 4) {
-                if (p.vec_c) {
-#pragma unroll
-                    for (int j = 0; j < TN; j += 4) {
-                        const int64_t gn = n0 + col(j);
-                        if (gn >= p.N) continue;              // N is a multiple of 4 here
-                        float4 v = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
-                        if (bias) {
-                            const float4 t = *reinterpret_cast<const float4*>(bias + gn);
-                            v = make_float4(v.x + t.x, v.y + t.y, v.z + t.z, v.w + t.w);
-                        }
-                        if constexpr (!std::is_same<TO, float>::value)
-                            v = make_float4(round_to_tf32(v.x), round_to_tf32(v.y), round_to_tf32(v.z), round_to_tf32(v.w));
-                        float4* dst = reinterpret_cast<float4*>(C + gm * p.ldc + gn);
-                        if (p.add) {
-                            const float4 t = *dst;
-                            v = make_float4(t.x + v.x, t.y + v.y, t.z + v.z, t.w + v.w);
-                        }
-                        *dst = v;
-                    }
-                    continue;
+    auto put = [&](int e, float4 v) {                      // unit e of the CTA's tile, numbered as the sums below do
+        const int t = e / (kWarpTile / 4), r = e / 8 % kWarpM, c4 = e % 8;
+        const int64_t gm = m0 + (t / WN) * kWarpM + r, gn = n0 + (t % WN) * kWarpN + c4 * 4;
+        if (gm >= p.M || gn >= p.N) return;
+        TO* dst = C + gm * p.ldc + gn;
+        if constexpr (sizeof(TO) == 4) {
+            if (p.vec_c) {                                // N is a multiple of 4 here
+                if (bias) v = add4(v, *reinterpret_cast<const float4*>(bias + gn));
+                if constexpr (std::is_same<TO, float>::value) {
+                    if (p.add) v = add4(*reinterpret_cast<const float4*>(dst), v);
+                } else {
+                    v = make_float4(round_to_tf32(v.x), round_to_tf32(v.y), round_to_tf32(v.z), round_to_tf32(v.w));
                 }
-            }
-#pragma unroll
-            for (int j = 0; j < TN; ++j) {
-                const int64_t gn = n0 + col(j);
-                if (gn < p.N) put(C + gm * p.ldc + gn, acc[i][j] + (bias ? bias[gn] : 0.f));
+                *reinterpret_cast<float4*>(dst) = v;
+                return;
             }
         }
-        if (sums && ty == 0) {
+        const float out[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int j = 0; j < TN; ++j)
-                if (n0 + col(j) < p.N) p.colsum[g][n0 + col(j)] = bsum[j] + (p.add ? p.colsum[g][n0 + col(j)] : 0.f);
+        for (int u = 0; u < 4; ++u) {
+            if (gn + u >= p.N) break;
+            float w = out[u] + (bias ? bias[gn + u] : 0.f);
+            if constexpr (std::is_same<TO, float>::value) {
+                if (p.add) w += dst[u];
+            }
+            dst[u] = from_f32<TO>(w);
         }
+    };
+    constexpr int kUnits = S::BM * S::BN / 4;
+    auto sliced = [&](int e) {                             // unit e added over the slices of this CTA, where it lies in smem
+        const int t = e / (kWarpTile / 4), at = unit(e / 8 % kWarpM, e % 8);
+        float4 v = *reinterpret_cast<const float4*>(smem + t * kWarpTile + at);
+#pragma unroll
+        for (int w = 1; w < S::WK; ++w) v = add4(v, *reinterpret_cast<const float4*>(smem + (w * S::TILES + t) * kWarpTile + at));
+        return v;
+    };
+    if (sums && tid < S::BN) {
+        float v = sum_s[tid];
+#pragma unroll
+        for (int w = 1; w < S::WK; ++w) v += sum_s[w * S::BN + tid];
+        if (split > 1) sum_s[tid] = v;
+        else if (n0 + tid < p.N) p.colsum[g][n0 + tid] = v + (p.add ? p.colsum[g][n0 + tid] : 0.f);
+    }
+    if (split == 1) {
+#pragma unroll 2
+        for (int e = tid; e < kUnits; e += 256) put(e, sliced(e));
         return;
     }
-    // Partial tiles to shared memory, then every CTA of the cluster adds its share of the tile over
-    // all of them, lowest K first.
+    // every CTA of the cluster adds its share of the tile over all of them, lowest K first
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) smem[row(i) * S::BN + col(j)] = acc[i][j];
-    if (sums && ty == 0) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j) smem[S::BM * S::BN + col(j)] = bsum[j];
+    auto place = [&](int e) { return e / (kWarpTile / 4) * kWarpTile + unit(e / 8 % kWarpM, e % 8); };
+    if (S::WK > 1) {
+#pragma unroll 2
+        for (int e = tid; e < kUnits; e += 256) *reinterpret_cast<float4*>(smem + place(e)) = sliced(e);
     }
     cluster.sync();
-    const float* part[kMaxSplit];
+    auto over_cluster = [&](int at) {
+        float4 t[kMaxSplit];
 #pragma unroll
-    for (int r = 0; r < kMaxSplit; ++r) part[r] = cluster.map_shared_rank(smem, r < split ? r : 0);
-    const int total = S::BM * S::BN + (sums ? S::BN : 0);
-    for (int e = ks * 256 + tid; e < total; e += split * 256) {
-        float v = part[0][e];
+        for (int r = 0; r < kMaxSplit; ++r)
+            if (r < split) t[r] = ld_cluster4(smem_at + at * 4, r);
+        float4 v = t[0];
 #pragma unroll
         for (int r = 1; r < kMaxSplit; ++r)
-            if (r < split) v += part[r][e];
-        const int64_t gn = n0 + e % S::BN;
-        if (gn >= p.N) continue;
-        if (e >= S::BM * S::BN) {
-            p.colsum[g][gn] = v + (p.add ? p.colsum[g][gn] : 0.f);
-        } else {
-            const int64_t gm = m0 + e / S::BN;
-            if (gm < p.M) put(C + gm * p.ldc + gn, v + (bias ? bias[gn] : 0.f));
+            if (r < split) v = add4(v, t[r]);
+        return v;
+    };
+    for (int e = ks * 256 + tid; e < kUnits; e += split * 256) put(e, over_cluster(place(e)));
+    if (sums && ks == 0 && tid < S::BN / 4) {
+        const float4 v = over_cluster(S::PARTS + tid * 4);
+        const float out[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t gn = n0 + tid * 4 + u;
+            if (gn < p.N) p.colsum[g][gn] = out[u] + (p.add ? p.colsum[g][gn] : 0.f);
         }
     }
     cluster.sync();                                       // nobody leaves while its partial tile is being read
 }
 
-template <typename TI, typename TO, bool A_M, bool B_K, int TM, int TN>
+template <typename TI, typename TO, bool A_M, bool B_K, int WM, int WN>
 int launch_tile(SimtParams& p, int groups, int split) {
-    using S = SimtTile<A_M, B_K, TM, TN>;
-    auto kern = gemm_simt_kernel<TI, TO, A_M, B_K, TM, TN>;
+    using S = SimtTile<A_M, B_K, WM, WN>;
+    auto kern = gemm_simt_kernel<TI, TO, A_M, B_K, WM, WN>;
     static bool configured = false;      // per process = per device: the library binds to one device
     if (!configured) {
-        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
+        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM > kSpreadSmem ? S::SMEM : kSpreadSmem));
         configured = true;
     }
     const int64_t tiles = ceil_div(p.M, S::BM) * ceil_div(p.N, S::BN);
     if (tiles * split > 0x7fffffffLL) return set_error(7, "gemm_simt: %lld x %lld outputs are too many for one launch", (long long)p.M, (long long)p.N);
     p.n_tiles = (int)ceil_div(p.N, S::BN);
     p.split = split;
-    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), S::SMEM, (unsigned)split, p));
+    const int smem = spread_smem(S::SMEM, tiles * split * groups);
+    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), smem, (unsigned)split, p));
     BOATCU_LAUNCH_OK("gemm_simt");
     return 0;
 }
@@ -306,20 +369,18 @@ template <typename TI, typename TO, bool A_M, bool B_K>
 int pick_tile(SimtParams& p, int groups) {
     const int64_t sms = sm_count();
     auto tiles = [&](int bm, int bn) { return ceil_div(p.M, bm) * ceil_div(p.N, bn); };
-    // 128 x 128 tiles (64 outputs per thread, bound by the FMA pipe) once they fill the GPU;
-    // 64 x 64 (bound by shared memory at about half that rate) with K split over a cluster while
-    // SMs would stay idle, at least 64 of K per CTA; 32 x 32 for outputs so small that even so
-    // most SMs would have nothing.  The split - the order of the sum - goes by the size of one problem
-    // alone, so that a group gives the bits of single calls.
-    const int64_t t64 = tiles(64, 64);
-    int64_t split = sms / t64;
+    // The largest tile that still gives every SM one: larger ones fetch less per product, smaller ones
+    // leave no SM idle.  Where even 64 x 32 does not fill the GPU, K is split over a cluster too, at
+    // least 64 of it per CTA.  The order of the sum goes by the size of one problem alone, so that a
+    // group gives the bits of single calls.
+    if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value)
+        if (tiles(128, 128) >= sms) return launch_tile<TI, TO, A_M, B_K, 2, 4>(p, groups, 1);
+    if (tiles(64, 64) >= sms) return launch_tile<TI, TO, A_M, B_K, 1, 2>(p, groups, 1);
+    int64_t split = sms / tiles(64, 32);
     if (split > p.K / 64) split = p.K / 64;
     if (split > kMaxSplit) split = kMaxSplit;
     if (split < 1) split = 1;
-    if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value)
-        if (split == 1 && tiles(128, 128) * groups >= sms) return launch_tile<TI, TO, A_M, B_K, 8, 8>(p, groups, 1);
-    if (split == 1 && t64 * groups * 4 <= sms) return launch_tile<TI, TO, A_M, B_K, 2, 2>(p, groups, 1);
-    return launch_tile<TI, TO, A_M, B_K, 4, 4>(p, groups, (int)split);
+    return launch_tile<TI, TO, A_M, B_K, 1, 1>(p, groups, (int)split);
 }
 
 template <typename TI, typename TO>
