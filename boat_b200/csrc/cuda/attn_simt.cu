@@ -6,8 +6,8 @@
 // outside the tensor-core kernels.  The S x S matrices are never written to memory:
 // probabilities are rebuilt from the saved log-sum-exp.
 //
-// A CTA of 256 threads (16 x 16) owns 64 rows and walks the other side in tiles of 64 rows.  A score
-// tile is 4 x 4 per thread, contracted along the head dimension with 16-byte shared loads of four
+// A CTA of 16 threads per 4 rows owns 64 rows - or 32, with half the threads, where 64 would leave SMs
+// without a CTA - and walks the other side in tiles of 64 rows.  A score tile is 4 x 4 per thread, contracted along the head dimension with 16-byte shared loads of four
 // elements; rows are HS+4 floats apart, so 8 lanes on 8 rows touch all banks once.  The tile's rows
 // stay with the 16 lanes that made them - soft-max statistics are shuffles, and the products with the
 // probabilities (P.V, dS.K, P^T.dO, dS^T.Q) read rows which the same half warp wrote: a walk has one CTA
@@ -25,34 +25,36 @@ namespace boatcu {
 
 namespace {
 
-constexpr int kRows = 64;             // rows owned and rows per walked tile
-constexpr int kThreads = 256;
+constexpr int kRows = 64;             // rows per walked tile
 constexpr int kLdP = kRows + 4;       // shared row pitch of a probability tile
 
-template <int HS>
+// OWN: rows a CTA owns (64 or 32)
+template <int HS, int OWN>
 struct Tiles {
     static constexpr int LD = HS + 4;
+    static constexpr int THREADS = OWN * 4;
+    static constexpr int OWN_FLOATS = OWN * LD;
     static constexpr int FLOATS = kRows * LD;
     static constexpr int CPT = HS / 16;                  // output columns per thread
     static constexpr int BUFS = HS <= 64 ? 2 : 1;        // walked tiles in flight
-    static constexpr int FWD_SMEM = (FLOATS * (1 + 2 * BUFS) + kRows * kLdP) * 4;
-    static constexpr int BWD_SMEM = (FLOATS * (2 + 2 * BUFS) + 2 * kRows * kLdP + 2 * 2 * kRows) * 4;
+    static constexpr int FWD_SMEM = (OWN_FLOATS + FLOATS * 2 * BUFS + OWN * kLdP) * 4;
+    static constexpr int BWD_SMEM = (OWN_FLOATS * 2 + FLOATS * 2 * BUFS + 2 * OWN * kLdP + 2 * 2 * kRows) * 4;
     static_assert(BWD_SMEM <= 227 * 1024, "shared memory budget");
 };
 
-// Rows r0..r0+63 of a [S, hs] matrix to shared rows LD apart; zeros beyond S and from hs to HS.
-template <int HS>
+// Rows r0..r0+ROWS-1 of a [S, hs] matrix to shared rows LD apart; zeros beyond S and from hs to HS.
+template <int HS, int ROWS, int THREADS>
 __device__ __forceinline__ void load_rows(float* dst, const float* src, int r0, int S, int hs, bool vec) {
     if (vec) {
 #pragma unroll
-        for (int e = threadIdx.x; e < kRows * HS / 4; e += kThreads) {
+        for (int e = threadIdx.x; e < ROWS * HS / 4; e += THREADS) {
             const int r = e / (HS / 4), c = (e % (HS / 4)) * 4;
             const bool in = r0 + r < S && c < hs;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * (HS + 4) + c)),
                          "l"(in ? src + (int64_t)(r0 + r) * hs + c : src), "r"(in ? 16 : 0) : "memory");
         }
     } else {
-        for (int e = threadIdx.x; e < kRows * HS; e += kThreads) {
+        for (int e = threadIdx.x; e < ROWS * HS; e += THREADS) {
             const int r = e / HS, c = e % HS;
             const bool in = r0 + r < S && c < hs;
             asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst + r * (HS + 4) + c)),
@@ -60,11 +62,11 @@ __device__ __forceinline__ void load_rows(float* dst, const float* src, int r0, 
         }
     }
 }
-template <int HS>
+template <int HS, int ROWS, int THREADS>
 __device__ __forceinline__ void load_rows(float* dst, const __nv_bfloat16* src, int r0, int S, int hs, bool vec) {
     if (vec) {
 #pragma unroll 4
-        for (int e = threadIdx.x; e < kRows * HS / 4; e += kThreads) {
+        for (int e = threadIdx.x; e < ROWS * HS / 4; e += THREADS) {
             const int r = e / (HS / 4), c = (e % (HS / 4)) * 4;
             uint2 v = make_uint2(0u, 0u);
             if (r0 + r < S && c < hs) v = *reinterpret_cast<const uint2*>(src + (int64_t)(r0 + r) * hs + c);
@@ -73,7 +75,7 @@ __device__ __forceinline__ void load_rows(float* dst, const __nv_bfloat16* src, 
             *reinterpret_cast<float4*>(dst + r * (HS + 4) + c) = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
     } else {
-        for (int e = threadIdx.x; e < kRows * HS; e += kThreads) {
+        for (int e = threadIdx.x; e < ROWS * HS; e += THREADS) {
             const int r = e / HS, c = e % HS;
             dst[r * (HS + 4) + c] = r0 + r < S && c < hs ? to_f32(src[(int64_t)(r0 + r) * hs + c]) : 0.f;
         }
@@ -177,28 +179,28 @@ __device__ __forceinline__ float row_sum(float v) {
 }
 
 // ---- forward -----------------------------------------------------------------------------------
-template <int HS, typename T>
-__global__ void __launch_bounds__(kThreads)
+template <int HS, int OWN, typename T>
+__global__ void __launch_bounds__(OWN * 4)
 attn_fwd_simt_kernel(int units, int S, int hs, int causal, float scale, int vec, const T* __restrict__ Q,
                      const T* __restrict__ K, const T* __restrict__ V, T* __restrict__ O, float* __restrict__ lse) {
-    using C = Tiles<HS>;
+    using C = Tiles<HS, OWN>;
     extern __shared__ __align__(16) float smem[];
     float* q_s = smem;
-    float* kv_s = q_s + C::FLOATS;                        // [BUFS][K, V]
+    float* kv_s = q_s + C::OWN_FLOATS;                        // [BUFS][K, V]
     float* p_s = kv_s + 2 * C::BUFS * C::FLOATS;
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-    const int n_tiles = (S + kRows - 1) / kRows;
-    const int unit = blockIdx.x % units, qt = n_tiles - 1 - blockIdx.x / units;      // long rows first when causal
+    const int n_own = (S + OWN - 1) / OWN;
+    const int unit = blockIdx.x % units, qt = n_own - 1 - blockIdx.x / units;        // long rows first when causal
     const int64_t base = (int64_t)unit * S * hs;
-    const int q0 = qt * kRows, n_kv = causal ? qt + 1 : n_tiles;
+    const int q0 = qt * OWN, n_kv = ((causal ? min(q0 + OWN, S) : S) + kRows - 1) / kRows;
     auto fetch = [&](int j) {
         float* b = kv_s + (j % C::BUFS) * 2 * C::FLOATS;
-        load_rows<HS>(b, K + base, j * kRows, S, hs, vec);
-        load_rows<HS>(b + C::FLOATS, V + base, j * kRows, S, hs, vec);
+        load_rows<HS, kRows, C::THREADS>(b, K + base, j * kRows, S, hs, vec);
+        load_rows<HS, kRows, C::THREADS>(b + C::FLOATS, V + base, j * kRows, S, hs, vec);
         commit();
     };
     griddep_sync();
-    load_rows<HS>(q_s, Q + base, q0, S, hs, vec);
+    load_rows<HS, OWN, C::THREADS>(q_s, Q + base, q0, S, hs, vec);
     fetch(0);
     float o[4][C::CPT], m[4], l[4];
 #pragma unroll
@@ -268,20 +270,21 @@ struct BwdArgs {
 };
 
 // KEYS: the CTA owns key rows (dK, dV), otherwise query rows (dQ).
-template <int HS, typename T, bool KEYS>
+template <int HS, int OWN, typename T, bool KEYS>
 __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile, float* smem) {
-    using C = Tiles<HS>;
+    using C = Tiles<HS, OWN>;
     float* own0 = smem;
-    float* own1 = own0 + C::FLOATS;
-    float* walk = own1 + C::FLOATS;                       // [BUFS][walk0, walk1]
+    float* own1 = own0 + C::OWN_FLOATS;
+    float* walk = own1 + C::OWN_FLOATS;                       // [BUFS][walk0, walk1]
     float* ds_s = walk + 2 * C::BUFS * C::FLOATS;
-    float* p_s = ds_s + kRows * kLdP;
-    float* stat = p_s + kRows * kLdP;                     // [2][lse[64], delta[64]] of the query rows
+    float* p_s = ds_s + OWN * kLdP;
+    float* stat = p_s + OWN * kLdP;                     // [2][lse[64], delta[64]] of the query rows
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
     const int S = a.S, hs = a.hs, n_tiles = (S + kRows - 1) / kRows;
     const int64_t base = (int64_t)unit * S * hs, sbase = (int64_t)unit * S;
-    const int r0 = tile * kRows;
-    const int first = KEYS && a.causal ? tile : 0, end = !KEYS && a.causal ? tile + 1 : n_tiles;
+    const int r0 = tile * OWN;
+    const int first = KEYS && a.causal ? r0 / kRows : 0;
+    const int end = !KEYS && a.causal ? min((r0 + OWN + kRows - 1) / kRows, n_tiles) : n_tiles;
     const T* w0 = (KEYS ? a.Q : a.K) + base;
     const T* w1 = (KEYS ? a.dO : a.V) + base;
     auto load_stats = [&](int q0, int buf) {
@@ -293,14 +296,14 @@ __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile
     };
     auto fetch = [&](int j) {
         float* b = walk + (j % C::BUFS) * 2 * C::FLOATS;
-        load_rows<HS>(b, w0, j * kRows, S, hs, a.vec);
-        load_rows<HS>(b + C::FLOATS, w1, j * kRows, S, hs, a.vec);
+        load_rows<HS, kRows, C::THREADS>(b, w0, j * kRows, S, hs, a.vec);
+        load_rows<HS, kRows, C::THREADS>(b + C::FLOATS, w1, j * kRows, S, hs, a.vec);
         commit();
         if (KEYS) load_stats(j * kRows, j & 1);
     };
     griddep_sync();
-    load_rows<HS>(own0, (KEYS ? a.K : a.Q) + base, r0, S, hs, a.vec);
-    load_rows<HS>(own1, (KEYS ? a.V : a.dO) + base, r0, S, hs, a.vec);
+    load_rows<HS, OWN, C::THREADS>(own0, (KEYS ? a.K : a.Q) + base, r0, S, hs, a.vec);
+    load_rows<HS, OWN, C::THREADS>(own1, (KEYS ? a.V : a.dO) + base, r0, S, hs, a.vec);
     if (!KEYS) load_stats(r0, 0);
     fetch(first);
     float acc0[4][C::CPT], acc1[4][C::CPT];
@@ -347,15 +350,15 @@ __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile
     }
 }
 
-template <int HS, typename T>
-__global__ void __launch_bounds__(kThreads)
+template <int HS, int OWN, typename T>
+__global__ void __launch_bounds__(OWN * 4)
 attn_bwd_simt_kernel(const BwdArgs<T> a) {
     extern __shared__ __align__(16) float smem[];
     // the longest walks first when causal: early key tiles, late query tiles
-    const int n_tiles = (a.S + kRows - 1) / kRows;
+    const int n_own = (a.S + OWN - 1) / OWN;
     const int b = blockIdx.x >> 1, unit = b % a.units, t = b / a.units;
-    if (blockIdx.x & 1) bwd_walk<HS, T, false>(a, unit, n_tiles - 1 - t, smem);
-    else                bwd_walk<HS, T, true>(a, unit, t, smem);
+    if (blockIdx.x & 1) bwd_walk<HS, OWN, T, false>(a, unit, n_own - 1 - t, smem);
+    else                bwd_walk<HS, OWN, T, true>(a, unit, t, smem);
 }
 
 bool rows_aligned(const void* const* ptrs, int n, int64_t hs, int es) {
@@ -364,30 +367,32 @@ bool rows_aligned(const void* const* ptrs, int n, int64_t hs, int es) {
     return ok;
 }
 
-template <int HS, typename T>
-int launch_fwd(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
+template <int HS, int OWN, typename T>
+int launch_fwd_own(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
                const void* V, void* O, float* lse) {
-    auto kern = attn_fwd_simt_kernel<HS, T>;
+    auto kern = attn_fwd_simt_kernel<HS, OWN, T>;
+    constexpr int smem = Tiles<HS, OWN>::FWD_SMEM;
     static bool configured = false;     // per process = per device: the library binds to one device
     if (!configured) {
-        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tiles<HS>::FWD_SMEM));
+        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem > kSpreadSmem ? smem : kSpreadSmem));
         configured = true;
     }
     const void* in[3] = {Q, K, V};
-    const unsigned grid = (unsigned)(units * ceil_div(S, kRows));
-    BOATCU_RUN(kern, grid, kThreads, Tiles<HS>::FWD_SMEM, (int)units, (int)S, hs, causal, scale, rows_aligned(in, 3, hs, sizeof(T)),
+    const unsigned grid = (unsigned)(units * ceil_div(S, OWN));
+    BOATCU_RUN(kern, grid, OWN * 4, spread_smem(smem, grid), (int)units, (int)S, hs, causal, scale, rows_aligned(in, 3, hs, sizeof(T)),
                                                              (const T*)Q, (const T*)K, (const T*)V, (T*)O, lse);
     BOATCU_LAUNCH_OK("attn_fwd_simt");
     return 0;
 }
 
-template <int HS, typename T>
-int launch_bwd(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
+template <int HS, int OWN, typename T>
+int launch_bwd_own(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
                const void* V, const void* dO, const float* lse, const float* delta, void* dQ, void* dK, void* dV) {
-    auto kern = attn_bwd_simt_kernel<HS, T>;
+    auto kern = attn_bwd_simt_kernel<HS, OWN, T>;
+    constexpr int smem = Tiles<HS, OWN>::BWD_SMEM;
     static bool configured = false;
     if (!configured) {
-        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Tiles<HS>::BWD_SMEM));
+        BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem > kSpreadSmem ? smem : kSpreadSmem));
         configured = true;
     }
     const void* in[4] = {Q, K, V, dO};
@@ -398,9 +403,23 @@ int launch_bwd(int64_t units, int64_t S, int hs, int causal, float scale, const 
     a.units = (int)units; a.S = (int)S; a.hs = hs; a.causal = causal;
     a.vec = rows_aligned(in, 4, hs, sizeof(T));
     a.scale = scale;
-    BOATCU_RUN(kern, (unsigned)(2 * units * ceil_div(S, kRows)), kThreads, Tiles<HS>::BWD_SMEM, a);
+    const unsigned grid = (unsigned)(2 * units * ceil_div(S, OWN));
+    BOATCU_RUN(kern, grid, OWN * 4, spread_smem(smem, grid), a);
     BOATCU_LAUNCH_OK("attn_bwd_simt");
     return 0;
+}
+
+// 64 owned rows make half as many fetches of the other side; 32 halve the longest walk of a CTA.  Below
+// about four 64-row CTAs per SM the length of the last walks decides, from there on the fetches do.
+bool own_half(int64_t ctas64) { return ctas64 < 4 * (int64_t)sm_count(); }
+
+template <int HS, typename T, typename... A>
+int launch_fwd(int64_t units, int64_t S, A... args) {
+    return own_half(units * ceil_div(S, 64)) ? launch_fwd_own<HS, 32, T>(units, S, args...) : launch_fwd_own<HS, 64, T>(units, S, args...);
+}
+template <int HS, typename T, typename... A>
+int launch_bwd(int64_t units, int64_t S, A... args) {
+    return own_half(2 * units * ceil_div(S, 64)) ? launch_bwd_own<HS, 32, T>(units, S, args...) : launch_bwd_own<HS, 64, T>(units, S, args...);
 }
 
 #define DISPATCH_HS(FN, ...)                                                                  \
@@ -420,7 +439,7 @@ int launch_bwd(int64_t units, int64_t S, int hs, int causal, float scale, const 
 
 int check_shape(int64_t units, int64_t S, int64_t hs) {
     if (hs > 128) return set_error(8, "attention: head size %lld > 128 is not supported", (long long)hs);
-    if (S > (1ll << 30) || units * ceil_div(S, kRows) > (1ll << 30))
+    if (S > (1ll << 30) || units * ceil_div(S, 32) > (1ll << 30))
         return set_error(8, "attention: %lld (batch x heads) units of %lld rows are too many for one launch", (long long)units, (long long)S);
     return 0;
 }
