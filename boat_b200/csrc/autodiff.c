@@ -74,8 +74,17 @@ void boat_variable_zero_grad(boat_variable_t* v) {
     }
 }
 
-/* grad += g, creating a zero grad of the data's shape first (autodiff.c:2482-2494). */
+/* grad += g, creating a zero grad of the data's shape first (autodiff.c:2482-2494).  Where both are FP32 in
+ * HBM the first contribution is copied instead of added to zeros: one launch, not two. */
 static bool accumulate(boat_variable_t* v, const boat_tensor_t* g) {
+    if (!v->grad && v->data->device == BOAT_DEVICE_CUDA && g->device == BOAT_DEVICE_CUDA &&
+        v->data->dtype == BOAT_DTYPE_FLOAT32 && g->dtype == BOAT_DTYPE_FLOAT32 && g->nelements == v->data->nelements) {
+        boat_tensor_t* copy = boat_tensor_create_uninit(v->data->shape, v->data->ndim, v->data->dtype, v->data->device);
+        if (!copy) return false;
+        boat_report("gradient copy", boat_cuda_scale((float*)copy->data, (const float*)g->data, 1.0f, (int64_t)g->nelements));
+        v->grad = copy;
+        return true;
+    }
     if (!v->grad) {
         v->grad = boat_tensor_create_like(v->data);
         if (!v->grad) return false;
@@ -96,11 +105,34 @@ static void accumulate_owned(boat_variable_t* v, boat_tensor_t* g) {
     boat_tensor_unref(g);
 }
 
+/* The three gradients of a variable that is query, key and value in one pass: v->grad (or g[0], which
+ * becomes it) += the others, in the order of the separate additions.  False where they are not all FP32
+ * arrays in HBM of v's size; g[0] is cleared when it was taken over. */
+static bool accumulate_three(boat_variable_t* v, boat_tensor_t** g) {
+    const boat_tensor_t* all[4] = {g[0], g[1], g[2], v->grad ? v->grad : v->data};
+    for (int i = 0; i < 4; ++i)
+        if (!all[i] || all[i]->device != BOAT_DEVICE_CUDA || all[i]->dtype != BOAT_DTYPE_FLOAT32 || all[i]->nelements != v->data->nelements)
+            return false;
+    int first = 0;
+    if (!v->grad) {
+        v->grad = g[0];
+        g[0] = NULL;
+        first = 1;
+    }
+    const float* x[3] = {(const float*)all[0]->data, (const float*)all[1]->data, (const float*)all[2]->data};
+    boat_report("gradient sum", boat_cuda_add_n((float*)v->grad->data, x + first, 3 - first, (int64_t)v->grad->nelements));
+    return true;
+}
+
 static void backward_attention(op_record_t* op, const boat_tensor_t* grad_output) {
     boat_tensor_t* g[3] = {NULL, NULL, NULL};
     if (!boat_attention_backward((boat_attention_t*)op->layer, grad_output, &g[0], &g[1], &g[2])) return;
-    for (int i = 0; i < 3; ++i)
-        if (g[i] && op->inputs[i] && op->inputs[i]->requires_grad && !accumulate(op->inputs[i], g[i])) break;
+    boat_variable_t* x = op->inputs[0];
+    const bool self = x && x->requires_grad && x == op->inputs[1] && x == op->inputs[2];
+    if (!(self && accumulate_three(x, g))) {
+        for (int i = 0; i < 3; ++i)
+            if (g[i] && op->inputs[i] && op->inputs[i]->requires_grad && !accumulate(op->inputs[i], g[i])) break;
+    }
     for (int i = 0; i < 3; ++i)
         if (g[i]) boat_tensor_unref(g[i]);
 }

@@ -91,6 +91,33 @@ __global__ void axpy_multi_kernel(const AxpyTable t, float alpha, int vec) {
     for (int64_t i = n4 * 4 + i0; i < n; i += step) y[i] = mul_add(alpha, x[i], y[i]);
 }
 
+// ---- y += x[0] + x[1] + ..., in that order: the gradient contributions of one variable ---------------
+constexpr int kMaxAddN = 4;
+struct AddTable {
+    const float* x[kMaxAddN];
+    int count;
+};
+__global__ void add_n_kernel(float* __restrict__ y, const AddTable t, int64_t n, int vec) {
+    griddep_sync();
+    const int64_t n4 = vec ? n / 4 : 0;
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < n4; i += step) {
+        float4 a[kMaxAddN], v = reinterpret_cast<const float4*>(y)[i];
+#pragma unroll
+        for (int k = 0; k < kMaxAddN; ++k)
+            if (k < t.count) a[k] = reinterpret_cast<const float4*>(t.x[k])[i];
+#pragma unroll
+        for (int k = 0; k < kMaxAddN; ++k)
+            if (k < t.count) v = make_float4(v.x + a[k].x, v.y + a[k].y, v.z + a[k].z, v.w + a[k].w);
+        reinterpret_cast<float4*>(y)[i] = v;
+    }
+    for (int64_t i = n4 * 4 + i0; i < n; i += step) {
+        float v = y[i];
+        for (int k = 0; k < t.count; ++k) v += t.x[k][i];
+        y[i] = v;
+    }
+}
+
 // ---- the SGD step of a layer that accumulates its gradients: y -= fl(lr*g), then g = 0 ----------------
 __global__ void sgd_clear_kernel(const AxpyTable t, float lr, int vec) {
     griddep_sync();
@@ -602,6 +629,24 @@ int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, co
     if (int rc = ensure_init()) return rc;
     BOATCU_RUN(axpy_multi_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, alpha, vec);
     BOATCU_LAUNCH_OK("axpy_multi");
+    return 0;
+}
+
+int boat_cuda_add_n(float* y, const float* const* x, int count, int64_t n) {
+    if (count < 1 || count > kMaxAddN) return set_error(11, "boat_cuda_add_n: %d terms (1 to %d)", count, kMaxAddN);
+    if (n <= 0) return 0;
+    if (int rc = ensure_init()) return rc;
+    if (!y || !x) return set_error(11, "boat_cuda_add_n: NULL operand");
+    AddTable t = {};
+    t.count = count;
+    bool vec = aligned16(y);
+    for (int k = 0; k < count; ++k) {
+        if (!x[k]) return set_error(11, "boat_cuda_add_n: NULL operand");
+        t.x[k] = x[k];
+        vec = vec && aligned16(x[k]);
+    }
+    BOATCU_RUN(add_n_kernel, grid_for(vec ? ceil_div(n, 4) : n, kThreads), kThreads, 0, y, t, n, vec ? 1 : 0);
+    BOATCU_LAUNCH_OK("add_n");
     return 0;
 }
 

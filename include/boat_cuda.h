@@ -204,6 +204,8 @@ int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64
 int boat_cuda_axpy(float* y, const float* x, float alpha, int64_t n);
 /* the same for `count` (1 to 8) pairs in one launch: y[i] += alpha * x[i], n[i] elements each */
 int boat_cuda_axpy_multi(float* const* y, const float* const* x, float alpha, const int64_t* n, int count);
+/* y += x[0] + x[1] + ... in that order, `count` (1 to 4) arrays of n elements */
+int boat_cuda_add_n(float* y, const float* const* x, int count, int64_t n);
 /* the SGD step of a layer that accumulates: y[i] -= lr * g[i] (rounded product), then g[i] = 0 */
 int boat_cuda_sgd_clear(float* const* y, float* const* g, float lr, const int64_t* n, int count);
 int boat_cuda_scale(float* y, const float* x, float alpha, int64_t n);
