@@ -234,6 +234,7 @@ PROTOTYPES = {
     "boat_cuda_convert_multi": (_I, [_P, _I, _P, _P, _I]),
     "boat_cuda_axpy": (_I, [_P, _P, _F, _I64]),
     "boat_cuda_sgd_clear": (_I, [_P, _P, _F, _P, _I]),
+    "boat_cuda_stage_copy": (_I, [_P, _P, _SZ, _I]),
     "boat_cuda_add_n": (_I, [_P, _P, _I, _I64]),
     "boat_cuda_axpy_multi": (_I, [_P, _P, _F, _P, _I]),
     "boat_cuda_scale": (_I, [_P, _P, _F, _I64]),

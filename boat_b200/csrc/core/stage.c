@@ -107,7 +107,7 @@ bool boat_bundle_send(boat_bundle_t* b, const boat_tensor_t* const* tensors, int
     }
     for (int i = 0; i < b->count; ++i) memcpy((char*)b->host + b->offset[i], b->tensor[i]->data, b->tensor[i]->nbytes);
     b->sent = true;
-    return boat_report("upload", boat_cuda_memcpy_h2d_async(b->dev, b->host, total)) == 0;
+    return boat_report("upload", boat_cuda_stage_copy(b->dev, b->host, total, 0)) == 0;
 }
 
 void* boat_bundle_find(const boat_bundle_t* b, const boat_tensor_t* t) {
@@ -123,11 +123,31 @@ void boat_bundle_settle(boat_bundle_t* b, bool synced) {
     b->host = NULL;
 }
 
-int boat_scatter_down(const void* dev, size_t total, void* const* host, const size_t* offset, const size_t* bytes, int n) {
+void* boat_landing_alloc(size_t bytes, bool direct, bool* on_host) {
+    void* p = direct && bytes <= BOAT_DIRECT_LIMIT ? boat_cuda_host_alloc(bytes) : NULL;
+    *on_host = p != NULL;
+    return p ? p : boat_dev_alloc(bytes);
+}
+
+void boat_landing_free(void* block, bool on_host, bool synced) {
+    if (on_host && !synced) boat_report("result", boat_cuda_sync());
+    if (on_host) boat_cuda_host_free(block);
+    else boat_dev_free(block);
+}
+
+int boat_scatter_down(const void* dev, bool on_host, size_t total, void* const* host, const size_t* offset, const size_t* bytes, int n) {
+    if (on_host) {
+        const int done = boat_cuda_sync();
+        for (int i = 0; i < n && done == 0; ++i) memcpy(host[i], (const char*)dev + offset[i], bytes[i]);
+        return done;
+    }
     char* image = total < BOAT_BUNDLE_LIMIT ? (char*)boat_cuda_host_alloc(total) : NULL;
     int rc = 0;
     if (image) {
-        rc = boat_cuda_memcpy_d2h(image, dev, total);
+        /* the offsets are multiples of 256 bytes: whole 16-byte units, in the block as in the image */
+        rc = boat_cuda_stage_copy(image, dev, total, 1);
+        const int done = boat_cuda_sync();
+        if (rc == 0) rc = done;
         for (int i = 0; i < n && rc == 0; ++i) memcpy(host[i], image + offset[i], bytes[i]);
         boat_cuda_host_free(image);
         return rc;

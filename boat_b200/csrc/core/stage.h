@@ -39,9 +39,15 @@ void*  boat_bundle_find(const boat_bundle_t* b, const boat_tensor_t* t);
 /* Ends the call: waits for the uploads unless `synced` (the host has waited for a later copy), and
  * gives the image back.  The HBM copy is the caller's to free (boat_dev_free(b->dev)). */
 void   boat_bundle_settle(boat_bundle_t* b, bool synced);
+/* The block that a call's results for the host are produced in.  `direct`: the kernels that write it use plain
+ * stores and none reads it back; then a small block is page-locked host memory, which they write over
+ * the bus, and no copy follows.  *on_host tells which it is; freed with boat_landing_free. */
+#define BOAT_DIRECT_LIMIT ((size_t)64 * 1024)
+void*  boat_landing_alloc(size_t bytes, bool direct, bool* on_host);
+void   boat_landing_free(void* block, bool on_host, bool synced);      /* synced: as for boat_bundle_settle */
 /* Copies n pieces of one device block (at `offset`, `bytes` long) to host memory and waits: small totals as
- * one copy through a page-locked image. */
-int    boat_scatter_down(const void* dev, size_t total, void* const* host, const size_t* offset, const size_t* bytes, int n);
+ * one copy through a page-locked image, no copy at all where the block is such an image (`on_host`). */
+int    boat_scatter_down(const void* dev, bool on_host, size_t total, void* const* host, const size_t* offset, const size_t* bytes, int n);
 static inline size_t boat_align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 /* Arithmetic for FP32/BF16 inputs outside the attention layer: BF16 storage -> BF16 tensor

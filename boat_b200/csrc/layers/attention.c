@@ -628,6 +628,7 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
     staged_params_t p;
     memset(&p, 0, sizeof p);
     void* d_out = NULL;
+    bool out_on_host = false;
     boat_tensor_t* result = NULL;
     bool synced = false;
     const bool pipelined = units / gran >= 2 && act_bytes >= PIPELINE_MIN_BYTES && pipeline_enabled() && on_host(query) &&
@@ -700,7 +701,7 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
                 goto done;
             }
         } else {
-            d_out = dev_alloc((size_t)T * H * storage_size(out_type));
+            d_out = boat_landing_alloc((size_t)T * H * storage_size(out_type), mma == BOAT_MMA_FP32, &out_on_host);
             if (!d_out) goto done;
             if (boat_report("output projection", boat_cuda_gemm(mma, 0, 0, T, H, H, a->d_ctx, H, p.w[WO], H, type,
                                                                 d_out, H, out_type, p.b[WO])) != 0)
@@ -708,7 +709,7 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
             result = boat_tensor_create_uninit(query->shape, query->ndim, query->dtype, query->device);
             if (!result) goto done;
             const size_t at = 0;
-            synced = boat_report("result transfer", boat_scatter_down(d_out, result->nbytes, &result->data, &at, &result->nbytes, 1)) == 0;
+            synced = boat_report("result transfer", boat_scatter_down(d_out, out_on_host, result->nbytes, &result->data, &at, &result->nbytes, 1)) == 0;
             if (!synced) {
                 boat_tensor_free(result);
                 result = NULL;
@@ -718,7 +719,7 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
     if (result) a->cached = true;
 done:
     boat_bundle_settle(&bundle, synced);
-    dev_free(d_out);
+    boat_landing_free(d_out, out_on_host, synced);
     release_params(&p);
     if (!result) {
         /* keep the input references (the reference does, attention.c:355-372) but no
@@ -842,7 +843,7 @@ static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output,
     void* down_host[4];
     size_t down_at[4], down_bytes[4], down_total = 0;
     int down = 0;
-    bool synced = false;
+    bool synced = false, down_on_host = false;
 
     if (!ensure_grads(a)) goto done;
     /* gradient sums of this layer's previous step still on the communication stream read the bucket
@@ -885,7 +886,7 @@ static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output,
         down_total += boat_align256(a->grad_bucket->nbytes);
     }
     if (down_total) {
-        d_down = dev_alloc(down_total);
+        d_down = boat_landing_alloc(down_total, mma == BOAT_MMA_FP32 && !pipelined && boat_cuda_comm_world() <= 1, &down_on_host);
         if (!d_down) goto done;
         if (!d_bucket) d_bucket = (float*)((char*)d_down + down_at[down - 1]);
     }
@@ -988,7 +989,7 @@ static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output,
         }
     }
     if (down_total) {
-        if (boat_report("gradient download", boat_scatter_down(d_down, down_total, down_host, down_at, down_bytes, down)) != 0) goto done;
+        if (boat_report("gradient download", boat_scatter_down(d_down, down_on_host, down_total, down_host, down_at, down_bytes, down)) != 0) goto done;
         synced = true;
     }
     ok = true;
@@ -996,7 +997,7 @@ done:
     boat_cuda_gemm_set_yielding(0);
     boat_bundle_settle(&bundle, synced);
     dev_free(bundle.dev);
-    dev_free(d_down);
+    boat_landing_free(d_down, down_on_host, synced);
     dev_free(scratch);
     for (int i = 0; i < 3; ++i) dev_free(d_dproj[i]);
     dev_free(d_dctx);
@@ -1076,7 +1077,7 @@ void boat_attention_update(boat_attention_t* a, float learning_rate) {
     }
     for (int k = 0; k < count; ++k) y[k] = (float*)(base + at[k]);
     if (boat_report("SGD step", boat_cuda_axpy_multi(y, (const float* const*)x, -learning_rate, n, count)) == 0)
-        synced = boat_report("parameter download", boat_scatter_down(base, total, host, at, bytes, count)) == 0;
+        synced = boat_report("parameter download", boat_scatter_down(base, false, total, host, at, bytes, count)) == 0;
 done:
     boat_bundle_settle(&bundle, synced);
     dev_free(bundle.dev);

@@ -6,6 +6,8 @@ hand host bytes in and out.  The class and method names follow the C functions t
 -> ``Variable``) so that tests read like the reference's own C tests.
 """
 import ctypes as C
+import math
+
 import numpy as np
 
 from . import capi
@@ -57,8 +59,7 @@ class Tensor:
     @property
     def shape(self):
         lib = capi.load()
-        p = lib.boat_tensor_shape(self.h)
-        return tuple(p[i] for i in range(lib.boat_tensor_ndim(self.h)))
+        return tuple(lib.boat_tensor_shape(self.h)[:lib.boat_tensor_ndim(self.h)])
 
     @property
     def dtype(self):
@@ -89,11 +90,12 @@ class Tensor:
 
     def host_view(self):
         """Writable numpy view of a CPU tensor's own memory (the boat_tensor_data() pointer)."""
-        if self.device != capi.DEVICE_CPU:
+        lib, h = capi.load(), self.h
+        if lib.boat_tensor_device(h) != capi.DEVICE_CPU:
             raise BoatError("host_view needs a CPU tensor")
-        n = int(np.prod(self.shape))
-        buf = (C.c_float * n).from_address(self.data_ptr)
-        return np.frombuffer(buf, dtype=np.float32).reshape(self.shape)
+        shape = lib.boat_tensor_shape(h)[:lib.boat_tensor_ndim(h)]
+        # one call builds the array: small programs spend more on this than on the bytes
+        return np.ndarray(shape, np.float32, (C.c_char * (4 * math.prod(shape))).from_address(lib.boat_tensor_data(h)))
 
     def set(self, a):
         """Overwrite the contents from a host FP32 array (H2D copy for CUDA tensors)."""

@@ -52,6 +52,9 @@ int         boat_cuda_memcpy_h2d(void* dst, const void* src_host, size_t bytes);
 int         boat_cuda_memcpy_h2d_async(void* dst, const void* src_host, size_t bytes);   /* in stream order; the source
                                                  must stay as it is until the library stream has passed the copy */
 int         boat_cuda_memcpy_d2h(void* dst_host, const void* src, size_t bytes);  /* returns after arrival */
+/* Asynchronous copy between HBM and a block of boat_cuda_host_alloc (down: from HBM to it); the cheapest way
+ * for a few hundred kilobytes. */
+int         boat_cuda_stage_copy(void* dst, const void* src, size_t bytes, int down);
 int         boat_cuda_memcpy_d2d(void* dst, const void* src, size_t bytes);       /* asynchronous on the stream */
 /* Copies on their own streams, one per direction, so that PCIe traffic overlaps kernels.
  * copies_after_compute: both copy streams wait for what has been launched (and allocated) on
