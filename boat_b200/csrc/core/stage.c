@@ -141,7 +141,7 @@ int boat_scatter_down(const void* dev, bool on_host, size_t total, void* const* 
         for (int i = 0; i < n && done == 0; ++i) memcpy(host[i], (const char*)dev + offset[i], bytes[i]);
         return done;
     }
-    char* image = total < BOAT_BUNDLE_LIMIT ? (char*)boat_cuda_host_alloc(total) : NULL;
+    char* image = total < BOAT_IMAGE_LIMIT ? (char*)boat_cuda_host_alloc(total) : NULL;
     int rc = 0;
     if (image) {
         /* the offsets are multiples of 256 bytes: whole 16-byte units, in the block as in the image */

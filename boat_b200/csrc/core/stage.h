@@ -23,7 +23,8 @@ boat_tensor_t* boat_emit_out_take(const int64_t* shape, size_t ndim, const boat_
  * host waits for it, which is all that small tensors cost; so those under BOAT_BUNDLE_LIMIT bytes are
  * packed into one page-locked image and go up as one copy, larger ones are sent one by one, and
  * nothing is waited for until the call ends. */
-#define BOAT_BUNDLE_LIMIT ((size_t)256 * 1024)
+#define BOAT_BUNDLE_LIMIT ((size_t)64 * 1024)          /* from here on tensors are page-locked: memory.c */
+#define BOAT_IMAGE_LIMIT ((size_t)256 * 1024)          /* results under this total come down as one copy */
 enum { BOAT_BUNDLE_MAX = 16 };
 typedef struct {
     void *host, *dev;                                    /* the image and its copy in HBM */
