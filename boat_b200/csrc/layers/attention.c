@@ -404,11 +404,15 @@ static boat_tensor_t* forward_pipelined(boat_attention_t* a, const boat_tensor_t
         for (int i = 0; i < 3; ++i)
             if (a->d_in_owned[i] && stage_rows(in[i], mma, type, a->d_in[i], raw[i], r0, nr, H) != 0) goto done;
         if (c == 0 && !stage_param_range(a, type, p, WQ, WV)) goto done;
+        const void* x[3];
+        void* y[3];
         for (int i = 0; i < 3; ++i) {
-            if (boat_report("projection", boat_cuda_gemm(mma, 0, 0, nr, H, H, (char*)a->d_in[i] + off, H, p->w[i], H, type,
-                                                         (char*)a->d_proj[i] + off, H, feed_type(mma, type), p->b[i])) != 0)
-                goto done;
+            x[i] = (char*)a->d_in[i] + off;
+            y[i] = (char*)a->d_proj[i] + off;
         }
+        if (boat_report("projections", boat_cuda_gemm_grouped(mma, 0, 0, 3, nr, H, H, x, H, (const void* const*)p->w, H, type, y, H,
+                                                              feed_type(mma, type), (const float* const*)p->b)) != 0)
+            goto done;
         if (boat_report("attention core",
                         boat_cuda_attn_fwd(mma, (b1 - b0) * a->gran, S, hs, a->config.causal_mask, 1.0f / sqrtf((float)hs),
                                            (char*)a->d_proj[0] + off, (char*)a->d_proj[1] + off, (char*)a->d_proj[2] + off,
@@ -488,8 +492,8 @@ static bool backward_pipelined(boat_attention_t* a, const boat_tensor_t* grad_ou
         const int64_t r0 = b0 * grows, nr = (b1 - b0) * grows;
         const size_t off = (size_t)(r0 * H) * tsz;
         if (stage_rows(grad_output, mma, type, d_go, raw_go, r0, nr, H) != 0) goto done;
-        /* Wo behind the first chunk of dOut; the other weights behind it, needed only after the
-         * attention-core backward of that chunk */
+        /* Wo behind the first chunk of dOut; the other weights behind it, each just before the input gradient that
+         * wants it, so that the first download does not wait for all of them */
         if (c == 0 && !stage_param_range(a, type, p, WO, WO)) goto done;
         /* d(ctx) = dOut . Wo^T */
         if (boat_report("dOut.Wo^T", boat_cuda_gemm(mma, 0, 1, nr, H, H, (char*)d_go + off, H, p->w[WO], H, type,
@@ -502,8 +506,8 @@ static bool backward_pipelined(boat_attention_t* a, const boat_tensor_t* grad_ou
                                            (char*)d_dproj[0] + off, (char*)d_dproj[1] + off, (char*)d_dproj[2] + off,
                                            scratch, scratch_bytes)) != 0)
             goto done;
-        if (c == 0 && !stage_param_range(a, type, p, WQ, WV)) goto done;
         for (int i = 0; i < 3; ++i) {
+            if (c == 0 && !stage_param_range(a, type, p, WQ + i, WQ + i)) goto done;
             const size_t osz = storage_size(out_type[i]), ooff = (size_t)(r0 * H) * osz;
             /* dX = dP . W^T */
             if (boat_report("dX", boat_cuda_gemm(mma, 0, 1, nr, H, H, (char*)d_dproj[i] + off, H, p->w[i], H, type,
