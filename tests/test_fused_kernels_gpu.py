@@ -1,0 +1,202 @@
+"""GPU tests of the fused kernels and of the branches of their dispatch, at the sizes where they change,
+against numpy in float64."""
+import ctypes as C
+import math
+
+import numpy as np
+import pytest
+
+from boat_b200 import capi, rng
+from boat_b200.host import Attention, DeviceBuffer, Tensor, Variable, check
+from gpu_driver import gpu_step
+from test_kernels_gpu import rel, run_core, run_gemm
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(bufs):
+    return (C.c_void_p * len(bufs))(*[b.p.value for b in bufs])
+
+
+def _bf(seed, stream, shape, scale=1.0):
+    return rng.bf16_round(rng.normal(seed, stream, shape) * np.float32(scale))
+
+
+def _gelu(x):
+    return 0.5 * x * (1 + np.tanh(math.sqrt(2 / math.pi) * (x + 0.044715 * x ** 3)))
+
+
+def _gelu_grad(x):
+    t = np.tanh(math.sqrt(2 / math.pi) * (x + 0.044715 * x ** 3))
+    return 0.5 * (1 + t) + 0.5 * x * (1 - t * t) * math.sqrt(2 / math.pi) * (1 + 3 * 0.044715 * x * x)
+
+
+# one tile, ragged rows and columns, K tails, many tiles; the last two are not for the tensor cores
+@pytest.mark.parametrize("shape", [(128, 64, 64), (333, 136, 200), (700, 768, 72), (2100, 520, 256), (40, 24, 16), (130, 70, 64)])
+@pytest.mark.parametrize("epilogue", [1, 2, 3], ids=["gelu", "gelu_grad", "add"])
+def test_gemm_epilogues(gpu_lib, shape, epilogue):
+    M, N, K = shape
+    tb = epilogue == 2
+    a, b = _bf(1, 0, (M, K)), _bf(1, 1, (N, K) if tb else (K, N), 1 / math.sqrt(K))
+    aux, bias = _bf(1, 2, (M, N)), None if tb else rng.normal(1, 3, (N,))
+    da, db, daux = (DeviceBuffer.from_numpy(t, bf16=True) for t in (a, b, aux))
+    dbias = DeviceBuffer.from_numpy(bias) if bias is not None else None
+    dc = DeviceBuffer(M * N * 2)
+    check(gpu_lib.boat_cuda_gemm_fused(capi.MMA_BF16, epilogue, 0, int(tb), M, N, K, da.p, K, db.p, K if tb else N, capi.CUDA_BF16,
+                                       dc.p, N, dbias.p if dbias else None, daux.p), "gemm_fused")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    z = a.astype(np.float64) @ (b.T if tb else b).astype(np.float64) + (0 if bias is None else bias)
+    got = dc.numpy((M, N), bf16=True)
+    if epilogue == 1:
+        assert rel(daux.numpy((M, N), bf16=True), z) <= 3e-3
+        z = _gelu(z)
+    else:
+        z = z * _gelu_grad(aux.astype(np.float64)) if epilogue == 2 else z + aux
+    assert rel(got, z) <= 5e-3
+
+
+@pytest.mark.parametrize("shape", [(128, 64, 64), (333, 768, 96), (2000, 320, 200)])
+@pytest.mark.parametrize("groups", [1, 2, 3])
+def test_gemm_sum_of_products(gpu_lib, shape, groups):
+    M, N, K = shape
+    a, b = [_bf(2, g, (M, K)) for g in range(groups)], [_bf(3, g, (N, K)) for g in range(groups)]
+    da, db = [DeviceBuffer.from_numpy(t, bf16=True) for t in a], [DeviceBuffer.from_numpy(t, bf16=True) for t in b]
+    dc = DeviceBuffer(M * N * 4)
+    check(gpu_lib.boat_cuda_gemm_sum(capi.MMA_BF16, 0, 1, groups, M, N, K, _table(da), K, _table(db), K, capi.CUDA_BF16, dc.p, N,
+                                     capi.CUDA_F32), "gemm_sum")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    assert rel(dc.numpy((M, N)), sum(x.astype(np.float64) @ y.astype(np.float64).T for x, y in zip(a, b))) <= 1e-5
+    assert gpu_lib.boat_cuda_gemm_sum(capi.MMA_FP32, 0, 1, groups, M, N, K, _table(da), K, _table(db), K, capi.CUDA_F32, dc.p, N,
+                                      capi.CUDA_F32) == 13
+
+
+# one CTA's tiles of every width, a pair's, and the split of FP32 results with its remainders
+@pytest.mark.parametrize("shape", [(128, 64, 64), (129, 200, 64), (1300, 768, 200), (2300, 1100, 136), (4096, 2304, 64)])
+@pytest.mark.parametrize("layout", [(0, 0), (0, 1)], ids=["nn", "nt"])
+def test_gemm_tile_shapes(gpu_lib, shape, layout):
+    got, ref = run_gemm(gpu_lib, capi.MMA_BF16, *layout, *shape, out_bf16=True)
+    assert rel(got, ref) <= 3e-3
+
+
+@pytest.mark.parametrize("shape", [(256, 192, 3000), (512, 512, 1500), (768, 520, 5000)])
+def test_gemm_split_of_fp32_results(gpu_lib, shape):
+    got, ref = run_gemm(gpu_lib, capi.MMA_BF16, 1, 0, *shape, bias=False)
+    assert rel(got, ref) <= 1e-5
+
+
+@pytest.mark.parametrize("bf", [False, True], ids=["fp32", "bf16"])
+@pytest.mark.parametrize("shape", [(64, 64, 200), (136, 72, 333), (256, 512, 3000)])
+def test_weight_grads_accumulate(gpu_lib, bf, shape):
+    I, O, T = shape
+    make = _bf if bf else (lambda s, i, sh: rng.normal(s, i, sh))
+    x, dy = make(4, 0, (T, I)), make(4, 1, (T, O))
+    w0, b0 = rng.normal(4, 2, (I, O)), rng.normal(4, 3, (O,))
+    dx, ddy = DeviceBuffer.from_numpy(x, bf16=bf), DeviceBuffer.from_numpy(dy, bf16=bf)
+    dw, db = DeviceBuffer.from_numpy(w0), DeviceBuffer.from_numpy(b0)
+    check(gpu_lib.boat_cuda_weight_grads(capi.MMA_BF16 if bf else capi.MMA_FP32, 1, I, O, T, _table([dx]), _table([ddy]),
+                                         capi.CUDA_BF16 if bf else capi.CUDA_F32, _table([dw]), _table([db]), 1), "weight_grads")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    assert rel(dw.numpy((I, O)), w0 + x.astype(np.float64).T @ dy.astype(np.float64)) <= 1e-5
+    assert np.abs(db.numpy((O,)) - (b0 + dy.astype(np.float64).sum(0))).max() <= 1e-6 * np.abs(dy).sum(0).max()
+
+
+@pytest.mark.parametrize("n", [1, 4, 1023, 4096, 100003])
+def test_elementwise_over_several_arrays(gpu_lib, n):
+    a = [rng.normal(5, i, (n,)) for i in range(4)]
+    y = DeviceBuffer.from_numpy(a[0])
+    x = [DeviceBuffer.from_numpy(t) for t in a[1:]]
+    check(gpu_lib.boat_cuda_add_n(y.p, _table(x), 3, n), "add_n")
+    want = ((a[0] + a[1]) + a[2]) + a[3]
+    assert np.array_equal(y.numpy((n,)), want)
+    sizes = (C.c_int64 * 2)(n, (n + 1) // 2)
+    w, g = [DeviceBuffer.from_numpy(t) for t in a[:2]], [DeviceBuffer.from_numpy(t) for t in a[2:]]
+    check(gpu_lib.boat_cuda_axpy_multi(_table(w), _table(g), C.c_float(-0.5), sizes, 2), "axpy_multi")
+    assert np.array_equal(w[0].numpy((n,)), a[0] - np.float32(0.5) * a[2])
+    check(gpu_lib.boat_cuda_sgd_clear(_table(w), _table(g), C.c_float(0.25), sizes, 2), "sgd_clear")
+    h = sizes[1]
+    assert np.array_equal(w[1].numpy((n,))[:h], (a[1] - np.float32(0.5) * a[3])[:h] - np.float32(0.25) * a[3][:h])
+    assert np.array_equal(w[1].numpy((n,))[h:], a[1][h:])
+    assert not g[0].numpy((n,)).any() and not g[1].numpy((n,))[:h].any() and np.array_equal(g[1].numpy((n,))[h:], a[3][h:])
+
+
+@pytest.mark.parametrize("nbytes", [4, 16, 4096 + 16, 1000004, 256 * 1024, 256 * 1024 + 16])
+def test_stage_copy(gpu_lib, nbytes):
+    src = rng.normal(6, 0, (nbytes // 4,))
+    up, down = (gpu_lib.boat_cuda_host_alloc(nbytes) for _ in range(2))
+    dev = DeviceBuffer(nbytes)
+    C.memmove(up, src.ctypes.data, nbytes)
+    check(gpu_lib.boat_cuda_stage_copy(dev.p, up, nbytes, 0), "up")
+    check(gpu_lib.boat_cuda_stage_copy(down, dev.p, nbytes, 1), "down")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    assert C.string_at(down, nbytes) == src.tobytes()
+    for p in (up, down):
+        gpu_lib.boat_cuda_host_free(p)
+
+
+# rows of less than a warp's width, the widths with registers of their own, and one beyond them
+@pytest.mark.parametrize("bf", [False, True], ids=["fp32", "bf16"])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (37, 100), (333, 768), (1000, 1024), (50, 4096), (9, 5000)])
+def test_layernorm_rows_and_residual_gradient(gpu_lib, bf, rows, cols):
+    make = _bf if bf else (lambda s, i, sh: rng.normal(s, i, sh))
+    x, dy, add = make(7, 0, (rows, cols)), make(7, 1, (rows, cols)), make(7, 2, (rows, cols))
+    gamma, beta = 1 + rng.normal(7, 3, (cols,)) * np.float32(0.1), rng.normal(7, 4, (cols,))
+    ty = capi.CUDA_BF16 if bf else capi.CUDA_F32
+    es = 2 if bf else 4
+    dx_, ddy, dadd = (DeviceBuffer.from_numpy(t, bf16=bf) for t in (x, dy, add))
+    dg, dbt = DeviceBuffer.from_numpy(gamma), DeviceBuffer.from_numpy(beta)
+    y, dx = DeviceBuffer(rows * cols * es), DeviceBuffer(rows * cols * es)
+    mean, rstd, dgam, dbet = (DeviceBuffer(4 * n) for n in (rows, rows, cols, cols))
+    check(gpu_lib.boat_cuda_layernorm_fwd(dx_.p, ty, rows, cols, dg.p, dbt.p, C.c_float(1e-5), y.p, mean.p, rstd.p), "fwd")
+    X, G = x.astype(np.float64), dy.astype(np.float64)
+    mu = X.mean(1, keepdims=True)
+    rs = 1 / np.sqrt(X.var(1, keepdims=True) + 1e-5)
+    hat = (X - mu) * rs
+    tol = 8e-3 if bf else 2e-6
+    assert rel(y.numpy((rows, cols), bf16=bf), hat * gamma + beta) <= tol
+    p = G * gamma
+    ref = (p - p.mean(1, keepdims=True) - hat * (p * hat).mean(1, keepdims=True)) * rs
+    for res, want in ((None, ref), (dadd.p, ref + add)):
+        check(gpu_lib.boat_cuda_layernorm_bwd_add(ddy.p, dx_.p, ty, rows, cols, dg.p, mean.p, rstd.p, res, dx.p, dgam.p, dbet.p), "bwd")
+        check(gpu_lib.boat_cuda_sync(), "sync")
+        assert rel(dx.numpy((rows, cols), bf16=bf), want) <= tol
+        assert np.abs(dgam.numpy((cols,)) - (G * hat).sum(0)).max() <= 1e-5 * np.abs(G * hat).sum(0).max()
+        assert np.abs(dbet.numpy((cols,)) - G.sum(0)).max() <= 1e-5 * np.abs(G).sum(0).max()
+
+
+# more work than SMs: every CTA of the persistent kernels takes several items, unevenly long ones when causal
+@pytest.mark.parametrize("hs,units,S", [(64, 170, 300), (128, 100, 520)])
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+def test_attention_core_with_several_items_per_cta(gpu_lib, hs, units, S, causal):
+    got, ref = run_core(gpu_lib, capi.MMA_BF16, units, S, hs, causal)
+    for key in ("o", "dq", "dk", "dv"):
+        assert rel(got[key], ref[key]) <= 2e-2, key
+
+
+# results written to page-locked memory, packed and separate copies, chunks of more than one batch entry
+@pytest.mark.parametrize("B,S,H,nh", [(2, 4, 32, 4), (3, 40, 128, 4), (5, 61, 256, 8), (6, 700, 256, 8)])
+def test_host_tensors_give_the_results_of_cuda_tensors(gpu_lib, B, S, H, nh):
+    n = lambda i, *s: rng.normal(8, i, s)  # noqa: E731
+    x = n(0, B, S, H)
+    inp = {"q": x, "k": x, "v": x, "w": [n(1 + i, H, H) / np.float32(math.sqrt(H)) for i in range(4)],
+           "b": [n(5 + i, H) for i in range(4)], "dout": n(9, B, S, H)}
+    host, cuda = (gpu_step(inp, nh, True, device=d, lr=0.1) for d in (capi.DEVICE_CPU, capi.DEVICE_CUDA))
+    for k in ("out", "dq", "dk", "dv"):
+        assert rel(host[k], cuda[k]) <= 1e-6, k
+    for k in ("dw", "db", "w_after"):
+        for i in range(4):
+            assert rel(host[k][i], cuda[k][i]) <= 1e-6 or np.abs(host[k][i]).max() <= 1e-5, (k, i)
+
+
+def test_self_attention_gradient_is_the_sum_of_three(gpu_lib):
+    B, S, H, nh = 2, 50, 64, 4
+    layer = Attention(H, nh, causal=True)
+    layer.to_device(capi.DEVICE_CUDA)
+    x, g = rng.normal(9, 0, (B, S, H)), rng.normal(9, 1, (B, S, H))
+    grads = []
+    for distinct in (False, True):
+        t = [Variable(Tensor.from_numpy(x, capi.DEVICE_CUDA)) for _ in range(3 if distinct else 1)]
+        q, k, v = t if distinct else t * 3
+        r = q.attention(layer, k, v) + q
+        r.backward(Tensor.from_numpy(g, capi.DEVICE_CUDA))
+        grads.append(sum(u.grad.numpy().astype(np.float64) for u in t))
+    assert rel(grads[0], grads[1]) <= 1e-6
