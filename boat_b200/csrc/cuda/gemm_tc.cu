@@ -436,12 +436,17 @@ struct Problem {
     void* aux;           // second result or operand of the epilogue, laid out like C
 };
 
-// A tile shape and what it costs, measured on B200 at 12 to 512 K-blocks (64 BF16): microseconds per K-block,
-// and once per launch (filling the ring, the epilogue that nothing overlaps).  Pairs on 256 x 256 are
-// fastest per FLOP (1440 TFLOP/s at 32768 x 2048 x 2048; a single CTA's 128 x 256 1220, 128 x 128 900,
-// 128 x 64 510) and slowest to start.
-struct Shape { int ctas, bn; double block_us, once_us; };
-constexpr Shape kShapes[4] = {{2, 256, 0.31, 2.7}, {1, 256, 0.34, 1.1}, {1, 128, 0.23, 0.6}, {1, 64, 0.20, 0.0}};
+// A tile shape and what it costs, measured on B200 with every shape forced on outputs of 128 x 1024 to
+// 8192 x 1024 and 1024 x 1024 x 8192: microseconds per K-block (128 bytes of K per row), and once per launch more than
+// the narrowest tile (filling the ring, the epilogue that nothing overlaps).  A K-block costs what its bytes cost to
+// bring to the SM; FP32 operands that lie along M or N add to that, since the tensor core then
+// reads them at about half its rate (block_us[1]: B, [2]: both).  Pairs on 256 x 256 are fastest per FLOP (1440
+// TFLOP/s BF16 at 32768 x 2048 x 2048; a single CTA's 128 x 256 1220, 128 x 128 900, 128 x 64 510) and slowest to start.
+struct Shape { int ctas, bn; double block_us[3], once_us; };
+constexpr Shape kShapes[4] = {{2, 256, {0.38, 0.50, 0.52}, 3.5},
+                              {1, 256, {0.44, 0.70, 0.90}, 1.3},
+                              {1, 128, {0.31, 0.47, 0.64}, 1.1},
+                              {1, 64, {0.30, 0.36, 0.44}, 0.0}};
 
 struct Plan {
     int64_t tiles, full, split;
@@ -449,13 +454,14 @@ struct Plan {
 };
 
 // Which tiles are cut along K, into how many pieces, and how long the launch should take.
-Plan make_plan(const Problem& q, const Shape& sh, int bk) {
+Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
+    const double block_us = sh.block_us[slow];
     const int64_t workers = sm_count() / sh.ctas, k_blocks = ceil_div(q.K, bk) * (q.chain ? q.groups : 1);
     Plan r;
     r.tiles = ceil_div(q.M, BM * sh.ctas) * ceil_div(q.N, sh.bn) * (q.chain ? 1 : q.groups);
     r.full = r.tiles;
     r.split = 1;
-    r.us = (double)ceil_div(r.tiles, workers) * (double)k_blocks * sh.block_us + sh.once_us;
+    r.us = (double)ceil_div(r.tiles, workers) * (double)k_blocks * block_us + sh.once_us;
     if (q.out_type != BOAT_CUDA_F32) return r;
     // FP32 results: the last, partly filled wave of tiles is cut so that its pieces come out even over
     // all workers; at least 8 K-blocks per piece, and no more than two pieces below K = 2048 (two
@@ -468,9 +474,9 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk) {
     if (q.K < 2048 && most > 2) most = 2;
     if (most > 32) most = 32;
     for (int64_t s = 2; s <= most && rest > 0; ++s) {
-        double piece = (double)k_blocks / (double)s * sh.block_us;
+        double piece = (double)k_blocks / (double)s * block_us;
         if (piece < out_us) piece = out_us;
-        const double t = (double)whole * (double)k_blocks * sh.block_us + (double)ceil_div(rest * s, workers) * piece + out_us +
+        const double t = (double)whole * (double)k_blocks * block_us + (double)ceil_div(rest * s, workers) * piece + out_us +
                          clear_us + sh.once_us;
         if (t < r.us) {
             r.us = t;
@@ -545,7 +551,7 @@ int pick_tile(const Problem& q) {
     int best = 0;
     Plan plan;
     for (int i = 0; i < 4; ++i) {
-        const Plan t = make_plan(q, kShapes[i], 128 / (int)sizeof(T));
+        const Plan t = make_plan(q, kShapes[i], 128 / (int)sizeof(T), sizeof(T) == 4 ? (int)A_MN + (int)B_MN : 0);
         if (i == 0 || t.us < plan.us) {
             plan = t;
             best = i;
