@@ -464,14 +464,14 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
     r.us = (double)ceil_div(r.tiles, workers) * (double)k_blocks * block_us + sh.once_us;
     if (q.out_type != BOAT_CUDA_F32) return r;
     // FP32 results: the last, partly filled wave of tiles is cut so that its pieces come out even over
-    // all workers; at least 8 K-blocks per piece, and no more than two pieces below K = 2048 (two
-    // addends give the same bits in either order).  An SM gets its part of a piece out at about 36 KB per
+    // all workers; at least 8 K-blocks per piece, and none below K = 2048: there a group of problems gives
+    // the bits of single calls, and the pieces hardly pay for clearing the output.  An SM gets its part of a piece out at about 36 KB per
     // microsecond, behind the next piece's main loop but for the last one; the output is cleared first.
     const int64_t rest = r.tiles % workers, whole = r.tiles / workers;
     const double out_us = BM * sh.bn * 4.0 / 36e3;
     const double clear_us = q.add ? 0.0 : 2.0 + (double)q.M * (double)q.N * q.groups * 4.0 / 4e6;
     int64_t most = k_blocks / 8;
-    if (q.K < 2048 && most > 2) most = 2;
+    if (q.K < 2048) most = 1;
     if (most > 32) most = 32;
     for (int64_t s = 2; s <= most && rest > 0; ++s) {
         double piece = (double)k_blocks / (double)s * block_us;
