@@ -5,21 +5,23 @@
 // the probabilities are rebuilt from the saved log-sum-exp tile by tile, and P and dS stay in
 // TF32 (never BF16), so the result holds the 5e-3 tolerance of TF32 arithmetic.
 //
-// Two kernels instead of one.  The BF16 backward keeps dS^T in shared memory because dQ = dS.K
+// Two kinds of CTA.  The BF16 backward keeps dS^T in shared memory because dQ = dS.K
 // wants dS with queries on the M side while dK = dS^T.Q wants it with keys on the M side; an
 // FP32 dS^T tile is 64 KB and does not fit beside double-staged FP32 Q/dO tiles.  Splitting the
 // work by output removes the tile altogether - each product then takes its left operand
 // straight from tensor memory, exactly where the softmax warps wrote it:
 //
-//   dq kernel   CTA = one 128-row query tile, walks the key tiles (like the forward)
+//   dQ          CTA = one 128-row query tile, walks the key tiles (like the forward)
 //       S  = Q.K^T, dP = dO.V^T             both operands from shared memory
 //       dS = P*(dP - delta)/sqrt(hs)        softmax warps, thread = query row, written over S
 //       dQ += dS.K                          A = dS from tensor memory, B = K with hs on the N side
-//   dkv kernel  CTA = one 128-row key tile, walks the query tiles that see it
+//   dK, dV      CTA = one 128-row key tile, walks the query tiles that see it
 //       S^T = K.Q^T, dP^T = V.dO^T
 //       P^T over S^T, dS^T over dP^T        softmax warps, thread = key row
 //       dV += P^T.dO,  dK += dS^T.Q         A from tensor memory, B = dO / Q with hs on the N side
-// dQ, dK, dV leave the kernels rounded to TF32: they feed the TF32 projection GEMMs.
+// One launch holds both kinds, the longer dK/dV ones first, so that the dQ ones fill the SMs that a last
+// wave of the others leaves idle.
+// dQ, dK, dV leave the kernel rounded to TF32: they feed the TF32 projection GEMMs.
 //
 // No scratch memory, no atomics, no reduction between CTAs: every output row is produced by one
 // CTA, so the results are deterministic.  The price is that S and dP are computed twice (7
@@ -27,7 +29,7 @@
 //
 // An FP32 operand that the tensor core reads along M or N must lie in shared memory with the
 // 128-byte swizzle in 32-byte units, one that it reads along K with the usual 16-byte units.
-// K (dq kernel) and Q, dO (dkv kernel) are needed both ways, so those tiles are loaded twice,
+// K (dQ) and Q, dO (dK, dV) are needed both ways, so those tiles are loaded twice,
 // once per tensor map; the second copy comes from L2.
 // Warp 0: TMA producer, warp 1: MMA issuer, warps 2-5: softmax and epilogue.
 #pragma once
@@ -45,16 +47,16 @@ struct Bwd32Cfg {
     static constexpr int SMEM_DQ = 2 * kBwd32Tile + 3 * kBwd32Tile + 1024 + 256;
     static constexpr int SMEM_DKV = 2 * kBwd32Tile + 4 * kBwd32Tile + 2048 + 1024 + 256;
     static constexpr uint32_t COL_S = 0, COL_DP = 128;
-    static constexpr uint32_t COL_DQ = 256;                     // dq kernel
-    static constexpr uint32_t COL_DV = 256, COL_DK = 320;       // dkv kernel
+    static constexpr uint32_t COL_DQ = 256;                     // dQ CTAs
+    static constexpr uint32_t COL_DV = 256, COL_DK = 320;       // dK, dV CTAs
     static constexpr uint32_t TMEM_COLS = 512;
 };
 
 struct Bwd32Params {
     const float* lse;      // [units*S]
     const float* delta;    // [units*S]
-    float* dQ;             // dq kernel
-    float* dK;             // dkv kernel
+    float* dQ;             // dQ CTAs
+    float* dK;             // dK, dV CTAs
     float* dV;
     int S, units, causal;
     float scale;
@@ -70,10 +72,8 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 // ------------------------------------------------------------------------------------------------
 // dQ: one query tile per CTA
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBwd32Threads, 1)
-attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                        const __grid_constant__ CUtensorMap map_k_mn, const __grid_constant__ CUtensorMap map_v,
-                        const __grid_constant__ CUtensorMap map_do, const Bwd32Params p) {
+__device__ __forceinline__ void bwd32_dq(int block, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_k_mn,
+                                         const CUtensorMap& map_v, const CUtensorMap& map_do, const Bwd32Params& p) {
     using C = Bwd32Cfg;
     constexpr int HS = kBwd32HS;
     extern __shared__ uint8_t smem_raw[];
@@ -94,8 +94,8 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
-    const int unit = blockIdx.x % p.units;
-    const int qt = n_tiles - 1 - blockIdx.x / p.units;       // long (late) rows first when causal
+    const int unit = block % p.units;
+    const int qt = n_tiles - 1 - block / p.units;       // long (late) rows first when causal
     const int n_kv = p.causal ? qt + 1 : n_tiles;
 
     if (threadIdx.x == 0) {
@@ -241,11 +241,9 @@ attn_bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 // ------------------------------------------------------------------------------------------------
 // dK, dV: one key tile per CTA
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBwd32Threads, 1)
-attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q_mn,
-                         const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                         const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_do_mn,
-                         const Bwd32Params p) {
+__device__ __forceinline__ void bwd32_dkv(int block, const CUtensorMap& map_q, const CUtensorMap& map_q_mn, const CUtensorMap& map_k,
+                                          const CUtensorMap& map_v, const CUtensorMap& map_do, const CUtensorMap& map_do_mn,
+                                          const Bwd32Params& p) {
     using C = Bwd32Cfg;
     constexpr int HS = kBwd32HS;
     extern __shared__ uint8_t smem_raw[];
@@ -269,8 +267,8 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
-    const int unit = blockIdx.x % p.units;
-    const int jt = blockIdx.x / p.units;                     // early key tiles have the long walks when causal
+    const int unit = block % p.units;
+    const int jt = block / p.units;                     // early key tiles have the long walks when causal
     const int i0 = p.causal ? jt : 0;
     const int n_q = n_tiles - i0;
 
@@ -443,6 +441,17 @@ attn_bwd_dkv_tf32_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         tc_fence_after_sync();
         tmem_dealloc(tmem_base, C::TMEM_COLS);
     }
+}
+
+struct Bwd32Maps {
+    CUtensorMap q, q_mn, k, k_mn, v, dout, dout_mn;      // _mn: read along the rows, 32-byte swizzle units
+};
+
+__global__ void __launch_bounds__(kBwd32Threads, 1)
+attn_bwd_tf32_kernel(const __grid_constant__ Bwd32Maps m, const __grid_constant__ Bwd32Params p) {
+    const int n = gridDim.x / 2;
+    if (blockIdx.x < n) bwd32_dkv(blockIdx.x, m.q, m.q_mn, m.k, m.v, m.dout, m.dout_mn, p);
+    else                bwd32_dq(blockIdx.x - n, m.q, m.k, m.k_mn, m.v, m.dout, p);
 }
 
 }  // namespace attn_tc

@@ -125,22 +125,22 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     return 0;
 }
 
-// FP32 storage, TF32 arithmetic, head size 64: a dQ kernel over query tiles and a dK/dV kernel over
-// key tiles; no scratch beyond delta.
+// FP32 storage, TF32 arithmetic, head size 64: one launch of CTAs over key tiles (dK, dV) and CTAs over
+// query tiles (dQ); no scratch beyond delta.
 int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const void* Q, const void* K, const void* V,
                     const void* dO, const float* lse, const float* delta, void* dQ, void* dK, void* dV) {
     using C = Bwd32Cfg;
-    constexpr int HS = kBwd32HS;
-    CUtensorMap mq, mq_mn, mk, mk_mn, mv, mdo, mdo_mn;
+    constexpr int HS = kBwd32HS, SMEM = C::SMEM_DKV > C::SMEM_DQ ? C::SMEM_DKV : C::SMEM_DQ;
+    Bwd32Maps m;
     // the same matrices with both shared-memory layouts: 16-byte swizzle units for operands read
     // along hs, 32-byte units for operands read along their rows
-    if (int rc = make_tensor_map_units(&mq, Q, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mq_mn, Q, 4, units, S, HS, kTile, true)) return rc;
-    if (int rc = make_tensor_map_units(&mk, K, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mk_mn, K, 4, units, S, HS, kTile, true)) return rc;
-    if (int rc = make_tensor_map_units(&mv, V, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mdo, dO, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mdo_mn, dO, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_units(&m.q, Q, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&m.q_mn, Q, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_units(&m.k, K, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&m.k_mn, K, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_units(&m.v, V, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&m.dout, dO, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&m.dout_mn, dO, 4, units, S, HS, kTile, true)) return rc;
     Bwd32Params p;
     p.lse = lse;
     p.delta = delta;
@@ -154,16 +154,13 @@ int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const voi
     p.status = kernel_status_ptr();
     static bool configured = false;     // per process = per device: the library binds to one device
     if (!configured) {
-        BOATCU_CHECK(cudaFuncSetAttribute(attn_bwd_dq_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_DQ));
-        BOATCU_CHECK(cudaFuncSetAttribute(attn_bwd_dkv_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_DKV));
+        BOATCU_CHECK(cudaFuncSetAttribute(attn_bwd_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
         configured = true;
     }
-    const unsigned grid = (unsigned)(units * ceil_div(S, kTile));
+    const unsigned grid = (unsigned)(2 * units * ceil_div(S, kTile));
     ProfileScope prof("attn_bwd_tc");
-    BOATCU_RUN(attn_bwd_dkv_tf32_kernel, grid, kBwd32Threads, C::SMEM_DKV, mq, mq_mn, mk, mv, mdo, mdo_mn, p);
-    BOATCU_LAUNCH_OK("attn_bwd_dkv_tf32");
-    BOATCU_RUN(attn_bwd_dq_tf32_kernel, grid, kBwd32Threads, C::SMEM_DQ, mq, mk, mk_mn, mv, mdo, p);
-    BOATCU_LAUNCH_OK("attn_bwd_dq_tf32");
+    BOATCU_RUN(attn_bwd_tf32_kernel, grid, kBwd32Threads, SMEM, m, p);
+    BOATCU_LAUNCH_OK("attn_bwd_tf32");
     return 0;
 }
 
