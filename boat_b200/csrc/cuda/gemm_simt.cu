@@ -15,7 +15,7 @@
 //
 // Before, with 4 x 4 outputs per thread: 1000 x 256 x 256 19.6 us, 4096 x 512 x 512 76 us (28 TFLOP/s),
 // 512 x 512 x 4096 (dW) 147 us; now 8.6,
-// 74 and 90 us.
+// 74 and 77 us.
 #include "common.cuh"
 #include <cooperative_groups.h>
 #include <type_traits>
@@ -371,12 +371,15 @@ int pick_tile(SimtParams& p, int groups) {
     auto tiles = [&](int bm, int bn) { return ceil_div(p.M, bm) * ceil_div(p.N, bn); };
     // The largest tile that still gives every SM one: larger ones fetch less per product, smaller ones
     // leave no SM idle.  Where even 64 x 32 does not fill the GPU, K is split over a cluster too, at
-    // least 64 of it per CTA.  The order of the sum goes by the size of one problem alone, so that a
+    // least 64 of it per CTA - and into two CTAs per SM where each still has 512: eight warps alone wait for
+    // one another's loads (512 x 512 x 4096 90 -> 77 us).  The order of the sum goes by the size of one problem alone, so that a
     // group gives the bits of single calls.
     if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value)
         if (tiles(128, 128) >= sms) return launch_tile<TI, TO, A_M, B_K, 2, 4>(p, groups, 1);
     if (tiles(64, 64) >= sms) return launch_tile<TI, TO, A_M, B_K, 1, 2>(p, groups, 1);
     int64_t split = sms / tiles(64, 32);
+    const int64_t two = 2 * sms / tiles(64, 32) < p.K / 512 ? 2 * sms / tiles(64, 32) : p.K / 512;
+    if (split < two) split = two;
     if (split > p.K / 64) split = p.K / 64;
     if (split > kMaxSplit) split = kMaxSplit;
     if (split < 1) split = 1;
