@@ -434,6 +434,7 @@ struct Problem {
     bool add;            // add to C instead of overwriting it (FP32)
     bool chain;          // one result: the sum of the groups' products
     void* aux;           // second result or operand of the epilogue, laid out like C
+    int results() const { return chain ? 1 : groups; }           // entries of C
 };
 
 // A tile shape and what it costs, measured on B200 with every shape forced on outputs of 128 x 1024 to
@@ -458,7 +459,7 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
     const double block_us = sh.block_us[slow];
     const int64_t workers = sm_count() / sh.ctas, k_blocks = ceil_div(q.K, bk) * (q.chain ? q.groups : 1);
     Plan r;
-    r.tiles = ceil_div(q.M, BM * sh.ctas) * ceil_div(q.N, sh.bn) * (q.chain ? 1 : q.groups);
+    r.tiles = ceil_div(q.M, BM * sh.ctas) * ceil_div(q.N, sh.bn) * q.results();
     r.full = r.tiles;
     r.split = 1;
     r.us = (double)ceil_div(r.tiles, workers) * (double)k_blocks * block_us + sh.once_us;
@@ -469,7 +470,7 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
     // microsecond, behind the next piece's main loop but for the last one; the output is cleared first.
     const int64_t rest = r.tiles % workers, whole = r.tiles / workers;
     const double out_us = BM * sh.bn * 4.0 / 36e3;
-    const double clear_us = q.add ? 0.0 : 2.0 + (double)q.M * (double)q.N * q.groups * 4.0 / 4e6;
+    const double clear_us = q.add ? 0.0 : 2.0 + (double)q.M * (double)q.N * q.results() * 4.0 / 4e6;
     int64_t most = k_blocks / 8;
     if (q.K < 2048) most = 1;
     if (most > 32) most = 32;
@@ -501,7 +502,7 @@ int launch(const Problem& q, const Plan& plan) {
         if (int rc = B_MN ? make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.ldb, C::BK, C::BK, C::ES == 4)
                           : make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.N, (uint64_t)q.K, (uint64_t)q.ldb, C::BNC, C::BK))
             return rc;
-        if (q.chain && g > 0) continue;
+        if (g >= q.results()) continue;
         if (int rc = make_tensor_map_2d(&maps.c[g], q.C[g], bf16_out ? 2 : 4, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, bf16_out ? 64 : 32))
             return rc;
         p.bias[g] = q.bias ? q.bias[g] : nullptr;
@@ -510,7 +511,7 @@ int launch(const Problem& q, const Plan& plan) {
         if (int rc = make_tensor_map_2d(&maps.aux, q.aux, 2, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, 64)) return rc;
     const int64_t full = plan.full, split = plan.split, tiles = plan.tiles, workers = sm_count() / CTAS;
     if (split > 1 && !q.add) {
-        for (int g = 0; g < q.groups; ++g) {
+        for (int g = 0; g < q.results(); ++g) {
             if (q.ldc == q.N) {
                 BOATCU_CHECK(cudaMemsetAsync(q.C[g], 0, (size_t)q.M * q.N * sizeof(float), stream()));
             } else {

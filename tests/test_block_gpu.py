@@ -225,3 +225,33 @@ def test_pre_ln_encoder_block_training_step(gpu_lib, bf16, B, S, d, nh, tol):
         bound.update(out=2.5e-2, dx=tol, dwq=4e-2)
     bad = {k: v for k, v in worst.items() if v > bound[k]}
     assert not bad, (bad, worst)
+
+
+def test_block_of_fp32_tensors_equals_separate_layer_calls(gpu_lib):
+    """The block sums the three input gradients of its attention layer in one product, from d_model 2048 on with K in
+    pieces; the layers called one by one give three gradients.  FP32 tensors, TF32 arithmetic in the attention layer.
+    The forward is the same operations.  The gradients ahead of the attention layer differ in the last bits (the residual
+    is added inside a pass or after it), so each of the four TF32 roundings between there and dx (of dr1, d(ctx), dS and
+    dQ/dK/dV) may go the other way: 4 * 2^-11 of the largest value."""
+    B, S, d, nh, dev = 1, 128, 2048, 32, capi.DEVICE_CUDA
+    inp = block_inputs(B, S, d, False)
+    blk = host.EncoderBlock(d, nh, causal=True, device=dev, mma=capi.MMA_TF32, params=inp)
+    x, t = Tensor.from_numpy(inp["x"], dev), Tensor.from_numpy(inp["target"], dev)
+    out, dx = blk.step(x, t)
+    want_out, want_dx = out.numpy(), dx.numpy()
+    blk.zero_dense_grads()
+    h1 = blk.ln1.forward(x)
+    r1 = host.lincomb(x, 1.0, blk.attn.forward(h1), 1.0)
+    h2 = host.reshape(blk.ln2.forward(r1), (B * S, d))
+    u = blk.fc1.forward(h2)
+    a = Tensor(gpu_lib.boat_gelu(u.h))
+    y = host.lincomb(r1, 1.0, host.reshape(blk.fc2.forward(a), (B, S, d)), 1.0)
+    g = host.lincomb(y, 2.0 / (B * S * d), t, -2.0 / (B * S * d))
+    du = Tensor(gpu_lib.boat_gelu_backward(blk.fc2.backward(host.reshape(g, (B * S, d))).h, u.h))
+    dr1 = host.lincomb(g, 1.0, blk.ln2.backward(host.reshape(blk.fc1.backward(du), (B, S, d))), 1.0)
+    gq, gk, gv = blk.attn.backward(dr1)
+    dh1 = host.lincomb(host.lincomb(gq, 1.0, gk, 1.0), 1.0, gv, 1.0)
+    got_dx = host.lincomb(dr1, 1.0, blk.ln1.backward(dh1), 1.0).numpy()
+    assert rel(y.numpy(), want_out) <= 1e-5
+    assert rel(got_dx, want_dx) <= 4 * 2.0 ** -11
+    blk.free()

@@ -70,6 +70,23 @@ def test_gemm_sum_of_products(gpu_lib, shape, groups):
                                       capi.CUDA_F32) == 13
 
 
+# FP32 results of few tiles and a long K are cut along K and added into a cleared output: the one output there is, and
+# of it the rows of the result alone.  The inputs are BF16 values, exact in either arithmetic.
+@pytest.mark.parametrize("mma", [capi.MMA_BF16, capi.MMA_TF32], ids=["bf16", "tf32"])
+@pytest.mark.parametrize("M,N,K,pad", [(128, 2048, 2048, 0), (333, 192, 2048, 64), (200, 256, 3072, 0)])
+def test_gemm_sum_of_products_with_split_k(gpu_lib, mma, M, N, K, pad):
+    bf, groups, ldc = mma == capi.MMA_BF16, 3, N + pad
+    a, b = [_bf(2, g, (M, K)) for g in range(groups)], [_bf(3, g, (N, K), 1 / math.sqrt(K)) for g in range(groups)]
+    da, db = [DeviceBuffer.from_numpy(t, bf16=bf) for t in a], [DeviceBuffer.from_numpy(t, bf16=bf) for t in b]
+    dc = DeviceBuffer.from_numpy(np.full((M, ldc), np.nan, np.float32))
+    check(gpu_lib.boat_cuda_gemm_sum(mma, 0, 1, groups, M, N, K, _table(da), K, _table(db), K, capi.CUDA_BF16 if bf else capi.CUDA_F32,
+                                     dc.p, ldc, capi.CUDA_F32), "gemm_sum")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    got = dc.numpy((M, ldc))
+    assert rel(got[:, :N], sum(x.astype(np.float64) @ y.astype(np.float64).T for x, y in zip(a, b))) <= 1e-5
+    assert np.isnan(got[:, N:]).all()
+
+
 # one CTA's tiles of every width, a pair's, and the split of FP32 results with its remainders
 @pytest.mark.parametrize("shape", [(128, 64, 64), (129, 200, 64), (1300, 768, 200), (2300, 1100, 136), (4096, 2304, 64)])
 @pytest.mark.parametrize("layout", [(0, 0), (0, 1)], ids=["nn", "nt"])
