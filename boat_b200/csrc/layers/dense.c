@@ -20,11 +20,6 @@ struct boat_dense_layer_t {
     bool use_bias;
     boat_tensor_t *weight, *bias, *grad_weight, *grad_bias;
     boat_tensor_t* cache_input;
-    /* BF16 copy of a CUDA weight, made by a forward and used again by the backward that follows it; trusted
-     * only in between, and not after a call that hands out or changes the weight (as the attention
-     * layer's, see there). */
-    void* shadow;
-    bool shadow_fresh;
 };
 
 boat_dense_layer_t* boat_dense_layer_create(size_t input_features, size_t output_features, bool use_bias) {
@@ -56,27 +51,7 @@ void boat_dense_layer_free(boat_dense_layer_t* l) {
     boat_tensor_t* all[5] = {l->weight, l->bias, l->grad_weight, l->grad_bias, l->cache_input};
     for (int i = 0; i < 5; ++i)
         if (all[i]) boat_tensor_free(all[i]);
-    boat_dev_free(l->shadow);
     boat_free(l);
-}
-
-/* The weight as an operand of storage `type` (*owned as boat_stage_in). */
-static void* stage_weight(boat_dense_layer_t* l, int type, bool backward, bool* owned) {
-    const boat_tensor_t* w = l->weight;
-    *owned = false;
-    if (type != BOAT_CUDA_BF16 || w->device != BOAT_DEVICE_CUDA || w->dtype != BOAT_DTYPE_FLOAT32)
-        return boat_stage_in(w, type, owned);
-    if (!l->shadow) {
-        l->shadow = boat_dev_alloc(l->in_features * l->out_features * 2);
-        l->shadow_fresh = false;
-        if (!l->shadow) return NULL;
-    }
-    const bool fresh = backward && l->shadow_fresh;
-    l->shadow_fresh = false;
-    if (!fresh && boat_report("weight conversion", boat_cuda_cast(l->shadow, BOAT_CUDA_BF16, w->data, BOAT_CUDA_F32, (int64_t)w->nelements)) != 0)
-        return NULL;
-    l->shadow_fresh = !backward;
-    return l->shadow;
 }
 
 /* Forward with element-wise work behind the product (BOAT_EPI_*; fused.h): `aux` is the residual to add (ADD),
@@ -94,7 +69,7 @@ static boat_tensor_t* dense_forward(boat_dense_layer_t* l, const boat_tensor_t* 
     const int64_t oshape[2] = {N, O};
     bool xo = false, wo = false, bo = false;
     void* dx = boat_stage_in(input, type, &xo);
-    void* dw = stage_weight(l, type, false, &wo);
+    void* dw = boat_stage_in(l->weight, type, &wo);
     float* db = l->bias ? (float*)boat_stage_in(l->bias, BOAT_CUDA_F32, &bo) : NULL;
     void* dy = boat_dev_alloc((size_t)N * O * boat_storage_size(type));
     void* aux = epilogue == BOAT_EPI_GELU ? boat_dev_alloc((size_t)N * O * boat_storage_size(type))
@@ -152,7 +127,7 @@ static boat_tensor_t* dense_backward(boat_dense_layer_t* l, const boat_tensor_t*
     bool xo = false, go = false, wo = false;
     void* dx = boat_stage_in(x, type, &xo);
     void* dg = boat_stage_in(grad_output, type, &go);
-    void* dw = stage_weight(l, type, true, &wo);
+    void* dw = boat_stage_in(l->weight, type, &wo);      /* anew: the caller may have written it since the forward */
     void* d_dx = boat_dev_alloc((size_t)N * I * boat_storage_size(type));
     /* CUDA gradients are added to where they lie; others take a trip through HBM */
     boat_tensor_t* grads[2] = {l->grad_weight, l->grad_bias};
@@ -198,7 +173,6 @@ boat_tensor_t* boat_dense_backward_gelu(boat_dense_layer_t* l, const boat_tensor
 
 BOAT_NOINLINE void boat_dense_layer_update(boat_dense_layer_t* l, float learning_rate) {
     if (!l) return;
-    l->shadow_fresh = false;
     boat_tensor_t* pairs[2][2] = {{l->weight, l->grad_weight}, {l->bias, l->grad_bias}};
     float *w_cuda[2], *g_cuda[2];
     int64_t n_cuda[2];
@@ -239,7 +213,7 @@ static void replace(boat_tensor_t** slot, boat_tensor_t* t) {
 void boat_dense_layer_set_weight(boat_dense_layer_t* l, boat_tensor_t* weight) {
     if (l && weight && weight->ndim == 2 && weight->shape[0] == (int64_t)l->in_features &&
         weight->shape[1] == (int64_t)l->out_features)
-        replace(&l->weight, weight), l->shadow_fresh = false;
+        replace(&l->weight, weight);
 }
 
 void boat_dense_layer_set_bias(boat_dense_layer_t* l, boat_tensor_t* bias) {
@@ -249,20 +223,13 @@ void boat_dense_layer_set_bias(boat_dense_layer_t* l, boat_tensor_t* bias) {
     }
 }
 
-boat_tensor_t* boat_dense_layer_get_weight(const boat_dense_layer_t* l) {
-    if (!l) return NULL;
-    ((boat_dense_layer_t*)l)->shadow_fresh = false;             /* the caller may write through it */
-    return l->weight;
-}
+boat_tensor_t* boat_dense_layer_get_weight(const boat_dense_layer_t* l) { return l ? l->weight : NULL; }
 boat_tensor_t* boat_dense_layer_get_bias(const boat_dense_layer_t* l) { return l ? l->bias : NULL; }
 boat_tensor_t* boat_dense_layer_get_grad_weight(const boat_dense_layer_t* l) { return l ? l->grad_weight : NULL; }
 boat_tensor_t* boat_dense_layer_get_grad_bias(const boat_dense_layer_t* l) { return l ? l->grad_bias : NULL; }
 
 int boat_dense_layer_to_device(boat_dense_layer_t* l, boat_device_t device) {
     if (!l) return 1;
-    boat_dev_free(l->shadow);
-    l->shadow = NULL;
-    l->shadow_fresh = false;
     boat_tensor_t** slots[4] = {&l->weight, &l->bias, &l->grad_weight, &l->grad_bias};
     for (int i = 0; i < 4; ++i) {
         boat_tensor_t* t = *slots[i];

@@ -139,6 +139,20 @@ def test_dense_layer_bf16_tensor_cores(gpu_lib):
     layer.free()
 
 
+def test_dense_backward_sees_a_weight_written_after_the_forward(gpu_lib):
+    """Through a weight tensor fetched before the forward, so that no call tells the layer of the change."""
+    N, I, O, dev = 256, 128, 192, capi.DEVICE_CUDA
+    x, g = rng.bf16_round(rng.normal(15, 0, (N, I))), rng.bf16_round(rng.normal(15, 1, (N, O)))
+    w = [rng.bf16_round(rng.normal(15, 2 + i, (I, O), 1 / 16.0)) for i in range(2)]
+    layer = Dense(gpu_lib, I, O, w[0], None, dev)
+    held = Tensor(gpu_lib.boat_dense_layer_get_weight(layer.h), own=False)
+    layer.forward(Tensor.from_numpy(x, dev, bf16=True))
+    held.set(w[1])
+    dx = layer.backward(Tensor.from_numpy(g, dev, bf16=True)).numpy()
+    assert rel(dx, g.astype(np.float64) @ w[1].astype(np.float64).T) <= TOL_BF16
+    layer.free()
+
+
 @pytest.mark.parametrize("bf16", [False, True], ids=["fp32", "bf16"])
 def test_gelu_forward_and_backward(gpu_lib, bf16):
     f = rng.bf16_round if bf16 else (lambda a: a)
