@@ -1,10 +1,11 @@
 // dispatch.cu - the extern "C" contraction and attention-core entry points: argument checks
 // and the choice between the tcgen05 kernels and the CUDA-core kernels.  The choice is by
-// shape only: a TF32 or BF16 request whose shape the tensor-core kernels do not cover
-// (head size other than 64 / 128, tiny or unaligned GEMMs)
+// shape and alignment only: a TF32 or BF16 request whose shape the tensor-core kernels do not cover
+// (head size other than 64 / 128, tiny or unaligned GEMMs, attention tensors that do not start on 16 bytes)
 // runs on the CUDA cores with the same storage types and FP32 FMA arithmetic - at least as
 // accurate as what was asked for, never less.
 #include "common.cuh"
+#include <initializer_list>
 
 using namespace boatcu;
 
@@ -16,6 +17,13 @@ size_t attn_bwd_tc_scratch_bytes(int mma, int64_t units, int64_t S, int64_t hs);
 int attn_bwd_tc(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,
                 const void* K, const void* V, const void* O, const void* dO, const float* lse, const float* delta,
                 int io_type, void* dQ, void* dK, void* dV, void* scratch, size_t scratch_bytes);
+}
+
+// The tensor-core attention kernels load tiles by TMA and store rows 16 bytes at a time.
+static bool aligned16(std::initializer_list<const void*> tensors) {
+    uintptr_t bits = 0;
+    for (const void* t : tensors) bits |= (uintptr_t)t;
+    return (bits & 15) == 0;
 }
 
 static int check_types(const char* who, int mma, int in_type) {
@@ -143,7 +151,7 @@ int boat_cuda_attn_fwd(int mma, int64_t units, int64_t S, int64_t hs, int causal
     if (units < 0 || S < 0 || hs < 0) return set_error(11, "boat_cuda_attn_fwd: negative size");
     if (units == 0 || S == 0 || hs == 0) return 0;
     if (!Q || !K || !V || !O || !lse) return set_error(11, "boat_cuda_attn_fwd: NULL operand");
-    if (mma != BOAT_MMA_FP32 && attn_tc_supported(mma, units, S, hs, io_type))
+    if (mma != BOAT_MMA_FP32 && aligned16({Q, K, V, O}) && attn_tc_supported(mma, units, S, hs, io_type))
         return attn_fwd_tc(mma, units, S, hs, causal, scale, Q, K, V, io_type, O, lse);
     {
         ProfileScope prof("attn_fwd_simt");
@@ -187,7 +195,7 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
     if (((uintptr_t)scratch & 255) != 0) return set_error(12, "boat_cuda_attn_bwd: scratch must be 256-byte aligned");
     float* delta = (float*)scratch;
     size_t delta_bytes = ((size_t)units * (size_t)S * sizeof(float) + 255) & ~(size_t)255;
-    tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && ((uintptr_t)O & 15) == 0 && attn_tc_supported(mma, units, S, hs, io_type);
+    tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && aligned16({Q, K, V, O, dO, dQ, dK, dV}) && attn_tc_supported(mma, units, S, hs, io_type);
     if (!(tensor_cores && mma == BOAT_MMA_BF16)) {      // the BF16 kernel's launcher makes its own, pre-scaled
         ProfileScope prof("attn_delta");
         if (int rc = rowdot(dO, O, io_type, units * S, hs, delta)) return rc;

@@ -202,6 +202,47 @@ def test_attention_core_on_partly_filled_tiles(gpu_lib, mma, hs, S, causal):
     assert np.abs(got["lse"] - ref["lse"]).max() <= 2e-2
 
 
+class _Shifted:
+    """A device array that starts one element (or none) behind an aligned address."""
+
+    def __init__(self, lib, shape, bf, shift, values=None):
+        self.lib, self.shape, self.bf = lib, shape, bf
+        self.nbytes = int(np.prod(shape)) * (2 if bf else 4)
+        self.buf = DeviceBuffer(self.nbytes + 16)
+        self.p = C.c_void_p(self.buf.p.value + shift * (2 if bf else 4))
+        if values is not None:
+            payload = rng.to_bf16_bits(values) if bf else np.ascontiguousarray(values, np.float32)
+            check(lib.boat_cuda_memcpy_h2d(self.p, payload.ctypes.data_as(C.c_void_p), self.nbytes))
+
+    def numpy(self):
+        raw = np.empty(self.shape, np.uint16 if self.bf else np.float32)
+        check(self.lib.boat_cuda_memcpy_d2h(raw.ctypes.data_as(C.c_void_p), self.p, self.nbytes))
+        return rng.from_bf16_bits(raw).reshape(self.shape) if self.bf else raw
+
+
+@pytest.mark.parametrize("mma,hs", [(capi.MMA_BF16, 64), (capi.MMA_BF16, 128), (capi.MMA_TF32, 64)],
+                         ids=["bf16_hs64", "bf16_hs128", "tf32_hs64"])
+@pytest.mark.parametrize("S", [200, 256], ids=["ragged", "whole_tiles"])
+@pytest.mark.parametrize("which", ["all", "q", "k", "v", "o", "do", "dq", "dk", "dv"])
+def test_attention_core_with_arrays_off_alignment(gpu_lib, mma, hs, S, which):
+    """Arrays that do not start on 16 bytes are for the CUDA cores, whichever of them it is."""
+    lib, bf, units = gpu_lib, mma == capi.MMA_BF16, 3
+    io, f, shape = capi.CUDA_BF16 if bf else capi.CUDA_F32, rng.bf16_round if bf else (lambda a: a), (units, S, hs)
+    q, k, v, go = (f(rng.normal(7, i, shape)) for i in range(4))
+    scale = 1.0 / np.sqrt(hs)
+    d = {n: _Shifted(lib, shape, bf, int(which in ("all", n)), val)
+         for n, val in dict(q=q, k=k, v=v, do=go, o=None, dq=None, dk=None, dv=None).items()}
+    lse = DeviceBuffer(units * S * 4)
+    check(lib.boat_cuda_attn_fwd(mma, units, S, hs, 1, C.c_float(scale), d["q"].p, d["k"].p, d["v"].p, io, d["o"].p, lse.p), "attn_fwd")
+    scratch = DeviceBuffer(max(lib.boat_cuda_attn_bwd_scratch_bytes(mma, units, S, hs), 256))
+    check(lib.boat_cuda_attn_bwd(mma, units, S, hs, 1, C.c_float(scale), d["q"].p, d["k"].p, d["v"].p, d["o"].p, d["do"].p, lse.p, io,
+                                 d["dq"].p, d["dk"].p, d["dv"].p, scratch.p, scratch.nbytes), "attn_bwd")
+    check(lib.boat_cuda_sync(), "sync")
+    ref = np_core(q, k, v, go, True, scale)
+    for key in ("o", "dq", "dk", "dv"):
+        assert rel(d[key].numpy(), ref[key]) <= TOL[mma], key
+
+
 def test_attention_core_large_scores_do_not_overflow(gpu_lib):
     """Rows whose running max keeps growing exercise the rescale of the accumulator."""
     lib = gpu_lib
