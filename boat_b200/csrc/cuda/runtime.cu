@@ -3,11 +3,11 @@
 // (src/core/memory.c:174-186 allocate_device/free_device and :230-247 copy/set, which were
 // malloc/memcpy/memset regardless of the device argument).
 #include "tc_common.cuh"
+#include "block_cache.h"
 #include <stdarg.h>
 #include <stdlib.h>
 #include <string.h>
 #include <atomic>
-#include <list>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
@@ -23,11 +23,6 @@ static int g_device = -1;                       // the one device this process's
 static int g_sm_count = 0;
 static cudaStream_t g_stream = 0;
 static std::atomic<uint64_t> g_launches{0};
-struct LiveBlock {
-    size_t bytes, block;                        // asked for, handed out
-};
-static std::unordered_map<void*, LiveBlock>* g_live = nullptr;
-static size_t g_live_bytes = 0;
 static unsigned int* g_status_host = nullptr;   // kernel status word, host view
 static unsigned int* g_status_dev = nullptr;    // the same word as kernels see it
 
@@ -76,12 +71,11 @@ static int init_locked(int device) {
         return set_error(3, "device %d is sm_%d%d; this library contains sm_100a code only",
                          dev, prop.major, prop.minor);
     }
-    // What leaves the block cache below stays in the driver's pool rather than being unmapped.
+    // What the block cache below gives back stays in the driver's pool rather than being unmapped.
     cudaMemPool_t pool;
     BOATCU_CHECK(cudaDeviceGetDefaultMemPool(&pool, dev));
     uint64_t keep = UINT64_MAX;
     BOATCU_CHECK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-    if (!g_live) g_live = new std::unordered_map<void*, LiveBlock>();
     BOATCU_CHECK(cudaHostAlloc((void**)&g_status_host, sizeof(unsigned int), cudaHostAllocMapped));
     *g_status_host = 0;
     BOATCU_CHECK(cudaHostGetDevicePointer((void**)&g_status_dev, g_status_host, 0));
@@ -201,23 +195,37 @@ int ensure_init() {
 using namespace boatcu;
 
 // ---- device memory ---------------------------------------------------------------------------
-// A step allocates and frees the same two dozen buffers every time.  Freed blocks are kept by size
-// and handed out again to the next request they fit (within an eighth), instead of a round trip
-// through the driver's pool for each: that round trip costs 1-4 us of host time, which small
-// steps are bound by, and now and then milliseconds when the pool has to remap memory (a step
-// of B16 S2048 d1024 took 1.9 ms of kernels and 1.9-2.7 ms in all).  Everything the library launches
-// is ordered on one stream, so a block freed there may be written by whatever is launched next.
-// Bounded by BOAT_DEVICE_CACHE_MB (default 8192): the longest unused blocks go back to the driver
-// when more than that lies idle; all of them when the stream changes or an allocation fails.
-struct CachedBlock;
-typedef std::multimap<size_t, CachedBlock> BlockCache;
-struct CachedBlock {
-    void* ptr;
-    std::list<BlockCache::iterator>::iterator age;
+// A step allocates and frees the same two dozen buffers every time.  Freed blocks are kept (block_cache.h) and
+// handed out again without the driver's pool, whose calls take 0.3 to 3 us of host time, which small steps are
+// bound by, and now and then milliseconds when it has to remap memory (a step of B16 S2048 d1024 took
+// 1.9 ms of kernels and 1.9-2.7 ms in all).  Everything the library launches is ordered on one
+// stream, so a block freed there may be written by whatever is launched next.  Bounded by BOAT_DEVICE_CACHE_MB
+// (default 8192; 0 keeps nothing): the longest unused memory goes back to the driver when more than that
+// lies idle, all of it when an allocation fails.
+//
+// Straight from and to the driver's pool, in the order of the stream: blocks allocated while the stream is being
+// captured, which belong to the graph, and all blocks on the per-thread default stream, which is a
+// different stream for every thread.
+class DriverPool : public BlockCache::Source {
+public:
+    cudaError_t error = cudaSuccess;              // of the last call that failed
+    void* take(size_t bytes) override {
+        void* p = nullptr;
+        const cudaError_t err = cudaMallocAsync(&p, bytes, g_stream);
+        if (err == cudaSuccess) return p;
+        cudaGetLastError();
+        error = err;
+        return nullptr;
+    }
+    void give(void* slab) override { note(cudaFreeAsync(slab, g_stream)); }
+    bool wait() override { return note(cudaDeviceSynchronize()); }
+
+private:
+    bool note(cudaError_t err) {
+        if (err != cudaSuccess) error = err;
+        return err == cudaSuccess;
+    }
 };
-static BlockCache* g_cache = new BlockCache();                                        // idle blocks by size
-static std::list<BlockCache::iterator>* g_cache_age = new std::list<BlockCache::iterator>();    // oldest first
-static size_t g_cache_bytes = 0;
 
 static size_t cache_cap() {
     static const size_t cap = [] {
@@ -228,17 +236,17 @@ static size_t cache_cap() {
     return cap;
 }
 
-// Gives the oldest idle blocks back until at most `limit` bytes are left (g_mu held).
-static int trim_cache(size_t limit) {
-    while (g_cache_bytes > limit) {
-        const auto it = g_cache_age->front();
-        void* p = it->second.ptr;
-        g_cache_bytes -= it->first;
-        g_cache_age->pop_front();
-        g_cache->erase(it);
-        BOATCU_CHECK(cudaFreeAsync(p, g_stream));
-    }
-    return 0;
+static DriverPool* g_pool = new DriverPool();
+static BlockCache* g_cache = nullptr;             // made by the first allocation
+static std::unordered_map<void*, size_t>* g_direct = new std::unordered_map<void*, size_t>();      // blocks beside the cache
+static size_t g_direct_bytes = 0;
+static uint64_t g_stream_id = 0;                  // of the library stream; 0: the legacy default stream
+static bool g_stream_cached = true;               // blocks of this stream go through the cache
+
+static bool capturing() {
+    if (g_stream == 0) return false;              // the legacy default stream cannot be captured
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(g_stream, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
 }
 
 extern "C" {
@@ -265,12 +273,16 @@ const char* boat_cuda_last_error(void) { return g_err; }
 void* boat_cuda_stream(void) { return (void*)g_stream; }
 
 int boat_cuda_set_stream(void* s) {
-    if ((cudaStream_t)s != g_stream && g_ready) {
-        // cached blocks are ordered behind the old stream only: hand them back to the driver on it
-        std::lock_guard<std::mutex> lk(g_mu);
-        trim_cache(0);
-    }
+    std::lock_guard<std::mutex> lk(g_mu);
+    // The old stream may be gone already: nothing is asked of it.
     g_stream = (cudaStream_t)s;
+    unsigned long long id = 0;
+    g_stream_cached = g_stream != cudaStreamPerThread;
+    if (g_stream != 0 && g_stream_cached && cudaStreamGetId(g_stream, &id) != cudaSuccess) {
+        cudaGetLastError();
+        g_stream_cached = false;
+    }
+    g_stream_id = id;
     return 0;
 }
 
@@ -347,48 +359,50 @@ int boat_cuda_malloc(void** ptr, size_t bytes) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
     std::lock_guard<std::mutex> lk(g_mu);
-    const size_t want = (bytes + 511) & ~(size_t)511;
-    size_t block = want;
-    auto it = g_cache->lower_bound(want);
-    if (it != g_cache->end() && it->first <= want + want / 8) {
-        block = it->first;
-        *ptr = it->second.ptr;
-        g_cache_age->erase(it->second.age);
-        g_cache->erase(it);
-        g_cache_bytes -= block;
-    } else {
-        cudaError_t err = cudaMallocAsync(ptr, block, g_stream);
-        if (err == cudaErrorMemoryAllocation && g_cache_bytes > 0) {
-            // what the cache holds may be what is missing; the driver's pool takes it back in stream order
-            cudaGetLastError();
-            trim_cache(0);
-            err = cudaMallocAsync(ptr, block, g_stream);
+    try {
+        if (cache_cap() > 0 && g_stream_cached && !capturing()) {
+            if (!g_cache) g_cache = new BlockCache(*g_pool, cache_cap());
+            *ptr = g_cache->get(bytes, g_stream_id);
+        } else if ((*ptr = g_pool->take(bytes)) != nullptr) {
+            (*g_direct)[*ptr] = bytes;
+            g_direct_bytes += bytes;
         }
-        BOATCU_CHECK(err);
+    } catch (const std::bad_alloc&) {
+        *ptr = nullptr;
+        return set_error(4, "boat_cuda_malloc: out of host memory");
     }
-    (*g_live)[*ptr] = LiveBlock{bytes, block};
-    g_live_bytes += bytes;
+    if (!*ptr)
+        return set_error(1000 + (int)g_pool->error, "boat_cuda_malloc: %zu bytes of device memory: %s", bytes, cudaGetErrorString(g_pool->error));
     return 0;
 }
 
 int boat_cuda_free(void* ptr) {
     if (!ptr) return 0;
     if (int rc = ensure_init()) return rc;
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        auto it = g_live->find(ptr);
-        if (it == g_live->end()) return set_error(5, "boat_cuda_free: %p was not allocated here", ptr);
-        g_live_bytes -= it->second.bytes;
-        const size_t block = it->second.block;
-        g_live->erase(it);
-        const auto entry = g_cache->insert({block, CachedBlock{ptr, {}}});
-        entry->second.age = g_cache_age->insert(g_cache_age->end(), entry);
-        g_cache_bytes += block;
-        return trim_cache(cache_cap());
+    std::lock_guard<std::mutex> lk(g_mu);
+    const auto direct = g_direct->find(ptr);
+    if (direct != g_direct->end()) {
+        g_direct_bytes -= direct->second;
+        g_direct->erase(direct);
+        BOATCU_CHECK(cudaFreeAsync(ptr, g_stream));
+        return 0;
     }
+    if (!g_cache || !g_cache->owns(ptr)) return set_error(5, "boat_cuda_free: %p was not allocated here", ptr);
+    if (capturing()) return set_error(7, "boat_cuda_free: %p was allocated outside the stream capture that is under way", ptr);
+    g_pool->error = cudaSuccess;
+    try {
+        g_cache->put(ptr, g_stream_id);
+    } catch (const std::bad_alloc&) {
+        return set_error(5, "boat_cuda_free: out of host memory");
+    }
+    BOATCU_CHECK(g_pool->error);
+    return 0;
 }
 
-size_t boat_cuda_bytes_in_use(void) { return g_live_bytes; }
+size_t boat_cuda_bytes_in_use(void) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    return g_direct_bytes + (g_cache ? g_cache->used_bytes() : 0);
+}
 uint64_t boat_cuda_launch_count(void) { return g_launches.load(); }
 
 int boat_cuda_memcpy_h2d(void* dst, const void* src, size_t bytes) {

@@ -44,7 +44,7 @@ int         boat_cuda_init(int device);          /* idempotent; device < 0: env 
 int         boat_cuda_device_count(void);        /* 0 when no usable GPU / driver */
 const char* boat_cuda_last_error(void);
 void*       boat_cuda_stream(void);              /* cudaStream_t the library launches on */
-int         boat_cuda_set_stream(void* stream);
+int         boat_cuda_set_stream(void* stream);   /* the caller orders the new stream behind the old one's work */
 int         boat_cuda_sync(void);                /* wait for the library stream and the copy streams */
 int         boat_cuda_malloc(void** ptr, size_t bytes);   /* stream-ordered pool allocation */
 int         boat_cuda_free(void* ptr);
