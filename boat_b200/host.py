@@ -384,6 +384,12 @@ class LayerNorm:
             capi.load().boat_layernorm_free(self.h)
         self.h = None
 
+    def __del__(self):
+        try:
+            self.free()
+        except Exception:
+            pass
+
 
 class Dense:
     """boat_dense_layer_t (include/boat/layers.h)."""
@@ -419,6 +425,12 @@ class Dense:
         if self.h:
             capi.load().boat_dense_layer_free(self.h)
         self.h = None
+
+    def __del__(self):
+        try:
+            self.free()
+        except Exception:
+            pass
 
 
 def reshape(t, shape):
@@ -484,3 +496,10 @@ class EncoderBlock:
             self.h = None
         for layer in (self.ln1, self.ln2, self.fc1, self.fc2, self.attn):
             layer.free()
+
+    def __del__(self):
+        try:
+            if self.h is not None:                   # the layers go with their own last reference
+                capi.load().boat_encoder_block_free(self.h)
+        except Exception:
+            pass

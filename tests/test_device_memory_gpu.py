@@ -1,12 +1,13 @@
 """Device memory across layers, sequence lengths and streams: what one use leaves serves the next."""
 import ctypes as C
+import gc
 
 import numpy as np
 import pytest
 import torch
 
 from boat_b200 import capi, rng
-from boat_b200.host import Attention, DeviceBuffer, Tensor, check
+from boat_b200.host import Attention, DeviceBuffer, EncoderBlock, Tensor, check
 
 pytestmark = pytest.mark.gpu
 
@@ -14,6 +15,30 @@ pytestmark = pytest.mark.gpu
 def free_bytes(lib):
     check(lib.boat_cuda_sync(), "sync")
     return torch.cuda.mem_get_info()[0]
+
+
+def test_new_blocks_live_on_what_the_last_one_left(gpu_lib):
+    """Twenty encoder blocks, one after another, each created, stepped and dropped."""
+    B, S, d, nh, dev = 4, 384, 512, 8, capi.DEVICE_CUDA
+    x, t = (Tensor.from_numpy(rng.normal(31, i, (B, S, d)), dev, bf16=True) for i in range(2))
+    used, free, ref = [], [], None
+    for i in range(20):
+        block = EncoderBlock(d, nh)
+        for j, layer in enumerate((block.fc1, block.fc2)):
+            w = Tensor(gpu_lib.boat_dense_layer_get_weight(layer.h), own=False)
+            w.set(rng.normal(32, j, w.shape, 0.02))
+        for n in Attention.PARAMS[:4]:
+            block.attn.param(n).set(rng.normal(33, ord(n[-1]), (d, d), 0.02))
+        out, dx = block.step(x, t)
+        got = out.numpy()
+        ref = got if ref is None else ref
+        assert np.array_equal(got, ref)
+        del block, out, dx, w
+        gc.collect()
+        used.append(gpu_lib.boat_cuda_bytes_in_use())
+        free.append(free_bytes(gpu_lib))
+    assert len(set(used)) == 1
+    assert len(set(free[1:])) == 1
 
 
 def test_steps_of_changing_lengths_settle(gpu_lib):
