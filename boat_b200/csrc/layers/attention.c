@@ -652,8 +652,9 @@ static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* que
     if (!pipelined) {
         const boat_tensor_t* t[3 + NPARAM] = {query, key, value};
         for (int i = 0; i < NPARAM; ++i) t[3 + i] = a->param[i];
-        if (!boat_bundle_send(&bundle, t, 3 + NPARAM)) goto done;
-        a->d_bundle = bundle.dev;
+        const bool sent = boat_bundle_send(&bundle, t, 3 + NPARAM);
+        a->d_bundle = bundle.dev;               /* released with the forward's state, also when the send failed */
+        if (!sent) goto done;
     }
     /* a host layer's parameters of a chunked call are brought up inside it, behind the first chunk */
     if (!(pipelined && a->device != BOAT_DEVICE_CUDA && prepare_late_params(a, mma, type, true, &p)) &&
