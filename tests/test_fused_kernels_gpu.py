@@ -22,13 +22,15 @@ def _bf(seed, stream, shape, scale=1.0):
     return rng.bf16_round(rng.normal(seed, stream, shape) * np.float32(scale))
 
 
+_erf = np.vectorize(math.erf, otypes=[np.float64])
+
+
 def _gelu(x):
-    return 0.5 * x * (1 + np.tanh(math.sqrt(2 / math.pi) * (x + 0.044715 * x ** 3)))
+    return 0.5 * x * (1 + _erf(x / math.sqrt(2)))
 
 
 def _gelu_grad(x):
-    t = np.tanh(math.sqrt(2 / math.pi) * (x + 0.044715 * x ** 3))
-    return 0.5 * (1 + t) + 0.5 * x * (1 - t * t) * math.sqrt(2 / math.pi) * (1 + 3 * 0.044715 * x * x)
+    return 0.5 * (1 + _erf(x / math.sqrt(2))) + x * np.exp(-0.5 * x * x) / math.sqrt(2 * math.pi)
 
 
 # one tile, ragged rows and columns, K tails, many tiles; the last two are not for the tensor cores
@@ -46,13 +48,21 @@ def test_gemm_epilogues(gpu_lib, shape, epilogue):
                                        dc.p, N, dbias.p if dbias else None, daux.p), "gemm_fused")
     check(gpu_lib.boat_cuda_sync(), "sync")
     z = a.astype(np.float64) @ (b.T if tb else b).astype(np.float64) + (0 if bias is None else bias)
-    got = dc.numpy((M, N), bf16=True)
+    got = dc.numpy((M, N), bf16=True).astype(np.float64)
+    if epilogue == 3:
+        assert rel(got, z + aux) <= 5e-3
+        return
+    # Element by element: one BF16 rounding (half of 2^-7), two where separate passes store the product in between (the
+    # shapes that are not for the tensor cores), FP32 sums (1e-5 of the largest), 3e-7 of the erf formula.  The tanh
+    # approximation of GELU, off by 2 % at -2.5, fails this.
     if epilogue == 1:
-        assert rel(daux.numpy((M, N), bf16=True), z) <= 3e-3
-        z = _gelu(z)
+        kept = daux.numpy((M, N), bf16=True).astype(np.float64)
+        assert rel(kept, z) <= 3e-3
+        want, slack = _gelu(kept), 3e-7 * np.abs(kept)
     else:
-        z = z * _gelu_grad(aux.astype(np.float64)) if epilogue == 2 else z + aux
-    assert rel(got, z) <= 5e-3
+        want, slack = z * _gelu_grad(aux.astype(np.float64)), 1e-5 * np.abs(z).max()
+    roundings = 2 if epilogue == 2 and (M < 128 or N % 8) else 1
+    assert (np.abs(got - want) <= roundings * 1.01 * 2.0 ** -8 * np.abs(want) + slack).all()
 
 
 @pytest.mark.parametrize("shape", [(128, 64, 64), (333, 768, 96), (2000, 320, 200)])
