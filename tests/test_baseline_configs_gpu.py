@@ -2,13 +2,13 @@
 
 The benchmark times sequence lengths, head sizes and unit counts far beyond the small parity
 cases: 64-tile walks, more (batch, head) units than the backward schedules together (several
-CTA groups, the last one short), both walk-pairing schedules, FP32 dQ sums of hundreds of MB.
+CTA groups, the last one short), FP32 dQ sums of hundreds of MB.
 These tests run exactly those shapes - as slices that the CPU restatement of the reference
 finishes in seconds - and compare with it per tensor:
 
   kernel ABI   boat_cuda_attn_fwd / _bwd on [units, S, hs] slices of configs 3, 4, 5 and of the
                target point (B=8, S=4096, head size 128), with more units than one CTA group
-               holds, under BOAT_BWD_PAIR=0 and 1
+               holds
   layer        boat_attention_forward / _backward for config 2 at full size (TF32) and for one
                batch entry of configs 3, 5 and (half the sequence) 4: out, dq, dk, dv, all dW, db
 
@@ -16,7 +16,6 @@ Tolerance: max|ours - ref| / max|ref| <= 2e-2 (BF16) / 5e-3 (TF32) per tensor; B
 BF16-rounded values to both sides.
 """
 import ctypes as C
-import os
 
 import numpy as np
 import pytest
@@ -45,7 +44,7 @@ _core_cache = {}
 
 def core_problem(name):
     """Seeded BF16-rounded q, k, v, dO of a slice and the restatement's o, dq, dk, dv (computed
-    once per process: both schedules are compared with the same reference)."""
+    once per process)."""
     if name not in _core_cache:
         units, S, hs, causal = CORE_SLICES[name]
         shape = (units, S, hs)
@@ -73,20 +72,11 @@ def run_core_bf16(lib, q, k, v, go, causal):
             "dv": gv.numpy(shape, bf16=True)}
 
 
-@pytest.mark.parametrize("pair", ["0", "1"], ids=["one_walk_per_cta", "two_walks_per_cta"])
 @pytest.mark.parametrize("name", list(CORE_SLICES))
-def test_attention_core_slice_of_benchmarked_config(gpu_lib, name, pair):
+def test_attention_core_slice_of_benchmarked_config(gpu_lib, name):
     q, k, v, go, ref = core_problem(name)
     causal = CORE_SLICES[name][3]
-    old = os.environ.get("BOAT_BWD_PAIR")
-    os.environ["BOAT_BWD_PAIR"] = pair
-    try:
-        got = run_core_bf16(gpu_lib, q, k, v, go, causal)
-    finally:
-        if old is None:
-            del os.environ["BOAT_BWD_PAIR"]
-        else:
-            os.environ["BOAT_BWD_PAIR"] = old
+    got = run_core_bf16(gpu_lib, q, k, v, go, causal)
     for key in ("o", "dq", "dk", "dv"):
         assert np.isfinite(got[key]).all(), (name, key)
         # every unit is held to the tolerance on its own scale: a wrong unit must not hide
@@ -108,21 +98,6 @@ def test_forward_unit_groups(gpu_lib, monkeypatch, group):
     for u in range(q.shape[0]):
         assert cases.rel_err(got["o"][u], ref["o"][u]) <= TOL_BF16, (group, u)
         assert cases.rel_err(got["dq"][u], ref["dq"][u]) <= TOL_BF16, (group, u)      # through the saved lse
-
-
-def test_schedule_default_matches_forced_choice(gpu_lib):
-    """Without BOAT_BWD_PAIR the launcher picks a schedule by problem size; whatever it picks
-    must give the numbers of that schedule when forced."""
-    name = "c3_S2048_hs64"
-    q, k, v, go, ref = core_problem(name)
-    old = os.environ.pop("BOAT_BWD_PAIR", None)
-    try:
-        got = run_core_bf16(gpu_lib, q, k, v, go, True)
-    finally:
-        if old is not None:
-            os.environ["BOAT_BWD_PAIR"] = old
-    for key in ("o", "dq", "dk", "dv"):
-        assert cases.rel_err(got[key], ref[key]) <= TOL_BF16, key
 
 
 def assert_step_close(res, ref, tol, what):

@@ -300,20 +300,18 @@ def test_profile_report_lists_kernel_families(gpu_lib):
     assert "gemm_tc_nn" in names and names["gemm_tc_nn"] > 0
 
 
-def test_backward_schedules_one_and_two_walks_per_cta():
-    """The tensor-core backward picks one or two key-tile walks per CTA from the problem size;
-    BOAT_BWD_PAIR forces either.  The attention-core and layer parity tests must pass under both
-    (sequence lengths of 1, 2, 3 and 8 tiles cover the unpaired middle tile and the causal pairing)."""
-    import os
-    import subprocess
-    import sys
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    for forced in ("0", "1"):
-        env = dict(os.environ, BOAT_BWD_PAIR=forced)
-        proc = subprocess.run([sys.executable, "-m", "pytest", "-x", "-q", "tests/test_kernels_gpu.py", "tests/test_parity_gpu.py",
-                               "-k", "attention_core or bf16_tensor_core or chunked"],
-                              cwd=root, env=env, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=900)
-        assert proc.returncode == 0, "BOAT_BWD_PAIR=%s:\n%s" % (forced, proc.stdout[-3000:])
+@pytest.mark.parametrize("hs,units,S", [(64, 700, 128), (64, 1100, 60), (64, 200, 385), (128, 300, 128), (128, 150, 300), (128, 70, 640)],
+                         ids=["one_tile", "part_of_a_tile", "ragged", "one_tile_hs128", "ragged_hs128", "five_tiles_hs128"])
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+def test_backward_walks_handed_over(gpu_lib, hs, units, S, causal):
+    """The BF16 backward starts a CTA per walk of a key tile and lets those on the SMs take over the others, a group of
+    units (64 MB of their data) after the other: more walks than SMs, walks of one tile, and numbers of units that
+    leave the last group short (512, 1092, 170, 256, 109 and 51 units make a group here)."""
+    got, ref = run_core(gpu_lib, capi.MMA_BF16, units, S, hs, causal)
+    for key in ("o", "dq", "dk", "dv"):
+        assert np.isfinite(got[key]).all(), key
+        for u in range(units):                        # each unit on its own scale
+            assert rel(got[key][u], ref[key][u]) <= TOL[capi.MMA_BF16], (key, u)
 
 
 # ---- several problems in one launch -------------------------------------------------------------
