@@ -8,6 +8,10 @@ int boat_storage_of(boat_dtype_t dt) { return dt == BOAT_DTYPE_BFLOAT16 ? BOAT_C
 size_t boat_storage_size(int type) { return type == BOAT_CUDA_BF16 ? 2 : 4; }
 bool boat_dtype_supported(boat_dtype_t dt) { return dt == BOAT_DTYPE_FLOAT32 || dt == BOAT_DTYPE_BFLOAT16; }
 
+bool boat_is_device_operand(const boat_tensor_t* t, int type, size_t n) {
+    return t->device == BOAT_DEVICE_CUDA && boat_dtype_supported(t->dtype) && boat_storage_of(t->dtype) == type && t->nelements == n;
+}
+
 void* boat_dev_alloc(size_t bytes) {
     void* p = NULL;
     if (boat_report("device allocation", boat_cuda_malloc(&p, bytes)) != 0) return NULL;

@@ -8,6 +8,9 @@
 int    boat_storage_of(boat_dtype_t dt);                 /* BOAT_CUDA_F32 / BOAT_CUDA_BF16 */
 size_t boat_storage_size(int type);
 bool   boat_dtype_supported(boat_dtype_t dt);            /* FLOAT32 or BFLOAT16 */
+/* Whether `t` is `n` elements of storage `type` in HBM: an operand that a kernel reads element by element beside
+ * another tensor of that size. */
+bool   boat_is_device_operand(const boat_tensor_t* t, int type, size_t n);
 void*  boat_dev_alloc(size_t bytes);                     /* NULL + message on failure */
 void   boat_dev_free(void* p);
 /* Device buffer with tensor `t` in storage `type`; *owned: caller must boat_dev_free it. */

@@ -760,6 +760,7 @@ static boat_tensor_t* forward_batch(boat_attention_t* a, const boat_tensor_t* qu
             in[i]->shape[2] != H)
             return NULL;
     }
+    if (residual && !boat_is_device_operand(residual, storage_of(query->dtype), query->nelements)) return NULL;
     return forward_rows(a, query, key, value, B * S, S, B * nh, nh, residual);
 }
 

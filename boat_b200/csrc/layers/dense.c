@@ -66,6 +66,7 @@ static boat_tensor_t* dense_forward(boat_dense_layer_t* l, const boat_tensor_t* 
     if (boat_report("CUDA start-up", boat_cuda_init(-1)) != 0) return NULL;
     const int mma = boat_default_mma(input->dtype), type = boat_storage_of(input->dtype);
     const int64_t N = input->shape[0], I = (int64_t)l->in_features, O = (int64_t)l->out_features;
+    if (residual && !boat_is_device_operand(residual, type, (size_t)(N * O))) return NULL;
     const int64_t oshape[2] = {N, O};
     bool xo = false, wo = false, bo = false;
     void* dx = boat_stage_in(input, type, &xo);
@@ -124,6 +125,7 @@ static boat_tensor_t* dense_backward(boat_dense_layer_t* l, const boat_tensor_t*
         return NULL;
     }
     const int mma = boat_default_mma(x->dtype), type = boat_storage_of(x->dtype);
+    if (pre_activation && !boat_is_device_operand(pre_activation, type, (size_t)(N * I))) return NULL;
     bool xo = false, go = false, wo = false;
     void* dx = boat_stage_in(x, type, &xo);
     void* dg = boat_stage_in(grad_output, type, &go);

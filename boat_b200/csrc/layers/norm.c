@@ -118,6 +118,7 @@ boat_tensor_t* boat_layernorm_backward_add(boat_layernorm_t* n, const boat_tenso
     if (grad_output->nelements != x->nelements || !boat_dtype_supported(grad_output->dtype)) return NULL;
     const int64_t H = (int64_t)n->config.normalized_shape, rows = n->rows;
     const int type = boat_storage_of(x->dtype);
+    if (residual && !boat_is_device_operand(residual, type, x->nelements)) return NULL;
     bool xo = false, yo = false, go = false;
     void* dx_in = boat_stage_in(x, type, &xo);
     void* dy = boat_stage_in(grad_output, type, &yo);

@@ -269,3 +269,24 @@ def test_block_of_fp32_tensors_equals_separate_layer_calls(gpu_lib):
     assert rel(y.numpy(), want_out) <= 1e-5
     assert rel(got_dx, want_dx) <= 4 * 2.0 ** -11
     blk.free()
+
+
+def test_block_refuses_layers_whose_sizes_do_not_meet(gpu_lib):
+    """The residuals and the kept pre-activation are operands inside other kernels; one of another size or type than the
+    tensor beside it is refused, as the separate operations did."""
+    B, S, d, dev = 2, 64, 128, capi.DEVICE_CUDA
+    x = Tensor.from_numpy(rng.normal(16, 0, (B, S, d)), dev, bf16=True)
+    for width in (64, 256):
+        blk = host.EncoderBlock(d, 2)
+        other = host.Dense(4 * d, width, device=dev)
+        h = gpu_lib.boat_encoder_block_create(blk.ln1.h, blk.attn.h, blk.ln2.h, blk.fc1.h, other.h)
+        assert not gpu_lib.boat_encoder_block_forward(h, x.h)
+        gpu_lib.boat_encoder_block_free(h)
+    # layers used elsewhere between the block's forward and backward: what they keep is of another type
+    for name in ("fc2", "ln2"):
+        blk = host.EncoderBlock(d, 2)
+        h = gpu_lib.boat_encoder_block_create(blk.ln1.h, blk.attn.h, blk.ln2.h, blk.fc1.h, blk.fc2.h)
+        out = Tensor(gpu_lib.boat_encoder_block_forward(h, x.h))
+        getattr(blk, name).forward(Tensor.from_numpy(np.ones((B * S, 4 * d if name == "fc2" else d), np.float32), dev))
+        assert not gpu_lib.boat_encoder_block_backward(h, out.h)
+        gpu_lib.boat_encoder_block_free(h)
