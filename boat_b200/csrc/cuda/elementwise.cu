@@ -326,7 +326,9 @@ __global__ void convert_multi_kernel(const ConvertTable t, int vec) {
 //     43 us);
 //   - from 32 MB per matrix on, independent CTAs on a full grid that add into a cleared output with
 //     atomics (28 us).
-// blockIdx.z selects one of several matrices of the same shape.
+// blockIdx.y is the column group, blockIdx.z selects one of several matrices of the same shape; a launch takes as many
+// groups as a grid has in y, from `first` on.
+constexpr int64_t kMaxGridY = 65535;
 constexpr int kMaxColsum = 4;
 constexpr int kColsumCluster = 8;
 struct ColsumTable {
@@ -335,14 +337,14 @@ struct ColsumTable {
 };
 
 template <typename T, int VEC, int LANES, int THREADS, bool CLUSTER>
-__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols, int add_to) {
+__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols, int64_t first, int add_to) {
     constexpr int ROWS = THREADS / LANES, COLS = LANES * VEC, UNROLL = 8;
     __shared__ float part[ROWS * COLS];
     __shared__ float folded[CLUSTER ? COLS : 1];
     griddep_sync();
     const T* __restrict__ X = (const T*)t.x[blockIdx.z];
     const int tx = threadIdx.x % LANES, ty = threadIdx.x / LANES;
-    const int64_t group0 = (int64_t)blockIdx.y * COLS, col0 = group0 + tx * VEC;
+    const int64_t group0 = (first + blockIdx.y) * COLS, col0 = group0 + tx * VEC;
     float acc[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) acc[v] = 0.f;
@@ -403,9 +405,13 @@ __global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__
 
 template <typename T, int VEC, int LANES>
 static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t cols, int count, bool add) {
-    BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)ceil_div(cols, LANES * VEC), (unsigned)count),
-                                  dim3(512), 0, kColsumCluster, t, rows, cols, add ? 1 : 0));
-    BOATCU_LAUNCH_OK("colsum");
+    const int64_t groups = ceil_div(cols, LANES * VEC);
+    for (int64_t first = 0; first < groups; first += kMaxGridY) {
+        const int64_t n = groups - first < kMaxGridY ? groups - first : kMaxGridY;
+        BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)n, (unsigned)count),
+                                      dim3(512), 0, kColsumCluster, t, rows, cols, first, add ? 1 : 0));
+        BOATCU_LAUNCH_OK("colsum");
+    }
     return 0;
 }
 
@@ -417,9 +423,12 @@ static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int c
         int64_t y = (int64_t)sm_count() * 8 / (groups * count);         // eight CTAs per SM
         if (y < 1) y = 1;
         if (y > ceil_div(rows, 8)) y = ceil_div(rows, 8);
-        BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, 32, 256, false>, dim3((unsigned)y, (unsigned)groups, (unsigned)count), dim3(256), 0, 1,
-                                      t, rows, cols, 0));
-        BOATCU_LAUNCH_OK("colsum");
+        for (int64_t first = 0; first < groups; first += kMaxGridY) {
+            const int64_t n = groups - first < kMaxGridY ? groups - first : kMaxGridY;
+            BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, 32, 256, false>, dim3((unsigned)y, (unsigned)n, (unsigned)count), dim3(256), 0, 1,
+                                          t, rows, cols, first, 0));
+            BOATCU_LAUNCH_OK("colsum");
+        }
         return 0;
     }
     // the runs of a row are 512 bytes where that makes enough CTAs for the GPU, else 256 or 128

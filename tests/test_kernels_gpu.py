@@ -412,6 +412,17 @@ def test_colsum_multi(gpu_lib, bf, rows, cols, count):
         assert np.abs(apart[i].numpy((cols,)) - ref).max() <= 1e-6 * scale
 
 
+@pytest.mark.parametrize("rows,cols", [(2, 2100001), (1, 8388604), (4, 2200001), (3, 8400000)])
+def test_colsum_of_more_columns_than_a_grid_dimension_holds(gpu_lib, rows, cols):
+    """65535 column groups of 32 or 128 columns, in either form (below and above 32 MB)."""
+    x = (rng.normal(22, 0, (rows, 4096)) * 64).round().astype(np.float32)      # whole numbers: exact sums
+    x = np.tile(x, (1, cols // 4096 + 1))[:, :cols]
+    dx, out = DeviceBuffer.from_numpy(x), DeviceBuffer(cols * 4)
+    check(gpu_lib.boat_cuda_colsum(dx.p, capi.CUDA_F32, rows, cols, out.p), "colsum")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    assert np.array_equal(out.numpy((cols,)), x.sum(axis=0))
+
+
 @pytest.mark.parametrize("sizes", [(1 << 20, 1 << 20, 1 << 20, 1 << 20), (4096, 8, 100000, 24), (7, 1001, 64)])
 def test_convert_multi_equals_single_conversions(gpu_lib, sizes):
     """Several FP32 tensors to BF16 / to TF32-valued FP32 in one launch: the bits of boat_cuda_cast /
