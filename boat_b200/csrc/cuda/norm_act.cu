@@ -5,8 +5,9 @@
 // per row, mean = sum/H, biased variance = sum((x-mean)^2)/H, y = (x-mean)/sqrt(var+eps)*w + b.
 // The reference has no LayerNorm backward (norm.c:397-402 is a stub) and no GELU
 // (src/ops/activation.c:298-302 is a stub); those follow the textbook formulas, with the
-// exact erf form of GELU.  One CTA per row keeps the row in shared memory, so a row is read
-// from HBM once per kernel; 128-bit accesses where the row length allows.
+// exact erf form of GELU.  A warp (forward) or a CTA (backward) holds a row in registers, so a row is read from HBM
+// once per kernel; rows that are no whole 16-byte vectors, or too long for that, are kept in the shared memory of a
+// CTA each.
 #include "common.cuh"
 #include "gelu.cuh"
 #include <initializer_list>
@@ -29,9 +30,10 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return t;
 }
 
+// vec: rows are whole 16-byte vectors and start on 16 bytes
 template <typename T>
-__device__ __forceinline__ void load_row(float* dst, const T* src, int cols) {
-    if (sizeof(T) == 2 && (cols & 7) == 0) {
+__device__ __forceinline__ void load_row(float* dst, const T* src, int cols, bool vec) {
+    if (sizeof(T) == 2 && vec) {
         for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) {
             uint4 v = reinterpret_cast<const uint4*>(src)[i];
             const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
@@ -42,7 +44,7 @@ __device__ __forceinline__ void load_row(float* dst, const T* src, int cols) {
                 dst[8 * i + 2 * k + 1] = f.y;
             }
         }
-    } else if (sizeof(T) == 4 && (cols & 3) == 0) {
+    } else if (sizeof(T) == 4 && vec) {
         for (int i = threadIdx.x; i < cols / 4; i += blockDim.x)
             reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
     } else {
@@ -51,8 +53,8 @@ __device__ __forceinline__ void load_row(float* dst, const T* src, int cols) {
 }
 
 template <typename T>
-__device__ __forceinline__ void store_row(T* dst, const float* src, int cols) {
-    if (sizeof(T) == 2 && (cols & 7) == 0) {
+__device__ __forceinline__ void store_row(T* dst, const float* src, int cols, bool vec) {
+    if (sizeof(T) == 2 && vec) {
         for (int i = threadIdx.x; i < cols / 8; i += blockDim.x) {
             uint4 o;
             __nv_bfloat162 h0 = __floats2bfloat162_rn(src[8 * i], src[8 * i + 1]);
@@ -65,7 +67,7 @@ __device__ __forceinline__ void store_row(T* dst, const float* src, int cols) {
             o.w = *reinterpret_cast<uint32_t*>(&h3);
             reinterpret_cast<uint4*>(dst)[i] = o;
         }
-    } else if (sizeof(T) == 4 && (cols & 3) == 0) {
+    } else if (sizeof(T) == 4 && vec) {
         for (int i = threadIdx.x; i < cols / 4; i += blockDim.x)
             reinterpret_cast<float4*>(dst)[i] = reinterpret_cast<const float4*>(src)[i];
     } else {
@@ -77,12 +79,12 @@ __device__ __forceinline__ void store_row(T* dst, const float* src, int cols) {
 template <typename T>
 __global__ void __launch_bounds__(kNormThreads)
 layernorm_fwd_kernel(const T* __restrict__ x, int cols, const float* __restrict__ gamma, const float* __restrict__ beta,
-                     float eps, T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out) {
+                     float eps, T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, bool vec) {
     griddep_sync();
     extern __shared__ float row[];          // [cols] + 32
     float* red = row + cols;
     const int64_t r = blockIdx.x;
-    load_row(row, x + r * cols, cols);
+    load_row(row, x + r * cols, cols, vec);
     __syncthreads();
     float s = 0.f;
     for (int i = threadIdx.x; i < cols; i += blockDim.x) s += row[i];
@@ -101,7 +103,7 @@ layernorm_fwd_kernel(const T* __restrict__ x, int cols, const float* __restrict_
         row[i] = n;
     }
     __syncthreads();
-    store_row(y + r * cols, row, cols);
+    store_row(y + r * cols, row, cols, vec);
     if (threadIdx.x == 0) {
         if (mean_out) mean_out[r] = mean;
         if (rstd_out) rstd_out[r] = rstd;
@@ -112,15 +114,15 @@ layernorm_fwd_kernel(const T* __restrict__ x, int cols, const float* __restrict_
 template <typename T>
 __global__ void __launch_bounds__(kNormThreads)
 layernorm_bwd_dx_kernel(const T* __restrict__ dy, const T* __restrict__ x, int cols, const float* __restrict__ gamma,
-                        const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx) {
+                        const float* __restrict__ mean, const float* __restrict__ rstd, T* __restrict__ dx, bool vec) {
     griddep_sync();
     extern __shared__ float smem[];         // g[cols], xhat[cols], 32
     float* g = smem;
     float* xh = smem + cols;
     float* red = xh + cols;
     const int64_t r = blockIdx.x;
-    load_row(g, dy + r * cols, cols);
-    load_row(xh, x + r * cols, cols);
+    load_row(g, dy + r * cols, cols, vec);
+    load_row(xh, x + r * cols, cols, vec);
     __syncthreads();
     const float m = mean[r], rs = rstd[r];
     float s1 = 0.f, s2 = 0.f;
@@ -136,7 +138,7 @@ layernorm_bwd_dx_kernel(const T* __restrict__ dy, const T* __restrict__ x, int c
     const float mgx = block_sum(s2, red) / (float)cols;
     for (int i = threadIdx.x; i < cols; i += blockDim.x) g[i] = rs * (g[i] - mg - xh[i] * mgx);
     __syncthreads();
-    store_row(dx + r * cols, g, cols);
+    store_row(dx + r * cols, g, cols, vec);
 }
 
 // ---- rows of whole 16-byte vectors -------------------------------------------------------------------
@@ -461,13 +463,15 @@ static int launch_gelu(void* out, const void* x, const void* dy, int64_t n) {
     return 0;
 }
 
-// Whether the kernels for rows of 16-byte vectors take this row length and these pointers.
+// Whether rows of this length in these arrays are whole 16-byte vectors at 16-byte addresses.
+static bool rows_of_vectors(int type, int64_t cols, std::initializer_list<const void*> ptrs) {
+    bool ok = cols % (type == BOAT_CUDA_BF16 ? 8 : 4) == 0;
+    for (const void* q : ptrs) ok = ok && aligned16(q);
+    return ok;
+}
+// Whether the kernels for such rows take this length.
 static bool rows_kernel_fits(int type, int64_t cols, std::initializer_list<const void*> ptrs) {
-    const int v = type == BOAT_CUDA_BF16 ? 8 : 4;
-    if (cols % v != 0 || cols / v > kNormMaxRowThreads) return false;
-    for (const void* q : ptrs)
-        if (((uintptr_t)q & 15) != 0) return false;
-    return true;
+    return cols / (type == BOAT_CUDA_BF16 ? 8 : 4) <= kNormMaxRowThreads && rows_of_vectors(type, cols, ptrs);
 }
 
 template <typename T, int NV>
@@ -537,16 +541,17 @@ int boat_cuda_layernorm_fwd(const void* x, int type, int64_t rows, int64_t cols,
     if (cols <= 8 * 32 * (type == BOAT_CUDA_BF16 ? 8 : 4) && rows_kernel_fits(type, cols, {x, y}))
         return type == BOAT_CUDA_BF16 ? layernorm_fwd_rows<__nv_bfloat16>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out)
                                       : layernorm_fwd_rows<float>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
+    const bool vec = rows_of_vectors(type, cols, {x, y});
     if (type == BOAT_CUDA_BF16) {
         auto k = layernorm_fwd_kernel<__nv_bfloat16>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const __nv_bfloat16*)x, (int)cols, gamma, beta, eps,
-                                                            (__nv_bfloat16*)y, mean_out, rstd_out);
+                                                            (__nv_bfloat16*)y, mean_out, rstd_out, vec);
     } else {
         auto k = layernorm_fwd_kernel<float>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const float*)x, (int)cols, gamma, beta, eps, (float*)y,
-                                                            mean_out, rstd_out);
+                                                            mean_out, rstd_out, vec);
     }
     BOATCU_LAUNCH_OK("layernorm_fwd");
     return 0;
@@ -569,6 +574,7 @@ int boat_cuda_layernorm_bwd_add(const void* dy, const void* x, int type, int64_t
                                       : layernorm_bwd_rows<float>(dy, x, rows, cols, gamma, mean, rstd, add, dx, dgamma, dbeta);
     if (dgamma) BOATCU_CHECK(cudaMemsetAsync(dgamma, 0, (size_t)cols * sizeof(float), stream()));
     if (dbeta) BOATCU_CHECK(cudaMemsetAsync(dbeta, 0, (size_t)cols * sizeof(float), stream()));
+    const bool vec = rows_of_vectors(type, cols, {dy, x, dx});
     dim3 pgrid((unsigned)ceil_div(cols, 32), 1);
     int64_t want = (int64_t)sm_count() * 8 / pgrid.x, max_y = ceil_div(rows, 8);
     pgrid.y = (unsigned)(want < 1 ? 1 : (want > max_y ? max_y : want));
@@ -576,7 +582,7 @@ int boat_cuda_layernorm_bwd_add(const void* dy, const void* x, int type, int64_t
         typedef __nv_bfloat16 bf;
         auto k = layernorm_bwd_dx_kernel<bf>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const bf*)dy, (const bf*)x, (int)cols, gamma, mean, rstd, (bf*)dx);
+        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const bf*)dy, (const bf*)x, (int)cols, gamma, mean, rstd, (bf*)dx, vec);
         BOATCU_LAUNCH_OK("layernorm_bwd_dx");
         if (dgamma || dbeta) {
             BOATCU_RUN(layernorm_bwd_params_kernel<bf>, pgrid, 256, 0, (const bf*)dy, (const bf*)x, rows, (int)cols, mean, rstd, dgamma, dbeta);
@@ -585,7 +591,7 @@ int boat_cuda_layernorm_bwd_add(const void* dy, const void* x, int type, int64_t
     } else {
         auto k = layernorm_bwd_dx_kernel<float>;
         BOATCU_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const float*)dy, (const float*)x, (int)cols, gamma, mean, rstd, (float*)dx);
+        BOATCU_RUN(k, (unsigned)rows, kNormThreads, smem, (const float*)dy, (const float*)x, (int)cols, gamma, mean, rstd, (float*)dx, vec);
         BOATCU_LAUNCH_OK("layernorm_bwd_dx");
         if (dgamma || dbeta) {
             BOATCU_RUN(layernorm_bwd_params_kernel<float>, pgrid, 256, 0, (const float*)dy, (const float*)x, rows, (int)cols, mean, rstd, dgamma, dbeta);

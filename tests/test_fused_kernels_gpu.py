@@ -9,7 +9,7 @@ import pytest
 from boat_b200 import capi, rng
 from boat_b200.host import Attention, DeviceBuffer, Tensor, Variable, check
 from gpu_driver import gpu_step
-from test_kernels_gpu import rel, run_core, run_gemm
+from test_kernels_gpu import Shifted, rel, run_core, run_gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -188,6 +188,27 @@ def test_layernorm_rows_and_residual_gradient(gpu_lib, bf, rows, cols):
         assert rel(dx.numpy((rows, cols), bf16=bf), want) <= tol
         assert np.abs(dgam.numpy((cols,)) - (G * hat).sum(0)).max() <= 1e-5 * np.abs(G * hat).sum(0).max()
         assert np.abs(dbet.numpy((cols,)) - G.sum(0)).max() <= 1e-5 * np.abs(G).sum(0).max()
+
+
+@pytest.mark.parametrize("bf", [False, True], ids=["fp32", "bf16"])
+@pytest.mark.parametrize("cols", [768, 5000])
+@pytest.mark.parametrize("which", ["x", "y", "dy", "dx", "gamma", "all"])
+def test_layernorm_of_arrays_off_alignment(gpu_lib, bf, cols, which):
+    rows, ty, tol = 37, capi.CUDA_BF16 if bf else capi.CUDA_F32, 8e-3 if bf else 2e-6
+    make = _bf if bf else (lambda s, i, sh: rng.normal(s, i, sh))
+    x, g, gamma = make(7, 0, (rows, cols)), make(7, 1, (rows, cols)), 1 + rng.normal(7, 3, (cols,)) * np.float32(0.1)
+    d = {n: Shifted(gpu_lib, (rows, cols), bf, int(which in (n, "all")), v) for n, v in dict(x=x, dy=g, y=None, dx=None).items()}
+    dg = Shifted(gpu_lib, (cols,), False, int(which in ("gamma", "all")), gamma)
+    mean, rstd, dgam, dbet = (DeviceBuffer(4 * n) for n in (rows, rows, cols, cols))
+    check(gpu_lib.boat_cuda_layernorm_fwd(d["x"].p, ty, rows, cols, dg.p, None, C.c_float(1e-5), d["y"].p, mean.p, rstd.p), "fwd")
+    check(gpu_lib.boat_cuda_layernorm_bwd(d["dy"].p, d["x"].p, ty, rows, cols, dg.p, mean.p, rstd.p, d["dx"].p, dgam.p, dbet.p), "bwd")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    X, G = x.astype(np.float64), g.astype(np.float64)
+    rs = 1 / np.sqrt(X.var(1, keepdims=True) + 1e-5)
+    hat, p = (X - X.mean(1, keepdims=True)) * rs, G * gamma
+    assert rel(d["y"].numpy(), hat * gamma) <= tol
+    assert rel(d["dx"].numpy(), (p - p.mean(1, keepdims=True) - hat * (p * hat).mean(1, keepdims=True)) * rs) <= tol
+    assert np.abs(dgam.numpy((cols,)) - (G * hat).sum(0)).max() <= 1e-5 * np.abs(G * hat).sum(0).max()
 
 
 # more work than SMs: every CTA of the persistent kernels takes several items, unevenly long ones when causal

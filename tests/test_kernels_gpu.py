@@ -202,7 +202,7 @@ def test_attention_core_on_partly_filled_tiles(gpu_lib, mma, hs, S, causal):
     assert np.abs(got["lse"] - ref["lse"]).max() <= 2e-2
 
 
-class _Shifted:
+class Shifted:
     """A device array that starts one element (or none) behind an aligned address."""
 
     def __init__(self, lib, shape, bf, shift, values=None):
@@ -230,7 +230,7 @@ def test_attention_core_with_arrays_off_alignment(gpu_lib, mma, hs, S, which):
     io, f, shape = capi.CUDA_BF16 if bf else capi.CUDA_F32, rng.bf16_round if bf else (lambda a: a), (units, S, hs)
     q, k, v, go = (f(rng.normal(7, i, shape)) for i in range(4))
     scale = 1.0 / np.sqrt(hs)
-    d = {n: _Shifted(lib, shape, bf, int(which in ("all", n)), val)
+    d = {n: Shifted(lib, shape, bf, int(which in ("all", n)), val)
          for n, val in dict(q=q, k=k, v=v, do=go, o=None, dq=None, dk=None, dv=None).items()}
     lse = DeviceBuffer(units * S * 4)
     check(lib.boat_cuda_attn_fwd(mma, units, S, hs, 1, C.c_float(scale), d["q"].p, d["k"].p, d["v"].p, io, d["o"].p, lse.p), "attn_fwd")
