@@ -17,7 +17,8 @@
 // The accumulator O is rescaled in tensor memory only when the running max has grown by more
 // than 2^8 (the warp votes), the exact correction is folded into the final 1/l.
 //
-// One thread issues the MMAs of all steps of all items in one order, steps of A and B alternating:
+// One lane, elected by a warp that stays in step, issues the MMAs of all steps of all items in one order, steps of A and
+// B alternating:
 //     S(0) .. S(NB-1) | P.V(0) S(NB) | P.V(1) S(NB+1) | ...
 // so that the exponentials of one tile run under the MMAs of the other.  S(i) takes the buffer of
 // step i-NB, whose P.V is ahead of it on the in-order tensor pipe.  With head size 64 there is room for

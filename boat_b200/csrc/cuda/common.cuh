@@ -137,8 +137,7 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
                   const void* K, const void* V, const void* O, const void* dO, const float* lse, int io_type, void* dQ,
                   void* dK, void* dV, void* scratch, size_t scratch_bytes);
 
-// tcgen05 implementations; return -1 (without setting an error) when the shape is outside
-// what the tensor-core kernels cover, so that the dispatcher can say so.
+// tcgen05 implementations, for what gemm_tc_supported takes.
 bool gemm_tc_supported(int mma, int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A,
                        int64_t lda, const void* B, int64_t ldb, int in_type, const void* C, int64_t ldc,
                        int out_type);

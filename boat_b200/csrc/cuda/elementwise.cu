@@ -321,11 +321,11 @@ __global__ void convert_multi_kernel(const ConvertTable t, int vec) {
 // A CTA's threads are LANES column lanes (16 bytes of a row each) x row lanes, eight rows' loads in flight
 // per thread; row lanes fold in shared memory.  Two ways to fold the CTAs of a column group:
 //   - a cluster of 8 CTAs, through distributed shared memory in a fixed order: one launch, no cleared
-//     output, the same bits every time.  3 x 8000 x 1024 BF16 in 9 us back to back (18 us the other way).
-//     But clusters pack unevenly onto SMs, which costs bandwidth once a matrix is large (32768 x 2048:
-//     43 us);
+//     output, the same bits every time.  3 x 8000 x 1024 BF16 back to back 14 us from HBM, 11 from L2 (18.5 the
+//     other way).  But clusters pack unevenly onto SMs, which costs bandwidth once a matrix is large (32768 x
+//     2048: 43 us);
 //   - from 32 MB per matrix on, independent CTAs on a full grid that add into a cleared output with
-//     atomics (28 us).
+//     atomics (27 us).
 // blockIdx.y is the column group, blockIdx.z selects one of several matrices of the same shape; a launch takes as many
 // groups as a grid has in y, from `first` on.
 constexpr int64_t kMaxGridY = 65535;

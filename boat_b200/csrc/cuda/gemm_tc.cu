@@ -14,15 +14,15 @@
 //   dW = X^T . dY   A = X  [K,M] M-major      B = dY [K,N] N-major
 //
 // Kernel shape: persistent, 192-thread CTAs, alone or as pairs on one tile (CTAS).  Warp 0 feeds a
-// shared-memory ring with TMA (128-byte swizzle, no multicast); one thread of warp 1 issues
-// tcgen05.mma and commits stages back to the producer; warps 2-5 drain the accumulator from tensor
+// shared-memory ring with TMA (128-byte swizzle, no multicast); warp 1 walks the stages in step and one
+// elected lane of it issues tcgen05.mma and commits stages back to the producer; warps 2-5 drain the accumulator from tensor
 // memory.  The accumulator is double-buffered in tensor memory (2 x BN columns) so that the epilogue
 // of one tile overlaps the main loop of the next.
 //
 // CTA pairs (cta_group::2, 256 x BN tiles): each CTA holds its 128 rows of A and half of B; the tensor
 // cores of both SMs read both halves of B.  A CTA then brings in and reads 32 KB per 64 of K instead of 48 -
 // a single CTA's 128 x 256 tile keeps the SM's shared-memory port 75 % busy with operands alone.  All
-// loads of a pair count on a barrier of the first CTA, whose thread issues the MMAs; its commits
+// loads of a pair count on a barrier of the first CTA, whose warp 1 issues the MMAs; its commits
 // arrive at both CTAs.
 //
 // Epilogue: a warp owns 32 rows of the tile.  It reads 64 BF16 (32 FP32) columns from tensor memory,
