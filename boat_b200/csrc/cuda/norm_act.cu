@@ -497,6 +497,15 @@ static int layernorm_fwd_rows(const void* x, int64_t rows, int64_t cols, const f
     return layernorm_fwd_launch<T, 8>(x, rows, cols, gamma, beta, eps, y, mean_out, rstd_out);
 }
 
+template <typename T, int R>
+static int layernorm_bwd_rows_launch(unsigned blocks, int threads, const void* dy, const void* x, int64_t rows, int64_t cols, const float* gamma,
+                                     const float* mean, const float* rstd, const void* add, void* dx, void* partial) {
+    BOATCU_RUN((layernorm_bwd_rows_kernel<T, R>), blocks, threads, 0, (const T*)dy, (const T*)x, rows, (int)cols, gamma, mean, rstd,
+               (const T*)add, (T*)dx, (float*)partial);
+    BOATCU_LAUNCH_OK("layernorm_bwd_rows");
+    return 0;
+}
+
 template <typename T>
 static int layernorm_bwd_rows(const void* dy, const void* x, int64_t rows, int64_t cols, const float* gamma,
                               const float* mean, const float* rstd, const void* add, void* dx, float* dgamma, float* dbeta) {
@@ -508,18 +517,13 @@ static int layernorm_bwd_rows(const void* dy, const void* x, int64_t rows, int64
     void* partial = nullptr;
     if (dgamma || dbeta)
         if (int rc = boat_cuda_malloc(&partial, 2 * (size_t)blocks * (size_t)cols * sizeof(float))) return rc;
-    if (four)
-        BOATCU_RUN((layernorm_bwd_rows_kernel<T, 4>), (unsigned)blocks, threads, 0, (const T*)dy, (const T*)x, rows, (int)cols, gamma, mean, rstd,
-                   (const T*)add, (T*)dx, (float*)partial);
-    else
-        BOATCU_RUN((layernorm_bwd_rows_kernel<T, 1>), (unsigned)blocks, threads, 0, (const T*)dy, (const T*)x, rows, (int)cols, gamma, mean, rstd,
-                   (const T*)add, (T*)dx, (float*)partial);
-    BOATCU_LAUNCH_OK("layernorm_bwd_rows");
-    if (!partial) return 0;
+    int rc = four ? layernorm_bwd_rows_launch<T, 4>((unsigned)blocks, threads, dy, x, rows, cols, gamma, mean, rstd, add, dx, partial)
+                  : layernorm_bwd_rows_launch<T, 1>((unsigned)blocks, threads, dy, x, rows, cols, gamma, mean, rstd, add, dx, partial);
+    if (!partial) return rc;
     const void* from[2] = {partial, (const float*)partial + blocks * cols};
     float* to[2] = {dgamma, dbeta};
     const int first = dgamma ? 0 : 1, count = (dgamma ? 1 : 0) + (dbeta ? 1 : 0);
-    const int rc = colsum_multi(from + first, BOAT_CUDA_F32, blocks, cols, to + first, count, false);
+    if (rc == 0) rc = colsum_multi(from + first, BOAT_CUDA_F32, blocks, cols, to + first, count, false);
     const int freed = boat_cuda_free(partial);
     return rc ? rc : freed;
 }
