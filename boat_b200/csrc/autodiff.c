@@ -81,7 +81,10 @@ static bool accumulate(boat_variable_t* v, const boat_tensor_t* g) {
         v->data->dtype == BOAT_DTYPE_FLOAT32 && g->dtype == BOAT_DTYPE_FLOAT32 && g->nelements == v->data->nelements) {
         boat_tensor_t* copy = boat_tensor_create_uninit(v->data->shape, v->data->ndim, v->data->dtype, v->data->device);
         if (!copy) return false;
-        boat_report("gradient copy", boat_cuda_scale((float*)copy->data, (const float*)g->data, 1.0f, (int64_t)g->nelements));
+        if (boat_report("gradient copy", boat_cuda_scale((float*)copy->data, (const float*)g->data, 1.0f, (int64_t)g->nelements)) != 0) {
+            boat_tensor_unref(copy);
+            return false;
+        }
         v->grad = copy;
         return true;
     }
