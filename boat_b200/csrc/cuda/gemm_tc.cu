@@ -13,10 +13,12 @@
 //   dX = dY . W^T   A = dY [M,K] K-major      B = W  [N,K] K-major
 //   dW = X^T . dY   A = X  [K,M] M-major      B = dY [K,N] N-major
 //
-// Kernel shape: persistent, 192-thread CTAs, alone or as pairs on one tile (CTAS).  Warp 0 feeds a
+// Kernel shape: persistent, 320-thread CTAs, alone or as pairs on one tile (CTAS).  Warp 0 feeds a
 // shared-memory ring with TMA (128-byte swizzle, no multicast); warp 1 walks the stages in step and one
-// elected lane of it issues tcgen05.mma and commits stages back to the producer; warps 2-5 drain the accumulator from tensor
-// memory.  The accumulator is double-buffered in tensor memory (2 x BN columns) so that the epilogue
+// elected lane of it issues tcgen05.mma and commits stages back to the producer; warps 2-9 drain the accumulator from tensor
+// memory.  Every warp that issues TMA or MMA does so as a whole, with one elected lane: a lone lane needed 310 to 580
+// cycles for the loads of a K-block, as long as its MMAs (32768 x 4096 x 1024 plain 196 -> 180 us, with GELU 266 -> 238, with its
+// derivative 332 -> 237; 1332 x 768 x 3072 15.2 -> 11.7).  The accumulator is double-buffered in tensor memory (2 x BN columns) so that the epilogue
 // of one tile overlaps the main loop of the next.
 //
 // CTA pairs (cta_group::2, 256 x BN tiles): each CTA holds its 128 rows of A and half of B; the tensor
@@ -25,7 +27,7 @@
 // loads of a pair count on a barrier of the first CTA, whose warp 1 issues the MMAs; its commits
 // arrive at both CTAs.
 //
-// Epilogue: a warp owns 32 rows of the tile.  It reads 64 BF16 (32 FP32) columns from tensor memory,
+// Epilogue: two warps per 32 rows of the tile, taking its boxes in turn.  A warp reads 64 BF16 (32 FP32) columns from tensor memory,
 // converts them, writes them as 128-byte rows to a swizzled staging box of its own and stores the box
 // with TMA.  (Storing from registers, where a lane holds a row, gave every 16-byte store a 32-byte
 // sector of its own: 786 TFLOP/s at 32768 x 4096 x 1024.)  The same boxes serve as
@@ -56,15 +58,16 @@ using namespace tc;
 namespace {
 
 constexpr int BM = 128;                          // rows of C per CTA
-constexpr int kThreads = 192;
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kMaxGroups = 4;
 constexpr int kBoxRows = 32;                     // rows of a staging box: one epilogue warp's rows
 constexpr int kStageBox = kBoxRows * 128;        // 32 rows x 128 bytes
 
 template <typename T, int CTAS, int BN, int EPI>
 struct Cfg {
-    // boxes per epilogue warp: two results in flight, and two of the second result or operand
-    static constexpr int BOXES = EPI == BOAT_EPI_NONE ? 2 : 4;
+    // boxes per epilogue warp: one result, and one of the second result or operand
+    static constexpr int BOXES = EPI == BOAT_EPI_NONE ? 1 : 2;
     static constexpr int ES = sizeof(T);
     static constexpr int BK = 128 / ES;             // one 128-byte swizzle row of K (or of M/N)
     static constexpr int UK = 32 / ES;              // K extent of one tcgen05.mma
@@ -73,7 +76,7 @@ struct Cfg {
     static constexpr int B_BYTES = BNC * 128;
     static constexpr int STAGE = A_BYTES + B_BYTES;
     static constexpr int CHUNK_BYTES = BK * 128;    // one [BK rows x 128 B] box of an MN-major operand
-    static constexpr int OUT_BYTES = 4 * BOXES * kStageBox;
+    static constexpr int OUT_BYTES = kEpiWarps * BOXES * kStageBox;
     static constexpr int FIT = (232448 - 1024 - 512 - OUT_BYTES) / STAGE;
     static constexpr int STAGES = FIT < 8 ? FIT : 8;
     static constexpr int SMEM = STAGES * STAGE + OUT_BYTES + 1024 /*alignment*/ + 512 /*barriers*/;
@@ -119,7 +122,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
     uint64_t* empty = bars + STAGES;              // [STAGES] MMA -> TMA
     uint64_t* acc_full = bars + 2 * STAGES;       // [2] MMA -> epilogue
     uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA (of the first CTA of a pair)
-    uint64_t* aux_full = bars + 2 * STAGES + 4;   // [4][2] an epilogue warp's operand boxes landed
+    uint64_t* aux_full = bars + 2 * STAGES + 4;   // [kEpiWarps] an epilogue warp's operand box landed
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 12);
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -156,9 +159,9 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4 * CTAS);
+            mbar_init(&acc_empty[b], kEpiWarps * CTAS);
         }
-        for (int b = 0; b < 8; ++b) mbar_init(&aux_full[b], 1);
+        for (int b = 0; b < kEpiWarps; ++b) mbar_init(&aux_full[b], 1);
         fence_barrier_init();
         for (int g = 0; g < p.groups; ++g) {
             tma_prefetch_desc(&maps.a[g]);
@@ -180,43 +183,63 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (int w = worker; w < work_items && ok; w += workers) {
-                const WorkItem t = item(w);
-                const int nb = t.n0 + (int)rank * C::BNC;             // this CTA's rows of B
-                for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
-                    if (rank == 0) mbar_arrive_expect_tx(&full[s], CTAS * C::STAGE);
-                    const int g = p.chain ? kb / k_one : t.g;
-                    const CUtensorMap* map_a = &maps.a[g];
-                    const CUtensorMap* map_b = &maps.b[g];
-                    const int k0 = (p.chain ? kb - g * k_one : kb) * C::BK;
-                    uint8_t* a_dst = a_smem + s * C::A_BYTES;
-                    uint8_t* b_dst = b_smem + s * C::B_BYTES;
+        // the whole warp in step, one elected lane issues: with the loop on a lone lane, whose operands cannot live in
+        // uniform registers, the three loads of a K-block took 310 cycles to issue (580 beside a GELU epilogue) and
+        // the tensor core waited for them half of its time
+        const bool leader = elect_one();
+        uint32_t s = 0, parity = 1;
+        bool ok = true;
+        for (int w = worker; w < work_items && ok; w += workers) {
+            const WorkItem t = item(w);
+            const int nb = t.n0 + (int)rank * C::BNC;                 // this CTA's rows of B
+            int g = t.g, k0 = t.kb0 * C::BK, k_end = t.kb1 * C::BK;
+            if (p.chain) {
+                g = t.kb0 / k_one;
+                k0 -= g * k_one * C::BK;
+                k_end -= g * k_one * C::BK;
+            }
+            for (;;) {                                                // one product of a chain, or all
+                const CUtensorMap* const map_a = &maps.a[g];
+                const CUtensorMap* const map_b = &maps.b[g];
+                const int stop = p.chain ? min(k_end, k_one * C::BK) : k_end;
+                for (; k0 < stop; k0 += C::BK) {
+                    if (!mbar_wait_warp(&empty[s], parity, p.status, kTimeoutProducer)) { ok = false; break; }
+                    uint8_t* const a_dst = a_smem + s * C::A_BYTES;
+                    uint8_t* const b_dst = b_smem + s * C::B_BYTES;
                     const uint32_t bar = CTAS == 2 ? peer_addr(&full[s], 0) : 0;
                     auto load = [&](uint8_t* dst, const CUtensorMap* map, int x, int y) {
                         if (CTAS == 2) tma_load_2d_pair(dst, map, bar, x, y);
                         else           tma_load_2d(dst, map, &full[s], x, y);
                     };
-                    if (A_MN) {
-                        for (int c = 0; c < BM / C::BK; ++c) load(a_dst + c * C::CHUNK_BYTES, map_a, t.m0 + c * C::BK, k0);
-                    } else {
-                        load(a_dst, map_a, k0, t.m0);
+                    if (leader) {
+                        if (rank == 0) mbar_arrive_expect_tx(&full[s], CTAS * C::STAGE);
+                        if (A_MN) {
+#pragma unroll
+                            for (int c = 0; c < BM / C::BK; ++c) load(a_dst + c * C::CHUNK_BYTES, map_a, t.m0 + c * C::BK, k0);
+                        } else {
+                            load(a_dst, map_a, k0, t.m0);
+                        }
+                        if (B_MN) {
+#pragma unroll
+                            for (int c = 0; c < C::BNC / C::BK; ++c) load(b_dst + c * C::CHUNK_BYTES, map_b, nb + c * C::BK, k0);
+                        } else {
+                            load(b_dst, map_b, k0, nb);
+                        }
                     }
-                    if (B_MN) {
-                        for (int c = 0; c < C::BNC / C::BK; ++c) load(b_dst + c * C::CHUNK_BYTES, map_b, nb + c * C::BK, k0);
-                    } else {
-                        load(b_dst, map_b, k0, nb);
+                    if (++s == STAGES) {
+                        s = 0;
+                        parity ^= 1;
                     }
                 }
+                if (!ok || k0 >= k_end) break;
+                ++g;
+                k0 = 0;
+                k_end -= k_one * C::BK;
             }
-            if (!ok) {
-                // give loads already in flight time to land before the CTA's memory goes away
-                for (int i = 0; i < 1000; ++i) __nanosleep(1000);
-            }
+        }
+        if (!ok) {
+            // give loads already in flight time to land before the CTA's memory goes away
+            for (int i = 0; i < 1000; ++i) __nanosleep(1000);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -226,7 +249,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
             const uint64_t a_desc0 = A_MN ? smem_desc_mn(smem_u32(a_smem), C::CHUNK_BYTES, TF32) : smem_desc_sw128(smem_u32(a_smem), 16, 1024);
             const uint64_t b_desc0 = B_MN ? smem_desc_mn(smem_u32(b_smem), C::CHUNK_BYTES, TF32) : smem_desc_sw128(smem_u32(b_smem), 16, 1024);
             const bool leader = elect_one();
-            uint32_t it = 0, acc_it = 0;
+            uint32_t s = 0, parity = 0, acc_it = 0;
             bool ok = true;
             for (int w = worker; w < work_items && ok; w += workers, ++acc_it) {
                 const WorkItem t = item(w);
@@ -234,9 +257,8 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                 if (!mbar_wait_warp(&acc_empty[buf], ((acc_it >> 1) & 1) ^ 1, p.status, kTimeoutMma)) { ok = false; break; }
                 tc_fence_after_sync();
                 const uint32_t d_tmem = tmem_base + buf * BN;
-                for (int kb = t.kb0; kb < t.kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!mbar_wait_warp(&full[s], (it / STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                for (int kb = t.kb0; kb < t.kb1; ++kb) {
+                    if (!mbar_wait_warp(&full[s], parity, p.status, kTimeoutMma)) { ok = false; break; }
                     tc_fence_after_sync();
                     const uint64_t a_desc = a_desc0 + (s * C::A_BYTES >> 4), b_desc = b_desc0 + (s * C::B_BYTES >> 4);
                     if (leader) {
@@ -251,6 +273,10 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                         if (CTAS == 2) mma_commit_pair(&empty[s]);
                         else           mma_commit(&empty[s]);
                     }
+                    if (++s == STAGES) {
+                        s = 0;
+                        parity ^= 1;
+                    }
                 }
                 if (ok && leader) {                   // accumulator complete
                     if (CTAS == 2) mma_commit_pair(&acc_full[buf]);
@@ -259,19 +285,24 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
             }
         }
     } else {
-        // ---------------- epilogue: warps 2..5 ----------------
+        // ---------------- epilogue: warps 2..9 ----------------
+        // two warps per quarter of the rows, box by box in turn
         const int lane_group = warp & 3;              // TMEM lanes this warp may touch
-        uint8_t* boxes = out_smem + lane_group * C::BOXES * kStageBox;        // results, then the second kind
-        uint32_t aux_it = 0;                          // operand boxes asked for so far
-        auto load_aux = [&](int x, int y) {           // by lane 0
-            const uint32_t b = aux_it & 1;
-            mbar_arrive_expect_tx(&aux_full[lane_group * 2 + b], kStageBox);
-            tma_load_2d(boxes + (2 + b) * kStageBox, &maps.aux, &aux_full[lane_group * 2 + b], x, y);
+        const int turn = (warp - 2) >> 2;
+        uint8_t* const box = out_smem + (warp - 2) * C::BOXES * kStageBox;    // result, then the second kind
+        uint8_t* const row = box + lane * 128;
+        uint8_t* const row2 = row + kStageBox;
+        uint64_t* const aux_bar = &aux_full[warp - 2];
+        uint32_t aux_it = 0;                          // operand boxes used so far
+        auto load_aux = [&](int x, int y) {           // by the leader
+            mbar_arrive_expect_tx(aux_bar, kStageBox);
+            tma_load_2d(box + kStageBox, &maps.aux, aux_bar, x, y);
         };
+        const bool leader = elect_one();
         const int swz = lane & 7;
         const bool bf16_out = p.out_type == BOAT_CUDA_BF16;
         const int step = bf16_out ? 64 : 32;          // columns per box
-        uint32_t acc_it = 0, box_it = 0;
+        uint32_t acc_it = 0;
         bool ok = true;
         for (int w = worker; w < work_items && ok; w += workers, ++acc_it) {
             const WorkItem t = item(w);
@@ -280,35 +311,36 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
             const bool bias16 = ((uintptr_t)bias & 15) == 0;
             const int buf = acc_it & 1;
             const int row0 = t.m0 + lane_group * 32;
-            if (AUX_IN) {
-                if (lane == 0) load_aux(t.n0, row0);
-                ++aux_it;
-            }
+            const int cols = min(BN, p.N - t.n0), c_first = turn * step;
+            if (AUX_IN && leader && c_first < cols) load_aux(t.n0 + c_first, row0);
             if (!mbar_wait_warp(&acc_full[buf], (acc_it >> 1) & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
             tc_fence_after_sync();
             const uint32_t t_addr = tmem_base + ((uint32_t)(lane_group * 32) << 16) + buf * BN;
-            const int cols = min(BN, p.N - t.n0);
-#pragma unroll 1
-            for (int c = 0; c < cols; c += step, ++box_it) {
-                uint8_t* box = boxes + (box_it & 1) * kStageBox;
-                // the stores that used this box (and its pair) last have read it
-                if (lane == 0) tma_wait_group_read1();
+            auto leave_accumulator = [&] {            // this warp's part of the tile is out of tensor memory
+                tc_fence_before_sync();
                 __syncwarp();
-                uint8_t* row = box + lane * 128;
+                if (leader) {
+                    if (CTAS == 2) mbar_arrive_peer(peer_addr(&acc_empty[buf], 0));
+                    else           mbar_arrive(&acc_empty[buf]);
+                }
+            };
+            if (c_first >= cols) leave_accumulator();
+#pragma unroll 1
+            for (int c = c_first; c < cols; c += 2 * step) {
                 const int col0 = t.n0 + c;
-                uint8_t* row2 = row + 2 * kStageBox;  // second result
+                uint4 aux[8];                         // the operand's row of the box
                 if (AUX_IN) {
-                    const uint32_t b = (aux_it - 1) & 1, par = ((aux_it - 1) >> 1) & 1;
-                    row2 = boxes + (2 + b) * kStageBox + lane * 128;
-                    if (c + step < cols) {            // the next operand box, under the work on this one
-                        if (lane == 0) load_aux(col0 + step, row0);
-                        ++aux_it;
-                    }
-                    if (!mbar_wait_warp(&aux_full[lane_group * 2 + b], par, p.status, kTimeoutEpilogue)) { ok = false; break; }
+                    if (!mbar_wait_warp(aux_bar, aux_it & 1, p.status, kTimeoutEpilogue)) { ok = false; break; }
+                    ++aux_it;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) aux[u] = *reinterpret_cast<const uint4*>(row2 + ((u ^ swz) << 4));
+                    __syncwarp();                     // the next one comes in under the work on this one
+                    if (leader && c + 2 * step < cols) load_aux(col0 + 2 * step, row0);
                 }
                 // one 32-column half of the box (all of an FP32 box) at a time
-#pragma unroll 1
-                for (int h = 0; h < step; h += 32) {
+#pragma unroll
+                for (int h = 0; h < 64; h += 32) {
+                    if (h == step) break;
                     uint32_t r[32];
                     tmem_ld32(t_addr + c + h, r);
                     tmem_wait_ld();
@@ -332,8 +364,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                     if (AUX_IN) {                     // BF16 only
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
-                            const uint4 q = *reinterpret_cast<const uint4*>(row2 + (((h / 8 + u) ^ swz) << 4));
-                            const uint32_t x[4] = {q.x, q.y, q.z, q.w};
+                            const uint32_t x[4] = {aux[h / 8 + u].x, aux[h / 8 + u].y, aux[h / 8 + u].z, aux[h / 8 + u].w};
 #pragma unroll
                             for (int e = 0; e < 4; ++e) {
                                 const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[e]));
@@ -346,6 +377,10 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                                 }
                             }
                         }
+                    }
+                    if (h == 0) {                     // the stores that used this box (and its pair) last have read it
+                        if (leader) tma_wait_group_read0();
+                        __syncwarp();
                     }
                     if (EPI == BOAT_EPI_GELU) {       // the rounded pre-activation, kept, then GELU of it
 #pragma unroll
@@ -383,28 +418,20 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                             *reinterpret_cast<float4*>(row + ((u ^ swz) << 4)) = make_float4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
                     }
                 }
-                if (c + step >= cols) {
-                    // the tile is out of tensor memory
-                    tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (CTAS == 2) mbar_arrive_peer(peer_addr(&acc_empty[buf], 0));
-                        else           mbar_arrive(&acc_empty[buf]);
-                    }
-                }
+                if (c + 2 * step >= cols) leave_accumulator();
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) {
+                if (leader) {
                     if (row0 < p.M) {
                         if (t.add) tma_reduce_add_2d(map_c, box, col0, row0);
                         else       tma_store_2d(map_c, box, col0, row0);
-                        if (EPI == BOAT_EPI_GELU) tma_store_2d(&maps.aux, box + 2 * kStageBox, col0, row0);
+                        if (EPI == BOAT_EPI_GELU) tma_store_2d(&maps.aux, box + kStageBox, col0, row0);
                     }
                     tma_commit_group();
                 }
             }
         }
-        if (lane == 0) tma_wait_group0();
+        if (leader) tma_wait_group0();
         if (AUX_IN && !ok)                            // an operand box may be in flight
             for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     }
