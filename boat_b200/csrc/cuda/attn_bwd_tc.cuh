@@ -226,42 +226,50 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
     if (warp == 0) {
         // ---------------- TMA producer, and the one who asks for work ----------------
-        if (lane == 0) {
-            bool ok = true;
-            uint32_t t = 0;                                  // tiles so far, of all walks
-            BwdWalk w = bwd_walk(p, blockIdx.x);
-            for (int r = 0; ok && w.n > 0; ++r) {
-                const int a = r % kBwdAnswers;
-                if (!mbar_wait(&work_empty[a], ((r / kBwdAnswers) & 1) ^ 1, p.status, kTimeoutProducer)) break;
+        // the whole warp in step, one elected lane issues, here as for the MMAs: a lone lane, whose operands cannot live
+        // in uniform registers, takes about 100 cycles per load
+        const bool leader = elect_one();
+        bool ok = true;
+        uint32_t t = 0;                                      // tiles so far, of all walks
+        BwdWalk w = bwd_walk(p, blockIdx.x);
+        for (int r = 0; ok && w.n > 0; ++r) {
+            const int a = r % kBwdAnswers;
+            if (!mbar_wait_warp(&work_empty[a], ((r / kBwdAnswers) & 1) ^ 1, p.status, kTimeoutProducer)) break;
+            if (leader) {
                 mbar_arrive_expect_tx(&work_full[a], 16);
                 request_next_cta(answers + a * 16, &work_full[a]);
-                const int kb = r % C::KV_BUFS;
-                uint8_t* k_dst = kv_smem + kb * 2 * C::TILE_BYTES;
-                if (!mbar_wait(&kv_empty[kb], ((r / C::KV_BUFS) & 1) ^ 1, p.status, kTimeoutProducer)) break;
+            }
+            const int kb = r % C::KV_BUFS;
+            uint8_t* k_dst = kv_smem + kb * 2 * C::TILE_BYTES;
+            if (!mbar_wait_warp(&kv_empty[kb], ((r / C::KV_BUFS) & 1) ^ 1, p.status, kTimeoutProducer)) break;
+            if (leader) {
                 mbar_arrive_expect_tx(&kv_full[kb], 2 * C::TILE_BYTES);
+#pragma unroll
                 for (int b = 0; b < C::NBOX; ++b) {
                     tma_load_3d(k_dst + b * kBoxBytes, &map_k, &kv_full[kb], b * 64, w.jt * kTile, w.unit);
                     tma_load_3d(k_dst + C::TILE_BYTES + b * kBoxBytes, &map_v, &kv_full[kb], b * 64, w.jt * kTile, w.unit);
                 }
-                const int64_t stat_base = (int64_t)w.unit * n_tiles * kTile;    // the statistics are padded to whole tiles
-                for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
-                    const int s = t % C::Q_STAGES;
-                    if (!mbar_wait(&q_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+            }
+            const int64_t stat_base = (int64_t)w.unit * n_tiles * kTile;    // the statistics are padded to whole tiles
+            for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
+                const int s = t % C::Q_STAGES;
+                if (!mbar_wait_warp(&q_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+                if (leader) {
                     mbar_arrive_expect_tx(&q_full[s], C::TILE_BYTES);
+#pragma unroll
                     for (int b = 0; b < C::NBOX; ++b)
                         tma_load_3d(q_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[s], b * 64, i * kTile, w.unit);
-                    // the tile's 128 exponent offsets and 128 deltas, into the buffer of its parity once
-                    // the tile before last has left it
-                    if (!mbar_wait(&stat_empty[t & 1], ((t >> 1) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+                }
+                // the tile's 128 exponent offsets and 128 deltas, into the buffer of its parity once
+                // the tile before last has left it
+                if (!mbar_wait_warp(&stat_empty[t & 1], ((t >> 1) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+                if (leader) {
                     mbar_arrive_expect_tx(&stat_full[t & 1], 1024);
                     bulk_load_1d(stat_s + (t & 1) * 256, p.lse2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
                     bulk_load_1d(stat_s + (t & 1) * 256 + 128, p.delta2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
                 }
-                if (!ok || !mbar_wait(&work_full[a], (r / kBwdAnswers) & 1, p.status, kTimeoutProducer)) break;
-                w = bwd_walk(p, taken_cta(answers + a * 16));
-                fence_proxy_async_smem();
-                mbar_arrive(&work_empty[a]);
             }
+            if (ok) w = next_walk(r, kTimeoutProducer, ok);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -568,7 +576,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // reading.  The dO tile two steps ahead is then loaded slot by slot on the same terms.
         const int lane_group = warp & 3;
         const int r = lane_group * 32 + lane;
-        const int tid128 = (warp - 10) * 32 + lane;
+        const bool issuer = warp == 10;                      // this warp issues, one elected lane of it
+        const bool leader = elect_one();
         const uint32_t lane_addr = (uint32_t)(lane_group * 32) << 16;
         const int swz = r & 7;
         // all but the most recent n reduction groups of this thread have been read out of shared memory
@@ -580,24 +589,27 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // Q_STAGES before it
         int ahead_r = 0, ahead_i = 0;                        // walk and tile of the next dO load
         BwdWalk ahead = bwd_walk(p, blockIdx.x);
-        auto load_do = [&](uint32_t t_load, auto before_box) {
+        auto load_do = [&](uint32_t t_load, auto before_box) {       // by the whole issuing warp
             if (ahead.n == 0) return;
             const int s = t_load % C::Q_STAGES;
-            mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
-            for (int b = 0; b < C::NBOX; ++b) {
-                before_box(b);
-                tma_load_3d(do_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_do, &do_full[s], b * 64, (ahead.i0 + ahead_i) * kTile, ahead.unit);
+            if (leader) {
+                mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
+#pragma unroll
+                for (int b = 0; b < C::NBOX; ++b) {
+                    before_box(b);
+                    tma_load_3d(do_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_do, &do_full[s], b * 64, (ahead.i0 + ahead_i) * kTile, ahead.unit);
+                }
             }
             if (++ahead_i == ahead.n) {
                 // ahead of the warp's own reading of this answer, so it is still there
                 const int a = ahead_r % kBwdAnswers;
-                const bool there = mbar_wait(&work_full[a], (ahead_r / kBwdAnswers) & 1, p.status, kTimeoutOther);
+                const bool there = mbar_wait_warp(&work_full[a], (ahead_r / kBwdAnswers) & 1, p.status, kTimeoutOther);
                 ahead = bwd_walk(p, there ? taken_cta(answers + a * 16) : -1);
                 ahead_i = 0;
                 ++ahead_r;
             }
         };
-        if (tid128 == 0)
+        if (issuer)
             for (uint32_t t0 = 0; t0 < C::Q_STAGES; ++t0) load_do(t0, [](int) {});
         __syncwarp();
         bool ok = true;
@@ -606,7 +618,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         for (int r_walk = 0; ok && w.n > 0; ++r_walk) {
         for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
             const int s = t % C::Q_STAGES;
-            if (tid128 == 0) drain_ok[0] = mbar_wait(dq_full, t & 1, p.status, kTimeoutOther) ? 1u : 0u;
+            if (issuer) {
+                const bool there = mbar_wait_warp(dq_full, t & 1, p.status, kTimeoutOther);
+                if (leader) drain_ok[0] = there ? 1u : 0u;
+            }
             named_barrier_sync(2, 128);
             if (drain_ok[0] == 0u) { ok = false; break; }
             tc_fence_after_sync();
@@ -627,7 +642,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             for (int b = 0; b < C::NBOX; ++b) stage_box(v[b], b);
             fence_proxy_async_smem();
             named_barrier_sync(2, 128);
-            if (tid128 == 0) {
+            if (issuer && leader) {
+#pragma unroll
                 for (int b = 0; b < C::NBOX; ++b) {
                     tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, b * 32, y, w.unit);
                     tma_commit_group();
@@ -640,22 +656,22 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             tmem_wait_ld();
             tc_fence_before_sync();
             named_barrier_sync(2, 128);                     // everybody holds the second half
-            if (tid128 == 0) mbar_arrive(dq_empty);         // the dQ columns are free
+            if (issuer && leader) mbar_arrive(dq_empty);    // the dQ columns are free
 #pragma unroll
             for (int b = 0; b < C::NBOX; ++b) {
                 // slot b was last used by the group issued NBOX groups ago
-                if (tid128 == 0) wait_read(C::NBOX - 1);
+                if (issuer && leader) wait_read(C::NBOX - 1);
                 named_barrier_sync(2, 128);                 // slot b has been read
                 stage_box(v[b], b);
                 fence_proxy_async_smem();
                 named_barrier_sync(2, 128);
-                if (tid128 == 0) {
+                if (issuer && leader) {
                     tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, (C::NBOX + b) * 32, y, w.unit);
                     tma_commit_group();
                 }
             }
             // the last group that used slot b has been read
-            if (tid128 == 0) load_do(t + C::Q_STAGES, [&](int b) { wait_read(C::NBOX - 1 - b); });
+            if (issuer) load_do(t + C::Q_STAGES, [&](int b) { wait_read(C::NBOX - 1 - b); });
             __syncwarp();
         }
         if (!ok) break;
@@ -663,7 +679,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         }
         // The CTA may end once the reductions have read their shared-memory source; that they have
         // landed in global memory by the time the next kernel runs is the grid's completion.
-        if (tid128 == 0) tma_wait_group_read0();
+        if (issuer && leader) tma_wait_group_read0();
     }
     tc_fence_before_sync();
     __syncthreads();

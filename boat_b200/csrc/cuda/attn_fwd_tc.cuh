@@ -244,46 +244,59 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     regs_release<80>();          // registers per thread from here: 80 + 208 + 208 <= 3 * 168 of the launch
     if (warp == 0) {
         // ---------------- TMA producer, and the one who asks for work ----------------
-        if (lane == 0) {
-            bool ok = true;
-            uint32_t kv = 0;                              // key/value tiles loaded so far
-            int index = blockIdx.x;
-            for (uint32_t n = 0; index >= 0 && ok; ++n) {
-                const FwdItem it = fwd_item(p, index);
-                // the next item, long before anybody needs it
-                const uint32_t w = n % WS;
-                if (!mbar_wait(&work_empty[w], ((n / WS) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+        // the whole warp in step, one elected lane issues (see the MMA issuer: the same holds for TMA)
+        const bool leader = elect_one();
+        bool ok = true;
+        uint32_t s = 0, par = 1;                          // key/value stage, parity of its next wait
+        int index = blockIdx.x;
+        for (uint32_t n = 0; index >= 0 && ok; ++n) {
+            const FwdItem it = fwd_item(p, index);
+            // the next item, long before anybody needs it
+            const uint32_t w = n % WS;
+            if (!mbar_wait_warp(&work_empty[w], ((n / WS) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+            if (leader) {
                 mbar_arrive_expect_tx(&work_full[w], 16);
                 request_next_cta(answers + w * 16, &work_full[w]);
-
-                const uint32_t qb = n % QB;
-                if (!mbar_wait(&q_empty[qb], ((n / QB) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
-                const int tiles = it.n_b > 0 ? 2 : 1, n_kv = it.n_a > it.n_b ? it.n_a : it.n_b;
+            }
+            const uint32_t qb = n % QB;
+            if (!mbar_wait_warp(&q_empty[qb], ((n / QB) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+            const int tiles = it.n_b > 0 ? 2 : 1, n_kv = it.n_a > it.n_b ? it.n_a : it.n_b;
+            if (leader) {
                 mbar_arrive_expect_tx(&q_full[qb], tiles * C::TILE_BYTES);
                 for (int g = 0; g < tiles; ++g)
+#pragma unroll
                     for (int b = 0; b < C::NBOX; ++b)
                         tma_load_3d(q_smem + (qb * 2 + g) * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[qb], b * C::BOXC,
                                     (it.qt + g) * kTile, it.unit);
-                for (int j = 0; j < n_kv; ++j, ++kv) {
-                    const int s = kv % ST;
-                    const uint32_t par = ((kv / ST) & 1) ^ 1;
-                    if (!mbar_wait(&k_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
+            }
+            for (int j = 0; j < n_kv; ++j) {
+                if (!mbar_wait_warp(&k_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
+                if (leader) {
                     mbar_arrive_expect_tx(&k_full[s], C::TILE_BYTES);
+#pragma unroll
                     for (int b = 0; b < C::NBOX; ++b)
                         tma_load_3d(k_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_k, &k_full[s], b * C::BOXC, j * kTile, it.unit);
-                    if (!mbar_wait(&v_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
+                }
+                if (!mbar_wait_warp(&v_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
+                if (leader) {
                     mbar_arrive_expect_tx(&v_full[s], C::TILE_BYTES);
+#pragma unroll
                     for (int b = 0; b < C::NBOX; ++b)
                         tma_load_3d(v_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_v, &v_full[s], b * C::BOXC, j * kTile, it.unit);
                 }
-                if (!ok || !mbar_wait(&work_full[w], (n / WS) & 1, p.status, kTimeoutProducer)) { ok = false; break; }
-                index = taken_cta(answers + w * 16);
-                fence_proxy_async_smem();
-                mbar_arrive(&work_empty[w]);
+                if (++s == ST) {
+                    s = 0;
+                    par ^= 1;
+                }
             }
-            if (!ok)
-                for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+            if (!ok || !mbar_wait_warp(&work_full[w], (n / WS) & 1, p.status, kTimeoutProducer)) { ok = false; break; }
+            index = taken_cta(answers + w * 16);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (leader) mbar_arrive(&work_empty[w]);
         }
+        if (!ok)
+            for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         // The whole warp runs this, in step, and one elected lane issues: everything but the instructions

@@ -130,7 +130,7 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
 int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const void* Q, const void* K, const void* V,
                     const void* dO, const float* lse, const float* delta, void* dQ, void* dK, void* dV) {
     using C = Bwd32Cfg;
-    constexpr int HS = kBwd32HS, SMEM = C::SMEM_DKV > C::SMEM_DQ ? C::SMEM_DKV : C::SMEM_DQ;
+    constexpr int HS = kBwd32HS, SMEM = C::SMEM;
     Bwd32Maps m;
     // the same matrices with both shared-memory layouts: 16-byte swizzle units for operands read
     // along hs, 32-byte units for operands read along their rows

@@ -127,6 +127,28 @@ def test_weight_grads_accumulate(gpu_lib, bf, shape):
     assert np.abs(db.numpy((O,)) - (b0 + dy.astype(np.float64).sum(0))).max() <= 1e-6 * np.abs(dy).sum(0).max()
 
 
+# one tile, remainders in each direction, K in pieces, every tile shape, CTA pairs, more tiles than SMs
+@pytest.mark.parametrize("mma", [capi.MMA_BF16, capi.MMA_TF32], ids=["bf16", "tf32"])
+@pytest.mark.parametrize("I,O,T,groups", [(128, 64, 64, 1), (136, 72, 333, 3), (520, 200, 1000, 2), (256, 512, 3000, 3), (2048, 1032, 700, 1),
+                                          (1024, 1024, 2500, 3)])
+def test_weight_grads_with_column_sums(gpu_lib, mma, I, O, T, groups):
+    bf = mma == capi.MMA_BF16
+    make = _bf if bf else (lambda s, i, sh: rng.normal(s, i, sh))
+    x, dy = [make(5, g, (T, I)) for g in range(groups)], [make(6, g, (T, O)) for g in range(groups)]
+    dx, ddy = ([DeviceBuffer.from_numpy(t, bf16=bf) for t in ts] for ts in (x, dy))
+    dw = [DeviceBuffer.from_numpy(np.full((I, O), np.nan, np.float32)) for _ in range(groups)]
+    db = [DeviceBuffer.from_numpy(np.full((O,), np.nan, np.float32)) for _ in range(groups)]
+    check(gpu_lib.boat_cuda_weight_grads(mma, groups, I, O, T, _table(dx), _table(ddy), capi.CUDA_BF16 if bf else capi.CUDA_F32,
+                                         _table(dw), _table(db), 0), "weight_grads")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    for g in range(groups):
+        y = dy[g].astype(np.float64)
+        assert rel(dw[g].numpy((I, O)), x[g].astype(np.float64).T @ y) <= (1e-5 if bf else 5e-3)
+        # FP32 sums of T terms in some order: random roundings of partial sums no larger than the sum of the magnitudes
+        # grow like sqrt(T) half units; four times that
+        assert (np.abs(db[g].numpy((O,)) - y.sum(0)) <= 4 * math.sqrt(T) * 2.0 ** -25 * np.abs(y).sum(0)).all()
+
+
 @pytest.mark.parametrize("n", [1, 4, 1023, 4096, 100003])
 def test_elementwise_over_several_arrays(gpu_lib, n):
     a = [rng.normal(5, i, (n,)) for i in range(4)]
@@ -218,6 +240,15 @@ def test_attention_core_with_several_items_per_cta(gpu_lib, hs, units, S, causal
     got, ref = run_core(gpu_lib, capi.MMA_BF16, units, S, hs, causal)
     for key in ("o", "dq", "dk", "dv"):
         assert rel(got[key], ref[key]) <= 2e-2, key
+
+
+# the staged TF32 backward: one key tile, two, the first that waits for a buffer used before, a remainder of one row
+@pytest.mark.parametrize("units,S", [(3, 40), (150, 256), (40, 385), (20, 1025)])
+@pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
+def test_tf32_attention_core_over_its_buffers(gpu_lib, units, S, causal):
+    got, ref = run_core(gpu_lib, capi.MMA_TF32, units, S, 64, causal)
+    for key in ("o", "dq", "dk", "dv"):
+        assert rel(got[key], ref[key]) <= 5e-3, key
 
 
 # results written to page-locked memory, packed and separate copies, chunks of more than one batch entry
