@@ -143,9 +143,10 @@ bool gemm_tc_supported(int mma, int trans_a, int trans_b, int64_t M, int64_t N, 
                        int out_type);
 int gemm_tc(int mma, int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
             const void* B, int64_t ldb, int in_type, void* C, int64_t ldc, int out_type, const float* bias);
-// C += op(A).op(B), FP32 output.
-int gemm_tc_accumulate(int mma, int trans_a, int trans_b, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
-                       const void* B, int64_t ldb, float* C, int64_t ldc);
+// boat_cuda_weight_grads: dW = X^T . dY (FP32) and, unless db is NULL, the column sums of dY, in one pass; with `add`
+// both are added to what is there.
+int gemm_tc_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T, const void* const* X, const void* const* dY,
+                         float* const* dW, float* const* db, bool add);
 // C = sum over the groups of op(A[g]).op(B[g]), one accumulator.
 int gemm_tc_sum(int mma, int trans_a, int trans_b, int groups, int64_t M, int64_t N, int64_t K, const void* const* A,
                 int64_t lda, const void* const* B, int64_t ldb, void* C, int64_t ldc, int out_type);

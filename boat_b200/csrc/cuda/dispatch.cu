@@ -130,18 +130,19 @@ int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T,
     bool ok = I > 0 && O > 0 && T > 0;
     for (int g = 0; g < groups; ++g) ok = ok && X[g] && dY[g] && dW[g];
     if (!ok && accumulate) return I > 0 && O > 0 && T <= 0 ? 0 : set_error(11, "boat_cuda_weight_grads: NULL operand");
-    const bool tensor_cores = ok && mma != BOAT_MMA_FP32 && gemm_tc_supported(mma, 1, 0, I, O, T, X[0], I, dY[0], O, store, dW[0], O, BOAT_CUDA_F32);
-    if (ok && (mma == BOAT_MMA_FP32 || (accumulate && !tensor_cores))) {
-        // the CUDA-core kernel has the rows of dY in its hands anyway: one launch, one pass
+    bool tensor_cores = ok && mma != BOAT_MMA_FP32;
+    for (int g = 0; g < groups && tensor_cores; ++g)
+        tensor_cores = gemm_tc_supported(mma, 1, 0, I, O, T, X[g], I, dY[g], O, store, dW[g], O, BOAT_CUDA_F32);
+    const bool sums = db && db[0];
+    for (int g = 0; g < groups && tensor_cores && sums; ++g) tensor_cores = db[g] != nullptr;
+    // either kernel has the rows of dY in its hands anyway: one launch, one pass
+    if (tensor_cores) return gemm_tc_weight_grads(mma, groups, I, O, T, X, dY, dW, sums ? db : nullptr, accumulate != 0);
+    if (ok && (mma == BOAT_MMA_FP32 || accumulate)) {
         ProfileScope prof("gemm_simt");
         return gemm_simt_grouped(1, 0, groups, I, O, T, X, I, dY, O, store, (void* const*)dW, O, BOAT_CUDA_F32, nullptr, db, accumulate != 0);
     }
-    if (accumulate) {
-        if (int rc = gemm_tc_accumulate(mma, 1, 0, I, O, T, X[0], I, dY[0], O, dW[0], O)) return rc;
-    } else if (int rc = boat_cuda_gemm_grouped(mma, 1, 0, groups, I, O, T, X, I, dY, O, in_type, (void* const*)dW, O, BOAT_CUDA_F32, nullptr)) {
-        return rc;
-    }
-    return db && db[0] ? colsum_multi(dY, in_type, T, O, db, groups, accumulate != 0) : 0;
+    if (int rc = boat_cuda_gemm_grouped(mma, 1, 0, groups, I, O, T, X, I, dY, O, in_type, (void* const*)dW, O, BOAT_CUDA_F32, nullptr)) return rc;
+    return sums ? colsum_multi(dY, in_type, T, O, db, groups, false) : 0;
 }
 
 int boat_cuda_attn_fwd(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,

@@ -37,6 +37,11 @@
 // pre-activation it came from, the product with GELU's derivative, a residual - whose second operand comes
 // in through the same kind of boxes.  Each saves a pass over [T, 4d] or [T, d] matrices.
 //
+// Weight gradients can carry the column sums of dY, the bias gradients (CSUM): four more warps add up what the first
+// row of tiles streams, 16 KB per K-block and CTA, behind the products.  As passes of their own the sums read dY again: 15 us
+// per 32768 x 1024 BF16 matrix at HBM rate, 5 to 7 us where a launch is the bound; step of 16 x 2048 x 1024 with Adam 1689 -> 1642
+// us, encoder block of 4 x 333 x 768 256 -> 239.
+//
 // A chained launch sums the products of its groups in one accumulator: the three input gradients of
 // self-attention are one gradient.
 //
@@ -59,6 +64,7 @@ namespace {
 
 constexpr int BM = 128;                          // rows of C per CTA
 constexpr int kEpiWarps = 8;
+constexpr int kSumWarps = 4;                     // launches with column sums only
 constexpr int kThreads = 64 + 32 * kEpiWarps;
 constexpr int kMaxGroups = 4;
 constexpr int kBoxRows = 32;                     // rows of a staging box: one epilogue warp's rows
@@ -90,6 +96,8 @@ struct GroupMaps {
 
 struct Params {
     const float* bias[kMaxGroups];
+    float* colsum[kMaxGroups];       // sums over K of B's columns
+    int colsum_add;      // ... are added to what is there
     int groups;
     int chain;           // the groups' products are summed into one result
     int M, N, K;
@@ -105,8 +113,8 @@ struct WorkItem {
     bool first, add;     // first piece of its tile (adds the bias); result is added to the output
 };
 
-template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI>
-__global__ void __launch_bounds__(kThreads, 1)
+template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI, bool CSUM>
+__global__ void __launch_bounds__(kThreads + (CSUM ? 32 * kSumWarps : 0), 1)
 gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ Params p) {
     using C = Cfg<T, CTAS, BN, EPI>;
     constexpr bool AUX_IN = EPI == BOAT_EPI_GELU_GRAD || EPI == BOAT_EPI_ADD;
@@ -124,6 +132,8 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
     uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2] epilogue -> MMA (of the first CTA of a pair)
     uint64_t* aux_full = bars + 2 * STAGES + 4;   // [kEpiWarps] an epilogue warp's operand box landed
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * STAGES + 12);
+    uint64_t* summed = bars + 2 * STAGES + 13;    // [STAGES] column sums -> TMA, behind `empty` (CSUM)
+    uint64_t* const refill = CSUM ? summed : empty;
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const uint32_t rank = CTAS == 2 ? cluster_rank() : 0;
@@ -156,6 +166,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
+            if (CSUM) mbar_init(&summed[s], kSumWarps);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
@@ -203,7 +214,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                 const CUtensorMap* const map_b = &maps.b[g];
                 const int stop = p.chain ? min(k_end, k_one * C::BK) : k_end;
                 for (; k0 < stop; k0 += C::BK) {
-                    if (!mbar_wait_warp(&empty[s], parity, p.status, kTimeoutProducer)) { ok = false; break; }
+                    if (!mbar_wait_warp(&refill[s], parity, p.status, kTimeoutProducer)) { ok = false; break; }
                     uint8_t* const a_dst = a_smem + s * C::A_BYTES;
                     uint8_t* const b_dst = b_smem + s * C::B_BYTES;
                     const uint32_t bar = CTAS == 2 ? peer_addr(&full[s], 0) : 0;
@@ -281,6 +292,75 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                 if (ok && leader) {                   // accumulator complete
                     if (CTAS == 2) mma_commit_pair(&acc_full[buf]);
                     else           mma_commit(&acc_full[buf]);
+                }
+            }
+        }
+    } else if (CSUM && warp >= 2 + kEpiWarps) {
+        // ---------------- column sums of B: warps 10..13 ----------------
+        // A tile of the first row of tiles adds up the rows of B that it streams anyway, once the tensor core is done with
+        // them (both CTAs of a pair hear of that; only the first hears of the loads), and hands the stage on to the
+        // producer.  A warp has a quarter of the columns, a lane 16 bytes of every RL-th row; the rows are dealt out so
+        // that the eight lanes of a shared-memory phase meet eight swizzle positions.  A K-block is summed for itself
+        // before it joins the total.
+        constexpr int PER = 16 / C::ES, UW = C::BNC / PER / kSumWarps, RL = 32 / UW, PH = UW < 8 ? 8 / UW : 1;
+        constexpr int PERIOD = TF32 ? 4 : 8, H = PERIOD / PH;
+        const int unit = (warp - 2 - kEpiWarps) * UW + lane % UW, rl = lane / UW, u8 = unit & 7;
+        const int row_first = (rl % PH) * H + (rl / PH) % H + rl / (PH * H) * (PH * H);
+        const uint8_t* const column = b_smem + (unit >> 3) * C::CHUNK_BYTES;
+        const bool leader = elect_one();
+        uint32_t s = 0, parity = 0;
+        bool ok = true;
+        for (int w = worker; w < work_items && ok; w += workers) {
+            const WorkItem t = item(w);
+            const bool mine = t.m0 == (int)rank * BM;
+            float total[PER];
+#pragma unroll
+            for (int e = 0; e < PER; ++e) total[e] = 0.f;
+            for (int kb = t.kb0; kb < t.kb1; ++kb) {
+                if (!mbar_wait_warp(&empty[s], parity, p.status, kTimeoutOther)) { ok = false; break; }
+                if (mine) {
+                    float sum[PER];
+#pragma unroll
+                    for (int e = 0; e < PER; ++e) sum[e] = 0.f;
+#pragma unroll
+                    for (int i = 0; i < C::BK / RL; ++i) {
+                        const int row = i * RL + row_first;
+                        const int at = TF32 ? ((((u8 >> 1) ^ (row & 3)) << 1) | (u8 & 1)) : (u8 ^ (row & 7));
+                        const uint4 q = *reinterpret_cast<const uint4*>(column + s * C::B_BYTES + row * 128 + (at << 4));
+                        const uint32_t x[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (TF32) {
+                                sum[e] += __uint_as_float(x[e]);
+                            } else {
+                                sum[2 * e % PER] += __uint_as_float(x[e] << 16);
+                                sum[(2 * e + 1) % PER] += __uint_as_float(x[e] & 0xffff0000u);
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < PER; ++e) total[e] += sum[e];
+                }
+                __syncwarp();
+                if (leader) mbar_arrive(&summed[s]);
+                if (++s == STAGES) {
+                    s = 0;
+                    parity ^= 1;
+                }
+            }
+            if (!ok || !mine) continue;
+#pragma unroll
+            for (int e = 0; e < PER; ++e)
+#pragma unroll
+                for (int d = UW; d < 32; d <<= 1) total[e] += __shfl_xor_sync(0xffffffffu, total[e], d);
+            const int col = t.n0 + (int)rank * C::BNC + unit * PER;
+            if (rl == 0) {
+                float* const out = p.colsum[t.g] + col;
+#pragma unroll
+                for (int e = 0; e < PER; ++e) {
+                    if (col + e >= p.N) break;
+                    if (t.add || p.colsum_add) atomicAdd(out + e, total[e]);
+                    else                       out[e] = total[e];
                 }
             }
         }
@@ -461,6 +541,7 @@ struct Problem {
     bool add;            // add to C instead of overwriting it (FP32)
     bool chain;          // one result: the sum of the groups' products
     void* aux;           // second result or operand of the epilogue, laid out like C
+    float* const* colsum;    // per group the sums over K of B's columns, written or (add) added to; NULL: none
     int results() const { return chain ? 1 : groups; }           // entries of C
 };
 
@@ -515,7 +596,22 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
     return r;
 }
 
-template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI>
+// Zeroes rows of N floats, ldc apart, behind each pointer; neighbours in memory in one go.
+int clear(float* const* out, int count, int64_t rows, int64_t N, int64_t ldc) {
+    for (int g = 0; g < count;) {
+        int n = 1;
+        while (ldc == N && g + n < count && out[g + n] == out[g] + n * rows * N) ++n;
+        if (ldc == N) {
+            BOATCU_CHECK(cudaMemsetAsync(out[g], 0, (size_t)n * rows * N * sizeof(float), stream()));
+        } else {
+            BOATCU_CHECK(cudaMemset2DAsync(out[g], (size_t)ldc * sizeof(float), 0, (size_t)N * sizeof(float), (size_t)rows, stream()));
+        }
+        g += n;
+    }
+    return 0;
+}
+
+template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI, bool CSUM>
 int launch(const Problem& q, const Plan& plan) {
     using C = Cfg<T, CTAS, BN, EPI>;
     GroupMaps maps;
@@ -538,14 +634,12 @@ int launch(const Problem& q, const Plan& plan) {
         if (int rc = make_tensor_map_2d(&maps.aux, q.aux, 2, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, 64)) return rc;
     const int64_t full = plan.full, split = plan.split, tiles = plan.tiles, workers = sm_count() / CTAS;
     if (split > 1 && !q.add) {
-        for (int g = 0; g < q.results(); ++g) {
-            if (q.ldc == q.N) {
-                BOATCU_CHECK(cudaMemsetAsync(q.C[g], 0, (size_t)q.M * q.N * sizeof(float), stream()));
-            } else {
-                BOATCU_CHECK(cudaMemset2DAsync(q.C[g], (size_t)q.ldc * sizeof(float), 0, (size_t)q.N * sizeof(float), (size_t)q.M, stream()));
-            }
-        }
+        if (int rc = clear((float* const*)q.C, q.results(), q.M, q.N, q.ldc)) return rc;
+        if (CSUM)
+            if (int rc = clear(q.colsum, q.groups, 1, q.N, q.N)) return rc;
     }
+    for (int g = 0; g < q.groups; ++g) p.colsum[g] = CSUM ? q.colsum[g] : nullptr;
+    p.colsum_add = q.add ? 1 : 0;
     p.groups = q.groups;
     p.chain = q.chain ? 1 : 0;
     p.M = (int)q.M;
@@ -556,7 +650,7 @@ int launch(const Problem& q, const Plan& plan) {
     p.split = (int)split;
     p.add_all = q.add ? 1 : 0;
     p.status = kernel_status_ptr();
-    auto kern = gemm_tc_kernel<T, A_MN, B_MN, CTAS, BN, EPI>;
+    auto kern = gemm_tc_kernel<T, A_MN, B_MN, CTAS, BN, EPI, CSUM>;
     static bool configured = false;     // per process = per device: the library binds to one device
     if (!configured) {
         BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
@@ -568,13 +662,13 @@ int launch(const Problem& q, const Plan& plan) {
     // stream has priority) get placed while the GEMM runs, not after it.
     const int64_t grid = (g_yielding || work < workers ? work : workers) * CTAS;
     ProfileScope prof(A_MN ? "gemm_tc_tn" : (B_MN ? "gemm_tc_nn" : "gemm_tc_nt"));
-    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)grid), dim3(kThreads), C::SMEM, CTAS, maps, p));
+    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)grid), dim3(kThreads + (CSUM ? 32 * kSumWarps : 0)), C::SMEM, CTAS, maps, p));
     BOATCU_LAUNCH_OK("gemm_tc");
     return 0;
 }
 
 // The tile shape with the shortest estimate.
-template <typename T, bool A_MN, bool B_MN, int EPI = BOAT_EPI_NONE>
+template <typename T, bool A_MN, bool B_MN, int EPI = BOAT_EPI_NONE, bool CSUM = false>
 int pick_tile(const Problem& q) {
     int best = 0;
     Plan plan;
@@ -586,10 +680,10 @@ int pick_tile(const Problem& q) {
         }
     }
     switch (best) {
-        case 0: return launch<T, A_MN, B_MN, 2, 256, EPI>(q, plan);
-        case 1: return launch<T, A_MN, B_MN, 1, 256, EPI>(q, plan);
-        case 2: return launch<T, A_MN, B_MN, 1, 128, EPI>(q, plan);
-        default: return launch<T, A_MN, B_MN, 1, 64, EPI>(q, plan);
+        case 0: return launch<T, A_MN, B_MN, 2, 256, EPI, CSUM>(q, plan);
+        case 1: return launch<T, A_MN, B_MN, 1, 256, EPI, CSUM>(q, plan);
+        case 2: return launch<T, A_MN, B_MN, 1, 128, EPI, CSUM>(q, plan);
+        default: return launch<T, A_MN, B_MN, 1, 64, EPI, CSUM>(q, plan);
     }
 }
 
@@ -625,22 +719,23 @@ int gemm_tc_grouped(int mma, int ta, int tb, int groups, int64_t M, int64_t N, i
                     const float* const* bias) {
     if (groups < 1 || groups > kMaxGroups) return set_error(11, "gemm_tc_grouped: %d groups (1..%d)", groups, kMaxGroups);
     if (int rc = ensure_init()) return rc;
-    const Problem q{groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, false, false, nullptr};
+    const Problem q{groups, M, N, K, A, lda, B, ldb, C, ldc, out_type, bias, false, false, nullptr, nullptr};
     return mma == BOAT_MMA_BF16 ? dispatch_layout<__nv_bfloat16>(ta, tb, q) : dispatch_layout<float>(ta, tb, q);
 }
 
-int gemm_tc_accumulate(int mma, int ta, int tb, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B,
-                       int64_t ldb, float* C, int64_t ldc) {
+int gemm_tc_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T, const void* const* X, const void* const* dY,
+                         float* const* dW, float* const* db, bool add) {
     if (int rc = ensure_init()) return rc;
-    void* c = C;
-    const Problem q{1, M, N, K, &A, lda, &B, ldb, &c, ldc, BOAT_CUDA_F32, nullptr, true, false, nullptr};
-    return mma == BOAT_MMA_BF16 ? dispatch_layout<__nv_bfloat16>(ta, tb, q) : dispatch_layout<float>(ta, tb, q);
+    const Problem q{groups, I, O, T, X, I, dY, O, (void* const*)dW, O, BOAT_CUDA_F32, nullptr, add, false, nullptr, db};
+    typedef __nv_bfloat16 bf;
+    if (!db) return mma == BOAT_MMA_BF16 ? pick_tile<bf, true, true>(q) : pick_tile<float, true, true>(q);
+    return mma == BOAT_MMA_BF16 ? pick_tile<bf, true, true, BOAT_EPI_NONE, true>(q) : pick_tile<float, true, true, BOAT_EPI_NONE, true>(q);
 }
 
 int gemm_tc_sum(int mma, int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
                 const void* const* B, int64_t ldb, void* C, int64_t ldc, int out_type) {
     if (int rc = ensure_init()) return rc;
-    const Problem q{groups, M, N, K, A, lda, B, ldb, &C, ldc, out_type, nullptr, false, true, nullptr};
+    const Problem q{groups, M, N, K, A, lda, B, ldb, &C, ldc, out_type, nullptr, false, true, nullptr, nullptr};
     return mma == BOAT_MMA_BF16 ? dispatch_layout<__nv_bfloat16>(ta, tb, q) : dispatch_layout<float>(ta, tb, q);
 }
 
@@ -651,7 +746,7 @@ bool gemm_tc_fused_supported(int epilogue, int ta, int tb) {
 int gemm_tc_fused(int epilogue, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda, const void* B, int64_t ldb,
                   void* C, int64_t ldc, const float* bias, void* aux) {
     if (int rc = ensure_init()) return rc;
-    const Problem q{1, M, N, K, &A, lda, &B, ldb, &C, ldc, BOAT_CUDA_BF16, &bias, false, false, aux};
+    const Problem q{1, M, N, K, &A, lda, &B, ldb, &C, ldc, BOAT_CUDA_BF16, &bias, false, false, aux, nullptr};
     typedef __nv_bfloat16 bf;
     if (epilogue == BOAT_EPI_GELU) return pick_tile<bf, false, true, BOAT_EPI_GELU>(q);
     if (epilogue == BOAT_EPI_ADD) return pick_tile<bf, false, true, BOAT_EPI_ADD>(q);
