@@ -244,11 +244,8 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (!mbar_wait_warp(&kv_empty[kb], ((r / C::KV_BUFS) & 1) ^ 1, p.status, kTimeoutProducer)) break;
             if (leader) {
                 mbar_arrive_expect_tx(&kv_full[kb], 2 * C::TILE_BYTES);
-#pragma unroll
-                for (int b = 0; b < C::NBOX; ++b) {
-                    tma_load_3d(k_dst + b * kBoxBytes, &map_k, &kv_full[kb], b * 64, w.jt * kTile, w.unit);
-                    tma_load_3d(k_dst + C::TILE_BYTES + b * kBoxBytes, &map_v, &kv_full[kb], b * 64, w.jt * kTile, w.unit);
-                }
+                tma_load_4d(k_dst, &map_k, &kv_full[kb], 0, w.jt * kTile, 0, w.unit);
+                tma_load_4d(k_dst + C::TILE_BYTES, &map_v, &kv_full[kb], 0, w.jt * kTile, 0, w.unit);
             }
             const int64_t stat_base = (int64_t)w.unit * n_tiles * kTile;    // the statistics are padded to whole tiles
             for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
@@ -256,9 +253,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 if (!mbar_wait_warp(&q_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
                 if (leader) {
                     mbar_arrive_expect_tx(&q_full[s], C::TILE_BYTES);
-#pragma unroll
-                    for (int b = 0; b < C::NBOX; ++b)
-                        tma_load_3d(q_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[s], b * 64, i * kTile, w.unit);
+                    tma_load_4d(q_smem + s * C::TILE_BYTES, &map_q, &q_full[s], 0, i * kTile, 0, w.unit);
                 }
                 // the tile's 128 exponent offsets and 128 deltas, into the buffer of its parity once
                 // the tile before last has left it

@@ -82,8 +82,7 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 // Loads a 128 x 64 tile; by the elected lane.
 __device__ __forceinline__ void bwd32_load(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int row, int unit) {
     mbar_arrive_expect_tx(bar, kBwd32Tile);
-#pragma unroll
-    for (int b = 0; b < 2; ++b) tma_load_3d(dst + b * kBoxBytes, map, bar, b * 32, row, unit);
+    tma_load_4d(dst, map, bar, 0, row, 0, unit);
 }
 
 // D[128 x 128] = A . B^T over hs, both tiles read along hs.
@@ -186,11 +185,8 @@ __device__ __forceinline__ void bwd32_dq(uint8_t* smem, int block, const CUtenso
         };
         if (leader) {
             mbar_arrive_expect_tx(q_full, 2 * kBwd32Tile);
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                tma_load_3d(q_smem + b * kBoxBytes, &map_q, q_full, b * 32, qt * kTile, unit);
-                tma_load_3d(do_smem + b * kBoxBytes, &map_do, q_full, b * 32, qt * kTile, unit);
-            }
+            tma_load_4d(q_smem, &map_q, q_full, 0, qt * kTile, 0, unit);
+            tma_load_4d(do_smem, &map_do, q_full, 0, qt * kTile, 0, unit);
         }
         load_k(0);
         load_v(0);
@@ -381,11 +377,8 @@ __device__ __forceinline__ void bwd32_dkv(uint8_t* smem, int block, const CUtens
         auto load_do = [&](int t) { load(t, do_smem + (t & 1) * kBwd32Tile, &map_do, &do_full[t & 1], &do_empty[t & 1], (t >> 1) & 1); };
         if (leader) {
             mbar_arrive_expect_tx(kv_full, 2 * kBwd32Tile);
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-                tma_load_3d(k_smem + b * kBoxBytes, &map_k, kv_full, b * 32, jt * kTile, unit);
-                tma_load_3d(v_smem + b * kBoxBytes, &map_v, kv_full, b * 32, jt * kTile, unit);
-            }
+            tma_load_4d(k_smem, &map_k, kv_full, 0, jt * kTile, 0, unit);
+            tma_load_4d(v_smem, &map_v, kv_full, 0, jt * kTile, 0, unit);
         }
         load_q(0);
         load_do(0);

@@ -264,25 +264,18 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             if (leader) {
                 mbar_arrive_expect_tx(&q_full[qb], tiles * C::TILE_BYTES);
                 for (int g = 0; g < tiles; ++g)
-#pragma unroll
-                    for (int b = 0; b < C::NBOX; ++b)
-                        tma_load_3d(q_smem + (qb * 2 + g) * C::TILE_BYTES + b * kBoxBytes, &map_q, &q_full[qb], b * C::BOXC,
-                                    (it.qt + g) * kTile, it.unit);
+                    tma_load_4d(q_smem + (qb * 2 + g) * C::TILE_BYTES, &map_q, &q_full[qb], 0, (it.qt + g) * kTile, 0, it.unit);
             }
             for (int j = 0; j < n_kv; ++j) {
                 if (!mbar_wait_warp(&k_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
                 if (leader) {
                     mbar_arrive_expect_tx(&k_full[s], C::TILE_BYTES);
-#pragma unroll
-                    for (int b = 0; b < C::NBOX; ++b)
-                        tma_load_3d(k_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_k, &k_full[s], b * C::BOXC, j * kTile, it.unit);
+                    tma_load_4d(k_smem + s * C::TILE_BYTES, &map_k, &k_full[s], 0, j * kTile, 0, it.unit);
                 }
                 if (!mbar_wait_warp(&v_empty[s], par, p.status, kTimeoutProducer)) { ok = false; break; }
                 if (leader) {
                     mbar_arrive_expect_tx(&v_full[s], C::TILE_BYTES);
-#pragma unroll
-                    for (int b = 0; b < C::NBOX; ++b)
-                        tma_load_3d(v_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_v, &v_full[s], b * C::BOXC, j * kTile, it.unit);
+                    tma_load_4d(v_smem + s * C::TILE_BYTES, &map_v, &v_full[s], 0, j * kTile, 0, it.unit);
                 }
                 if (++s == ST) {
                     s = 0;

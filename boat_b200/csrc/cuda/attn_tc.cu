@@ -16,11 +16,11 @@ int launch_fwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
                void* O, float* lse) {
     using C = FwdCfg<T, HS>;
     CUtensorMap mq, mk, mv;
-    if (int rc = make_tensor_map_units(&mq, Q, C::ES, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mk, K, C::ES, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&mq, Q, C::ES, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&mk, K, C::ES, units, S, HS, kTile)) return rc;
     // V is read by the tensor core along its contiguous head dimension: FP32 needs the
     // 32-byte-unit swizzle for that
-    if (int rc = make_tensor_map_units(&mv, V, C::ES, units, S, HS, kTile, C::TF32)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&mv, V, C::ES, units, S, HS, kTile, C::TF32)) return rc;
     FwdParams p;
     p.O = O;
     p.lse = lse;
@@ -83,9 +83,9 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     CUtensorMap mq, mk, mv, mdo, mdq;
     const int64_t n_tiles = ceil_div(S, kTile);
     const int64_t stat_rows = units * n_tiles * kTile;        // the statistics are padded to whole tiles
-    if (int rc = make_tensor_map_units(&mq, Q, 2, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mk, K, 2, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mv, V, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&mq, Q, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&mk, K, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&mv, V, 2, units, S, HS, kTile)) return rc;
     if (int rc = make_tensor_map_units(&mdo, dO, 2, units, S, HS, kTile)) return rc;
     if (int rc = make_tensor_map_units(&mdq, dq_accum, 4, units, S, HS, kTile)) return rc;   // FP32 reduce-add target
     const size_t n = (size_t)units * (size_t)S * HS;
@@ -134,13 +134,13 @@ int launch_bwd_tf32(int64_t units, int64_t S, int causal, float scale, const voi
     Bwd32Maps m;
     // the same matrices with both shared-memory layouts: 16-byte swizzle units for operands read
     // along hs, 32-byte units for operands read along their rows
-    if (int rc = make_tensor_map_units(&m.q, Q, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&m.q_mn, Q, 4, units, S, HS, kTile, true)) return rc;
-    if (int rc = make_tensor_map_units(&m.k, K, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&m.k_mn, K, 4, units, S, HS, kTile, true)) return rc;
-    if (int rc = make_tensor_map_units(&m.v, V, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&m.dout, dO, 4, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&m.dout_mn, dO, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&m.q, Q, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&m.q_mn, Q, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&m.k, K, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&m.k_mn, K, 4, units, S, HS, kTile, true)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&m.v, V, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&m.dout, dO, 4, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_unit_tiles(&m.dout_mn, dO, 4, units, S, HS, kTile, true)) return rc;
     Bwd32Params p;
     p.lse = lse;
     p.delta = delta;

@@ -104,6 +104,7 @@ struct Params {
     int out_type;
     int full;            // tiles done in one piece; the rest is split along K
     int split;
+    int wide_a, wide_b;  // an operand read along M or N comes as one copy per stage (make_tensor_map_chunks)
     int add_all;         // every tile adds to the output, not only the pieces of split tiles
     unsigned int* status;
 };
@@ -222,15 +223,23 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                         if (CTAS == 2) tma_load_2d_pair(dst, map, bar, x, y);
                         else           tma_load_2d(dst, map, &full[s], x, y);
                     };
+                    auto load_columns = [&](uint8_t* dst, const CUtensorMap* map, int column) {
+                        if (CTAS == 2) tma_load_3d_pair(dst, map, bar, 0, k0, column);
+                        else           tma_load_3d(dst, map, &full[s], 0, k0, column);
+                    };
                     if (leader) {
                         if (rank == 0) mbar_arrive_expect_tx(&full[s], CTAS * C::STAGE);
-                        if (A_MN) {
+                        if (A_MN && p.wide_a) {
+                            load_columns(a_dst, map_a, t.m0 / C::BK);
+                        } else if (A_MN) {
 #pragma unroll
                             for (int c = 0; c < BM / C::BK; ++c) load(a_dst + c * C::CHUNK_BYTES, map_a, t.m0 + c * C::BK, k0);
                         } else {
                             load(a_dst, map_a, k0, t.m0);
                         }
-                        if (B_MN) {
+                        if (B_MN && p.wide_b) {
+                            load_columns(b_dst, map_b, nb / C::BK);
+                        } else if (B_MN) {
 #pragma unroll
                             for (int c = 0; c < C::BNC / C::BK; ++c) load(b_dst + c * C::CHUNK_BYTES, map_b, nb + c * C::BK, k0);
                         } else {
@@ -452,8 +461,9 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                                     v[8 * u + 2 * e] += f.x;
                                     v[8 * u + 2 * e + 1] += f.y;
                                 } else {
-                                    v[8 * u + 2 * e] *= gelu_grad_f(f.x);
-                                    v[8 * u + 2 * e + 1] *= gelu_grad_f(f.y);
+                                    float& v0 = v[8 * u + 2 * e];
+                                    float& v1 = v[8 * u + 2 * e + 1];
+                                    GeluPair::unpack(GeluPair::mul(GeluPair::pack(v0, v1), GeluPair(f.x, f.y).grad()), v0, v1);
                                 }
                             }
                         }
@@ -471,8 +481,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                                 __nv_bfloat162 q = __floats2bfloat162_rn(v[8 * u + 2 * e], v[8 * u + 2 * e + 1]);
                                 o[e] = *reinterpret_cast<uint32_t*>(&q);
                                 const float2 f = __bfloat1622float2(q);
-                                v[8 * u + 2 * e] = gelu_f(f.x);
-                                v[8 * u + 2 * e + 1] = gelu_f(f.y);
+                                GeluPair(f.x, f.y).value(v[8 * u + 2 * e], v[8 * u + 2 * e + 1]);
                             }
                             *reinterpret_cast<uint4*>(row2 + (((h / 8 + u) ^ swz) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
                         }
@@ -596,18 +605,39 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
     return r;
 }
 
-// Zeroes rows of N floats, ldc apart, behind each pointer; neighbours in memory in one go.
-int clear(float* const* out, int count, int64_t rows, int64_t N, int64_t ldc) {
-    for (int g = 0; g < count;) {
-        int n = 1;
-        while (ldc == N && g + n < count && out[g + n] == out[g] + n * rows * N) ++n;
-        if (ldc == N) {
-            BOATCU_CHECK(cudaMemsetAsync(out[g], 0, (size_t)n * rows * N * sizeof(float), stream()));
-        } else {
-            BOATCU_CHECK(cudaMemset2DAsync(out[g], (size_t)ldc * sizeof(float), 0, (size_t)N * sizeof(float), (size_t)rows, stream()));
-        }
-        g += n;
+// Zeroes every output of a launch that adds pieces to them, and their column sums: one launch, in order with the others.
+// (A memset per output also keeps the GEMM from being set up behind the kernel before it.)
+struct ClearTable {
+    float* out[2 * kMaxGroups];      // matrices of `rows` rows, then vectors
+    int64_t rows, N, ldc;
+    int matrices;
+};
+
+__global__ void __launch_bounds__(256) clear_kernel(const ClearTable t) {
+    griddep_sync();
+    float* const out = t.out[blockIdx.y];
+    const bool matrix = (int)blockIdx.y < t.matrices;
+    const int64_t ld = matrix ? t.ldc : t.N, n = (matrix ? t.rows : 1) * t.N;
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    if (ld == t.N && n % 4 == 0 && ((uintptr_t)out & 15) == 0) {
+        for (int64_t i = first; i < n / 4; i += step) reinterpret_cast<float4*>(out)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
     }
+    for (int64_t i = first; i < n; i += step) out[i / t.N * ld + i % t.N] = 0.f;
+}
+
+int clear(const Problem& q, bool sums) {
+    ClearTable t;
+    t.rows = q.M;
+    t.N = q.N;
+    t.ldc = q.ldc;
+    t.matrices = q.results();
+    int count = 0;
+    for (int g = 0; g < t.matrices; ++g) t.out[count++] = (float*)q.C[g];
+    for (int g = 0; g < q.groups && sums; ++g) t.out[count++] = q.colsum[g];
+    const int64_t blocks = ceil_div(q.M * q.N, 256 * 4 * 4), most = 4 * sm_count();
+    BOATCU_RUN(clear_kernel, dim3((unsigned)(blocks < most ? blocks : most), (unsigned)count), 256, 0, t);
+    BOATCU_LAUNCH_OK("gemm_tc clear");
     return 0;
 }
 
@@ -617,13 +647,18 @@ int launch(const Problem& q, const Plan& plan) {
     GroupMaps maps;
     Params p;
     const bool bf16_out = q.out_type == BOAT_CUDA_BF16;
+    p.wide_a = q.M % C::BK == 0;
+    p.wide_b = q.N % C::BK == 0;
     for (int g = 0; g < q.groups; ++g) {
-        // A: K-major -> matrix [M rows, K cols], box [BM, BK].  M-major -> stored [K rows, M cols], box [BK, BK].
-        if (int rc = A_MN ? make_tensor_map_2d(&maps.a[g], q.A[g], C::ES, (uint64_t)q.K, (uint64_t)q.M, (uint64_t)q.lda, C::BK, C::BK, C::ES == 4)
-                          : make_tensor_map_2d(&maps.a[g], q.A[g], C::ES, (uint64_t)q.M, (uint64_t)q.K, (uint64_t)q.lda, BM, C::BK))
+        // A: K-major -> matrix [M rows, K cols], box [BM, BK].  M-major -> stored [K rows, M cols], boxes [BK, BK], all of them
+        // in one copy where the rows are whole 128-byte columns.
+        if (int rc = !A_MN      ? make_tensor_map_2d(&maps.a[g], q.A[g], C::ES, (uint64_t)q.M, (uint64_t)q.K, (uint64_t)q.lda, BM, C::BK)
+                     : p.wide_a ? make_tensor_map_chunks(&maps.a[g], q.A[g], C::ES, (uint64_t)q.K, (uint64_t)q.M, (uint64_t)q.lda, C::BK, BM / C::BK, C::ES == 4)
+                                : make_tensor_map_2d(&maps.a[g], q.A[g], C::ES, (uint64_t)q.K, (uint64_t)q.M, (uint64_t)q.lda, C::BK, C::BK, C::ES == 4))
             return rc;
-        if (int rc = B_MN ? make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.ldb, C::BK, C::BK, C::ES == 4)
-                          : make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.N, (uint64_t)q.K, (uint64_t)q.ldb, C::BNC, C::BK))
+        if (int rc = !B_MN      ? make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.N, (uint64_t)q.K, (uint64_t)q.ldb, C::BNC, C::BK)
+                     : p.wide_b ? make_tensor_map_chunks(&maps.b[g], q.B[g], C::ES, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.ldb, C::BK, C::BNC / C::BK, C::ES == 4)
+                                : make_tensor_map_2d(&maps.b[g], q.B[g], C::ES, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.ldb, C::BK, C::BK, C::ES == 4))
             return rc;
         if (g >= q.results()) continue;
         if (int rc = make_tensor_map_2d(&maps.c[g], q.C[g], bf16_out ? 2 : 4, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, bf16_out ? 64 : 32))
@@ -634,9 +669,7 @@ int launch(const Problem& q, const Plan& plan) {
         if (int rc = make_tensor_map_2d(&maps.aux, q.aux, 2, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, 64)) return rc;
     const int64_t full = plan.full, split = plan.split, tiles = plan.tiles, workers = sm_count() / CTAS;
     if (split > 1 && !q.add) {
-        if (int rc = clear((float* const*)q.C, q.results(), q.M, q.N, q.ldc)) return rc;
-        if (CSUM)
-            if (int rc = clear(q.colsum, q.groups, 1, q.N, q.N)) return rc;
+        if (int rc = clear(q, CSUM)) return rc;
     }
     for (int g = 0; g < q.groups; ++g) p.colsum[g] = CSUM ? q.colsum[g] : nullptr;
     p.colsum_add = q.add ? 1 : 0;

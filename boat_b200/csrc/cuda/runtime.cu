@@ -125,7 +125,7 @@ static int encode_map(CUtensorMap* map, const void* base, int esize, int rank, c
         return set_error(31, "tensor map: base or row pitch not 16-byte aligned");
     if (box[0] * (uint32_t)esize != 128 || box[1] > 256 || box[1] == 0)
         return set_error(31, "tensor map: box must be 128 bytes wide and at most 256 rows");
-    cuuint32_t estr[3] = {1, 1, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
     CUtensorMapDataType dt = esize == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     CUresult r = g_encode(map, dt, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
@@ -143,12 +143,30 @@ int make_tensor_map_2d(CUtensorMap* map, const void* base, int esize, uint64_t r
     return encode_map(map, base, esize, 2, dims, strides, box, atom32);
 }
 
+int make_tensor_map_chunks(CUtensorMap* map, const void* base, int esize, uint64_t rows, uint64_t cols, uint64_t ld,
+                           uint32_t box_rows, uint32_t chunks, bool atom32) {
+    const uint64_t wide = 128u / (uint64_t)esize;
+    cuuint64_t dims[3] = {wide, rows, cols / wide};
+    cuuint64_t strides[2] = {ld * (uint64_t)esize, 128};
+    cuuint32_t box[3] = {(cuuint32_t)wide, box_rows, chunks};
+    return encode_map(map, base, esize, 3, dims, strides, box, atom32);
+}
+
 int make_tensor_map_units(CUtensorMap* map, const void* base, int esize, uint64_t units, uint64_t S, uint64_t hs,
                           uint32_t box_rows, bool atom32) {
     cuuint64_t dims[3] = {hs, S, units};
     cuuint64_t strides[2] = {hs * (uint64_t)esize, S * hs * (uint64_t)esize};
     cuuint32_t box[3] = {128u / (uint32_t)esize, box_rows, 1};
     return encode_map(map, base, esize, 3, dims, strides, box, atom32);
+}
+
+int make_tensor_map_unit_tiles(CUtensorMap* map, const void* base, int esize, uint64_t units, uint64_t S, uint64_t hs,
+                               uint32_t box_rows, bool atom32) {
+    const uint64_t wide = 128u / (uint64_t)esize, pitch = hs * (uint64_t)esize;
+    cuuint64_t dims[4] = {wide, S, hs / wide, units};
+    cuuint64_t strides[3] = {pitch, 128, S * pitch};
+    cuuint32_t box[4] = {(cuuint32_t)wide, box_rows, (cuuint32_t)(hs / wide), 1};
+    return encode_map(map, base, esize, 4, dims, strides, box, atom32);
 }
 
 // ---- per-kernel timing ---------------------------------------------------------------------

@@ -24,12 +24,21 @@ unsigned int take_kernel_status();
 // tensor core reads along M or N) instead of the usual 16-byte unit.
 int make_tensor_map_2d(CUtensorMap* map, const void* base, int esize, uint64_t rows, uint64_t cols, uint64_t ld,
                        uint32_t box_rows, uint32_t box_cols, bool atom32 = false);
+// The same matrix as columns of 128 bytes, [rows, 128 bytes, columns]: a box of box_rows rows and `chunks` columns lands in
+// shared memory column after column, as an operand that the tensor core reads along M or N lies there, with one
+// copy instead of one per column.  The matrix's rows must be whole columns.
+int make_tensor_map_chunks(CUtensorMap* map, const void* base, int esize, uint64_t rows, uint64_t cols, uint64_t ld,
+                           uint32_t box_rows, uint32_t chunks, bool atom32);
 // The attention kernels' view of a [units*S, hs] matrix: [units, S, hs] with a box of one unit, box_rows
 // rows and 128 bytes.  A box that crosses the end of its unit reads zeros there, and a reduction or
 // store of such a box leaves the next unit alone - a sequence length need not be a multiple of the
 // tile.
 int make_tensor_map_units(CUtensorMap* map, const void* base, int esize, uint64_t units, uint64_t S, uint64_t hs,
                           uint32_t box_rows, bool atom32 = false);
+// The same with a box of whole rows, [units, columns of 128 bytes, S, 128 bytes]: its columns land one after the other, a tile
+// per copy.
+int make_tensor_map_unit_tiles(CUtensorMap* map, const void* base, int esize, uint64_t units, uint64_t S, uint64_t hs,
+                               uint32_t box_rows, bool atom32 = false);
 
 namespace tc {
 
@@ -120,6 +129,12 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
         ::"r"(smem_u32(smem_dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int w) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
         : "memory");
 }
 // Untiled bulk copy global -> shared (no multicast): `bytes` (a multiple of 16) from a 16-byte
@@ -239,6 +254,12 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
     asm volatile(
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(smem_u32(smem_dst)), "l"((uint64_t)map), "r"(bar_cluster_addr), "r"(x), "r"(y)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(smem_dst)), "l"((uint64_t)map), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
 
