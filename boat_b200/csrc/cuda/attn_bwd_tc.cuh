@@ -59,6 +59,8 @@ struct BwdCfg {
     static constexpr int NBOX = ROWB / 128;
     static constexpr int TILE_BYTES = NBOX * kBoxBytes;       // one 128 x HS BF16 tile
     static constexpr int DS_BYTES = 2 * kBoxBytes;             // dS^T: 128 x 128 BF16
+    // With head size 64 dQ leaves through a staging area of its own; with 128 through the tile's idle dO stage.
+    static constexpr int DQ_BYTES = HS == 64 ? 128 * HS * 4 : 0;
     // Q / dO stages: three when they fit (head size 64), so that the dO tile loaded behind a
     // dQ read-out is not needed before the tile after next
     static constexpr int Q_STAGES = HS == 64 ? 3 : 2;
@@ -66,7 +68,7 @@ struct BwdCfg {
     // K,V + Q,dO stages + dS^T + two (lse, delta) buffers + barriers.  With head size 128 this
     // is 231,808 of the 232,448 bytes a CTA may have, so the base must come 1024-byte aligned
     // from the launch (checked at kernel entry) - there is no room for manual alignment slack.
-    static constexpr int SMEM = KV_BUFS * 2 * TILE_BYTES + Q_STAGES * 2 * TILE_BYTES + DS_BYTES + 2048 + 384;
+    static constexpr int SMEM = KV_BUFS * 2 * TILE_BYTES + Q_STAGES * 2 * TILE_BYTES + DS_BYTES + DQ_BYTES + 2048 + 448;
     // tensor memory columns
     // R0 (columns 0..127) holds S^T, then P^T.  With head size 64 dP^T has 128 columns of its
     // own.  With head size 128 nothing is left (R0 + dQ + dV + dK = 512), and dP^T borrows the dQ
@@ -75,9 +77,14 @@ struct BwdCfg {
     // the softmax warps have read dP^T anyway.  Either way dP^T of a tile is issued before the
     // softmax warps ask for it, and they go from the exponentials straight on to dS^T.
     static constexpr bool DP_OWN = 256 + 3 * HS <= 512;
+    // With head size 64 P^T has columns of its own too (128 BF16 in 64 columns), so that the scores of the next tile, and
+    // likewise its dP^T, follow as soon as the softmax warps have taken this tile's into registers, and are there when
+    // those ask for them.
     static constexpr uint32_t COL_S = 0;
     static constexpr uint32_t COL_DQ = DP_OWN ? 256 : 128, COL_DV = COL_DQ + HS, COL_DK = COL_DQ + 2 * HS;
     static constexpr uint32_t COL_DP = DP_OWN ? 128 : COL_DQ;
+    static constexpr uint32_t COL_P = DP_OWN ? 256 + 3 * HS : COL_S;
+    static constexpr uint32_t P_HALF = DP_OWN ? 32 : 64;      // from the first half of a row of P^T to the second
     static constexpr uint32_t TMEM_COLS = 512;
 };
 
@@ -144,12 +151,12 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     uint8_t* q_smem = kv_smem + C::KV_BUFS * 2 * C::TILE_BYTES;        // [Q_STAGES]
     uint8_t* do_smem = q_smem + C::Q_STAGES * C::TILE_BYTES;           // [Q_STAGES]
     uint8_t* ds_smem = do_smem + C::Q_STAGES * C::TILE_BYTES;
-    float* stat_s = (float*)(ds_smem + C::DS_BYTES);                   // [2][-lse*log2e[128], -delta/sqrt(hs)[128]]
+    uint8_t* dq_smem = ds_smem + C::DS_BYTES;
+    float* stat_s = (float*)(dq_smem + C::DQ_BYTES);                   // [2][-lse*log2e[128], -delta/sqrt(hs)[128]]
     uint64_t* bars = (uint64_t*)(stat_s + 512);
     uint64_t* kv_full = bars;                   // [KV_BUFS]
     uint64_t* q_full = bars + 16;               // [Q_STAGES] Q tile landed
     uint64_t* s_full = bars + 5;                // S^T complete
-    uint64_t* ds_full = bars + 6;               // dS^T in smem (256 arrivals)
     uint64_t* dq_full = bars + 7;               // all MMAs of the tile complete
     uint64_t* dq_empty = bars + 8;              // dQ is out of its TMEM columns
     uint64_t* all_done = bars + 9;
@@ -161,10 +168,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     uint64_t* acc_free = bars + 2;              // dK, dV of the walk are out of tensor memory (256 arrivals)
     uint64_t* stat_full = bars + 11;            // [2] the tile's statistics landed
     uint64_t* stat_empty = bars + 13;           // [2] phase B of the tile is over (256 arrivals)
+    uint64_t* s_read = bars + 4;                // the softmax warps hold S^T (256 arrivals; head size 64)
+    uint64_t* ds_empty = bars + 6;              // dK of the tile is complete: the dS^T tile may be overwritten (head size 64)
+    uint64_t* do_empty = bars + 48;             // [Q_STAGES] dP^T and dV of the tile are complete (head size 64)
+    uint64_t* dp_read = bars + 15;              // ... and dP^T
     uint64_t* work_full = bars + 28;            // [kBwdAnswers] the answer to a request for work is there
     uint64_t* work_empty = bars + 32;           // [kBwdAnswers] producer, MMA issuer, softmax and dQ warps have read it
     uint8_t* answers = (uint8_t*)(bars + 36);   // [kBwdAnswers] 16 bytes
     uint32_t* tmem_slot = (uint32_t*)(bars + 44);
+    // [2] dS^T in smem (256 arrivals).  Two in turn: with head size 64 dP^T of tile t+1 is issued before the wait for dS^T(t), so
+    // dS^T(t+1) may be there by the time the MMA issuer gets to that wait.
+    uint64_t* ds_full = bars + 46;
     volatile uint32_t* drain_ok = tmem_slot + 3;       // outcome of the dQ warps' wait
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
@@ -179,13 +193,18 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             mbar_init(&q_full[s], 1);
             mbar_init(&do_full[s], 1);
             mbar_init(&q_empty[s], 1);
+            mbar_init(&do_empty[s], 1);
         }
         mbar_init(s_full, 1);
-        mbar_init(ds_full, 256);
+        mbar_init(&ds_full[0], 256);
+        mbar_init(&ds_full[1], 256);
+        mbar_init(s_read, 256);
+        mbar_init(dp_read, 256);
         mbar_init(p_full, 256);
         mbar_init(dp_full, 1);
         mbar_init(dq_full, 1);
-        mbar_init(dq_empty, 1);
+        mbar_init(dq_empty, C::DQ_BYTES ? 4 : 1);
+        mbar_init(ds_empty, 1);
         mbar_init(all_done, 1);
         mbar_init(acc_free, 256);
         for (int b = 0; b < kBwdAnswers; ++b) {
@@ -263,6 +282,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     bulk_load_1d(stat_s + (t & 1) * 256, p.lse2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
                     bulk_load_1d(stat_s + (t & 1) * 256 + 128, p.delta2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
                 }
+                if (C::DQ_BYTES) {
+                    if (!mbar_wait_warp(&do_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+                    if (leader) {
+                        mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
+                        tma_load_3d(do_smem + s * C::TILE_BYTES, &map_do, &do_full[s], 0, i * kTile, w.unit);
+                    }
+                }
             }
             if (ok) w = next_walk(r, kTimeoutProducer, ok);
         }
@@ -282,7 +308,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             const uint64_t k_mn = smem_desc_mn(smem_u32(kv_smem), kBoxBytes, false), q_mn = smem_desc_mn(smem_u32(q_smem), kBoxBytes, false);
             const uint64_t do_mn = smem_desc_mn(smem_u32(do_smem), kBoxBytes, false), ds_mn = smem_desc_mn(smem_u32(ds_smem), kBoxBytes, false);
             // Issue order on the (in-order) tensor pipe, per tile t:
-            //   dV(t) S(t+1) | dQ(t) dK(t) | dP(t+1)
+            //   dV(t) S(t+1) | dQ(t) dK(t) | dP(t+1)          with head size 64: S(t+1) | dV(t) | dP(t+1) | dQ(t) dK(t)
             // dV follows phase A; S^T of the next tile overwrites R0 right behind it (dV, ahead on
             // the pipe, is the only reader of P^T).  dK and dQ need dS^T from phase B.  dP^T of the
             // next tile follows them: into its own columns (head size 64), or into the dQ columns
@@ -344,6 +370,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                         if (last && !mbar_wait_warp(&kv_full[kb_next], ((r + 1) / C::KV_BUFS) & 1, p.status, kTimeoutMma)) return false;
                         return issue_s(t + 1, kb_next);
                     };
+                    if (C::DP_OWN && more) {
+                        if (!mbar_wait_warp(s_read, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                        if (!next_s()) { ok = false; break; }
+                    }
                     if (!mbar_wait_warp(p_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
                     if (!mbar_wait_warp(&do_full[s], (t / C::Q_STAGES) & 1, p.status, kTimeoutMma)) { ok = false; break; }
                     // the previous walk's dK, dV must have left tensor memory
@@ -352,12 +382,17 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     if (leader) {
 #pragma unroll
                         for (int kk = 0; kk < kTile / 16; ++kk)      // dV += P^T . dO      (K = 128 query rows)
-                            mma_ts<false>(tmem_base + C::COL_DV, tmem_base + C::COL_S + (kk / 4) * 64 + (kk % 4) * 8,
+                            mma_ts<false>(tmem_base + C::COL_DV, tmem_base + C::COL_P + (kk / 4) * C::P_HALF + (kk % 4) * 8,
                                           do_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
+                        if (C::DQ_BYTES) mma_commit(&do_empty[s]);
+                    }
+                    if (C::DP_OWN && more) {
+                        if (!mbar_wait_warp(dp_read, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                        if (!issue_dp(t + 1, kb_next)) { ok = false; break; }
                     }
                     // R0 is free as soon as dV, ahead on the pipe, has read P^T
-                    if (early && !next_s()) { ok = false; break; }
-                    if (!mbar_wait_warp(ds_full, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                    if (!C::DP_OWN && early && !next_s()) { ok = false; break; }
+                    if (!mbar_wait_warp(&ds_full[t & 1], (t >> 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
                     if (t > 0) {
                         // the previous dQ must have left its TMEM columns
                         if (!mbar_wait_warp(dq_empty, (t - 1) & 1, p.status, kTimeoutMma)) { ok = false; break; }
@@ -377,17 +412,18 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                             const uint32_t off = ((kk / 4) * kBoxBytes + (kk % 4) * 32) >> 4;
                             mma_ss<false>(tmem_base + C::COL_DK, ds_desc + off, q_d + (kk * 2048 >> 4), idesc_acc, !first || kk > 0);
                         }
+                        if (C::DQ_BYTES) mma_commit(ds_empty);
                         mma_commit(&q_empty[s]);  // also: the dS^T tile is no longer read
                         if (last) {
                             mma_commit(&kv_empty[kb]);              // K and V of the walk are no longer read
                             mma_commit(all_done);                   // and its dK, dV are complete
                         }
                     }
-                    if (more && !early && !next_s()) { ok = false; break; }
+                    if (!C::DP_OWN && more && !early && !next_s()) { ok = false; break; }
                     // dS^T of tile t is in shared memory, so the softmax warps are done with dP^T(t)
-                    if (more) {
+                    if (!C::DP_OWN && more) {
                         // borrowed columns: this tile's dQ, just issued, has to complete and leave them first
-                        if (!C::DP_OWN && !mbar_wait_warp(dq_empty, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
+                        if (!mbar_wait_warp(dq_empty, t & 1, p.status, kTimeoutMma)) { ok = false; break; }
                         if (!issue_dp(t + 1, kb_next)) { ok = false; break; }
                     }
                 }
@@ -459,6 +495,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 tmem_ld32(tmem_base + C::COL_S + lane_addr + col0, s0);
                 tmem_ld32(tmem_base + C::COL_S + lane_addr + col0 + 32, s1);
                 tmem_wait_ld();
+                if (C::DP_OWN) {
+                    tc_fence_before_sync();
+                    mbar_arrive(s_read);
+                }
                 // The mask test is a compile-time flag of the loop body: a branch per group of
                 // columns would end the compiler's scheduling region there and leave the warp
                 // running each group's FMA -> exp2 -> convert chain at its latency.
@@ -503,8 +543,13 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
                     for (int x = 0; x < 32; ++x) ph[x] = 0u;
                 }
-                // P^T over this thread's own S^T columns: 64 BF16 = 32 columns starting at col0
-                tmem_st32(tmem_base + C::COL_S + lane_addr + col0, ph);
+                // P^T(t-1) has been read: dP^T(t) was issued behind the dV that read it.  (Phase B wants dP^T(t) anyway.)
+                if (C::DP_OWN) {
+                    if (!mbar_wait_warp(dp_full, t & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
+                    tc_fence_after_sync();
+                }
+                // 64 BF16 = 32 columns; with head size 128 the first of this thread's own S^T columns
+                tmem_st32(tmem_base + C::COL_P + lane_addr + half * C::P_HALF, ph);
             }
             tmem_wait_st();
             tc_fence_before_sync();
@@ -517,13 +562,20 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 mbar_arrive(acc_free);
             }
             // ---- phase B: dS^T = P^T * (dP^T - delta) / sqrt(hs) ----
-            if (!mbar_wait_warp(dp_full, t & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
-            tc_fence_after_sync();
+            if (!C::DP_OWN) {
+                if (!mbar_wait_warp(dp_full, t & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
+                tc_fence_after_sync();
+            }
             {
                 uint32_t d0[32], d1[32];
                 tmem_ld32(tmem_base + C::COL_DP + lane_addr + col0, d0);
                 tmem_ld32(tmem_base + C::COL_DP + lane_addr + col0 + 32, d1);
                 tmem_wait_ld();
+                if (C::DP_OWN) {
+                    tc_fence_before_sync();
+                    mbar_arrive(dp_read);
+                    if (t > 0 && !mbar_wait_warp(ds_empty, (t - 1) & 1, p.status, kTimeoutSoftmax)) { ok = false; break; }
+                }
 #pragma unroll
                 for (int half32 = 0; half32 < 2; ++half32) {
 #pragma unroll
@@ -551,7 +603,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 }
             }
             fence_proxy_async_smem();
-            mbar_arrive(ds_full);
+            mbar_arrive(&ds_full[t & 1]);
             mbar_arrive(&stat_empty[t & 1]);                 // this tile's statistics are no longer read
         }
         jt_before = w.jt;
@@ -560,6 +612,59 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         w = next_walk(r_walk, kTimeoutSoftmax, ok);
         if (ok && w.n == 0) store_dkdv(unit_before, jt_before, r_walk & 1);
         }
+    } else if constexpr (C::DQ_BYTES != 0) {
+        // ---------------- dQ reduction, head size 64: warps 10..13, thread = query row ----------------
+        // Each warp by itself: its 32 rows of the tile from tensor memory to two boxes of its own (32 rows x 128 bytes) and
+        // from there, by TMA reduce-add, into the sum.  It waits for the reductions of the tile before to have read the
+        // boxes, and for nobody else.  All four warps through the tile's dO stage, with a barrier per step and the dO tiles
+        // loaded behind it, took 3300 cycles a tile, all of the tile's period: with scores and dP^T ahead 256 units of
+        // 2048 rows, causal, with preparation and cast took 541 us before and 519 now, 512 of 1024 518 and 503.  What bounds a
+        // tile now is shared memory (304 KB, 2375 cycles): without exponentials, statistics and reductions it still takes 460.
+        // (Tried on this: one half of the softmax warps half a tile behind the other 528; dS^T in tensor memory as dK's
+        // operand, in P^T's columns, 608.)
+        const int lane_group = warp & 3;
+        const uint32_t t_dq = tmem_base + C::COL_DQ + ((uint32_t)(lane_group * 32) << 16);
+        uint8_t* const boxes = dq_smem + lane_group * (C::DQ_BYTES / 4);
+        uint8_t* const row = boxes + lane * 128;
+        const int swz = lane & 7;
+        const bool leader = elect_one();
+        bool ok = true;
+        uint32_t t = 0;                                      // tiles so far, of all walks
+        BwdWalk w = bwd_walk(p, blockIdx.x);
+        for (int r_walk = 0; ok && w.n > 0; ++r_walk) {
+            for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
+                if (!mbar_wait_warp(dq_full, t & 1, p.status, kTimeoutOther)) { ok = false; break; }
+                tc_fence_after_sync();
+                uint32_t v[HS / 32][32];
+#pragma unroll
+                for (int b = 0; b < HS / 32; ++b) tmem_ld32(t_dq + b * 32, v[b]);
+                tmem_wait_ld();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (leader) {
+                    mbar_arrive(dq_empty);                   // this warp's part of the dQ columns is free
+                    tma_wait_group_read0();
+                }
+                __syncwarp();
+#pragma unroll
+                for (int b = 0; b < HS / 32; ++b)
+#pragma unroll
+                    for (int u = 0; u < 8; ++u)
+                        *reinterpret_cast<uint4*>(row + b * 4096 + ((u ^ swz) << 4)) = make_uint4(v[b][4 * u], v[b][4 * u + 1], v[b][4 * u + 2], v[b][4 * u + 3]);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (leader && i * kTile + lane_group * 32 < p.S) {
+#pragma unroll
+                    for (int b = 0; b < HS / 32; ++b) tma_reduce_add_3d(&map_dq, boxes + b * 4096, b * 32, i * kTile + lane_group * 32, w.unit);
+                    tma_commit_group();
+                }
+            }
+            if (!ok) break;
+            w = next_walk(r_walk, kTimeoutOther, ok);
+        }
+        // The CTA may end once the reductions have read their shared-memory source; that they have
+        // landed in global memory by the time the next kernel runs is the grid's completion.
+        if (leader) tma_wait_group_read0();
     } else {
         // ---------------- dQ reduction: warps 10..13, thread = query row ----------------
         // The FP32 dQ tile is HS/32 boxes of 128 rows x 128 bytes (16 KB each), twice what the tile's
