@@ -286,6 +286,7 @@ int boat_cuda_allreduce_join(void) {
     if (!g_pending) return 0;
     if (!g_nccl.fake) {
         BOATCU_CHECK(cudaEventRecord(g_ev_done, g_comm_stream));
+        ordinary_launch_next();
         BOATCU_CHECK(cudaStreamWaitEvent(stream(), g_ev_done, 0));
     }
     g_pending = false;

@@ -57,8 +57,50 @@ __device__ __forceinline__ void griddep_sync() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// GEMMs, and the passes that prepare their operands and outputs, name the memory they read and write (LaunchTurn).  Such a
+// kernel lets its successor's CTAs be placed only once it has passed its own wait (kRelease): what came before it is
+// complete when they run.  A successor that also names its memory, and touches none that matters to the kernels which may still
+// be running, does not wait for them (kBeside): a weight gradient beside an input gradient, a conversion beside either.  It
+// fills the SMs as they come free, without the gap between two launches, and waits for its predecessor at its
+// end instead, so that its completion still implies that of all kernels before it.
+// Encoder block of 4 x 333 x 768 BF16: 227 us with every kernel waiting, 217 so; residual attention of 4 x 250 x 256 FP32 155 and 147.
+enum Follow { kRelease = 1, kBeside = 2 };
+__device__ __forceinline__ void griddep_enter(int follow) {
+    if (follow != kBeside) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void griddep_leave(int follow) {
+    if (follow == kBeside) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// One launch on the library stream.  Holds the order of launches still while it lives, so that the kernels
+// before are the ones it is compared with.  reads() and writes() name what the kernel touches, all of it; follow() then says
+// how it is to be launched.  A turn that names nothing is an ordinary launch, and so is what follows a copy, a memset or a wait for
+// an event on the stream.
+class LaunchTurn {
+public:
+    LaunchTurn();
+    ~LaunchTurn();
+    LaunchTurn(const LaunchTurn&) = delete;
+    void reads(const void* p, size_t bytes) { name(p, bytes, false); }
+    void writes(const void* p, size_t bytes) { name(p, bytes, true); }
+    // rows of `cols` elements of `es` bytes, ld elements apart
+    void reads(const void* p, int64_t rows, int64_t cols, int64_t ld, size_t es) { reads(p, span(rows, cols, ld, es)); }
+    void writes(const void* p, int64_t rows, int64_t cols, int64_t ld, size_t es) { writes(p, span(rows, cols, ld, es)); }
+    int follow();
+
+private:
+    static size_t span(int64_t rows, int64_t cols, int64_t ld, size_t es) { return rows > 0 && cols > 0 ? (size_t)((rows - 1) * ld + cols) * es : 0; }
+    void name(const void* p, size_t bytes, bool written);
+    bool named_, beside_;
+    int before_;                     // ranges of the kernels before that may still run
+};
+
+// Something other than a named kernel comes next on the library stream, or the stream changes.
+void ordinary_launch_next();
+
 template <typename... P, typename... A>
-inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
+inline cudaError_t launch_in_turn(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -74,6 +116,11 @@ inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, s
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
+    LaunchTurn turn;
+    return launch_in_turn(kern, grid, block, smem, cluster, static_cast<A&&>(args)...);
+}
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Dynamic shared memory of a launch of `ctas` CTAs that need `smem` bytes each: so much that no SM takes
@@ -86,6 +133,8 @@ inline int spread_smem(int smem, int64_t ctas) {
     return smem > least ? smem : least;
 }
 
+#define BOATCU_RUN_IN_TURN(kern, grid, block, smem, ...) \
+    BOATCU_CHECK(boatcu::launch_in_turn(kern, dim3(grid), dim3(block), smem, 1, __VA_ARGS__))
 #define BOATCU_RUN(kern, grid, block, smem, ...) \
     BOATCU_CHECK(boatcu::launch_dependent(kern, dim3(grid), dim3(block), smem, 1, __VA_ARGS__))
 

@@ -130,8 +130,8 @@ __global__ void add_n_kernel(float* __restrict__ y, const AddTable t, int64_t n,
 }
 
 // ---- the SGD step of a layer that accumulates its gradients: y -= fl(lr*g), then g = 0 ----------------
-__global__ void sgd_clear_kernel(const AxpyTable t, float lr, int vec) {
-    griddep_sync();
+__global__ void sgd_clear_kernel(const AxpyTable t, float lr, int vec, int follow) {
+    griddep_enter(follow);
     float* __restrict__ y = t.y[blockIdx.y];
     float* __restrict__ g = const_cast<float*>(t.x[blockIdx.y]);
     const int64_t n = t.n[blockIdx.y], n4 = vec ? n / 4 : 0;
@@ -145,6 +145,7 @@ __global__ void sgd_clear_kernel(const AxpyTable t, float lr, int vec) {
         y[i] = mul_add(-lr, g[i], y[i]);
         g[i] = 0.f;
     }
+    griddep_leave(follow);
 }
 
 // ---- y = a * b -------------------------------------------------------------------------------
@@ -187,8 +188,8 @@ __global__ void add_bias_kernel(float* __restrict__ y, const float* __restrict__
 // ---- y = alpha*a + beta*b on FP32 or BF16 storage (residual adds, differences, MSE gradient) ----
 template <typename T>
 __global__ void lincomb_kernel(T* __restrict__ y, const T* __restrict__ a, float alpha, const T* __restrict__ b,
-                               float beta, int64_t n, int vec) {
-    griddep_sync();
+                               float beta, int64_t n, int vec, int follow) {
+    griddep_enter(follow);
     constexpr int V = 16 / sizeof(T);
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -206,11 +207,12 @@ __global__ void lincomb_kernel(T* __restrict__ y, const T* __restrict__ a, float
     } else {
         for (; i < n; i += step) y[i] = from_f32<T>(alpha * to_f32(a[i]) + beta * to_f32(b[i]));
     }
+    griddep_leave(follow);
 }
 
 // ---- casts -----------------------------------------------------------------------------------
-__global__ void cast_f32_to_bf16(__nv_bfloat16* __restrict__ dst, const float* __restrict__ src, int64_t n, int vec) {
-    griddep_sync();
+__global__ void cast_f32_to_bf16(__nv_bfloat16* __restrict__ dst, const float* __restrict__ src, int64_t n, int vec, int follow) {
+    griddep_enter(follow);
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {   // 8 elements: two 128-bit loads, one 128-bit store
@@ -228,10 +230,11 @@ __global__ void cast_f32_to_bf16(__nv_bfloat16* __restrict__ dst, const float* _
     } else {
         for (; i < n; i += step) dst[i] = __float2bfloat16_rn(src[i]);
     }
+    griddep_leave(follow);
 }
 
-__global__ void cast_bf16_to_f32(float* __restrict__ dst, const __nv_bfloat16* __restrict__ src, int64_t n, int vec) {
-    griddep_sync();
+__global__ void cast_bf16_to_f32(float* __restrict__ dst, const __nv_bfloat16* __restrict__ src, int64_t n, int vec, int follow) {
+    griddep_enter(follow);
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {
@@ -248,6 +251,7 @@ __global__ void cast_bf16_to_f32(float* __restrict__ dst, const __nv_bfloat16* _
     } else {
         for (; i < n; i += step) dst[i] = __bfloat162float(src[i]);
     }
+    griddep_leave(follow);
 }
 
 // ---- y = x rounded to the nearest TF32 value (10-bit mantissa), still stored as FP32 -------------
@@ -260,8 +264,8 @@ __device__ __forceinline__ float round_tf32(float x) {
     return __uint_as_float(r);
 }
 
-__global__ void round_tf32_kernel(float* __restrict__ y, const float* __restrict__ x, int64_t n, int vec) {
-    griddep_sync();
+__global__ void round_tf32_kernel(float* __restrict__ y, const float* __restrict__ x, int64_t n, int vec, int follow) {
+    griddep_enter(follow);
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     if (vec) {
@@ -273,6 +277,7 @@ __global__ void round_tf32_kernel(float* __restrict__ y, const float* __restrict
     } else {
         for (; i < n; i += step) y[i] = round_tf32(x[i]);
     }
+    griddep_leave(follow);
 }
 
 // ---- several FP32 tensors to BF16 or to TF32-valued FP32, one launch ----------------------------
@@ -285,8 +290,8 @@ struct ConvertTable {
 
 // blockIdx.y = tensor; vec: every tensor is 16-byte aligned with a multiple of 8 elements
 template <bool TO_BF16>
-__global__ void convert_multi_kernel(const ConvertTable t, int vec) {
-    griddep_sync();
+__global__ void convert_multi_kernel(const ConvertTable t, int vec, int follow) {
+    griddep_enter(follow);
     const float* __restrict__ src = t.src[blockIdx.y];
     const int64_t n = t.n[blockIdx.y];
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -315,6 +320,7 @@ __global__ void convert_multi_kernel(const ConvertTable t, int vec) {
             else         ((float*)t.dst[blockIdx.y])[i] = round_tf32(src[i]);
         }
     }
+    griddep_leave(follow);
 }
 
 // ---- column sums: out[j] = sum_i X[i,j] ------------------------------------------------------
@@ -337,11 +343,11 @@ struct ColsumTable {
 };
 
 template <typename T, int VEC, int LANES, int THREADS, bool CLUSTER>
-__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols, int64_t first, int add_to) {
+__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols, int64_t first, int add_to, int follow) {
     constexpr int ROWS = THREADS / LANES, COLS = LANES * VEC, UNROLL = 8;
     __shared__ float part[ROWS * COLS];
     __shared__ float folded[CLUSTER ? COLS : 1];
-    griddep_sync();
+    griddep_enter(follow);
     const T* __restrict__ X = (const T*)t.x[blockIdx.z];
     const int tx = threadIdx.x % LANES, ty = threadIdx.x / LANES;
     const int64_t group0 = (first + blockIdx.y) * COLS, col0 = group0 + tx * VEC;
@@ -401,6 +407,7 @@ __global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__
         }
         cluster.sync();
     }
+    griddep_leave(follow);
 }
 
 template <typename T, int VEC, int LANES>
@@ -408,8 +415,13 @@ static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t col
     const int64_t groups = ceil_div(cols, LANES * VEC);
     for (int64_t first = 0; first < groups; first += kMaxGridY) {
         const int64_t n = groups - first < kMaxGridY ? groups - first : kMaxGridY;
-        BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)n, (unsigned)count),
-                                      dim3(512), 0, kColsumCluster, t, rows, cols, first, add ? 1 : 0));
+        LaunchTurn turn;
+        for (int i = 0; i < count; ++i) {
+            turn.reads(t.x[i], (size_t)rows * cols * sizeof(T));
+            turn.writes(t.out[i], (size_t)cols * 4);
+        }
+        BOATCU_CHECK(launch_in_turn(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)n, (unsigned)count),
+                                    dim3(512), 0, kColsumCluster, t, rows, cols, first, add ? 1 : 0, turn.follow()));
         BOATCU_LAUNCH_OK("colsum");
     }
     return 0;
@@ -426,7 +438,7 @@ static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int c
         for (int64_t first = 0; first < groups; first += kMaxGridY) {
             const int64_t n = groups - first < kMaxGridY ? groups - first : kMaxGridY;
             BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, 32, 256, false>, dim3((unsigned)y, (unsigned)n, (unsigned)count), dim3(256), 0, 1,
-                                          t, rows, cols, first, 0));
+                                          t, rows, cols, first, 0, (int)kRelease));
             BOATCU_LAUNCH_OK("colsum");
         }
         return 0;
@@ -674,7 +686,8 @@ int boat_cuda_stage_copy(void* dst, const void* src, size_t bytes, int down) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
     if (bytes > kStageKernelBytes || !aligned16(dst) || !aligned16(src) || bytes % 16) {
-        BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, stream()));
+        ordinary_launch_next();
+    BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, stream()));
         return 0;
     }
     const int64_t n = (int64_t)(bytes / 16);
@@ -691,7 +704,13 @@ int boat_cuda_sgd_clear(float* const* y, float* const* g, float lr, const int64_
     if (int rc = fill_axpy_table("boat_cuda_sgd_clear", y, g, n, count, t, vec, longest)) return rc;
     if (longest <= 0) return 0;
     if (int rc = ensure_init()) return rc;
-    BOATCU_RUN(sgd_clear_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, lr, vec);
+    LaunchTurn turn;
+    for (int i = 0; i < count; ++i) {
+        turn.writes(y[i], (size_t)n[i] * 4);
+        turn.writes(g[i], (size_t)n[i] * 4);
+    }
+    BOATCU_RUN_IN_TURN(sgd_clear_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, lr,
+                       vec, turn.follow());
     BOATCU_LAUNCH_OK("sgd_clear");
     return 0;
 }
@@ -722,10 +741,14 @@ int boat_cuda_cast(void* dst, int dst_type, const void* src, int src_type, int64
     int vec = aligned16(dst) && aligned16(src) && (n % 8) == 0;
     int grid = grid_for(vec ? n / 8 : n, kThreads);
     ProfileScope prof("cast");
+    LaunchTurn turn;
+    turn.reads(src, (size_t)n * type_size(src_type));
+    turn.writes(dst, (size_t)n * type_size(dst_type));
+    const int follow = turn.follow();
     if (dst_type == BOAT_CUDA_BF16)
-        BOATCU_RUN(cast_f32_to_bf16, grid, kThreads, 0, (__nv_bfloat16*)dst, (const float*)src, n, vec);
+        BOATCU_RUN_IN_TURN(cast_f32_to_bf16, grid, kThreads, 0, (__nv_bfloat16*)dst, (const float*)src, n, vec, follow);
     else
-        BOATCU_RUN(cast_bf16_to_f32, grid, kThreads, 0, (float*)dst, (const __nv_bfloat16*)src, n, vec);
+        BOATCU_RUN_IN_TURN(cast_bf16_to_f32, grid, kThreads, 0, (float*)dst, (const __nv_bfloat16*)src, n, vec, follow);
     BOATCU_LAUNCH_OK("cast");
     return 0;
 }
@@ -737,11 +760,16 @@ int boat_cuda_lincomb(void* y, const void* a, float alpha, const void* b, float 
     int vec = aligned16(y) && aligned16(a) && aligned16(b) && (n % V) == 0;
     int grid = grid_for(vec ? n / V : n, kThreads);
     ProfileScope prof("lincomb");
+    LaunchTurn turn;
+    turn.reads(a, (size_t)n * type_size(type));
+    turn.reads(b, (size_t)n * type_size(type));
+    turn.writes(y, (size_t)n * type_size(type));
+    const int follow = turn.follow();
     if (type == BOAT_CUDA_BF16)
-        BOATCU_RUN(lincomb_kernel<__nv_bfloat16>, grid, kThreads, 0, (__nv_bfloat16*)y, (const __nv_bfloat16*)a, alpha,
-                                                                       (const __nv_bfloat16*)b, beta, n, vec);
+        BOATCU_RUN_IN_TURN(lincomb_kernel<__nv_bfloat16>, grid, kThreads, 0, (__nv_bfloat16*)y, (const __nv_bfloat16*)a, alpha,
+                                                                       (const __nv_bfloat16*)b, beta, n, vec, follow);
     else
-        BOATCU_RUN(lincomb_kernel<float>, grid, kThreads, 0, (float*)y, (const float*)a, alpha, (const float*)b, beta, n, vec);
+        BOATCU_RUN_IN_TURN(lincomb_kernel<float>, grid, kThreads, 0, (float*)y, (const float*)a, alpha, (const float*)b, beta, n, vec, follow);
     BOATCU_LAUNCH_OK("lincomb");
     return 0;
 }
@@ -751,7 +779,10 @@ int boat_cuda_round_tf32(float* y, const float* x, int64_t n) {
     if (int rc = ensure_init()) return rc;
     int vec = aligned16(y) && aligned16(x) && (n % 4) == 0;
     ProfileScope prof("round_tf32");
-    BOATCU_RUN(round_tf32_kernel, grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, y, x, n, vec);
+    LaunchTurn turn;
+    turn.reads(x, (size_t)n * 4);
+    turn.writes(y, (size_t)n * 4);
+    BOATCU_RUN_IN_TURN(round_tf32_kernel, grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, y, x, n, vec, turn.follow());
     BOATCU_LAUNCH_OK("round_tf32");
     return 0;
 }
@@ -820,8 +851,14 @@ int boat_cuda_convert_multi(void* const* dst, int dst_type, const float* const* 
     if (per_tensor > cap) per_tensor = cap;
     dim3 grid((unsigned)per_tensor, (unsigned)count, 1);
     ProfileScope prof("cast");
-    if (dst_type == BOAT_CUDA_BF16) BOATCU_RUN(convert_multi_kernel<true>, grid, kThreads, 0, t, vec);
-    else                            BOATCU_RUN(convert_multi_kernel<false>, grid, kThreads, 0, t, vec);
+    LaunchTurn turn;
+    for (int i = 0; i < count; ++i) {
+        turn.reads(src[i], (size_t)n[i] * 4);
+        turn.writes(dst[i], (size_t)n[i] * type_size(dst_type));
+    }
+    const int follow = turn.follow();
+    if (dst_type == BOAT_CUDA_BF16) BOATCU_RUN_IN_TURN(convert_multi_kernel<true>, grid, kThreads, 0, t, vec, follow);
+    else                            BOATCU_RUN_IN_TURN(convert_multi_kernel<false>, grid, kThreads, 0, t, vec, follow);
     BOATCU_LAUNCH_OK("convert_multi");
     return 0;
 }

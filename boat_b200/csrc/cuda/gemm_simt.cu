@@ -38,6 +38,7 @@ struct SimtParams {
     int64_t M, N, K, lda, ldb, ldc;
     int n_tiles, split;
     int vec_a, vec_b, vec_c;         // 16-byte accesses possible
+    int follow;                      // how the launch follows the one before (Follow)
     int add;                         // add to C and colsum instead of overwriting them (FP32 output)
 };
 
@@ -176,7 +177,7 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     auto row = [&](int i) { return A_M ? (i / 4) * 32 + lm * 4 + i % 4 : lm + 8 * i; };
     auto col = [&](int j) { return B_K ? ln + 4 * j : (j / 4) * 16 + ln * 4 + j % 4; };
 
-    griddep_sync();
+    griddep_enter(p.follow);
     // the first rounds only fetch, so that the code of a fetch is there once
     for (int s = s0 - (S::STAGES - 1); s < s1; ++s) {
         if (s >= s0) {
@@ -311,6 +312,7 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     if (split == 1) {
 #pragma unroll 2
         for (int e = tid; e < kUnits; e += 256) put(e, sliced(e));
+        griddep_leave(p.follow);
         return;
     }
     // every CTA of the cluster adds its share of the tile over all of them, lowest K first
@@ -344,6 +346,7 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
         }
     }
     cluster.sync();                                       // nobody leaves while its partial tile is being read
+    griddep_leave(p.follow);
 }
 
 template <typename TI, typename TO, bool A_M, bool B_K, int WM, int WN>
@@ -360,7 +363,18 @@ int launch_tile(SimtParams& p, int groups, int split) {
     p.n_tiles = (int)ceil_div(p.N, S::BN);
     p.split = split;
     const int smem = spread_smem(S::SMEM, tiles * split * groups);
-    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), smem, (unsigned)split, p));
+    {
+        LaunchTurn turn;
+        for (int g = 0; g < groups; ++g) {
+            turn.reads(p.A[g], A_M ? p.K : p.M, A_M ? p.M : p.K, p.lda, sizeof(TI));
+            turn.reads(p.B[g], B_K ? p.N : p.K, B_K ? p.K : p.N, p.ldb, sizeof(TI));
+            turn.writes(p.C[g], p.M, p.N, p.ldc, sizeof(TO));
+            turn.reads(p.bias[g], (size_t)p.N * 4);
+            turn.writes(p.colsum[g], (size_t)p.N * 4);
+        }
+        p.follow = turn.follow();
+        BOATCU_CHECK(launch_in_turn(kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), smem, (unsigned)split, p));
+    }
     BOATCU_LAUNCH_OK("gemm_simt");
     return 0;
 }

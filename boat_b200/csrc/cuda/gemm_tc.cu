@@ -105,6 +105,7 @@ struct Params {
     int full;            // tiles done in one piece; the rest is split along K
     int split;
     int wide_a, wide_b;  // an operand read along M or N comes as one copy per stage (make_tensor_map_chunks)
+    int follow;          // how the launch follows the one before (Follow)
     int add_all;         // every tile adds to the output, not only the pieces of split tiles
     unsigned int* status;
 };
@@ -186,7 +187,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         if (CTAS == 2) tmem_alloc_pair(tmem_slot, C::TMEM_COLS);
         else           tmem_alloc(tmem_slot, C::TMEM_COLS);
     }
-    griddep_sync();
+    griddep_enter(p.follow);
     tc_fence_before_sync();
     __syncthreads();
     if (CTAS == 2) cluster_sync_all();            // the peer's barriers exist before anything arrives there
@@ -532,6 +533,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         if (CTAS == 2) tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
         else           tmem_dealloc(tmem_base, C::TMEM_COLS);
     }
+    griddep_leave(p.follow);
 }
 
 bool g_yielding = false;
@@ -554,17 +556,17 @@ struct Problem {
     int results() const { return chain ? 1 : groups; }           // entries of C
 };
 
-// A tile shape and what it costs, measured on B200 with every shape forced on outputs of 128 x 1024 to
-// 8192 x 1024 and 1024 x 1024 x 8192: microseconds per K-block (128 bytes of K per row), and once per launch more than
-// the narrowest tile (filling the ring, the epilogue that nothing overlaps).  A K-block costs what its bytes cost to
-// bring to the SM; FP32 operands that lie along M or N add to that, since the tensor core then
-// reads them at about half its rate (block_us[1]: B, [2]: both).  Pairs on 256 x 256 are fastest per FLOP (1440
-// TFLOP/s BF16 at 32768 x 2048 x 2048; a single CTA's 128 x 256 1220, 128 x 128 900, 128 x 64 510) and slowest to start.
-struct Shape { int ctas, bn; double block_us[3], once_us; };
-constexpr Shape kShapes[4] = {{2, 256, {0.38, 0.50, 0.52}, 3.5},
-                              {1, 256, {0.44, 0.70, 0.90}, 1.3},
-                              {1, 128, {0.31, 0.47, 0.64}, 1.1},
-                              {1, 64, {0.30, 0.36, 0.44}, 0.0}};
+// A tile shape and what it costs, measured on B200 with every shape forced on 66 outputs from 128 x 1024 to 8192 x 1024 with K
+// of 512 to 3072: microseconds per K-block (128 bytes of K per row, either type) on a full GPU, [1] with A read along M, and
+// once per launch more than the narrowest tile, which has about 3.5 (filling the ring, the epilogue that nothing
+// overlaps).  A K-block costs what its bytes cost to bring to the SM: 24, 32, 48 KB per CTA.  The choice is within 0.5 % of the
+// best shape on average, 7 % at worst (K of 3072 at 8000 x 1024: pairs 36 us, 128 x 256 37, 128 x 128 43, 128 x 64 59;
+// 1332 x 768: 20, 18, 12, 11.5).
+struct Shape { int ctas, bn; double block_us[2], once_us; };
+constexpr Shape kShapes[4] = {{2, 256, {0.29, 0.28}, 2.6},
+                              {1, 256, {0.32, 0.38}, 1.0},
+                              {1, 128, {0.18, 0.22}, 0.3},
+                              {1, 64, {0.156, 0.18}, 0.0}};
 
 struct Plan {
     int64_t tiles, full, split;
@@ -572,8 +574,8 @@ struct Plan {
 };
 
 // Which tiles are cut along K, into how many pieces, and how long the launch should take.
-Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
-    const double block_us = sh.block_us[slow];
+Plan make_plan(const Problem& q, const Shape& sh, int bk, bool a_mn) {
+    const double block_us = sh.block_us[a_mn];
     const int64_t workers = sm_count() / sh.ctas, k_blocks = ceil_div(q.K, bk) * (q.chain ? q.groups : 1);
     Plan r;
     r.tiles = ceil_div(q.M, BM * sh.ctas) * ceil_div(q.N, sh.bn) * q.results();
@@ -610,20 +612,21 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk, int slow) {
 struct ClearTable {
     float* out[2 * kMaxGroups];      // matrices of `rows` rows, then vectors
     int64_t rows, N, ldc;
-    int matrices;
+    int matrices, follow;
 };
 
 __global__ void __launch_bounds__(256) clear_kernel(const ClearTable t) {
-    griddep_sync();
+    griddep_enter(t.follow);
     float* const out = t.out[blockIdx.y];
     const bool matrix = (int)blockIdx.y < t.matrices;
     const int64_t ld = matrix ? t.ldc : t.N, n = (matrix ? t.rows : 1) * t.N;
     const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     if (ld == t.N && n % 4 == 0 && ((uintptr_t)out & 15) == 0) {
         for (int64_t i = first; i < n / 4; i += step) reinterpret_cast<float4*>(out)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
+    } else {
+        for (int64_t i = first; i < n; i += step) out[i / t.N * ld + i % t.N] = 0.f;
     }
-    for (int64_t i = first; i < n; i += step) out[i / t.N * ld + i % t.N] = 0.f;
+    griddep_leave(t.follow);
 }
 
 int clear(const Problem& q, bool sums) {
@@ -636,7 +639,10 @@ int clear(const Problem& q, bool sums) {
     for (int g = 0; g < t.matrices; ++g) t.out[count++] = (float*)q.C[g];
     for (int g = 0; g < q.groups && sums; ++g) t.out[count++] = q.colsum[g];
     const int64_t blocks = ceil_div(q.M * q.N, 256 * 4 * 4), most = 4 * sm_count();
-    BOATCU_RUN(clear_kernel, dim3((unsigned)(blocks < most ? blocks : most), (unsigned)count), 256, 0, t);
+    LaunchTurn turn;
+    for (int i = 0; i < count; ++i) turn.writes(t.out[i], i < t.matrices ? q.M : 1, q.N, i < t.matrices ? q.ldc : q.N, 4);
+    t.follow = turn.follow();
+    BOATCU_CHECK(launch_in_turn(clear_kernel, dim3((unsigned)(blocks < most ? blocks : most), (unsigned)count), dim3(256), 0, 1, t));
     BOATCU_LAUNCH_OK("gemm_tc clear");
     return 0;
 }
@@ -695,7 +701,20 @@ int launch(const Problem& q, const Plan& plan) {
     // stream has priority) get placed while the GEMM runs, not after it.
     const int64_t grid = (g_yielding || work < workers ? work : workers) * CTAS;
     ProfileScope prof(A_MN ? "gemm_tc_tn" : (B_MN ? "gemm_tc_nn" : "gemm_tc_nt"));
-    BOATCU_CHECK(launch_dependent(kern, dim3((unsigned)grid), dim3(kThreads + (CSUM ? 32 * kSumWarps : 0)), C::SMEM, CTAS, maps, p));
+    {
+        LaunchTurn turn;
+        for (int g = 0; g < q.groups; ++g) {
+            turn.reads(q.A[g], A_MN ? q.K : q.M, A_MN ? q.M : q.K, q.lda, C::ES);
+            turn.reads(q.B[g], B_MN ? q.K : q.N, B_MN ? q.N : q.K, q.ldb, C::ES);
+            if (g >= q.results()) continue;
+            turn.writes(q.C[g], q.M, q.N, q.ldc, bf16_out ? 2 : 4);
+            turn.reads(p.bias[g], (size_t)q.N * 4);
+            turn.writes(p.colsum[g], (size_t)q.N * 4);
+        }
+        turn.writes(q.aux, q.M, q.N, q.ldc, 2);
+        p.follow = turn.follow();
+        BOATCU_CHECK(launch_in_turn(kern, dim3((unsigned)grid), dim3(kThreads + (CSUM ? 32 * kSumWarps : 0)), C::SMEM, CTAS, maps, p));
+    }
     BOATCU_LAUNCH_OK("gemm_tc");
     return 0;
 }
@@ -706,7 +725,7 @@ int pick_tile(const Problem& q) {
     int best = 0;
     Plan plan;
     for (int i = 0; i < 4; ++i) {
-        const Plan t = make_plan(q, kShapes[i], 128 / (int)sizeof(T), sizeof(T) == 4 ? (int)A_MN + (int)B_MN : 0);
+        const Plan t = make_plan(q, kShapes[i], 128 / (int)sizeof(T), A_MN);
         if (i == 0 || t.us < plan.us) {
             plan = t;
             best = i;

@@ -220,10 +220,10 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(kNormThreads)
 layernorm_fwd_rows_kernel(const T* __restrict__ x, int64_t rows, int cols, const float* __restrict__ gamma,
                           const float* __restrict__ beta, float eps, T* __restrict__ y, float* __restrict__ mean_out,
-                          float* __restrict__ rstd_out) {
+                          float* __restrict__ rstd_out, int follow) {
     constexpr int V = Vec16<T>::N;
     extern __shared__ __align__(16) float params[];          // gamma, beta
-    griddep_sync();
+    griddep_enter(follow);
     for (int i = threadIdx.x; i < cols; i += kNormThreads) {
         params[i] = gamma ? gamma[i] : 1.f;
         params[cols + i] = beta ? beta[i] : 0.f;
@@ -281,6 +281,7 @@ layernorm_fwd_rows_kernel(const T* __restrict__ x, int64_t rows, int cols, const
             if (rstd_out) rstd_out[r] = rstd;
         }
     }
+    griddep_leave(follow);
 }
 
 // dx as in layernorm_bwd_dx_kernel, plus `add` (a residual branch's gradient) if given.  A thread owns one
@@ -480,8 +481,15 @@ static int layernorm_fwd_launch(const void* x, int64_t rows, int64_t cols, const
     const size_t smem = 2 * (size_t)cols * sizeof(float);
     int64_t blocks = ceil_div(rows, kNormThreads / 32);
     if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-    BOATCU_RUN((layernorm_fwd_rows_kernel<T, NV>), (unsigned)blocks, kNormThreads, smem, (const T*)x, rows, (int)cols, gamma, beta, eps, (T*)y,
-               mean_out, rstd_out);
+    LaunchTurn turn;
+    turn.reads(x, (size_t)rows * cols * sizeof(T));
+    turn.reads(gamma, (size_t)cols * 4);
+    turn.reads(beta, (size_t)cols * 4);
+    turn.writes(y, (size_t)rows * cols * sizeof(T));
+    turn.writes(mean_out, (size_t)rows * 4);
+    turn.writes(rstd_out, (size_t)rows * 4);
+    BOATCU_RUN_IN_TURN((layernorm_fwd_rows_kernel<T, NV>), (unsigned)blocks, kNormThreads, smem, (const T*)x, rows, (int)cols, gamma, beta, eps, (T*)y,
+                       mean_out, rstd_out, turn.follow());
     BOATCU_LAUNCH_OK("layernorm_fwd_rows");
     return 0;
 }

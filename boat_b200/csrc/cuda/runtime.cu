@@ -36,6 +36,50 @@ int set_error(int status, const char* fmt, ...) {
 
 cudaStream_t stream() { return g_stream; }
 bool ready() { return g_ready; }
+// The launches that may still be running, as the ranges they named: the last kRelease launch and those beside it.
+struct NamedRange {
+    uintptr_t lo, hi;
+    bool written;
+};
+constexpr int kMaxRanges = 96;
+static std::mutex g_turn;                      // one launch at a time
+static NamedRange g_ranges[kMaxRanges];
+static int g_range_count = 0;                  // 0: the next launch is an ordinary one
+static bool g_range_overflow = false;          // the present launch touches more than the table holds
+static cudaStream_t g_range_stream = 0;
+
+LaunchTurn::LaunchTurn() : named_(false), beside_(false) {
+    g_turn.lock();
+    if (g_range_stream != g_stream) g_range_count = 0;
+    g_range_overflow = false;
+    before_ = g_range_count;
+}
+void LaunchTurn::name(const void* p, size_t bytes, bool written) {
+    named_ = true;
+    if (!p || bytes == 0) return;
+    if (g_range_count == kMaxRanges) g_range_overflow = true;
+    else g_ranges[g_range_count++] = NamedRange{(uintptr_t)p, (uintptr_t)p + bytes, written};
+}
+int LaunchTurn::follow() {
+    beside_ = before_ > 0 && !g_range_overflow;
+    for (int i = before_; i < g_range_count && beside_; ++i)
+        for (int j = 0; j < before_ && beside_; ++j)
+            beside_ = g_ranges[i].hi <= g_ranges[j].lo || g_ranges[j].hi <= g_ranges[i].lo || !(g_ranges[i].written || g_ranges[j].written);
+    return beside_ ? kBeside : kRelease;
+}
+LaunchTurn::~LaunchTurn() {
+    if (!named_ || g_range_overflow) {
+        g_range_count = 0;
+    } else if (!beside_) {                      // the kernels before are complete once this one lets go
+        for (int i = before_; i < g_range_count; ++i) g_ranges[i - before_] = g_ranges[i];
+        g_range_count -= before_;
+    }
+    g_range_stream = g_stream;
+    g_turn.unlock();
+}
+
+void ordinary_launch_next() { LaunchTurn turn; }
+
 void count_launch(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
 
 static int pick_device(int requested) {
@@ -293,6 +337,7 @@ void* boat_cuda_stream(void) { return (void*)g_stream; }
 int boat_cuda_set_stream(void* s) {
     std::lock_guard<std::mutex> lk(g_mu);
     // The old stream may be gone already: nothing is asked of it.
+    ordinary_launch_next();
     g_stream = (cudaStream_t)s;
     unsigned long long id = 0;
     g_stream_cached = g_stream != cudaStreamPerThread;
@@ -343,6 +388,7 @@ int boat_cuda_upload_async(void* dst, const void* src, size_t bytes) {
 
 int boat_cuda_join_uploads(void) {
     if (!g_up) return 0;
+    ordinary_launch_next();
     BOATCU_CHECK(cudaEventRecord(g_up_done, g_up));
     BOATCU_CHECK(cudaStreamWaitEvent(g_stream, g_up_done, 0));
     return 0;
@@ -426,6 +472,7 @@ uint64_t boat_cuda_launch_count(void) { return g_launches.load(); }
 int boat_cuda_memcpy_h2d(void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
+    ordinary_launch_next();
     BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g_stream));
     BOATCU_CHECK(cudaStreamSynchronize(g_stream));
     return 0;
@@ -434,6 +481,7 @@ int boat_cuda_memcpy_h2d(void* dst, const void* src, size_t bytes) {
 int boat_cuda_memcpy_h2d_async(void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
+    ordinary_launch_next();
     BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, g_stream));
     return 0;
 }
@@ -441,6 +489,7 @@ int boat_cuda_memcpy_h2d_async(void* dst, const void* src, size_t bytes) {
 int boat_cuda_memcpy_d2h(void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
+    ordinary_launch_next();
     BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, g_stream));
     BOATCU_CHECK(cudaStreamSynchronize(g_stream));
     return report_kernel_status("boat_cuda_memcpy_d2h");
@@ -449,6 +498,7 @@ int boat_cuda_memcpy_d2h(void* dst, const void* src, size_t bytes) {
 int boat_cuda_memcpy_d2d(void* dst, const void* src, size_t bytes) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
+    ordinary_launch_next();
     BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, g_stream));
     return 0;
 }
@@ -456,6 +506,7 @@ int boat_cuda_memcpy_d2d(void* dst, const void* src, size_t bytes) {
 int boat_cuda_memset(void* dst, int value, size_t bytes) {
     if (bytes == 0) return 0;
     if (int rc = ensure_init()) return rc;
+    ordinary_launch_next();
     BOATCU_CHECK(cudaMemsetAsync(dst, value, bytes, g_stream));
     return 0;
 }

@@ -242,6 +242,50 @@ def test_attention_core_with_several_items_per_cta(gpu_lib, hs, units, S, causal
         assert rel(got[key], ref[key]) <= 2e-2, key
 
 
+# Kernels that name their memory run beside one another when they touch nothing of each other's: a random sequence over
+# few buffers, where most neighbours do depend on each other - read after write, write after read, write after write, over
+# windows that overlap in part - gives the bits of the same sequence with a wait after every call.
+@pytest.mark.parametrize("mma", [capi.MMA_FP32, capi.MMA_BF16], ids=["fp32", "bf16"])
+@pytest.mark.parametrize("n", [64, 256])
+@pytest.mark.parametrize("seed", [0, 1, 2])
+def test_kernels_beside_one_another(gpu_lib, mma, n, seed):
+    bf = mma == capi.MMA_BF16
+    ty, es, count = (capi.CUDA_BF16, 2, 5) if bf else (capi.CUDA_F32, 4, 5)
+    first = rng.normal(8, seed, (count * n, n)) / np.float32(math.sqrt(n))
+
+    def play(wait):
+        pick = np.random.default_rng(seed)
+        block = DeviceBuffer.from_numpy(_bf(8, seed, (count * n, n), 1 / math.sqrt(n)) if bf else first, bf16=bf)
+        wide, grads = DeviceBuffer.from_numpy(first), DeviceBuffer(n * n * 4)
+        at = lambda rows: C.c_void_p(block.p.value + rows * n * es)
+        for _ in range(80):
+            # n rows each, from any eighth of the block: neighbours overlap in part
+            x, y, z = (int(r) * n // 8 for r in pick.choice(8 * (count - 1) + 1, 3, replace=False))
+            if abs(z - x) < n or abs(z - y) < n:            # a result over its own operand is no valid call
+                z = (max(x, y) + n) if max(x, y) + 2 * n <= count * n else min(x, y) - n
+                if z < 0 or abs(z - x) < n or abs(z - y) < n:
+                    continue
+            what = int(pick.integers(6))
+            if what < 3:
+                check(gpu_lib.boat_cuda_gemm(mma, int(what == 2), int(what == 1), n, n, n, at(x), n, at(y), n, ty, at(z), n, ty, None), "gemm")
+            elif what < 4 and not bf:                       # fresh values, so that products of products stay in range
+                check(gpu_lib.boat_cuda_lincomb(at(z), C.c_void_p(wide.p.value + x * n * 4), C.c_float(0.75), C.c_void_p(wide.p.value + y * n * 4),
+                                                C.c_float(-0.5), ty, n * n), "lincomb")
+            elif bf:
+                check(gpu_lib.boat_cuda_cast(at(z), ty, C.c_void_p(wide.p.value + x * n * 4), capi.CUDA_F32, n * n), "cast")
+            else:
+                check(gpu_lib.boat_cuda_weight_grads(mma, 1, n, n, n, (C.c_void_p * 1)(at(x).value), (C.c_void_p * 1)(at(y).value), ty,
+                                                     _table([grads]), None, 0), "dw")
+            if wait:
+                check(gpu_lib.boat_cuda_sync(), "sync")
+        check(gpu_lib.boat_cuda_sync(), "sync")
+        return block.numpy((count * n, n), bf16=bf), grads.numpy((n, n))
+
+    (a, ga), (b, gb) = play(False), play(True)
+    assert np.isfinite(b).mean() > 0.5
+    assert a.tobytes() == b.tobytes() and (bf or ga.tobytes() == gb.tobytes())
+
+
 # the staged TF32 backward: one key tile, two, the first that waits for a buffer used before, a remainder of one row
 @pytest.mark.parametrize("units,S", [(3, 40), (150, 256), (40, 385), (20, 1025)])
 @pytest.mark.parametrize("causal", [False, True], ids=["full", "causal"])
