@@ -264,6 +264,7 @@ template <typename T>
 struct BwdArgs {
     const T *Q, *K, *V, *dO;
     const float *lse, *delta;
+    const T* O;                      // not NULL: delta is not given, the CTAs make it from O and dO
     T *dQ, *dK, *dV;
     int units, S, hs, causal, vec;
     float scale;
@@ -288,7 +289,30 @@ __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile
     const T* w0 = (KEYS ? a.Q : a.K) + base;
     const T* w1 = (KEYS ? a.dO : a.V) + base;
     auto load_stats = [&](int q0, int buf) {
-        if (threadIdx.x < 2 * kRows) {
+        if (a.O) {
+            // delta of 64 query rows, TPR neighbouring threads per row
+            constexpr int TPR = C::THREADS / kRows;
+            const int r = threadIdx.x / TPR, part = threadIdx.x % TPR;
+            const int64_t at = base + (int64_t)(q0 + r) * hs;
+            float sum = 0.f;
+            if (q0 + r < S) {
+                if (sizeof(T) == 4 && a.vec) {
+                    for (int c = part; c < hs / 4; c += TPR) {
+                        const float4 x = reinterpret_cast<const float4*>(a.O + at)[c], y = reinterpret_cast<const float4*>(a.dO + at)[c];
+                        sum += x.x * y.x + x.y * y.y + x.z * y.z + x.w * y.w;
+                    }
+                } else {
+                    for (int c = part; c < hs; c += TPR) sum += to_f32(a.O[at + c]) * to_f32(a.dO[at + c]);
+                }
+            }
+#pragma unroll
+            for (int w = 1; w < TPR; w <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, w);
+            float* st = stat + buf * 2 * kRows;
+            if (part == 0) {
+                st[r] = q0 + r < S ? a.lse[sbase + q0 + r] : 0.f;
+                st[kRows + r] = sum;
+            }
+        } else if (threadIdx.x < 2 * kRows) {
             const int r = threadIdx.x & (kRows - 1);
             const float* src = threadIdx.x < kRows ? a.lse : a.delta;
             stat[buf * 2 * kRows + threadIdx.x] = q0 + r < S ? src[sbase + q0 + r] : 0.f;
@@ -299,13 +323,12 @@ __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile
         load_rows<HS, kRows, C::THREADS>(b, w0, j * kRows, S, hs, a.vec);
         load_rows<HS, kRows, C::THREADS>(b + C::FLOATS, w1, j * kRows, S, hs, a.vec);
         commit();
-        if (KEYS) load_stats(j * kRows, j & 1);
     };
     griddep_sync();
     load_rows<HS, OWN, C::THREADS>(own0, (KEYS ? a.K : a.Q) + base, r0, S, hs, a.vec);
     load_rows<HS, OWN, C::THREADS>(own1, (KEYS ? a.V : a.dO) + base, r0, S, hs, a.vec);
-    if (!KEYS) load_stats(r0, 0);
     fetch(first);
+    load_stats(KEYS ? first * kRows : r0, KEYS ? first & 1 : 0);
     float acc0[4][C::CPT], acc1[4][C::CPT];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -319,6 +342,7 @@ __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile
         wait_all();
         __syncthreads();
         if (C::BUFS == 2 && j + 1 < end) fetch(j + 1);
+        if (KEYS && !a.O && j + 1 < end) load_stats((j + 1) * kRows, (j + 1) & 1);
         const float* x0 = walk + (j % C::BUFS) * 2 * C::FLOATS;
         const float* x1 = x0 + C::FLOATS;
         float s[4][4], dp[4][4];
@@ -341,6 +365,8 @@ __device__ __forceinline__ void bwd_walk(const BwdArgs<T>& a, int unit, int tile
         accumulate<HS>(ds_s, x0, ty, tx, acc0);
         if (KEYS) accumulate<HS>(p_s, x1, ty, tx, acc1);
         __syncwarp();
+        // behind the tile's products: unlike the loads above, these are waited for
+        if (KEYS && a.O && j + 1 < end) load_stats((j + 1) * kRows, (j + 1) & 1);
     }
     if (KEYS) {
         store_rows<HS, T>(a.dK + base, r0, S, hs, ty, tx, acc0);
@@ -387,7 +413,7 @@ int launch_fwd_own(int64_t units, int64_t S, int hs, int causal, float scale, co
 
 template <int HS, int OWN, typename T>
 int launch_bwd_own(int64_t units, int64_t S, int hs, int causal, float scale, const void* Q, const void* K,
-               const void* V, const void* dO, const float* lse, const float* delta, void* dQ, void* dK, void* dV) {
+               const void* V, const void* O, const void* dO, const float* lse, const float* delta, void* dQ, void* dK, void* dV) {
     auto kern = attn_bwd_simt_kernel<HS, OWN, T>;
     constexpr int smem = Tiles<HS, OWN>::BWD_SMEM;
     static bool configured = false;
@@ -395,13 +421,14 @@ int launch_bwd_own(int64_t units, int64_t S, int hs, int causal, float scale, co
         BOATCU_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem > kSpreadSmem ? smem : kSpreadSmem));
         configured = true;
     }
-    const void* in[4] = {Q, K, V, dO};
+    const void* in[5] = {Q, K, V, dO, O ? O : dO};
     BwdArgs<T> a;
+    a.O = (const T*)O;
     a.Q = (const T*)Q; a.K = (const T*)K; a.V = (const T*)V; a.dO = (const T*)dO;
     a.lse = lse; a.delta = delta;
     a.dQ = (T*)dQ; a.dK = (T*)dK; a.dV = (T*)dV;
     a.units = (int)units; a.S = (int)S; a.hs = hs; a.causal = causal;
-    a.vec = rows_aligned(in, 4, hs, sizeof(T));
+    a.vec = rows_aligned(in, 5, hs, sizeof(T));
     a.scale = scale;
     const unsigned grid = (unsigned)(2 * units * ceil_div(S, OWN));
     BOATCU_RUN(kern, grid, OWN * 4, spread_smem(smem, grid), a);
@@ -454,13 +481,19 @@ int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale,
     DISPATCH_HS(launch_fwd, units, S, (int)hs, causal, scale, Q, K, V, O, lse);
 }
 
+// Up to two tiles the CTAs make delta themselves: they read O and dO once per walk, and a launch is saved.
+// Beyond, a pass of its own reads them once.  8 units of 64 x 16: 7.3 us with the pass, 6.2 without; 32 units of 250 x 32: 37.7 and
+// 38.8.
+bool attn_bwd_simt_makes_delta(int64_t S, int io_type) { return io_type == BOAT_CUDA_F32 && S <= 2 * kRows; }
+
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
-                  const void* V, const void* dO, const float* lse, const float* delta, int io_type, void* dQ,
+                  const void* V, const void* O, const void* dO, const float* lse, const float* delta, int io_type, void* dQ,
                   void* dK, void* dV) {
     if (units <= 0 || S <= 0 || hs <= 0) return 0;
     if (int rc = ensure_init()) return rc;
     if (int rc = check_shape(units, S, hs)) return rc;
-    DISPATCH_HS(launch_bwd, units, S, (int)hs, causal, scale, Q, K, V, dO, lse, delta, dQ, dK, dV);
+    const void* from = attn_bwd_simt_makes_delta(S, io_type) ? O : nullptr;
+    DISPATCH_HS(launch_bwd, units, S, (int)hs, causal, scale, Q, K, V, from, dO, lse, delta, dQ, dK, dV);
 }
 
 }  // namespace boatcu

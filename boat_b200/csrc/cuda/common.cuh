@@ -176,8 +176,10 @@ int gemm_simt_grouped(int trans_a, int trans_b, int groups, int64_t M, int64_t N
 int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count, bool add);
 int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, int io_type, void* O, float* lse);
+// Where attn_bwd_simt_makes_delta says so it works delta out from O and dO; else `delta` is given (rowdot).
+bool attn_bwd_simt_makes_delta(int64_t S, int io_type);
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
-                  const void* V, const void* dO, const float* lse, const float* delta, int io_type,
+                  const void* V, const void* O, const void* dO, const float* lse, const float* delta, int io_type,
                   void* dQ, void* dK, void* dV);
 
 // boat_cuda_attn_bwd with a say in the kernels: without `tensor_cores` the CUDA-core ones, whose scratch is

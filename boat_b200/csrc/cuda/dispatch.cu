@@ -197,7 +197,8 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
     float* delta = (float*)scratch;
     size_t delta_bytes = ((size_t)units * (size_t)S * sizeof(float) + 255) & ~(size_t)255;
     tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && aligned16({Q, K, V, O, dO, dQ, dK, dV}) && attn_tc_supported(mma, units, S, hs, io_type);
-    if (!(tensor_cores && mma == BOAT_MMA_BF16)) {      // the BF16 kernel's launcher makes its own, pre-scaled
+    // the BF16 kernel's launcher makes its own, pre-scaled
+    if (tensor_cores ? mma != BOAT_MMA_BF16 : !attn_bwd_simt_makes_delta(S, io_type)) {
         ProfileScope prof("attn_delta");
         if (int rc = rowdot(dO, O, io_type, units * S, hs, delta)) return rc;
     }
@@ -206,7 +207,7 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
                            (char*)scratch + delta_bytes, scratch_bytes - delta_bytes);
     {
         ProfileScope prof("attn_bwd_simt");
-        if (int rc = attn_bwd_simt(units, S, hs, causal, scale, Q, K, V, dO, lse, delta, io_type, dQ, dK, dV)) return rc;
+        if (int rc = attn_bwd_simt(units, S, hs, causal, scale, Q, K, V, O, dO, lse, delta, io_type, dQ, dK, dV)) return rc;
     }
     if (mma == BOAT_MMA_TF32) {
         const int64_t n = units * S * hs;

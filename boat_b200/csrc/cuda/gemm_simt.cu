@@ -13,9 +13,9 @@
 // the CTAs of a cluster, through distributed shared memory, each in a fixed order: the result does not
 // vary from run to run.  The column sums of B that a bias gradient wants come from the same pass.
 //
-// Before, with 4 x 4 outputs per thread: 1000 x 256 x 256 19.6 us, 4096 x 512 x 512 76 us (28 TFLOP/s),
-// 512 x 512 x 4096 (dW) 147 us; now 8.6,
-// 74 and 77 us.
+// 1000 x 256 x 256 takes 8.1 us, 4096 x 512 x 512 63 (34 TFLOP/s), 512 x 512 x 4096 (dW) 65; a register-only loop of these
+// multiply-adds reaches 57 TFLOP/s.  Stages of 64 along K where a warp has an eighth of them (8 between two barriers, not 4): 8.7 -> 8.1
+// us, three 512 x 512 x 4096 226 -> 198.
 #include "common.cuh"
 #include <cooperative_groups.h>
 #include <type_traits>
@@ -24,7 +24,6 @@ namespace boatcu {
 
 namespace {
 
-constexpr int kBK = 32;              // K per stage
 constexpr int kMaxGroups = 4;
 constexpr int kMaxSplit = 8;         // portable cluster size
 constexpr int kWarpM = 64, kWarpN = 32, kWarpTile = kWarpM * kWarpN;
@@ -66,7 +65,7 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(
 // operand is stored [K, X] and a tile is kBK rows of XT columns, else it is [X, K] and a tile is XT rows
 // of kBK columns.  What does not change along K is worked out once: with 16-byte copies a thread keeps
 // one column of every tile, so that a copy inside the matrix costs little more than itself.
-template <typename T, int XT, bool K_ROWS, int LD>
+template <typename T, int XT, bool K_ROWS, int LD, int kBK>
 struct TileLoader {
     static constexpr int ROWS = K_ROWS ? kBK : XT, COLS = K_ROWS ? XT : kBK;
     static constexpr int PER_ROW = COLS / 4, ROW_STEP = 256 / PER_ROW;
@@ -125,10 +124,11 @@ struct TileLoader {
 template <bool A_M, bool B_K, int WM, int WN>
 struct SimtTile {
     static constexpr int BM = kWarpM * WM, BN = kWarpN * WN, TILES = WM * WN, WK = 8 / TILES;
+    static constexpr int kBK = WK == 8 ? 64 : 32;         // K per stage
     static constexpr int LDA = A_M ? BM + 4 : kBK + 4, LDB = B_K ? kBK + 4 : BN + 4;
     static constexpr int A_FLOATS = A_M ? kBK * LDA : BM * LDA, B_FLOATS = B_K ? BN * LDB : kBK * LDB;
     static constexpr int STAGE = A_FLOATS + B_FLOATS;
-    static constexpr int STAGES = WK > 1 ? 4 : 3;
+    static constexpr int STAGES = WK > 1 && WK < 8 ? 4 : 3;
     static constexpr int PARTS = 8 * kWarpTile, SUMS = 8 * kWarpN;      // the partial tiles take the stages' place
     static constexpr int SMEM = (STAGES * STAGE > PARTS + SUMS ? STAGES * STAGE : PARTS + SUMS) * 4;
     static_assert(2 * (SMEM + 1024) <= 228 * 1024, "two CTAs per SM");
@@ -149,6 +149,7 @@ template <typename TI, typename TO, bool A_M, bool B_K, int WM, int WN>
 __global__ void __launch_bounds__(256, 2)
 gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     using S = SimtTile<A_M, B_K, WM, WN>;
+    constexpr int kBK = S::kBK;
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lm = lane >> 2, ln = lane & 3;
     const int wk = warp / S::TILES, wm = warp % S::TILES / WN, wn = warp % WN;
@@ -162,8 +163,8 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
     constexpr bool kSums = A_M && !B_K;                   // a weight gradient
     const bool sums = kSums && p.colsum[g] != nullptr && m0 == 0;
 
-    const TileLoader<TI, S::BM, A_M, S::LDA> load_a(A, p.lda, m0, p.M);
-    const TileLoader<TI, S::BN, !B_K, S::LDB> load_b(B, p.ldb, n0, p.N);
+    const TileLoader<TI, S::BM, A_M, S::LDA, kBK> load_a(A, p.lda, m0, p.M);
+    const TileLoader<TI, S::BN, !B_K, S::LDB, kBK> load_b(B, p.ldb, n0, p.N);
 
     const uint32_t smem_at = (uint32_t)__cvta_generic_to_shared(smem);
     float acc[8][8], bsum = 0.f;                          // bsum: column `lane` of the warp tile
@@ -383,14 +384,20 @@ template <typename TI, typename TO, bool A_M, bool B_K>
 int pick_tile(SimtParams& p, int groups) {
     const int64_t sms = sm_count();
     auto tiles = [&](int bm, int bn) { return ceil_div(p.M, bm) * ceil_div(p.N, bn); };
-    // The largest tile that still gives every SM one: larger ones fetch less per product, smaller ones
-    // leave no SM idle.  Where even 64 x 32 does not fill the GPU, K is split over a cluster too, at
-    // least 64 of it per CTA - and into two CTAs per SM where each still has 512: eight warps alone wait for
-    // one another's loads (512 x 512 x 4096 90 -> 77 us).  The order of the sum goes by the size of one problem alone, so that a
-    // group gives the bits of single calls.
-    if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value)
-        if (tiles(128, 128) >= sms) return launch_tile<TI, TO, A_M, B_K, 2, 4>(p, groups, 1);
+    // Larger tiles fetch less per product, smaller ones leave no SM idle.  128 x 128 pays from three quarters of the SMs on (4096 x
+    // 512 x 512, 128 of them: 63 us, 64 x 64 74; three such 175 and 202), 128 x 64 from six tenths (3000 x 256 x 256, 96: 19.8 and 21.0;
+    // three 34.9 and 40.8; but 1000 x 256 x 256, 32 of them: 20, 64 x 32 8.1).  Where 64 x 64 does not fill the GPU but does so with K cut
+    // in up to four, and 512 of it for each CTA of the cluster, that is next (512 x 512 x 4096 65 us, 64 x 32 69).  Else 64 x 32 with K
+    // split over a cluster, at least 64 of it per CTA - and into two CTAs per SM where each still has 512: eight warps alone wait for
+    // one another's loads.  The order of the sum goes by the size of one problem alone, so that a group gives the bits of single
+    // calls.
+    if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
+        if (tiles(128, 128) * 4 >= sms * 3) return launch_tile<TI, TO, A_M, B_K, 2, 4>(p, groups, 1);
+        if (tiles(128, 64) * 10 >= sms * 6) return launch_tile<TI, TO, A_M, B_K, 2, 2>(p, groups, 1);
+    }
     if (tiles(64, 64) >= sms) return launch_tile<TI, TO, A_M, B_K, 1, 2>(p, groups, 1);
+    const int in = tiles(64, 64) * 2 >= sms ? 2 : 4;
+    if (tiles(64, 64) * in >= sms && p.K / in >= 512) return launch_tile<TI, TO, A_M, B_K, 1, 2>(p, groups, in);
     int64_t split = sms / tiles(64, 32);
     const int64_t two = 2 * sms / tiles(64, 32) < p.K / 512 ? 2 * sms / tiles(64, 32) : p.K / 512;
     if (split < two) split = two;
