@@ -25,15 +25,14 @@
 // 128 that is all of it and dP^T borrows the dQ columns: the dQ warps take a tile's dQ into
 // registers and shared memory within a few hundred cycles of its completion, and the next dQ
 // product only comes after the softmax warps have consumed dP^T.  With head size 64 dP^T has 128
-// columns of its own.  In both cases dP^T is issued a tile ahead, S^T of tile t+1 follows dV of
-// tile t on the pipe, and the softmax warps - the critical resource - go from the exponentials
+// columns of its own, and P^T 64.  In both cases dP^T is issued a tile ahead, and S^T of tile t+1 follows dV of
+// tile t on the pipe - with head size 64 the softmax warps' taking of tile t's - so that those go from the exponentials
 // (A) straight to dS^T (B) without waiting for the tensor pipe.
 //
 // dQ of a query tile gets one contribution per key tile; CTAs add theirs into an FP32 buffer
 // with TMA reduce-add (cp.reduce.async.bulk.tensor), and a cast kernel turns the sum into the
-// output type afterwards.  Four dedicated warps move the dQ tile out of tensor memory through
-// the tile's dO stage, which is idle once the tile's MMAs are complete, half a tile at a time;
-// the thread that issues the reductions then loads the dO tile two steps ahead into it.  An SM
+// output type afterwards.  Four dedicated warps move the dQ tile out of tensor memory, through
+// a staging area or (head size 128) the tile's dO stage, which is idle once the tile's MMAs are complete.  An SM
 // gets reductions out at only about 20 bytes per clock (measured alike for TMA reduce-add and
 // for red.global.add.v4.f32, which also stalls the softmax warps' shared memory traffic), so
 // the read-out of a tile takes most of a tile period - off the critical path.
@@ -41,7 +40,7 @@
 // themselves inside a walk: the per-row statistics of a query tile (-lse*log2e and
 // -delta/sqrt(hs), pre-scaled by a small kernel) are brought in by the producer with two bulk
 // copies per tile.
-// Warp 0: TMA producer (K, V, Q, statistics), warp 1: MMA issuer, warps 2-9: softmax + final dK/dV store
+// Warp 0: TMA producer (K, V, Q, dO, statistics), warp 1: MMA issuer, warps 2-9: softmax + final dK/dV store
 // (two warps per TMEM lane group, 64 query columns each), warps 10-13: dQ reduction.
 #pragma once
 #include <type_traits>
@@ -170,7 +169,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     uint64_t* stat_empty = bars + 13;           // [2] phase B of the tile is over (256 arrivals)
     uint64_t* s_read = bars + 4;                // the softmax warps hold S^T (256 arrivals; head size 64)
     uint64_t* ds_empty = bars + 6;              // dK of the tile is complete: the dS^T tile may be overwritten (head size 64)
-    uint64_t* do_empty = bars + 48;             // [Q_STAGES] dP^T and dV of the tile are complete (head size 64)
+    uint64_t* do_empty = bars + 48;             // [Q_STAGES] the tile's dO is free: dP^T and dV complete, or (head size 128) dQ through it
     uint64_t* dp_read = bars + 15;              // ... and dP^T
     uint64_t* work_full = bars + 28;            // [kBwdAnswers] the answer to a request for work is there
     uint64_t* work_empty = bars + 32;           // [kBwdAnswers] producer, MMA issuer, softmax and dQ warps have read it
@@ -179,7 +178,6 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     // [2] dS^T in smem (256 arrivals).  Two in turn: with head size 64 dP^T of tile t+1 is issued before the wait for dS^T(t), so
     // dS^T(t+1) may be there by the time the MMA issuer gets to that wait.
     uint64_t* ds_full = bars + 46;
-    volatile uint32_t* drain_ok = tmem_slot + 3;       // outcome of the dQ warps' wait
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
@@ -193,7 +191,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
             mbar_init(&q_full[s], 1);
             mbar_init(&do_full[s], 1);
             mbar_init(&q_empty[s], 1);
-            mbar_init(&do_empty[s], 1);
+            mbar_init(&do_empty[s], C::DQ_BYTES ? 1 : 4);
         }
         mbar_init(s_full, 1);
         mbar_init(&ds_full[0], 256);
@@ -203,7 +201,7 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         mbar_init(p_full, 256);
         mbar_init(dp_full, 1);
         mbar_init(dq_full, 1);
-        mbar_init(dq_empty, C::DQ_BYTES ? 4 : 1);
+        mbar_init(dq_empty, 4);
         mbar_init(ds_empty, 1);
         mbar_init(all_done, 1);
         mbar_init(acc_free, 256);
@@ -282,12 +280,10 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
                     bulk_load_1d(stat_s + (t & 1) * 256, p.lse2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
                     bulk_load_1d(stat_s + (t & 1) * 256 + 128, p.delta2 + stat_base + i * kTile, 512, &stat_full[t & 1]);
                 }
-                if (C::DQ_BYTES) {
-                    if (!mbar_wait_warp(&do_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
-                    if (leader) {
-                        mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
-                        tma_load_3d(do_smem + s * C::TILE_BYTES, &map_do, &do_full[s], 0, i * kTile, w.unit);
-                    }
+                if (!mbar_wait_warp(&do_empty[s], ((t / C::Q_STAGES) & 1) ^ 1, p.status, kTimeoutProducer)) { ok = false; break; }
+                if (leader) {
+                    mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
+                    tma_load_4d(do_smem + s * C::TILE_BYTES, &map_do, &do_full[s], 0, i * kTile, 0, w.unit);
                 }
             }
             if (ok) w = next_walk(r, kTimeoutProducer, ok);
@@ -612,20 +608,21 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         w = next_walk(r_walk, kTimeoutSoftmax, ok);
         if (ok && w.n == 0) store_dkdv(unit_before, jt_before, r_walk & 1);
         }
-    } else if constexpr (C::DQ_BYTES != 0) {
-        // ---------------- dQ reduction, head size 64: warps 10..13, thread = query row ----------------
-        // Each warp by itself: its 32 rows of the tile from tensor memory to two boxes of its own (32 rows x 128 bytes) and
-        // from there, by TMA reduce-add, into the sum.  It waits for the reductions of the tile before to have read the
-        // boxes, and for nobody else.  All four warps through the tile's dO stage, with a barrier per step and the dO tiles
-        // loaded behind it, took 3300 cycles a tile, all of the tile's period: with scores and dP^T ahead 256 units of
-        // 2048 rows, causal, with preparation and cast took 541 us before and 519 now, 512 of 1024 518 and 503.  What bounds a
-        // tile now is shared memory (304 KB, 2375 cycles): without exponentials, statistics and reductions it still takes 460.
-        // (Tried on this: one half of the softmax warps half a tile behind the other 528; dS^T in tensor memory as dK's
-        // operand, in P^T's columns, 608.)
+    } else {
+        // ---------------- dQ reduction: warps 10..13, thread = query row ----------------
+        // Each warp by itself: its 32 rows of the tile, 64 columns at a time, from tensor memory to two boxes of its own (32
+        // rows x 128 bytes) and from there, by TMA reduce-add, into the sum.  With head size 64 the boxes are an area of their
+        // own; with 128 they are a quarter of the tile's dO stage, which is idle once the tile's MMAs are complete, and the
+        // stage is handed back to the producer when the four warps' reductions have read it.  The second 64 columns are
+        // taken into registers before anything else, since the next dP^T waits for the dQ columns.
+        // (All four warps in step, through 128-row boxes, with a barrier for each move and the dO tiles loaded behind it, took
+        // 3300 cycles a tile at head size 64, all of the tile's period: with scores and dP^T ahead 256 units of 2048 rows,
+        // causal, with preparation and cast took 541 us before and 519 now, 512 of 1024 518 and 503.  What bounds a tile
+        // there now is shared memory (304 KB, 2375 cycles): without exponentials, statistics and reductions it still takes
+        // 460.  Tried on this: one half of the softmax warps half a tile behind the other 528; dS^T in tensor memory as dK's
+        // operand, in P^T's columns, 608.  Head size 128, 64 units of 4096 rows: 783 and 765.)
         const int lane_group = warp & 3;
         const uint32_t t_dq = tmem_base + C::COL_DQ + ((uint32_t)(lane_group * 32) << 16);
-        uint8_t* const boxes = dq_smem + lane_group * (C::DQ_BYTES / 4);
-        uint8_t* const row = boxes + lane * 128;
         const int swz = lane & 7;
         const bool leader = elect_one();
         bool ok = true;
@@ -633,30 +630,63 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         BwdWalk w = bwd_walk(p, blockIdx.x);
         for (int r_walk = 0; ok && w.n > 0; ++r_walk) {
             for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
+                const int s = t % C::Q_STAGES, y = i * kTile + lane_group * 32;
+                uint8_t* const boxes = (C::DQ_BYTES ? dq_smem : do_smem + s * C::TILE_BYTES) + lane_group * 8192;
+                uint32_t v[2][32];
+                auto take = [&](int col) {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) tmem_ld32(t_dq + col + b * 32, v[b]);
+                    tmem_wait_ld();
+                };
+                auto stage = [&] {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+#pragma unroll
+                        for (int u = 0; u < 8; ++u)
+                            *reinterpret_cast<uint4*>(boxes + b * 4096 + lane * 128 + ((u ^ swz) << 4)) = make_uint4(v[b][4 * u], v[b][4 * u + 1], v[b][4 * u + 2], v[b][4 * u + 3]);
+                };
+                auto send = [&](int col) {                   // by the leader
+                    if (y < p.S) {
+#pragma unroll
+                        for (int b = 0; b < 2; ++b) tma_reduce_add_3d(&map_dq, boxes + b * 4096, col + b * 32, y, w.unit);
+                    }
+                    tma_commit_group();
+                };
                 if (!mbar_wait_warp(dq_full, t & 1, p.status, kTimeoutOther)) { ok = false; break; }
                 tc_fence_after_sync();
-                uint32_t v[HS / 32][32];
-#pragma unroll
-                for (int b = 0; b < HS / 32; ++b) tmem_ld32(t_dq + b * 32, v[b]);
-                tmem_wait_ld();
-                tc_fence_before_sync();
-                __syncwarp();
-                if (leader) {
-                    mbar_arrive(dq_empty);                   // this warp's part of the dQ columns is free
-                    tma_wait_group_read0();
-                }
-                __syncwarp();
-#pragma unroll
-                for (int b = 0; b < HS / 32; ++b)
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        *reinterpret_cast<uint4*>(row + b * 4096 + ((u ^ swz) << 4)) = make_uint4(v[b][4 * u], v[b][4 * u + 1], v[b][4 * u + 2], v[b][4 * u + 3]);
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (leader && i * kTile + lane_group * 32 < p.S) {
-#pragma unroll
-                    for (int b = 0; b < HS / 32; ++b) tma_reduce_add_3d(&map_dq, boxes + b * 4096, b * 32, i * kTile + lane_group * 32, w.unit);
-                    tma_commit_group();
+                take(0);
+                if (C::DQ_BYTES) {
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (leader) {
+                        mbar_arrive(dq_empty);               // this warp's part of the dQ columns is free
+                        tma_wait_group_read0();
+                    }
+                    __syncwarp();
+                    stage();
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (leader) send(0);
+                } else {
+                    stage();
+                    take(64);
+                    tc_fence_before_sync();
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (leader) {
+                        mbar_arrive(dq_empty);
+                        send(0);
+                        tma_wait_group_read0();
+                    }
+                    __syncwarp();
+                    stage();
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (leader) {
+                        send(64);
+                        tma_wait_group_read0();
+                        mbar_arrive(&do_empty[s]);
+                    }
                 }
             }
             if (!ok) break;
@@ -665,121 +695,6 @@ attn_bwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
         // The CTA may end once the reductions have read their shared-memory source; that they have
         // landed in global memory by the time the next kernel runs is the grid's completion.
         if (leader) tma_wait_group_read0();
-    } else {
-        // ---------------- dQ reduction: warps 10..13, thread = query row ----------------
-        // The FP32 dQ tile is HS/32 boxes of 128 rows x 128 bytes (16 KB each), twice what the tile's
-        // dO stage holds - the stage is idle once the tile's MMAs are complete and serves as the
-        // staging area, one box per slot.  The first half of the boxes goes straight through their
-        // slots; the second half is taken into registers at once (which frees the tensor-memory
-        // columns) and follows box by box, each as soon as the reduction that used its slot has
-        // been read out - so the TMA unit always has the next box queued behind the one it is
-        // reading.  The dO tile two steps ahead is then loaded slot by slot on the same terms.
-        const int lane_group = warp & 3;
-        const int r = lane_group * 32 + lane;
-        const bool issuer = warp == 10;                      // this warp issues, one elected lane of it
-        const bool leader = elect_one();
-        const uint32_t lane_addr = (uint32_t)(lane_group * 32) << 16;
-        const int swz = r & 7;
-        // all but the most recent n reduction groups of this thread have been read out of shared memory
-        auto wait_read = [](int n) {
-            if (n == 0) tma_wait_group_read0();
-            else tma_wait_group_read1();
-        };
-        // dO tiles: the first Q_STAGES are loaded here, every later one into the stage of the tile
-        // Q_STAGES before it
-        int ahead_r = 0, ahead_i = 0;                        // walk and tile of the next dO load
-        BwdWalk ahead = bwd_walk(p, blockIdx.x);
-        auto load_do = [&](uint32_t t_load, auto before_box) {       // by the whole issuing warp
-            if (ahead.n == 0) return;
-            const int s = t_load % C::Q_STAGES;
-            if (leader) {
-                mbar_arrive_expect_tx(&do_full[s], C::TILE_BYTES);
-#pragma unroll
-                for (int b = 0; b < C::NBOX; ++b) {
-                    before_box(b);
-                    tma_load_3d(do_smem + s * C::TILE_BYTES + b * kBoxBytes, &map_do, &do_full[s], b * 64, (ahead.i0 + ahead_i) * kTile, ahead.unit);
-                }
-            }
-            if (++ahead_i == ahead.n) {
-                // ahead of the warp's own reading of this answer, so it is still there
-                const int a = ahead_r % kBwdAnswers;
-                const bool there = mbar_wait_warp(&work_full[a], (ahead_r / kBwdAnswers) & 1, p.status, kTimeoutOther);
-                ahead = bwd_walk(p, there ? taken_cta(answers + a * 16) : -1);
-                ahead_i = 0;
-                ++ahead_r;
-            }
-        };
-        if (issuer)
-            for (uint32_t t0 = 0; t0 < C::Q_STAGES; ++t0) load_do(t0, [](int) {});
-        __syncwarp();
-        bool ok = true;
-        uint32_t t = 0;                                      // tiles so far, of all walks
-        BwdWalk w = bwd_walk(p, blockIdx.x);
-        for (int r_walk = 0; ok && w.n > 0; ++r_walk) {
-        for (int i = w.i0; i < w.i0 + w.n; ++i, ++t) {
-            const int s = t % C::Q_STAGES;
-            if (issuer) {
-                const bool there = mbar_wait_warp(dq_full, t & 1, p.status, kTimeoutOther);
-                if (leader) drain_ok[0] = there ? 1u : 0u;
-            }
-            named_barrier_sync(2, 128);
-            if (drain_ok[0] == 0u) { ok = false; break; }
-            tc_fence_after_sync();
-            const int y = i * kTile;
-            uint8_t* stage = do_smem + s * C::TILE_BYTES;
-            auto stage_box = [&](const uint32_t (&v)[32], int slot) {
-                uint8_t* row = stage + slot * kBoxBytes + r * 128;
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    *reinterpret_cast<uint4*>(row + ((u ^ swz) << 4)) = make_uint4(v[4 * u], v[4 * u + 1], v[4 * u + 2], v[4 * u + 3]);
-            };
-            uint32_t v[C::NBOX][32];
-            // boxes 0 .. NBOX-1: tensor memory -> registers -> their slots -> one reduction group each
-#pragma unroll
-            for (int b = 0; b < C::NBOX; ++b) tmem_ld32(tmem_base + C::COL_DQ + lane_addr + b * 32, v[b]);
-            tmem_wait_ld();
-#pragma unroll
-            for (int b = 0; b < C::NBOX; ++b) stage_box(v[b], b);
-            fence_proxy_async_smem();
-            named_barrier_sync(2, 128);
-            if (issuer && leader) {
-#pragma unroll
-                for (int b = 0; b < C::NBOX; ++b) {
-                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, b * 32, y, w.unit);
-                    tma_commit_group();
-                }
-            }
-            // boxes NBOX .. 2*NBOX-1 wait in registers; the TMEM columns are free as soon as they are loaded
-#pragma unroll
-            for (int b = 0; b < C::NBOX; ++b)
-                tmem_ld32(tmem_base + C::COL_DQ + lane_addr + (C::NBOX + b) * 32, v[b]);
-            tmem_wait_ld();
-            tc_fence_before_sync();
-            named_barrier_sync(2, 128);                     // everybody holds the second half
-            if (issuer && leader) mbar_arrive(dq_empty);    // the dQ columns are free
-#pragma unroll
-            for (int b = 0; b < C::NBOX; ++b) {
-                // slot b was last used by the group issued NBOX groups ago
-                if (issuer && leader) wait_read(C::NBOX - 1);
-                named_barrier_sync(2, 128);                 // slot b has been read
-                stage_box(v[b], b);
-                fence_proxy_async_smem();
-                named_barrier_sync(2, 128);
-                if (issuer && leader) {
-                    tma_reduce_add_3d(&map_dq, stage + b * kBoxBytes, (C::NBOX + b) * 32, y, w.unit);
-                    tma_commit_group();
-                }
-            }
-            // the last group that used slot b has been read
-            if (issuer) load_do(t + C::Q_STAGES, [&](int b) { wait_read(C::NBOX - 1 - b); });
-            __syncwarp();
-        }
-        if (!ok) break;
-        w = next_walk(r_walk, kTimeoutOther, ok);
-        }
-        // The CTA may end once the reductions have read their shared-memory source; that they have
-        // landed in global memory by the time the next kernel runs is the grid's completion.
-        if (issuer && leader) tma_wait_group_read0();
     }
     tc_fence_before_sync();
     __syncthreads();

@@ -86,8 +86,8 @@ int launch_bwd(int64_t units, int64_t S, int causal, float scale, const void* Q,
     if (int rc = make_tensor_map_unit_tiles(&mq, Q, 2, units, S, HS, kTile)) return rc;
     if (int rc = make_tensor_map_unit_tiles(&mk, K, 2, units, S, HS, kTile)) return rc;
     if (int rc = make_tensor_map_unit_tiles(&mv, V, 2, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mdo, dO, 2, units, S, HS, kTile)) return rc;
-    if (int rc = make_tensor_map_units(&mdq, dq_accum, 4, units, S, HS, C::DQ_BYTES ? 32 : kTile)) return rc;   // FP32 reduce-add target
+    if (int rc = make_tensor_map_unit_tiles(&mdo, dO, 2, units, S, HS, kTile)) return rc;
+    if (int rc = make_tensor_map_units(&mdq, dq_accum, 4, units, S, HS, 32)) return rc;   // FP32 reduce-add target
     const size_t n = (size_t)units * (size_t)S * HS;
     BwdParams p;
     p.lse2 = stats2;
