@@ -127,7 +127,8 @@ __device__ __forceinline__ void bwd32_dq(uint8_t* smem, int block, const CUtenso
     uint8_t* v_smem = k_smem + kBwd32Tile;           // [2]
     uint8_t* kmn_smem = v_smem + 2 * kBwd32Tile;     // [2] K read along the key rows (dQ)
     uint64_t* bars = (uint64_t*)(smem + 7 * kBwd32Tile + 2048);
-    uint64_t* q_full = bars;            // Q and dO landed
+    uint64_t* q_full = bars;            // Q landed
+    uint64_t* do_full = bars + 1;       // dO landed
     uint64_t* k_full = bars + 2;        // K landed
     uint64_t* k_empty = bars + 3;       // ... and the tile's S is complete
     uint64_t* v_full = bars + 4;        // [2]
@@ -183,12 +184,10 @@ __device__ __forceinline__ void bwd32_dq(uint8_t* smem, int block, const CUtenso
             ok = mbar_wait_warp(&kmn_empty[j & 1], ((j >> 1) & 1) ^ 1, p.status, kTimeoutProducer);
             if (ok && leader) bwd32_load(kmn_smem + (j & 1) * kBwd32Tile, &map_k_mn, &kmn_full[j & 1], j * kTile, unit);
         };
-        if (leader) {
-            mbar_arrive_expect_tx(q_full, 2 * kBwd32Tile);
-            tma_load_4d(q_smem, &map_q, q_full, 0, qt * kTile, 0, unit);
-            tma_load_4d(do_smem, &map_do, q_full, 0, qt * kTile, 0, unit);
-        }
+        // what the first product wants comes first
+        if (leader) bwd32_load(q_smem, &map_q, q_full, qt * kTile, unit);
         load_k(0);
+        if (leader) bwd32_load(do_smem, &map_do, do_full, qt * kTile, unit);
         load_v(0);
         load_kmn(0);
         load_v(1);
@@ -231,6 +230,7 @@ __device__ __forceinline__ void bwd32_dq(uint8_t* smem, int block, const CUtenso
             }
         };
         issue_s(0);
+        ok = ok && mbar_wait_warp(do_full, 0, p.status, kTimeoutMma);
         issue_dp(0);
         issue_s(1);
         for (int j = 0; j < n_kv && ok; ++j) {
@@ -319,7 +319,8 @@ __device__ __forceinline__ void bwd32_dkv(uint8_t* smem, int block, const CUtens
     uint8_t* do_smem = domn_smem + kBwd32Tile;       // [2] dO read along hs (dP)
     float* stat_s = (float*)(smem + 7 * kBwd32Tile); // [2][-lse*log2e [128], -delta/sqrt(hs) [128]]
     uint64_t* bars = (uint64_t*)(stat_s + 512);
-    uint64_t* kv_full = bars;
+    uint64_t* k_full = bars;
+    uint64_t* v_full = bars + 18;
     uint64_t* q_full = bars + 1;
     uint64_t* q_empty = bars + 2;       // S^T of the tile complete
     uint64_t* qmn_full = bars + 3;
@@ -335,7 +336,7 @@ __device__ __forceinline__ void bwd32_dkv(uint8_t* smem, int block, const CUtens
     uint64_t* p_full = bars + 14;       // [2]
     uint64_t* ds_full = bars + 16;      // dS^T written over dP^T (256 arrivals)
     uint64_t* acc_done = bars + 17;     // last dV, dK MMAs complete
-    uint32_t* tmem_slot = (uint32_t*)(bars + 18);
+    uint32_t* tmem_slot = (uint32_t*)(bars + 19);
 
     const int warp = warp_index(), lane = threadIdx.x & 31;
     const int n_tiles = (p.S + kTile - 1) / kTile;
@@ -345,7 +346,7 @@ __device__ __forceinline__ void bwd32_dkv(uint8_t* smem, int block, const CUtens
     const int n_q = n_tiles - i0;
 
     if (threadIdx.x == 0) {
-        for (int b = 0; b < 18; ++b) mbar_init(&bars[b], &bars[b] >= p_full && &bars[b] <= ds_full ? kBwd32Softmax : 1);
+        for (int b = 0; b < 19; ++b) mbar_init(&bars[b], &bars[b] >= p_full && &bars[b] <= ds_full ? kBwd32Softmax : 1);
         fence_barrier_init();
         tma_prefetch_desc(&map_q);
         tma_prefetch_desc(&map_q_mn);
@@ -375,12 +376,10 @@ __device__ __forceinline__ void bwd32_dkv(uint8_t* smem, int block, const CUtens
         auto load_qmn = [&](int t) { load(t, qmn_smem, &map_q_mn, qmn_full, qmn_empty, t & 1); };
         auto load_domn = [&](int t) { load(t, domn_smem, &map_do_mn, domn_full, domn_empty, t & 1); };
         auto load_do = [&](int t) { load(t, do_smem + (t & 1) * kBwd32Tile, &map_do, &do_full[t & 1], &do_empty[t & 1], (t >> 1) & 1); };
-        if (leader) {
-            mbar_arrive_expect_tx(kv_full, 2 * kBwd32Tile);
-            tma_load_4d(k_smem, &map_k, kv_full, 0, jt * kTile, 0, unit);
-            tma_load_4d(v_smem, &map_v, kv_full, 0, jt * kTile, 0, unit);
-        }
+        // what the first product wants comes first
+        if (leader) bwd32_load(k_smem, &map_k, k_full, jt * kTile, unit);
         load_q(0);
+        if (leader) bwd32_load(v_smem, &map_v, v_full, jt * kTile, unit);
         load_do(0);
         load_domn(0);
         load_qmn(0);
@@ -400,7 +399,7 @@ __device__ __forceinline__ void bwd32_dkv(uint8_t* smem, int block, const CUtens
         const uint64_t q_d = smem_desc_sw128(smem_u32(q_smem), 16, 1024), do_d = smem_desc_sw128(smem_u32(do_smem), 16, 1024);
         const uint64_t q_mn = smem_desc_mn(smem_u32(qmn_smem), kBoxBytes, true), do_mn = smem_desc_mn(smem_u32(domn_smem), kBoxBytes, true);
         const bool leader = elect_one();
-        bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutMma);
+        bool ok = mbar_wait_warp(k_full, 0, p.status, kTimeoutMma);
         auto issue_s = [&](int t) {
             if (!ok || t >= n_q) return;
             ok = mbar_wait_warp(q_full, t & 1, p.status, kTimeoutMma);
@@ -424,6 +423,7 @@ __device__ __forceinline__ void bwd32_dkv(uint8_t* smem, int block, const CUtens
             }
         };
         issue_s(0);
+        ok = ok && mbar_wait_warp(v_full, 0, p.status, kTimeoutMma);
         issue_dp(0);
         issue_s(1);
         for (int t = 0; t < n_q && ok; ++t) {

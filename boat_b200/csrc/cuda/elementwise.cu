@@ -30,8 +30,8 @@ __device__ __forceinline__ float mul_add(float alpha, float x, float y) { return
 
 // ---- y = alpha*x (+ y), 4 floats per access -------------------------------------------
 template <bool ACCUM>
-__global__ void axpy_vec4(float* __restrict__ y, const float* __restrict__ x, float alpha, int64_t n4) {
-    griddep_sync();
+__global__ void axpy_vec4(float* __restrict__ y, const float* __restrict__ x, float alpha, int64_t n4, int follow) {
+    griddep_enter(follow);
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     float4* y4 = reinterpret_cast<float4*>(y);
@@ -47,24 +47,30 @@ __global__ void axpy_vec4(float* __restrict__ y, const float* __restrict__ x, fl
         }
         y4[i] = r;
     }
+    griddep_leave(follow);
 }
 
 template <bool ACCUM>
-__global__ void axpy_scalar(float* __restrict__ y, const float* __restrict__ x, float alpha, int64_t n) {
-    griddep_sync();
+__global__ void axpy_scalar(float* __restrict__ y, const float* __restrict__ x, float alpha, int64_t n, int follow) {
+    griddep_enter(follow);
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     int64_t step = (int64_t)gridDim.x * blockDim.x;
     for (; i < n; i += step) y[i] = ACCUM ? mul_add(alpha, x[i], y[i]) : alpha * x[i];
+    griddep_leave(follow);
 }
 
 template <bool ACCUM>
 static int launch_axpy(float* y, const float* x, float alpha, int64_t n) {
     if (n <= 0) return 0;
     if (int rc = ensure_init()) return rc;
+    LaunchTurn turn;
+    turn.reads(x, (size_t)n * 4);
+    turn.writes(y, (size_t)n * 4);
+    const int follow = turn.follow();
     if (aligned16(y) && aligned16(x) && (n % 4) == 0) {
-        BOATCU_RUN(axpy_vec4<ACCUM>, grid_for(n / 4, kThreads), kThreads, 0, y, x, alpha, n / 4);
+        BOATCU_RUN_IN_TURN(axpy_vec4<ACCUM>, grid_for(n / 4, kThreads), kThreads, 0, y, x, alpha, n / 4, follow);
     } else {
-        BOATCU_RUN(axpy_scalar<ACCUM>, grid_for(n, kThreads), kThreads, 0, y, x, alpha, n);
+        BOATCU_RUN_IN_TURN(axpy_scalar<ACCUM>, grid_for(n, kThreads), kThreads, 0, y, x, alpha, n, follow);
     }
     BOATCU_LAUNCH_OK("axpy");
     return 0;
