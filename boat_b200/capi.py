@@ -227,6 +227,7 @@ PROTOTYPES = {
     "boat_cuda_gemm_set_yielding": (_I, [_I]),
     "boat_cuda_gemm_grouped": (_I, [_I, _I, _I, _I, _I64, _I64, _I64, _P, _I64, _P, _I64, _I, _P, _I64, _I, _P]),
     "boat_cuda_gemm_fused": (_I, [_I, _I, _I, _I, _I64, _I64, _I64, _P, _I64, _P, _I64, _I, _P, _I64, _P, _P]),
+    "boat_cuda_linear_grads": (_I, [_I, _I, _I64, _I64, _I64, _P, _P, _P, _P, _P, _P]),
     "boat_cuda_gemm_sum": (_I, [_I, _I, _I, _I, _I64, _I64, _I64, _P, _I64, _P, _I64, _I, _P, _I64, _I]),
     "boat_cuda_weight_grads": (_I, [_I, _I, _I64, _I64, _I64, _P, _P, _I, _P, _P, _I]),
     "boat_cuda_colsum": (_I, [_P, _I, _I64, _I64, _P]),

@@ -172,6 +172,9 @@ int attn_bwd_prepare(const void* dO, const void* O, const float* lse, int64_t un
 int gemm_simt_grouped(int trans_a, int trans_b, int groups, int64_t M, int64_t N, int64_t K, const void* const* A,
                       int64_t lda, const void* const* B, int64_t ldb, int in_type, void* const* C, int64_t ldc,
                       int out_type, const float* const* bias, float* const* colsum, bool add = false);
+// boat_cuda_linear_grads in FP32 on the CUDA cores, for problems so small that one launch is worth it; 13 for others.
+int gemm_simt_grads(int groups, int64_t T, int64_t I, int64_t O, const void* const* X, const void* const* dY, const void* const* W,
+                    void* const* dX, float* const* dW, float* const* db);
 // boat_cuda_colsum_multi, with `add` adding to the outputs.
 int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count, bool add);
 int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,

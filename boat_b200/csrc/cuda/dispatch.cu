@@ -145,6 +145,17 @@ int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T,
     return sums ? colsum_multi(dY, in_type, T, O, db, groups, false) : 0;
 }
 
+int boat_cuda_linear_grads(int mma, int groups, int64_t T, int64_t I, int64_t O, const void* const* X, const void* const* dY,
+                           const void* const* W, void* const* dX, float* const* dW, float* const* db) {
+    if (groups < 1 || groups > 4) return set_error(11, "boat_cuda_linear_grads: %d groups (1 to 4)", groups);
+    if (!X || !dY || !W || !dX || !dW) return set_error(11, "boat_cuda_linear_grads: NULL operand table");
+    if (mma != BOAT_MMA_FP32 || T <= 0 || I <= 0 || O <= 0) return 13;
+    for (int g = 0; g < groups; ++g)
+        if (!X[g] || !dY[g] || !W[g] || !dX[g] || !dW[g]) return set_error(11, "boat_cuda_linear_grads: NULL operand");
+    ProfileScope prof("gemm_simt");
+    return gemm_simt_grads(groups, T, I, O, X, dY, W, dX, dW, db);
+}
+
 int boat_cuda_attn_fwd(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q,
                        const void* K, const void* V, int io_type, void* O, float* lse) {
     if (int rc = check_types("boat_cuda_attn_fwd", mma, io_type)) return rc;

@@ -145,16 +145,15 @@ template <int N> __device__ __forceinline__ void load_shared(float (&v)[N], cons
     }
 }
 
+// CTA `block` of problem g.  Where K is split, the blocks of one tile are the CTAs of a cluster.
 template <typename TI, typename TO, bool A_M, bool B_K, int WM, int WN>
-__global__ void __launch_bounds__(256, 2)
-gemm_simt_kernel(const __grid_constant__ SimtParams p) {
+__device__ __forceinline__ void simt_tile(const SimtParams& p, int block, int g, float* smem) {
     using S = SimtTile<A_M, B_K, WM, WN>;
     constexpr int kBK = S::kBK;
-    extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lm = lane >> 2, ln = lane & 3;
     const int wk = warp / S::TILES, wm = warp % S::TILES / WN, wn = warp % WN;
-    const int g = blockIdx.z, split = p.split;
-    const int ks = blockIdx.x % split, tile = blockIdx.x / split;
+    const int split = p.split;
+    const int ks = block % split, tile = block / split;
     const int64_t m0 = (int64_t)(tile / p.n_tiles) * S::BM, n0 = (int64_t)(tile % p.n_tiles) * S::BN;
     const TI* A = (const TI*)p.A[g];
     const TI* B = (const TI*)p.B[g];
@@ -351,6 +350,37 @@ gemm_simt_kernel(const __grid_constant__ SimtParams p) {
 }
 
 template <typename TI, typename TO, bool A_M, bool B_K, int WM, int WN>
+__global__ void __launch_bounds__(256, 2)
+gemm_simt_kernel(const __grid_constant__ SimtParams p) {
+    extern __shared__ __align__(16) float smem[];
+    simt_tile<TI, TO, A_M, B_K, WM, WN>(p, blockIdx.x, blockIdx.z, smem);
+}
+
+// The weight gradients of a few small projections and, behind them, their input gradients, which read the same dY: one
+// launch instead of two.  dw_blocks, dx_blocks: CTAs per group.
+__global__ void __launch_bounds__(256, 2)
+gemm_simt_grads_kernel(const __grid_constant__ SimtParams dw, const __grid_constant__ SimtParams dx, int groups, int dw_blocks, int dx_blocks) {
+    extern __shared__ __align__(16) float smem[];
+    int b = blockIdx.x;
+    if (b < groups * dw_blocks) {
+        simt_tile<float, float, true, false, 1, 1>(dw, b % dw_blocks, b / dw_blocks, smem);
+        return;
+    }
+    b -= groups * dw_blocks;
+    if (b < groups * dx_blocks) simt_tile<float, float, false, true, 1, 1>(dx, b % dx_blocks, b / dx_blocks, smem);
+}
+
+void name_memory(LaunchTurn& turn, const SimtParams& p, int groups, bool a_m, bool b_k, size_t in_size, size_t out_size) {
+    for (int g = 0; g < groups; ++g) {
+        turn.reads(p.A[g], a_m ? p.K : p.M, a_m ? p.M : p.K, p.lda, in_size);
+        turn.reads(p.B[g], b_k ? p.N : p.K, b_k ? p.K : p.N, p.ldb, in_size);
+        turn.writes(p.C[g], p.M, p.N, p.ldc, out_size);
+        turn.reads(p.bias[g], (size_t)p.N * 4);
+        turn.writes(p.colsum[g], (size_t)p.N * 4);
+    }
+}
+
+template <typename TI, typename TO, bool A_M, bool B_K, int WM, int WN>
 int launch_tile(SimtParams& p, int groups, int split) {
     using S = SimtTile<A_M, B_K, WM, WN>;
     auto kern = gemm_simt_kernel<TI, TO, A_M, B_K, WM, WN>;
@@ -366,13 +396,7 @@ int launch_tile(SimtParams& p, int groups, int split) {
     const int smem = spread_smem(S::SMEM, tiles * split * groups);
     {
         LaunchTurn turn;
-        for (int g = 0; g < groups; ++g) {
-            turn.reads(p.A[g], A_M ? p.K : p.M, A_M ? p.M : p.K, p.lda, sizeof(TI));
-            turn.reads(p.B[g], B_K ? p.N : p.K, B_K ? p.K : p.N, p.ldb, sizeof(TI));
-            turn.writes(p.C[g], p.M, p.N, p.ldc, sizeof(TO));
-            turn.reads(p.bias[g], (size_t)p.N * 4);
-            turn.writes(p.colsum[g], (size_t)p.N * 4);
-        }
+        name_memory(turn, p, groups, A_M, B_K, sizeof(TI), sizeof(TO));
         p.follow = turn.follow();
         BOATCU_CHECK(launch_in_turn(kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), smem, (unsigned)split, p));
     }
@@ -380,10 +404,12 @@ int launch_tile(SimtParams& p, int groups, int split) {
     return 0;
 }
 
-template <typename TI, typename TO, bool A_M, bool B_K>
-int pick_tile(SimtParams& p, int groups) {
+struct Choice { int wm, wn, split; };
+
+// Tile and split of K for an M x N x K problem; fp32: FP32 in and out.
+Choice choose(int64_t M, int64_t N, int64_t K, bool fp32) {
     const int64_t sms = sm_count();
-    auto tiles = [&](int bm, int bn) { return ceil_div(p.M, bm) * ceil_div(p.N, bn); };
+    auto tiles = [&](int bm, int bn) { return ceil_div(M, bm) * ceil_div(N, bn); };
     // Larger tiles fetch less per product, smaller ones leave no SM idle.  128 x 128 pays from three quarters of the SMs on (4096 x
     // 512 x 512, 128 of them: 63 us, 64 x 64 74; three such 175 and 202), 128 x 64 from six tenths (3000 x 256 x 256, 96: 19.8 and 21.0;
     // three 34.9 and 40.8; but 1000 x 256 x 256, 32 of them: 20, 64 x 32 8.1).  Where 64 x 64 does not fill the GPU but does so with K cut
@@ -391,20 +417,30 @@ int pick_tile(SimtParams& p, int groups) {
     // split over a cluster, at least 64 of it per CTA - and into two CTAs per SM where each still has 512: eight warps alone wait for
     // one another's loads.  The order of the sum goes by the size of one problem alone, so that a group gives the bits of single
     // calls.
-    if constexpr (std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
-        if (tiles(128, 128) * 4 >= sms * 3) return launch_tile<TI, TO, A_M, B_K, 2, 4>(p, groups, 1);
-        if (tiles(128, 64) * 10 >= sms * 6) return launch_tile<TI, TO, A_M, B_K, 2, 2>(p, groups, 1);
-    }
-    if (tiles(64, 64) >= sms) return launch_tile<TI, TO, A_M, B_K, 1, 2>(p, groups, 1);
+    if (fp32 && tiles(128, 128) * 4 >= sms * 3) return {2, 4, 1};
+    if (fp32 && tiles(128, 64) * 10 >= sms * 6) return {2, 2, 1};
+    if (tiles(64, 64) >= sms) return {1, 2, 1};
     const int in = tiles(64, 64) * 2 >= sms ? 2 : 4;
-    if (tiles(64, 64) * in >= sms && p.K / in >= 512) return launch_tile<TI, TO, A_M, B_K, 1, 2>(p, groups, in);
+    if (tiles(64, 64) * in >= sms && K / in >= 512) return {1, 2, in};
     int64_t split = sms / tiles(64, 32);
-    const int64_t two = 2 * sms / tiles(64, 32) < p.K / 512 ? 2 * sms / tiles(64, 32) : p.K / 512;
+    const int64_t two = 2 * sms / tiles(64, 32) < K / 512 ? 2 * sms / tiles(64, 32) : K / 512;
     if (split < two) split = two;
-    if (split > p.K / 64) split = p.K / 64;
+    if (split > K / 64) split = K / 64;
     if (split > kMaxSplit) split = kMaxSplit;
     if (split < 1) split = 1;
-    return launch_tile<TI, TO, A_M, B_K, 1, 1>(p, groups, (int)split);
+    return {1, 1, (int)split};
+}
+
+template <typename TI, typename TO, bool A_M, bool B_K>
+int pick_tile(SimtParams& p, int groups) {
+    constexpr bool fp32 = std::is_same<TI, float>::value && std::is_same<TO, float>::value;
+    const Choice c = choose(p.M, p.N, p.K, fp32);
+    if constexpr (fp32) {
+        if (c.wm == 2 && c.wn == 4) return launch_tile<TI, TO, A_M, B_K, 2, 4>(p, groups, 1);
+        if (c.wm == 2) return launch_tile<TI, TO, A_M, B_K, 2, 2>(p, groups, 1);
+    }
+    if (c.wn == 2) return launch_tile<TI, TO, A_M, B_K, 1, 2>(p, groups, c.split);
+    return launch_tile<TI, TO, A_M, B_K, 1, 1>(p, groups, c.split);
 }
 
 template <typename TI, typename TO>
@@ -415,13 +451,8 @@ int pick_layout(SimtParams& p, int groups, int ta, int tb) {
     return pick_tile<TI, TO, true, true>(p, groups);
 }
 
-}  // namespace
-
-int gemm_simt_grouped(int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
-                      const void* const* B, int64_t ldb, int in_type, void* const* C, int64_t ldc, int out_type,
-                      const float* const* bias, float* const* colsum, bool add) {
-    if (M <= 0 || N <= 0) return 0;
-    if (int rc = ensure_init()) return rc;
+SimtParams make_params(int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda, const void* const* B, int64_t ldb,
+                       void* const* C, int64_t ldc, const float* const* bias, float* const* colsum, bool add) {
     SimtParams p;
     p.M = M; p.N = N; p.K = K; p.lda = lda; p.ldb = ldb; p.ldc = ldc;
     p.add = add ? 1 : 0;
@@ -439,6 +470,17 @@ int gemm_simt_grouped(int ta, int tb, int groups, int64_t M, int64_t N, int64_t 
         p.vec_b = p.vec_b && ((uintptr_t)B[s] & 15) == 0;
         p.vec_c = p.vec_c && (((uintptr_t)C[s] | (uintptr_t)p.bias[g]) & 15) == 0;
     }
+    return p;
+}
+
+}  // namespace
+
+int gemm_simt_grouped(int ta, int tb, int groups, int64_t M, int64_t N, int64_t K, const void* const* A, int64_t lda,
+                      const void* const* B, int64_t ldb, int in_type, void* const* C, int64_t ldc, int out_type,
+                      const float* const* bias, float* const* colsum, bool add) {
+    if (M <= 0 || N <= 0) return 0;
+    if (int rc = ensure_init()) return rc;
+    SimtParams p = make_params(groups, M, N, K, A, lda, B, ldb, C, ldc, bias, colsum, add);
     typedef __nv_bfloat16 bf;
     const bool bf_in = in_type == BOAT_CUDA_BF16;
     if (out_type == BOAT_CUDA_F32_TF32)
@@ -446,6 +488,39 @@ int gemm_simt_grouped(int ta, int tb, int groups, int64_t M, int64_t N, int64_t 
     if (out_type == BOAT_CUDA_F32)
         return bf_in ? pick_layout<bf, float>(p, groups, ta, tb) : pick_layout<float, float>(p, groups, ta, tb);
     return bf_in ? pick_layout<bf, bf>(p, groups, ta, tb) : pick_layout<float, bf>(p, groups, ta, tb);
+}
+
+int gemm_simt_grads(int groups, int64_t T, int64_t I, int64_t O, const void* const* X, const void* const* dY, const void* const* W,
+                    void* const* dX, float* const* dW, float* const* db) {
+    if (int rc = ensure_init()) return rc;
+    const Choice cw = choose(I, O, T, true), cx = choose(T, I, O, true);
+    const int64_t dw_blocks = ceil_div(I, kWarpM) * ceil_div(O, kWarpN) * cw.split, dx_blocks = ceil_div(T, kWarpM) * ceil_div(I, kWarpN);
+    // Both of them small tiles, and an SM for every CTA: what it costs to launch is then most of the cost.  (2 x 64 tokens of width
+    // 64, 12 CTAs each: the host's part of a layer's backward 17.9 us, 11.8 with both pairs in one launch; the step 42.3 and 36.5.)
+    if (cw.wn != 1 || cx.wn != 1 || cx.split != 1 || groups * (dw_blocks + dx_blocks) > sm_count()) return 13;
+    SimtParams w = make_params(groups, I, O, T, X, I, dY, O, (void* const*)dW, O, nullptr, db, false);
+    SimtParams x = make_params(groups, T, I, O, dY, O, W, O, dX, I, nullptr, nullptr, false);
+    w.n_tiles = (int)ceil_div(O, kWarpN);
+    w.split = cw.split;
+    x.n_tiles = (int)ceil_div(I, kWarpN);
+    x.split = 1;
+    using Sw = SimtTile<true, false, 1, 1>;
+    using Sx = SimtTile<false, true, 1, 1>;
+    constexpr int need = Sw::SMEM > Sx::SMEM ? Sw::SMEM : Sx::SMEM;
+    static bool configured = false;      // per process = per device: the library binds to one device
+    if (!configured) {
+        BOATCU_CHECK(cudaFuncSetAttribute(gemm_simt_grads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, need > kSpreadSmem ? need : kSpreadSmem));
+        configured = true;
+    }
+    const int64_t grid = ceil_div(groups * (dw_blocks + dx_blocks), cw.split) * cw.split;       // whole clusters
+    LaunchTurn turn;
+    name_memory(turn, w, groups, true, false, 4, 4);
+    name_memory(turn, x, groups, false, true, 4, 4);
+    w.follow = x.follow = turn.follow();
+    BOATCU_CHECK(launch_in_turn(gemm_simt_grads_kernel, dim3((unsigned)grid), dim3(256), spread_smem(need, grid), (unsigned)cw.split, w, x, groups,
+                                (int)dw_blocks, (int)dx_blocks));
+    BOATCU_LAUNCH_OK("gemm_simt_grads");
+    return 0;
 }
 
 }  // namespace boatcu

@@ -313,6 +313,14 @@ enum { MAX_CHUNKS = 8 };
  * per activation tensor (40 us of PCIe) on.  Below, a call sends what it needs up front. */
 #define PIPELINE_MIN_BYTES ((size_t)2 << 20)
 
+/* boat_cuda_linear_grads where there is one: a program may bring kernels of its own with fewer entries. */
+#pragma weak boat_cuda_linear_grads
+static int linear_grads(int mma, int groups, int64_t T, int64_t H, const void* const* x, const void* const* dy, const void* const* w,
+                        void* const* dx, float* const* dw, float* const* db) {
+    if (!boat_cuda_linear_grads) return 13;
+    return boat_cuda_linear_grads(mma, groups, T, H, H, x, dy, w, dx, dw, db);
+}
+
 static bool on_host(const boat_tensor_t* t) { return t->device != BOAT_DEVICE_CUDA; }
 
 /* BOAT_HOST_PIPELINE=0 in the environment selects the one-piece path for host tensors too. */
@@ -922,11 +930,15 @@ static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output,
     /* output projection: d(ctx) = dOut . Wo^T,  dWo = ctx^T . dOut,  dbo = colsum(dOut) */
     d_dctx = dev_alloc(act_bytes);
     if (!d_dctx) goto done;
-    if (boat_report("dOut.Wo^T", boat_cuda_gemm(mma, 0, 1, T, H, H, d_go, H, p.w[WO], H, type, d_dctx, H, feed_type(mma, type), NULL)) != 0) goto done;
     {
         const void* x[1] = {a->d_ctx};
         const void* dy[1] = {d_go};
-        if (boat_report("dWo", boat_cuda_weight_grads(mma, 1, H, H, T, x, dy, type, &d_dw[WO], bias ? &d_db[WO] : NULL, 0)) != 0) goto done;
+        int rc = linear_grads(mma, 1, T, H, x, dy, (const void* const*)&p.w[WO], &d_dctx, &d_dw[WO], bias ? &d_db[WO] : NULL);
+        if (rc == 13) {
+            rc = boat_cuda_gemm(mma, 0, 1, T, H, H, d_go, H, p.w[WO], H, type, d_dctx, H, feed_type(mma, type), NULL);
+            if (rc == 0) rc = boat_cuda_weight_grads(mma, 1, H, H, T, x, dy, type, &d_dw[WO], bias ? &d_db[WO] : NULL, 0);
+        }
+        if (boat_report("dOut.Wo^T and dWo", rc) != 0) goto done;
     }
     /* Data parallel with overlap: dWo and dbo are final here, long before the step ends - their
      * sum over the ranks runs under the attention-core backward. */
@@ -955,8 +967,22 @@ static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output,
 
     /* input projections: dW = X^T . dP and db = colsum(dP) first - with overlap their sum over
      * the ranks then runs under the three dX = dP . W^T GEMMs that follow */
-    if (boat_report("dW", boat_cuda_weight_grads(mma, 3, H, H, T, (const void* const*)a->d_in, (const void* const*)d_dproj,
-                                                 type, d_dw, bias ? d_db : NULL, 0)) != 0)
+    bool both = false;                              /* a small FP32 layer: dW and dX in one launch */
+    if (!sum && !overlap) {
+        void* target[3];
+        bool fp32 = true;
+        for (int i = 0, k = 0; i < 3; ++i) {
+            target[i] = gin[i]->device == BOAT_DEVICE_CUDA ? gin[i]->data : (char*)d_down + down_at[k++];
+            fp32 = fp32 && storage_of(gin[i]->dtype) == BOAT_CUDA_F32;
+        }
+        const int rc = fp32 ? linear_grads(mma, 3, T, H, (const void* const*)a->d_in, (const void* const*)d_dproj, (const void* const*)p.w,
+                                           target, d_dw, bias ? d_db : NULL)
+                            : 13;
+        if (rc != 13 && boat_report("dW and dX", rc) != 0) goto done;
+        both = rc == 0;
+    }
+    if (!both && boat_report("dW", boat_cuda_weight_grads(mma, 3, H, H, T, (const void* const*)a->d_in, (const void* const*)d_dproj,
+                                                          type, d_dw, bias ? d_db : NULL, 0)) != 0)
         goto done;
     if (overlap && a->grad_overlap == 1) {
         float* piece[2] = {d_dw[WQ], d_db[WQ]};            /* dWq|dWk|dWv and dbq|dbk|dbv are contiguous */
@@ -967,7 +993,9 @@ static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output,
     }
     const bool yield = overlap && a->grad_overlap == 1;      /* a sum was just started beside these GEMMs */
     if (yield) boat_cuda_gemm_set_yielding(1);
-    if (sum) {
+    if (both) {
+        /* dX is there */
+    } else if (sum) {
         /* the three input gradients are one: summed in the accumulator, or - where the tensor cores do not
          * take the shape - product by product */
         const int out_type = storage_of(gin[0]->dtype);

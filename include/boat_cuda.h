@@ -138,6 +138,12 @@ int boat_cuda_gemm_sum(int mma, int trans_a, int trans_b, int groups, int64_t M,
 int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T, const void* const* X,
                            const void* const* dY, int in_type, float* const* dW, float* const* db, int accumulate);
 
+/* boat_cuda_weight_grads (without accumulate) and the input gradients dX = dY . W^T of the same projections in one launch, all
+ * FP32: for problems of a few tiles, where the launch is most of the cost.  W [I,O]; dX [T,I] must overlap none of the other
+ * operands.  Returns 13, without an error text and without having done anything, where two launches are as good. */
+int boat_cuda_linear_grads(int mma, int groups, int64_t T, int64_t I, int64_t O, const void* const* X, const void* const* dY,
+                           const void* const* W, void* const* dX, float* const* dW, float* const* db);
+
 /* ---- attention core: replaces scaled_dot_product_attention_impl
  *      (src/layers/attention.c:882-1079) ------------------------------------------------
  * Q,K,V,O are [units, S, hs] contiguous: unit u = (b*nh + h) is the block at element

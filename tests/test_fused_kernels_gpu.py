@@ -242,6 +242,26 @@ def test_attention_core_with_several_items_per_cta(gpu_lib, hs, units, S, causal
         assert rel(got[key], ref[key]) <= 2e-2, key
 
 
+# one tile, K split over a cluster with CTAs left over in the last one, ragged and unaligned sizes, the largest taken
+@pytest.mark.parametrize("T,I,O,groups", [(8, 32, 32, 1), (128, 64, 64, 3), (200, 40, 72, 2), (33, 13, 9, 3), (300, 64, 32, 4), (640, 96, 64, 1)])
+def test_linear_grads_in_one_launch(gpu_lib, T, I, O, groups):
+    x, dy, w = ([rng.normal(9, 10 * k + g, s) for g in range(groups)] for k, s in enumerate([(T, I), (T, O), (I, O)]))
+    dx, ddy, dw_ = ([DeviceBuffer.from_numpy(t) for t in ts] for ts in (x, dy, w))
+    got, want = ([[DeviceBuffer.from_numpy(np.full(s, np.nan, np.float32)) for _ in range(groups)] for s in ((T, I), (I, O), (O,))] for _ in range(2))
+    check(gpu_lib.boat_cuda_linear_grads(capi.MMA_FP32, groups, T, I, O, _table(dx), _table(ddy), _table(dw_), *map(_table, got)), "linear_grads")
+    check(gpu_lib.boat_cuda_weight_grads(capi.MMA_FP32, groups, I, O, T, _table(dx), _table(ddy), capi.CUDA_F32, _table(want[1]), _table(want[2]), 0), "dw")
+    check(gpu_lib.boat_cuda_gemm_grouped(capi.MMA_FP32, 0, 1, groups, T, I, O, _table(ddy), O, _table(dw_), O, capi.CUDA_F32, _table(want[0]), I,
+                                         capi.CUDA_F32, None), "dx")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    for a, b, shape in zip(got, want, ((T, I), (I, O), (O,))):
+        for g in range(groups):
+            assert a[g].numpy(shape).tobytes() == b[g].numpy(shape).tobytes()
+    assert rel(got[0][0].numpy((T, I)), dy[0].astype(np.float64) @ w[0].astype(np.float64).T) <= 1e-6
+    # larger problems, and other arithmetic, are two launches
+    assert gpu_lib.boat_cuda_linear_grads(capi.MMA_FP32, 1, 100000, I, O, _table(dx), _table(ddy), _table(dw_), *map(_table, got)) == 13
+    assert gpu_lib.boat_cuda_linear_grads(capi.MMA_TF32, 1, T, I, O, _table(dx), _table(ddy), _table(dw_), *map(_table, got)) == 13
+
+
 # Kernels that name their memory run beside one another when they touch nothing of each other's: a random sequence over
 # few buffers, where most neighbours do depend on each other - read after write, write after read, write after write, over
 # windows that overlap in part - gives the bits of the same sequence with a wait after every call.
