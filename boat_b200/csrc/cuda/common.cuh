@@ -175,8 +175,8 @@ int gemm_simt_grouped(int trans_a, int trans_b, int groups, int64_t M, int64_t N
 // boat_cuda_linear_grads in FP32 on the CUDA cores, for problems so small that one launch is worth it; 13 for others.
 int gemm_simt_grads(int groups, int64_t T, int64_t I, int64_t O, const void* const* X, const void* const* dY, const void* const* W,
                     void* const* dX, float* const* dW, float* const* db);
-// boat_cuda_colsum_multi, with `add` adding to the outputs.
-int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count, bool add);
+// boat_cuda_colsum_multi
+int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count);
 int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, int io_type, void* O, float* lse);
 // Where attn_bwd_simt_makes_delta says so it works delta out from O and dO; else `delta` is given (rowdot).

@@ -142,7 +142,7 @@ int boat_cuda_weight_grads(int mma, int groups, int64_t I, int64_t O, int64_t T,
         return gemm_simt_grouped(1, 0, groups, I, O, T, X, I, dY, O, store, (void* const*)dW, O, BOAT_CUDA_F32, nullptr, db, accumulate != 0);
     }
     if (int rc = boat_cuda_gemm_grouped(mma, 1, 0, groups, I, O, T, X, I, dY, O, in_type, (void* const*)dW, O, BOAT_CUDA_F32, nullptr)) return rc;
-    return sums ? colsum_multi(dY, in_type, T, O, db, groups, false) : 0;
+    return sums ? colsum_multi(dY, in_type, T, O, db, groups) : 0;
 }
 
 int boat_cuda_linear_grads(int mma, int groups, int64_t T, int64_t I, int64_t O, const void* const* X, const void* const* dY,

@@ -349,7 +349,7 @@ struct ColsumTable {
 };
 
 template <typename T, int VEC, int LANES, int THREADS, bool CLUSTER>
-__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols, int64_t first, int add_to, int follow) {
+__global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__ ColsumTable t, int64_t rows, int64_t cols, int64_t first, int follow) {
     constexpr int ROWS = THREADS / LANES, COLS = LANES * VEC, UNROLL = 8;
     __shared__ float part[ROWS * COLS];
     __shared__ float folded[CLUSTER ? COLS : 1];
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__
 #pragma unroll
                 for (int r = 0; r < kColsumCluster; ++r) s += cluster.map_shared_rank(folded, r)[c];
                 float* o = t.out[blockIdx.z] + group0 + c;
-                if (group0 + c < cols) *o = add_to ? *o + s : s;
+                if (group0 + c < cols) *o = s;
             }
         }
         cluster.sync();
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(THREADS) colsum_kernel(const __grid_constant__
 }
 
 template <typename T, int VEC, int LANES>
-static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t cols, int count, bool add) {
+static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t cols, int count) {
     const int64_t groups = ceil_div(cols, LANES * VEC);
     for (int64_t first = 0; first < groups; first += kMaxGridY) {
         const int64_t n = groups - first < kMaxGridY ? groups - first : kMaxGridY;
@@ -427,16 +427,16 @@ static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t col
             turn.writes(t.out[i], (size_t)cols * 4);
         }
         BOATCU_CHECK(launch_in_turn(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)n, (unsigned)count),
-                                    dim3(512), 0, kColsumCluster, t, rows, cols, first, add ? 1 : 0, turn.follow()));
+                                    dim3(512), 0, kColsumCluster, t, rows, cols, first, turn.follow()));
         BOATCU_LAUNCH_OK("colsum");
     }
     return 0;
 }
 
 template <typename T, int VEC>
-static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int count, bool add) {
+static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int count) {
     if (rows * cols * (int64_t)sizeof(T) >= (32ll << 20)) {
-        for (int i = 0; i < count && !add; ++i) BOATCU_CHECK(cudaMemsetAsync(t.out[i], 0, (size_t)cols * sizeof(float), stream()));
+        for (int i = 0; i < count; ++i) BOATCU_CHECK(cudaMemsetAsync(t.out[i], 0, (size_t)cols * sizeof(float), stream()));
         const int64_t groups = ceil_div(cols, 32 * VEC);
         int64_t y = (int64_t)sm_count() * 8 / (groups * count);         // eight CTAs per SM
         if (y < 1) y = 1;
@@ -444,7 +444,7 @@ static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int c
         for (int64_t first = 0; first < groups; first += kMaxGridY) {
             const int64_t n = groups - first < kMaxGridY ? groups - first : kMaxGridY;
             BOATCU_CHECK(launch_dependent(colsum_kernel<T, VEC, 32, 256, false>, dim3((unsigned)y, (unsigned)n, (unsigned)count), dim3(256), 0, 1,
-                                          t, rows, cols, first, 0, (int)kRelease));
+                                          t, rows, cols, first, (int)kRelease));
             BOATCU_LAUNCH_OK("colsum");
         }
         return 0;
@@ -452,9 +452,9 @@ static int launch_colsum(const ColsumTable& t, int64_t rows, int64_t cols, int c
     // the runs of a row are 512 bytes where that makes enough CTAs for the GPU, else 256 or 128
     auto ctas = [&](int lanes) { return ceil_div(cols, lanes * VEC) * kColsumCluster * count; };
     const int64_t enough = (int64_t)sm_count() * 4 / 5;
-    if (ctas(32) >= enough) return launch_colsum_cluster<T, VEC, 32>(t, rows, cols, count, add);
-    if (ctas(16) >= enough) return launch_colsum_cluster<T, VEC, 16>(t, rows, cols, count, add);
-    return launch_colsum_cluster<T, VEC, 8>(t, rows, cols, count, add);
+    if (ctas(32) >= enough) return launch_colsum_cluster<T, VEC, 32>(t, rows, cols, count);
+    if (ctas(16) >= enough) return launch_colsum_cluster<T, VEC, 16>(t, rows, cols, count);
+    return launch_colsum_cluster<T, VEC, 8>(t, rows, cols, count);
 }
 
 // ---- what the BF16 tensor-core backward starts from, in one pass over dO and O --------------------------
@@ -796,7 +796,7 @@ int boat_cuda_round_tf32(float* y, const float* x, int64_t n) {
 }  // extern "C"
 
 namespace boatcu {
-int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count, bool add) {
+int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count) {
     if (cols <= 0 || count <= 0) return 0;
     if (count > kMaxColsum) return set_error(11, "boat_cuda_colsum_multi: %d matrices (1 to %d)", count, kMaxColsum);
     if (!X || !out) return set_error(11, "boat_cuda_colsum_multi: NULL table");
@@ -814,8 +814,8 @@ int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, f
     }
     if (rows < 0) rows = 0;
     if (x_type == BOAT_CUDA_BF16)
-        return can_vec ? launch_colsum<__nv_bfloat16, 8>(t, rows, cols, count, add) : launch_colsum<__nv_bfloat16, 1>(t, rows, cols, count, add);
-    return can_vec ? launch_colsum<float, 4>(t, rows, cols, count, add) : launch_colsum<float, 1>(t, rows, cols, count, add);
+        return can_vec ? launch_colsum<__nv_bfloat16, 8>(t, rows, cols, count) : launch_colsum<__nv_bfloat16, 1>(t, rows, cols, count);
+    return can_vec ? launch_colsum<float, 4>(t, rows, cols, count) : launch_colsum<float, 1>(t, rows, cols, count);
 }
 
 }  // namespace boatcu
@@ -823,7 +823,7 @@ int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, f
 extern "C" {
 
 int boat_cuda_colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count) {
-    return colsum_multi(X, x_type, rows, cols, out, count, false);
+    return colsum_multi(X, x_type, rows, cols, out, count);
 }
 
 int boat_cuda_colsum(const void* X, int x_type, int64_t rows, int64_t cols, float* out) {

@@ -351,6 +351,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
 #pragma unroll
                     for (int e = 0; e < PER; ++e) total[e] += sum[e];
                 }
+                fence_proxy_async_smem();             // the reads are done before the producer's next copy into the stage
                 __syncwarp();
                 if (leader) mbar_arrive(&summed[s]);
                 if (++s == STAGES) {
@@ -424,7 +425,11 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
                     ++aux_it;
 #pragma unroll
                     for (int u = 0; u < 8; ++u) aux[u] = *reinterpret_cast<const uint4*>(row2 + ((u ^ swz) << 4));
-                    __syncwarp();                     // the next one comes in under the work on this one
+                    // The next one comes in under the work on this one, into the same box: not before every lane's reads have been
+                    // performed.  Without the fence they may still be queued when the copy lands (16 bytes of a row in
+                    // one of a hundred steps).
+                    fence_proxy_async_smem();
+                    __syncwarp();
                     if (leader && c + 2 * step < cols) load_aux(col0 + 2 * step, row0);
                 }
                 // one 32-column half of the box (all of an FP32 box) at a time

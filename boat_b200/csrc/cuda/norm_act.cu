@@ -531,7 +531,7 @@ static int layernorm_bwd_rows(const void* dy, const void* x, int64_t rows, int64
     const void* from[2] = {partial, (const float*)partial + blocks * cols};
     float* to[2] = {dgamma, dbeta};
     const int first = dgamma ? 0 : 1, count = (dgamma ? 1 : 0) + (dbeta ? 1 : 0);
-    if (rc == 0) rc = colsum_multi(from + first, BOAT_CUDA_F32, blocks, cols, to + first, count, false);
+    if (rc == 0) rc = colsum_multi(from + first, BOAT_CUDA_F32, blocks, cols, to + first, count);
     const int freed = boat_cuda_free(partial);
     return rc ? rc : freed;
 }
