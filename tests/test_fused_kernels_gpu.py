@@ -65,6 +65,22 @@ def test_gemm_epilogues(gpu_lib, shape, epilogue):
     assert (np.abs(got - want) <= roundings * 1.01 * 2.0 ** -8 * np.abs(want) + slack).all()
 
 
+# The operand of the epilogue comes through one shared-memory box per warp, asked for again as soon as it has been read: many
+# tiles per CTA, many times, the same bits each time.
+@pytest.mark.parametrize("epilogue", [2, 3], ids=["gelu_grad", "add"])
+def test_gemm_epilogue_operand_boxes_are_read_in_time(gpu_lib, epilogue):
+    M, N, K, tb = 8192, 1024, 256, epilogue == 2
+    da, db, daux = (DeviceBuffer.from_numpy(_bf(11, i, sh), bf16=True) for i, sh in enumerate([(M, K), (N, K) if tb else (K, N), (M, N)]))
+    dc, first = DeviceBuffer(M * N * 2), None
+    for _ in range(300):
+        check(gpu_lib.boat_cuda_gemm_fused(capi.MMA_BF16, epilogue, 0, int(tb), M, N, K, da.p, K, db.p, K if tb else N, capi.CUDA_BF16,
+                                           dc.p, N, None, daux.p), "gemm_fused")
+        check(gpu_lib.boat_cuda_sync(), "sync")
+        got = dc.numpy((M, N), bf16=True)
+        first = got if first is None else first
+        assert (got == first).all()
+
+
 @pytest.mark.parametrize("shape", [(128, 64, 64), (333, 768, 96), (2000, 320, 200)])
 @pytest.mark.parametrize("groups", [1, 2, 3])
 def test_gemm_sum_of_products(gpu_lib, shape, groups):
