@@ -197,6 +197,8 @@ PROTOTYPES = {
     "boat_cuda_last_error": (C.c_char_p, []),
     "boat_cuda_stream": (_P, []),
     "boat_cuda_set_stream": (_I, [_P]),
+    "boat_cuda_launches_begin": (None, []),
+    "boat_cuda_launches_end": (None, []),
     "boat_cuda_sync": (_I, []),
     "boat_cuda_malloc": (_I, [_PP, _SZ]),
     "boat_cuda_free": (_I, [_P]),

@@ -183,7 +183,7 @@ static void backward_op(op_record_t* op, const boat_tensor_t* g) {
     }
 }
 
-void boat_variable_backward(boat_variable_t* v, boat_tensor_t* grad_output) {
+static void backward_from(boat_variable_t* v, boat_tensor_t* grad_output) {
     if (!v || !v->requires_grad) return;
     boat_tensor_t* seed = grad_output;
     if (!seed) {
@@ -214,12 +214,18 @@ void boat_variable_backward(boat_variable_t* v, boat_tensor_t* grad_output) {
             for (int j = 0; j < i; ++j) seen = seen || v->producer->inputs[j] == in;
             if (in && !seen && in->requires_grad && in->grad && in->producer) {
                 boat_tensor_ref(in->grad);
-                boat_variable_backward(in, in->grad);
+                backward_from(in, in->grad);
                 boat_tensor_unref(in->grad);
             }
         }
     }
     if (seed != grad_output) boat_tensor_unref(seed);
+}
+
+void boat_variable_backward(boat_variable_t* v, boat_tensor_t* grad_output) {
+    boat_cuda_launches_begin();
+    backward_from(v, grad_output);
+    boat_cuda_launches_end();
 }
 
 void boat_variable_backward_full(const boat_variable_t* v) { boat_variable_backward((boat_variable_t*)v, NULL); }

@@ -63,6 +63,8 @@ __device__ __forceinline__ void griddep_sync() {
 // be running, does not wait for them (kBeside): a weight gradient beside an input gradient, a conversion beside either.  It
 // fills the SMs as they come free, without the gap between two launches, and waits for its predecessor at its
 // end instead, so that its completion still implies that of all kernels before it.
+// Only within a sequence (boat_cuda_launches_begin): the first launch of one, and every launch outside one, waits for whatever is
+// before it on the stream, a program's own kernels or NCCL's too (launch_order.h).
 // Encoder block of 4 x 333 x 768 BF16: 227 us with every kernel waiting, 217 so; residual attention of 4 x 250 x 256 FP32 155 and 147.
 enum Follow { kRelease = 1, kBeside = 2 };
 __device__ __forceinline__ void griddep_enter(int follow) {
@@ -92,8 +94,6 @@ public:
 private:
     static size_t span(int64_t rows, int64_t cols, int64_t ld, size_t es) { return rows > 0 && cols > 0 ? (size_t)((rows - 1) * ld + cols) * es : 0; }
     void name(const void* p, size_t bytes, bool written);
-    bool named_, beside_;
-    int before_;                     // ranges of the kernels before that may still run
 };
 
 // Something other than a named kernel comes next on the library stream, or the stream changes.

@@ -4,6 +4,7 @@
 // malloc/memcpy/memset regardless of the device argument).
 #include "tc_common.cuh"
 #include "block_cache.h"
+#include "launch_order.h"
 #include <stdarg.h>
 #include <stdlib.h>
 #include <string.h>
@@ -36,49 +37,28 @@ int set_error(int status, const char* fmt, ...) {
 
 cudaStream_t stream() { return g_stream; }
 bool ready() { return g_ready; }
-// The launches that may still be running, as the ranges they named: the last kRelease launch and those beside it.
-struct NamedRange {
-    uintptr_t lo, hi;
-    bool written;
-};
-constexpr int kMaxRanges = 96;
+// ---- launches beside one another (launch_order.h) ------------------------------------------------
 static std::mutex g_turn;                      // one launch at a time
-static NamedRange g_ranges[kMaxRanges];
-static int g_range_count = 0;                  // 0: the next launch is an ordinary one
-static bool g_range_overflow = false;          // the present launch touches more than the table holds
-static cudaStream_t g_range_stream = 0;
+static LaunchOrder g_order;
+static std::atomic<uint64_t> g_sequences{0};
+static thread_local uint64_t t_sequence = 0;   // of this thread, while t_sequence_depth > 0
+static thread_local int t_sequence_depth = 0;
 
-LaunchTurn::LaunchTurn() : named_(false), beside_(false) {
+LaunchTurn::LaunchTurn() {
     g_turn.lock();
-    if (g_range_stream != g_stream) g_range_count = 0;
-    g_range_overflow = false;
-    before_ = g_range_count;
-}
-void LaunchTurn::name(const void* p, size_t bytes, bool written) {
-    named_ = true;
-    if (!p || bytes == 0) return;
-    if (g_range_count == kMaxRanges) g_range_overflow = true;
-    else g_ranges[g_range_count++] = NamedRange{(uintptr_t)p, (uintptr_t)p + bytes, written};
-}
-int LaunchTurn::follow() {
-    beside_ = before_ > 0 && !g_range_overflow;
-    for (int i = before_; i < g_range_count && beside_; ++i)
-        for (int j = 0; j < before_ && beside_; ++j)
-            beside_ = g_ranges[i].hi <= g_ranges[j].lo || g_ranges[j].hi <= g_ranges[i].lo || !(g_ranges[i].written || g_ranges[j].written);
-    return beside_ ? kBeside : kRelease;
+    g_order.begin({t_sequence_depth > 0 ? t_sequence : 0, (const void*)g_stream});
 }
 LaunchTurn::~LaunchTurn() {
-    if (!named_ || g_range_overflow) {
-        g_range_count = 0;
-    } else if (!beside_) {                      // the kernels before are complete once this one lets go
-        for (int i = before_; i < g_range_count; ++i) g_ranges[i - before_] = g_ranges[i];
-        g_range_count -= before_;
-    }
-    g_range_stream = g_stream;
+    g_order.end();
     g_turn.unlock();
 }
+void LaunchTurn::name(const void* p, size_t bytes, bool written) { g_order.name(p, bytes, written); }
+int LaunchTurn::follow() { return g_order.beside() ? kBeside : kRelease; }
 
-void ordinary_launch_next() { LaunchTurn turn; }
+void ordinary_launch_next() {
+    std::lock_guard<std::mutex> lk(g_turn);
+    g_order.interrupt();
+}
 
 void count_launch(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
 
@@ -347,6 +327,14 @@ int boat_cuda_set_stream(void* s) {
     }
     g_stream_id = id;
     return 0;
+}
+
+void boat_cuda_launches_begin(void) {
+    if (t_sequence_depth++ == 0) t_sequence = ++g_sequences;
+}
+
+void boat_cuda_launches_end(void) {
+    if (t_sequence_depth > 0) --t_sequence_depth;
 }
 
 // ---- copies that overlap kernels -----------------------------------------------------------------

@@ -625,9 +625,9 @@ void boat_attention_free(boat_attention_t* a) {
  * units form one indivisible piece when host tensors are moved in chunks.  Inputs are [.., H]
  * tensors of T*H elements each; the result has the query's shape.  A CUDA `residual` of the query's dtype
  * is added to the result. */
-static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
-                                   const boat_tensor_t* value, int64_t T, int64_t S, int64_t units, int64_t gran,
-                                   const boat_tensor_t* residual) {
+static boat_tensor_t* forward_steps(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
+                                    const boat_tensor_t* value, int64_t T, int64_t S, int64_t units, int64_t gran,
+                                    const boat_tensor_t* residual) {
     const boat_tensor_t* in[3] = {query, key, value};
     const int64_t H = (int64_t)a->config.hidden_size, hs = (int64_t)a->config.head_size;
     if (boat_report("CUDA start-up", boat_cuda_init(-1)) != 0) return NULL;
@@ -755,6 +755,15 @@ done:
     return result;
 }
 
+static boat_tensor_t* forward_rows(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
+                                   const boat_tensor_t* value, int64_t T, int64_t S, int64_t units, int64_t gran,
+                                   const boat_tensor_t* residual) {
+    boat_cuda_launches_begin();
+    boat_tensor_t* result = forward_steps(a, query, key, value, T, S, units, gran, residual);
+    boat_cuda_launches_end();
+    return result;
+}
+
 static boat_tensor_t* forward_batch(boat_attention_t* a, const boat_tensor_t* query, const boat_tensor_t* key,
                                     const boat_tensor_t* value, const boat_tensor_t* residual) {
     if (!a || !query || !key || !value) return NULL;
@@ -834,8 +843,8 @@ static bool ensure_grads(boat_attention_t* a) {
 }
 
 /* `sum`: one tensor was query, key and value; *grad_query gets its gradient, the others nothing. */
-static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output, boat_tensor_t** grad_query,
-                          boat_tensor_t** grad_key, boat_tensor_t** grad_value, bool sum) {
+static bool backward_steps(boat_attention_t* a, const boat_tensor_t* grad_output, boat_tensor_t** grad_query,
+                           boat_tensor_t** grad_key, boat_tensor_t** grad_value, bool sum) {
     if (!a || !grad_output) {
         printf("[ERROR] boat_attention_backward: invalid arguments\n");
         return false;
@@ -1058,6 +1067,14 @@ done:
         else if (gin[i]) boat_tensor_free(gin[i]);
     }
     return true;
+}
+
+static bool backward_impl(boat_attention_t* a, const boat_tensor_t* grad_output, boat_tensor_t** grad_query,
+                          boat_tensor_t** grad_key, boat_tensor_t** grad_value, bool sum) {
+    boat_cuda_launches_begin();
+    const bool ok = backward_steps(a, grad_output, grad_query, grad_key, grad_value, sum);
+    boat_cuda_launches_end();
+    return ok;
 }
 
 bool boat_attention_backward(boat_attention_t* a, const boat_tensor_t* grad_output, boat_tensor_t** grad_query,

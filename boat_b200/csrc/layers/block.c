@@ -71,7 +71,7 @@ static boat_tensor_t* drop(boat_tensor_t* t, boat_tensor_t* keep) {
     return keep;
 }
 
-boat_tensor_t* boat_encoder_block_forward(boat_encoder_block_t* b, const boat_tensor_t* x) {
+static boat_tensor_t* forward_steps(boat_encoder_block_t* b, const boat_tensor_t* x) {
     if (!b || !x || x->ndim != 3) return NULL;
     const int64_t T = x->shape[0] * x->shape[1], d = x->shape[2];
     const int64_t flat[2] = {T, d};
@@ -114,7 +114,7 @@ boat_tensor_t* boat_encoder_block_forward(boat_encoder_block_t* b, const boat_te
     return out;
 }
 
-boat_tensor_t* boat_encoder_block_backward(boat_encoder_block_t* b, const boat_tensor_t* grad_output) {
+static boat_tensor_t* backward_steps(boat_encoder_block_t* b, const boat_tensor_t* grad_output) {
     if (!b || !grad_output || !b->u) return NULL;
     const int64_t T = b->shape[0] * b->shape[1], d = b->shape[2];
     if ((int64_t)grad_output->nelements != T * d) return NULL;
@@ -175,6 +175,20 @@ boat_tensor_t* boat_encoder_block_backward(boat_encoder_block_t* b, const boat_t
     }
     drop(g2, NULL); drop(da, NULL); drop(du, NULL); drop(dh2_3, NULL); drop(dh2, NULL); drop(dln2, NULL);
     drop(dr1, NULL); drop(gq, NULL); drop(gk, NULL); drop(gv, NULL); drop(s1, NULL); drop(dh1, NULL); drop(dln1, NULL);
+    return dx;
+}
+
+boat_tensor_t* boat_encoder_block_forward(boat_encoder_block_t* b, const boat_tensor_t* x) {
+    boat_cuda_launches_begin();
+    boat_tensor_t* out = forward_steps(b, x);
+    boat_cuda_launches_end();
+    return out;
+}
+
+boat_tensor_t* boat_encoder_block_backward(boat_encoder_block_t* b, const boat_tensor_t* grad_output) {
+    boat_cuda_launches_begin();
+    boat_tensor_t* dx = backward_steps(b, grad_output);
+    boat_cuda_launches_end();
     return dx;
 }
 

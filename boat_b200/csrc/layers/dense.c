@@ -56,7 +56,7 @@ void boat_dense_layer_free(boat_dense_layer_t* l) {
 
 /* Forward with element-wise work behind the product (BOAT_EPI_*; fused.h): `aux` is the residual to add (ADD),
  * or receives the pre-activation (GELU). */
-static boat_tensor_t* dense_forward(boat_dense_layer_t* l, const boat_tensor_t* input, int epilogue, const boat_tensor_t* residual,
+static boat_tensor_t* forward_steps(boat_dense_layer_t* l, const boat_tensor_t* input, int epilogue, const boat_tensor_t* residual,
                                     boat_tensor_t** pre_activation) {
     if (!l || !input) return NULL;
     boat_tensor_ref((boat_tensor_t*)input);
@@ -97,6 +97,14 @@ static boat_tensor_t* dense_forward(boat_dense_layer_t* l, const boat_tensor_t* 
     return out;
 }
 
+static boat_tensor_t* dense_forward(boat_dense_layer_t* l, const boat_tensor_t* input, int epilogue, const boat_tensor_t* residual,
+                                    boat_tensor_t** pre_activation) {
+    boat_cuda_launches_begin();
+    boat_tensor_t* out = forward_steps(l, input, epilogue, residual, pre_activation);
+    boat_cuda_launches_end();
+    return out;
+}
+
 boat_tensor_t* boat_dense_layer_forward(boat_dense_layer_t* l, const boat_tensor_t* input) {
     return dense_forward(l, input, BOAT_EPI_NONE, NULL, NULL);
 }
@@ -111,7 +119,7 @@ boat_tensor_t* boat_dense_forward_add(boat_dense_layer_t* l, const boat_tensor_t
 }
 
 /* Backward; with `pre_activation` the layer's input was GELU of it, and its gradient is returned. */
-static boat_tensor_t* dense_backward(boat_dense_layer_t* l, const boat_tensor_t* grad_output, const boat_tensor_t* pre_activation) {
+static boat_tensor_t* backward_steps(boat_dense_layer_t* l, const boat_tensor_t* grad_output, const boat_tensor_t* pre_activation) {
     if (!l || !grad_output || !l->cache_input) return NULL;
     const boat_tensor_t* x = l->cache_input;
     if (x->ndim != 2 || grad_output->ndim != 2) {
@@ -162,6 +170,13 @@ static boat_tensor_t* dense_backward(boat_dense_layer_t* l, const boat_tensor_t*
     if (xo) boat_dev_free(dx);
     if (go) boat_dev_free(dg);
     if (wo) boat_dev_free(dw);
+    return out;
+}
+
+static boat_tensor_t* dense_backward(boat_dense_layer_t* l, const boat_tensor_t* grad_output, const boat_tensor_t* pre_activation) {
+    boat_cuda_launches_begin();
+    boat_tensor_t* out = backward_steps(l, grad_output, pre_activation);
+    boat_cuda_launches_end();
     return out;
 }
 

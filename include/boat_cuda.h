@@ -45,6 +45,12 @@ int         boat_cuda_device_count(void);        /* 0 when no usable GPU / drive
 const char* boat_cuda_last_error(void);
 void*       boat_cuda_stream(void);              /* cudaStream_t the library launches on */
 int         boat_cuda_set_stream(void* stream);   /* the caller orders the new stream behind the old one's work */
+/* A sequence of launches: between the two calls this thread launches through the library and nobody puts anything else on
+ * its stream.  Within it a kernel that touches none of the memory of those still running need not wait for them.  The
+ * layers open one around the body of a forward or backward; sequences nest.  The first launch of a sequence, and every
+ * call outside one, waits for all that is before it on the stream, whoever put it there. */
+void        boat_cuda_launches_begin(void);
+void        boat_cuda_launches_end(void);
 int         boat_cuda_sync(void);                /* wait for the library stream and the copy streams */
 int         boat_cuda_malloc(void** ptr, size_t bytes);   /* stream-ordered pool allocation */
 int         boat_cuda_free(void* ptr);

@@ -16,6 +16,9 @@ static int step(void) { return calls++ == fail_at ? 99 : 0; }
 int boat_cuda_init(int device) { (void)device; return step(); }
 int boat_cuda_device_count(void) { return 1; }
 const char* boat_cuda_last_error(void) { return "made up"; }
+static int open_sequences;
+void boat_cuda_launches_begin(void) { ++open_sequences; }
+void boat_cuda_launches_end(void) { --open_sequences; }
 int boat_cuda_sync(void) { return step(); }
 size_t boat_cuda_bytes_in_use(void) { return 0; }
 int boat_cuda_malloc(void** p, size_t n) {
@@ -131,6 +134,10 @@ static int run(int B, int S, int H, boat_device_t device, int fail) {
     boat_tensor_free(g);
     if (device_blocks || pinned_blocks) {
         printf("%d x %d x %d on device %d, call %d failing: %d device and %d pinned blocks left\n", B, S, H, (int)device, fail, device_blocks, pinned_blocks);
+        exit(1);
+    }
+    if (open_sequences) {
+        printf("%d x %d x %d on device %d, call %d failing: %d launch sequences left open\n", B, S, H, (int)device, fail, open_sequences);
         exit(1);
     }
     return made;

@@ -278,7 +278,7 @@ def test_linear_grads_in_one_launch(gpu_lib, T, I, O, groups):
     assert gpu_lib.boat_cuda_linear_grads(capi.MMA_TF32, 1, T, I, O, _table(dx), _table(ddy), _table(dw_), *map(_table, got)) == 13
 
 
-# Kernels that name their memory run beside one another when they touch nothing of each other's: a random sequence over
+# Within a sequence of launches, kernels that name their memory run beside one another when they touch nothing of each other's: one over
 # few buffers, where most neighbours do depend on each other - read after write, write after read, write after write, over
 # windows that overlap in part - gives the bits of the same sequence with a wait after every call.
 @pytest.mark.parametrize("mma", [capi.MMA_FP32, capi.MMA_BF16], ids=["fp32", "bf16"])
@@ -294,6 +294,7 @@ def test_kernels_beside_one_another(gpu_lib, mma, n, seed):
         block = DeviceBuffer.from_numpy(_bf(8, seed, (count * n, n), 1 / math.sqrt(n)) if bf else first, bf16=bf)
         wide, grads = DeviceBuffer.from_numpy(first), DeviceBuffer(n * n * 4)
         at = lambda rows: C.c_void_p(block.p.value + rows * n * es)
+        gpu_lib.boat_cuda_launches_begin()
         for _ in range(80):
             # n rows each, from any eighth of the block: neighbours overlap in part
             x, y, z = (int(r) * n // 8 for r in pick.choice(8 * (count - 1) + 1, 3, replace=False))
@@ -314,6 +315,7 @@ def test_kernels_beside_one_another(gpu_lib, mma, n, seed):
                                                      _table([grads]), None, 0), "dw")
             if wait:
                 check(gpu_lib.boat_cuda_sync(), "sync")
+        gpu_lib.boat_cuda_launches_end()
         check(gpu_lib.boat_cuda_sync(), "sync")
         return block.numpy((count * n, n), bf16=bf), grads.numpy((n, n))
 

@@ -1,0 +1,89 @@
+"""Work of the program's own on the library's stream, between calls of the library: it sees what the call before has written, and
+the call behind sees what it has written."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from boat_b200 import capi, rng
+from boat_b200.host import Attention, Tensor, check
+
+pytestmark = pytest.mark.gpu
+B, S, D, NH = 4, 128, 256, 4
+
+
+class _Memory:
+    """A library tensor's memory for torch."""
+
+    def __init__(self, t):
+        self.__cuda_array_interface__ = {"shape": t.shape, "typestr": "<f4", "data": (t.data_ptr, False), "version": 2}
+
+
+def _torch(t):
+    return torch.as_tensor(_Memory(t), device="cuda")
+
+
+def _train(mma, wait, steps=8):
+    """Steps of a layer whose weights, input and upstream gradient torch kernels write between the library's calls; no call of either
+    is followed by a wait unless `wait`."""
+    layer = Attention(D, NH, causal=True)
+    layer.to_device(capi.DEVICE_CUDA)
+    layer.set_precision(mma)
+    for i, name in enumerate(Attention.PARAMS):
+        p = layer.param(name)
+        p.set(rng.normal(41, i, p.shape, 0.06))
+    x, g = (Tensor.from_numpy(rng.normal(42, i, (B, S, D)), capi.DEVICE_CUDA) for i in range(2))
+    settle = torch.cuda.synchronize if wait else lambda: None
+    settle()
+    kept = []
+    for _ in range(steps):
+        out = layer.forward(x)
+        settle()
+        _torch(g).mul_(0.9).add_(_torch(out), alpha=0.1)
+        settle()
+        grads = layer.backward(g)
+        settle()
+        for name in Attention.PARAMS:
+            _torch(layer.param(name)).sub_(_torch(layer.param("grad_" + name)), alpha=1e-3)
+        _torch(x).add_(_torch(grads[0]), alpha=1e-2)
+        settle()
+        kept.append((out, grads))
+    result = [x.numpy(), g.numpy(), kept[-1][0].numpy()] + [layer.param(n).numpy() for n in Attention.PARAMS]
+    layer.free()
+    return result
+
+
+def _on(lib, stream, f):
+    if stream is None:
+        return f()
+    try:
+        check(lib.boat_cuda_set_stream(stream.cuda_stream))
+        with torch.cuda.stream(stream):
+            return f()
+    finally:
+        torch.cuda.synchronize()
+        check(lib.boat_cuda_set_stream(None))
+
+
+@pytest.mark.parametrize("mma", [capi.MMA_FP32, capi.MMA_TF32], ids=["fp32", "tf32"])
+@pytest.mark.parametrize("own", [False, True], ids=["default stream", "a stream of its own"])
+def test_kernels_of_the_program_between_two_calls(gpu_lib, mma, own):
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream() if own else None
+    got, want = (_on(gpu_lib, stream, lambda: _train(mma, wait)) for wait in (False, True))
+    for a, b in zip(got, want):
+        assert np.isfinite(a).all() and a.tobytes() == b.tobytes()
+
+
+def test_two_threads_on_one_stream(gpu_lib):
+    want = _train(capi.MMA_FP32, True)
+    got = {}
+    threads = [threading.Thread(target=lambda i=i: got.__setitem__(i, _train(capi.MMA_FP32, False))) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        for a, b in zip(got[i], want):
+            assert a.tobytes() == b.tobytes()
