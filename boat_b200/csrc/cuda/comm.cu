@@ -165,6 +165,7 @@ static int agree_on_length(int64_t n) {
     if (!d) return set_error(24, "all-reduce: no memory for the bucket-length agreement (%s)", boat_cuda_last_error());
     int64_t h[2] = {n, -n};
     int rc = small_put(d, h, sizeof h);
+    ordinary_launch_next();
     if (rc == 0)
         rc = settle("bucket-length agreement",
                     g_nccl.AllReduce(d, d, 2, ncclInt64, ncclMax, g_comm, g_nccl.fake ? (cudaStream_t)0 : stream()),
@@ -243,6 +244,7 @@ int boat_cuda_allreduce_sum_f32(float* buf, int64_t n) {
     if (g_world <= 1 || n <= 0) return 0;
     if (!g_comm) return set_error(22, "boat_cuda_allreduce_sum_f32: no communicator");
     if (int rc = agree_on_length(n)) return rc;
+    ordinary_launch_next();                          // what follows on the library stream waits for the sum
     return settle("gradient all-reduce",
                   g_nccl.AllReduce(buf, buf, (size_t)n, ncclFloat32, ncclSum, g_comm,
                                    g_nccl.fake ? (cudaStream_t)0 : stream()),

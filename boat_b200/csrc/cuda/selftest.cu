@@ -31,6 +31,7 @@ extern "C" int boat_cuda_selftest_wait_timeout(uint64_t limit_ns) {
     if (int rc = ensure_init()) return rc;
     if (limit_ns == 0 || limit_ns > 1000000000ull)
         return set_error(11, "boat_cuda_selftest_wait_timeout: limit must be between 1 ns and 1 s");
+    ordinary_launch_next();
     wait_timeout_kernel<<<1, 32, 0, stream()>>>(kernel_status_ptr(), (unsigned long long)limit_ns);
     BOATCU_LAUNCH_OK("wait_timeout_selftest");
     return 0;
