@@ -19,12 +19,14 @@ public:
     struct Place {
         uint64_t sequence;       // 0: none, the launch stands alone
         const void* stream;
-        bool operator==(const Place& o) const { return sequence == o.sequence && stream == o.stream; }
+        bool per_thread;         // the handle stands for another stream in every thread: nothing follows from it
+        bool alone() const { return sequence == 0 || per_thread; }
+        bool operator==(const Place& o) const { return sequence == o.sequence && stream == o.stream && per_thread == o.per_thread; }
     };
 
     // One launch: begin, name() for all that it touches, beside(), end.
     void begin(const Place& place) {
-        if (place.sequence == 0 || !(place == place_)) count_ = 0;
+        if (place.alone() || !(place == place_)) count_ = 0;
         place_ = place;
         before_ = count_;
         named_ = overflow_ = beside_ = false;
@@ -44,7 +46,7 @@ public:
         return beside_;
     }
     void end() {
-        if (!named_ || overflow_ || place_.sequence == 0) {
+        if (!named_ || overflow_ || place_.alone()) {
             count_ = 0;
         } else if (!beside_) {                  // the launches before are complete once this one lets its successors go
             for (int i = before_; i < count_; ++i) ranges_[i - before_] = ranges_[i];
@@ -64,7 +66,7 @@ private:
     int count_ = 0;              // 0: the next launch waits
     int before_ = 0;             // ranges of the launches before the present one
     bool named_ = false, overflow_ = false, beside_ = false;
-    Place place_ = {0, nullptr};
+    Place place_ = {0, nullptr, false};
 };
 
 }  // namespace boatcu

@@ -46,7 +46,7 @@ static thread_local int t_sequence_depth = 0;
 
 LaunchTurn::LaunchTurn() {
     g_turn.lock();
-    g_order.begin({t_sequence_depth > 0 ? t_sequence : 0, (const void*)g_stream});
+    g_order.begin({t_sequence_depth > 0 ? t_sequence : 0, (const void*)g_stream, g_stream == cudaStreamPerThread});
 }
 LaunchTurn::~LaunchTurn() {
     g_order.end();

@@ -34,7 +34,7 @@ static void launch_unnamed(LaunchOrder& o, LaunchOrder::Place at) {
 
 static void within_a_sequence() {
     LaunchOrder o;
-    const LaunchOrder::Place at = {1, &stream_a};
+    const LaunchOrder::Place at = {1, &stream_a, false};
     expect(!launch(o, at, {X, Y}, {dW}), "the first launch of a sequence waits");
     expect(launch(o, at, {Y, W}, {dX}), "what depends on nothing that runs goes beside");
     expect(!launch(o, at, {dX}, {Z}), "read after write");
@@ -52,45 +52,47 @@ static void within_a_sequence() {
 // library's launches alone, in which nothing writes W.
 static void a_kernel_of_the_program_between_two_calls() {
     LaunchOrder o;
-    launch(o, {1, &stream_a}, {Y, W}, {dX});
-    expect(!launch(o, {2, &stream_a}, {X, W}, {Z}), "the first launch of the next call");
-    launch(o, {0, &stream_a}, {Y, W}, {dX});
-    expect(!launch(o, {0, &stream_a}, {X, W}, {Z}), "calls outside a sequence");
-    launch(o, {0, &stream_a}, {Y, W}, {dX});
-    expect(!launch(o, {3, &stream_a}, {X, W}, {Z}), "a sequence behind such a call");
+    launch(o, {1, &stream_a, false}, {Y, W}, {dX});
+    expect(!launch(o, {2, &stream_a, false}, {X, W}, {Z}), "the first launch of the next call");
+    launch(o, {0, &stream_a, false}, {Y, W}, {dX});
+    expect(!launch(o, {0, &stream_a, false}, {X, W}, {Z}), "calls outside a sequence");
+    launch(o, {0, &stream_a, false}, {Y, W}, {dX});
+    expect(!launch(o, {3, &stream_a, false}, {X, W}, {Z}), "a sequence behind such a call");
 }
 
 // A sum over the ranks on the library stream, which the table does not see, then a step on the summed gradients.
 static void a_collective_between_two_calls() {
     LaunchOrder o;
-    launch(o, {1, &stream_a}, {X, Y}, {dW});
-    launch(o, {1, &stream_a}, {Y, W}, {dX});
-    launch(o, {1, &stream_a}, {Z}, {Y});
-    expect(!launch(o, {0, &stream_a}, {dW}, {W}), "a step on gradients that were just summed");
+    launch(o, {1, &stream_a, false}, {X, Y}, {dW});
+    launch(o, {1, &stream_a, false}, {Y, W}, {dX});
+    launch(o, {1, &stream_a, false}, {Z}, {Y});
+    expect(!launch(o, {0, &stream_a, false}, {dW}, {W}), "a step on gradients that were just summed");
 }
 
 // Two threads, whose launches go to one stream or, on the per-thread default stream, to two under one handle: B writes Y,
 // A's launches take B's out of the table, B reads Y.
-static void two_threads_take_turns() {
+static void two_threads_take_turns(bool per_thread) {
     LaunchOrder o;
-    const LaunchOrder::Place a = {1, &stream_a}, b = {2, &stream_a};
+    const LaunchOrder::Place a = {1, &stream_a, per_thread}, b = {2, &stream_a, per_thread};
     launch(o, b, {X}, {Y});
     expect(!launch(o, a, {W}, {dW}), "A behind B");
     expect(!launch(o, a, {dW}, {dX}), "A behind itself");
     expect(!launch(o, b, {Y}, {Z}), "B behind A");
+    expect(launch(o, b, {W}, {dX}) == !per_thread, "beside, but on no per-thread stream");
 }
 
 static void another_stream() {
     LaunchOrder o;
-    launch(o, {1, &stream_a}, {X}, {Y});
-    expect(!launch(o, {1, &stream_b}, {W}, {Z}), "the first launch on another stream");
+    launch(o, {1, &stream_a, false}, {X}, {Y});
+    expect(!launch(o, {1, &stream_b, false}, {W}, {Z}), "the first launch on another stream");
 }
 
 int main() {
     within_a_sequence();
     a_kernel_of_the_program_between_two_calls();
     a_collective_between_two_calls();
-    two_threads_take_turns();
+    two_threads_take_turns(false);
+    two_threads_take_turns(true);
     another_stream();
     printf("ok\n");
     return 0;

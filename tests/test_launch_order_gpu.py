@@ -76,14 +76,29 @@ def test_kernels_of_the_program_between_two_calls(gpu_lib, mma, own):
         assert np.isfinite(a).all() and a.tobytes() == b.tobytes()
 
 
-def test_two_threads_on_one_stream(gpu_lib):
+PER_THREAD = 2          # cudaStreamPerThread
+
+
+@pytest.mark.parametrize("per_thread", [False, True], ids=["one stream", "a stream per thread"])
+def test_two_threads(gpu_lib, per_thread):
     want = _train(capi.MMA_FP32, True)
     got = {}
-    threads = [threading.Thread(target=lambda i=i: got.__setitem__(i, _train(capi.MMA_FP32, False))) for i in range(2)]
-    for t in threads:
-        t.start()
-    for t in threads:
-        t.join()
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.ExternalStream(PER_THREAD) if per_thread else torch.cuda.default_stream()):
+            got[i] = _train(capi.MMA_FP32, False)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    try:
+        check(gpu_lib.boat_cuda_set_stream(PER_THREAD if per_thread else None))
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        torch.cuda.synchronize()
+        check(gpu_lib.boat_cuda_set_stream(None))
     for i in range(2):
         for a, b in zip(got[i], want):
             assert a.tobytes() == b.tobytes()
