@@ -90,17 +90,22 @@ public:
     void reads(const void* p, int64_t rows, int64_t cols, int64_t ld, size_t es) { reads(p, span(rows, cols, ld, es)); }
     void writes(const void* p, int64_t rows, int64_t cols, int64_t ld, size_t es) { writes(p, span(rows, cols, ld, es)); }
     int follow();
+    cudaError_t launched(cudaError_t err) {      // a turn without a launch that worked leaves nothing to be beside of
+        launched_ = err == cudaSuccess;
+        return err;
+    }
 
 private:
     static size_t span(int64_t rows, int64_t cols, int64_t ld, size_t es) { return rows > 0 && cols > 0 ? (size_t)((rows - 1) * ld + cols) * es : 0; }
     void name(const void* p, size_t bytes, bool written);
+    bool launched_ = false;
 };
 
 // Something other than a named kernel comes next on the library stream, or the stream changes.
 void ordinary_launch_next();
 
 template <typename... P, typename... A>
-inline cudaError_t launch_in_turn(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
+inline cudaError_t launch_in_turn(LaunchTurn& turn, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -114,12 +119,12 @@ inline cudaError_t launch_in_turn(void (*kern)(P...), dim3 grid, dim3 block, siz
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    return turn.launched(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
 }
 template <typename... P, typename... A>
 inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, A&&... args) {
     LaunchTurn turn;
-    return launch_in_turn(kern, grid, block, smem, cluster, static_cast<A&&>(args)...);
+    return launch_in_turn(turn, kern, grid, block, smem, cluster, static_cast<A&&>(args)...);
 }
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
@@ -133,8 +138,8 @@ inline int spread_smem(int smem, int64_t ctas) {
     return smem > least ? smem : least;
 }
 
-#define BOATCU_RUN_IN_TURN(kern, grid, block, smem, ...) \
-    BOATCU_CHECK(boatcu::launch_in_turn(kern, dim3(grid), dim3(block), smem, 1, __VA_ARGS__))
+#define BOATCU_RUN_IN_TURN(turn, kern, grid, block, smem, ...) \
+    BOATCU_CHECK(boatcu::launch_in_turn(turn, kern, dim3(grid), dim3(block), smem, 1, __VA_ARGS__))
 #define BOATCU_RUN(kern, grid, block, smem, ...) \
     BOATCU_CHECK(boatcu::launch_dependent(kern, dim3(grid), dim3(block), smem, 1, __VA_ARGS__))
 

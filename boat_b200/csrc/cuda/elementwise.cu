@@ -68,9 +68,9 @@ static int launch_axpy(float* y, const float* x, float alpha, int64_t n) {
     turn.writes(y, (size_t)n * 4);
     const int follow = turn.follow();
     if (aligned16(y) && aligned16(x) && (n % 4) == 0) {
-        BOATCU_RUN_IN_TURN(axpy_vec4<ACCUM>, grid_for(n / 4, kThreads), kThreads, 0, y, x, alpha, n / 4, follow);
+        BOATCU_RUN_IN_TURN(turn, axpy_vec4<ACCUM>, grid_for(n / 4, kThreads), kThreads, 0, y, x, alpha, n / 4, follow);
     } else {
-        BOATCU_RUN_IN_TURN(axpy_scalar<ACCUM>, grid_for(n, kThreads), kThreads, 0, y, x, alpha, n, follow);
+        BOATCU_RUN_IN_TURN(turn, axpy_scalar<ACCUM>, grid_for(n, kThreads), kThreads, 0, y, x, alpha, n, follow);
     }
     BOATCU_LAUNCH_OK("axpy");
     return 0;
@@ -426,7 +426,7 @@ static int launch_colsum_cluster(const ColsumTable& t, int64_t rows, int64_t col
             turn.reads(t.x[i], (size_t)rows * cols * sizeof(T));
             turn.writes(t.out[i], (size_t)cols * 4);
         }
-        BOATCU_CHECK(launch_in_turn(colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)n, (unsigned)count),
+        BOATCU_CHECK(launch_in_turn(turn, colsum_kernel<T, VEC, LANES, 512, true>, dim3(kColsumCluster, (unsigned)n, (unsigned)count),
                                     dim3(512), 0, kColsumCluster, t, rows, cols, first, turn.follow()));
         BOATCU_LAUNCH_OK("colsum");
     }
@@ -715,7 +715,7 @@ int boat_cuda_sgd_clear(float* const* y, float* const* g, float lr, const int64_
         turn.writes(y[i], (size_t)n[i] * 4);
         turn.writes(g[i], (size_t)n[i] * 4);
     }
-    BOATCU_RUN_IN_TURN(sgd_clear_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, lr,
+    BOATCU_RUN_IN_TURN(turn, sgd_clear_kernel, dim3((unsigned)grid_for(vec ? ceil_div(longest, 4) : longest, kThreads), (unsigned)count), kThreads, 0, t, lr,
                        vec, turn.follow());
     BOATCU_LAUNCH_OK("sgd_clear");
     return 0;
@@ -752,9 +752,9 @@ int boat_cuda_cast(void* dst, int dst_type, const void* src, int src_type, int64
     turn.writes(dst, (size_t)n * type_size(dst_type));
     const int follow = turn.follow();
     if (dst_type == BOAT_CUDA_BF16)
-        BOATCU_RUN_IN_TURN(cast_f32_to_bf16, grid, kThreads, 0, (__nv_bfloat16*)dst, (const float*)src, n, vec, follow);
+        BOATCU_RUN_IN_TURN(turn, cast_f32_to_bf16, grid, kThreads, 0, (__nv_bfloat16*)dst, (const float*)src, n, vec, follow);
     else
-        BOATCU_RUN_IN_TURN(cast_bf16_to_f32, grid, kThreads, 0, (float*)dst, (const __nv_bfloat16*)src, n, vec, follow);
+        BOATCU_RUN_IN_TURN(turn, cast_bf16_to_f32, grid, kThreads, 0, (float*)dst, (const __nv_bfloat16*)src, n, vec, follow);
     BOATCU_LAUNCH_OK("cast");
     return 0;
 }
@@ -772,10 +772,10 @@ int boat_cuda_lincomb(void* y, const void* a, float alpha, const void* b, float 
     turn.writes(y, (size_t)n * type_size(type));
     const int follow = turn.follow();
     if (type == BOAT_CUDA_BF16)
-        BOATCU_RUN_IN_TURN(lincomb_kernel<__nv_bfloat16>, grid, kThreads, 0, (__nv_bfloat16*)y, (const __nv_bfloat16*)a, alpha,
+        BOATCU_RUN_IN_TURN(turn, lincomb_kernel<__nv_bfloat16>, grid, kThreads, 0, (__nv_bfloat16*)y, (const __nv_bfloat16*)a, alpha,
                                                                        (const __nv_bfloat16*)b, beta, n, vec, follow);
     else
-        BOATCU_RUN_IN_TURN(lincomb_kernel<float>, grid, kThreads, 0, (float*)y, (const float*)a, alpha, (const float*)b, beta, n, vec, follow);
+        BOATCU_RUN_IN_TURN(turn, lincomb_kernel<float>, grid, kThreads, 0, (float*)y, (const float*)a, alpha, (const float*)b, beta, n, vec, follow);
     BOATCU_LAUNCH_OK("lincomb");
     return 0;
 }
@@ -788,7 +788,7 @@ int boat_cuda_round_tf32(float* y, const float* x, int64_t n) {
     LaunchTurn turn;
     turn.reads(x, (size_t)n * 4);
     turn.writes(y, (size_t)n * 4);
-    BOATCU_RUN_IN_TURN(round_tf32_kernel, grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, y, x, n, vec, turn.follow());
+    BOATCU_RUN_IN_TURN(turn, round_tf32_kernel, grid_for(vec ? n / 4 : n, kThreads), kThreads, 0, y, x, n, vec, turn.follow());
     BOATCU_LAUNCH_OK("round_tf32");
     return 0;
 }
@@ -863,8 +863,8 @@ int boat_cuda_convert_multi(void* const* dst, int dst_type, const float* const* 
         turn.writes(dst[i], (size_t)n[i] * type_size(dst_type));
     }
     const int follow = turn.follow();
-    if (dst_type == BOAT_CUDA_BF16) BOATCU_RUN_IN_TURN(convert_multi_kernel<true>, grid, kThreads, 0, t, vec, follow);
-    else                            BOATCU_RUN_IN_TURN(convert_multi_kernel<false>, grid, kThreads, 0, t, vec, follow);
+    if (dst_type == BOAT_CUDA_BF16) BOATCU_RUN_IN_TURN(turn, convert_multi_kernel<true>, grid, kThreads, 0, t, vec, follow);
+    else                            BOATCU_RUN_IN_TURN(turn, convert_multi_kernel<false>, grid, kThreads, 0, t, vec, follow);
     BOATCU_LAUNCH_OK("convert_multi");
     return 0;
 }

@@ -398,7 +398,7 @@ int launch_tile(SimtParams& p, int groups, int split) {
         LaunchTurn turn;
         name_memory(turn, p, groups, A_M, B_K, sizeof(TI), sizeof(TO));
         p.follow = turn.follow();
-        BOATCU_CHECK(launch_in_turn(kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), smem, (unsigned)split, p));
+        BOATCU_CHECK(launch_in_turn(turn, kern, dim3((unsigned)(tiles * split), 1, (unsigned)groups), dim3(256), smem, (unsigned)split, p));
     }
     BOATCU_LAUNCH_OK("gemm_simt");
     return 0;
@@ -517,7 +517,7 @@ int gemm_simt_grads(int groups, int64_t T, int64_t I, int64_t O, const void* con
     name_memory(turn, w, groups, true, false, 4, 4);
     name_memory(turn, x, groups, false, true, 4, 4);
     w.follow = x.follow = turn.follow();
-    BOATCU_CHECK(launch_in_turn(gemm_simt_grads_kernel, dim3((unsigned)grid), dim3(256), spread_smem(need, grid), (unsigned)cw.split, w, x, groups,
+    BOATCU_CHECK(launch_in_turn(turn, gemm_simt_grads_kernel, dim3((unsigned)grid), dim3(256), spread_smem(need, grid), (unsigned)cw.split, w, x, groups,
                                 (int)dw_blocks, (int)dx_blocks));
     BOATCU_LAUNCH_OK("gemm_simt_grads");
     return 0;

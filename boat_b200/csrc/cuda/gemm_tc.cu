@@ -647,7 +647,7 @@ int clear(const Problem& q, bool sums) {
     LaunchTurn turn;
     for (int i = 0; i < count; ++i) turn.writes(t.out[i], i < t.matrices ? q.M : 1, q.N, i < t.matrices ? q.ldc : q.N, 4);
     t.follow = turn.follow();
-    BOATCU_CHECK(launch_in_turn(clear_kernel, dim3((unsigned)(blocks < most ? blocks : most), (unsigned)count), dim3(256), 0, 1, t));
+    BOATCU_CHECK(launch_in_turn(turn, clear_kernel, dim3((unsigned)(blocks < most ? blocks : most), (unsigned)count), dim3(256), 0, 1, t));
     BOATCU_LAUNCH_OK("gemm_tc clear");
     return 0;
 }
@@ -718,7 +718,7 @@ int launch(const Problem& q, const Plan& plan) {
         }
         turn.writes(q.aux, q.M, q.N, q.ldc, 2);
         p.follow = turn.follow();
-        BOATCU_CHECK(launch_in_turn(kern, dim3((unsigned)grid), dim3(kThreads + (CSUM ? 32 * kSumWarps : 0)), C::SMEM, CTAS, maps, p));
+        BOATCU_CHECK(launch_in_turn(turn, kern, dim3((unsigned)grid), dim3(kThreads + (CSUM ? 32 * kSumWarps : 0)), C::SMEM, CTAS, maps, p));
     }
     BOATCU_LAUNCH_OK("gemm_tc");
     return 0;

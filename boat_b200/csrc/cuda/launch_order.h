@@ -24,7 +24,7 @@ public:
         bool operator==(const Place& o) const { return sequence == o.sequence && stream == o.stream && per_thread == o.per_thread; }
     };
 
-    // One launch: begin, name() for all that it touches, beside(), end.
+    // One launch: begin, name() for all that it touches, beside(), end - which is told whether it got onto the stream.
     void begin(const Place& place) {
         if (place.alone() || !(place == place_)) count_ = 0;
         place_ = place;
@@ -45,8 +45,8 @@ public:
                 beside_ = ranges_[i].hi <= ranges_[j].lo || ranges_[j].hi <= ranges_[i].lo || !(ranges_[i].written || ranges_[j].written);
         return beside_;
     }
-    void end() {
-        if (!named_ || overflow_ || place_.alone()) {
+    void end(bool launched) {
+        if (!launched || !named_ || overflow_ || place_.alone()) {
             count_ = 0;
         } else if (!beside_) {                  // the launches before are complete once this one lets its successors go
             for (int i = before_; i < count_; ++i) ranges_[i - before_] = ranges_[i];

@@ -488,7 +488,7 @@ static int layernorm_fwd_launch(const void* x, int64_t rows, int64_t cols, const
     turn.writes(y, (size_t)rows * cols * sizeof(T));
     turn.writes(mean_out, (size_t)rows * 4);
     turn.writes(rstd_out, (size_t)rows * 4);
-    BOATCU_RUN_IN_TURN((layernorm_fwd_rows_kernel<T, NV>), (unsigned)blocks, kNormThreads, smem, (const T*)x, rows, (int)cols, gamma, beta, eps, (T*)y,
+    BOATCU_RUN_IN_TURN(turn, (layernorm_fwd_rows_kernel<T, NV>), (unsigned)blocks, kNormThreads, smem, (const T*)x, rows, (int)cols, gamma, beta, eps, (T*)y,
                        mean_out, rstd_out, turn.follow());
     BOATCU_LAUNCH_OK("layernorm_fwd_rows");
     return 0;

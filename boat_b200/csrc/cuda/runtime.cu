@@ -49,7 +49,7 @@ LaunchTurn::LaunchTurn() {
     g_order.begin({t_sequence_depth > 0 ? t_sequence : 0, (const void*)g_stream, g_stream == cudaStreamPerThread});
 }
 LaunchTurn::~LaunchTurn() {
-    g_order.end();
+    g_order.end(launched_);
     g_turn.unlock();
 }
 void LaunchTurn::name(const void* p, size_t bytes, bool written) { g_order.name(p, bytes, written); }

@@ -23,13 +23,13 @@ static bool launch(LaunchOrder& o, LaunchOrder::Place at, List reads, List write
     for (const char* p : reads) o.name(p, 64, false);
     for (const char* p : writes) o.name(p, 64, true);
     const bool beside = o.beside();
-    o.end();
+    o.end(true);
     return beside;
 }
 
 static void launch_unnamed(LaunchOrder& o, LaunchOrder::Place at) {
     o.begin(at);
-    o.end();
+    o.end(true);
 }
 
 static void within_a_sequence() {
@@ -87,6 +87,23 @@ static void another_stream() {
     expect(!launch(o, {1, &stream_b, false}, {W}, {Z}), "the first launch on another stream");
 }
 
+// A launch that fails - of which nothing runs - takes no place in the table, and the launches before it may still be running.
+static void a_launch_that_fails() {
+    LaunchOrder o;
+    const LaunchOrder::Place at = {1, &stream_a, false};
+    launch(o, at, {X}, {Y});
+    o.begin(at);
+    o.name(Y, 64, false);
+    o.name(Z, 64, true);
+    expect(!o.beside(), "what depends on the one before");
+    o.end(false);
+    expect(!launch(o, at, {Y}, {dX}), "the first launch behind one that failed");
+    launch(o, at, {X}, {Y});
+    o.begin(at);
+    o.end(false);                                   // a turn that ends before its launch
+    expect(!launch(o, at, {Y}, {dX}), "the first launch behind none");
+}
+
 int main() {
     within_a_sequence();
     a_kernel_of_the_program_between_two_calls();
@@ -94,6 +111,7 @@ int main() {
     two_threads_take_turns(false);
     two_threads_take_turns(true);
     another_stream();
+    a_launch_that_fails();
     printf("ok\n");
     return 0;
 }
