@@ -20,8 +20,11 @@ public:
         uint64_t sequence;       // 0: none, the launch stands alone
         const void* stream;
         bool per_thread;         // the handle stands for another stream in every thread: nothing follows from it
+        uint64_t capture;        // of the stream, while it is being captured: what goes into a graph does not run now
         bool alone() const { return sequence == 0 || per_thread; }
-        bool operator==(const Place& o) const { return sequence == o.sequence && stream == o.stream && per_thread == o.per_thread; }
+        bool operator==(const Place& o) const {
+            return sequence == o.sequence && stream == o.stream && per_thread == o.per_thread && capture == o.capture;
+        }
     };
 
     // One launch: begin, name() for all that it touches, beside(), end - which is told whether it got onto the stream.
@@ -66,7 +69,7 @@ private:
     int count_ = 0;              // 0: the next launch waits
     int before_ = 0;             // ranges of the launches before the present one
     bool named_ = false, overflow_ = false, beside_ = false;
-    Place place_ = {0, nullptr, false};
+    Place place_ = {0, nullptr, false, 0};
 };
 
 }  // namespace boatcu

@@ -44,9 +44,22 @@ static std::atomic<uint64_t> g_sequences{0};
 static thread_local uint64_t t_sequence = 0;   // of this thread, while t_sequence_depth > 0
 static thread_local int t_sequence_depth = 0;
 
+// The capture that the library stream is in, 0 for none.
+static bool current_capture(uint64_t& id) {
+    id = 0;
+    if (g_stream == 0 || g_stream == cudaStreamLegacy) return true;         // cannot be captured
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    if (cudaStreamGetCaptureInfo(g_stream, &status, &capture) != cudaSuccess) return cudaGetLastError(), false;
+    if (status != cudaStreamCaptureStatusNone) id = capture;
+    return true;
+}
+
 LaunchTurn::LaunchTurn() {
     g_turn.lock();
-    g_order.begin({t_sequence_depth > 0 ? t_sequence : 0, (const void*)g_stream, g_stream == cudaStreamPerThread});
+    LaunchOrder::Place place = {t_sequence_depth > 0 ? t_sequence : 0, (const void*)g_stream, g_stream == cudaStreamPerThread, 0};
+    if (!place.alone() && !current_capture(place.capture)) place.sequence = 0;
+    g_order.begin(place);
 }
 LaunchTurn::~LaunchTurn() {
     g_order.end(launched_);

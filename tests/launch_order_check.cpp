@@ -34,7 +34,7 @@ static void launch_unnamed(LaunchOrder& o, LaunchOrder::Place at) {
 
 static void within_a_sequence() {
     LaunchOrder o;
-    const LaunchOrder::Place at = {1, &stream_a, false};
+    const LaunchOrder::Place at = {1, &stream_a, false, 0};
     expect(!launch(o, at, {X, Y}, {dW}), "the first launch of a sequence waits");
     expect(launch(o, at, {Y, W}, {dX}), "what depends on nothing that runs goes beside");
     expect(!launch(o, at, {dX}, {Z}), "read after write");
@@ -52,28 +52,28 @@ static void within_a_sequence() {
 // library's launches alone, in which nothing writes W.
 static void a_kernel_of_the_program_between_two_calls() {
     LaunchOrder o;
-    launch(o, {1, &stream_a, false}, {Y, W}, {dX});
-    expect(!launch(o, {2, &stream_a, false}, {X, W}, {Z}), "the first launch of the next call");
-    launch(o, {0, &stream_a, false}, {Y, W}, {dX});
-    expect(!launch(o, {0, &stream_a, false}, {X, W}, {Z}), "calls outside a sequence");
-    launch(o, {0, &stream_a, false}, {Y, W}, {dX});
-    expect(!launch(o, {3, &stream_a, false}, {X, W}, {Z}), "a sequence behind such a call");
+    launch(o, {1, &stream_a, false, 0}, {Y, W}, {dX});
+    expect(!launch(o, {2, &stream_a, false, 0}, {X, W}, {Z}), "the first launch of the next call");
+    launch(o, {0, &stream_a, false, 0}, {Y, W}, {dX});
+    expect(!launch(o, {0, &stream_a, false, 0}, {X, W}, {Z}), "calls outside a sequence");
+    launch(o, {0, &stream_a, false, 0}, {Y, W}, {dX});
+    expect(!launch(o, {3, &stream_a, false, 0}, {X, W}, {Z}), "a sequence behind such a call");
 }
 
 // A sum over the ranks on the library stream, which the table does not see, then a step on the summed gradients.
 static void a_collective_between_two_calls() {
     LaunchOrder o;
-    launch(o, {1, &stream_a, false}, {X, Y}, {dW});
-    launch(o, {1, &stream_a, false}, {Y, W}, {dX});
-    launch(o, {1, &stream_a, false}, {Z}, {Y});
-    expect(!launch(o, {0, &stream_a, false}, {dW}, {W}), "a step on gradients that were just summed");
+    launch(o, {1, &stream_a, false, 0}, {X, Y}, {dW});
+    launch(o, {1, &stream_a, false, 0}, {Y, W}, {dX});
+    launch(o, {1, &stream_a, false, 0}, {Z}, {Y});
+    expect(!launch(o, {0, &stream_a, false, 0}, {dW}, {W}), "a step on gradients that were just summed");
 }
 
 // Two threads, whose launches go to one stream or, on the per-thread default stream, to two under one handle: B writes Y,
 // A's launches take B's out of the table, B reads Y.
 static void two_threads_take_turns(bool per_thread) {
     LaunchOrder o;
-    const LaunchOrder::Place a = {1, &stream_a, per_thread}, b = {2, &stream_a, per_thread};
+    const LaunchOrder::Place a = {1, &stream_a, per_thread, 0}, b = {2, &stream_a, per_thread, 0};
     launch(o, b, {X}, {Y});
     expect(!launch(o, a, {W}, {dW}), "A behind B");
     expect(!launch(o, a, {dW}, {dX}), "A behind itself");
@@ -83,14 +83,26 @@ static void two_threads_take_turns(bool per_thread) {
 
 static void another_stream() {
     LaunchOrder o;
-    launch(o, {1, &stream_a, false}, {X}, {Y});
-    expect(!launch(o, {1, &stream_b, false}, {W}, {Z}), "the first launch on another stream");
+    launch(o, {1, &stream_a, false, 0}, {X}, {Y});
+    expect(!launch(o, {1, &stream_b, false, 0}, {W}, {Z}), "the first launch on another stream");
+}
+
+// The stream goes into a capture and out of it: what is launched in between goes into a graph and does not run now.
+static void a_capture_begins_or_ends() {
+    LaunchOrder o;
+    const LaunchOrder::Place eager = {1, &stream_a, false, 0}, captured = {1, &stream_a, false, 7}, next = {1, &stream_a, false, 8};
+    launch(o, eager, {X}, {Y});
+    expect(!launch(o, captured, {W}, {Z}), "the first launch of a capture");
+    expect(launch(o, captured, {W}, {dX}), "beside another of the capture");
+    expect(!launch(o, eager, {Y}, {dW}), "the first launch behind a capture");
+    launch(o, captured, {X}, {Y});
+    expect(!launch(o, next, {W}, {Z}), "the first launch of the next capture");
 }
 
 // A launch that fails - of which nothing runs - takes no place in the table, and the launches before it may still be running.
 static void a_launch_that_fails() {
     LaunchOrder o;
-    const LaunchOrder::Place at = {1, &stream_a, false};
+    const LaunchOrder::Place at = {1, &stream_a, false, 0};
     launch(o, at, {X}, {Y});
     o.begin(at);
     o.name(Y, 64, false);
@@ -111,6 +123,7 @@ int main() {
     two_threads_take_turns(false);
     two_threads_take_turns(true);
     another_stream();
+    a_capture_begins_or_ends();
     a_launch_that_fails();
     printf("ok\n");
     return 0;

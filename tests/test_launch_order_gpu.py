@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from boat_b200 import capi, rng
-from boat_b200.host import Attention, Tensor, check
+from boat_b200.host import Attention, DeviceBuffer, Tensor, check
 
 pytestmark = pytest.mark.gpu
 B, S, D, NH = 4, 128, 256, 4
@@ -102,3 +102,34 @@ def test_two_threads(gpu_lib, per_thread):
     for i in range(2):
         for a, b in zip(got[i], want):
             assert a.tobytes() == b.tobytes()
+
+
+def test_a_capture_within_a_sequence(gpu_lib):
+    """Products into a graph between eager ones, some of either independent of one another; the graph runs at the end."""
+    n, stream, graph = 192, torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    host = [rng.normal(43, i, (n, n)) / np.float32(14) for i in range(3)]
+
+    def play():
+        x, w, v = (DeviceBuffer.from_numpy(a) for a in host)
+        out = [DeviceBuffer(n * n * 4) for _ in range(6)]
+        gemm = lambda c, a, b: check(gpu_lib.boat_cuda_gemm(capi.MMA_FP32, 0, 0, n, n, n, a.p, n, b.p, n, capi.CUDA_F32, c.p, n,  # noqa: E731
+                                                            capi.CUDA_F32, None))
+        gpu_lib.boat_cuda_launches_begin()
+        gemm(out[0], x, w)
+        with torch.cuda.graph(graph, stream=stream):
+            gemm(out[1], v, out[2])
+            gemm(out[3], v, w)
+        gemm(out[2], out[0], w)
+        gemm(out[4], x, x)
+        gemm(out[5], out[2], out[4])
+        gpu_lib.boat_cuda_launches_end()
+        graph.replay()
+        return [b.numpy((n, n)) for b in out]
+
+    got = _on(gpu_lib, stream, play)
+    x, w, v = (a.astype(np.float64) for a in host)
+    want = [x @ w, v @ (x @ w @ w), x @ w @ w, v @ w, x @ x, (x @ w @ w) @ (x @ x)]
+    for a, b in zip(got, want):
+        # sums of n products in FP32, three deep: 3 * sqrt(n) * 2^-24 of the norms in the mean, with a margin of ten
+        assert np.linalg.norm(a - b) <= 30 * np.sqrt(n) * 2.0**-24 * np.linalg.norm(b)
+    del graph
