@@ -98,6 +98,8 @@ struct Params {
     const float* bias[kMaxGroups];
     float* colsum[kMaxGroups];       // sums over K of B's columns
     int colsum_add;      // ... are added to what is there
+    float* part_sums;    // [groups][split][N]: those of the pieces of split tiles
+    unsigned int* arrived;           // zeros: pieces whose sums are there, per group, column of tiles, CTA of a pair and warp
     int groups;
     int chain;           // the groups' products are summed into one result
     int M, N, K;
@@ -112,7 +114,8 @@ struct Params {
 
 struct WorkItem {
     int g, m0, n0, kb0, kb1;
-    bool first, add;     // first piece of its tile (adds the bias); result is added to the output
+    int part, pieces;    // which piece of its tile; the first adds the bias
+    bool add;            // result is added to the output
 };
 
 template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI, bool CSUM>
@@ -151,16 +154,15 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         // pieces of one K range are neighbours: the CTAs at work together share the rows they stream
         const int rest = tiles - p.full;
         const int tile = w < p.full ? w : p.full + (w - p.full) % rest;
-        const int part = w < p.full ? 0 : (w - p.full) / rest;
-        const int pieces = w < p.full ? 1 : p.split;
+        it.part = w < p.full ? 0 : (w - p.full) / rest;
+        it.pieces = w < p.full ? 1 : p.split;
         const int mn = tile / results;
         it.g = tile % results;
         it.m0 = (mn / n_tiles) * BM * CTAS + (int)rank * BM;
         it.n0 = (mn % n_tiles) * BN;
-        it.kb0 = (int)((int64_t)part * k_blocks / pieces);
-        it.kb1 = (int)((int64_t)(part + 1) * k_blocks / pieces);
-        it.first = part == 0;
-        it.add = pieces > 1 || p.add_all;
+        it.kb0 = (int)((int64_t)it.part * k_blocks / it.pieces);
+        it.kb1 = (int)((int64_t)(it.part + 1) * k_blocks / it.pieces);
+        it.add = it.pieces > 1 || p.add_all;
         return it;
     };
 
@@ -311,7 +313,8 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         // them (both CTAs of a pair hear of that; only the first hears of the loads), and hands the stage on to the
         // producer.  A warp has a quarter of the columns, a lane 16 bytes of every RL-th row; the rows are dealt out so
         // that the eight lanes of a shared-memory phase meet eight swizzle positions.  A K-block is summed for itself
-        // before it joins the total.
+        // before it joins the total.  Where the tile is one of several pieces of K the sums wait beside those of the others, and
+        // the warp that comes last adds them up in the order of the pieces: the same bits every time.
         constexpr int PER = 16 / C::ES, UW = C::BNC / PER / kSumWarps, RL = 32 / UW, PH = UW < 8 ? 8 / UW : 1;
         constexpr int PERIOD = TF32 ? 4 : 8, H = PERIOD / PH;
         const int unit = (warp - 2 - kEpiWarps) * UW + lane % UW, rl = lane / UW, u8 = unit & 7;
@@ -365,14 +368,31 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
 #pragma unroll
                 for (int d = UW; d < 32; d <<= 1) total[e] += __shfl_xor_sync(0xffffffffu, total[e], d);
             const int col = t.n0 + (int)rank * C::BNC + unit * PER;
+            if (t.pieces > 1) {
+                float* const parts = p.part_sums + (int64_t)t.g * t.pieces * p.N + col;
+                if (rl == 0) {
+#pragma unroll
+                    for (int e = 0; e < PER; ++e)
+                        if (col + e < p.N) parts[(int64_t)t.part * p.N + e] = total[e];
+                }
+                __threadfence();
+                __syncwarp();
+                unsigned int before = 0;
+                if (lane == 0) before = atomicAdd(p.arrived + ((t.g * n_tiles + t.n0 / BN) * CTAS + (int)rank) * kSumWarps + warp - 2 - kEpiWarps, 1u);
+                if (__shfl_sync(0xffffffffu, before, 0) + 1 != (unsigned int)t.pieces) continue;
+                __threadfence();
+#pragma unroll
+                for (int e = 0; e < PER; ++e) total[e] = 0.f;
+                for (int i = 0; i < t.pieces; ++i)
+#pragma unroll
+                    for (int e = 0; e < PER; ++e)
+                        if (col + e < p.N) total[e] += __ldcg(parts + (int64_t)i * p.N + e);
+            }
             if (rl == 0) {
                 float* const out = p.colsum[t.g] + col;
 #pragma unroll
-                for (int e = 0; e < PER; ++e) {
-                    if (col + e >= p.N) break;
-                    if (t.add || p.colsum_add) atomicAdd(out + e, total[e]);
-                    else                       out[e] = total[e];
-                }
+                for (int e = 0; e < PER; ++e)
+                    if (col + e < p.N) out[e] = p.colsum_add ? out[e] + total[e] : total[e];
             }
         }
     } else {
@@ -398,7 +418,7 @@ gemm_tc_kernel(const __grid_constant__ GroupMaps maps, const __grid_constant__ P
         for (int w = worker; w < work_items && ok; w += workers, ++acc_it) {
             const WorkItem t = item(w);
             const CUtensorMap* map_c = &maps.c[t.g];
-            const float* const bias = t.first ? p.bias[t.g] : nullptr;
+            const float* const bias = t.part == 0 ? p.bias[t.g] : nullptr;
             const bool bias16 = ((uintptr_t)bias & 15) == 0;
             const int buf = acc_it & 1;
             const int row0 = t.m0 + lane_group * 32;
@@ -612,11 +632,11 @@ Plan make_plan(const Problem& q, const Shape& sh, int bk, bool a_mn) {
     return r;
 }
 
-// Zeroes every output of a launch that adds pieces to them, and their column sums: one launch, in order with the others.
-// (A memset per output also keeps the GEMM from being set up behind the kernel before it.)
+// Zeroes every output of a launch that adds pieces to them, and the counters of its column sums: one launch, in order with the
+// others.  (A memset per output also keeps the GEMM from being set up behind the kernel before it.)
 struct ClearTable {
-    float* out[2 * kMaxGroups];      // matrices of `rows` rows, then vectors
-    int64_t rows, N, ldc;
+    float* out[kMaxGroups + 1];      // matrices of `rows` rows, then the counters
+    int64_t rows, N, ldc, counters;
     int matrices, follow;
 };
 
@@ -624,33 +644,56 @@ __global__ void __launch_bounds__(256) clear_kernel(const ClearTable t) {
     griddep_enter(t.follow);
     float* const out = t.out[blockIdx.y];
     const bool matrix = (int)blockIdx.y < t.matrices;
-    const int64_t ld = matrix ? t.ldc : t.N, n = (matrix ? t.rows : 1) * t.N;
+    const int64_t ld = matrix ? t.ldc : t.counters, row = matrix ? t.N : t.counters, n = matrix ? t.rows * t.N : t.counters;
     const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
-    if (ld == t.N && n % 4 == 0 && ((uintptr_t)out & 15) == 0) {
+    if (ld == row && n % 4 == 0 && ((uintptr_t)out & 15) == 0) {
         for (int64_t i = first; i < n / 4; i += step) reinterpret_cast<float4*>(out)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     } else {
-        for (int64_t i = first; i < n; i += step) out[i / t.N * ld + i % t.N] = 0.f;
+        for (int64_t i = first; i < n; i += step) out[i / row * ld + i % row] = 0.f;
     }
     griddep_leave(t.follow);
 }
 
-int clear(const Problem& q, bool sums) {
+int clear(const Problem& q, unsigned int* arrived, int64_t counters) {
     ClearTable t;
     t.rows = q.M;
     t.N = q.N;
     t.ldc = q.ldc;
-    t.matrices = q.results();
+    t.matrices = q.add ? 0 : q.results();
+    t.counters = counters;
     int count = 0;
     for (int g = 0; g < t.matrices; ++g) t.out[count++] = (float*)q.C[g];
-    for (int g = 0; g < q.groups && sums; ++g) t.out[count++] = q.colsum[g];
-    const int64_t blocks = ceil_div(q.M * q.N, 256 * 4 * 4), most = 4 * sm_count();
+    if (counters) t.out[count++] = (float*)arrived;
+    if (count == 0) return 0;
+    const int64_t blocks = ceil_div(q.add ? counters : q.M * q.N, 256 * 4 * 4), most = 4 * sm_count();
     LaunchTurn turn;
-    for (int i = 0; i < count; ++i) turn.writes(t.out[i], i < t.matrices ? q.M : 1, q.N, i < t.matrices ? q.ldc : q.N, 4);
+    for (int g = 0; g < t.matrices; ++g) turn.writes(t.out[g], q.M, q.N, q.ldc, 4);
+    turn.writes(arrived, (size_t)counters * 4);
     t.follow = turn.follow();
     BOATCU_CHECK(launch_in_turn(turn, clear_kernel, dim3((unsigned)(blocks < most ? blocks : most), (unsigned)count), dim3(256), 0, 1, t));
     BOATCU_LAUNCH_OK("gemm_tc clear");
     return 0;
 }
+
+// Memory of one launch for the column sums of split tiles, counters and then sums.  Given back in the order of the stream.
+struct PartSums {
+    unsigned int* arrived = nullptr;
+    float* sums = nullptr;
+    int64_t counters = 0;
+    size_t bytes = 0;
+    int take(int64_t count, int64_t values) {
+        counters = ceil_div(count, 4) * 4;
+        bytes = (size_t)(counters + values) * 4;
+        void* block = nullptr;
+        if (int rc = boat_cuda_malloc(&block, bytes)) return rc;
+        arrived = (unsigned int*)block;
+        sums = (float*)(arrived + counters);
+        return 0;
+    }
+    ~PartSums() {
+        if (arrived) boat_cuda_free(arrived);
+    }
+};
 
 template <typename T, bool A_MN, bool B_MN, int CTAS, int BN, int EPI, bool CSUM>
 int launch(const Problem& q, const Plan& plan) {
@@ -679,9 +722,15 @@ int launch(const Problem& q, const Plan& plan) {
     if (EPI != BOAT_EPI_NONE)
         if (int rc = make_tensor_map_2d(&maps.aux, q.aux, 2, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)q.ldc, kBoxRows, 64)) return rc;
     const int64_t full = plan.full, split = plan.split, tiles = plan.tiles, workers = sm_count() / CTAS;
-    if (split > 1 && !q.add) {
-        if (int rc = clear(q, CSUM)) return rc;
-    }
+    // the sums of split tiles: those of the first row of tiles, which come first
+    const int64_t n_tiles = ceil_div(q.N, BN), summing = n_tiles * q.groups;
+    PartSums parts;
+    if (CSUM && split > 1 && full < summing)
+        if (int rc = parts.take(summing * CTAS * kSumWarps, q.groups * split * q.N)) return rc;
+    if (split > 1)
+        if (int rc = clear(q, parts.arrived, parts.counters)) return rc;
+    p.part_sums = parts.sums;
+    p.arrived = parts.arrived;
     for (int g = 0; g < q.groups; ++g) p.colsum[g] = CSUM ? q.colsum[g] : nullptr;
     p.colsum_add = q.add ? 1 : 0;
     p.groups = q.groups;
@@ -717,6 +766,7 @@ int launch(const Problem& q, const Plan& plan) {
             turn.writes(p.colsum[g], (size_t)q.N * 4);
         }
         turn.writes(q.aux, q.M, q.N, q.ldc, 2);
+        turn.writes(parts.arrived, parts.bytes);
         p.follow = turn.follow();
         BOATCU_CHECK(launch_in_turn(turn, kern, dim3((unsigned)grid), dim3(kThreads + (CSUM ? 32 * kSumWarps : 0)), C::SMEM, CTAS, maps, p));
     }

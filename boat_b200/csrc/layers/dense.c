@@ -155,11 +155,12 @@ static boat_tensor_t* backward_steps(boat_dense_layer_t* l, const boat_tensor_t*
     /* a bias set on a layer created without one has no gradient tensor to add to: its gradient is dropped */
     boat_tensor_t* out = NULL;
     if (rc == 0 && dx && dg && dw && d_dx && target[0]) {
-        rc = pre_activation ? boat_cuda_gemm_fused(mma, BOAT_EPI_GELU_GRAD, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, NULL, pre_activation->data)
-                            : boat_cuda_gemm(mma, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, type, NULL);
+        /* first the weight gradient, which may wait for counters that it clears; the input gradient runs beside it */
+        rc = boat_cuda_weight_grads(mma, 1, I, O, N, (const void* const*)&dx, (const void* const*)&dg, type, &target[0],
+                                    target[1] ? &target[1] : NULL, 1);
         if (rc == 0)
-            rc = boat_cuda_weight_grads(mma, 1, I, O, N, (const void* const*)&dx, (const void* const*)&dg, type, &target[0],
-                                        target[1] ? &target[1] : NULL, 1);
+            rc = pre_activation ? boat_cuda_gemm_fused(mma, BOAT_EPI_GELU_GRAD, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, NULL, pre_activation->data)
+                                : boat_cuda_gemm(mma, 0, 1, N, I, O, dg, O, dw, O, type, d_dx, I, type, NULL);
         for (int i = 0; i < 2 && rc == 0; ++i)
             if (staged[i] && target[i]) rc = boat_cuda_memcpy_d2h(grads[i]->data, target[i], grads[i]->nbytes);
         if (boat_report("dense backward", rc) == 0) out = boat_emit_out_take(x->shape, 2, x, &d_dx, type);

@@ -165,6 +165,30 @@ def test_weight_grads_with_column_sums(gpu_lib, mma, I, O, T, groups):
         assert (np.abs(db[g].numpy((O,)) - y.sum(0)) <= 4 * math.sqrt(T) * 2.0 ** -25 * np.abs(y).sum(0)).all()
 
 
+# column sums over K in pieces: few and many of them, groups, CTA pairs, ragged columns, added to what is there
+@pytest.mark.parametrize("mma", [capi.MMA_BF16, capi.MMA_TF32], ids=["bf16", "tf32"])
+@pytest.mark.parametrize("I,O,T,groups,add", [(1024, 1024, 8000, 3, 0), (128, 64, 20000, 1, 0), (256, 520, 9001, 1, 1), (1024, 1024, 8000, 1, 1),
+                                              (1024, 4096, 4096, 1, 1)])
+def test_column_sums_have_the_same_bits_every_time(gpu_lib, mma, I, O, T, groups, add):
+    bf = mma == capi.MMA_BF16
+    make = _bf if bf else (lambda s, i, sh: rng.normal(s, i, sh))
+    x, dy = [make(9, g, (T, I)) for g in range(groups)], [make(10, g, (T, O)) for g in range(groups)]
+    dx, ddy = ([DeviceBuffer.from_numpy(t, bf16=bf) for t in ts] for ts in (x, dy))
+    dw, first = DeviceBuffer(groups * I * O * 4), rng.normal(11, 0, (O,))
+    outs = [DeviceBuffer.from_numpy(first) for _ in range(24 * groups)]
+    for i in range(0, 24 * groups, groups):
+        check(gpu_lib.boat_cuda_weight_grads(mma, groups, I, O, T, _table(dx), _table(ddy), capi.CUDA_BF16 if bf else capi.CUDA_F32,
+                                             (C.c_void_p * groups)(*[dw.p.value + g * I * O * 4 for g in range(groups)]), _table(outs[i:i + groups]),
+                                             add), "weight_grads")
+    check(gpu_lib.boat_cuda_sync(), "sync")
+    for g in range(groups):
+        got = [b.numpy((O,)) for b in outs[g::groups]]
+        y = dy[g].astype(np.float64)
+        want, size = y.sum(0) + (first if add else 0), np.abs(y).sum(0) + np.abs(first)
+        assert (np.abs(got[0] - want) <= 4 * math.sqrt(T) * 2.0 ** -25 * size).all()         # as above
+        assert all(np.array_equal(got[0], b) for b in got)
+
+
 @pytest.mark.parametrize("n", [1, 4, 1023, 4096, 100003])
 def test_elementwise_over_several_arrays(gpu_lib, n):
     a = [rng.normal(5, i, (n,)) for i in range(4)]
