@@ -492,8 +492,7 @@ int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale,
     if (units <= 0 || S <= 0 || hs <= 0) return 0;
     if (int rc = ensure_init()) return rc;
     if (int rc = check_shape(units, S, hs)) return rc;
-    const void* from = attn_bwd_simt_makes_delta(S, io_type) ? O : nullptr;
-    DISPATCH_HS(launch_bwd, units, S, (int)hs, causal, scale, Q, K, V, from, dO, lse, delta, dQ, dK, dV);
+    DISPATCH_HS(launch_bwd, units, S, (int)hs, causal, scale, Q, K, V, O, dO, lse, delta, dQ, dK, dV);
 }
 
 }  // namespace boatcu

@@ -184,7 +184,8 @@ int gemm_simt_grads(int groups, int64_t T, int64_t I, int64_t O, const void* con
 int colsum_multi(const void* const* X, int x_type, int64_t rows, int64_t cols, float* const* out, int count);
 int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, int io_type, void* O, float* lse);
-// Where attn_bwd_simt_makes_delta says so it works delta out from O and dO; else `delta` is given (rowdot).
+// With O it works delta out from O and dO, for what attn_bwd_simt_makes_delta takes and where no result shares memory with O; without,
+// `delta` is given (rowdot).
 bool attn_bwd_simt_makes_delta(int64_t S, int io_type);
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, const void* O, const void* dO, const float* lse, const float* delta, int io_type,

@@ -26,6 +26,13 @@ static bool aligned16(std::initializer_list<const void*> tensors) {
     return (bits & 15) == 0;
 }
 
+// Whether any of `others`, `bytes` long each like `t`, shares memory with it.
+static bool overlaps(const void* t, std::initializer_list<const void*> others, size_t bytes) {
+    for (const void* o : others)
+        if ((uintptr_t)o < (uintptr_t)t + bytes && (uintptr_t)t < (uintptr_t)o + bytes) return true;
+    return false;
+}
+
 static int check_types(const char* who, int mma, int in_type) {
     if (mma < BOAT_MMA_FP32 || mma > BOAT_MMA_BF16) return set_error(10, "%s: unknown arithmetic %d", who, mma);
     if (in_type != BOAT_CUDA_F32 && in_type != BOAT_CUDA_BF16 && in_type != BOAT_CUDA_F32_TF32)
@@ -208,8 +215,10 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
     float* delta = (float*)scratch;
     size_t delta_bytes = ((size_t)units * (size_t)S * sizeof(float) + 255) & ~(size_t)255;
     tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && aligned16({Q, K, V, O, dO, dQ, dK, dV}) && attn_tc_supported(mma, units, S, hs, io_type);
-    // the BF16 kernel's launcher makes its own, pre-scaled
-    if (tensor_cores ? mma != BOAT_MMA_BF16 : !attn_bwd_simt_makes_delta(S, io_type)) {
+    // The BF16 kernel's launcher makes its own, pre-scaled.  CTAs of the CUDA-core kernel may, but read O while others write results:
+    // one that lies over O wants delta made before.
+    const bool own_delta = !tensor_cores && attn_bwd_simt_makes_delta(S, io_type) && !overlaps(O, {dQ, dK, dV}, (size_t)(units * S * hs) * type_size(io_type));
+    if (tensor_cores ? mma != BOAT_MMA_BF16 : !own_delta) {
         ProfileScope prof("attn_delta");
         if (int rc = rowdot(dO, O, io_type, units * S, hs, delta)) return rc;
     }
@@ -218,7 +227,7 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
                            (char*)scratch + delta_bytes, scratch_bytes - delta_bytes);
     {
         ProfileScope prof("attn_bwd_simt");
-        if (int rc = attn_bwd_simt(units, S, hs, causal, scale, Q, K, V, O, dO, lse, delta, io_type, dQ, dK, dV)) return rc;
+        if (int rc = attn_bwd_simt(units, S, hs, causal, scale, Q, K, V, own_delta ? O : nullptr, dO, lse, delta, io_type, dQ, dK, dV)) return rc;
     }
     if (mma == BOAT_MMA_TF32) {
         const int64_t n = units * S * hs;

@@ -167,7 +167,8 @@ int boat_cuda_attn_fwd(int mma, int64_t units, int64_t S, int64_t hs, int causal
  * Recomputes P = exp(scale*QK^T - lse) tile by tile and produces
  *   dV = P^T dO, dP = dO V^T, dS = P * (dP - delta) * scale, dQ = dS K, dK = dS^T Q
  * with delta_i = sum_d dO[i,d]*O[i,d] (equal to the reference's sum_j dP_ij P_ij,
- * attention.c:1472-1488).  `scratch` is device memory the kernels may use freely:
+ * attention.c:1472-1488).  dQ, dK or dV may lie over O; apart from that no result shares memory
+ * with an operand or another result.  `scratch` is device memory the kernels may use freely:
  * boat_cuda_attn_bwd_scratch_bytes() gives the size needed for a problem. */
 size_t boat_cuda_attn_bwd_scratch_bytes(int mma, int64_t units, int64_t S, int64_t hs);
 int boat_cuda_attn_bwd(int mma, int64_t units, int64_t S, int64_t hs, int causal, float scale,

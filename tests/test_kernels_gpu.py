@@ -190,6 +190,39 @@ def test_attention_core_matches_float64(gpu_lib, mma, hs, S, causal):
     assert np.abs(got["lse"] - ref["lse"]).max() <= (1e-4 if mma == capi.MMA_FP32 else 2e-2)
 
 
+# A result over O, of which the caller has no more need: the gradients of separate memory, also where the CTAs make delta themselves
+@pytest.mark.parametrize("over", [0, 1, 2], ids=["dq", "dk", "dv"])
+@pytest.mark.parametrize("mma,units,S,hs", [(capi.MMA_FP32, 600, 4, 16), (capi.MMA_FP32, 200, 100, 32), (capi.MMA_FP32, 40, 128, 64), (capi.MMA_FP32, 20, 200, 16),
+                                            (capi.MMA_TF32, 40, 300, 64), (capi.MMA_BF16, 40, 300, 64), (capi.MMA_BF16, 30, 100, 32)])
+def test_a_result_of_the_backward_may_lie_over_o(gpu_lib, mma, units, S, hs, over):
+    bf = mma == capi.MMA_BF16
+    io, es, n, shape = (capi.CUDA_BF16 if bf else capi.CUDA_F32), (2 if bf else 4), units * S * hs, (units, S, hs)
+    host = [rng.normal(12, i, shape) for i in range(4)]
+    q, k, v, go = (DeviceBuffer.from_numpy(rng.bf16_round(a) if bf else a, bf16=bf) for a in host)
+    scale, lse, nbytes = C.c_float(1.0 / np.sqrt(hs)), DeviceBuffer(units * S * 4), gpu_lib.boat_cuda_attn_bwd_scratch_bytes(mma, units, S, hs)
+    scratch, results = DeviceBuffer(max(nbytes, 256)), []
+    # the second half of O and the first of the result share memory in the last round
+    for shift in (None, 0, n // 2 // 8 * 8):
+        room = DeviceBuffer(2 * n * es)
+        o = C.c_void_p(room.p.value)
+        out = [DeviceBuffer(n * es) for _ in range(3)]
+        at = [b.p for b in out]
+        if shift is not None:
+            at[over] = C.c_void_p(room.p.value + shift * es)
+        check(gpu_lib.boat_cuda_attn_fwd(mma, units, S, hs, 1, scale, q.p, k.p, v.p, io, o, lse.p), "attn_fwd")
+        check(gpu_lib.boat_cuda_attn_bwd(mma, units, S, hs, 1, scale, q.p, k.p, v.p, o, go.p, lse.p, io, at[0], at[1], at[2], scratch.p, scratch.nbytes),
+              "attn_bwd")
+        check(gpu_lib.boat_cuda_sync(), "sync")
+        if shift is not None:
+            whole = room.numpy((2 * n,), bf16=bf)[shift:shift + n].reshape(shape)
+        results.append([whole if shift is not None and i == over else b.numpy(shape, bf16=bf) for i, b in enumerate(out)])
+    for got in results[1:]:
+        for i, (a, b) in enumerate(zip(got, results[0])):
+            # delta in another order of its sum (FP32: that path's tolerance), dQ in another order of its tiles (BF16: a unit of its last place
+            # is 2^-8 of the value); the rest is computed alike
+            assert np.isfinite(b).all() and rel(a, b) <= (2.0**-7 if bf and i == 0 else TOL[capi.MMA_FP32]), i
+
+
 @pytest.mark.parametrize("mma,hs", [(capi.MMA_BF16, 64), (capi.MMA_BF16, 128), (capi.MMA_TF32, 64)],
                          ids=["bf16_hs64", "bf16_hs128", "tf32_hs64"])
 @pytest.mark.parametrize("S", [2, 64, 127, 129, 200, 257, 500])
