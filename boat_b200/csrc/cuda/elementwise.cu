@@ -693,7 +693,7 @@ int boat_cuda_stage_copy(void* dst, const void* src, size_t bytes, int down) {
     if (int rc = ensure_init()) return rc;
     if (bytes > kStageKernelBytes || !aligned16(dst) || !aligned16(src) || bytes % 16) {
         ordinary_launch_next();
-    BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, stream()));
+        BOATCU_CHECK(cudaMemcpyAsync(dst, src, bytes, down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, stream()));
         return 0;
     }
     const int64_t n = (int64_t)(bytes / 16);
