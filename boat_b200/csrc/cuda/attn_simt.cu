@@ -481,10 +481,17 @@ int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale,
     DISPATCH_HS(launch_fwd, units, S, (int)hs, causal, scale, Q, K, V, O, lse);
 }
 
-// Up to two tiles the CTAs make delta themselves: they read O and dO once per walk, and a launch is saved.
-// Beyond, a pass of its own reads them once.  8 units of 64 x 16: 7.3 us with the pass, 6.2 without; 32 units of 250 x 32: 37.7 and
-// 38.8.
-bool attn_bwd_simt_makes_delta(int64_t S, int io_type) { return io_type == BOAT_CUDA_F32 && S <= 2 * kRows; }
+// Where the launch of a pass for delta (1.1 to 1.4 us) is more than what each CTA's reading of O and dO costs: up to eight CTAs of 64
+// rows per SM, one tile, or two of head size 64 and less.  With the pass and without, us, operands in L2:
+//   8 units of 64 x 16       7.1    6.0        64 units of 64 x 64     15.8   14.7      512 units of 64 x 64     81.4   80.8
+//   2048 units of 8 x 16    91.6   94.9        2048 units of 64 x 64    310    314      8192 units of 8 x 64     1051   1107
+//   64 units of 128 x 16    18.1   17.0        64 units of 100 x 32    21.7   20.8      512 units of 100 x 16    70.0   71.4
+//   8 units of 128 x 64     18.6   18.5        64 units of 128 x 64    34.9   35.5      512 units of 128 x 64     215    220
+//   8 units of 100 x 128    34.2   34.9        64 units of 128 x 128   83.2   87.6      64 units of 192 x 32     34.8   35.4
+bool attn_bwd_simt_makes_delta(int64_t units, int64_t S, int64_t hs, int io_type) {
+    const int64_t tiles = ceil_div(S, kRows);
+    return io_type == BOAT_CUDA_F32 && 2 * units * tiles < 8 * (int64_t)sm_count() && (tiles == 1 || (tiles == 2 && hs <= 64));
+}
 
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, const void* O, const void* dO, const float* lse, const float* delta, int io_type, void* dQ,

@@ -186,7 +186,7 @@ int attn_fwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale,
                   const void* V, int io_type, void* O, float* lse);
 // With O it works delta out from O and dO, for what attn_bwd_simt_makes_delta takes and where no result shares memory with O; without,
 // `delta` is given (rowdot).
-bool attn_bwd_simt_makes_delta(int64_t S, int io_type);
+bool attn_bwd_simt_makes_delta(int64_t units, int64_t S, int64_t hs, int io_type);
 int attn_bwd_simt(int64_t units, int64_t S, int64_t hs, int causal, float scale, const void* Q, const void* K,
                   const void* V, const void* O, const void* dO, const float* lse, const float* delta, int io_type,
                   void* dQ, void* dK, void* dV);

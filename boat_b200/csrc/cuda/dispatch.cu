@@ -217,7 +217,7 @@ int attn_bwd_core(int mma, bool tensor_cores, int64_t units, int64_t S, int64_t 
     tensor_cores = tensor_cores && mma != BOAT_MMA_FP32 && aligned16({Q, K, V, O, dO, dQ, dK, dV}) && attn_tc_supported(mma, units, S, hs, io_type);
     // The BF16 kernel's launcher makes its own, pre-scaled.  CTAs of the CUDA-core kernel may, but read O while others write results:
     // one that lies over O wants delta made before.
-    const bool own_delta = !tensor_cores && attn_bwd_simt_makes_delta(S, io_type) && !overlaps(O, {dQ, dK, dV}, (size_t)(units * S * hs) * type_size(io_type));
+    const bool own_delta = !tensor_cores && attn_bwd_simt_makes_delta(units, S, hs, io_type) && !overlaps(O, {dQ, dK, dV}, (size_t)(units * S * hs) * type_size(io_type));
     if (tensor_cores ? mma != BOAT_MMA_BF16 : !own_delta) {
         ProfileScope prof("attn_delta");
         if (int rc = rowdot(dO, O, io_type, units * S, hs, delta)) return rc;

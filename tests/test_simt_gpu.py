@@ -48,6 +48,14 @@ def test_exact_attention_core_edges(gpu_lib, S, hs, causal):
         assert rel(got[key], ref[key]) <= 1e-5, key
 
 
+# delta made by the CTAs or by a pass of its own: the last and first numbers of units, tiles and head sizes of either (148 SMs)
+@pytest.mark.parametrize("units,S,hs", [(591, 6, 16), (592, 6, 16), (295, 65, 16), (296, 65, 16), (5, 128, 64), (5, 128, 65), (5, 129, 16)])
+def test_attention_backward_with_delta_of_either_kind(gpu_lib, units, S, hs):
+    got, ref = run_core(gpu_lib, capi.MMA_FP32, units, S, hs, True)
+    for key in ("dq", "dk", "dv"):
+        assert rel(got[key], ref[key]) <= 1e-5, key
+
+
 @pytest.mark.parametrize("S,hs", [(70, 16), (129, 32), (66, 80)])
 def test_cuda_core_attention_on_bf16_storage(gpu_lib, S, hs):
     got, ref = run_core(gpu_lib, capi.MMA_BF16, 2, S, hs, True)
