@@ -313,14 +313,6 @@ enum { MAX_CHUNKS = 8 };
  * per activation tensor (40 us of PCIe) on.  Below, a call sends what it needs up front. */
 #define PIPELINE_MIN_BYTES ((size_t)2 << 20)
 
-/* boat_cuda_linear_grads where there is one: a program may bring kernels of its own with fewer entries. */
-#pragma weak boat_cuda_linear_grads
-static int linear_grads(int mma, int groups, int64_t T, int64_t H, const void* const* x, const void* const* dy, const void* const* w,
-                        void* const* dx, float* const* dw, float* const* db) {
-    if (!boat_cuda_linear_grads) return 13;
-    return boat_cuda_linear_grads(mma, groups, T, H, H, x, dy, w, dx, dw, db);
-}
-
 static bool on_host(const boat_tensor_t* t) { return t->device != BOAT_DEVICE_CUDA; }
 
 /* BOAT_HOST_PIPELINE=0 in the environment selects the one-piece path for host tensors too. */
@@ -942,7 +934,7 @@ static bool backward_steps(boat_attention_t* a, const boat_tensor_t* grad_output
     {
         const void* x[1] = {a->d_ctx};
         const void* dy[1] = {d_go};
-        int rc = linear_grads(mma, 1, T, H, x, dy, (const void* const*)&p.w[WO], &d_dctx, &d_dw[WO], bias ? &d_db[WO] : NULL);
+        int rc = boat_cuda_linear_grads(mma, 1, T, H, H, x, dy, (const void* const*)&p.w[WO], &d_dctx, &d_dw[WO], bias ? &d_db[WO] : NULL);
         if (rc == 13) {
             rc = boat_cuda_gemm(mma, 0, 1, T, H, H, d_go, H, p.w[WO], H, type, d_dctx, H, feed_type(mma, type), NULL);
             if (rc == 0) rc = boat_cuda_weight_grads(mma, 1, H, H, T, x, dy, type, &d_dw[WO], bias ? &d_db[WO] : NULL, 0);
@@ -984,8 +976,8 @@ static bool backward_steps(boat_attention_t* a, const boat_tensor_t* grad_output
             target[i] = gin[i]->device == BOAT_DEVICE_CUDA ? gin[i]->data : (char*)d_down + down_at[k++];
             fp32 = fp32 && storage_of(gin[i]->dtype) == BOAT_CUDA_F32;
         }
-        const int rc = fp32 ? linear_grads(mma, 3, T, H, (const void* const*)a->d_in, (const void* const*)d_dproj, (const void* const*)p.w,
-                                           target, d_dw, bias ? d_db : NULL)
+        const int rc = fp32 ? boat_cuda_linear_grads(mma, 3, T, H, H, (const void* const*)a->d_in, (const void* const*)d_dproj,
+                                                     (const void* const*)p.w, target, d_dw, bias ? d_db : NULL)
                             : 13;
         if (rc != 13 && boat_report("dW and dX", rc) != 0) goto done;
         both = rc == 0;

@@ -94,6 +94,12 @@ int boat_cuda_weight_grads(int mma, int g, int64_t I, int64_t O, int64_t T, cons
     (void)mma; (void)g; (void)I; (void)O; (void)T; (void)X; (void)dY; (void)it; (void)dW; (void)db; (void)acc;
     return step();
 }
+/* the packed calls have both pairs of products in one launch, the larger ones are told 13: by launches of their own */
+int boat_cuda_linear_grads(int mma, int g, int64_t T, int64_t I, int64_t O, const void* const* X, const void* const* dY, const void* const* W, void* const* dX,
+                           float* const* dW, float* const* db) {
+    (void)mma; (void)g; (void)I; (void)O; (void)X; (void)dY; (void)W; (void)dX; (void)dW; (void)db;
+    return T <= 8 ? step() : 13;
+}
 int boat_cuda_attn_fwd(int mma, int64_t u, int64_t S, int64_t hs, int c, float sc, const void* Q, const void* K, const void* V, int t, void* O, float* lse) {
     (void)mma; (void)u; (void)S; (void)hs; (void)c; (void)sc; (void)Q; (void)K; (void)V; (void)t; (void)O; (void)lse;
     return step();
