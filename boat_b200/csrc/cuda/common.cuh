@@ -62,10 +62,13 @@ __device__ __forceinline__ void griddep_sync() {
 // complete when they run.  A successor that also names its memory, and touches none that matters to the kernels which may still
 // be running, does not wait for them (kBeside): a weight gradient beside an input gradient, a conversion beside either.  It
 // fills the SMs as they come free, without the gap between two launches, and waits for its predecessor at its
-// end instead, so that its completion still implies that of all kernels before it.
+// end instead, so that its completion still implies that of all kernels before it.  A weight gradient that is split along K
+// and overwrites its output waits behind the launch that clears it, and so for what is before that; what follows it may run
+// beside it.
 // Only within a sequence (boat_cuda_launches_begin): the first launch of one, and every launch outside one, waits for whatever is
 // before it on the stream, a program's own kernels or NCCL's too (launch_order.h).
-// Encoder block of 4 x 333 x 768 BF16: 227 us with every kernel waiting, 217 so; residual attention of 4 x 250 x 256 FP32 155 and 147.
+// The step with every kernel waiting and so: encoder block of 4 x 333 x 768 BF16 225 us and 218, residual attention of 4 x 250 x 256
+// FP32 149 and 142, 8 x 512 x 512 TF32 177 and 171, 8 x 1000 x 1024 BF16 350 and 345; a lone forward of 1 x 128 x 1024 23 and 23.
 enum Follow { kRelease = 1, kBeside = 2 };
 __device__ __forceinline__ void griddep_enter(int follow) {
     if (follow != kBeside) asm volatile("griddepcontrol.wait;" ::: "memory");
