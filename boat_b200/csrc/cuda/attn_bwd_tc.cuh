@@ -64,10 +64,11 @@ struct BwdCfg {
     // dQ read-out is not needed before the tile after next
     static constexpr int Q_STAGES = HS == 64 ? 3 : 2;
     static constexpr int KV_BUFS = HS == 64 ? 2 : 1;          // K and V of this walk, and of the next where they fit
-    // K,V + Q,dO stages + dS^T + two (lse, delta) buffers + barriers.  With head size 128 this
-    // is 231,808 of the 232,448 bytes a CTA may have, so the base must come 1024-byte aligned
-    // from the launch (checked at kernel entry) - there is no room for manual alignment slack.
+    // K,V + Q,dO stages + dS^T + dQ + two (lse, delta) buffers + barriers.  There is no room for manual alignment slack, so the
+    // base must come 1024-byte aligned from the launch (checked at kernel entry).
     static constexpr int SMEM = KV_BUFS * 2 * TILE_BYTES + Q_STAGES * 2 * TILE_BYTES + DS_BYTES + DQ_BYTES + 2048 + 448;
+    static constexpr int kMaxSmem = 232448;                   // of a CTA
+    static_assert(SMEM <= kMaxSmem && SMEM + 1023 > kMaxSmem, "no room for alignment slack, and none needed");
     // tensor memory columns
     // R0 (columns 0..127) holds S^T, then P^T.  With head size 64 dP^T has 128 columns of its
     // own.  With head size 128 nothing is left (R0 + dQ + dV + dK = 512), and dP^T borrows the dQ
